@@ -253,7 +253,7 @@ int b200q_gptq_zero_dead_columns(const float* diag, int64_t diag_stride, int64_t
  * b200q_gptq_factor_workspace_bytes(K) bytes.
  *
  * Streams: all work is ordered on `stream`.  Unless the environment has B200Q_LOOKAHEAD=0, the
- * bulk of each rank-128 update is launched on a helper stream that the library creates once per
+ * bulk of each rank-512 update is launched on a helper stream that the library creates once per
  * (device, `stream`) and keeps; it is forked from and joined to `stream` with events before the
  * call returns, so callers see ordinary stream semantics (b200q_gptq_sweep does the same).  The
  * helper streams and the per-thread cache of TMA descriptors are the library's only hidden
@@ -294,17 +294,33 @@ int b200q_gptq_sweep(float* Wf, int64_t N, int64_t K, int64_t ldf, const float* 
  * per-module calls of gptq_quantize.py:67-264 are otherwise bound by launch overhead).  Every
  * pointer argument is a DEVICE array of `count` device pointers.
  *
- * b200q_gptq_factor_batched: H[i] (K x K floats, leading dimension ldh) -> U[i] in place, as
- * b200q_gptq_factor does, one thread block per problem; K <= 4096 (meant for K <= 2048).
- * scratch[i]: K*K floats each (b200q_gptq_factor_batched_workspace_bytes(K, count) in total).
- * status: int32 [count][4], cleared by the call; status[i][0] = B200Q_NOT_POSITIVE_DEFINITE and
- * status[i][1] = first bad column + 1 (in reversed column order) when problem i failed.
+ * b200q_gptq_factor_many: H[i] (K x K floats, leading dimension ldh) -> U[i] in place, as
+ * b200q_gptq_factor does, every launch serving all problems; K <= 4096.  workspace:
+ * b200q_gptq_factor_many_workspace_bytes(K, count) bytes, 16-byte aligned.  status: int32
+ * [count][4], cleared by the call; status[i][0] = B200Q_NOT_POSITIVE_DEFINITE and status[i][1] =
+ * first bad column + 1 (in reversed column order) when problem i failed, status[i][2] =
+ * B200Q_ERR_DEVICE if a bounded wait expired.
  *
- * b200q_gptq_sweep_batched: the sweep of b200q_gptq_sweep for `count` weights of one shape
- * [N, K], one quantisation scheme and one scale dtype, blocksize 128.  A thread block carries 64
- * rows of one weight through every column block, trailing updates included (float32 FMA).
- * U may be NULL (identity for all) and so may zp, col_group and global_scale (absent for all);
- * losses[i]: float [N]. */
+ * b200q_gptq_sweep_many: the sweep of b200q_gptq_sweep for `count` weights of one shape [N, K],
+ * one quantisation scheme and one scale dtype.  U may be NULL (identity for all) and so may zp,
+ * col_group and global_scale (absent for all); losses[i]: float [N].  Weights that share a factor
+ * share its operand form: distinct_u lists the `distinct` different factors and u_index (device
+ * int32 [count], NULL: one each) says which one weight i uses; U[i] == distinct_u[u_index[i]].
+ * workspace: b200q_gptq_sweep_many_workspace_bytes bytes, 16-byte aligned, status word first as in
+ * b200q_gptq_sweep.
+ *
+ * b200q_gptq_factor_batched / b200q_gptq_sweep_batched: the same two calls without a workspace
+ * argument (scratch[i], K*K floats each, is accepted and not used; blocksize must be 128): what
+ * they need is taken from the stream's memory pool and given back before they return. */
+size_t b200q_gptq_factor_many_workspace_bytes(int64_t K, int count);
+int b200q_gptq_factor_many(float* const* H, int count, int64_t K, int64_t ldh, void* workspace, int* status,
+                           void* stream);
+size_t b200q_gptq_sweep_many_workspace_bytes(int64_t N, int64_t K, int count, int distinct);
+int b200q_gptq_sweep_many(float* const* W, const float* const* U, const float* const* distinct_u, int distinct,
+                          const int32_t* u_index, const void* const* scale, int sdtype, const void* const* zp,
+                          const int32_t* const* col_group, const float* const* global_scale, float* const* losses,
+                          int count, int64_t N, int64_t K, int64_t ldw, int64_t ldu, const b200q_qargs* qa,
+                          void* workspace, void* stream);
 /* The gather / scatter around the batched sweep, for `count` weights of one shape (device arrays
  * of device pointers): Wf[i] = float32 copy of W[i] with its columns permuted by perm[i] (perm
  * NULL: identity for all) and the columns whose dead_diag[i][c] is 0 zeroed (dead_diag NULL: none),

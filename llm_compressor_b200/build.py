@@ -24,8 +24,8 @@ SOURCES = [
     "mse_observer.cu",
     "hessian_syrk.cu",
     "gptq_solve.cu",
+    "gptq_factor.cu",
     "gptq_sweep.cu",
-    "gptq_small.cu",
     "tgemm_tf32.cu",
 ]
 

@@ -1,13 +1,14 @@
-// GPTQ solve, part 2: the blockwise column sweep.
+// GPTQ solve, part 2: the column sweep, for one weight or a batch of weights of one shape.
 //
-// Rows of W are independent, so they are spread over lanes: a warp owns 32 rows of the current
-// 128-column block and each lane sweeps its own row (see sweep_block_kernel).  The 128x128
-// diagonal block of U sits in shared memory.  The quantisation error of the block goes to a
-// [N,128] scratch panel and the update of all later columns is one fp32-accurate tensor-core
-// tile GEMM  W[:, after] -= Err * U[block, after].
+// Rows of W are independent and the columns of a row form one dependent chain: quantise column i, divide the error
+// by U[i,i], subtract its multiple of U[i, i+1:] from the rest of the row.  The columns are taken in superblocks of
+// up to 512.  Inside one, a CTA carries 32 rows through all columns with everything in shared memory
+// (sweep_block_kernel); between superblocks the rest of the matrix takes W[:, after] -= Err * U[block, after] as one
+// fp32-accurate tensor-core product (tgemm).  What the reference calls its block size only orders float32 operations
+// and does not change the result otherwise, so it does not decide the split here.
 //
-// Rounding follows the reference's sequence of separate float32 operations (product, then
-// subtraction; true divisions), so that the propagated errors agree.
+// Each correction is one fused multiply-add (the reference rounds the product first), true divisions decide a code
+// wherever an ulp could matter.
 #include <cstdlib>
 
 #include "common.cuh"
@@ -16,266 +17,402 @@
 namespace b200q {
 namespace sweep {
 
-constexpr int kMaxBlock = 128;
-constexpr size_t kSweepHeaderBytes = 256;   // status word at the start of the workspace
+constexpr int kMaxBlock = 128;               // largest block size callers may ask for
+constexpr size_t kSweepHeaderBytes = 256;    // status word at the start of the workspace
+constexpr int kRows = 32;                    // rows of a CTA: a lane each
+constexpr int kMicro = 16;                   // columns a lane keeps in registers at a time
+constexpr int kThreads = 256;
+constexpr int WLD = kRows + 1;
+
+// One pointer per operand, or (table set) a device array with one per problem.
+template <class T> struct Ptr {
+  T* one; T* const* table;
+  __device__ __forceinline__ T* at(int b) const { return table ? table[b] : one; }
+};
 
 struct Params {
-  float* W; int64_t ldw; int64_t N; int64_t K;
-  const float* U; int64_t ldu;
-  const void* scale; const void* zp; const int32_t* col_group; const float* gscale;
+  Ptr<float> W; Ptr<const float> U; Ptr<const void> scale; Ptr<const void> zp;
+  Ptr<const int32_t> col_group; Ptr<const float> gscale; Ptr<float> losses;
+  int64_t N, K, ldw, ldu;
   int strategy, group_size, block_h, zp_kind;
   int64_t groups_per_row;
   QRange qr;
-  float* err_hi; float* err_lo; int64_t lde;   // the block's errors [N, lde] as the hi / lo operand split of the
-                                               // trailing update's tile products (null: no trailing update)
-  float* losses;
-  int i1, bs;                // block start and width (<= 128)
-  int first;                 // first block: losses are overwritten
+  float* err_hi; float* err_lo; int64_t lde, err_batch;   // operand form of the superblock's errors (null: nothing after it)
+  int i1, sb;                                             // superblock: first column, width
 };
 
-// SB: scale tensor is bf16 (and no global scale) -> dequantised value rounded to bf16.
-//
-// Lane-per-row version.  A warp owns 32 rows; lane r keeps row r of the current 16-column
-// sub-block in registers, so the quantisation of a column is done once per row (not once per
-// lane) and the rank-1 corrections inside the sub-block are plain register arithmetic with the
-// row of U broadcast from shared memory.  The other columns of the 128-column block sit in a
-// shared-memory tile (column-major, one word per row and column: lanes hit distinct banks) and
-// take the 16 corrections of a finished sub-block in one pass, column by column, in the same
-// order of operations as the column-at-a-time formulation (product, then subtraction), so the
-// results are bit-identical to it.
-constexpr int kMaxWarps = 8;      // warps of a CTA that own row batches
-constexpr int kCtaThreads = 256;  // all threads help with the loads of the U block
-constexpr int kSub = 16;          // columns kept in registers at a time (code size grows with its square)
-
-__host__ __device__ inline size_t sweep_smem_bytes(int warps) {
-  return ((size_t)kMaxBlock * kMaxBlock + (size_t)kMaxBlock * (32 * warps + 1) + 64) * sizeof(float);
+__host__ __device__ constexpr size_t smem_bytes(int superblock) {
+  return (size_t)(superblock * WLD            // W, column-major
+                  + 3 * kMicro * superblock   // rows of U of three micro-blocks
+                  + 2 * kMicro * WLD          // errors of two micro-blocks
+                  + 2 * 3 * kMicro * kRows    // scale, 1 / scale, zero point of two micro-blocks
+                  + 2 * superblock) * sizeof(float);   // 1 / U[i,i], parameter column
 }
 
-// KIND: the code type (CodeKind), a compile-time constant so that the quantisation of a column - the
-// critical path of the whole sweep - is a short inline sequence without dispatch.
+__device__ __forceinline__ void cp_async16(float* dst, const float* src, int src_bytes) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(src_bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ void fma2(uint64_t& d, uint64_t a, uint64_t b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ uint64_t pair(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpair(uint64_t v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+
+// What bounds it: the chain of 512 columns, about 65 cycles each for the quantisation (product with 1 / s at both
+// ends of an interval, clamp, round, dequantise, difference, product with the reciprocal pivot, correction of the
+// next column).  So one warp of the CTA does nothing but the chain: 16 columns at a time in registers, a lane per
+// row.  The other seven apply a finished micro-block's 16 errors to the columns two micro-blocks on and later (the
+// columns next in line are corrected by the chain warp itself), write its errors out as the operand of the trailing
+// product, and fetch parameters and rows of U ahead.  One barrier per micro-block.
 template <int SDT, bool GLOBAL, int KIND>
-__global__ void __launch_bounds__(kCtaThreads) sweep_block_kernel(Params p, int warps) {
+__global__ void __launch_bounds__(kThreads) sweep_block_kernel(const __grid_constant__ Params p, int superblock) {
   constexpr bool SB = Elem<SDT>::is_bf16 && !GLOBAL;
   const float qmin = p.qr.qmin, qmax = p.qr.qmax;
-  extern __shared__ float sm[];
-  const int WLD = 32 * warps + 1;
-  float* sU = sm;                                   // [128][128] row i, local column c (identity when U is null)
-  float* sW = sU + kMaxBlock * kMaxBlock;           // [128][WLD] column c, row slot
-  __shared__ float s_rd[kMaxBlock];                 // 1 / U[i][i]
-  __shared__ int s_grp[kMaxBlock];                  // parameter column (group / block column) of each column
-  __shared__ int s_same[kMaxBlock / kSub];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int bs = p.bs;
-  // U block (only c >= r is ever read): 16-byte loads when the layout allows, several in flight
-  {
-    const bool vec = p.U && ((p.ldu & 3) == 0) && ((((uintptr_t)p.U) & 15) == 0) && ((p.i1 & 3) == 0);
-    constexpr int kQuads = kMaxBlock * kMaxBlock / 4;
-#pragma unroll 4
-    for (int idx = threadIdx.x; idx < kQuads; idx += blockDim.x) {
-      const int r = idx >> 5, c = (idx & 31) << 2;
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (r < bs && c + 3 >= r) {
-        if (!p.U) {
-          v.x = (r == c) ? 1.0f : 0.0f; v.y = (r == c + 1) ? 1.0f : 0.0f;
-          v.z = (r == c + 2) ? 1.0f : 0.0f; v.w = (r == c + 3) ? 1.0f : 0.0f;
-        } else {
-          const float* src = p.U + (int64_t)(p.i1 + r) * p.ldu + (p.i1 + c);
-          if (vec && c + 3 < bs) {
-            v = *reinterpret_cast<const float4*>(src);
-          } else {
-            if (c < bs) v.x = src[0];
-            if (c + 1 < bs) v.y = src[1];
-            if (c + 2 < bs) v.z = src[2];
-            if (c + 3 < bs) v.w = src[3];
-          }
+  extern __shared__ __align__(16) float sm[];
+  float* sU = sm;                                      // [3][kMicro][superblock]
+  float* sP = sU + 3 * kMicro * superblock;            // [2][3][kMicro][kRows]
+  float* sRd = sP + 2 * 3 * kMicro * kRows;            // [superblock]
+  int* sGrp = reinterpret_cast<int*>(sRd + superblock);// [superblock]
+  float* sE = sRd + 2 * superblock;                    // [2][kMicro][WLD]
+  float* sW = sE + 2 * kMicro * WLD;                   // [superblock][WLD]
+  const int job = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int sb = p.sb, micros = (sb + kMicro - 1) / kMicro;
+  float* __restrict__ W = p.W.at(job) + p.i1;
+  const float* __restrict__ U = p.U.at(job);
+  if (U) U += (int64_t)p.i1 * p.ldu + p.i1;
+  const void* scale = p.scale.at(job);
+  const void* zp = p.zp.at(job);
+  const int32_t* col_group = p.col_group.at(job);
+  const float g = GLOBAL ? *p.gscale.at(job) : 1.0f;
+  const int64_t row0 = (int64_t)blockIdx.x * kRows, row = row0 + lane;
+  const bool live = row < p.N;
+  const bool vecu = U && ((p.ldu & 3) == 0) && ((((uintptr_t)U) & 15) == 0);
+  int64_t pbase;
+  switch (p.strategy) {
+    case B200Q_TENSOR: pbase = 0; break;
+    case B200Q_CHANNEL: pbase = row; break;
+    case B200Q_BLOCK: pbase = (row / p.block_h) * p.groups_per_row; break;
+    default: pbase = row * p.groups_per_row; break;
+  }
+  // rows of U of micro-block m, columns from its own first one on (columns beyond sb are zero)
+  auto fetch_u = [&](int m, int t0, int nt) {
+    float* dst = sU + (m % 3) * kMicro * superblock;
+    const int c0 = m * kMicro, quads = (micros * kMicro - c0) >> 2;
+    for (int idx = t0; idx < kMicro * quads; idx += nt) {
+      const int t = idx / quads, c = c0 + (idx - t * quads) * 4, i = c0 + t;
+      float* d = dst + t * superblock + c;
+      if (vecu) {
+        const int bytes = (i < sb && c < sb) ? (sb - c >= 4 ? 16 : (sb - c) * 4) : 0;
+        cp_async16(d, bytes ? U + (int64_t)i * p.ldu + c : U, bytes);
+      } else {
+        for (int k = 0; k < 4; ++k) {
+          float v = (i == c + k) ? 1.0f : 0.0f;
+          if (U) v = (i < sb && c + k < sb) ? U[(int64_t)i * p.ldu + c + k] : 0.0f;
+          d[k] = v;
         }
       }
-      *reinterpret_cast<float4*>(sU + idx * 4) = v;
     }
-  }
-  for (int i = threadIdx.x; i < kMaxBlock; i += blockDim.x) {
+    cp_async_commit();
+  };
+  // parameters of micro-block m's columns for the CTA's rows (columns beyond sb: unit scale)
+  auto fetch_params = [&](int m, int w0, int nw) {
+    float* dst = sP + (m & 1) * 3 * kMicro * kRows + lane;
+#pragma unroll 3
+    for (int t = w0; t < kMicro; t += nw) {
+      const int c = m * kMicro + t;
+      float s = 1.0f, z = 0.0f;
+      if (c < sb && live) {
+        const int64_t pi = pbase + sGrp[c];
+        s = Elem<SDT>::load((const typename Elem<SDT>::type*)scale + pi);
+        if (GLOBAL) s = __fdiv_rn(s, g);
+        if (zp) z = load_zp(zp, p.zp_kind, pi);
+      }
+      dst[t * kRows] = s;
+      dst[(kMicro + t) * kRows] = __frcp_rn(s);
+      dst[(2 * kMicro + t) * kRows] = z;
+    }
+  };
+  fetch_u(0, tid, kThreads);
+  if (micros > 1) fetch_u(1, tid, kThreads); else cp_async_commit();
+  for (int c = tid; c < micros * kMicro; c += kThreads) {
     float d = 1.0f;
     int grp = 0;
-    if (i < bs) {
-      if (p.U) d = p.U[(int64_t)(p.i1 + i) * p.ldu + (p.i1 + i)];
-      const int col = p.i1 + i;
-      grp = (p.strategy == B200Q_TENSOR || p.strategy == B200Q_CHANNEL)
-                ? 0 : (p.col_group ? p.col_group[col] : col / p.group_size);
+    if (c < sb) {
+      if (U) d = U[(int64_t)c * p.ldu + c];
+      const int col = p.i1 + c;
+      grp = (p.strategy == B200Q_TENSOR || p.strategy == B200Q_CHANNEL) ? 0 : (col_group ? col_group[col] : col / p.group_size);
     }
-    s_rd[i] = __frcp_rn(d);
-    s_grp[i] = grp;
+    sRd[c] = __frcp_rn(d);
+    sGrp[c] = grp;
+  }
+  // tile in: rows coalesced, columns transposed; a warp takes four rows
+  for (int r = warp * 4; r < warp * 4 + 4; ++r) {
+    const bool in = row0 + r < p.N;
+    const float* src = W + (row0 + r) * p.ldw;
+#pragma unroll 4
+    for (int c = lane; c < micros * kMicro; c += 32) sW[c * WLD + r] = (in && c < sb) ? src[c] : 0.0f;
   }
   __syncthreads();
-  if (threadIdx.x < kMaxBlock / kSub) {   // does one (scale, zero point) govern the whole sub-block?
-    bool same = true;
-    for (int t = 1; t < kSub; ++t) same = same && s_grp[threadIdx.x * kSub + t] == s_grp[threadIdx.x * kSub];
-    s_same[threadIdx.x] = same ? 1 : 0;
-  }
+  fetch_params(0, warp, kThreads / 32);
+  cp_async_wait<1>();
   __syncthreads();
-  const float g = GLOBAL ? *p.gscale : 1.0f;
-  const bool has_zp = p.zp != nullptr;
-  float* myW = sW + warp * 32;   // this warp's 32 row slots
-  const int64_t batches = (p.N + 31) / 32;
-  if (warp >= warps) return;   // no CTA-wide barrier below this point
 
-  for (int64_t batch = (int64_t)blockIdx.x * warps + warp; batch < batches; batch += (int64_t)gridDim.x * warps) {
-    const int64_t row0 = batch * 32, row = row0 + lane;
-    const bool live = row < p.N;
-    // tile in: coalesced rows, transposed into the column-major tile
-#pragma unroll 8
-    for (int r = 0; r < 32; ++r) {
-      const int64_t rr = row0 + r;
+  float loss = 0.0f;
+  float e[kMicro];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int c = lane + 32 * k;
-        float v = 0.0f;
-        if (rr < p.N && c < bs) v = p.W[rr * p.ldw + p.i1 + c];
-        myW[c * WLD + r] = v;
-      }
-    }
-    __syncwarp();
-    int64_t pbase;
-    switch (p.strategy) {
-      case B200Q_TENSOR: pbase = 0; break;
-      case B200Q_CHANNEL: pbase = row; break;
-      case B200Q_BLOCK: pbase = (row / p.block_h) * p.groups_per_row; break;
-      default: pbase = row * p.groups_per_row; break;
-    }
-    float loss = 0.0f;
-    int cur_grp = -1;
-    float s = 1.0f, z = 0.0f, rs = 1.0f;
+  for (int t = 0; t < kMicro; ++t) e[t] = 0.0f;
 #pragma unroll 1
-    for (int sub = 0; sub * kSub < bs; ++sub) {
-      const int c0 = sub * kSub;
-      // Quantisation parameters of the sub-block's columns, fetched before the dependent chain
-      // starts.  Columns at or beyond bs (the ragged last block) are zero columns with a unit
-      // pivot and zero rows of U: they run through the same code and change nothing.
-      float sv[kSub], rsv[kSub], zv[kSub];
-      if (s_same[sub]) {   // uniform
-        const int grp = s_grp[c0];
-        if (grp != cur_grp) {
-          cur_grp = grp;
-          if (live) {
-            const int64_t pi = pbase + grp;
-            s = Elem<SDT>::load((const typename Elem<SDT>::type*)p.scale + pi);
-            if (GLOBAL) s = __fdiv_rn(s, g);
-            rs = __frcp_rn(s);
-            if (has_zp) z = load_zp(p.zp, p.zp_kind, pi);
+  for (int m = 0; m < micros; ++m) {
+    const int c0 = m * kMicro;
+    const float* u_prev = sU + ((m + 2) % 3) * kMicro * superblock;
+    if (warp == 0) {
+      const float* u = sU + (m % 3) * kMicro * superblock + c0;
+      float w[kMicro];
+      {
+        // the errors of the micro-block before this one
+        uint64_t v[kMicro / 2];
+#pragma unroll
+        for (int k = 0; k < kMicro / 2; ++k) v[k] = pair(sW[(c0 + 2 * k) * WLD + lane], sW[(c0 + 2 * k + 1) * WLD + lane]);
+        if (m > 0) {
+#pragma unroll
+          for (int t = 0; t < kMicro; ++t) {
+            const uint64_t ne = pair(-e[t], -e[t]);
+#pragma unroll
+            for (int k = 0; k < kMicro / 4; ++k) {
+              const ulonglong2 uu = *reinterpret_cast<const ulonglong2*>(u_prev + t * superblock + c0 + 4 * k);
+              fma2(v[2 * k], ne, uu.x);
+              fma2(v[2 * k + 1], ne, uu.y);
+            }
           }
         }
 #pragma unroll
-        for (int t = 0; t < kSub; ++t) { sv[t] = s; rsv[t] = rs; zv[t] = z; }
-      } else {             // act-order: every column may have its own group
-        cur_grp = -1;
-#pragma unroll
-        for (int t = 0; t < kSub; ++t) {
-          float st = 1.0f, zt = 0.0f;
-          if (live) {
-            const int64_t pi = pbase + s_grp[c0 + t];
-            st = Elem<SDT>::load((const typename Elem<SDT>::type*)p.scale + pi);
-            if (GLOBAL) st = __fdiv_rn(st, g);
-            if (has_zp) zt = load_zp(p.zp, p.zp_kind, pi);
-          }
-          sv[t] = st; rsv[t] = __frcp_rn(st); zv[t] = zt;
-        }
+        for (int k = 0; k < kMicro / 2; ++k) unpair(v[k], w[2 * k], w[2 * k + 1]);
       }
-      float w[kSub], e[kSub], rd[kSub];
+      const float* par = sP + (m & 1) * 3 * kMicro * kRows + lane;
+      float sv[kMicro], rsv[kMicro], zv[kMicro], rd[kMicro];
 #pragma unroll
-      for (int t = 0; t < kSub; ++t) { w[t] = myW[(c0 + t) * WLD + lane]; rd[t] = s_rd[c0 + t]; }
+      for (int t = 0; t < kMicro; ++t) {
+        sv[t] = par[t * kRows]; rsv[t] = par[(kMicro + t) * kRows]; zv[t] = par[(2 * kMicro + t) * kRows];
+        rd[t] = sRd[c0 + t];
+      }
 #pragma unroll
-      for (int t = 0; t < kSub; ++t) {
-        const int i = c0 + t;
+      for (int t = 0; t < kMicro; ++t) {
         const float wi = w[t];
         const float q = fake_quant_f32<KIND, SB>(wi, sv[t], rsv[t], zv[t], qmin, qmax);
-        const float diff = __fsub_rn(wi, q);
         // loss and error use the reciprocal of the pivot (an ulp from the reference's divisions)
-        const float tt = __fmul_rn(diff, rd[t]);
+        const float tt = __fmul_rn(__fsub_rn(wi, q), rd[t]);
         loss = fmaf(tt, tt, loss);
         e[t] = tt;
         w[t] = q;
-        const float4* urow = reinterpret_cast<const float4*>(sU + i * kMaxBlock + c0);
 #pragma unroll
-        for (int k4 = (t + 1) / 4; k4 < kSub / 4; ++k4) {
-          const float4 u = urow[k4];
-          if (4 * k4 + 0 > t) w[4 * k4 + 0] = __fsub_rn(w[4 * k4 + 0], __fmul_rn(tt, u.x));
-          if (4 * k4 + 1 > t) w[4 * k4 + 1] = __fsub_rn(w[4 * k4 + 1], __fmul_rn(tt, u.y));
-          if (4 * k4 + 2 > t) w[4 * k4 + 2] = __fsub_rn(w[4 * k4 + 2], __fmul_rn(tt, u.z));
-          if (4 * k4 + 3 > t) w[4 * k4 + 3] = __fsub_rn(w[4 * k4 + 3], __fmul_rn(tt, u.w));
+        for (int k4 = (t + 1) / 4; k4 < kMicro / 4; ++k4) {
+          const float4 uu = *reinterpret_cast<const float4*>(u + t * superblock + 4 * k4);
+          if (4 * k4 + 0 > t) w[4 * k4 + 0] = fmaf(-tt, uu.x, w[4 * k4 + 0]);
+          if (4 * k4 + 1 > t) w[4 * k4 + 1] = fmaf(-tt, uu.y, w[4 * k4 + 1]);
+          if (4 * k4 + 2 > t) w[4 * k4 + 2] = fmaf(-tt, uu.z, w[4 * k4 + 2]);
+          if (4 * k4 + 3 > t) w[4 * k4 + 3] = fmaf(-tt, uu.w, w[4 * k4 + 3]);
         }
       }
-      // quantised values back into the tile; the errors go straight to the panel the trailing
-      // update reads: 16 consecutive floats per row
+      float* eo = sE + (m & 1) * kMicro * WLD + lane;
 #pragma unroll
-      for (int t = 0; t < kSub; ++t) myW[(c0 + t) * WLD + lane] = w[t];
-      if (live && p.err_hi) {
-        float4* dh = reinterpret_cast<float4*>(p.err_hi + row * p.lde + c0);
-        float4* dl = reinterpret_cast<float4*>(p.err_lo + row * p.lde + c0);
+      for (int t = 0; t < kMicro; ++t) { sW[(c0 + t) * WLD + lane] = w[t]; eo[t * WLD] = e[t]; }
+    } else {
+      if (m > 0) {
+        const float* ei = sE + ((m - 1) & 1) * kMicro * WLD + lane;
+        uint64_t ne[kMicro];
 #pragma unroll
-        for (int t = 0; t < kSub; t += 4) {
-          float h[4], l[4];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) { h[j] = tgemm::tf32_rn(e[t + j]); l[j] = tgemm::tf32_rn(e[t + j] - h[j]); }
-          dh[t / 4] = make_float4(h[0], h[1], h[2], h[3]);
-          dl[t / 4] = make_float4(l[0], l[1], l[2], l[3]);
-        }
-      }
-      // the later columns of the block take this sub-block's corrections: v -= e * u as a packed
-      // product and a packed sum with -e (two float32 lanes per instruction, each rounded like the
-      // scalar operations)
-      uint64_t ne2[kSub];
-#pragma unroll
-      for (int t = 0; t < kSub; ++t) asm("mov.b64 %0, {%1, %1};" : "=l"(ne2[t]) : "f"(-e[t]));
-      // eight columns per pass: four independent chains of packed sums hide the latency of the adds
-      // (the tile is 128 columns wide, so a ragged block's last pass stays inside it)
+        for (int t = 0; t < kMicro; ++t) { const float x = -ei[t * WLD]; ne[t] = pair(x, x); }
 #pragma unroll 1
-      for (int c = c0 + kSub; c < bs; c += 8) {
-        uint64_t v[4];
+        for (int c = c0 + kMicro + (warp - 1) * 8; c < micros * kMicro; c += 7 * 8) {
+          uint64_t v[4];
 #pragma unroll
-        for (int h = 0; h < 4; ++h)
-          asm("mov.b64 %0, {%1, %2};" : "=l"(v[h]) : "f"(myW[(c + 2 * h) * WLD + lane]), "f"(myW[(c + 2 * h + 1) * WLD + lane]));
+          for (int h = 0; h < 4; ++h) v[h] = pair(sW[(c + 2 * h) * WLD + lane], sW[(c + 2 * h + 1) * WLD + lane]);
 #pragma unroll
-        for (int t = 0; t < kSub; ++t) {
-          const ulonglong2 ua = *reinterpret_cast<const ulonglong2*>(sU + (c0 + t) * kMaxBlock + c);
-          const ulonglong2 ub = *reinterpret_cast<const ulonglong2*>(sU + (c0 + t) * kMaxBlock + c + 4);
-          const uint64_t u[4] = {ua.x, ua.y, ub.x, ub.y};
+          for (int t = 0; t < kMicro; ++t) {
+            const ulonglong2 ua = *reinterpret_cast<const ulonglong2*>(u_prev + t * superblock + c);
+            const ulonglong2 ub = *reinterpret_cast<const ulonglong2*>(u_prev + t * superblock + c + 4);
+            fma2(v[0], ne[t], ua.x); fma2(v[1], ne[t], ua.y); fma2(v[2], ne[t], ub.x); fma2(v[3], ne[t], ub.y);
+          }
 #pragma unroll
           for (int h = 0; h < 4; ++h) {
-            uint64_t pr;
-            asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(pr) : "l"(ne2[t]), "l"(u[h]));
-            asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v[h]) : "l"(v[h]), "l"(pr));
+            float lo, hi;
+            unpair(v[h], lo, hi);
+            sW[(c + 2 * h) * WLD + lane] = lo; sW[(c + 2 * h + 1) * WLD + lane] = hi;
           }
         }
-#pragma unroll
-        for (int h = 0; h < 4; ++h) {
-          float lo, hi;
-          asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v[h]));
-          myW[(c + 2 * h) * WLD + lane] = lo; myW[(c + 2 * h + 1) * WLD + lane] = hi;
-        }
       }
+      if (m + 1 < micros) fetch_params(m + 1, warp - 1, 7);
     }
-    if (live && p.err_hi) {   // zero padding of the operand rows up to their leading dimension
-      for (int c = (bs + kSub - 1) / kSub * kSub; c < (int)p.lde; c += 4) {
-        *reinterpret_cast<float4*>(p.err_hi + row * p.lde + c) = make_float4(0.f, 0.f, 0.f, 0.f);
-        *reinterpret_cast<float4*>(p.err_lo + row * p.lde + c) = make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-    }
-    __syncwarp();
-    // tile out
-    for (int r = 0; r < 32; ++r) {
-      const int64_t rr = row0 + r;
-      if (rr >= p.N) break;
+    // the errors of micro-block `of`, four columns of a row per thread
+    auto store_errors = [&](int of, int t) {
+      const int r = t & 31, q = (t >> 5) * 4;
+      if (t >= 128 || row0 + r >= p.N) return;
+      const float* ei = sE + (of & 1) * kMicro * WLD + r;
+      float h[4], l[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        const int c = lane + 32 * k;
-        if (c < bs) p.W[rr * p.ldw + p.i1 + c] = myW[c * WLD + r];
+        const float x = ei[(q + k) * WLD];
+        h[k] = tgemm::tf32_rn(x);
+        l[k] = tgemm::tf32_rn(x - h[k]);
       }
+      const int64_t at = job * p.err_batch + (row0 + r) * p.lde + of * kMicro + q;
+      *reinterpret_cast<float4*>(p.err_hi + at) = make_float4(h[0], h[1], h[2], h[3]);
+      *reinterpret_cast<float4*>(p.err_lo + at) = make_float4(l[0], l[1], l[2], l[3]);
+    };
+    if (p.err_hi && m > 0 && warp > 0) store_errors(m - 1, tid - 32);
+    cp_async_wait<0>();
+    __syncthreads();
+    if (m + 2 < micros && warp > 0) {   // the buffer of micro-block m - 1 is free
+      fetch_u(m + 2, tid - 32, kThreads - 32);
     }
-    if (live) {
-      const float half = loss * 0.5f;
-      p.losses[row] = p.first ? half : p.losses[row] + half;
-    }
-    __syncwarp();
+    if (m + 1 == micros && p.err_hi) store_errors(m, tid);   // (a superblock with columns after it is a whole one)
   }
+  // tile out
+  for (int r = warp * 4; r < warp * 4 + 4; ++r) {
+    if (row0 + r >= p.N) break;
+    float* dst = W + (row0 + r) * p.ldw;
+#pragma unroll 4
+    for (int c = lane; c < sb; c += 32) dst[c] = sW[c * WLD + r];
+  }
+  if (warp == 0 && live) {
+    float* lo = p.losses.at(job);
+    const float half = loss * 0.5f;
+    lo[row] = p.i1 == 0 ? half : lo[row] + half;
+  }
+}
+
+// Superblock width.  With at most one CTA per SM the chain decides and 512 columns halve the launches and the traffic
+// of the trailing products; with more rows than that the CTA's own updates (width / 2 multiply-adds per element) do,
+// and 256 columns leave room for two CTAs per SM.
+static int superblock_of(int64_t ctas) { return ctas <= kNumSMs ? 512 : 256; }
+// The trailing product is split in the columns the next superblock needs and the rest on a helper stream only while
+// a superblock's CTAs leave half of the GPU idle.
+static bool look_ahead(int64_t ctas) { return ctas <= kNumSMs / 2; }
+
+struct Layout {
+  int sb, sets;
+  int64_t rows_n, rows_k, err, ub;   // rows per problem of the operands; floats of one hi or lo array
+  size_t bytes;
+};
+static Layout layout_of(int64_t N, int64_t K, int batch, int distinct_u, bool may_overlap) {
+  const int64_t ctas = (N + kRows - 1) / kRows * batch;
+  Layout l;
+  l.sb = superblock_of(ctas);
+  l.sets = may_overlap && look_ahead(ctas) ? 2 : 1;
+  l.rows_n = (N + 127) / 128 * 128; l.rows_k = (K + 127) / 128 * 128;
+  l.err = l.rows_n * l.sb * batch; l.ub = l.rows_k * l.sb * distinct_u;
+  l.bytes = kSweepHeaderBytes + (K > l.sb ? (size_t)(2 * l.sets * (l.err + l.ub)) * sizeof(float) : 0) + 64;
+  return l;
+}
+
+// `Ud` / `u_index`: the distinct factors of a batch and the one each problem uses (null: the single U, or one each)
+static int sweep(Params p, int sdtype, bool global, int batch, const float* const* Ud, int distinct_u,
+                 const int32_t* u_index, bool may_overlap, void* workspace, cudaStream_t st) {
+  const int64_t N = p.N, K = p.K;
+  const bool has_u = p.U.one || p.U.table;
+  const Layout l = layout_of(N, K, batch, distinct_u, may_overlap);
+  // header of the workspace: a status word that a bounded wait expiring inside one of the trailing products sets to
+  // B200Q_ERR_DEVICE (cleared here, read by the caller afterwards)
+  int* status = (int*)workspace;
+  float* err = (float*)((char*)workspace + kSweepHeaderBytes);   // [sets][hi, lo]
+  float* ub = err + 2 * l.sets * l.err;                          // [sets][hi, lo]
+  B200Q_TRY(cudaMemsetAsync(status, 0, sizeof(int), st));
+  void (*kern)(const Params, int) = nullptr;
+#define B200Q_SWEEP_PICK(SDT)                                                                                              \
+  do {                                                                                                                     \
+    if (p.qr.kind == kInt) kern = global ? sweep_block_kernel<SDT, true, kInt> : sweep_block_kernel<SDT, false, kInt>;      \
+    else if (p.qr.kind == kFp8) kern = global ? sweep_block_kernel<SDT, true, kFp8> : sweep_block_kernel<SDT, false, kFp8>; \
+    else kern = global ? sweep_block_kernel<SDT, true, kFp4> : sweep_block_kernel<SDT, false, kFp4>;                        \
+  } while (0)
+  if (sdtype == B200Q_BF16) B200Q_SWEEP_PICK(B200Q_BF16);
+  else if (sdtype == B200Q_F32) B200Q_SWEEP_PICK(B200Q_F32);
+  else return B200Q_ERR_UNSUPPORTED;
+#undef B200Q_SWEEP_PICK
+  // always the largest size: host threads on other streams launch the same kernel with other widths
+  B200Q_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(512)));
+  const int ctas = (int)((N + kRows - 1) / kRows);
+  tgemm::SideStream* side = l.sets == 2 && has_u && K > 2 * l.sb ? tgemm::side_stream(st) : nullptr;
+  bool side_busy = false;
+  int rc;
+  auto split_u = [&](int64_t i1, int which, cudaStream_t on) -> int {
+    // operand form of U[i1 : i1 + sb, i1 + sb :] (independent of the sweep: kept off its chain)
+    const int64_t i2 = i1 + l.sb;
+    if (i2 >= K) return B200Q_OK;
+    float* hi = ub + (int64_t)which * 2 * l.ub;
+    return tgemm::split_transposed(p.U.one ? p.U.one + i1 * p.ldu + i2 : nullptr, Ud, i1 * p.ldu + i2, p.ldu, l.sb,
+                                   (int)(K - i2), hi, hi + l.ub, l.sb, l.rows_k * l.sb, distinct_u, on);
+  };
+  if (has_u && (rc = split_u(0, 0, st))) return rc;
+  int blk = 0;
+  for (int64_t i1 = 0; i1 < K; i1 += l.sb, ++blk) {
+    const int w = (int)(K - i1 < l.sb ? K - i1 : l.sb), which = l.sets == 2 ? blk & 1 : 0;
+    const int64_t i2 = i1 + w;
+    const bool trailing = i2 < K && has_u;
+    p.i1 = (int)i1; p.sb = w;
+    p.err_hi = trailing ? err + (int64_t)which * 2 * l.err : nullptr;
+    p.err_lo = trailing ? p.err_hi + l.err : nullptr;
+    p.lde = l.sb; p.err_batch = l.rows_n * l.sb;
+    kern<<<dim3(ctas, batch), kThreads, smem_bytes(l.sb), st>>>(p, l.sb);
+    B200Q_LAUNCH_CHECK();
+    if (!trailing) continue;
+    // W[:, i2:] -= Err[N, w] * U[i1:i2, i2:]
+    float* bhi = ub + (int64_t)which * 2 * l.ub;
+    tgemm::Job j;
+    j.A = tgemm::Operand{p.err_hi, p.err_lo, l.sb, l.rows_n * batch, l.rows_n, 0};
+    j.B = tgemm::Operand{bhi, bhi + l.ub, l.sb, l.rows_k * distinct_u, l.rows_k, 0};
+    j.b_index = u_index;
+    j.M = (int)N; j.N = (int)(K - i2); j.Kd = w; j.batch = batch; j.alpha = -1.0f; j.beta = 1.0f;
+    if (p.W.one) j.C = p.W.one + i2;
+    j.c_table = p.W.table; j.c_offset = i2; j.ldc = p.ldw; j.status = status;
+    if (!side) {
+      if ((rc = tgemm::launch(j, st))) return rc;
+      if ((rc = split_u(i2, l.sets == 2 ? which ^ 1 : 0, st))) return rc;
+      continue;
+    }
+    tgemm::Job far = j;
+    if (j.N > l.sb) j.N = l.sb;
+    B200Q_TRY(cudaEventRecord(side->ready, st));
+    B200Q_TRY(cudaStreamWaitEvent(side->stream, side->ready, 0));
+    // the far columns of the superblock before, and this one's operand form of U made behind them
+    if (side_busy) B200Q_TRY(cudaStreamWaitEvent(st, side->done, 0));
+    if ((rc = tgemm::launch(j, st))) return rc;
+    if (far.N > l.sb) {
+      far.B.row0 = l.sb; far.N -= l.sb; far.max_ctas = kNumSMs - ctas * batch;
+      if (p.W.one) far.C = p.W.one + i2 + l.sb;
+      far.c_offset = i2 + l.sb;
+      if ((rc = tgemm::launch(far, side->stream))) return rc;
+    }
+    // the next superblock's slice of U: its buffer was last read by the superblock before this one
+    if ((rc = split_u(i2, which ^ 1, side->stream))) return rc;
+    B200Q_TRY(cudaEventRecord(side->done, side->stream));
+    side_busy = true;
+  }
+  if (side_busy) B200Q_TRY(cudaStreamWaitEvent(st, side->done, 0));
+  return B200Q_OK;
+}
+
+static int fill_scheme(Params* p, const b200q_qargs* qa, int64_t N, int64_t K, const int32_t* col_group) {
+  int rc = make_qrange(qa, &p->qr); if (rc) return rc;
+  ParamMap pm;
+  rc = make_param_map(qa, N, K, col_group, &pm); if (rc) return rc;
+  p->strategy = qa->strategy;
+  p->group_size = (qa->strategy == B200Q_BLOCK) ? qa->block_w : qa->group_size;
+  if (p->group_size <= 0) p->group_size = 1;
+  p->block_h = qa->block_h > 0 ? qa->block_h : 1;
+  p->zp_kind = qa->zp_kind;
+  p->groups_per_row = pm.groups_per_row;
+  return B200Q_OK;
 }
 
 }  // namespace sweep
@@ -286,12 +423,8 @@ using namespace b200q;
 extern "C" {
 
 size_t b200q_gptq_sweep_workspace_bytes(int64_t N, int64_t K, int blocksize) {
-  using b200q::sweep::kSweepHeaderBytes;
   if (N <= 0 || K <= 0 || blocksize <= 0) return 0;
-  // error panel [N][128] + two sets of (hi/lo copies of it, hi/lo copies of a 128-row panel of U):
-  // consecutive blocks alternate between the sets because of the look-ahead
-  const size_t np = (size_t)((N + 127) / 128 * 128), kp = (size_t)((K + 127) / 128 * 128);
-  return kSweepHeaderBytes + (np * 128 * 5 + 4 * 128 * kp) * sizeof(float) + 64;
+  return sweep::layout_of(N, K, 1, 1, true).bytes;
 }
 
 int b200q_gptq_sweep(float* Wf, int64_t N, int64_t K, int64_t ldf, const float* U, int64_t ldu, const void* scale,
@@ -303,130 +436,49 @@ int b200q_gptq_sweep(float* Wf, int64_t N, int64_t K, int64_t ldf, const float* 
   if (((uintptr_t)workspace) & 15) return B200Q_ERR_ARG;
   if (blocksize <= 0 || blocksize > kMaxBlock) return B200Q_ERR_UNSUPPORTED;
   Params p;
-  int rc = make_qrange(qa, &p.qr); if (rc) return rc;
-  ParamMap pm;
-  rc = make_param_map(qa, N, K, col_group, &pm); if (rc) return rc;
-  p.W = Wf; p.ldw = ldf; p.N = N; p.K = K; p.U = U; p.ldu = ldu;
-  p.scale = scale; p.zp = zp; p.col_group = col_group; p.gscale = gscale;
-  p.strategy = qa->strategy;
-  p.group_size = (qa->strategy == B200Q_BLOCK) ? qa->block_w : qa->group_size;
-  p.block_h = qa->block_h > 0 ? qa->block_h : 1;
-  p.zp_kind = qa->zp_kind;
-  p.groups_per_row = pm.groups_per_row;
-  // header of the workspace: a status word that a bounded wait expiring inside one of the
-  // trailing-update GEMMs sets to B200Q_ERR_DEVICE (cleared here, read by the caller afterwards)
-  int* gemm_status = (int*)workspace;
-  float* ws_f = (float*)((char*)workspace + kSweepHeaderBytes);
-  p.err_hi = p.err_lo = nullptr;
-  p.lde = tgemm::split_ld(blocksize);
-  const size_t np128 = (size_t)((N + 127) / 128 * 128) * 128, kp128 = (size_t)((K + 127) / 128 * 128) * 128;
-  float* sa_base = ws_f + np128;             // [2][hi, lo][np128]: the sweep kernel writes a block's errors here
-  float* sb_base = sa_base + 4 * np128;      // [2][hi, lo][kp128]
-  p.losses = losses;
+  int rc = fill_scheme(&p, qa, N, K, col_group); if (rc) return rc;
+  p.W = {Wf, nullptr}; p.U = {U, nullptr}; p.scale = {scale, nullptr}; p.zp = {zp, nullptr};
+  p.col_group = {col_group, nullptr}; p.gscale = {gscale, nullptr}; p.losses = {losses, nullptr};
+  p.N = N; p.K = K; p.ldw = ldf; p.ldu = ldu;
+  return sweep::sweep(p, sdtype, gscale != nullptr, 1, nullptr, 1, nullptr, true, workspace, (cudaStream_t)stream);
+}
+
+size_t b200q_gptq_sweep_many_workspace_bytes(int64_t N, int64_t K, int count, int distinct) {
+  if (N <= 0 || K <= 0 || count <= 0 || distinct <= 0) return 0;
+  return sweep::layout_of(N, K, count, distinct, false).bytes;
+}
+
+int b200q_gptq_sweep_many(float* const* W, const float* const* U, const float* const* distinct_u, int distinct,
+                          const int32_t* u_index, const void* const* scale, int sdtype, const void* const* zp,
+                          const int32_t* const* col_group, const float* const* gscale, float* const* losses, int count,
+                          int64_t N, int64_t K, int64_t ldw, int64_t ldu, const b200q_qargs* qa, void* workspace,
+                          void* stream) {
+  using namespace b200q::sweep;
+  if (!W || !scale || !losses || !qa || !workspace || count <= 0 || N <= 0 || K <= 0 || ldw < K || (U && ldu < K)) return B200Q_ERR_ARG;
+  if (count > 65535 || (U && (!distinct_u || distinct <= 0 || distinct > 65535)) || ((uintptr_t)workspace) & 15) return B200Q_ERR_ARG;
+  Params p;
+  int rc = fill_scheme(&p, qa, N, K, nullptr); if (rc) return rc;
+  p.W = {nullptr, W}; p.U = {nullptr, U}; p.scale = {nullptr, scale}; p.zp = {nullptr, zp};
+  p.col_group = {nullptr, col_group}; p.gscale = {nullptr, gscale}; p.losses = {nullptr, losses};
+  p.N = N; p.K = K; p.ldw = ldw; p.ldu = ldu;
+  return sweep::sweep(p, sdtype, gscale != nullptr, count, distinct_u, U ? distinct : 1, u_index, false, workspace,
+                      (cudaStream_t)stream);
+}
+
+int b200q_gptq_sweep_batched(float* const* W, const float* const* U, const void* const* scale, int sdtype,
+                             const void* const* zp, const int32_t* const* col_group, const float* const* gscale,
+                             float* const* losses, int count, int64_t N, int64_t K, int64_t ldw, int64_t ldu,
+                             const b200q_qargs* qa, int blocksize, void* stream) {
+  if (count <= 0 || N <= 0 || K <= 0) return B200Q_ERR_ARG;
+  if (blocksize != 128) return B200Q_ERR_UNSUPPORTED;
+  // no workspace in this entry point's arguments: taken from the stream's memory pool for the call
+  void* ws = nullptr;
   cudaStream_t st = (cudaStream_t)stream;
-  B200Q_TRY(cudaMemsetAsync(gemm_status, 0, sizeof(int), st));
-  // warps per CTA: one 32-row batch per warp; few rows -> small CTAs so that every SM gets work
-  const int64_t batches = (N + 31) / 32;
-  int warps = (int)((batches + kNumSMs - 1) / kNumSMs);
-  warps = warps < 1 ? 1 : (warps > kMaxWarps ? kMaxWarps : warps);
-  void (*kern)(Params, int) = nullptr;
-#define B200Q_SWEEP_PICK(SDT)                                                                              \
-  do {                                                                                                     \
-    if (p.qr.kind == kInt) kern = gscale ? sweep_block_kernel<SDT, true, kInt> : sweep_block_kernel<SDT, false, kInt>;      \
-    else if (p.qr.kind == kFp8) kern = gscale ? sweep_block_kernel<SDT, true, kFp8> : sweep_block_kernel<SDT, false, kFp8>; \
-    else kern = gscale ? sweep_block_kernel<SDT, true, kFp4> : sweep_block_kernel<SDT, false, kFp4>;       \
-  } while (0)
-  if (sdtype == B200Q_BF16) B200Q_SWEEP_PICK(B200Q_BF16);
-  else if (sdtype == B200Q_F32) B200Q_SWEEP_PICK(B200Q_F32);
-  else return B200Q_ERR_UNSUPPORTED;
-#undef B200Q_SWEEP_PICK
-  // always the largest size: host threads on other streams launch the same kernel with other sizes
-  B200Q_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)sweep_smem_bytes(kMaxWarps)));
-  // With the look-ahead the far part of a trailing update runs beside the next block's sweep and
-  // leaves `reserve` SMs to it: pack the row batches into that many CTAs when they fit (a warp is
-  // latency-bound, several per SM cost little).
-  tgemm::SideStream* side = U ? tgemm::side_stream(st) : nullptr;
-  static const int kSweepReserve = [] {
-    const char* e = getenv("B200Q_SWEEP_RESERVE");
-    const int v = e ? atoi(e) : 32;
-    return v < 8 ? 8 : (v > kNumSMs / 2 ? kNumSMs / 2 : v);
-  }();
-  int reserve = tgemm::side_reserve();
-  if (side && batches <= (int64_t)kSweepReserve * kMaxWarps) {
-    reserve = kSweepReserve;
-    const int w = (int)((batches + reserve - 1) / reserve);
-    if (w > warps) warps = w;
-  }
-  int64_t ctas = (batches + warps - 1) / warps;
-  const int grid = (int)(ctas < 2 * kNumSMs ? ctas : 2 * kNumSMs);
-  const size_t smem = sweep_smem_bytes(warps);
-  // Look-ahead: the trailing update of a block is split in the next 128 columns (which the next
-  // block's sweep reads; caller's stream) and the columns after them, which a helper stream
-  // updates while the next block is swept.
-  bool side_busy = false;
-  int blk = 0;
-  auto split_u = [&](int64_t j1, int which, cudaStream_t on) -> int {
-    // hi / lo operand form of U[j1 : j1 + bs, j1 + bs :] (independent of the sweep: kept off its chain)
-    const int bsj = (int)((K - j1) < blocksize ? (K - j1) : blocksize);
-    const int64_t j2 = j1 + bsj;
-    float* hi = sb_base + (size_t)which * 2 * kp128;
-    return tgemm::split_transposed(U + j1 * ldu + j2, ldu, bsj, (int)(K - j2), hi, hi + kp128, on);
-  };
-  if (U && K > blocksize) { rc = split_u(0, 0, st); if (rc) return rc; }
-  for (int64_t i1 = 0; i1 < K; i1 += blocksize, ++blk) {
-    const int bs = (int)((K - i1) < blocksize ? (K - i1) : blocksize);
-    const int64_t i2 = i1 + bs;
-    const bool trailing = i2 < K && U;
-    float* sa_hi = sa_base + (size_t)(blk & 1) * 2 * np128;
-    float* sa_lo = sa_hi + np128;
-    p.i1 = (int)i1; p.bs = bs; p.first = (i1 == 0);
-    p.err_hi = trailing ? sa_hi : nullptr; p.err_lo = trailing ? sa_lo : nullptr;
-    p.lde = tgemm::split_ld(bs);
-    kern<<<grid, kCtaThreads, smem, st>>>(p, warps);
-    B200Q_LAUNCH_CHECK();
-    if (trailing) {
-      // W[:, i2:] -= Err[N, bs] * U[i1:i2, i2:]   (3xTF32 on the tensor cores)
-      const int rest = (int)(K - i2);
-      float* sb_hi = sb_base + (size_t)(blk & 1) * 2 * kp128;
-      float* sb_lo = sb_hi + kp128;
-      const int64_t ld = tgemm::split_ld(bs);
-      const tgemm::Split A{sa_hi, sa_lo, ld};
-      const bool more = K - i2 > blocksize;     // the next block has a trailing update too
-      if (!side) {
-        rc = tgemm::launch(tgemm::kNT, A, tgemm::Split{sb_hi, sb_lo, ld}, Wf + i2, ldf, (int)N, rest, bs, -1.0f, 1.0f,
-                           tgemm::kAllTiles, gemm_status, st);
-        if (rc) return rc;
-        if (more) { rc = split_u(i2, (blk + 1) & 1, st); if (rc) return rc; }
-        continue;
-      }
-      const int near = rest < 128 ? rest : 128;
-      B200Q_TRY(cudaEventRecord(side->ready, st));
-      B200Q_TRY(cudaStreamWaitEvent(side->stream, side->ready, 0));
-      // the far columns of the block before, and this block's operand form of U made behind them
-      if (side_busy) B200Q_TRY(cudaStreamWaitEvent(st, side->done, 0));
-      rc = tgemm::launch(tgemm::kNT, A, tgemm::Split{sb_hi, sb_lo, ld}, Wf + i2, ldf, (int)N, near, bs, -1.0f, 1.0f,
-                         tgemm::kAllTiles, gemm_status, st);
-      if (rc) return rc;
-      if (rest > near) {
-        rc = tgemm::launch(tgemm::kNT, A, tgemm::Split{sb_hi + (int64_t)near * ld, sb_lo + (int64_t)near * ld, ld},
-                           Wf + i2 + near, ldf, (int)N, rest - near, bs, -1.0f, 1.0f, tgemm::kAllTiles, gemm_status,
-                           side->stream, 0, kNumSMs - reserve);
-        if (rc) return rc;
-        // the next block's slice of U: its buffer was last read by the block before this one
-        // (near part before `ready`, far part earlier on the helper stream)
-        if (more) { rc = split_u(i2, (blk + 1) & 1, side->stream); if (rc) return rc; }
-        B200Q_TRY(cudaEventRecord(side->done, side->stream));
-        side_busy = true;
-      } else if (more) {
-        // no far part (blocks narrower than the 128 near columns): the helper stream is idle and
-        // was waited for above, the slice is made on the caller's stream
-        rc = split_u(i2, (blk + 1) & 1, st); if (rc) return rc;
-      }
-    }
-  }
-  if (side_busy) B200Q_TRY(cudaStreamWaitEvent(st, side->done, 0));
-  return B200Q_OK;
+  B200Q_TRY(cudaMallocAsync(&ws, b200q_gptq_sweep_many_workspace_bytes(N, K, count, count), st));
+  const int rc = b200q_gptq_sweep_many(W, U, U, count, nullptr, scale, sdtype, zp, col_group, gscale, losses, count, N, K,
+                                       ldw, ldu, qa, ws, stream);
+  B200Q_TRY(cudaFreeAsync(ws, st));
+  return rc;
 }
 
 }  // extern "C"

@@ -1,22 +1,27 @@
 // fp32-accurate tile GEMM on the tensor cores (tcgen05, kind::tf32, "3xTF32").
 //
-//   C[M,N] = beta * C + alpha * A[M,Kd] * B[N,Kd]^T,   Kd <= 128 (the GPTQ block width)
+//   C[M,N] = beta * C + alpha * A[M,Kd] * B[N,Kd]^T,   Kd <= 512
 //
-// Each float32 operand x is given as two tf32-exact arrays hi = tf32(x), lo = tf32(x - hi)
-// (split_kernel; split_transposed_kernel for an operand stored [Kd][N]); every k-step issues three
-// MMAs into one TMEM accumulator, hi*hi + hi*lo + lo*hi, which keeps ~22 significant bits per
-// product with float32 accumulation: as accurate as the SIMT float32 GEMM it replaces for the
-// factorisation and the sweep's trailing updates, at tensor-core speed.
+// Each float32 operand x is given as two tf32-exact arrays hi = tf32(x), lo = tf32(x - hi); every
+// k-step issues three MMAs into one TMEM accumulator, hi*hi + hi*lo + lo*hi, which keeps ~22
+// significant bits per product with float32 accumulation: as accurate as a SIMT float32 GEMM for
+// the factorisation and the sweep's trailing updates, at tensor-core speed.
 //
-// Structure: persistent CTAs, each with a contiguous range of the row-major tile list.  Warp 0 =
-// TMA producer: the A operand of a block row (all k-chunks, hi and lo, 128 KiB) is loaded once and
-// stays in shared memory while the tiles of that row are computed; B chunks (hi, lo of 32 k-values,
-// 32 KiB) stream through a two-stage ring; the C tile is prefetched into L2.  Warp 1 = MMA issuer
-// and TMEM owner (two 128-column accumulators).  Warps 2-9 = epilogue: the loads of the old C
-// values are issued before the wait for the accumulator, tcgen05.ld, a transpose through a
-// per-warp shared-memory tile so that every global access is a row-contiguous float4, alpha /
-// beta, bounds.  Tile sets: all, lower block triangle, and the sets of the one-pass factorisation
-// (see tgemm_tf32.cuh).  All mbarrier waits are bounded; no cluster launch, no multicast.
+// Structure: persistent CTAs, each with a contiguous range of the tile list (128 x TN tiles).  Warp 0
+// streams 32-deep chunks of both operands (A_hi, A_lo, B_hi, B_lo) through a shared-memory ring by
+// TMA.  Warp 1 issues the MMAs and owns TMEM.  A contraction is cut into slices of 128: each slice
+// accumulates in its own TMEM buffer (two, used in turn) and the epilogue (warps 4-11) adds the slices
+// in registers, so no tensor-core accumulation chain is longer than 128 whatever Kd is, and C is
+// read and written once per launch.
+//
+// Why Kd up to 512: a rank-128 update of a 128 x 128 tile moves 128 KB of C for 1.7 us of MMA work,
+// which made the factorisation HBM-bound (222 us for 6105 tiles, 43 % of DRAM, tensor pipe 40 %).
+// At rank 512 the C traffic per flop is a quarter and the launch count drops with it.
+// Why three tile widths: the operands of a chunk come from L2 at 64 B/clk and SM for TN = 256, 85 for
+// 128 and 128 for 64, so wide tiles run closer to the tensor pipe, narrow ones spread a small update
+// over more SMs; pick_width() takes whatever finishes its waves first.
+//
+// All mbarrier waits are bounded; no cluster launch, no multicast.
 #include <cuda.h>
 
 #include <cstdlib>
@@ -28,19 +33,18 @@
 namespace b200q {
 namespace tgemm {
 
-constexpr int kTile = 128;          // output tile is 128 x 128
-constexpr int kChunkK = 32;         // fp32 elements per 128-byte row
-constexpr int kOpBytes = kTile * kChunkK * 4;    // one hi or lo part of one 32-deep k-chunk: 16 KiB
-constexpr int kMaxChunks = 4;                     // Kd <= 128
-constexpr int kABytes = kMaxChunks * 2 * kOpBytes;   // resident A operand: 4 chunks x (hi, lo) = 128 KiB
-constexpr int kStages = 2;                        // ring of B chunks
-constexpr int kStageBytes = 2 * kOpBytes;         // B_hi, B_lo of one chunk: 32 KiB
-constexpr int kEpiWarps = 8;                      // two warps per TMEM lane quarter, two column chunks each
+constexpr int kChunkK = 32;                          // fp32 elements per 128-byte row
+constexpr int kSliceChunks = 4;                      // 128-deep slice: one accumulation chain
+constexpr int kAPart = kTile * kChunkK * 4;          // A_hi or A_lo of a chunk: 16 KiB
+constexpr int kRingBytes = 196608;                   // 2, 3 or 4 stages for TN = 256, 128, 64
+constexpr int kEpiWarps = 8;                         // two per TMEM lane quarter, each half of the columns
 constexpr int kEpiBytes = kEpiWarps * 32 * 33 * 4;   // per-warp staging tiles of the epilogue
-constexpr int kOperandBytes = kABytes + kStages * kStageBytes;
-constexpr int kSmemBytes = kOperandBytes + 1024 + 256 + kEpiBytes;
-constexpr int kThreads = 64 + 32 * kEpiWarps;
-constexpr int kTmemCols = 256;
+constexpr int kSmemBytes = kRingBytes + 1024 + 256 + kEpiBytes;
+constexpr int kFirstEpiWarp = 4;                    // warpgroup 0: producer, MMA issuer, two idle warps
+constexpr int kThreads = 32 * (kFirstEpiWarp + kEpiWarps);
+// 384 threads at 168 registers; warpgroup 0 gives up 96 a thread and the epilogue's two take 48 each
+// (72 + 216 + 216 = 3 * 168), so that a thread can hold 128 sums
+constexpr int kIssueRegs = 72, kEpiRegs = 216;
 constexpr long long kWaitCycles = 4000000000LL;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -87,15 +91,12 @@ __device__ __forceinline__ void mma_tf32(uint32_t d_tmem, uint64_t a_desc, uint6
       "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-        "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr) : "memory");
 }
 // shared-memory matrix descriptor, 128-byte swizzle, descriptor version 1
@@ -108,83 +109,60 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t lbo_bytes
   d |= (uint64_t)2 << 61;
   return d;
 }
-// D fp32, A/B tf32, A K-major, B K-major (NT) or MN-major (NN), M = N = 128
-__host__ __device__ constexpr uint32_t instr_desc(bool b_mn_major) {
-  return (1u << 4) | (2u << 7) | (2u << 10) | ((b_mn_major ? 1u : 0u) << 16) |
-         ((uint32_t)(kTile >> 3) << 17) | ((uint32_t)(kTile >> 4) << 24);
+// D fp32, A/B tf32, both K-major, M = 128, N = tn
+__host__ __device__ constexpr uint32_t instr_desc(int tn) {
+  return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(tn >> 3) << 17) | ((uint32_t)(kTile >> 4) << 24);
 }
 
 struct Params {
-  float* C; int64_t ldc;
-  int M, N, Kd;
-  float alpha, beta;
-  int tiles_m, tiles_n, mask;
-  int skip;   // kSkipBlockTiles: index of the skipped column block
-  int64_t num_tiles;
-  int trans;
-  int prefetch_c;
-  int* status;
+  Job j;
+  int row_tiles, tn_log2;
+  int64_t num_tiles;                    // over all problems
+  uint16_t start[kNumSMs][3];           // (problem, row tile, column tile) each CTA starts at
 };
 
-__device__ __forceinline__ void tile_from_index(const Params& p, int64_t t, int& tm, int& tn) {
-  if (p.mask == kLowerTiles) {
-    int i = (int)((sqrt(8.0 * (double)t + 1.0) - 1.0) * 0.5);
-    while ((int64_t)i * (i + 1) / 2 > t) --i;
-    while ((int64_t)(i + 1) * (i + 2) / 2 <= t) ++i;
-    tm = i;
-    tn = (int)(t - (int64_t)i * (i + 1) / 2);
-  } else if (p.mask == kSkipBlockFirst) {
-    if (t < p.skip) { tm = 0; tn = (int)t; }
-    else if (t == p.skip) { tm = 0; tn = p.skip + 1; }
-    else { tm = (int)(t - p.skip); tn = p.skip + 1; }
-  } else if (p.mask == kSkipBlockRest) {
-    const int64_t left = (int64_t)(p.tiles_m - 1) * p.skip;
-    if (t < left) {
-      tm = 1 + (int)(t / p.skip);
-      tn = (int)(t - (int64_t)(tm - 1) * p.skip);
-    } else {
-      const int64_t u = t - left;
-      int i = (int)((sqrt(8.0 * (double)u + 1.0) - 1.0) * 0.5);
-      while ((int64_t)i * (i + 1) / 2 > u) --i;
-      while ((int64_t)(i + 1) * (i + 2) / 2 <= u) ++i;
-      tm = i + 1;
-      tn = p.skip + 2 + (int)(u - (int64_t)i * (i + 1) / 2);
-    }
-  } else if (p.mask == kSkipBlockTiles) {
-    const int64_t left = (int64_t)p.tiles_m * p.skip;
-    if (t < left) {
-      tm = (int)(t / p.skip);
-      tn = (int)(t - (int64_t)tm * p.skip);
-    } else {
-      const int64_t u = t - left;
-      int i = (int)((sqrt(8.0 * (double)u + 1.0) - 1.0) * 0.5);
-      while ((int64_t)i * (i + 1) / 2 > u) --i;
-      while ((int64_t)(i + 1) * (i + 2) / 2 <= u) ++i;
-      tm = i;
-      tn = p.skip + 1 + (int)(u - (int64_t)i * (i + 1) / 2);
-    }
-  } else {
-    tm = (int)(t / p.tiles_n);
-    tn = (int)(t - (int64_t)tm * p.tiles_n);
+__host__ __device__ __forceinline__ int tile_row(const Job& j, int tm) {
+  int r = j.row_begin + tm * kTile;
+  if (j.set == kPanel && r >= j.skip0) r += j.skip1 - j.skip0;
+  return r;
+}
+// column tiles of row tile tm (they are contiguous from column 0)
+__host__ __device__ __forceinline__ int col_tiles(const Job& j, int tm, int tn_log2) {
+  int lim = j.N;
+  if (j.set == kLower || j.set == kBulk) {
+    const int r = tile_row(j, tm);
+    const int diag = (j.set == kBulk && r < j.skip1) ? j.skip0 : r + kTile;
+    lim = diag < lim ? diag : lim;
+  }
+  return (lim + (1 << tn_log2) - 1) >> tn_log2;
+}
+__host__ __device__ __forceinline__ void next_tile(const Params& p, int& b, int& tm, int& tn) {
+  ++tn;
+  while (tn >= col_tiles(p.j, tm, p.tn_log2)) {   // a row tile may have no column at all
+    tn = 0;
+    if (++tm == p.row_tiles) { tm = 0; ++b; return; }
   }
 }
 
+template <int TN, bool SPLIT_OUT>
 __global__ void __launch_bounds__(kThreads, 1)
 tgemm_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ CUtensorMap a_lo,
              const __grid_constant__ CUtensorMap b_hi, const __grid_constant__ CUtensorMap b_lo,
-             const __grid_constant__ CUtensorMap c_map, Params p) {
+             const __grid_constant__ Params p) {
+  constexpr int kBPart = TN * kChunkK * 4;
+  constexpr int kStageBytes = 2 * kAPart + 2 * kBPart;
+  constexpr int kStages = kRingBytes / kStageBytes;
+  constexpr uint32_t kTmemCols = 2 * TN;
   extern __shared__ unsigned char smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   unsigned char* aligned = smem_raw + (base - raw);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(aligned + kOperandBytes);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(aligned + kRingBytes);
   const uint32_t bar0 = smem_u32(bars);
   auto full_bar = [&](int s) { return bar0 + 8u * s; };
   auto empty_bar = [&](int s) { return bar0 + 8u * (kStages + s); };
   auto accf_bar = [&](int b) { return bar0 + 8u * (2 * kStages + b); };
   auto acce_bar = [&](int b) { return bar0 + 8u * (2 * kStages + 2 + b); };
-  const uint32_t afull_bar = bar0 + 8u * (2 * kStages + 4), aempty_bar = bar0 + 8u * (2 * kStages + 5);
-  const uint32_t b_base = base + kABytes;   // ring of B chunks behind the resident A operand
   __shared__ uint32_t s_tmem_base;
   __shared__ volatile int s_abort;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -192,194 +170,199 @@ tgemm_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ C
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(accf_bar(b), 1); mbar_init(acce_bar(b), kEpiWarps); }
-    mbar_init(afull_bar, 1); mbar_init(aempty_bar, 1);
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem_base)),
-                 "r"((uint32_t)kTmemCols) : "memory");
+                 "r"(kTmemCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = s_tmem_base;
-  const int chunks = (p.Kd + kChunkK - 1) / kChunkK;
-  // Every CTA takes a contiguous range of the tile list.  The list is row-major, so consecutive
-  // tiles of a CTA mostly share their block row: the A operand of a block row (all k-chunks, hi
-  // and lo) is loaded once and stays in shared memory while only B chunks stream through the ring.
-  const int64_t t_begin = p.num_tiles * blockIdx.x / gridDim.x;
-  const int64_t t_end = p.num_tiles * (blockIdx.x + 1) / gridDim.x;
+  const Job& j = p.j;
+  const int chunks = (j.Kd + kChunkK - 1) / kChunkK;
+  const int64_t count = p.num_tiles * (blockIdx.x + 1) / gridDim.x - p.num_tiles * blockIdx.x / gridDim.x;
+  int b = p.start[blockIdx.x][0], tm = p.start[blockIdx.x][1], tn = p.start[blockIdx.x][2];
 
-  if (warp == 0) {
-    if (lane == 0) {
+  if (warp < kFirstEpiWarp) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kIssueRegs));
+    if (warp == 0 && lane == 0) {
       int stage = 0;
-      uint32_t phase = 0, a_par = 0;
-      int cur_tm = -1;
+      uint32_t phase = 0;
       bool ok = true;
-      for (int64_t t = t_begin; t < t_end && ok; ++t) {
-        int tm, tn;
-        tile_from_index(p, t, tm, tn);
-        if (p.prefetch_c) {
-          // pull the C tile into L2 while this tile's operands stream in: the epilogue's
-          // read-modify-write then meets L2 latency instead of HBM latency
-#pragma unroll
-          for (int q = 0; q < 4; ++q)
-            asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(&c_map),
-                         "r"(tn * kTile + q * 32), "r"(tm * kTile) : "memory");
-        }
-        if (tm != cur_tm) {
-          if (cur_tm >= 0) {   // the MMAs of the previous block row have read A
-            if (!mbar_wait(aempty_bar, a_par, &s_abort)) { ok = false; break; }
-            a_par ^= 1u;
-          }
-          cur_tm = tm;
-          mbar_expect_tx(afull_bar, (uint32_t)(chunks * 2 * kOpBytes));
-          for (int c = 0; c < chunks; ++c) {
-            // A parts: box [32 k][128 rows] at (k, row)
-            tma_load_2d(base + (c * 2) * kOpBytes, &a_hi, afull_bar, c * kChunkK, tm * kTile);
-            tma_load_2d(base + (c * 2 + 1) * kOpBytes, &a_lo, afull_bar, c * kChunkK, tm * kTile);
-          }
-        }
+      for (int64_t i = 0; i < count && ok; ++i, next_tile(p, b, tm, tn)) {
+        const int ra = (int)(b * j.A.batch_rows) + j.A.row0 + tile_row(j, tm);
+        const int rb = (int)((j.b_index ? j.b_index[b] : b) * j.B.batch_rows) + j.B.row0 + tn * TN;
         for (int c = 0; c < chunks; ++c) {
           if (!mbar_wait(empty_bar(stage), phase ^ 1u, &s_abort)) { ok = false; break; }
           mbar_expect_tx(full_bar(stage), kStageBytes);
-          const uint32_t sb = b_base + stage * kStageBytes;
-          tma_load_2d(sb, &b_hi, full_bar(stage), c * kChunkK, tn * kTile);
-          tma_load_2d(sb + kOpBytes, &b_lo, full_bar(stage), c * kChunkK, tn * kTile);
+          const uint32_t s = base + stage * kStageBytes;
+          tma_load_2d(s, &a_hi, full_bar(stage), c * kChunkK, ra);
+          tma_load_2d(s + 2 * kAPart, &b_hi, full_bar(stage), c * kChunkK, rb);
+          tma_load_2d(s + 2 * kAPart + kBPart, &b_lo, full_bar(stage), c * kChunkK, rb);
+          tma_load_2d(s + kAPart, &a_lo, full_bar(stage), c * kChunkK, ra);
           if (++stage == kStages) { stage = 0; phase ^= 1u; }
         }
       }
     }
-  } else if (warp == 1) {
-    int stage = 0;
-    uint32_t phase = 0, a_par = 0;
-    int local = 0, cur_tm = -1;
+    if (warp == 1) {
+    int stage = 0, slice = 0;
+    uint32_t phase = 0;
     bool ok = true;
-    const uint32_t idesc = instr_desc(false);
-    for (int64_t t = t_begin; t < t_end && ok; ++t, ++local) {
-      int tm, tn, next_tm = -1, next_tn;
-      tile_from_index(p, t, tm, tn);
-      if (t + 1 < t_end) tile_from_index(p, t + 1, next_tm, next_tn);
-      const int buf = local & 1;
-      const uint32_t acc_phase = (uint32_t)((local >> 1) & 1);
-      if (!mbar_wait(acce_bar(buf), acc_phase ^ 1u, &s_abort)) { ok = false; break; }
-      if (tm != cur_tm) {
-        if (!mbar_wait(afull_bar, a_par, &s_abort)) { ok = false; break; }
-        a_par ^= 1u;
-        cur_tm = tm;
-      }
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t d_tmem = tmem_base + (uint32_t)(buf * kTile);
+    constexpr uint32_t idesc = instr_desc(TN);
+    for (int64_t i = 0; i < count && ok; ++i) {
       for (int c = 0; c < chunks; ++c) {
+        const int buf = slice & 1;
+        const bool first = (c % kSliceChunks) == 0, last = (c % kSliceChunks) == kSliceChunks - 1 || c == chunks - 1;
+        if (first && !mbar_wait(acce_bar(buf), (uint32_t)(((slice >> 1) & 1) ^ 1), &s_abort)) { ok = false; break; }
         if (!mbar_wait(full_bar(stage), phase, &s_abort)) { ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (lane == 0) {
-          const uint32_t sa = base + (c * 2) * kOpBytes;
-          const uint32_t sb = b_base + stage * kStageBytes;
+          const uint32_t d_tmem = tmem_base + (uint32_t)(buf * TN);
+          const uint32_t sa = base + stage * kStageBytes, sb = sa + 2 * kAPart;
 #pragma unroll
           for (int kk = 0; kk < kChunkK / 8; ++kk) {
             // K-major, 128-byte rows: 8-row groups 1024 bytes apart; a k-step of 8 tf32 is 32 bytes
             const uint64_t ah = make_desc(sa + kk * 32, 16, 1024);
-            const uint64_t al = make_desc(sa + kOpBytes + kk * 32, 16, 1024);
+            const uint64_t al = make_desc(sa + kAPart + kk * 32, 16, 1024);
             const uint64_t bh = make_desc(sb + kk * 32, 16, 1024);
-            const uint64_t bl = make_desc(sb + kOpBytes + kk * 32, 16, 1024);
-            mma_tf32(d_tmem, ah, bh, idesc, (c | kk) ? 1u : 0u);
+            const uint64_t bl = make_desc(sb + kBPart + kk * 32, 16, 1024);
+            mma_tf32(d_tmem, ah, bh, idesc, (first && kk == 0) ? 0u : 1u);
             mma_tf32(d_tmem, ah, bl, idesc, 1u);
             mma_tf32(d_tmem, al, bh, idesc, 1u);
           }
           tc_commit(empty_bar(stage));
-          if (c == chunks - 1) {
-            tc_commit(accf_bar(buf));
-            if (next_tm >= 0 && next_tm != tm) tc_commit(aempty_bar);   // A may be replaced
-          }
+          if (last) tc_commit(accf_bar(buf));
         }
         __syncwarp();
+        if (last) ++slice;
         if (++stage == kStages) { stage = 0; phase ^= 1u; }
       }
     }
+    }
   } else {
-    const int q = warp & 3;
-    int local = 0;
-    bool ok = true;
-    const bool vec = ((p.ldc & 3) == 0) && ((((uintptr_t)p.C) & 15) == 0);
-    // per-warp staging tile [32 rows][33]: accumulator rows come out of TMEM one row per lane;
-    // going through shared memory lets every global access cover whole 128-byte row segments
-    float* stage = reinterpret_cast<float*>(aligned + kOperandBytes + 256) + (warp - 2) * (32 * 33);
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kEpiRegs));
+    constexpr int kHalf = TN / 2;          // columns of this warp
+    const int q = warp & 3, half = (warp - kFirstEpiWarp) >> 2;
+    // per-warp staging tile [32 rows][33]: accumulator rows come out of TMEM one row per lane; going
+    // through shared memory lets every global access cover whole 128-byte row segments
+    float* stage = reinterpret_cast<float*>(aligned + kRingBytes + 256) + (warp - kFirstEpiWarp) * (32 * 33);
     const int sub_row = lane >> 3, sub_col = (lane & 7) * 4;  // 4 rows x 8 float4 per instruction
-    for (int64_t t = t_begin; t < t_end && ok; ++t, ++local) {
-      int tm, tn;
-      tile_from_index(p, t, tm, tn);
-      const int buf = local & 1;
-      const uint32_t acc_phase = (uint32_t)((local >> 1) & 1);
-      const int row0 = tm * kTile + q * 32;
-      // warps 2-5 take column chunks 0 and 1, warps 6-9 chunks 2 and 3
-      const int c_first = (warp - 2) >= 4 ? 2 : 0;
-      // the old values of C do not depend on the accumulator: their loads go out before the wait
-      // for the MMAs, so that memory latency and tensor-core time overlap
-      float4 h[2][8];
-      bool fast[2];
+    int slice = 0;
+    bool ok = true;
+    for (int64_t i = 0; i < count && ok; ++i, next_tile(p, b, tm, tn)) {
+      const int row0 = tile_row(j, tm) + q * 32, colw = tn * TN + half * kHalf;
+      float sum[kHalf];
+      for (int c = 0; c < chunks; c += kSliceChunks, ++slice) {
+        const int buf = slice & 1;
+        if (!mbar_wait(accf_bar(buf), (uint32_t)((slice >> 1) & 1), &s_abort)) { ok = false; break; }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        const int col0 = tn * kTile + (c_first + k) * 32;
-        fast[k] = vec && col0 + 31 < p.N;
+        for (int k = 0; k < kHalf / 16; ++k) {
+          uint32_t r[16];
+          tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * TN + half * kHalf + k * 16), r);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int row = row0 + i * 4 + sub_row;
-          h[k][i] = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (fast[k] && p.beta != 0.0f && row < p.M)
-            h[k][i] = *reinterpret_cast<const float4*>(p.C + (int64_t)row * p.ldc + col0 + sub_col);
+          for (int e = 0; e < 16; ++e)
+            sum[k * 16 + e] = (c == 0) ? __uint_as_float(r[e]) : sum[k * 16 + e] + __uint_as_float(r[e]);
         }
-      }
-      if (!mbar_wait(accf_bar(buf), acc_phase, &s_abort)) { ok = false; break; }
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        const int c = c_first + k;
-        const int col0 = tn * kTile + c * 32;
-        if (col0 >= p.N) break;
-        uint32_t r[32];
-        tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * kTile + c * 32), r);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-        for (int j = 0; j < 32; ++j) stage[lane * 33 + j] = __uint_as_float(r[j]) * p.alpha;
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
-        const int cc = col0 + sub_col;
-        if (fast[k]) {
+        if (lane == 0) mbar_arrive(acce_bar(buf));
+      }
+      if (!ok) break;
+      float* C = nullptr;
+      bool vec = true;
+      if (!SPLIT_OUT) {
+        C = j.c_table ? j.c_table[b] + j.c_offset : j.C + (int64_t)b * j.c_batch;
+        vec = ((j.ldc & 3) == 0) && ((((uintptr_t)C) & 15) == 0);
+      }
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int lr = i * 4 + sub_row, row = row0 + lr;
-            if (row < p.M) {
-              const float* sp = stage + lr * 33 + sub_col;
-              float4 o;
-              o.x = p.beta * h[k][i].x + sp[0]; o.y = p.beta * h[k][i].y + sp[1];
-              o.z = p.beta * h[k][i].z + sp[2]; o.w = p.beta * h[k][i].w + sp[3];
-              *reinterpret_cast<float4*>(p.C + (int64_t)row * p.ldc + cc) = o;
+      for (int k = 0; k < kHalf / 32; ++k) {
+        const int col0 = colw + k * 32;
+        if (col0 >= j.N) break;   // warp-uniform
+        const int cc = col0 + sub_col;
+        if constexpr (SPLIT_OUT) {
+          if (j.X && row0 < j.xt_rows && row0 + lane < j.M) {
+            // lanes hold consecutive rows: the transposed store is contiguous as it stands
+            float* x = j.X + (int64_t)b * j.x_batch + row0 + lane;
+#pragma unroll
+            for (int e = 0; e < 32; ++e)
+              if (col0 + e < j.N) x[(int64_t)(col0 + e) * j.ldx] = j.alpha * sum[k * 32 + e];
+          }
+          if (j.out_hi) {
+#pragma unroll
+            for (int e = 0; e < 32; ++e) stage[lane * 33 + e] = sum[k * 32 + e] * j.alpha;
+            __syncwarp();
+#pragma unroll
+            for (int s = 0; s < 8; ++s) {
+              const int lr = s * 4 + sub_row, row = row0 + lr;
+              if (row < j.M) {
+                const float* sp = stage + lr * 33 + sub_col;
+                float4 h, l;
+                h.x = tf32_rn(sp[0]); h.y = tf32_rn(sp[1]); h.z = tf32_rn(sp[2]); h.w = tf32_rn(sp[3]);
+                l.x = tf32_rn(sp[0] - h.x); l.y = tf32_rn(sp[1] - h.y);
+                l.z = tf32_rn(sp[2] - h.z); l.w = tf32_rn(sp[3] - h.w);
+                const int64_t at = (int64_t)b * j.out_batch + (int64_t)(row + j.out_row0) * j.out_ld + cc;
+                *reinterpret_cast<float4*>(j.out_hi + at) = h;
+                *reinterpret_cast<float4*>(j.out_lo + at) = l;
+              }
             }
+            __syncwarp();
           }
         } else {
-          for (int i = 0; i < 8; ++i) {
-            const int lr = i * 4 + sub_row, row = row0 + lr;
-            if (row >= p.M) continue;
-            for (int j = 0; j < 4; ++j)
-              if (cc + j < p.N) {
-                float* d = p.C + (int64_t)row * p.ldc + cc + j;
-                const float old = (p.beta != 0.0f) ? *d : 0.0f;
-                *d = p.beta * old + stage[lr * 33 + sub_col + j];
+          const float beta = (col0 >= j.fresh0 && col0 < j.fresh1) ? 0.0f : j.beta;
+          const bool fast = vec && col0 + 31 < j.N;
+#pragma unroll
+          for (int e = 0; e < 32; ++e) stage[lane * 33 + e] = sum[k * 32 + e] * j.alpha;
+          __syncwarp();
+          if (fast) {
+            float* c = C + (int64_t)(row0 + sub_row) * j.ldc + cc;
+#pragma unroll
+            for (int s0 = 0; s0 < 8; s0 += 4) {
+              float4 h[4];
+#pragma unroll
+              for (int s = 0; s < 4; ++s) {
+                h[s] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (beta != 0.0f && row0 + (s0 + s) * 4 + sub_row < j.M)
+                  h[s] = *reinterpret_cast<const float4*>(c + (int64_t)((s0 + s) * 4) * j.ldc);
               }
+#pragma unroll
+              for (int s = 0; s < 4; ++s) {
+                const int lr = (s0 + s) * 4 + sub_row;
+                if (row0 + lr < j.M) {
+                  const float* sp = stage + lr * 33 + sub_col;
+                  float4 o;
+                  o.x = beta * h[s].x + sp[0]; o.y = beta * h[s].y + sp[1];
+                  o.z = beta * h[s].z + sp[2]; o.w = beta * h[s].w + sp[3];
+                  *reinterpret_cast<float4*>(c + (int64_t)((s0 + s) * 4) * j.ldc) = o;
+                }
+              }
+            }
+          } else {
+            for (int s = 0; s < 8; ++s) {
+              const int lr = s * 4 + sub_row, row = row0 + lr;
+              if (row >= j.M) continue;
+              for (int e = 0; e < 4; ++e)
+                if (cc + e < j.N) {
+                  float* d = C + (int64_t)row * j.ldc + cc + e;
+                  const float old = (beta != 0.0f) ? *d : 0.0f;
+                  *d = beta * old + stage[lr * 33 + sub_col + e];
+                }
+            }
           }
+          __syncwarp();
         }
-        __syncwarp();
       }
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) mbar_arrive(acce_bar(buf));
     }
   }
 
   if (s_abort) {
-    if (threadIdx.x == 0 && p.status) atomicCAS(p.status, 0, B200Q_ERR_DEVICE);
+    if (threadIdx.x == 0 && j.status)
+      for (int k = 0; k < j.batch; ++k) atomicCAS(j.status + k * j.status_stride, 0, B200Q_ERR_DEVICE);
     const long long t0 = clock64();
     while (clock64() - t0 < 2000000LL) __nanosleep(1000);
   }
@@ -387,8 +370,7 @@ tgemm_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ C
   __syncthreads();
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)kTmemCols)
-                 : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
   }
 }
 
@@ -410,23 +392,33 @@ __global__ void split_kernel(const float* __restrict__ src, int64_t ld_src, int 
   }
 }
 
-// Transposing variant: src is [rows][cols]; hi/lo are [cols][ld_dst] (row c holds src[:, c]),
-// zero-padded to ld_dst.  Turns a [Kd][N] operand into the K-major [N][Kd] form the MMA reads.
-__global__ void __launch_bounds__(256) split_transposed_kernel(const float* __restrict__ src, int64_t ld_src,
-                                                                      int rows, int cols, float* __restrict__ hi,
-                                                                      float* __restrict__ lo, int64_t ld_dst) {
+// Transposing variant: row c of hi/lo (ld_dst floats) holds column c of src, zero-padded.  Turns a
+// [Kd][N] operand into the K-major [N][Kd] form the MMA reads.  blockIdx.y = problem.
+__global__ void __launch_bounds__(256) split_transposed_kernel(const float* __restrict__ src0,
+                                                               const float* const* __restrict__ table,
+                                                               int64_t src_offset, int64_t ld_src, int rows, int cols,
+                                                               float* __restrict__ hi, float* __restrict__ lo,
+                                                               int64_t ld_dst, int64_t dst_batch) {
   __shared__ float tile[32][33];
+  const float* __restrict__ src = table ? table[blockIdx.y] + src_offset : src0;
+  hi += (int64_t)blockIdx.y * dst_batch;
+  lo += (int64_t)blockIdx.y * dst_batch;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
   const int tiles_c = (cols + 31) / 32, tiles_r = (int)(ld_dst / 32);
-  for (int64_t t = blockIdx.x; t < (int64_t)tiles_c * tiles_r; t += gridDim.x) {
-    const int tc = (int)(t % tiles_c), tr = (int)(t / tiles_c);
-    for (int r = ty; r < 32; r += 8) {
-      const int gr = tr * 32 + r, gc = tc * 32 + tx;
-      tile[r][tx] = (gr < rows && gc < cols) ? src[(int64_t)gr * ld_src + gc] : 0.0f;
+  for (int t = blockIdx.x; t < tiles_c * tiles_r; t += gridDim.x) {
+    const int tc = t % tiles_c, tr = t / tiles_c;
+    float v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int gr = tr * 32 + ty + 8 * k, gc = tc * 32 + tx;
+      v[k] = (gr < rows && gc < cols) ? src[(int64_t)gr * ld_src + gc] : 0.0f;
     }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) tile[ty + 8 * k][tx] = v[k];
     __syncthreads();
-    for (int c = ty; c < 32; c += 8) {
-      const int gc = tc * 32 + c, gr = tr * 32 + tx;  // output row = source column
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int c = ty + 8 * k, gc = tc * 32 + c, gr = tr * 32 + tx;  // output row = source column
       if (gc < cols) {
         const float x = tile[tx][c];
         const float h = tf32_rn(x);
@@ -454,11 +446,11 @@ inline EncodeTiledFn encode_fn() {
   }();
   return fn;
 }
-// fp32 matrix [rows][cols] (cols contiguous, ld elements per row), boxes of [box_rows][32 cols]
-inline bool make_map(CUtensorMap* m, const float* base, int64_t rows, int64_t cols, int64_t ld, int box_rows) {
+// fp32 matrix [rows][ld], boxes of [box_rows][32 columns]
+inline bool make_map(CUtensorMap* m, const float* base, int64_t rows, int64_t ld, int box_rows) {
   EncodeTiledFn enc = encode_fn();
   if (!enc) return false;
-  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  cuuint64_t dims[2] = {(cuuint64_t)ld, (cuuint64_t)rows};
   cuuint64_t strides[1] = {(cuuint64_t)ld * 4};
   cuuint32_t box[2] = {32u, (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1, 1};
@@ -476,35 +468,34 @@ int split(const float* src, int64_t ld_src, int rows, int cols, float* hi, float
   return B200Q_OK;
 }
 
-// src [rows][cols] -> hi/lo [cols][split_ld(rows)]
-int split_transposed(const float* src, int64_t ld_src, int rows, int cols, float* hi, float* lo,
-                            cudaStream_t st) {
+int split_transposed(const float* src, const float* const* table, int64_t src_offset, int64_t ld_src, int rows, int cols,
+                     float* hi, float* lo, int64_t ld_dst, int64_t dst_batch, int batch, cudaStream_t st) {
   if (rows <= 0 || cols <= 0) return B200Q_OK;
-  const int64_t ld = split_ld(rows);
-  const int64_t tiles = (int64_t)((cols + 31) / 32) * (ld / 32);
-  split_transposed_kernel<<<grid_for(tiles, 8), 256, 0, st>>>(src, ld_src, rows, cols, hi, lo, ld);
+  const int64_t tiles = (int64_t)((cols + 31) / 32) * (ld_dst / 32);
+  const int cap = batch > 1 ? 8 * kNumSMs / batch + 1 : 8 * kNumSMs;
+  dim3 grid((unsigned)(tiles < cap ? tiles : cap), (unsigned)batch, 1);
+  split_transposed_kernel<<<grid, 256, 0, st>>>(src, table, src_offset, ld_src, rows, cols, hi, lo, ld_dst, dst_batch);
   B200Q_LAUNCH_CHECK();
   return B200Q_OK;
 }
 
-// Tensor maps are cached per (array, leading dimension): a map covers the whole capacity of a
-// split buffer (rows up to 2^30, OOB rows never exist), so one encode serves every launch that
-// reads that buffer.  Rows beyond the operand's extent hold stale values; they only reach output
-// rows / columns that the epilogue masks.  Columns beyond Kd are zero (the split pads them).
-struct MapKey { const float* base; int64_t ld; };
+// Tensor maps are cached per (array, shape, box): one encode serves every launch that reads an operand
+// buffer.  Rows beyond an operand's extent inside its buffer may hold anything; they only reach
+// output rows / columns that the epilogue masks.  Columns beyond Kd are zero (the splits pad them).
+struct MapKey { const float* base; int64_t ld, rows; int box; };
 struct MapCache {
-  static constexpr int kSlots = 16;
+  static constexpr int kSlots = 32;
   MapKey key[kSlots];
   CUtensorMap map[kSlots];
   int used = 0, next = 0;
   // Copies the map out: a later get() may evict the slot it came from.
-  bool get(const float* base, int64_t ld, CUtensorMap* out) {
+  bool get(const float* base, int64_t ld, int64_t rows, int box, CUtensorMap* out) {
     for (int i = 0; i < used; ++i)
-      if (key[i].base == base && key[i].ld == ld) { *out = map[i]; return true; }
+      if (key[i].base == base && key[i].ld == ld && key[i].rows == rows && key[i].box == box) { *out = map[i]; return true; }
     int slot = (used < kSlots) ? used++ : (next++ % kSlots);
-    key[slot] = MapKey{nullptr, 0};
-    if (!make_map(&map[slot], base, (int64_t)1 << 30, ld, ld, kTile)) return false;
-    key[slot] = MapKey{base, ld};
+    key[slot] = MapKey{nullptr, 0, 0, 0};
+    if (!make_map(&map[slot], base, rows, ld, box)) return false;
+    key[slot] = MapKey{base, ld, rows, box};
     *out = map[slot];
     return true;
   }
@@ -514,57 +505,85 @@ inline MapCache& map_cache() {
   return c;
 }
 
-// A: [M][Kd] split;  B: [N][Kd] split (K-major; [Kd][N] operands go through split_transposed).
-int launch(int trans, Split A, Split B, float* C, int64_t ldc, int M, int N, int Kd, float alpha, float beta,
-           int mask, int* status, cudaStream_t st, int mask_arg, int max_ctas) {
-  if (M <= 0 || N <= 0 || Kd <= 0) return B200Q_OK;
-  if (mask == kSkipBlockRest && M <= kTile) return B200Q_OK;   // a single row block has no rest
-  if (Kd > 128 || (A.ld & 31) || (B.ld & 31) || A.ld < Kd || B.ld < Kd) return B200Q_ERR_ARG;
-  if (trans != kNT) return B200Q_ERR_UNSUPPORTED;
+static int64_t count_tiles(const Job& j, int row_tiles, int tn_log2) {
+  if (j.set == kAll || j.set == kPanel) return (int64_t)row_tiles * col_tiles(j, 0, tn_log2);
+  int64_t n = 0;
+  for (int tm = 0; tm < row_tiles; ++tm) n += col_tiles(j, tm, tn_log2);
+  return n;
+}
+
+// Tile width: SM cycles of the busiest CTA.  A 32-deep chunk takes the longer of its MMAs (12 of 32 / 64 /
+// 128 cycles) and the arrival of its operands from L2 (about 64 B/clk and SM); the last tile's epilogue,
+// about 20 cycles per column, is not hidden.
+static int pick_width(const Job& j, int row_tiles, int ctas) {
+  const double chunk[3] = {800.0, 1150.0, 1700.0};
+  const int chunks = (j.Kd + kChunkK - 1) / kChunkK;
+  int best = 6;
+  double best_cost = 0.0;
+  for (int w = 6; w <= 8; ++w) {
+    const int64_t tiles = count_tiles(j, row_tiles, w) * j.batch;
+    const double cost = (double)((tiles + ctas - 1) / ctas) * chunks * chunk[w - 6] + 20.0 * (1 << w);
+    if (w == 6 || cost < best_cost) { best = w; best_cost = cost; }
+  }
+  return best;
+}
+
+template <int TN>
+static int launch_width(const Params& p, int grid, cudaStream_t st) {
+  const Job& j = p.j;
   MapCache& mc = map_cache();
   CUtensorMap mah, mal, mbh, mbl;
-  if (!mc.get(A.hi, A.ld, &mah) || !mc.get(A.lo, A.ld, &mal) || !mc.get(B.hi, B.ld, &mbh) ||
-      !mc.get(B.lo, B.ld, &mbl)) {
+  if (!mc.get(j.A.hi, j.A.ld, j.A.rows, kTile, &mah) || !mc.get(j.A.lo, j.A.ld, j.A.rows, kTile, &mal) ||
+      !mc.get(j.B.hi, j.B.ld, j.B.rows, TN, &mbh) || !mc.get(j.B.lo, j.B.ld, j.B.rows, TN, &mbl)) {
     set_last_error("cuTensorMapEncodeTiled (tgemm)", cudaErrorInvalidValue);
     return B200Q_ERR_CUDA;
   }
-  Params p;
-  p.C = C; p.ldc = ldc; p.M = M; p.N = N; p.Kd = Kd; p.alpha = alpha; p.beta = beta; p.mask = mask; p.trans = trans;
-  p.tiles_m = (M + kTile - 1) / kTile; p.tiles_n = (N + kTile - 1) / kTile;
-  p.skip = mask_arg;
-  p.num_tiles = (mask == kLowerTiles) ? (int64_t)p.tiles_m * (p.tiles_m + 1) / 2
-              : (mask == kSkipBlockTiles) ? (int64_t)p.tiles_m * mask_arg + (int64_t)p.tiles_m * (p.tiles_m + 1) / 2
-              : (mask == kSkipBlockFirst) ? (int64_t)mask_arg + p.tiles_m
-              : (mask == kSkipBlockRest) ? (int64_t)(p.tiles_m - 1) * mask_arg + (int64_t)p.tiles_m * (p.tiles_m - 1) / 2
-              : (int64_t)p.tiles_m * p.tiles_n;
-  p.status = status;
+  const bool split_out = j.out_hi || j.X;
   static thread_local int attr_device = -1;
   int dev = 0;
   B200Q_TRY(cudaGetDevice(&dev));
   if (attr_device != dev) {
-    B200Q_TRY(cudaFuncSetAttribute(tgemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
+    B200Q_TRY(cudaFuncSetAttribute(tgemm_kernel<TN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
+    B200Q_TRY(cudaFuncSetAttribute(tgemm_kernel<TN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
     attr_device = dev;
   }
-  // map of C for the L2 prefetch (needs 16-byte aligned rows); any valid map when unused
-  CUtensorMap mc_c = mah;
-  p.prefetch_c = 0;
-  if (beta != 0.0f && (ldc & 3) == 0 && (((uintptr_t)C) & 15) == 0 &&
-      make_map(&mc_c, C, M, N, ldc, kTile))
-    p.prefetch_c = 1;
-  int grid = (int)(p.num_tiles < kNumSMs ? p.num_tiles : kNumSMs);
-  if (max_ctas > 0 && grid > max_ctas) grid = max_ctas;
-  tgemm_kernel<<<grid, kThreads, kSmemBytes, st>>>(mah, mal, mbh, mbl, mc_c, p);
+  if (split_out) tgemm_kernel<TN, true><<<grid, kThreads, kSmemBytes, st>>>(mah, mal, mbh, mbl, p);
+  else tgemm_kernel<TN, false><<<grid, kThreads, kSmemBytes, st>>>(mah, mal, mbh, mbl, p);
   B200Q_LAUNCH_CHECK();
   return B200Q_OK;
 }
 
-int side_reserve() {
-  static const int r = [] {
-    const char* e = getenv("B200Q_SIDE_RESERVE");
-    int v = e ? atoi(e) : 16;   // measured best for K = 14336 among 0 / 16 / 32 / 48
-    return v < 0 ? 0 : (v > kNumSMs / 2 ? kNumSMs / 2 : v);
-  }();
-  return r;
+int launch(const Job& j, cudaStream_t st) {
+  if (j.Kd <= 0 || j.batch <= 0) return B200Q_OK;
+  if (j.Kd > kMaxDepth || j.batch > 65535 || (j.A.ld & 31) || (j.B.ld & 31) || j.A.ld < j.Kd || j.B.ld < j.Kd)
+    return B200Q_ERR_ARG;
+  Params p;
+  p.j = j;
+  if (j.set == kPanel) {
+    const int above = j.skip0 / kTile, below = j.M > j.skip1 ? (j.M - j.skip1 + kTile - 1) / kTile : 0;
+    p.row_tiles = above + below;
+  } else {
+    p.row_tiles = j.M > j.row_begin ? (j.M - j.row_begin + kTile - 1) / kTile : 0;
+  }
+  if (p.row_tiles <= 0 || j.N <= 0) return B200Q_OK;
+  const int ctas = j.max_ctas > 0 && j.max_ctas < kNumSMs ? j.max_ctas : kNumSMs;
+  p.tn_log2 = pick_width(j, p.row_tiles, ctas);
+  const int64_t per_problem = count_tiles(j, p.row_tiles, p.tn_log2);
+  p.num_tiles = per_problem * j.batch;
+  const int grid = (int)(p.num_tiles < ctas ? p.num_tiles : ctas);
+  // where each CTA's range starts: problem, row tile, column tile
+  int tm = 0;
+  int64_t before = 0, of = 0;   // tiles before row tile tm of problem `of`
+  for (int i = 0; i < grid; ++i) {
+    const int64_t t = p.num_tiles * i / grid, b = t / per_problem, in = t - b * per_problem;
+    if (b != of) { of = b; tm = 0; before = 0; }
+    int64_t n;
+    while (in >= before + (n = col_tiles(j, tm, p.tn_log2))) { before += n; ++tm; }
+    p.start[i][0] = (uint16_t)b; p.start[i][1] = (uint16_t)tm; p.start[i][2] = (uint16_t)(in - before);
+  }
+  if (p.tn_log2 == 8) return launch_width<256>(p, grid, st);
+  if (p.tn_log2 == 7) return launch_width<128>(p, grid, st);
+  return launch_width<64>(p, grid, st);
 }
 
 SideStream* side_stream(cudaStream_t like) {
@@ -588,6 +607,7 @@ SideStream* side_stream(cudaStream_t like) {
   e.device = dev; e.like = like;
   if (cudaStreamCreateWithPriority(&e.s.stream, cudaStreamNonBlocking, prio) != cudaSuccess ||
       cudaEventCreateWithFlags(&e.s.ready, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&e.s.next, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&e.s.done, cudaEventDisableTiming) != cudaSuccess) {
     (void)cudaGetLastError();
     return nullptr;

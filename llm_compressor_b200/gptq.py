@@ -293,7 +293,7 @@ def quantize_weights_batched(modules, quant_args, factors, blocksize: int = 128,
     """``quantize_weight(..., defer=True)`` for many small modules of one weight shape and one
     quantisation scheme, each with its own (deferred) factor, with all the column sweeps in one
     launch.  Returns ``[(loss, dict), ...]`` in the order of ``modules``: the losses are 0-dim
-    device tensors and the dicts carry no ``"_status"`` (the batched sweep has no bounded wait).
+    device tensors and the first dict carries the sweep's ``"_status"`` for all of them.
     As with the deferred single call, the caller resolves the factors afterwards and redoes the
     modules whose factorisation failed."""
     weights = [m.weight.data if isinstance(m.weight, torch.nn.Parameter) else m.weight for m in modules]
@@ -312,10 +312,13 @@ def quantize_weights_batched(modules, quant_args, factors, blocksize: int = 128,
             raise ValueError(f"{name} must be present for all modules of a batch or for none")
         return None if vals[0] is None else vals
 
-    losses = ops.gptq_sweep_batched([i.W for i in inputs], [i.factor.U for i in inputs], column("scale"),
+    losses, status = ops.gptq_sweep_batched([i.W for i in inputs], [i.factor.U for i in inputs], column("scale"),
                                     column("zero_point"), first.args, col_groups=column("col_group"),
-                                    global_scales=column("global_scale"), blocksize=blocksize)
+                                    global_scales=column("global_scale"), blocksize=blocksize,
+                                            return_status=True)
     sums = losses.sum(dim=1)
     back = ops.scatter_columns_cast_batched([i.W for i in inputs], first.final_dtype,
                                             None if perms[0] is None else perms)
-    return [(sums[k], _sweep_output(i, weight=back[k])) for k, i in enumerate(inputs)]
+    done = [(sums[k], _sweep_output(i, weight=back[k])) for k, i in enumerate(inputs)]
+    done[0][1]["_status"] = status
+    return done

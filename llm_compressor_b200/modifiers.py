@@ -789,7 +789,7 @@ class GPTQModifier(QuantizationMixin):
                 else:
                     done = [gptq.quantize_weight(m, q, None, blocksize=self.block_size, percdamp=self.dampening_frac,
                                                  factor=f, defer=True) for m, q, f in items]
-                    words += [out.pop("_status", None) for _, out in done]
+                words += [out.pop("_status", None) for _, out in done]
             queued += [(m, q, f, loss, out) for (m, q, f), (loss, out) in zip(items, done)]
         self._trace("job_swept", jobs[0][0])
         self._check_status_words(words)

@@ -422,8 +422,7 @@ def _pointer_table(rows) -> torch.Tensor:
 
 
 def gptq_factor_batched(Hs) -> torch.Tensor:
-    """In place H -> U for a list of small Hessians of one size, one thread block each, in one
-    launch.  Returns the device status words, int32 [count, 4] (see ``gptq_factor_async``)."""
+    """In place H -> U for a list of Hessians of one size, every launch serving all of them.  Returns the device status words, int32 [count, 4] (see ``gptq_factor_async``)."""
     _need_cuda(*Hs)
     lib = _lib.load()
     K, ld = Hs[0].shape[0], Hs[0].stride(0)
@@ -431,11 +430,12 @@ def gptq_factor_batched(Hs) -> torch.Tensor:
         if H.shape != (K, K) or H.stride(0) != ld or H.stride(1) != 1 or H.dtype != torch.float32:
             raise ValueError("batched factorisation needs float32 Hessians of one size and one layout")
     count = len(Hs)
-    scratch = torch.empty((count, K * K), dtype=torch.float32, device=Hs[0].device)
-    status = torch.empty((count, 4), dtype=torch.int32, device=Hs[0].device)
-    table = _pointer_table([Hs, list(scratch.unbind(0))])
-    check(lib.b200q_gptq_factor_batched(ptr(table[0]), ptr(table[1]), count, K, ld, ptr(status), stream_ptr()),
-          "b200q_gptq_factor_batched")
+    dev = Hs[0].device
+    ws = torch.empty(lib.b200q_gptq_factor_many_workspace_bytes(K, count), dtype=torch.uint8, device=dev)
+    status = torch.empty((count, 4), dtype=torch.int32, device=dev)
+    table = _pointer_table([Hs])
+    check(lib.b200q_gptq_factor_many(ptr(table[0]), count, K, ld, ptr(ws), ptr(status), stream_ptr()),
+          "b200q_gptq_factor_many")
     return status
 
 
@@ -480,10 +480,13 @@ def scatter_columns_cast_batched(wfs, dtype: torch.dtype, perms=None) -> torch.T
 
 
 def gptq_sweep_batched(wfs, Us, scales, zps, args: QuantizationArgs, col_groups=None, global_scales=None,
-                       blocksize=128) -> torch.Tensor:
+                       blocksize=128, return_status: bool = False):
     """The column sweep, in place, on a list of float32 weights of one shape that share the
     quantisation scheme, in one launch.  ``Us``, ``zps``, ``col_groups``, ``global_scales``: a list
-    with one tensor per weight, or None for all.  Returns the per-row losses [count, N]."""
+    with one tensor per weight, or None for all.  Returns the per-row losses [count, N], and with
+    ``return_status`` also the call's device status word (see ``gptq_sweep``)."""
+    if blocksize != 128:
+        raise ValueError("the batched sweep takes blocksize 128")
     count = len(wfs)
     N, K, ld = _2d(wfs[0])
     dev = wfs[0].device
@@ -510,14 +513,28 @@ def gptq_sweep_batched(wfs, Us, scales, zps, args: QuantizationArgs, col_groups=
         raise ValueError("batched sweep needs scales of one dtype and one shape")
     losses = torch.empty((count, N), dtype=torch.float32, device=dev)
     table = _pointer_table([wfs, Us, scales, zps, col_groups, global_scales, list(losses.unbind(0))])
+    distinct, index = table[1], None
+    ndistinct = count if Us is not None else 1
+    if Us is not None:
+        # weights that share a factor (the gate / up projections of all experts) share its operand form
+        place = {}
+        order = [place.setdefault(U.data_ptr(), len(place)) for U in Us]
+        ndistinct = len(place)
+        if ndistinct < count:
+            distinct = torch.tensor(list(place), dtype=torch.int64, device=dev)
+            index = torch.tensor(order, dtype=torch.int32, device=dev)
+    lib = _lib.load()
+    ws = torch.empty(lib.b200q_gptq_sweep_many_workspace_bytes(N, K, count, ndistinct), dtype=torch.uint8, device=dev)
 
     def row(i, present):
         return ptr(table[i]) if present is not None else None
 
-    check(_lib.load().b200q_gptq_sweep_batched(
-        ptr(table[0]), row(1, Us), ptr(table[2]), sdt, row(3, zps), row(4, col_groups), row(5, global_scales),
-        ptr(table[6]), count, N, K, ld, ldu, args.c_struct(), int(blocksize), stream_ptr()),
-        "b200q_gptq_sweep_batched")
+    check(lib.b200q_gptq_sweep_many(
+        ptr(table[0]), row(1, Us), ptr(distinct) if Us is not None else None, ndistinct, ptr(index), ptr(table[2]), sdt,
+        row(3, zps), row(4, col_groups), row(5, global_scales), ptr(table[6]), count, N, K, ld, ldu, args.c_struct(),
+        ptr(ws), stream_ptr()), "b200q_gptq_sweep_many")
+    if return_status:
+        return losses, ws[:4].view(torch.int32)
     return losses
 
 
