@@ -31,44 +31,70 @@ constexpr int OB = 512;          // outer block
 constexpr int kThreads = 256;
 constexpr int LD = NB + 4;       // shared-memory stride: 16-byte rows, float4 accesses of 8 consecutive rows conflict-free
 
+constexpr int64_t kScratchFloats = 2LL * OB * NB;   // of the square: P [512][128] and X [128][512]
+
 struct Mat {                     // the batch's work matrices and status words
   float* A; int64_t batch, lda;
   int* status;
 };
 
-__device__ __forceinline__ uint64_t pack2(float a, float b) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
+__device__ __forceinline__ void cp_async16(float* dst, const float* src, int src_bytes) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(src_bytes) : "memory");
 }
-__device__ __forceinline__ void fma2(uint64_t& d, uint64_t a, uint64_t b) {
-  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
-}
-__device__ __forceinline__ float sum2(uint64_t v) {
-  float a, b;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-  return a + b;
-}
-// 32-deep dot products of R rows and C columns of shared memory, both with the contraction contiguous; packed
-// float32 pairs along the contraction, so that a float4 load feeds two FFMA2 without shuffling
-template <int R, int C>
-__device__ __forceinline__ void dots(const float* (&row)[R], const float* (&col)[C], int depth, uint64_t (&acc)[R][C]) {
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Products inside the square: warp-level 16 x 8 x 8 tf32 MMAs on operands in shared memory, three per product of
+// hi / lo splits as in tgemm.  Tiles of 16 are too small for tcgen05 (its operands would have to be rewritten in
+// swizzled form between two steps of the chain); measured here, these MMAs retire 512 multiply-adds a cycle and SM,
+// 170 of float32 accuracy, and need a sixth of the shared-memory loads of a register-tiled FFMA2 product.
+__device__ __forceinline__ uint32_t tf32_bits(float x) { return (__float_as_uint(x) + 0x1000u) & 0xFFFFE000u; }
+template <int N>
+__device__ __forceinline__ void split_frag(const float (&x)[N], uint32_t (&hi)[N], uint32_t (&lo)[N]) {
 #pragma unroll
-  for (int r = 0; r < R; ++r)
-#pragma unroll
-    for (int c = 0; c < C; ++c) acc[r][c] = 0;
-#pragma unroll 2
-  for (int m = 0; m < depth; m += 4) {
-    ulonglong2 a[R], b[C];
-#pragma unroll
-    for (int r = 0; r < R; ++r) a[r] = *reinterpret_cast<const ulonglong2*>(row[r] + m);
-#pragma unroll
-    for (int c = 0; c < C; ++c) b[c] = *reinterpret_cast<const ulonglong2*>(col[c] + m);
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-#pragma unroll
-      for (int c = 0; c < C; ++c) { fma2(acc[r][c], a[r].x, b[c].x); fma2(acc[r][c], a[r].y, b[c].y); }
+  for (int i = 0; i < N; ++i) {
+    hi[i] = tf32_bits(x[i]);
+    lo[i] = tf32_bits(x[i] - __uint_as_float(hi[i]));
   }
+}
+__device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+  asm(
+      "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+// acc[j] += A[16 x depth] B_j[8 x depth]^T, B_j = rows 8 j .. 8 j + 7 of B.  Lane (g, t) = (lane / 4, lane % 4) ends
+// with rows g, g + 8 and columns 2 t, 2 t + 1.  A: contraction contiguous, row stride lda; B: element (n, k) at
+// n * sn + k * sk.
+template <int NT, int UNROLL>
+__device__ __forceinline__ void mma_block(const float* A, int lda, const float* B, int sn, int sk, int depth, int lane,
+                                          float (&acc)[NT][4]) {
+  const float* a0 = A + (lane >> 2) * lda + (lane & 3);
+  const float* b0 = B + (lane >> 2) * sn + (lane & 3) * sk;
+  // the three products accumulate apart: a warp issues in order, and an MMA whose accumulator the one before it
+  // still has stalls everything behind it for some 35 cycles
+  float part[2][NT][4] = {};
+#pragma unroll UNROLL
+  for (int k = 0; k < depth; k += 8) {
+    const float x[4] = {a0[k], a0[k + 8 * lda], a0[k + 4], a0[k + 8 * lda + 4]};
+    float y[NT][2];
+#pragma unroll
+    for (int j = 0; j < NT; ++j) { y[j][0] = b0[j * 8 * sn + k * sk]; y[j][1] = b0[j * 8 * sn + (k + 4) * sk]; }
+    uint32_t ah[4], al[4], bh[NT][2], bl[NT][2];
+    split_frag(x, ah, al);
+#pragma unroll
+    for (int j = 0; j < NT; ++j) split_frag(y[j], bh[j], bl[j]);
+#pragma unroll
+    for (int j = 0; j < NT; ++j) mma_tf32(acc[j], ah, bh[j]);
+#pragma unroll
+    for (int j = 0; j < NT; ++j) mma_tf32(part[0][j], ah, bl[j]);
+#pragma unroll
+    for (int j = 0; j < NT; ++j) mma_tf32(part[1][j], al, bh[j]);
+  }
+#pragma unroll
+  for (int j = 0; j < NT; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[j][e] += part[0][j][e] + part[1][j][e];
 }
 
 // ---------------------------------------------------------------------------------------
@@ -76,34 +102,32 @@ __device__ __forceinline__ void dots(const float* (&row)[R], const float* (&col)
 //
 // One CTA on the critical path, so the design is about latency.  The identity is appended below the block, which
 // turns the triangular inverse into more rows of the same elimination (a row e_i ends as row i of L^-T): at every
-// 32-column step exactly four 32-row blocks take part, one per warp.  A step:
-//   warp 0 factors the 32 x 32 diagonal block in registers, a lane per row, about 95 cycles a column: the next pivot
-//          is formed by its own lane and broadcast before the other columns are updated; meanwhile the other seven
-//          warps finish the update by the step before
-//   four warps substitute their 32 rows, a lane per row, against the transposed block in shared memory
-//   all warps bring the next diagonal block up to date
-// 11 us for 128 columns; the register-tiled version with a barrier per column that this replaces took 58.
-constexpr int kCholSmemFloats = 2 * NB * LD + 32 * 36 + 32;
+// 16-column step exactly eight 16-row blocks take part.  A step:
+//   warp 0 brings the 16 x 16 diagonal block up to date and factors it in registers, a lane per row: the next pivot
+//          is formed by its own lane and broadcast before the other columns are updated, no branches.  Meanwhile the
+//          other seven warps apply the step before to everything else.
+//   four warps substitute the 128 active rows, a row a lane
+constexpr int W16 = 16;
+constexpr int kCholSmemFloats = 2 * NB * LD + W16 * 20 + W16;
+
+// active row block s (0..7) of step kb: identity rows up to kb, whose inverse is being born, matrix rows after it
+__device__ __forceinline__ float* active_row(float* R, int ar, int kb) {
+  return R + ((ar >> 4) <= kb ? NB + ar : ar) * LD;
+}
 
 __global__ void __launch_bounds__(kThreads, 1) chol_diag_kernel(Mat mt, int k0, int n) {
   extern __shared__ __align__(16) float sm[];
   float* R = sm;                    // rows 0..127: the block, then L; rows 128..255: the identity, then L^-T
-  float* Lt = R + 2 * NB * LD;      // [32][36] transposed diagonal block of the step
-  float* rinv = Lt + 32 * 36;       // [32]
+  float* Lt = R + 2 * NB * LD;      // [16][20] transposed diagonal block of the step
+  float* rinv = Lt + W16 * 20;      // [16]
   float* A = mt.A + blockIdx.x * mt.batch + (int64_t)k0 * mt.lda + k0;
-  int* status = mt.status + 4 * blockIdx.x;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-#pragma unroll 4
+#pragma unroll 16
   for (int idx = tid; idx < NB * NB / 4; idx += kThreads) {
     const int r = idx >> 5, c = (idx & 31) << 2;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     float* e = &v.x;
-    if (r < n && c <= r) {
-      if (c + 3 < n) v = *reinterpret_cast<const float4*>(A + (int64_t)r * mt.lda + c);
-      else
-        for (int k = 0; k < 4; ++k)
-          if (c + k < n) e[k] = A[(int64_t)r * mt.lda + c + k];
-    }
+    if (r < n && c <= r) v = *reinterpret_cast<const float4*>(A + (int64_t)r * mt.lda + c);   // (rows are padded to 32)
     float4 id = make_float4(0.f, 0.f, 0.f, 0.f);
     float* d = &id.x;
 #pragma unroll
@@ -115,234 +139,279 @@ __global__ void __launch_bounds__(kThreads, 1) chol_diag_kernel(Mat mt, int k0, 
     *reinterpret_cast<float4*>(R + (NB + r) * LD + c) = id;
   }
   __syncthreads();
-  for (int kb = 0; kb < 4; ++kb) {
-    const int c0 = kb * 32;
+  int bad = 0;   // first pivot that is not positive, + 1
+#pragma unroll 1
+  for (int kb = 0; kb < 8; ++kb) {
+    const int c0 = kb * W16, p0 = c0 - W16;
     if (warp == 0) {
-      float a[32];
-      const float* src = R + (c0 + lane) * LD + c0;
+      if (kb > 0) {   // the diagonal block takes the step before
+        float acc[2][4] = {};
+        float* o = R + (c0 + (lane >> 2)) * LD + c0 + 2 * (lane & 3);
+        float2 old[2][2];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) old[j][h] = *reinterpret_cast<float2*>(o + h * 8 * LD + 8 * j);
+        mma_block<2, 2>(R + c0 * LD + p0, LD, R + c0 * LD + p0, LD, 1, W16, lane, acc);
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+            *reinterpret_cast<float2*>(o + h * 8 * LD + 8 * j) =
+                make_float2(old[j][h].x - acc[j][2 * h], old[j][h].y - acc[j][2 * h + 1]);
+        __syncwarp();
+      }
+      float a[W16];
+      const float* src = R + (c0 + (lane & 15)) * LD + c0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
         const float4 v = *reinterpret_cast<const float4*>(src + 4 * q);
         a[4 * q] = v.x; a[4 * q + 1] = v.y; a[4 * q + 2] = v.z; a[4 * q + 3] = v.w;
       }
-      float piv = __shfl_sync(0xffffffffu, a[0], 0);
+      float piv = __shfl_sync(0xffffffffu, a[0], 0), ri = 0.0f;
 #pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        if (!(piv > 0.0f)) {   // also true for NaN; uniform
-          if (lane == 0 && atomicCAS(status, 0, B200Q_NOT_POSITIVE_DEFINITE) == 0) status[1] = k0 + c0 + j + 1;
-          piv = 1.0f;
-        }
-        float r = rsqrtf(piv);
-        r = fmaf(0.5f * r, fmaf(-piv * r, r, 1.0f), r);   // one Newton step: within an ulp of 1 / sqrt
-        const float l = (lane == j) ? piv * r : a[j] * r;
-        if (j + 1 < 32) piv = __shfl_sync(0xffffffffu, fmaf(-l, l, a[j + 1]), j + 1);
+      for (int j = 0; j < W16; ++j) {
+        // (a pivot that is not a positive normal number makes garbage from here on, and is reported)
+        bad = (!(piv >= 1.17549435e-38f) && bad == 0) ? c0 + j + 1 : bad;
+        float r;
+        asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(piv));
+        // one Newton step r (1.5 - piv r^2 / 2), within an ulp of 1 / sqrt, folded into the column's scaling
+        const float u = fmaf(-(0.5f * piv) * r, r, 1.5f);
+        const float l = (a[j] * r) * u;
+        if (j + 1 < W16) piv = __shfl_sync(0xffffffffu, fmaf(-l, l, a[j + 1]), j + 1);
         a[j] = l;
-        if (lane == j) rinv[j] = r;
+        ri = (lane == j) ? r * u : ri;
 #pragma unroll
-        for (int c = j + 1; c < 32; ++c) a[c] = fmaf(-l, __shfl_sync(0xffffffffu, l, c), a[c]);
+        for (int c = j + 1; c < W16; ++c) a[c] = fmaf(-l, __shfl_sync(0xffffffffu, l, c), a[c]);
       }
+      if (lane < W16) {
 #pragma unroll
-      for (int j = 0; j < 32; ++j) Lt[j * 36 + lane] = (j <= lane) ? a[j] : 0.0f;
+        for (int j = 0; j < W16; ++j) Lt[j * 20 + lane] = (j <= lane) ? a[j] : 0.0f;
+        rinv[lane] = ri;
+      }
     } else if (kb > 0) {
-      // the rest of the update by step kb - 1: every active row block x the columns from c0 on, but the next
-      // diagonal block, which is done already.  A warp per 32 x 32 block, 8 rows x 4 columns a lane.
-      const int p0 = c0 - 32, nc = 4 - kb;
-      for (int t = warp - 1; t < 4 * nc - 1; t += 7) {
-        const int u = t + 1;                                  // task 0 is the diagonal block
-        const int rb = (kb + u / nc) & 3, cb = kb + u % nc;   // row blocks kb, kb+1, ... wrapping to the identity rows
-        const int r0 = (rb >= kb ? rb * 32 : NB + rb * 32) + (lane >> 3) * 8, cc = cb * 32 + (lane & 7);
-        if (rb >= kb && cb > rb) continue;                    // above the diagonal
-        const float *row[8], *col[4];
+      // everything else takes the step before: the eight row blocks that were active then x the columns from c0 on,
+      // on and below the diagonal.  A warp takes 16 rows x 32 columns at a time.
+      // Task list: kb identity row blocks with `wide` pairs of column blocks each, then matrix row blocks r = 0, 1, ...
+      // (s = kb + r) with r / 2 + 1 pairs.  (Counted out in closed form: a loop over all tasks that skips the other
+      // warps' costs 180 cycles a skip, mostly instruction fetch.)
+      const int wide = (9 - kb) / 2, left = kb * wide, half = (8 - kb) / 2;
+      const int all = left + half * (half + 1) + (kb & 1) * (half + 1);
+      for (int t = warp - 1; t < all; t += 7) {
+        int s, g;
+        if (t < left) {
+          s = t / wide; g = t - s * wide;
+        } else {
+          const int u = t - left, q = (u >= 2) + (u >= 6) + (u >= 12);
+          g = u - q * (q + 1); s = kb + 2 * q;
+          if (g > q) { g -= q + 1; ++s; }
+        }
+        {
+          const bool matrix = s >= kb;
+          float* rows = R + ((matrix ? 0 : NB) + s * W16) * LD;
+          const int cc = c0 + g * 32;
+          float acc[4][4] = {};
+          float* o = rows + (lane >> 2) * LD + cc + 2 * (lane & 3);
+          float2 old[4][2];   // (all of them before the products: loads cannot pass the stores below)
 #pragma unroll
-        for (int i = 0; i < 8; ++i) row[i] = R + (r0 + i) * LD + p0;
+          for (int j = 0; j < 4; ++j)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) col[i] = R + (cc + 8 * i) * LD + p0;
-        uint64_t acc[8][4];
-        dots<8, 4>(row, col, 32, acc);
+            for (int h = 0; h < 2; ++h)
+              if (cc + 8 * j < NB) old[j][h] = *reinterpret_cast<float2*>(o + h * 8 * LD + 8 * j);
+          mma_block<4, 2>(rows + p0, LD, R + cc * LD + p0, LD, 1, W16, lane, acc);
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+          for (int j = 0; j < 4; ++j) {
+            const int cb = (cc >> 4) + (j >> 1);
+            if (cb >= 8 || (matrix && (cb > s || (s == kb && cb == kb)))) continue;   // outside, above, warp 0's
 #pragma unroll
-          for (int q = 0; q < 4; ++q) R[(r0 + i) * LD + cc + 8 * q] -= sum2(acc[i][q]);
+            for (int h = 0; h < 2; ++h)
+              *reinterpret_cast<float2*>(o + h * 8 * LD + 8 * j) =
+                  make_float2(old[j][h].x - acc[j][2 * h], old[j][h].y - acc[j][2 * h + 1]);
+          }
+        }
       }
     }
     __syncthreads();
     if (warp < 4) {
-      // block s: identity rows up to kb (their inverse is being born), rows of the matrix after it
-      float* row = R + ((warp <= kb ? NB : 0) + warp * 32 + lane) * LD + c0;
-      float a[32];
+      float a[W16];
+      float* row = active_row(R, warp * 32 + lane, kb) + c0;
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
+      for (int q = 0; q < 4; ++q) {
         const float4 v = *reinterpret_cast<const float4*>(row + 4 * q);
         a[4 * q] = v.x; a[4 * q + 1] = v.y; a[4 * q + 2] = v.z; a[4 * q + 3] = v.w;
       }
 #pragma unroll
-      for (int j = 0; j < 32; ++j) {
+      for (int j = 0; j < W16; ++j) {
         const float y = a[j] * rinv[j];
         a[j] = y;
 #pragma unroll
-        for (int q = (j + 1) / 4; q < 8; ++q) {
-          const float4 l = *reinterpret_cast<const float4*>(Lt + j * 36 + 4 * q);
-          if (4 * q > j) a[4 * q] = fmaf(-y, l.x, a[4 * q]);
-          if (4 * q + 1 > j) a[4 * q + 1] = fmaf(-y, l.y, a[4 * q + 1]);
-          if (4 * q + 2 > j) a[4 * q + 2] = fmaf(-y, l.z, a[4 * q + 2]);
-          if (4 * q + 3 > j) a[4 * q + 3] = fmaf(-y, l.w, a[4 * q + 3]);
+        for (int q = (j + 1) / 4; q < 4; ++q) {
+          const float4 l4 = *reinterpret_cast<const float4*>(Lt + j * 20 + 4 * q);
+          const float l[4] = {l4.x, l4.y, l4.z, l4.w};
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            if (4 * q + k > j) a[4 * q + k] = fmaf(-y, l[k], a[4 * q + k]);
         }
       }
 #pragma unroll
-      for (int q = 0; q < 8; ++q)
+      for (int q = 0; q < 4; ++q)
         *reinterpret_cast<float4*>(row + 4 * q) = make_float4(a[4 * q], a[4 * q + 1], a[4 * q + 2], a[4 * q + 3]);
     }
     __syncthreads();
-    if (kb < 3) {   // next diagonal block: a lane per row, four columns a warp
-      const int d0 = c0 + 32;
-      const float* row[1] = {R + (d0 + lane) * LD + c0};
-      const float* col[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) col[i] = R + (d0 + warp * 4 + i) * LD + c0;
-      uint64_t acc[1][4];
-      dots<1, 4>(row, col, 32, acc);
-      float* o = R + (d0 + lane) * LD + d0 + warp * 4;
-      float4 v = *reinterpret_cast<float4*>(o);
-      v.x -= sum2(acc[0][0]); v.y -= sum2(acc[0][1]); v.z -= sum2(acc[0][2]); v.w -= sum2(acc[0][3]);
-      *reinterpret_cast<float4*>(o) = v;
-      __syncthreads();
-    }
   }
-  // D[j][i] = (L^-T)[i][j]: a lane reads four columns of its row i, the lanes of a store hold consecutive i
-#pragma unroll 4
-  for (int idx = tid; idx < NB * NB / 4; idx += kThreads) {
-    const int i = idx & 127, j = (idx >> 7) << 2;
-    const float4 v = *reinterpret_cast<const float4*>(R + (NB + i) * LD + j);
-    const float e[4] = {v.x, v.y, v.z, v.w};
+  if (tid == 0 && bad) {
+    int* status = mt.status + 4 * blockIdx.x;
+    if (atomicCAS(status, 0, B200Q_NOT_POSITIVE_DEFINITE) == 0) status[1] = k0 + bad;
+  }
+  // D[j][i] = (L^-T)[i][j], zero above the diagonal; a thread turns 4 x 4 entries round
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
-      if (j + k < n && i < n) A[(int64_t)(j + k) * mt.lda + i] = (i <= j + k) ? e[k] : 0.0f;
+  for (int it = 0; it < NB * NB / 16 / kThreads; ++it) {
+    const int u = it * 8 + warp, i = (lane & 1) * 4 + (u & 15) * 8, j = (lane >> 1) * 4 + (u >> 4) * 64;
+    float v[4][4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float4 q = *reinterpret_cast<const float4*>(R + (NB + i + k) * LD + j);
+      v[k][0] = q.x; v[k][1] = q.y; v[k][2] = q.z; v[k][3] = q.w;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (j + k >= n) continue;
+      float* o = A + (int64_t)(j + k) * mt.lda + i;
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (i + e > j + k) v[e][k] = 0.0f;
+      if (i + 3 < n) *reinterpret_cast<float4*>(o) = make_float4(v[0][k], v[1][k], v[2][k], v[3][k]);
+      else
+        for (int e = 0; e < 4; ++e)
+          if (i + e < n) o[e] = v[e][k];
+    }
   }
 }
 
 // ---------------------------------------------------------------------------------------
-// Inside the square at K0 (n columns), step k: everything the diagonal block's inverse D multiplies.  A CTA owns 16
-// "vectors" of 128: rows r below the block (P[r] = A[r, blk] D^T, into the scratch P), then columns c left of it
-// (X[blk, c] = D S[blk, c], in place).  D is triangular, so output j needs only the first j + 1 terms.
+// Inside the square at K0 (n columns), step k: everything the diagonal block's inverse D multiplies.  Two CTAs own 16
+// "vectors" of 128, each 64 of their outputs: rows r below the block (P[r] = A[r, blk] D^T, into the scratch P), then
+// columns c left of it (X[blk, c] = D S[blk, c], into the scratch X; the update kernel puts them in their place).  D is
+// triangular, so output j needs only the first j + 1 terms.  The time is that of fetching D from L2.
 constexpr int kVec = 16;
-constexpr int kPanelSmemFloats = (NB + kVec) * LD;
+constexpr int kPanelSmemFloats = (NB / 2 + kVec) * LD;
 
 __global__ void __launch_bounds__(kThreads) panel_kernel(Mat mt, float* P0, int K0, int n, int k) {
   extern __shared__ __align__(16) float sm[];
-  float* D = sm;                 // [128][LD]
-  float* V = D + NB * LD;        // [16][LD] the CTA's vectors, contraction contiguous
-  float* A = mt.A + blockIdx.y * mt.batch + (int64_t)K0 * mt.lda + K0;
-  float* P = P0 + (int64_t)blockIdx.y * OB * NB;
+  float* D = sm;                   // [64][LD] rows of D
+  float* V = D + NB / 2 * LD;      // [16][LD] the vectors, contraction contiguous
+  const float* A = mt.A + blockIdx.y * mt.batch + (int64_t)K0 * mt.lda + K0;
+  float* P = P0 + (int64_t)blockIdx.y * kScratchFloats;
   const int tid = threadIdx.x, b0 = k * NB, bn = n - b0 < NB ? n - b0 : NB, below = n - b0 - bn;
-  const int below_ctas = (below + kVec - 1) / kVec;
-  const bool rows = (int)blockIdx.x < below_ctas;
-  const int v0 = rows ? b0 + bn + blockIdx.x * kVec : ((int)blockIdx.x - below_ctas) * kVec;
-  const float* Dk = A + (int64_t)b0 * mt.lda + b0;
-#pragma unroll 8
-  for (int idx = tid; idx < NB * NB / 4; idx += kThreads) {
-    const int r = idx >> 5, c = (idx & 31) << 2;
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (r < bn && c <= r) {
-      if (c + 3 < bn) v = *reinterpret_cast<const float4*>(Dk + (int64_t)r * mt.lda + c);
-      else {
-        float* e = &v.x;
-        for (int q = 0; q < 4; ++q)
-          if (c + q < bn) e[q] = Dk[(int64_t)r * mt.lda + c + q];
-      }
+  const int below_ctas = (below + kVec - 1) / kVec, unit = blockIdx.x >> 1, half = (blockIdx.x & 1) * 64;
+  const bool rows = unit < below_ctas;
+  const int v0 = rows ? b0 + bn + unit * kVec : (unit - below_ctas) * kVec;
+  const int depth = half + 64;
+  if (half >= bn) return;
+  for (int idx = tid; idx < 64 * (depth / 4); idx += kThreads) {
+    const int r = idx / (depth / 4), c = (idx - r * (depth / 4)) * 4, j = half + r;
+    const int left = (j < bn && c < bn) ? bn - c : 0;
+    cp_async16(D + r * LD + c, left ? A + (int64_t)(b0 + j) * mt.lda + b0 + c : A, left >= 4 ? 16 : left * 4);
+  }
+  if (rows) {
+    for (int idx = tid; idx < kVec * (depth / 4); idx += kThreads) {
+      const int v = idx / (depth / 4), c = (idx - v * (depth / 4)) * 4;
+      const int left = (v0 + v < n && c < bn) ? bn - c : 0;
+      cp_async16(V + v * LD + c, left ? A + (int64_t)(v0 + v) * mt.lda + b0 + c : A, left >= 4 ? 16 : left * 4);
     }
-    *reinterpret_cast<float4*>(D + r * LD + c) = v;
+  } else {
+    float x[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int idx = tid + i * kThreads, v = idx & 15, m = idx >> 4;
+      x[i] = (m < bn && m < depth) ? A[(int64_t)(b0 + m) * mt.lda + v0 + v] : 0.0f;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int idx = tid + i * kThreads;
+      V[(idx & 15) * LD + (idx >> 4)] = x[i];
+    }
   }
-  for (int idx = tid; idx < kVec * NB; idx += kThreads) {
-    const int v = rows ? idx >> 7 : idx & 15, m = rows ? idx & 127 : idx >> 4;
-    float x = 0.0f;
-    if (m < bn && (rows ? v0 + v < n : true))
-      x = rows ? A[(int64_t)(v0 + v) * mt.lda + b0 + m] : A[(int64_t)(b0 + m) * mt.lda + v0 + v];
-    V[v * LD + m] = x;
-  }
+  cp_async_wait_all();
   __syncthreads();
-  // outputs 4 vectors x 2 entries of D's rows per thread; a warp's rows of D are 32 consecutive ones
-  const int warp = tid >> 5, lane = tid & 31;
-  const int vq = lane & 3, j0 = (warp & 3) * 32 + (lane >> 2), jh = (warp >> 2) * 16;
-  const float *row[4], *col[2];
+  // a warp: 16 vectors x 8 outputs
+  const int warp = tid >> 5, lane = tid & 31, j0 = warp * 8;
+  float acc[1][4] = {};
+  mma_block<1, 4>(V, LD, D + j0 * LD, LD, 1, half + j0 + 8, lane, acc);
+  const int v = v0 + (lane >> 2), j = half + j0 + 2 * (lane & 3);
 #pragma unroll
-  for (int i = 0; i < 4; ++i) row[i] = V + (vq + 4 * i) * LD;
-#pragma unroll
-  for (int i = 0; i < 2; ++i) col[i] = D + (j0 + jh + 8 * i) * LD;
-  uint64_t acc[4][2];
-  dots<4, 2>(row, col, (warp & 3) * 32 + 32, acc);
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int v = v0 + vq + 4 * i, j = j0 + jh + 8 * q;
-      const float x = sum2(acc[i][q]);
-      if (j >= bn) continue;
-      if (rows) { if (v < n) P[(int64_t)v * NB + j] = x; }
-      else A[(int64_t)(b0 + j) * mt.lda + v] = x;
-    }
+  for (int e = 0; e < 4; ++e) {
+    const int vv = v + (e >> 1) * 8, jj = j + (e & 1);
+    if (jj >= bn) continue;
+    if (rows) { if (vv < n) P[(int64_t)vv * NB + jj] = acc[0][e]; }
+    else P[(int64_t)OB * NB + (int64_t)jj * OB + vv] = acc[0][e];
+  }
 }
 
 // Inside the square, step k: rows below the block take -P times X (columns left), D (the block's own columns, which
-// start from zero) and P^T (columns right, on and below the diagonal).  A CTA owns a 32 x 32 tile.
-constexpr int kUpdSmemFloats = 2 * 32 * LD;
+// start from zero) and P^T (columns right, on and below the diagonal); the block row itself takes X.  A CTA owns a
+// 32 x 32 tile, a warp 16 x 8 of it.
+constexpr int kUpdSmemFloats = 32 * LD + NB * 40;
 
-__global__ void __launch_bounds__(kThreads) square_update_kernel(Mat mt, const float* P0, int K0, int n, int k) {
+__global__ void __launch_bounds__(kThreads) square_update_kernel(Mat mt, const float* P0, int K0, int n, int k, int tiles) {
   extern __shared__ __align__(16) float sm[];
   float* Ps = sm;                // [32][LD]
-  float* Qs = Ps + 32 * LD;      // [32][LD] second operand, contraction contiguous
+  float* Qs = Ps + 32 * LD;      // second operand: [32][LD] contraction contiguous, or [128][40] column contiguous
   float* A = mt.A + blockIdx.y * mt.batch + (int64_t)K0 * mt.lda + K0;
-  const float* P = P0 + (int64_t)blockIdx.y * OB * NB;
+  const float* P = P0 + (int64_t)blockIdx.y * kScratchFloats;
+  const float* X = P + (int64_t)OB * NB;
   const int tid = threadIdx.x, b0 = k * NB, r_begin = b0 + NB;
+  if ((int)blockIdx.x >= tiles) {   // 32 x 32 of X into its place
+    const int u = blockIdx.x - tiles, y0 = (u & 3) * 32, x0 = (u >> 2) * 32, y = y0 + (tid >> 3), x = x0 + (tid & 7) * 4;
+    if (b0 + y < n)
+      *reinterpret_cast<float4*>(A + (int64_t)(b0 + y) * mt.lda + x) = *reinterpret_cast<const float4*>(X + (int64_t)y * OB + x);
+    return;
+  }
   // tile list: row tile i (32 rows from r_begin on) has r_begin / 32 + i + 1 column tiles
   const int base = r_begin / 32;
   int i = 0, t = blockIdx.x;
   while (t >= base + i + 1) { t -= base + i + 1; ++i; }
   const int r0 = r_begin + i * 32, c0 = t * 32;
   const bool right = c0 >= r_begin, own = !right && c0 >= b0;
-#pragma unroll 4
-  for (int idx = tid; idx < 32 * NB / 4; idx += kThreads) {
-    const int r = idx >> 5, m = (idx & 31) << 2;
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (r0 + r < n) v = *reinterpret_cast<const float4*>(P + (int64_t)(r0 + r) * NB + m);
-    *reinterpret_cast<float4*>(Ps + r * LD + m) = v;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int idx = tid + q * kThreads, r = idx >> 5, m = (idx & 31) << 2;
+    cp_async16(Ps + r * LD + m, P + (int64_t)(r0 + r < n ? r0 + r : 0) * NB + m, r0 + r < n ? 16 : 0);
   }
   if (right) {
-#pragma unroll 4
-    for (int idx = tid; idx < 32 * NB / 4; idx += kThreads) {
-      const int r = idx >> 5, m = (idx & 31) << 2;
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (c0 + r < n) v = *reinterpret_cast<const float4*>(P + (int64_t)(c0 + r) * NB + m);
-      *reinterpret_cast<float4*>(Qs + r * LD + m) = v;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int idx = tid + q * kThreads, r = idx >> 5, m = (idx & 31) << 2;
+      cp_async16(Qs + r * LD + m, P + (int64_t)(c0 + r < n ? c0 + r : 0) * NB + m, c0 + r < n ? 16 : 0);
     }
   } else {
-    // X or D of block row k (all 128 rows exist: there are rows below): four rows of one column per float4
-#pragma unroll 4
-    for (int idx = tid; idx < 32 * NB / 4; idx += kThreads) {
-      const int c = idx & 31, m = (idx >> 5) << 2;
-      const float* src = A + (int64_t)(b0 + m) * mt.lda + c0 + c;
-      *reinterpret_cast<float4*>(Qs + c * LD + m) =
-          make_float4(src[0], src[mt.lda], src[2 * mt.lda], src[3 * mt.lda]);
+    // D or X of block row k, which has all its 128 rows: there are rows below
+    const float* src = own ? A + (int64_t)b0 * mt.lda + c0 : X + c0;
+    const int64_t ld = own ? mt.lda : OB;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int idx = tid + q * kThreads, m = idx >> 3, c = (idx & 7) << 2;
+      cp_async16(Qs + m * 40 + c, src + (int64_t)m * ld + c, 16);
     }
   }
+  const int warp = tid >> 5, lane = tid & 31, tr = (warp & 1) * 16, tc = (warp >> 1) * 8;
+  const int r = r0 + tr + (lane >> 2), c = c0 + tc + 2 * (lane & 3);
+  float old[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const int rr = r + (e >> 1) * 8, cc = c + (e & 1);
+    old[e] = (!own && rr < n && cc < n) ? A[(int64_t)rr * mt.lda + cc] : 0.0f;
+  }
+  cp_async_wait_all();
   __syncthreads();
-  const int warp = tid >> 5, lane = tid & 31;
-  const int r = (warp & 3) * 8 + (lane >> 3) * 2, c = (warp >> 2) * 16 + (lane & 7);
-  const float* row[2] = {Ps + r * LD, Ps + (r + 1) * LD};
-  const float* col[2] = {Qs + c * LD, Qs + (c + 8) * LD};
-  float old[2][2];
+  float acc[1][4] = {};
+  if (right) mma_block<1, 4>(Ps + tr * LD, LD, Qs + tc * LD, LD, 1, NB, lane, acc);
+  else mma_block<1, 4>(Ps + tr * LD, LD, Qs + tc, 1, 40, NB, lane, acc);
 #pragma unroll
-  for (int y = 0; y < 2; ++y)
-#pragma unroll
-    for (int x = 0; x < 2; ++x)
-      old[y][x] = (!own && r0 + r + y < n && c0 + c + 8 * x < n) ? A[(int64_t)(r0 + r + y) * mt.lda + c0 + c + 8 * x] : 0.0f;
-  uint64_t acc[2][2];
-  dots<2, 2>(row, col, NB, acc);
-#pragma unroll
-  for (int y = 0; y < 2; ++y)
-#pragma unroll
-    for (int x = 0; x < 2; ++x)
-      if (r0 + r + y < n && c0 + c + 8 * x < n)
-        A[(int64_t)(r0 + r + y) * mt.lda + c0 + c + 8 * x] = old[y][x] - sum2(acc[y][x]);
+  for (int e = 0; e < 4; ++e) {
+    const int rr = r + (e >> 1) * 8, cc = c + (e & 1);
+    if (rr < n && cc < n) A[(int64_t)rr * mt.lda + cc] = old[e] - acc[0][e];
+  }
 }
 
 // ---------------------------------------------------------------------------------------
@@ -437,7 +506,7 @@ static int64_t round_up(int64_t v, int64_t m) { return (v + m - 1) / m * m; }
 // more than one outer block) three operand panels with a row per matrix row
 static int64_t problem_floats(int64_t K) {
   const int64_t rows = round_up(K, NB);
-  return K * round_up(K, 32) + OB * NB + (K > OB ? 2 * OB * OB + 6 * rows * OB : 0);
+  return K * round_up(K, 32) + kScratchFloats + (K > OB ? 2 * OB * OB + 6 * rows * OB : 0);
 }
 
 // SMs the bulk of an update leaves to the chain beside it: the square's kernels are small (24 to 120 CTAs of which
@@ -454,7 +523,7 @@ static int factor(float* H, float* const* Hs, int batch, int64_t K, int64_t ldh,
   Mat mt;
   mt.A = ws; mt.batch = K * lda; mt.lda = lda; mt.status = status;
   float* P = ws + (int64_t)batch * K * lda;
-  float* d_hi = P + (int64_t)batch * OB * NB;
+  float* d_hi = P + (int64_t)batch * kScratchFloats;
   float* d_lo = d_hi + (int64_t)batch * OB * OB;
   float* a_hi = d_lo + (int64_t)batch * OB * OB;          // panel before its product with D, and S[o,:o]^T
   const int64_t cap = (int64_t)batch * rows * OB, pb = rows * OB;
@@ -481,17 +550,14 @@ static int factor(float* H, float* const* Hs, int batch, int64_t K, int64_t ldh,
       const int bn = n - k * NB < NB ? n - k * NB : NB, below = n - k * NB - bn;
       chol_diag_kernel<<<batch, kThreads, chol_smem, st>>>(mt, (int)K0 + k * NB, bn);
       B200Q_LAUNCH_CHECK();
-      const int vec_ctas = (below + kVec - 1) / kVec + k * NB / kVec;
-      if (vec_ctas) {
-        panel_kernel<<<dim3(vec_ctas, batch), kThreads, panel_smem, st>>>(mt, P, (int)K0, n, k);
-        B200Q_LAUNCH_CHECK();
-      }
-      if (below > 0) {
-        const int rt = (below + 31) / 32, base = (k + 1) * (NB / 32);
-        square_update_kernel<<<dim3(rt * base + rt * (rt + 1) / 2, batch), kThreads, kUpdSmemFloats * sizeof(float), st>>>(
-            mt, P, (int)K0, n, k);
-        B200Q_LAUNCH_CHECK();
-      }
+      const int units = (below + kVec - 1) / kVec + k * NB / kVec;
+      if (units == 0) continue;
+      panel_kernel<<<dim3(2 * units, batch), kThreads, panel_smem, st>>>(mt, P, (int)K0, n, k);
+      B200Q_LAUNCH_CHECK();
+      const int rt = (below + 31) / 32, base = (k + 1) * (NB / 32), tiles = rt * base + rt * (rt + 1) / 2;
+      square_update_kernel<<<dim3(tiles + k * 16, batch), kThreads, kUpdSmemFloats * sizeof(float), st>>>(
+          mt, P, (int)K0, n, k, tiles);
+      B200Q_LAUNCH_CHECK();
     }
     if (K0 == 0 && last) break;
     float* q_hi = q_base + (step & 1) * 2 * cap;
