@@ -22,7 +22,9 @@ constexpr size_t kSweepHeaderBytes = 256;    // status word at the start of the 
 constexpr int kRows = 32;                    // rows of a CTA: a lane each
 constexpr int kMicro = 16;                   // columns a lane keeps in registers at a time
 constexpr int kThreads = 256;
-constexpr int WLD = kRows + 1;
+constexpr int WLD = kRows + 4, ELD = kRows + 8;   // columns of W and of the errors in shared memory: the strides
+                                                  // make the MMA fragments' accesses conflict-free
+__host__ __device__ constexpr int u_stride(int superblock) { return superblock + 8; }   // likewise
 
 // One pointer per operand, or (table set) a device array with one per problem.
 template <class T> struct Ptr {
@@ -42,11 +44,11 @@ struct Params {
 };
 
 __host__ __device__ constexpr size_t smem_bytes(int superblock) {
-  return (size_t)(superblock * WLD            // W, column-major
-                  + 3 * kMicro * superblock   // rows of U of three micro-blocks
-                  + 2 * kMicro * WLD          // errors of two micro-blocks
-                  + 2 * 3 * kMicro * kRows    // scale, 1 / scale, zero point of two micro-blocks
-                  + 2 * superblock) * sizeof(float);   // 1 / U[i,i], parameter column
+  return (size_t)(3 * kMicro * u_stride(superblock)   // rows of U of three micro-blocks
+                  + 2 * 4 * kMicro * kRows            // parameters of two micro-blocks
+                  + 2 * superblock                    // 1 / U[i,i], parameter column
+                  + 2 * kMicro * ELD                  // errors of two micro-blocks
+                  + superblock * WLD) * sizeof(float);   // W, column-major
 }
 
 __device__ __forceinline__ void cp_async16(float* dst, const float* src, int src_bytes) {
@@ -69,23 +71,72 @@ __device__ __forceinline__ void unpair(uint64_t v, float& lo, float& hi) {
   asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
 }
 
-// What bounds it: the chain of 512 columns, about 65 cycles each for the quantisation (product with 1 / s at both
-// ends of an interval, clamp, round, dequantise, difference, product with the reciprocal pivot, correction of the
-// next column).  So one warp of the CTA does nothing but the chain: 16 columns at a time in registers, a lane per
-// row.  The other seven apply a finished micro-block's 16 errors to the columns two micro-blocks on and later (the
-// columns next in line are corrected by the chain warp itself), write its errors out as the operand of the trailing
-// product, and fetch parameters and rows of U ahead.  One barrier per micro-block.
-template <int SDT, bool GLOBAL, int KIND>
+// ---- quantisation of a column on the chain
+// The code of x is settled by x * (1 / s) taken slightly low and slightly high: equal codes mean that the ulps between
+// the product and the reference's division cannot matter.  Whether they are equal is not waited for column by column:
+// a micro-block whose flags show a difference anywhere (some per mille of them) is swept again by the exact rules.
+constexpr float kMargin = 0x1p-21f;   // > the 2^-22 by which reciprocal, product and division can differ in all
+
+template <int KIND>
+__device__ __forceinline__ float code_of(float v, float qmin, float qmax) {
+  v = fminf(fmaxf(v, qmin), qmax);
+  if constexpr (KIND == kInt) {
+    return (v + 12582912.0f) - 12582912.0f;   // 1.5 * 2^23: rounds to nearest even (the sign of a zero is put back later)
+  } else if constexpr (KIND == kFp8) {
+    return e4m3_round(v);
+  } else {
+    uint32_t h;   // through the hardware's E2M1 pair and back
+    asm("{\n\t.reg .b8 b;\n\tcvt.rn.satfinite.e2m1x2.f32 b, %1, %1;\n\tcvt.rn.f16x2.e2m1x2 %0, b;\n\t}" : "=r"(h) : "f"(v));
+    return __half2float(__ushort_as_half((unsigned short)(h & 0xFFFFu)));
+  }
+}
+// bf16 rounding with the result already in place as a float
+__device__ __forceinline__ float bf16_in_place(float v) {
+  uint32_t d;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(v), "f"(0.0f));
+  return __uint_as_float(d);
+}
+template <int KIND, bool SB, bool ZP>
+__device__ __forceinline__ float dequant(float q, float s, float z) {
+  if (ZP) {
+    q = q - z;
+    if (SB && KIND != kInt) q = bf16_in_place(q);   // (integer differences are exact in bf16)
+  }
+  q = q * s;
+  return SB ? bf16_in_place(q) : q;
+}
+
+// three tf32 MMAs per product of hi / lo splits, as in tgemm
+__device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) {
+  hi = (__float_as_uint(x) + 0x1000u) & 0xFFFFE000u;
+  lo = (__float_as_uint(x - __uint_as_float(hi)) + 0x1000u) & 0xFFFFE000u;
+}
+__device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+
+// What bounds it: the chain of columns, some 45 cycles each for the quantisation (product with 1 / s, clamp, round,
+// dequantise, difference, product with the reciprocal pivot, correction of the next column).  So one warp of the CTA
+// does nothing but the chain: 16 columns at a time in registers, a lane per row.  The other seven apply a finished
+// micro-block's 16 errors to the columns two micro-blocks on and later as warp-level tensor-core products (a float32
+// FMA formulation spends its time on the broadcast loads of U: 480 cycles a column against the chain's own), write its
+// errors out as the operand of the trailing product, and fetch parameters and rows of U ahead.  The columns next in
+// line are corrected by the chain warp itself.  One barrier per micro-block.
+template <int SDT, bool GLOBAL, int KIND, bool ZP>
 __global__ void __launch_bounds__(kThreads) sweep_block_kernel(const __grid_constant__ Params p, int superblock) {
   constexpr bool SB = Elem<SDT>::is_bf16 && !GLOBAL;
   const float qmin = p.qr.qmin, qmax = p.qr.qmax;
   extern __shared__ __align__(16) float sm[];
-  float* sU = sm;                                      // [3][kMicro][superblock]
-  float* sP = sU + 3 * kMicro * superblock;            // [2][3][kMicro][kRows]
-  float* sRd = sP + 2 * 3 * kMicro * kRows;            // [superblock]
+  const int ULD = u_stride(superblock);
+  float* sU = sm;                                      // [3][kMicro][ULD]
+  float* sP = sU + 3 * kMicro * ULD;                   // [2][scale, low and high 1 / scale, zero point][kMicro][kRows]
+  float* sRd = sP + 2 * 4 * kMicro * kRows;            // [superblock]
   int* sGrp = reinterpret_cast<int*>(sRd + superblock);// [superblock]
-  float* sE = sRd + 2 * superblock;                    // [2][kMicro][WLD]
-  float* sW = sE + 2 * kMicro * WLD;                   // [superblock][WLD]
+  float* sE = sRd + 2 * superblock;                    // [2][kMicro][ELD]
+  float* sW = sE + 2 * kMicro * ELD;                   // [superblock][WLD]
+  __shared__ int s_odd;                                // some scale is outside the range the low / high test covers
   const int job = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int sb = p.sb, micros = (sb + kMicro - 1) / kMicro;
   float* __restrict__ W = p.W.at(job) + p.i1;
@@ -98,6 +149,7 @@ __global__ void __launch_bounds__(kThreads) sweep_block_kernel(const __grid_cons
   const int64_t row0 = (int64_t)blockIdx.x * kRows, row = row0 + lane;
   const bool live = row < p.N;
   const bool vecu = U && ((p.ldu & 3) == 0) && ((((uintptr_t)U) & 15) == 0);
+  const bool vecw = ((p.ldw & 3) == 0) && ((((uintptr_t)W) & 15) == 0) && (sb & 3) == 0;
   int64_t pbase;
   switch (p.strategy) {
     case B200Q_TENSOR: pbase = 0; break;
@@ -107,11 +159,11 @@ __global__ void __launch_bounds__(kThreads) sweep_block_kernel(const __grid_cons
   }
   // rows of U of micro-block m, columns from its own first one on (columns beyond sb are zero)
   auto fetch_u = [&](int m, int t0, int nt) {
-    float* dst = sU + (m % 3) * kMicro * superblock;
+    float* dst = sU + (m % 3) * kMicro * ULD;
     const int c0 = m * kMicro, quads = (micros * kMicro - c0) >> 2;
     for (int idx = t0; idx < kMicro * quads; idx += nt) {
       const int t = idx / quads, c = c0 + (idx - t * quads) * 4, i = c0 + t;
-      float* d = dst + t * superblock + c;
+      float* d = dst + t * ULD + c;
       if (vecu) {
         const int bytes = (i < sb && c < sb) ? (sb - c >= 4 ? 16 : (sb - c) * 4) : 0;
         cp_async16(d, bytes ? U + (int64_t)i * p.ldu + c : U, bytes);
@@ -127,22 +179,33 @@ __global__ void __launch_bounds__(kThreads) sweep_block_kernel(const __grid_cons
   };
   // parameters of micro-block m's columns for the CTA's rows (columns beyond sb: unit scale)
   auto fetch_params = [&](int m, int w0, int nw) {
-    float* dst = sP + (m & 1) * 3 * kMicro * kRows + lane;
-#pragma unroll 3
-    for (int t = w0; t < kMicro; t += nw) {
-      const int c = m * kMicro + t;
-      float s = 1.0f, z = 0.0f;
-      if (c < sb && live) {
+    float* dst = sP + (m & 1) * 4 * kMicro * kRows + lane;
+    float sv[3], zv[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const int t = w0 + k * nw, c = m * kMicro + t;
+      sv[k] = 1.0f; zv[k] = 0.0f;
+      if (t < kMicro && c < sb && live) {
         const int64_t pi = pbase + sGrp[c];
-        s = Elem<SDT>::load((const typename Elem<SDT>::type*)scale + pi);
-        if (GLOBAL) s = __fdiv_rn(s, g);
-        if (zp) z = load_zp(zp, p.zp_kind, pi);
+        sv[k] = Elem<SDT>::load((const typename Elem<SDT>::type*)scale + pi);
+        if (ZP) zv[k] = load_zp(zp, p.zp_kind, pi);
       }
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const int t = w0 + k * nw;
+      if (t >= kMicro) continue;
+      float s = sv[k];
+      if (GLOBAL) s = __fdiv_rn(s, g);
+      const float rs = __frcp_rn(s);
+      if (!(s >= 0x1p-100f && s <= 0x1p100f)) s_odd = 1;
       dst[t * kRows] = s;
-      dst[(kMicro + t) * kRows] = __frcp_rn(s);
-      dst[(2 * kMicro + t) * kRows] = z;
+      dst[(kMicro + t) * kRows] = rs * (1.0f - kMargin);
+      dst[(2 * kMicro + t) * kRows] = rs * (1.0f + kMargin);
+      dst[(3 * kMicro + t) * kRows] = zv[k];
     }
   };
+  if (tid == 0) s_odd = 0;
   fetch_u(0, tid, kThreads);
   if (micros > 1) fetch_u(1, tid, kThreads); else cp_async_commit();
   for (int c = tid; c < micros * kMicro; c += kThreads) {
@@ -156,12 +219,26 @@ __global__ void __launch_bounds__(kThreads) sweep_block_kernel(const __grid_cons
     sRd[c] = __frcp_rn(d);
     sGrp[c] = grp;
   }
-  // tile in: rows coalesced, columns transposed; a warp takes four rows
-  for (int r = warp * 4; r < warp * 4 + 4; ++r) {
-    const bool in = row0 + r < p.N;
-    const float* src = W + (row0 + r) * p.ldw;
-#pragma unroll 4
-    for (int c = lane; c < micros * kMicro; c += 32) sW[c * WLD + r] = (in && c < sb) ? src[c] : 0.0f;
+  // tile in: a lane per row, eight columns (a whole sector) at a time
+  if (vecw) {
+    for (int c = warp * 8; c < micros * kMicro; c += 8 * (kThreads / 32)) {
+      float4 v[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        v[h] = (live && c + 4 * h < sb) ? *reinterpret_cast<const float4*>(W + row * p.ldw + c + 4 * h)
+                                        : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float* d = sW + (c + 4 * h) * WLD + lane;
+        d[0] = v[h].x; d[WLD] = v[h].y; d[2 * WLD] = v[h].z; d[3 * WLD] = v[h].w;
+      }
+    }
+  } else {
+    for (int r = warp * 4; r < warp * 4 + 4; ++r) {
+      const bool in = row0 + r < p.N;
+      const float* src = W + (row0 + r) * p.ldw;
+      for (int c = lane; c < micros * kMicro; c += 32) sW[c * WLD + r] = (in && c < sb) ? src[c] : 0.0f;
+    }
   }
   __syncthreads();
   fetch_params(0, warp, kThreads / 32);
@@ -175,9 +252,9 @@ __global__ void __launch_bounds__(kThreads) sweep_block_kernel(const __grid_cons
 #pragma unroll 1
   for (int m = 0; m < micros; ++m) {
     const int c0 = m * kMicro;
-    const float* u_prev = sU + ((m + 2) % 3) * kMicro * superblock;
+    const float* u_prev = sU + ((m + 2) % 3) * kMicro * ULD;
     if (warp == 0) {
-      const float* u = sU + (m % 3) * kMicro * superblock + c0;
+      const float* u = sU + (m % 3) * kMicro * ULD + c0;
       float w[kMicro];
       {
         // the errors of the micro-block before this one
@@ -190,7 +267,7 @@ __global__ void __launch_bounds__(kThreads) sweep_block_kernel(const __grid_cons
             const uint64_t ne = pair(-e[t], -e[t]);
 #pragma unroll
             for (int k = 0; k < kMicro / 4; ++k) {
-              const ulonglong2 uu = *reinterpret_cast<const ulonglong2*>(u_prev + t * superblock + c0 + 4 * k);
+              const ulonglong2 uu = *reinterpret_cast<const ulonglong2*>(u_prev + t * ULD + c0 + 4 * k);
               fma2(v[2 * k], ne, uu.x);
               fma2(v[2 * k + 1], ne, uu.y);
             }
@@ -199,57 +276,108 @@ __global__ void __launch_bounds__(kThreads) sweep_block_kernel(const __grid_cons
 #pragma unroll
         for (int k = 0; k < kMicro / 2; ++k) unpair(v[k], w[2 * k], w[2 * k + 1]);
       }
-      const float* par = sP + (m & 1) * 3 * kMicro * kRows + lane;
-      float sv[kMicro], rsv[kMicro], zv[kMicro], rd[kMicro];
+      // kept for the exact pass, should it be needed
+#pragma unroll
+      for (int t = 0; t < kMicro; ++t) sW[(c0 + t) * WLD + lane] = w[t];
+      const float* par = sP + (m & 1) * 4 * kMicro * kRows + lane;
+      bool differ = false;
 #pragma unroll
       for (int t = 0; t < kMicro; ++t) {
-        sv[t] = par[t * kRows]; rsv[t] = par[(kMicro + t) * kRows]; zv[t] = par[(2 * kMicro + t) * kRows];
-        rd[t] = sRd[c0 + t];
-      }
-#pragma unroll
-      for (int t = 0; t < kMicro; ++t) {
-        const float wi = w[t];
-        const float q = fake_quant_f32<KIND, SB>(wi, sv[t], rsv[t], zv[t], qmin, qmax);
+        const float s = par[t * kRows], rlo = par[(kMicro + t) * kRows], rhi = par[(2 * kMicro + t) * kRows];
+        const float z = ZP ? par[(3 * kMicro + t) * kRows] : 0.0f, mz = ZP ? fabsf(z) * (0.5f * kMargin) : 0.0f;
+        const float wi = w[t], lo = fmaf(wi, rlo, z - mz);
+        const float qc = code_of<KIND>(lo, qmin, qmax);
+        differ |= qc != code_of<KIND>(fmaf(wi, rhi, z + mz), qmin, qmax);
+        const float q = dequant<KIND, SB, ZP>(qc, s, z);
         // loss and error use the reciprocal of the pivot (an ulp from the reference's divisions)
-        const float tt = __fmul_rn(__fsub_rn(wi, q), rd[t]);
-        loss = fmaf(tt, tt, loss);
+        const float tt = __fmul_rn(__fsub_rn(wi, q), sRd[c0 + t]);
         e[t] = tt;
-        w[t] = q;
+        // a zero has the sign of the quotient: x / s + 0 is -0 for a small negative x, and stays it
+        w[t] = (KIND == kInt && (!ZP || (q == 0.0f && z == 0.0f))) ? copysignf(q, lo) : q;
 #pragma unroll
         for (int k4 = (t + 1) / 4; k4 < kMicro / 4; ++k4) {
-          const float4 uu = *reinterpret_cast<const float4*>(u + t * superblock + 4 * k4);
+          const float4 uu = *reinterpret_cast<const float4*>(u + t * ULD + 4 * k4);
           if (4 * k4 + 0 > t) w[4 * k4 + 0] = fmaf(-tt, uu.x, w[4 * k4 + 0]);
           if (4 * k4 + 1 > t) w[4 * k4 + 1] = fmaf(-tt, uu.y, w[4 * k4 + 1]);
           if (4 * k4 + 2 > t) w[4 * k4 + 2] = fmaf(-tt, uu.z, w[4 * k4 + 2]);
           if (4 * k4 + 3 > t) w[4 * k4 + 3] = fmaf(-tt, uu.w, w[4 * k4 + 3]);
         }
       }
-      float* eo = sE + (m & 1) * kMicro * WLD + lane;
-#pragma unroll
-      for (int t = 0; t < kMicro; ++t) { sW[(c0 + t) * WLD + lane] = w[t]; eo[t * WLD] = e[t]; }
-    } else {
-      if (m > 0) {
-        const float* ei = sE + ((m - 1) & 1) * kMicro * WLD + lane;
-        uint64_t ne[kMicro];
-#pragma unroll
-        for (int t = 0; t < kMicro; ++t) { const float x = -ei[t * WLD]; ne[t] = pair(x, x); }
+      float* eo = sE + (m & 1) * kMicro * ELD + lane;
+      if (__any_sync(0xffffffffu, differ) || s_odd) {
+        // by the exact rules, column by column in shared memory
 #pragma unroll 1
-        for (int c = c0 + kMicro + (warp - 1) * 8; c < micros * kMicro; c += 7 * 8) {
-          uint64_t v[4];
+        for (int t = 0; t < kMicro; ++t) {
+          float* wt = sW + (c0 + t) * WLD + lane;
+          const float wi = *wt, s = par[t * kRows], z = ZP ? par[(3 * kMicro + t) * kRows] : 0.0f;
+          const float q = dequant_code<SB>(round_code_k<KIND>(__fdiv_rn(wi, s) + z, qmin, qmax), s, z);
+          const float tt = __fmul_rn(__fsub_rn(wi, q), sRd[c0 + t]);
+          *wt = q;
+          eo[t * ELD] = tt;
+          for (int k = t + 1; k < kMicro; ++k) {
+            float* wk = sW + (c0 + k) * WLD + lane;
+            *wk = fmaf(-tt, u[t * ULD + k], *wk);
+          }
+        }
 #pragma unroll
-          for (int h = 0; h < 4; ++h) v[h] = pair(sW[(c + 2 * h) * WLD + lane], sW[(c + 2 * h + 1) * WLD + lane]);
+        for (int t = 0; t < kMicro; ++t) e[t] = eo[t * ELD];
+      } else {
 #pragma unroll
-          for (int t = 0; t < kMicro; ++t) {
-            const ulonglong2 ua = *reinterpret_cast<const ulonglong2*>(u_prev + t * superblock + c);
-            const ulonglong2 ub = *reinterpret_cast<const ulonglong2*>(u_prev + t * superblock + c + 4);
-            fma2(v[0], ne[t], ua.x); fma2(v[1], ne[t], ua.y); fma2(v[2], ne[t], ub.x); fma2(v[3], ne[t], ub.y);
+        for (int t = 0; t < kMicro; ++t) { sW[(c0 + t) * WLD + lane] = w[t]; eo[t * ELD] = e[t]; }
+      }
+#pragma unroll
+      for (int t = 0; t < kMicro; ++t) loss = fmaf(e[t], e[t], loss);
+    } else {
+      if (m > 0 && m + 1 < micros) {
+        // W[32 rows, 16 columns at a time] -= E[32, 16] U[16, columns]
+        const float* ei = sE + ((m - 1) & 1) * kMicro * ELD + (lane & 3) * ELD + (lane >> 2);
+        uint32_t ah[2][2][4], al[2][2][4];   // [row tile][k step]
+#pragma unroll
+        for (int y = 0; y < 2; ++y)
+#pragma unroll
+          for (int ks = 0; ks < 2; ++ks)
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              split_tf32(ei[(ks * 8 + (k >> 1) * 4) * ELD + y * 16 + (k & 1) * 8], ah[y][ks][k], al[y][ks][k]);
+#pragma unroll 1
+        for (int mc = m + warp; mc < micros; mc += 7) {
+          const int c = mc * kMicro;
+          float* o = sW + (c + 2 * (lane & 3)) * WLD + (lane >> 2);
+          const float* ub = u_prev + (lane & 3) * ULD + c + (lane >> 2);
+          float old[2][2][4], acc[2][2][4] = {}, part[2][2][4] = {};   // [row tile][column tile]
+#pragma unroll
+          for (int y = 0; y < 2; ++y)
+#pragma unroll
+            for (int x = 0; x < 2; ++x)
+#pragma unroll
+              for (int k = 0; k < 4; ++k) old[y][x][k] = o[(x * 8 + (k & 1)) * WLD + y * 16 + (k >> 1) * 8];
+#pragma unroll
+          for (int ks = 0; ks < 2; ++ks) {
+            uint32_t bh[2][2], bl[2][2];
+#pragma unroll
+            for (int x = 0; x < 2; ++x)
+#pragma unroll
+              for (int k = 0; k < 2; ++k) split_tf32(ub[(ks * 8 + k * 4) * ULD + x * 8], bh[x][k], bl[x][k]);
+#pragma unroll
+            for (int y = 0; y < 2; ++y)
+#pragma unroll
+              for (int x = 0; x < 2; ++x) mma_tf32(acc[y][x], ah[y][ks], bh[x]);
+#pragma unroll
+            for (int y = 0; y < 2; ++y)
+#pragma unroll
+              for (int x = 0; x < 2; ++x) mma_tf32(part[y][x], ah[y][ks], bl[x]);
+#pragma unroll
+            for (int y = 0; y < 2; ++y)
+#pragma unroll
+              for (int x = 0; x < 2; ++x) mma_tf32(part[y][x], al[y][ks], bh[x]);
           }
 #pragma unroll
-          for (int h = 0; h < 4; ++h) {
-            float lo, hi;
-            unpair(v[h], lo, hi);
-            sW[(c + 2 * h) * WLD + lane] = lo; sW[(c + 2 * h + 1) * WLD + lane] = hi;
-          }
+          for (int y = 0; y < 2; ++y)
+#pragma unroll
+            for (int x = 0; x < 2; ++x)
+#pragma unroll
+              for (int k = 0; k < 4; ++k)
+                o[(x * 8 + (k & 1)) * WLD + y * 16 + (k >> 1) * 8] = old[y][x][k] - (acc[y][x][k] + part[y][x][k]);
         }
       }
       if (m + 1 < micros) fetch_params(m + 1, warp - 1, 7);
@@ -258,11 +386,11 @@ __global__ void __launch_bounds__(kThreads) sweep_block_kernel(const __grid_cons
     auto store_errors = [&](int of, int t) {
       const int r = t & 31, q = (t >> 5) * 4;
       if (t >= 128 || row0 + r >= p.N) return;
-      const float* ei = sE + (of & 1) * kMicro * WLD + r;
+      const float* ei = sE + (of & 1) * kMicro * ELD + r;
       float h[4], l[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        const float x = ei[(q + k) * WLD];
+        const float x = ei[(q + k) * ELD];
         h[k] = tgemm::tf32_rn(x);
         l[k] = tgemm::tf32_rn(x - h[k]);
       }
@@ -273,17 +401,25 @@ __global__ void __launch_bounds__(kThreads) sweep_block_kernel(const __grid_cons
     if (p.err_hi && m > 0 && warp > 0) store_errors(m - 1, tid - 32);
     cp_async_wait<0>();
     __syncthreads();
-    if (m + 2 < micros && warp > 0) {   // the buffer of micro-block m - 1 is free
-      fetch_u(m + 2, tid - 32, kThreads - 32);
-    }
+    if (m + 2 < micros && warp > 0) fetch_u(m + 2, tid - 32, kThreads - 32);   // the buffer of micro-block m - 1 is free
     if (m + 1 == micros && p.err_hi) store_errors(m, tid);   // (a superblock with columns after it is a whole one)
   }
   // tile out
-  for (int r = warp * 4; r < warp * 4 + 4; ++r) {
-    if (row0 + r >= p.N) break;
-    float* dst = W + (row0 + r) * p.ldw;
-#pragma unroll 4
-    for (int c = lane; c < sb; c += 32) dst[c] = sW[c * WLD + r];
+  if (vecw) {
+    for (int c = warp * 8; c < sb; c += 8 * (kThreads / 32)) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float* d = sW + (c + 4 * h) * WLD + lane;
+        if (live && c + 4 * h < sb)
+          *reinterpret_cast<float4*>(W + row * p.ldw + c + 4 * h) = make_float4(d[0], d[WLD], d[2 * WLD], d[3 * WLD]);
+      }
+    }
+  } else {
+    for (int r = warp * 4; r < warp * 4 + 4; ++r) {
+      if (row0 + r >= p.N) break;
+      float* dst = W + (row0 + r) * p.ldw;
+      for (int c = lane; c < sb; c += 32) dst[c] = sW[c * WLD + r];
+    }
   }
   if (warp == 0 && live) {
     float* lo = p.losses.at(job);
@@ -328,17 +464,20 @@ static int sweep(Params p, int sdtype, bool global, int batch, const float* cons
   float* err = (float*)((char*)workspace + kSweepHeaderBytes);   // [sets][hi, lo]
   float* ub = err + 2 * l.sets * l.err;                          // [sets][hi, lo]
   B200Q_TRY(cudaMemsetAsync(status, 0, sizeof(int), st));
+  const bool with_zp = p.zp.one || p.zp.table;
   void (*kern)(const Params, int) = nullptr;
-#define B200Q_SWEEP_PICK(SDT)                                                                                              \
-  do {                                                                                                                     \
-    if (p.qr.kind == kInt) kern = global ? sweep_block_kernel<SDT, true, kInt> : sweep_block_kernel<SDT, false, kInt>;      \
-    else if (p.qr.kind == kFp8) kern = global ? sweep_block_kernel<SDT, true, kFp8> : sweep_block_kernel<SDT, false, kFp8>; \
-    else kern = global ? sweep_block_kernel<SDT, true, kFp4> : sweep_block_kernel<SDT, false, kFp4>;                        \
+#define B200Q_SWEEP_KIND(SDT, G, K) kern = with_zp ? sweep_block_kernel<SDT, G, K, true> : sweep_block_kernel<SDT, G, K, false>
+#define B200Q_SWEEP_PICK(SDT)                                                                                            \
+  do {                                                                                                                   \
+    if (p.qr.kind == kInt) { if (global) B200Q_SWEEP_KIND(SDT, true, kInt); else B200Q_SWEEP_KIND(SDT, false, kInt); }       \
+    else if (p.qr.kind == kFp8) { if (global) B200Q_SWEEP_KIND(SDT, true, kFp8); else B200Q_SWEEP_KIND(SDT, false, kFp8); } \
+    else { if (global) B200Q_SWEEP_KIND(SDT, true, kFp4); else B200Q_SWEEP_KIND(SDT, false, kFp4); }                       \
   } while (0)
   if (sdtype == B200Q_BF16) B200Q_SWEEP_PICK(B200Q_BF16);
   else if (sdtype == B200Q_F32) B200Q_SWEEP_PICK(B200Q_F32);
   else return B200Q_ERR_UNSUPPORTED;
 #undef B200Q_SWEEP_PICK
+#undef B200Q_SWEEP_KIND
   // always the largest size: host threads on other streams launch the same kernel with other widths
   B200Q_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(512)));
   const int ctas = (int)((N + kRows - 1) / kRows);

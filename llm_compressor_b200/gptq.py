@@ -276,7 +276,9 @@ def quantize_weight(module, quant_args, hessian: Optional[torch.Tensor], blocksi
     the call without ``defer`` (after re-observing the weight) if the factorisation turned out
     to have failed."""
     inp = _sweep_input(module, quant_args, hessian, percdamp, factor)
-    losses, status = ops.gptq_sweep(inp.W, inp.factor.U, inp.scale, inp.zero_point, inp.args, blocksize=blocksize,
+    # (a symmetric scheme's zero points are all zero: the sweep does without them)
+    zero_point = None if inp.args.symmetric else inp.zero_point
+    losses, status = ops.gptq_sweep(inp.W, inp.factor.U, inp.scale, zero_point, inp.args, blocksize=blocksize,
                                     col_group=inp.col_group, global_scale=inp.global_scale, return_status=True)
     out = _sweep_output(inp)
     if defer:
@@ -313,7 +315,7 @@ def quantize_weights_batched(modules, quant_args, factors, blocksize: int = 128,
         return None if vals[0] is None else vals
 
     losses, status = ops.gptq_sweep_batched([i.W for i in inputs], [i.factor.U for i in inputs], column("scale"),
-                                    column("zero_point"), first.args, col_groups=column("col_group"),
+                                    None if first.args.symmetric else column("zero_point"), first.args, col_groups=column("col_group"),
                                     global_scales=column("global_scale"), blocksize=blocksize,
                                             return_status=True)
     sums = losses.sum(dim=1)
