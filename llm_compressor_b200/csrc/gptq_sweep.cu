@@ -41,23 +41,30 @@ struct Params {
   QRange qr;
   float* err_hi; float* err_lo; int64_t lde, err_batch;   // operand form of the superblock's errors (null: nothing after it)
   int i1, sb;                                             // superblock: first column, width
+  int sdtype;                                             // of the scales
+  int* status;                                            // set if a bounded wait expires
 };
 
 __host__ __device__ constexpr size_t smem_bytes(int superblock) {
   return (size_t)(3 * kMicro * u_stride(superblock)   // rows of U of three micro-blocks
                   + 2 * 4 * kMicro * kRows            // parameters of two micro-blocks
                   + 2 * superblock                    // 1 / U[i,i], parameter column
+                  + 32                                // one parameter column for all of a micro-block?
                   + 2 * kMicro * ELD                  // errors of two micro-blocks
                   + superblock * WLD) * sizeof(float);   // W, column-major
 }
 
-__device__ __forceinline__ void cp_async16(float* dst, const float* src, int src_bytes) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(src_bytes) : "memory");
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void bulk_copy(float* dst, const float* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+__device__ __forceinline__ bool bar_ready(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred P1;\n\tmbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\tselp.b32 %0, 1, 0, P1;\n\t}"
+      : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+  return ok != 0;
 }
 __device__ __forceinline__ void fma2(uint64_t& d, uint64_t a, uint64_t b) {
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
@@ -117,39 +124,75 @@ __device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], 
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
-// What bounds it: the chain of columns, some 45 cycles each for the quantisation (product with 1 / s, clamp, round,
+// What bounds it: the chain of columns, some 60 cycles each for the quantisation (product with 1 / s, clamp, round,
 // dequantise, difference, product with the reciprocal pivot, correction of the next column).  So one warp of the CTA
-// does nothing but the chain: 16 columns at a time in registers, a lane per row.  The other seven apply a finished
-// micro-block's 16 errors to the columns two micro-blocks on and later as warp-level tensor-core products (a float32
-// FMA formulation spends its time on the broadcast loads of U: 480 cycles a column against the chain's own), write its
-// errors out as the operand of the trailing product, and fetch parameters and rows of U ahead.  The columns next in
-// line are corrected by the chain warp itself.  One barrier per micro-block.
-template <int SDT, bool GLOBAL, int KIND, bool ZP>
-__global__ void __launch_bounds__(kThreads) sweep_block_kernel(const __grid_constant__ Params p, int superblock) {
-  constexpr bool SB = Elem<SDT>::is_bf16 && !GLOBAL;
+// does nothing but the chain: 16 columns at a time in registers, a lane per row.  Others apply a finished micro-block's
+// 16 errors to the columns two micro-blocks on and later as warp-level tensor-core products (a float32 FMA formulation
+// spends its time on the broadcast loads of U: 480 cycles a column against the chain's own), taking tasks of 16 or 32
+// columns from a counter.  Duties beside that: warp 4, which shares the chain warp's scheduler and takes no tasks, asks
+// for rows of U by bulk copies (as per-thread copies they block the warps that issue them: all CTAs want the same rows at
+// the same time); warp 5 fetches parameters; warp 6 writes the errors out as the operand of the trailing product.  The
+// columns next in line are corrected by the chain warp itself.  One barrier per micro-block.
+template <int SBLK, bool SB, int KIND, bool ZP>
+__global__ void __launch_bounds__(kThreads, SBLK == 512 ? 1 : 2) sweep_block_kernel(const __grid_constant__ Params p) {
   const float qmin = p.qr.qmin, qmax = p.qr.qmax;
   extern __shared__ __align__(16) float sm[];
-  const int ULD = u_stride(superblock);
+  constexpr int ULD = u_stride(SBLK);
+  constexpr int XT = SBLK == 512 ? 4 : 2;              // column tiles of 8 per task (registers: one CTA per SM or two)
   float* sU = sm;                                      // [3][kMicro][ULD]
   float* sP = sU + 3 * kMicro * ULD;                   // [2][scale, low and high 1 / scale, zero point][kMicro][kRows]
-  float* sRd = sP + 2 * 4 * kMicro * kRows;            // [superblock]
-  int* sGrp = reinterpret_cast<int*>(sRd + superblock);// [superblock]
-  float* sE = sRd + 2 * superblock;                    // [2][kMicro][ELD]
-  float* sW = sE + 2 * kMicro * ELD;                   // [superblock][WLD]
+  float* sRd = sP + 2 * 4 * kMicro * kRows;            // [SBLK]
+  int* sGrp = reinterpret_cast<int*>(sRd + SBLK);      // [SBLK]
+  int* sSame = sGrp + SBLK;                            // [32]
+  float* sE = sRd + 2 * SBLK + 32;                     // [2][kMicro][ELD]
+  float* sW = sE + 2 * kMicro * ELD;                   // [SBLK][WLD]
   __shared__ int s_odd;                                // some scale is outside the range the low / high test covers
+  __shared__ int s_next[2];                            // next task of the helpers
+  __shared__ __align__(8) uint64_t s_bar[3];           // rows of U of a micro-block have arrived
   const int job = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int sb = p.sb, micros = (sb + kMicro - 1) / kMicro;
   float* __restrict__ W = p.W.at(job) + p.i1;
   const float* __restrict__ U = p.U.at(job);
   if (U) U += (int64_t)p.i1 * p.ldu + p.i1;
-  const void* scale = p.scale.at(job);
-  const void* zp = p.zp.at(job);
-  const int32_t* col_group = p.col_group.at(job);
-  const float g = GLOBAL ? *p.gscale.at(job) : 1.0f;
   const int64_t row0 = (int64_t)blockIdx.x * kRows, row = row0 + lane;
   const bool live = row < p.N;
-  const bool vecu = U && ((p.ldu & 3) == 0) && ((((uintptr_t)U) & 15) == 0);
+  const bool bulk = U && ((p.ldu & 3) == 0) && ((((uintptr_t)U) & 15) == 0) && (sb % kMicro) == 0;
   const bool vecw = ((p.ldw & 3) == 0) && ((((uintptr_t)W) & 15) == 0) && (sb & 3) == 0;
+  // rows of U of micro-block m, columns from its own first one on (columns beyond sb are zero).  Called by a whole
+  // warp; with bulk copies one lane does it.
+  auto fetch_u = [&](int m) {
+    float* dst = sU + (m % 3) * kMicro * ULD;
+    const int c0 = m * kMicro, c_end = micros * kMicro;
+    if (bulk) {
+      if (lane == 0) {
+        const uint32_t bytes = (uint32_t)(c_end - c0) * 4, bar = smem_u32(&s_bar[m % 3]);
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes * kMicro) : "memory");
+        for (int t = 0; t < kMicro; ++t)
+          bulk_copy(dst + t * ULD + c0, U + (int64_t)(c0 + t) * p.ldu + c0, bytes, bar);
+      }
+      return;
+    }
+    for (int t = 0; t < kMicro; ++t) {
+      const int i = c0 + t;
+      for (int c = c0 + lane; c < c_end; c += 32) {
+        float v = (i == c) ? 1.0f : 0.0f;
+        if (U) v = (i < sb && c < sb) ? U[(int64_t)i * p.ldu + c] : 0.0f;
+        dst[t * ULD + c] = v;
+      }
+    }
+  };
+  auto wait_u = [&](int m) {
+    if (!bulk) return;
+    const uint32_t bar = smem_u32(&s_bar[m % 3]), parity = (uint32_t)(m / 3) & 1u;
+    if (bar_ready(bar, parity)) return;
+    const long long t0 = clock64();
+    while (!bar_ready(bar, parity))
+      if (clock64() - t0 > 4000000000LL) { atomicCAS(p.status, 0, B200Q_ERR_DEVICE); break; }
+  };
+  // parameters of micro-block m's columns for the CTA's rows, by one warp (columns beyond sb: unit scale)
+  const void* scale = p.scale.at(job);
+  const void* zp = p.zp.at(job);
+  const float* gs = p.gscale.at(job);
   int64_t pbase;
   switch (p.strategy) {
     case B200Q_TENSOR: pbase = 0; break;
@@ -157,57 +200,48 @@ __global__ void __launch_bounds__(kThreads) sweep_block_kernel(const __grid_cons
     case B200Q_BLOCK: pbase = (row / p.block_h) * p.groups_per_row; break;
     default: pbase = row * p.groups_per_row; break;
   }
-  // rows of U of micro-block m, columns from its own first one on (columns beyond sb are zero)
-  auto fetch_u = [&](int m, int t0, int nt) {
-    float* dst = sU + (m % 3) * kMicro * ULD;
-    const int c0 = m * kMicro, quads = (micros * kMicro - c0) >> 2;
-    for (int idx = t0; idx < kMicro * quads; idx += nt) {
-      const int t = idx / quads, c = c0 + (idx - t * quads) * 4, i = c0 + t;
-      float* d = dst + t * ULD + c;
-      if (vecu) {
-        const int bytes = (i < sb && c < sb) ? (sb - c >= 4 ? 16 : (sb - c) * 4) : 0;
-        cp_async16(d, bytes ? U + (int64_t)i * p.ldu + c : U, bytes);
-      } else {
-        for (int k = 0; k < 4; ++k) {
-          float v = (i == c + k) ? 1.0f : 0.0f;
-          if (U) v = (i < sb && c + k < sb) ? U[(int64_t)i * p.ldu + c + k] : 0.0f;
-          d[k] = v;
-        }
-      }
-    }
-    cp_async_commit();
-  };
-  // parameters of micro-block m's columns for the CTA's rows (columns beyond sb: unit scale)
-  auto fetch_params = [&](int m, int w0, int nw) {
+  auto fetch_params = [&](int m) {
     float* dst = sP + (m & 1) * 4 * kMicro * kRows + lane;
-    float sv[3], zv[3];
+    const int c0 = m * kMicro;
+    const bool same = sSame[m] != 0;
+    float sv[kMicro], zv[kMicro];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      const int t = w0 + k * nw, c = m * kMicro + t;
-      sv[k] = 1.0f; zv[k] = 0.0f;
-      if (t < kMicro && c < sb && live) {
-        const int64_t pi = pbase + sGrp[c];
-        sv[k] = Elem<SDT>::load((const typename Elem<SDT>::type*)scale + pi);
-        if (ZP) zv[k] = load_zp(zp, p.zp_kind, pi);
+    for (int t = 0; t < kMicro; ++t) {   // all loads before their first use
+      sv[t] = 1.0f; zv[t] = 0.0f;
+      if ((t == 0 || !same) && c0 + t < sb && live) {
+        const int64_t pi = pbase + sGrp[c0 + t];
+        sv[t] = p.sdtype == B200Q_BF16 ? __bfloat162float(((const __nv_bfloat16*)scale)[pi]) : ((const float*)scale)[pi];
+        if (ZP) zv[t] = load_zp(zp, p.zp_kind, pi);
       }
     }
+    const float g = gs ? *gs : 1.0f;
+    float s = 1.0f, lo = 1.0f, hi = 1.0f, z = 0.0f;
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      const int t = w0 + k * nw;
-      if (t >= kMicro) continue;
-      float s = sv[k];
-      if (GLOBAL) s = __fdiv_rn(s, g);
-      const float rs = __frcp_rn(s);
-      if (!(s >= 0x1p-100f && s <= 0x1p100f)) s_odd = 1;
+    for (int t = 0; t < kMicro; ++t) {
+      if (t == 0 || !same) {
+        s = sv[t]; z = zv[t];
+        if (gs) s = __fdiv_rn(s, g);
+        const float rs = __frcp_rn(s);
+        if (!(s >= 0x1p-100f && s <= 0x1p100f)) s_odd = 1;
+        lo = rs * (1.0f - kMargin); hi = rs * (1.0f + kMargin);
+      }
       dst[t * kRows] = s;
-      dst[(kMicro + t) * kRows] = rs * (1.0f - kMargin);
-      dst[(2 * kMicro + t) * kRows] = rs * (1.0f + kMargin);
-      dst[(3 * kMicro + t) * kRows] = zv[k];
+      dst[(kMicro + t) * kRows] = lo;
+      dst[(2 * kMicro + t) * kRows] = hi;
+      if (ZP) dst[(3 * kMicro + t) * kRows] = z;
     }
   };
-  if (tid == 0) s_odd = 0;
-  fetch_u(0, tid, kThreads);
-  if (micros > 1) fetch_u(1, tid, kThreads); else cp_async_commit();
+  if (tid == 32) {
+    s_odd = 0; s_next[0] = s_next[1] = 0;
+    for (int k = 0; k < 3; ++k) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&s_bar[k])) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    __syncwarp();
+    fetch_u(0);
+    if (micros > 1) fetch_u(1);
+  }
+  const int32_t* col_group = p.col_group.at(job);
   for (int c = tid; c < micros * kMicro; c += kThreads) {
     float d = 1.0f;
     int grp = 0;
@@ -221,6 +255,7 @@ __global__ void __launch_bounds__(kThreads) sweep_block_kernel(const __grid_cons
   }
   // tile in: a lane per row, eight columns (a whole sector) at a time
   if (vecw) {
+#pragma unroll 4
     for (int c = warp * 8; c < micros * kMicro; c += 8 * (kThreads / 32)) {
       float4 v[2];
 #pragma unroll
@@ -241,11 +276,37 @@ __global__ void __launch_bounds__(kThreads) sweep_block_kernel(const __grid_cons
     }
   }
   __syncthreads();
-  fetch_params(0, warp, kThreads / 32);
-  cp_async_wait<1>();
+  if (tid < micros) {
+    bool same = true;
+    for (int t = 1; t < kMicro; ++t) same = same && (tid * kMicro + t >= sb || sGrp[tid * kMicro + t] == sGrp[tid * kMicro]);
+    sSame[tid] = same ? 1 : 0;
+  }
+  __syncthreads();
+  if (warp == 5) fetch_params(0);
+  wait_u(0);
   __syncthreads();
 
-  float loss = 0.0f;
+  float loss = 0.0f;   // of warp 6's rows, a lane each
+  // the errors of micro-block `of`: their squares into the loss, and out as operand rows
+  auto finish_errors = [&](int of) {
+    const float* ei = sE + (of & 1) * kMicro * ELD + lane;
+    float x[kMicro];
+#pragma unroll
+    for (int t = 0; t < kMicro; ++t) { x[t] = ei[t * ELD]; loss = fmaf(x[t], x[t], loss); }
+    if (!p.err_hi || !live) return;
+    const int64_t at = job * p.err_batch + row * p.lde + of * kMicro;
+#pragma unroll
+    for (int q = 0; q < kMicro; q += 4) {
+      float h[4], l[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        h[k] = tgemm::tf32_rn(x[q + k]);
+        l[k] = tgemm::tf32_rn(x[q + k] - h[k]);
+      }
+      *reinterpret_cast<float4*>(p.err_hi + at + q) = make_float4(h[0], h[1], h[2], h[3]);
+      *reinterpret_cast<float4*>(p.err_lo + at + q) = make_float4(l[0], l[1], l[2], l[3]);
+    }
+  };
   float e[kMicro];
 #pragma unroll
   for (int t = 0; t < kMicro; ++t) e[t] = 0.0f;
@@ -276,9 +337,6 @@ __global__ void __launch_bounds__(kThreads) sweep_block_kernel(const __grid_cons
 #pragma unroll
         for (int k = 0; k < kMicro / 2; ++k) unpair(v[k], w[2 * k], w[2 * k + 1]);
       }
-      // kept for the exact pass, should it be needed
-#pragma unroll
-      for (int t = 0; t < kMicro; ++t) sW[(c0 + t) * WLD + lane] = w[t];
       const float* par = sP + (m & 1) * 4 * kMicro * kRows + lane;
       bool differ = false;
 #pragma unroll
@@ -305,7 +363,14 @@ __global__ void __launch_bounds__(kThreads) sweep_block_kernel(const __grid_cons
       }
       float* eo = sE + (m & 1) * kMicro * ELD + lane;
       if (__any_sync(0xffffffffu, differ) || s_odd) {
-        // by the exact rules, column by column in shared memory
+        // by the exact rules, column by column in shared memory, where the tile still is as the micro-block found it
+        const float* e_prev = sE + ((m + 1) & 1) * kMicro * ELD + lane;
+#pragma unroll 1
+        for (int k = 0; k < kMicro && m > 0; ++k) {
+          float v = sW[(c0 + k) * WLD + lane];
+          for (int t = 0; t < kMicro; ++t) v = fmaf(-e_prev[t * ELD], u_prev[t * ULD + c0 + k], v);
+          sW[(c0 + k) * WLD + lane] = v;
+        }
 #pragma unroll 1
         for (int t = 0; t < kMicro; ++t) {
           float* wt = sW + (c0 + t) * WLD + lane;
@@ -325,11 +390,14 @@ __global__ void __launch_bounds__(kThreads) sweep_block_kernel(const __grid_cons
 #pragma unroll
         for (int t = 0; t < kMicro; ++t) { sW[(c0 + t) * WLD + lane] = w[t]; eo[t * ELD] = e[t]; }
       }
-#pragma unroll
-      for (int t = 0; t < kMicro; ++t) loss = fmaf(e[t], e[t], loss);
+    } else if (warp == 4) {
+      if (m > 0 && m + 1 < micros) fetch_u(m + 1);   // into the buffer of micro-block m - 2
+      if (lane == 0) s_next[(m + 1) & 1] = 0;        // (nobody takes from it before the barrier)
     } else {
+      if (warp == 5 && m + 1 < micros) fetch_params(m + 1);
+      if (warp == 6 && m > 0) finish_errors(m - 1);
       if (m > 0 && m + 1 < micros) {
-        // W[32 rows, 16 columns at a time] -= E[32, 16] U[16, columns]
+        // W[32 rows, columns of a task] -= E[32, 16] U[16, columns]
         const float* ei = sE + ((m - 1) & 1) * kMicro * ELD + (lane & 3) * ELD + (lane >> 2);
         uint32_t ah[2][2][4], al[2][2][4];   // [row tile][k step]
 #pragma unroll
@@ -340,72 +408,63 @@ __global__ void __launch_bounds__(kThreads) sweep_block_kernel(const __grid_cons
             for (int k = 0; k < 4; ++k)
               split_tf32(ei[(ks * 8 + (k >> 1) * 4) * ELD + y * 16 + (k & 1) * 8], ah[y][ks][k], al[y][ks][k]);
 #pragma unroll 1
-        for (int mc = m + warp; mc < micros; mc += 7) {
-          const int c = mc * kMicro;
+        while (true) {
+          int task = 0;
+          if (lane == 0) task = atomicAdd(&s_next[m & 1], 1);
+          const int c = (m + 1) * kMicro + __shfl_sync(0xffffffffu, task, 0) * (XT * 8);
+          if (c >= micros * kMicro) break;
+          const bool whole = XT == 2 || c + XT * 8 <= micros * kMicro;   // else only the first 16 columns exist
           float* o = sW + (c + 2 * (lane & 3)) * WLD + (lane >> 2);
           const float* ub = u_prev + (lane & 3) * ULD + c + (lane >> 2);
-          float old[2][2][4], acc[2][2][4] = {}, part[2][2][4] = {};   // [row tile][column tile]
+          float old[2][XT][4], acc[2][XT][4] = {}, part[2][XT][4] = {};   // [row tile][column tile]
 #pragma unroll
-          for (int y = 0; y < 2; ++y)
+          for (int x = 0; x < XT; ++x)
+            if (x < 2 || whole) {
 #pragma unroll
-            for (int x = 0; x < 2; ++x)
+              for (int y = 0; y < 2; ++y)
 #pragma unroll
-              for (int k = 0; k < 4; ++k) old[y][x][k] = o[(x * 8 + (k & 1)) * WLD + y * 16 + (k >> 1) * 8];
+                for (int k = 0; k < 4; ++k) old[y][x][k] = o[(x * 8 + (k & 1)) * WLD + y * 16 + (k >> 1) * 8];
+            }
 #pragma unroll
           for (int ks = 0; ks < 2; ++ks) {
-            uint32_t bh[2][2], bl[2][2];
+            uint32_t bh[XT][2], bl[XT][2];
 #pragma unroll
-            for (int x = 0; x < 2; ++x)
+            for (int x = 0; x < XT; ++x)
 #pragma unroll
-              for (int k = 0; k < 2; ++k) split_tf32(ub[(ks * 8 + k * 4) * ULD + x * 8], bh[x][k], bl[x][k]);
-#pragma unroll
-            for (int y = 0; y < 2; ++y)
-#pragma unroll
-              for (int x = 0; x < 2; ++x) mma_tf32(acc[y][x], ah[y][ks], bh[x]);
+              for (int k = 0; k < 2; ++k)
+                split_tf32((x < 2 || whole) ? ub[(ks * 8 + k * 4) * ULD + x * 8] : 0.0f, bh[x][k], bl[x][k]);
 #pragma unroll
             for (int y = 0; y < 2; ++y)
 #pragma unroll
-              for (int x = 0; x < 2; ++x) mma_tf32(part[y][x], ah[y][ks], bl[x]);
+              for (int x = 0; x < XT; ++x) mma_tf32(acc[y][x], ah[y][ks], bh[x]);
 #pragma unroll
             for (int y = 0; y < 2; ++y)
 #pragma unroll
-              for (int x = 0; x < 2; ++x) mma_tf32(part[y][x], al[y][ks], bh[x]);
+              for (int x = 0; x < XT; ++x) mma_tf32(part[y][x], ah[y][ks], bl[x]);
+#pragma unroll
+            for (int y = 0; y < 2; ++y)
+#pragma unroll
+              for (int x = 0; x < XT; ++x) mma_tf32(part[y][x], al[y][ks], bh[x]);
           }
 #pragma unroll
-          for (int y = 0; y < 2; ++y)
+          for (int x = 0; x < XT; ++x)
+            if (x < 2 || whole) {
 #pragma unroll
-            for (int x = 0; x < 2; ++x)
+              for (int y = 0; y < 2; ++y)
 #pragma unroll
-              for (int k = 0; k < 4; ++k)
-                o[(x * 8 + (k & 1)) * WLD + y * 16 + (k >> 1) * 8] = old[y][x][k] - (acc[y][x][k] + part[y][x][k]);
+                for (int k = 0; k < 4; ++k)
+                  o[(x * 8 + (k & 1)) * WLD + y * 16 + (k >> 1) * 8] = old[y][x][k] - (acc[y][x][k] + part[y][x][k]);
+            }
         }
       }
-      if (m + 1 < micros) fetch_params(m + 1, warp - 1, 7);
     }
-    // the errors of micro-block `of`, four columns of a row per thread
-    auto store_errors = [&](int of, int t) {
-      const int r = t & 31, q = (t >> 5) * 4;
-      if (t >= 128 || row0 + r >= p.N) return;
-      const float* ei = sE + (of & 1) * kMicro * ELD + r;
-      float h[4], l[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const float x = ei[(q + k) * ELD];
-        h[k] = tgemm::tf32_rn(x);
-        l[k] = tgemm::tf32_rn(x - h[k]);
-      }
-      const int64_t at = job * p.err_batch + (row0 + r) * p.lde + of * kMicro + q;
-      *reinterpret_cast<float4*>(p.err_hi + at) = make_float4(h[0], h[1], h[2], h[3]);
-      *reinterpret_cast<float4*>(p.err_lo + at) = make_float4(l[0], l[1], l[2], l[3]);
-    };
-    if (p.err_hi && m > 0 && warp > 0) store_errors(m - 1, tid - 32);
-    cp_async_wait<0>();
+    if (m + 1 < micros) wait_u(m + 1);
     __syncthreads();
-    if (m + 2 < micros && warp > 0) fetch_u(m + 2, tid - 32, kThreads - 32);   // the buffer of micro-block m - 1 is free
-    if (m + 1 == micros && p.err_hi) store_errors(m, tid);   // (a superblock with columns after it is a whole one)
   }
+  if (warp == 6) finish_errors(micros - 1);   // (a superblock with columns after it is a whole one)
   // tile out
   if (vecw) {
+#pragma unroll 2
     for (int c = warp * 8; c < sb; c += 8 * (kThreads / 32)) {
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
@@ -421,7 +480,7 @@ __global__ void __launch_bounds__(kThreads) sweep_block_kernel(const __grid_cons
       for (int c = lane; c < sb; c += 32) dst[c] = sW[c * WLD + r];
     }
   }
-  if (warp == 0 && live) {
+  if (warp == 6 && live) {
     float* lo = p.losses.at(job);
     const float half = loss * 0.5f;
     lo[row] = p.i1 == 0 ? half : lo[row] + half;
@@ -464,22 +523,23 @@ static int sweep(Params p, int sdtype, bool global, int batch, const float* cons
   float* err = (float*)((char*)workspace + kSweepHeaderBytes);   // [sets][hi, lo]
   float* ub = err + 2 * l.sets * l.err;                          // [sets][hi, lo]
   B200Q_TRY(cudaMemsetAsync(status, 0, sizeof(int), st));
-  const bool with_zp = p.zp.one || p.zp.table;
-  void (*kern)(const Params, int) = nullptr;
-#define B200Q_SWEEP_KIND(SDT, G, K) kern = with_zp ? sweep_block_kernel<SDT, G, K, true> : sweep_block_kernel<SDT, G, K, false>
-#define B200Q_SWEEP_PICK(SDT)                                                                                            \
-  do {                                                                                                                   \
-    if (p.qr.kind == kInt) { if (global) B200Q_SWEEP_KIND(SDT, true, kInt); else B200Q_SWEEP_KIND(SDT, false, kInt); }       \
-    else if (p.qr.kind == kFp8) { if (global) B200Q_SWEEP_KIND(SDT, true, kFp8); else B200Q_SWEEP_KIND(SDT, false, kFp8); } \
-    else { if (global) B200Q_SWEEP_KIND(SDT, true, kFp4); else B200Q_SWEEP_KIND(SDT, false, kFp4); }                       \
+  if (sdtype != B200Q_BF16 && sdtype != B200Q_F32) return B200Q_ERR_UNSUPPORTED;
+  p.sdtype = sdtype; p.status = status;
+  const bool with_zp = p.zp.one || p.zp.table, bf16_values = sdtype == B200Q_BF16 && !global;
+  void (*kern)(const Params) = nullptr;
+#define B200Q_SWEEP_ZP(S, B, K) kern = with_zp ? sweep_block_kernel<S, B, K, true> : sweep_block_kernel<S, B, K, false>
+#define B200Q_SWEEP_SB(S, K) do { if (bf16_values) B200Q_SWEEP_ZP(S, true, K); else B200Q_SWEEP_ZP(S, false, K); } while (0)
+#define B200Q_SWEEP_PICK(S)                            \
+  do {                                                 \
+    if (p.qr.kind == kInt) B200Q_SWEEP_SB(S, kInt);      \
+    else if (p.qr.kind == kFp8) B200Q_SWEEP_SB(S, kFp8); \
+    else B200Q_SWEEP_SB(S, kFp4);                        \
   } while (0)
-  if (sdtype == B200Q_BF16) B200Q_SWEEP_PICK(B200Q_BF16);
-  else if (sdtype == B200Q_F32) B200Q_SWEEP_PICK(B200Q_F32);
-  else return B200Q_ERR_UNSUPPORTED;
+  if (l.sb == 512) B200Q_SWEEP_PICK(512); else B200Q_SWEEP_PICK(256);
 #undef B200Q_SWEEP_PICK
-#undef B200Q_SWEEP_KIND
-  // always the largest size: host threads on other streams launch the same kernel with other widths
-  B200Q_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(512)));
+#undef B200Q_SWEEP_SB
+#undef B200Q_SWEEP_ZP
+  B200Q_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(l.sb)));
   const int ctas = (int)((N + kRows - 1) / kRows);
   tgemm::SideStream* side = l.sets == 2 && has_u && K > 2 * l.sb ? tgemm::side_stream(st) : nullptr;
   bool side_busy = false;
@@ -502,7 +562,7 @@ static int sweep(Params p, int sdtype, bool global, int batch, const float* cons
     p.err_hi = trailing ? err + (int64_t)which * 2 * l.err : nullptr;
     p.err_lo = trailing ? p.err_hi + l.err : nullptr;
     p.lde = l.sb; p.err_batch = l.rows_n * l.sb;
-    kern<<<dim3(ctas, batch), kThreads, smem_bytes(l.sb), st>>>(p, l.sb);
+    kern<<<dim3(ctas, batch), kThreads, smem_bytes(l.sb), st>>>(p);
     B200Q_LAUNCH_CHECK();
     if (!trailing) continue;
     // W[:, i2:] -= Err[N, w] * U[i1:i2, i2:]
