@@ -21,7 +21,8 @@ constexpr int kMaxBlock = 128;               // largest block size callers may a
 constexpr size_t kSweepHeaderBytes = 256;    // status word at the start of the workspace
 constexpr int kRows = 32;                    // rows of a CTA: a lane each
 constexpr int kMicro = 16;                   // columns a lane keeps in registers at a time
-constexpr int kThreads = 256;
+// 12 warps where a CTA has its SM to itself, 8 where two share one
+constexpr int warps_of(int superblock) { return superblock == 512 ? 12 : 8; }
 constexpr int WLD = kRows + 4, ELD = kRows + 8;   // columns of W and of the errors in shared memory: the strides
                                                   // make the MMA fragments' accesses conflict-free
 __host__ __device__ constexpr int u_stride(int superblock) { return superblock + 8; }   // likewise
@@ -129,16 +130,20 @@ __device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], 
 // does nothing but the chain: 16 columns at a time in registers, a lane per row.  Others apply a finished micro-block's
 // 16 errors to the columns two micro-blocks on and later as warp-level tensor-core products (a float32 FMA formulation
 // spends its time on the broadcast loads of U: 480 cycles a column against the chain's own), taking tasks of 16 or 32
-// columns from a counter.  Duties beside that: warp 4, which shares the chain warp's scheduler and takes no tasks, asks
-// for rows of U by bulk copies (as per-thread copies they block the warps that issue them: all CTAs want the same rows at
-// the same time); warp 5 fetches parameters; warp 6 writes the errors out as the operand of the trailing product.  The
-// columns next in line are corrected by the chain warp itself.  One barrier per micro-block.
+// columns from a counter.  Duties beside that: the warps that share the chain warp's scheduler take no tasks, they fetch
+// parameters and ask for rows of U by bulk copies (as per-thread copies they block the warps that issue them: all CTAs
+// want the same rows at the same time); warp 6 writes the errors out as the operand of the trailing product.  The columns
+// next in line are corrected by the chain warp itself.  One barrier per micro-block.  Every role is a latency-bound
+// stream of instructions, a quarter of its stalls instruction fetch, hence short loops rather than unrolled code off
+// the chain.
 template <int SBLK, bool SB, int KIND, bool ZP>
-__global__ void __launch_bounds__(kThreads, SBLK == 512 ? 1 : 2) sweep_block_kernel(const __grid_constant__ Params p) {
+__global__ void __launch_bounds__(32 * warps_of(SBLK), SBLK == 512 ? 1 : 2) sweep_block_kernel(const __grid_constant__ Params p) {
   const float qmin = p.qr.qmin, qmax = p.qr.qmax;
   extern __shared__ __align__(16) float sm[];
   constexpr int ULD = u_stride(SBLK);
-  constexpr int XT = SBLK == 512 ? 4 : 2;              // column tiles of 8 per task (registers: one CTA per SM or two)
+  constexpr int NW = warps_of(SBLK), NT = 32 * NW;
+  constexpr int kFetchWarp = NW > 8 ? 8 : 4, kParamWarp = NW > 8 ? 4 : 5;
+  constexpr int XT = 2;                                // column tiles of 8 per task
   float* sU = sm;                                      // [3][kMicro][ULD]
   float* sP = sU + 3 * kMicro * ULD;                   // [2][scale, low and high 1 / scale, zero point][kMicro][kRows]
   float* sRd = sP + 2 * 4 * kMicro * kRows;            // [SBLK]
@@ -204,31 +209,47 @@ __global__ void __launch_bounds__(kThreads, SBLK == 512 ? 1 : 2) sweep_block_ker
     float* dst = sP + (m & 1) * 4 * kMicro * kRows + lane;
     const int c0 = m * kMicro;
     const bool same = sSame[m] != 0;
-    float sv[kMicro], zv[kMicro];
-#pragma unroll
-    for (int t = 0; t < kMicro; ++t) {   // all loads before their first use
-      sv[t] = 1.0f; zv[t] = 0.0f;
-      if ((t == 0 || !same) && c0 + t < sb && live) {
-        const int64_t pi = pbase + sGrp[c0 + t];
-        sv[t] = p.sdtype == B200Q_BF16 ? __bfloat162float(((const __nv_bfloat16*)scale)[pi]) : ((const float*)scale)[pi];
-        if (ZP) zv[t] = load_zp(zp, p.zp_kind, pi);
-      }
-    }
     const float g = gs ? *gs : 1.0f;
-    float s = 1.0f, lo = 1.0f, hi = 1.0f, z = 0.0f;
-#pragma unroll
-    for (int t = 0; t < kMicro; ++t) {
-      if (t == 0 || !same) {
-        s = sv[t]; z = zv[t];
-        if (gs) s = __fdiv_rn(s, g);
-        const float rs = __frcp_rn(s);
-        if (!(s >= 0x1p-100f && s <= 0x1p100f)) s_odd = 1;
-        lo = rs * (1.0f - kMargin); hi = rs * (1.0f + kMargin);
-      }
+    auto put = [&](int t, float s) {
+      if (gs) s = __fdiv_rn(s, g);
+      const float rs = __frcp_rn(s);
+      if (!(s >= 0x1p-100f && s <= 0x1p100f)) s_odd = 1;
       dst[t * kRows] = s;
-      dst[(kMicro + t) * kRows] = lo;
-      dst[(2 * kMicro + t) * kRows] = hi;
-      if (ZP) dst[(3 * kMicro + t) * kRows] = z;
+      dst[(kMicro + t) * kRows] = rs * (1.0f - kMargin);
+      dst[(2 * kMicro + t) * kRows] = rs * (1.0f + kMargin);
+    };
+    auto load = [&](int t, float& s, float& z) {
+      s = 1.0f; z = 0.0f;
+      if (c0 + t < sb && live) {
+        const int64_t pi = pbase + sGrp[c0 + t];
+        s = p.sdtype == B200Q_BF16 ? __bfloat162float(((const __nv_bfloat16*)scale)[pi]) : ((const float*)scale)[pi];
+        if (ZP) z = load_zp(zp, p.zp_kind, pi);
+      }
+    };
+    if (same) {
+      float s, z;
+      load(0, s, z);
+      put(0, s);
+      s = dst[0];
+      const float lo = dst[kMicro * kRows], hi = dst[2 * kMicro * kRows];
+#pragma unroll
+      for (int t = 0; t < kMicro; ++t) {
+        dst[t * kRows] = s;
+        dst[(kMicro + t) * kRows] = lo;
+        dst[(2 * kMicro + t) * kRows] = hi;
+        if (ZP) dst[(3 * kMicro + t) * kRows] = z;
+      }
+    } else {
+      float s[kMicro], z[kMicro];
+#pragma unroll
+      for (int t = 0; t < kMicro; ++t) load(t, s[t], z[t]);   // all of them on their way before the first is used
+#pragma unroll
+      for (int t = 0; t < kMicro; ++t) {
+        dst[t * kRows] = s[t];
+        if (ZP) dst[(3 * kMicro + t) * kRows] = z[t];
+      }
+#pragma unroll 1
+      for (int t = 0; t < kMicro; ++t) put(t, dst[t * kRows]);
     }
   };
   if (tid == 32) {
@@ -242,7 +263,7 @@ __global__ void __launch_bounds__(kThreads, SBLK == 512 ? 1 : 2) sweep_block_ker
     if (micros > 1) fetch_u(1);
   }
   const int32_t* col_group = p.col_group.at(job);
-  for (int c = tid; c < micros * kMicro; c += kThreads) {
+  for (int c = tid; c < micros * kMicro; c += NT) {
     float d = 1.0f;
     int grp = 0;
     if (c < sb) {
@@ -256,7 +277,7 @@ __global__ void __launch_bounds__(kThreads, SBLK == 512 ? 1 : 2) sweep_block_ker
   // tile in: a lane per row, eight columns (a whole sector) at a time
   if (vecw) {
 #pragma unroll 4
-    for (int c = warp * 8; c < micros * kMicro; c += 8 * (kThreads / 32)) {
+    for (int c = warp * 8; c < micros * kMicro; c += 8 * (NW)) {
       float4 v[2];
 #pragma unroll
       for (int h = 0; h < 2; ++h)
@@ -269,7 +290,7 @@ __global__ void __launch_bounds__(kThreads, SBLK == 512 ? 1 : 2) sweep_block_ker
       }
     }
   } else {
-    for (int r = warp * 4; r < warp * 4 + 4; ++r) {
+    for (int r = warp; r < kRows; r += NW) {
       const bool in = row0 + r < p.N;
       const float* src = W + (row0 + r) * p.ldw;
       for (int c = lane; c < micros * kMicro; c += 32) sW[c * WLD + r] = (in && c < sb) ? src[c] : 0.0f;
@@ -282,7 +303,7 @@ __global__ void __launch_bounds__(kThreads, SBLK == 512 ? 1 : 2) sweep_block_ker
     sSame[tid] = same ? 1 : 0;
   }
   __syncthreads();
-  if (warp == 5) fetch_params(0);
+  if (warp == kParamWarp) fetch_params(0);
   wait_u(0);
   __syncthreads();
 
@@ -390,11 +411,15 @@ __global__ void __launch_bounds__(kThreads, SBLK == 512 ? 1 : 2) sweep_block_ker
 #pragma unroll
         for (int t = 0; t < kMicro; ++t) { sW[(c0 + t) * WLD + lane] = w[t]; eo[t * ELD] = e[t]; }
       }
-    } else if (warp == 4) {
-      if (m > 0 && m + 1 < micros) fetch_u(m + 1);   // into the buffer of micro-block m - 2
-      if (lane == 0) s_next[(m + 1) & 1] = 0;        // (nobody takes from it before the barrier)
+    } else if ((warp & 3) == 0) {
+      if (warp == kFetchWarp) {
+        if (m > 0 && m + 1 < micros) fetch_u(m + 1);   // into the buffer of micro-block m - 2
+        if (lane == 0) s_next[(m + 1) & 1] = 0;        // (nobody takes from it before the barrier)
+      } else if (m + 1 < micros) {
+        fetch_params(m + 1);
+      }
     } else {
-      if (warp == 5 && m + 1 < micros) fetch_params(m + 1);
+      if (kParamWarp == 5 && warp == 5 && m + 1 < micros) fetch_params(m + 1);
       if (warp == 6 && m > 0) finish_errors(m - 1);
       if (m > 0 && m + 1 < micros) {
         // W[32 rows, columns of a task] -= E[32, 16] U[16, columns]
@@ -465,7 +490,7 @@ __global__ void __launch_bounds__(kThreads, SBLK == 512 ? 1 : 2) sweep_block_ker
   // tile out
   if (vecw) {
 #pragma unroll 2
-    for (int c = warp * 8; c < sb; c += 8 * (kThreads / 32)) {
+    for (int c = warp * 8; c < sb; c += 8 * (NW)) {
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const float* d = sW + (c + 4 * h) * WLD + lane;
@@ -474,7 +499,7 @@ __global__ void __launch_bounds__(kThreads, SBLK == 512 ? 1 : 2) sweep_block_ker
       }
     }
   } else {
-    for (int r = warp * 4; r < warp * 4 + 4; ++r) {
+    for (int r = warp; r < kRows; r += NW) {
       if (row0 + r >= p.N) break;
       float* dst = W + (row0 + r) * p.ldw;
       for (int c = lane; c < sb; c += 32) dst[c] = sW[c * WLD + r];
@@ -562,7 +587,7 @@ static int sweep(Params p, int sdtype, bool global, int batch, const float* cons
     p.err_hi = trailing ? err + (int64_t)which * 2 * l.err : nullptr;
     p.err_lo = trailing ? p.err_hi + l.err : nullptr;
     p.lde = l.sb; p.err_batch = l.rows_n * l.sb;
-    kern<<<dim3(ctas, batch), kThreads, smem_bytes(l.sb), st>>>(p);
+    kern<<<dim3(ctas, batch), 32 * warps_of(l.sb), smem_bytes(l.sb), st>>>(p);
     B200Q_LAUNCH_CHECK();
     if (!trailing) continue;
     // W[:, i2:] -= Err[N, w] * U[i1:i2, i2:]
