@@ -10,6 +10,7 @@
 // Each correction is one fused multiply-add (the reference rounds the product first), true divisions decide a code
 // wherever an ulp could matter.
 #include <cstdlib>
+#include <type_traits>
 
 #include "common.cuh"
 #include "tgemm_tf32.cuh"
@@ -125,17 +126,74 @@ __device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], 
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
+// A micro-block's errors as MMA operand: rows of the CTA x columns of the micro-block, [row tile][k step]
+struct ErrFrag { uint32_t hi[2][2][4], lo[2][2][4]; };
+// `upto12`: only the first twelve columns exist yet
+__device__ __forceinline__ void load_errors(const float* e, int lane, bool upto12, ErrFrag& f) {
+  const float* ei = e + (lane & 3) * ELD + (lane >> 2);
+#pragma unroll
+  for (int y = 0; y < 2; ++y)
+#pragma unroll
+    for (int ks = 0; ks < 2; ++ks)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const bool out = upto12 && ks == 1 && k >= 2;
+        split_tf32(out ? 0.0f : ei[(ks * 8 + (k >> 1) * 4) * ELD + y * 16 + (k & 1) * 8], f.hi[y][ks][k], f.lo[y][ks][k]);
+      }
+}
+// W[32 rows, 16 columns] -= E[32, 16] U[16, 16 columns]; `w`, `u`: the first of the columns
+template <int ULD>
+__device__ __forceinline__ void apply_errors(const ErrFrag& f, const float* u, float* w, int lane) {
+  float* o = w + 2 * (lane & 3) * WLD + (lane >> 2);
+  const float* ub = u + (lane & 3) * ULD + (lane >> 2);
+  float old[2][2][4], acc[2][2][4] = {}, part[2][2][4] = {};   // [row tile][column tile]
+#pragma unroll
+  for (int y = 0; y < 2; ++y)
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) old[y][x][k] = o[(x * 8 + (k & 1)) * WLD + y * 16 + (k >> 1) * 8];
+#pragma unroll
+  for (int ks = 0; ks < 2; ++ks) {
+    uint32_t bh[2][2], bl[2][2];
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+#pragma unroll
+      for (int k = 0; k < 2; ++k) split_tf32(ub[(ks * 8 + k * 4) * ULD + x * 8], bh[x][k], bl[x][k]);
+#pragma unroll
+    for (int y = 0; y < 2; ++y)
+#pragma unroll
+      for (int x = 0; x < 2; ++x) mma_tf32(acc[y][x], f.hi[y][ks], bh[x]);
+#pragma unroll
+    for (int y = 0; y < 2; ++y)
+#pragma unroll
+      for (int x = 0; x < 2; ++x) mma_tf32(part[y][x], f.hi[y][ks], bl[x]);
+#pragma unroll
+    for (int y = 0; y < 2; ++y)
+#pragma unroll
+      for (int x = 0; x < 2; ++x) mma_tf32(part[y][x], f.lo[y][ks], bh[x]);
+  }
+#pragma unroll
+  for (int y = 0; y < 2; ++y)
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        o[(x * 8 + (k & 1)) * WLD + y * 16 + (k >> 1) * 8] = old[y][x][k] - (acc[y][x][k] + part[y][x][k]);
+}
+
 // What bounds it: the chain of columns, some 60 cycles each for the quantisation (product with 1 / s, clamp, round,
 // dequantise, difference, product with the reciprocal pivot, correction of the next column).  So one warp of the CTA
 // does nothing but the chain: 16 columns at a time in registers, a lane per row.  Others apply a finished micro-block's
 // 16 errors to the columns two micro-blocks on and later as warp-level tensor-core products (a float32 FMA formulation
-// spends its time on the broadcast loads of U: 480 cycles a column against the chain's own), taking tasks of 16 or 32
-// columns from a counter.  Duties beside that: the warps that share the chain warp's scheduler take no tasks, they fetch
-// parameters and ask for rows of U by bulk copies (as per-thread copies they block the warps that issue them: all CTAs
-// want the same rows at the same time); warp 6 writes the errors out as the operand of the trailing product.  The columns
-// next in line are corrected by the chain warp itself.  One barrier per micro-block.  Every role is a latency-bound
-// stream of instructions, a quarter of its stalls instruction fetch, hence short loops rather than unrolled code off
-// the chain.
+// spends its time on the broadcast loads of U: 480 cycles a column against the chain's own), taking tasks of 16 columns
+// from a counter.  The columns next in line take the first twelve errors from a warp that waits for them while the chain
+// is on the last four, and those four from the chain warp.  Duties beside that: the warps that share the chain warp's
+// scheduler fetch parameters and ask for rows of U by bulk copies (as per-thread copies they block the warps that issue
+// them: all CTAs want the same rows at the same time), and take tasks only while these, not the chain, decide; warp 6
+// writes the errors out as the operand of the trailing product.  One barrier per micro-block.  Every role is a
+// latency-bound stream of instructions, a quarter of its stalls instruction fetch, hence short loops rather than
+// unrolled code off the chain.
 template <int SBLK, bool SB, int KIND, bool ZP>
 __global__ void __launch_bounds__(32 * warps_of(SBLK), SBLK == 512 ? 1 : 2) sweep_block_kernel(const __grid_constant__ Params p) {
   const float qmin = p.qr.qmin, qmax = p.qr.qmax;
@@ -143,7 +201,8 @@ __global__ void __launch_bounds__(32 * warps_of(SBLK), SBLK == 512 ? 1 : 2) swee
   constexpr int ULD = u_stride(SBLK);
   constexpr int NW = warps_of(SBLK), NT = 32 * NW;
   constexpr int kFetchWarp = NW > 8 ? 8 : 4, kParamWarp = NW > 8 ? 4 : 5;
-  constexpr int XT = 2;                                // column tiles of 8 per task
+  constexpr int kNextWarp = NW > 8 ? 9 : 1;            // brings the next micro-block's columns up to date
+  constexpr int kHead = 12;                            // its share of a micro-block's errors
   float* sU = sm;                                      // [3][kMicro][ULD]
   float* sP = sU + 3 * kMicro * ULD;                   // [2][scale, low and high 1 / scale, zero point][kMicro][kRows]
   float* sRd = sP + 2 * 4 * kMicro * kRows;            // [SBLK]
@@ -335,17 +394,20 @@ __global__ void __launch_bounds__(32 * warps_of(SBLK), SBLK == 512 ? 1 : 2) swee
   for (int m = 0; m < micros; ++m) {
     const int c0 = m * kMicro;
     const float* u_prev = sU + ((m + 2) % 3) * kMicro * ULD;
+    const float* u = sU + (m % 3) * kMicro * ULD + c0;
     if (warp == 0) {
-      const float* u = sU + (m % 3) * kMicro * ULD + c0;
+      float* wcol = sW + c0 * WLD + lane;
+      float* eo = sE + (m & 1) * kMicro * ELD + lane;
+      const float* par = sP + (m & 1) * 4 * kMicro * kRows + lane;
       float w[kMicro];
       {
-        // the errors of the micro-block before this one
+        // the last errors of the micro-block before this one
         uint64_t v[kMicro / 2];
 #pragma unroll
-        for (int k = 0; k < kMicro / 2; ++k) v[k] = pair(sW[(c0 + 2 * k) * WLD + lane], sW[(c0 + 2 * k + 1) * WLD + lane]);
+        for (int k = 0; k < kMicro / 2; ++k) v[k] = pair(wcol[2 * k * WLD], wcol[(2 * k + 1) * WLD]);
         if (m > 0) {
 #pragma unroll
-          for (int t = 0; t < kMicro; ++t) {
+          for (int t = kHead; t < kMicro; ++t) {
             const uint64_t ne = pair(-e[t], -e[t]);
 #pragma unroll
             for (int k = 0; k < kMicro / 4; ++k) {
@@ -358,130 +420,102 @@ __global__ void __launch_bounds__(32 * warps_of(SBLK), SBLK == 512 ? 1 : 2) swee
 #pragma unroll
         for (int k = 0; k < kMicro / 2; ++k) unpair(v[k], w[2 * k], w[2 * k + 1]);
       }
-      const float* par = sP + (m & 1) * 4 * kMicro * kRows + lane;
-      bool differ = false;
+      // columns [begin, end) in registers; true if the test of some code failed
+      auto chain = [&](auto begin, auto end) -> bool {
+        bool differ = false;
 #pragma unroll
-      for (int t = 0; t < kMicro; ++t) {
-        const float s = par[t * kRows], rlo = par[(kMicro + t) * kRows], rhi = par[(2 * kMicro + t) * kRows];
-        const float z = ZP ? par[(3 * kMicro + t) * kRows] : 0.0f, mz = ZP ? fabsf(z) * (0.5f * kMargin) : 0.0f;
-        const float wi = w[t], lo = fmaf(wi, rlo, z - mz);
-        const float qc = code_of<KIND>(lo, qmin, qmax);
-        differ |= qc != code_of<KIND>(fmaf(wi, rhi, z + mz), qmin, qmax);
-        const float q = dequant<KIND, SB, ZP>(qc, s, z);
-        // loss and error use the reciprocal of the pivot (an ulp from the reference's divisions)
-        const float tt = __fmul_rn(__fsub_rn(wi, q), sRd[c0 + t]);
-        e[t] = tt;
-        // a zero has the sign of the quotient: x / s + 0 is -0 for a small negative x, and stays it
-        w[t] = (KIND == kInt && (!ZP || (q == 0.0f && z == 0.0f))) ? copysignf(q, lo) : q;
+        for (int t = begin; t < end; ++t) {
+          const float s = par[t * kRows], rlo = par[(kMicro + t) * kRows], rhi = par[(2 * kMicro + t) * kRows];
+          const float z = ZP ? par[(3 * kMicro + t) * kRows] : 0.0f, mz = ZP ? fabsf(z) * (0.5f * kMargin) : 0.0f;
+          const float wi = w[t], lo = fmaf(wi, rlo, z - mz);
+          const float qc = code_of<KIND>(lo, qmin, qmax);
+          differ |= qc != code_of<KIND>(fmaf(wi, rhi, z + mz), qmin, qmax);
+          const float q = dequant<KIND, SB, ZP>(qc, s, z);
+          // loss and error use the reciprocal of the pivot (an ulp from the reference's divisions)
+          const float tt = __fmul_rn(__fsub_rn(wi, q), sRd[c0 + t]);
+          e[t] = tt;
+          // a zero has the sign of the quotient: x / s + 0 is -0 for a small negative x, and stays it
+          w[t] = (KIND == kInt && (!ZP || (q == 0.0f && z == 0.0f))) ? copysignf(q, lo) : q;
 #pragma unroll
-        for (int k4 = (t + 1) / 4; k4 < kMicro / 4; ++k4) {
-          const float4 uu = *reinterpret_cast<const float4*>(u + t * ULD + 4 * k4);
-          if (4 * k4 + 0 > t) w[4 * k4 + 0] = fmaf(-tt, uu.x, w[4 * k4 + 0]);
-          if (4 * k4 + 1 > t) w[4 * k4 + 1] = fmaf(-tt, uu.y, w[4 * k4 + 1]);
-          if (4 * k4 + 2 > t) w[4 * k4 + 2] = fmaf(-tt, uu.z, w[4 * k4 + 2]);
-          if (4 * k4 + 3 > t) w[4 * k4 + 3] = fmaf(-tt, uu.w, w[4 * k4 + 3]);
+          for (int k4 = (t + 1) / 4; k4 < kMicro / 4; ++k4) {
+            const float4 uu = *reinterpret_cast<const float4*>(u + t * ULD + 4 * k4);
+            if (4 * k4 + 0 > t) w[4 * k4 + 0] = fmaf(-tt, uu.x, w[4 * k4 + 0]);
+            if (4 * k4 + 1 > t) w[4 * k4 + 1] = fmaf(-tt, uu.y, w[4 * k4 + 1]);
+            if (4 * k4 + 2 > t) w[4 * k4 + 2] = fmaf(-tt, uu.z, w[4 * k4 + 2]);
+            if (4 * k4 + 3 > t) w[4 * k4 + 3] = fmaf(-tt, uu.w, w[4 * k4 + 3]);
+          }
         }
-      }
-      float* eo = sE + (m & 1) * kMicro * ELD + lane;
-      if (__any_sync(0xffffffffu, differ) || s_odd) {
-        // by the exact rules, column by column in shared memory, where the tile still is as the micro-block found it
-        const float* e_prev = sE + ((m + 1) & 1) * kMicro * ELD + lane;
+        return __any_sync(0xffffffffu, differ);
+      };
+      // columns from `begin` on by the exact rules, one by one in shared memory
+      auto exact = [&](int begin) {
 #pragma unroll 1
-        for (int k = 0; k < kMicro && m > 0; ++k) {
-          float v = sW[(c0 + k) * WLD + lane];
-          for (int t = 0; t < kMicro; ++t) v = fmaf(-e_prev[t * ELD], u_prev[t * ULD + c0 + k], v);
-          sW[(c0 + k) * WLD + lane] = v;
-        }
-#pragma unroll 1
-        for (int t = 0; t < kMicro; ++t) {
-          float* wt = sW + (c0 + t) * WLD + lane;
-          const float wi = *wt, s = par[t * kRows], z = ZP ? par[(3 * kMicro + t) * kRows] : 0.0f;
+        for (int t = begin; t < kMicro; ++t) {
+          const float wi = wcol[t * WLD], s = par[t * kRows], z = ZP ? par[(3 * kMicro + t) * kRows] : 0.0f;
           const float q = dequant_code<SB>(round_code_k<KIND>(__fdiv_rn(wi, s) + z, qmin, qmax), s, z);
           const float tt = __fmul_rn(__fsub_rn(wi, q), sRd[c0 + t]);
-          *wt = q;
+          wcol[t * WLD] = q;
           eo[t * ELD] = tt;
-          for (int k = t + 1; k < kMicro; ++k) {
-            float* wk = sW + (c0 + k) * WLD + lane;
-            *wk = fmaf(-tt, u[t * ULD + k], *wk);
-          }
+          for (int k = t + 1; k < kMicro; ++k) wcol[k * WLD] = fmaf(-tt, u[t * ULD + k], wcol[k * WLD]);
         }
 #pragma unroll
-        for (int t = 0; t < kMicro; ++t) e[t] = eo[t * ELD];
+        for (int t = kHead; t < kMicro; ++t) e[t] = eo[t * ELD];
+      };
+      auto announce = [&] {   // the first errors are there
+        if (m + 1 < micros) asm volatile("bar.arrive 1, 64;" ::: "memory");
+      };
+      float w0[kMicro];   // as the micro-block found it
+#pragma unroll
+      for (int t = 0; t < kMicro; ++t) w0[t] = w[t];
+      if (!chain(std::integral_constant<int, 0>(), std::integral_constant<int, kHead>()) && !s_odd) {
+#pragma unroll
+        for (int t = 0; t < kHead; ++t) eo[t * ELD] = e[t];
+        announce();
+#pragma unroll
+        for (int t = 0; t < kMicro; ++t) wcol[t * WLD] = w[t];
+        if (!chain(std::integral_constant<int, kHead>(), std::integral_constant<int, kMicro>())) {
+#pragma unroll
+          for (int t = kHead; t < kMicro; ++t) { wcol[t * WLD] = w[t]; eo[t * ELD] = e[t]; }
+        } else {
+          exact(kHead);
+        }
       } else {
 #pragma unroll
-        for (int t = 0; t < kMicro; ++t) { sW[(c0 + t) * WLD + lane] = w[t]; eo[t * ELD] = e[t]; }
+        for (int t = 0; t < kMicro; ++t) wcol[t * WLD] = w0[t];
+        exact(0);
+        announce();
       }
-    } else if ((warp & 3) == 0) {
+    } else if (m + 1 < micros) {
+      const bool beside = (warp & 3) == 0;   // the chain warp's scheduler
       if (warp == kFetchWarp) {
-        if (m > 0 && m + 1 < micros) fetch_u(m + 1);   // into the buffer of micro-block m - 2
-        if (lane == 0) s_next[(m + 1) & 1] = 0;        // (nobody takes from it before the barrier)
-      } else if (m + 1 < micros) {
-        fetch_params(m + 1);
+        if (m > 0) fetch_u(m + 1);                // into the buffer of micro-block m - 2
+        if (lane == 0) s_next[(m + 1) & 1] = 0;   // (nobody takes from it before the barrier)
       }
-    } else {
-      if (kParamWarp == 5 && warp == 5 && m + 1 < micros) fetch_params(m + 1);
+      if (warp == kParamWarp) fetch_params(m + 1);
       if (warp == 6 && m > 0) finish_errors(m - 1);
-      if (m > 0 && m + 1 < micros) {
-        // W[32 rows, columns of a task] -= E[32, 16] U[16, columns]
-        const float* ei = sE + ((m - 1) & 1) * kMicro * ELD + (lane & 3) * ELD + (lane >> 2);
-        uint32_t ah[2][2][4], al[2][2][4];   // [row tile][k step]
-#pragma unroll
-        for (int y = 0; y < 2; ++y)
-#pragma unroll
-          for (int ks = 0; ks < 2; ++ks)
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-              split_tf32(ei[(ks * 8 + (k >> 1) * 4) * ELD + y * 16 + (k & 1) * 8], ah[y][ks][k], al[y][ks][k]);
+      ErrFrag f;
+      if (m > 0 && (!beside || micros - m > 16)) {
+        load_errors(sE + ((m - 1) & 1) * kMicro * ELD, lane, false, f);
+        if (warp == kNextWarp) {
+          apply_errors<ULD>(f, u_prev + c0 + kMicro, sW + (c0 + kMicro) * WLD, lane);
+        } else {
 #pragma unroll 1
-        while (true) {
-          int task = 0;
-          if (lane == 0) task = atomicAdd(&s_next[m & 1], 1);
-          const int c = (m + 1) * kMicro + __shfl_sync(0xffffffffu, task, 0) * (XT * 8);
-          if (c >= micros * kMicro) break;
-          const bool whole = XT == 2 || c + XT * 8 <= micros * kMicro;   // else only the first 16 columns exist
-          float* o = sW + (c + 2 * (lane & 3)) * WLD + (lane >> 2);
-          const float* ub = u_prev + (lane & 3) * ULD + c + (lane >> 2);
-          float old[2][XT][4], acc[2][XT][4] = {}, part[2][XT][4] = {};   // [row tile][column tile]
-#pragma unroll
-          for (int x = 0; x < XT; ++x)
-            if (x < 2 || whole) {
-#pragma unroll
-              for (int y = 0; y < 2; ++y)
-#pragma unroll
-                for (int k = 0; k < 4; ++k) old[y][x][k] = o[(x * 8 + (k & 1)) * WLD + y * 16 + (k >> 1) * 8];
-            }
-#pragma unroll
-          for (int ks = 0; ks < 2; ++ks) {
-            uint32_t bh[XT][2], bl[XT][2];
-#pragma unroll
-            for (int x = 0; x < XT; ++x)
-#pragma unroll
-              for (int k = 0; k < 2; ++k)
-                split_tf32((x < 2 || whole) ? ub[(ks * 8 + k * 4) * ULD + x * 8] : 0.0f, bh[x][k], bl[x][k]);
-#pragma unroll
-            for (int y = 0; y < 2; ++y)
-#pragma unroll
-              for (int x = 0; x < XT; ++x) mma_tf32(acc[y][x], ah[y][ks], bh[x]);
-#pragma unroll
-            for (int y = 0; y < 2; ++y)
-#pragma unroll
-              for (int x = 0; x < XT; ++x) mma_tf32(part[y][x], ah[y][ks], bl[x]);
-#pragma unroll
-            for (int y = 0; y < 2; ++y)
-#pragma unroll
-              for (int x = 0; x < XT; ++x) mma_tf32(part[y][x], al[y][ks], bh[x]);
+          while (true) {
+            int task = 0;
+            if (lane == 0) task = atomicAdd(&s_next[m & 1], 1);
+            const int c = c0 + (2 + __shfl_sync(0xffffffffu, task, 0)) * kMicro;
+            if (c >= micros * kMicro) break;
+            apply_errors<ULD>(f, u_prev + c, sW + c * WLD, lane);
           }
-#pragma unroll
-          for (int x = 0; x < XT; ++x)
-            if (x < 2 || whole) {
-#pragma unroll
-              for (int y = 0; y < 2; ++y)
-#pragma unroll
-                for (int k = 0; k < 4; ++k)
-                  o[(x * 8 + (k & 1)) * WLD + y * 16 + (k >> 1) * 8] = old[y][x][k] - (acc[y][x][k] + part[y][x][k]);
-            }
         }
       }
+      if (warp == kNextWarp) {
+        asm volatile("bar.sync 1, 64;" ::: "memory");
+        load_errors(sE + (m & 1) * kMicro * ELD, lane, true, f);
+        apply_errors<ULD>(f, u + kMicro, sW + (c0 + kMicro) * WLD, lane);
+      }
+    } else if (warp == 6 && m > 0) {
+      finish_errors(m - 1);
     }
     if (m + 1 < micros) wait_u(m + 1);
     __syncthreads();
