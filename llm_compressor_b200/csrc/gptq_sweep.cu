@@ -189,9 +189,9 @@ __device__ __forceinline__ void apply_errors(const ErrFrag& f, const float* u, f
 // spends its time on the broadcast loads of U: 480 cycles a column against the chain's own), taking tasks of 16 columns
 // from a counter.  The columns next in line take the first twelve errors from a warp that waits for them while the chain
 // is on the last four, and those four from the chain warp.  Duties beside that: the warps that share the chain warp's
-// scheduler fetch parameters and ask for rows of U by bulk copies (as per-thread copies they block the warps that issue
-// them: all CTAs want the same rows at the same time), and take tasks only while these, not the chain, decide; warp 6
-// writes the errors out as the operand of the trailing product.  One barrier per micro-block.  Every role is a
+// scheduler ask for rows of U by bulk copies (as per-thread copies they block the warps that issue them: all CTAs want
+// the same rows at the same time), and take tasks only while these, not the chain, decide; warp 5 fetches parameters,
+// warp 6 writes the errors out as the operand of the trailing product.  One barrier per micro-block.  Every role is a
 // latency-bound stream of instructions, a quarter of its stalls instruction fetch, hence short loops rather than
 // unrolled code off the chain.
 template <int SBLK, bool SB, int KIND, bool ZP>
@@ -200,7 +200,6 @@ __global__ void __launch_bounds__(32 * warps_of(SBLK), SBLK == 512 ? 1 : 2) swee
   extern __shared__ __align__(16) float sm[];
   constexpr int ULD = u_stride(SBLK);
   constexpr int NW = warps_of(SBLK), NT = 32 * NW;
-  constexpr int kFetchWarp = NW > 8 ? 8 : 4, kParamWarp = NW > 8 ? 4 : 5;
   constexpr int kNextWarp = NW > 8 ? 9 : 1;            // brings the next micro-block's columns up to date
   constexpr int kHead = 12;                            // its share of a micro-block's errors
   float* sU = sm;                                      // [3][kMicro][ULD]
@@ -222,22 +221,26 @@ __global__ void __launch_bounds__(32 * warps_of(SBLK), SBLK == 512 ? 1 : 2) swee
   const bool live = row < p.N;
   const bool bulk = U && ((p.ldu & 3) == 0) && ((((uintptr_t)U) & 15) == 0) && (sb % kMicro) == 0;
   const bool vecw = ((p.ldw & 3) == 0) && ((((uintptr_t)W) & 15) == 0) && (sb & 3) == 0;
-  // rows of U of micro-block m, columns from its own first one on (columns beyond sb are zero).  Called by a whole
-  // warp; with bulk copies one lane does it.
-  auto fetch_u = [&](int m) {
+  // `ROWS` rows from t0 on of U's micro-block m, columns from its own first one on (columns beyond sb are zero).
+  // Called by whole warps; with bulk copies one lane of each works, the one with t0 = 0 announces the bytes.
+  auto fetch_u = [&](int m, int t0, auto ROWS) {
     float* dst = sU + (m % 3) * kMicro * ULD;
     const int c0 = m * kMicro, c_end = micros * kMicro;
     if (bulk) {
       if (lane == 0) {
         const uint32_t bytes = (uint32_t)(c_end - c0) * 4, bar = smem_u32(&s_bar[m % 3]);
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes * kMicro) : "memory");
-        for (int t = 0; t < kMicro; ++t)
-          bulk_copy(dst + t * ULD + c0, U + (int64_t)(c0 + t) * p.ldu + c0, bytes, bar);
+        if (t0 == 0)
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes * kMicro) : "memory");
+#pragma unroll
+        for (int t = 0; t < ROWS; ++t)
+          bulk_copy(dst + (t0 + t) * ULD + c0, U + (int64_t)(c0 + t0 + t) * p.ldu + c0, bytes, bar);
       }
       return;
     }
-    for (int t = 0; t < kMicro; ++t) {
+#pragma unroll 1
+    for (int t = t0; t < t0 + ROWS; ++t) {
       const int i = c0 + t;
+#pragma unroll 1
       for (int c = c0 + lane; c < c_end; c += 32) {
         float v = (i == c) ? 1.0f : 0.0f;
         if (U) v = (i < sb && c < sb) ? U[(int64_t)i * p.ldu + c] : 0.0f;
@@ -245,6 +248,8 @@ __global__ void __launch_bounds__(32 * warps_of(SBLK), SBLK == 512 ? 1 : 2) swee
       }
     }
   };
+  // a warp of twelve asks for half of a micro-block's rows, of eight for all
+  constexpr std::integral_constant<int, NW == 12 ? kMicro / 2 : kMicro> kAskRows;
   auto wait_u = [&](int m) {
     if (!bulk) return;
     const uint32_t bar = smem_u32(&s_bar[m % 3]), parity = (uint32_t)(m / 3) & 1u;
@@ -291,7 +296,7 @@ __global__ void __launch_bounds__(32 * warps_of(SBLK), SBLK == 512 ? 1 : 2) swee
       put(0, s);
       s = dst[0];
       const float lo = dst[kMicro * kRows], hi = dst[2 * kMicro * kRows];
-#pragma unroll
+#pragma unroll 4
       for (int t = 0; t < kMicro; ++t) {
         dst[t * kRows] = s;
         dst[(kMicro + t) * kRows] = lo;
@@ -318,8 +323,8 @@ __global__ void __launch_bounds__(32 * warps_of(SBLK), SBLK == 512 ? 1 : 2) swee
   }
   if (warp == 1) {
     __syncwarp();
-    fetch_u(0);
-    if (micros > 1) fetch_u(1);
+#pragma unroll 1
+    for (int m = 0; m < micros && m < 2; ++m) fetch_u(m, 0, std::integral_constant<int, kMicro>());
   }
   const int32_t* col_group = p.col_group.at(job);
   for (int c = tid; c < micros * kMicro; c += NT) {
@@ -362,7 +367,7 @@ __global__ void __launch_bounds__(32 * warps_of(SBLK), SBLK == 512 ? 1 : 2) swee
     sSame[tid] = same ? 1 : 0;
   }
   __syncthreads();
-  if (warp == kParamWarp) fetch_params(0);
+  if (warp == 5) fetch_params(0);
   wait_u(0);
   __syncthreads();
 
@@ -464,9 +469,6 @@ __global__ void __launch_bounds__(32 * warps_of(SBLK), SBLK == 512 ? 1 : 2) swee
       auto announce = [&] {   // the first errors are there
         if (m + 1 < micros) asm volatile("bar.arrive 1, 64;" ::: "memory");
       };
-      float w0[kMicro];   // as the micro-block found it
-#pragma unroll
-      for (int t = 0; t < kMicro; ++t) w0[t] = w[t];
       if (!chain(std::integral_constant<int, 0>(), std::integral_constant<int, kHead>()) && !s_odd) {
 #pragma unroll
         for (int t = 0; t < kHead; ++t) eo[t * ELD] = e[t];
@@ -480,18 +482,22 @@ __global__ void __launch_bounds__(32 * warps_of(SBLK), SBLK == 512 ? 1 : 2) swee
           exact(kHead);
         }
       } else {
-#pragma unroll
-        for (int t = 0; t < kMicro; ++t) wcol[t * WLD] = w0[t];
+        // (the tile still is as the micro-block found it, without the last errors of the one before)
+#pragma unroll 1
+        for (int k = 0; k < kMicro && m > 0; ++k) {
+          float v = wcol[k * WLD];
+          for (int t = kHead; t < kMicro; ++t)
+            v = fmaf(-sE[((m + 1) & 1) * kMicro * ELD + t * ELD + lane], u_prev[t * ULD + c0 + k], v);
+          wcol[k * WLD] = v;
+        }
         exact(0);
         announce();
       }
     } else if (m + 1 < micros) {
       const bool beside = (warp & 3) == 0;   // the chain warp's scheduler
-      if (warp == kFetchWarp) {
-        if (m > 0) fetch_u(m + 1);                // into the buffer of micro-block m - 2
-        if (lane == 0) s_next[(m + 1) & 1] = 0;   // (nobody takes from it before the barrier)
-      }
-      if (warp == kParamWarp) fetch_params(m + 1);
+      if (beside && m > 0) fetch_u(m + 1, (warp - 4) * (kAskRows / 4), kAskRows);   // into the buffer of micro-block m - 2
+      if (tid == 32) s_next[(m + 1) & 1] = 0;   // (nobody takes from it before the barrier)
+      if (warp == 5) fetch_params(m + 1);
       if (warp == 6 && m > 0) finish_errors(m - 1);
       ErrFrag f;
       if (m > 0 && (!beside || micros - m > 16)) {
