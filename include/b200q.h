@@ -163,6 +163,14 @@ int b200q_quantize_pack(const void* W, int wdtype, int64_t N, int64_t K, int64_t
                         const float* global_scale, const b200q_qargs* qa, int pack_int8,
                         void* out, void* stream);
 
+/* Q(W * s) / s with one scale per column, as the AWQ search evaluates a grid point
+ * (src/llmcompressor/modifiers/transform/awq/base.py:647-709): bf16(W * s), a memoryless min-max
+ * observation of it, fake quantisation, division by s in float32, rounding to bf16.  bf16 weights,
+ * int4 / int8 codes with one scale per group (a power of two, 8..256) or row of at most 16384 columns;
+ * everything else returns B200Q_ERR_UNSUPPORTED.  col_scale: float [K]; out: bf16 [N, K]. */
+int b200q_scaled_fake_quantize(const void* W, int wdtype, int64_t N, int64_t K, int64_t ldw, const float* col_scale,
+                               const b200q_qargs* qa, void* out, void* stream);
+
 /* Asymmetric zero points packed along dim 0 (pack_to_int32(zp, bits, packed_dim=0),
  * CT/compressors/pack_quantized/base.py:70-73): zp int8 [N,G] -> int32 [ceil(N*bits/32), G]. */
 int b200q_pack_zero_points(const int8_t* zp, int64_t N, int64_t G, int num_bits, int32_t* out,

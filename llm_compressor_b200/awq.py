@@ -167,6 +167,12 @@ def scaled_fake_quantize(weights, scales: torch.Tensor, layers, parent=None) -> 
     fake-quantised, divided by s in float32 and rounded again (base.py:647-709).  Under
     TENSOR_GROUP the q/k/v or gate/up siblings inside ``parent`` share their global scale, as
     ``fuse_weight_observers(parent)`` arranges in the reference."""
+    # schemes whose parameters come from the weight alone: one kernel per layer
+    schemes = [layer.quantization_scheme.weights for layer in layers]
+    if all(a.strategy != "tensor_group" for a in schemes):
+        done = [ops.scaled_fake_quantize(w, scales, a) for w, a in zip(weights, schemes)]
+        if all(d is not None for d in done):
+            return done
     view = scales.view(1, -1)
     scaled = [(w * view).to(w.dtype) for w in weights]
     saved = [(getattr(layer, "weight_observer", None), layer.weight.data) for layer in layers]

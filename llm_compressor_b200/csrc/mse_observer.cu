@@ -20,7 +20,7 @@ namespace mse {
 
 struct Cfg {
   int symmetric, scale_kind, zp_kind, mx_offset;
-  float qmin, qmax, half_range, range, eps;
+  float qmin, qmax, half_range, range, eps, inv_half_range;
   int kind;
   int steps, patience;
   double grid;
@@ -41,7 +41,8 @@ __device__ __forceinline__ void qparams_local(float mn, float mx, const Cfg& c, 
       float e = (biased == 0) ? 0.0f : fminf(fmaxf((float)(biased - c.mx_offset), 0.0f), 255.0f);
       s = __uint_as_float(e >= 1.0f ? ((uint32_t)e << 23) : 0x00400000u);
     } else {
-      s = rnd_if<TB>(__fdiv_rn(amax, c.half_range));
+      // (bf16 statistics: the product with the reciprocal rounds to the same bf16 value, see qparams_one)
+      s = TB ? bf16r(amax * c.inv_half_range) : __fdiv_rn(amax, c.half_range);
       if (c.scale_kind == B200Q_SCALE_FP8) s = e4m3_round(fminf(fmaxf(s, -448.0f), 448.0f));
     }
     zp = 0.0f;
@@ -132,16 +133,30 @@ __global__ void __launch_bounds__(256) mse_group_kernel(const void* __restrict__
 }
 
 // ---------------------------------------------------------------------------------------
-// bf16 weights, integer codes, GROUP strategies: the same search with packed bf16x2 arithmetic.
-// torch evaluates the candidate with element-wise bf16 ops; for bf16 operands a packed
-// HADD2 / HMUL2 gives exactly the rounded result of the float32 operation followed by a
-// rounding to bf16 (the _rn forms of the intrinsics: the plain ones let the compiler fuse the
-// product and the subtraction into one FMA with a single rounding), so add-zero-point, clamp, round-to-integer (magic number 192 for 4 bits,
-// h2rint otherwise), dequantise, subtract and abs run two elements per instruction.  The two
-// places where float32 is needed keep an exact fallback: the quotient x/s is formed as x*(1/s)
-// and the power as exp2(norm*log2 d); a lane whose value lies within a few float ulps of a bf16
-// rounding midpoint (3 ulps for the quotient, 192 for the power, twice the error bound of the
-// MUFU functions at these magnitudes) recomputes that element with the IEEE division / powf.
+// bf16 weights: the same search in packed bf16x2 arithmetic with the power read from a table.
+//
+// torch evaluates a candidate with element-wise bf16 ops.  For bf16 operands a packed HADD2 / HMUL2 / HFMA2 gives
+// exactly the rounded result of the float32 operation followed by a rounding to bf16 (the _rn forms of the intrinsics:
+// the plain ones let the compiler fuse a product and a subtraction into one rounding).  The quotient bf16(x / s) is
+// fma(x, r_hi, fma(x, r_lo, +0)) with 1 / s split into two bf16 parts, exact for every pair of bf16 significands (see
+// stream_kernels.cuh); scales outside 2^-100 .. 2^100 take element-wise divisions.  The error |q - x| is a bf16 value,
+// so its rounded power is one of 32768: a table in shared memory, made once per call with powf.
+//
+// What bounds it: the table look-ups (about three cycles a warp, bank conflicts of 32 random entries) and about ten
+// instructions an element.  Evaluating exp2(norm * log2 d) instead costs two special-function results, checks against
+// rounding midpoints and a fallback: 685 us for 20 candidates on 4096 x 4096.
+constexpr int kTable = 32768;
+constexpr size_t kTableBytes = kTable * 2;
+
+__global__ void __launch_bounds__(256) make_table_kernel(__nv_bfloat16* __restrict__ table, float norm, int* __restrict__ ctl,
+                                                         int n) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  const float d = __uint_as_float((uint32_t)i << 16);
+  if (i < kTable) table[i] = __float2bfloat16_rn(d == 0.0f ? 0.0f : powf(d, norm));
+  if (blockIdx.x == 0)
+    for (int k = threadIdx.x; k < n; k += 256) ctl[k] = 0;
+}
+
 __device__ __forceinline__ uint32_t bf2_of(float v) {
   __nv_bfloat162 r = __float2bfloat162_rn(v);
   return *reinterpret_cast<uint32_t*>(&r);
@@ -151,42 +166,127 @@ __device__ __forceinline__ uint32_t bf2_pack(float hi, float lo) {
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
   return d;
 }
-#define B200Q_BF2(op, a, b) ([&] { __nv_bfloat162 r_ = op(*reinterpret_cast<const __nv_bfloat162*>(&(a)), \
-                                                         *reinterpret_cast<const __nv_bfloat162*>(&(b)));   \
-                                   return *reinterpret_cast<uint32_t*>(&r_); }())
+#define B200Q_BF2(op, ...) ([&] { __nv_bfloat162 r_ = op(__VA_ARGS__); return *reinterpret_cast<uint32_t*>(&r_); }())
+#define B200Q_B(v) *reinterpret_cast<const __nv_bfloat162*>(&(v))
 
-template <bool FOUR_BIT>
-__global__ void __launch_bounds__(256) mse_group_bf16_int_kernel(const void* __restrict__ W, int64_t N, int64_t K,
-                                                                 int64_t ldw, int g, Cfg c, int* __restrict__ ctl,
-                                                                 int pass, void* __restrict__ mn_out,
-                                                                 void* __restrict__ mx_out) {
+enum MseKind { kMseInt4 = 0, kMseInt8 = 1, kMseFp8 = 2, kMseFp4 = 3 };
+
+// what the elements need from one candidate
+struct Cand {
+  float s, z;
+  uint32_t rhi2, rlo2, s2, z2;
+  bool slow;
+};
+__device__ __forceinline__ Cand make_cand(float smn, float smx, const Cfg& c) {
+  Cand q;
+  qparams_local<true>(smn, smx, c, q.s, q.z);
+  const float rs = __frcp_rn(q.s), rhi = bf16r(rs);
+  q.rhi2 = bf2_of(rhi); q.rlo2 = bf2_of(rs - rhi); q.s2 = bf2_of(q.s); q.z2 = bf2_of(q.z);
+  q.slow = !(q.s >= 0x1p-100f && q.s <= 0x1p100f);
+  return q;
+}
+// |fake_quantize(x) - x| of a pair, sign bits cleared
+template <int KIND, bool SYM>
+__device__ __forceinline__ uint32_t pair_error(uint32_t w, const Cand& q, uint32_t qmin2, uint32_t qmax2) {
+  const uint32_t zero = 0u, magic = 0x43404340u;   // {192, 192}: integers are 1 apart in [128, 256)
+  uint32_t v = B200Q_BF2(__hfma2, B200Q_B(w), B200Q_B(q.rlo2), B200Q_B(zero));
+  v = B200Q_BF2(__hfma2, B200Q_B(w), B200Q_B(q.rhi2), B200Q_B(v));
+  if (!SYM) v = B200Q_BF2(__hadd2_rn, B200Q_B(v), B200Q_B(q.z2));
+  if (KIND == kMseInt4 || KIND == kMseInt8) {
+    v = B200Q_BF2(__hmax2, B200Q_B(v), B200Q_B(qmin2));
+    v = B200Q_BF2(__hmin2, B200Q_B(v), B200Q_B(qmax2));
+    if (KIND == kMseInt4) {
+      v = B200Q_BF2(__hadd2_rn, B200Q_B(v), B200Q_B(magic));
+      v = B200Q_BF2(__hsub2_rn, B200Q_B(v), B200Q_B(magic));
+    } else {
+      v = B200Q_BF2(h2rint, B200Q_B(v));
+    }
+  } else {
+    // through the hardware's code (round to nearest even, saturating) and back
+    const float lo = __uint_as_float(v << 16), hi = __uint_as_float(v & 0xFFFF0000u);
+    uint32_t h;
+    if (KIND == kMseFp8)
+      asm("{\n\t.reg .b16 b;\n\tcvt.rn.satfinite.e4m3x2.f32 b, %2, %1;\n\tcvt.rn.f16x2.e4m3x2 %0, b;\n\t}" : "=r"(h) : "f"(lo), "f"(hi));
+    else
+      asm("{\n\t.reg .b8 b;\n\tcvt.rn.satfinite.e2m1x2.f32 b, %2, %1;\n\tcvt.rn.f16x2.e2m1x2 %0, b;\n\t}" : "=r"(h) : "f"(lo), "f"(hi));
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h));
+    v = bf2_pack(f.y, f.x);
+  }
+  if (!SYM) v = B200Q_BF2(__hsub2_rn, B200Q_B(v), B200Q_B(q.z2));
+  v = B200Q_BF2(__hmul2_rn, B200Q_B(v), B200Q_B(q.s2));
+  v = B200Q_BF2(__hsub2_rn, B200Q_B(v), B200Q_B(w));
+  return v & 0x7FFF7FFFu;
+}
+// error sum of a chunk of 8 elements, in element order
+template <int KIND, bool SYM>
+__device__ __forceinline__ float chunk_error(const uint32_t (&w)[4], const Cand& q, uint32_t qmin2, uint32_t qmax2,
+                                             const Cfg& c, const unsigned short* __restrict__ tab) {
+  float err = 0.0f;
+  if (q.slow) {
+    for (int k = 0; k < 4; ++k) {
+      err += elem_error<true>(__uint_as_float(w[k] << 16), q.s, q.z, c);
+      err += elem_error<true>(__uint_as_float(w[k] & 0xFFFF0000u), q.s, q.z, c);
+    }
+    return err;
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const uint32_t d = pair_error<KIND, SYM>(w[k], q, qmin2, qmax2);
+    err += __uint_as_float((uint32_t)tab[d & 0xFFFFu] << 16);
+    err += __uint_as_float((uint32_t)tab[d >> 16] << 16);
+  }
+  return err;
+}
+__device__ __forceinline__ void load_table(uint4* dst, const __nv_bfloat16* __restrict__ table) {
+#pragma unroll 4
+  for (int i = threadIdx.x; i < (int)(kTableBytes / 16); i += blockDim.x) dst[i] = reinterpret_cast<const uint4*>(table)[i];
+}
+__device__ __forceinline__ void chunk_range(const uint4& raw, float& lo, float& hi) {
+  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const float a = __uint_as_float(w[k] << 16), b = __uint_as_float(w[k] & 0xFFFF0000u);
+    lo = fminf(lo, fminf(a, b)); hi = fmaxf(hi, fmaxf(a, b));
+  }
+}
+
+// GROUP strategies.  The chunks of a group are shared by L lanes, R each (L apart), so that a candidate's parameters
+// are derived once per R * 8 elements.  The chunk sums are added in the order of a butterfly over all chunks of the
+// group, whatever R is.
+template <int KIND, bool SYM, int R>
+__global__ void __launch_bounds__(256) mse_group_bf16_kernel(const void* __restrict__ W, int64_t N, int64_t K, int64_t ldw,
+                                                             int g, Cfg c, const __nv_bfloat16* __restrict__ table,
+                                                             int* __restrict__ ctl, int pass, void* __restrict__ mn_out,
+                                                             void* __restrict__ mx_out) {
   using T = __nv_bfloat16;
+  extern __shared__ __align__(16) unsigned short s_table[];
   __shared__ float s_shrink[1024];
   const int limit = (pass == 0) ? c.steps : ctl[0];
   if (pass == 1 && limit >= c.steps) return;  // the search never stopped early
-  for (int i = threadIdx.x; i < limit; i += blockDim.x) s_shrink[i] = shrink_factor(i, c.grid);
+  load_table(reinterpret_cast<uint4*>(s_table), table);
+  for (int i = threadIdx.x; i < limit && i < 1024; i += blockDim.x) s_shrink[i] = shrink_factor(i, c.grid);
   __syncthreads();
-  const int lanes = g >> 3;
-  const int64_t cpr = K >> 3, total = N * cpr, gpr = K / g;
-  const QRange qr{c.qmin, c.qmax, c.kind};
-  const uint32_t qmin2 = bf2_of(c.qmin), qmax2 = bf2_of(c.qmax), magic = 0x43404340u;  // {192, 192}
-  for (int64_t ch = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; ch < ((total + 31) & ~31LL);
-       ch += (int64_t)gridDim.x * blockDim.x) {
-    const bool live = ch < total;
-    uint32_t w[4] = {0u, 0u, 0u, 0u};
+  const int L = (g >> 3) / R;
+  const int64_t gpr = K / g, total = N * gpr * L;
+  const uint32_t qmin2 = bf2_of(c.qmin), qmax2 = bf2_of(c.qmax);
+  for (int64_t slot = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; slot < ((total + 31) & ~31LL);
+       slot += (int64_t)gridDim.x * blockDim.x) {
+    const bool live = slot < total;
+    const int64_t gi = live ? slot / L : 0, row = gi / gpr;
+    const int j = (int)(slot - gi * L);
+    uint32_t w[R][4];
     float lo = INFINITY, hi = -INFINITY;
-    int64_t row = 0, cc = 0;
-    if (live) {
-      row = ch / cpr; cc = ch - row * cpr;
-      const uint4 raw = *reinterpret_cast<const uint4*>((const T*)W + row * ldw + cc * 8);
-      w[0] = raw.x; w[1] = raw.y; w[2] = raw.z; w[3] = raw.w;
+    const T* src = (const T*)W + row * ldw + (gi - row * gpr) * g + j * 8;
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const float a = __uint_as_float(w[k] << 16), b = __uint_as_float(w[k] & 0xFFFF0000u);
-        lo = fminf(lo, fminf(a, b)); hi = fmaxf(hi, fmaxf(a, b));
+    for (int k = 0; k < R; ++k) {
+      uint4 raw = make_uint4(0u, 0u, 0u, 0u);
+      if (live) {
+        raw = __ldg(reinterpret_cast<const uint4*>(src + (int64_t)k * L * 8));
+        chunk_range(raw, lo, hi);
       }
+      w[k][0] = raw.x; w[k][1] = raw.y; w[k][2] = raw.z; w[k][3] = raw.w;
     }
-    for (int o = lanes >> 1; o > 0; o >>= 1) {
+    for (int o = L >> 1; o > 0; o >>= 1) {
       lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
       hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
     }
@@ -194,65 +294,104 @@ __global__ void __launch_bounds__(256) mse_group_bf16_int_kernel(const void* __r
     float best_err = 3.3895313892515355e38f;  // finfo(bfloat16).max
     float best_mn = mn, best_mx = mx;
     for (int i = 0; i < limit; ++i) {
-      const float p = s_shrink[i];
+      const float p = i < 1024 ? s_shrink[i] : shrink_factor(i, c.grid);
       const float smn = bf16r(mn * p), smx = bf16r(mx * p);
-      float s, z;
-      qparams_local<true>(smn, smx, c, s, z);
-      const float rs = __frcp_rn(s);
-      const uint32_t s2 = bf2_of(s), z2 = bf2_of(z);
-      float err = 0.0f;
+      const Cand q = make_cand(smn, smx, c);
+      float part[R];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const float x0 = __uint_as_float(w[k] << 16), x1 = __uint_as_float(w[k] & 0xFFFF0000u);
-        const float q0 = x0 * rs, q1 = x1 * rs;
-        // quotients within 3 ulps of a bf16 midpoint (half-word 0x8000) take the IEEE division
-        const uint32_t mq = (__byte_perm(__float_as_uint(q0), __float_as_uint(q1), 0x5410) + 0x80048004u) & 0xFFF0FFF0u;
-        uint32_t cq = bf2_pack(q1, q0);
-        if (((mq & 0xFFFFu) == 0u) || ((mq >> 16) == 0u))
-          cq = bf2_pack(bf16r(__fdiv_rn(x1, s)), bf16r(__fdiv_rn(x0, s)));
-        uint32_t v = c.symmetric ? cq : B200Q_BF2(__hadd2_rn, cq, z2);
-        v = B200Q_BF2(__hmax2, v, qmin2);
-        v = B200Q_BF2(__hmin2, v, qmax2);
-        if (FOUR_BIT) {
-          v = B200Q_BF2(__hadd2_rn, v, magic);   // integers are 1 apart in [128, 256): rounds to nearest even
-          v = B200Q_BF2(__hsub2_rn, v, magic);
-        } else {
-          __nv_bfloat162 r_ = h2rint(*reinterpret_cast<const __nv_bfloat162*>(&v));
-          v = *reinterpret_cast<uint32_t*>(&r_);
-        }
-        if (!c.symmetric) v = B200Q_BF2(__hsub2_rn, v, z2);
-        v = B200Q_BF2(__hmul2_rn, v, s2);
-        v = B200Q_BF2(__hsub2_rn, v, w[k]);
-        v &= 0x7FFF7FFFu;   // |.|
-        const float d0 = __uint_as_float(v << 16), d1 = __uint_as_float(v & 0xFFFF0000u);
-        float e0 = exp2f(c.norm * __log2f(d0)), e1 = exp2f(c.norm * __log2f(d1));
-        e0 = (d0 == 0.0f) ? 0.0f : e0;
-        e1 = (d1 == 0.0f) ? 0.0f : e1;
-        // powers within 192 ulps of a bf16 midpoint, or outside the range where the MUFU error
-        // bounds hold, are recomputed with powf
-        const uint32_t l0 = __float_as_uint(e0) & 0xFFFFu, l1 = __float_as_uint(e1) & 0xFFFFu;
-        // (|log2 d| <= 20 keeps the error of norm * log2 d below 80 ulps of the result)
-        if ((d0 != 0.0f) && (((l0 - 0x7F40u) & 0xFFFFu) <= 0x180u || !(d0 > 9.6e-7f && d0 < 1.0e6f))) e0 = powf(d0, c.norm);
-        if ((d1 != 0.0f) && (((l1 - 0x7F40u) & 0xFFFFu) <= 0x180u || !(d1 > 9.6e-7f && d1 < 1.0e6f))) e1 = powf(d1, c.norm);
-        const uint32_t eb = bf2_pack(e1, e0);
-        err += __uint_as_float(eb << 16);
-        err += __uint_as_float(eb & 0xFFFF0000u);
-      }
-      for (int o = lanes >> 1; o > 0; o >>= 1) err += __shfl_xor_sync(0xffffffffu, err, o);
+      for (int k = 0; k < R; ++k) part[k] = chunk_error<KIND, SYM>(w[k], q, qmin2, qmax2, c, s_table);
+      float err = R == 4 ? (part[0] + part[R / 2]) + (part[R / 4] + part[R - 1]) : R == 2 ? part[0] + part[R - 1] : part[0];
+      for (int o = L >> 1; o > 0; o >>= 1) err += __shfl_xor_sync(0xffffffffu, err, o);
       err = bf16r(err);
       if (live && err < best_err) {
         best_err = err; best_mn = smn; best_mx = smx;
-        if (pass == 0 && (cc % lanes) == 0 && ((volatile int*)ctl)[1 + i] == 0) atomicOr(&ctl[1 + i], 1);
+        if (pass == 0 && j == 0 && ((volatile int*)ctl)[1 + i] == 0) atomicOr(&ctl[1 + i], 1);
       }
     }
-    if (live && (cc % lanes) == 0) {
-      int64_t gi = row * gpr + (cc * 8) / g;
+    if (live && j == 0) {
       ((T*)mn_out)[gi] = __float2bfloat16_rn(best_mn);
       ((T*)mx_out)[gi] = __float2bfloat16_rn(best_mx);
     }
   }
 }
+
+// CHANNEL and BLOCK strategies: a CTA per row or bh x bw block, kept packed in shared memory (blocks that stick out of
+// the matrix are completed with zeros, as in mse_tile_kernel).  Candidates are evaluated four at a time, so that the
+// CTA-wide sum costs a barrier for four.
+template <int KIND, bool SYM>
+__global__ void __launch_bounds__(256) mse_tile_bf16_kernel(const void* __restrict__ W, int64_t N, int64_t K, int64_t ldw,
+                                                            int bh, int bw, Cfg c, const __nv_bfloat16* __restrict__ table,
+                                                            int* __restrict__ ctl, int pass, void* __restrict__ mn_out,
+                                                            void* __restrict__ mx_out) {
+  using T = __nv_bfloat16;
+  extern __shared__ __align__(16) unsigned short s_table[];
+  uint4* data = reinterpret_cast<uint4*>(s_table + kTable);
+  __shared__ float s_part[2][8][4], s_lo[8], s_hi[8];
+  const int limit = (pass == 0) ? c.steps : ctl[0];
+  if (pass == 1 && limit >= c.steps) return;
+  load_table(reinterpret_cast<uint4*>(s_table), table);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int cw = bw >> 3, chunks = bh * cw;
+  const int64_t gpr = (K + bw - 1) / bw, groups = ((N + bh - 1) / bh) * gpr;
+  const uint32_t qmin2 = bf2_of(c.qmin), qmax2 = bf2_of(c.qmax);
+  for (int64_t grp = blockIdx.x; grp < groups; grp += gridDim.x) {
+    const int64_t r0 = (grp / gpr) * bh, c0 = (grp % gpr) * bw;
+    float lo = INFINITY, hi = -INFINITY;
+    for (int x = threadIdx.x; x < chunks; x += 256) {
+      const int y = x / cw;
+      const int64_t r = r0 + y, cc = c0 + (x - y * cw) * 8;
+      uint4 raw = make_uint4(0u, 0u, 0u, 0u);
+      if (r < N && cc < K) raw = __ldg(reinterpret_cast<const uint4*>((const T*)W + r * ldw + cc));
+      data[x] = raw;
+      chunk_range(raw, lo, hi);
+    }
+    lo = warp_min(lo); hi = warp_max(hi);
+    if (lane == 0) { s_lo[warp] = lo; s_hi[warp] = hi; }
+    __syncthreads();
+    for (int w = 0; w < 8; ++w) { lo = fminf(lo, s_lo[w]); hi = fmaxf(hi, s_hi[w]); }
+    const float mn = bf16r(lo * c.expand), mx = bf16r(hi * c.expand);
+    float best_err = 3.3895313892515355e38f, best_mn = mn, best_mx = mx;
+    for (int i0 = 0, turn = 0; i0 < limit; i0 += 4, turn ^= 1) {
+      Cand q[4];
+      float smn[4], smx[4], err[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float p = shrink_factor(i0 + k, c.grid);
+        smn[k] = bf16r(mn * p); smx[k] = bf16r(mx * p);
+        q[k] = make_cand(smn[k], smx[k], c);
+      }
+      for (int x = threadIdx.x; x < chunks; x += 256) {
+        const uint4 raw = data[x];
+        const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) err[k] += chunk_error<KIND, SYM>(w, q[k], qmin2, qmax2, c, s_table);
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        err[k] = warp_sum(err[k]);
+        if (lane == 0) s_part[turn][warp][k] = err[k];
+      }
+      __syncthreads();
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        float tot = 0.0f;
+        for (int w = 0; w < 8; ++w) tot += s_part[turn][w][k];
+        tot = bf16r(tot);
+        if (i0 + k < limit && tot < best_err) {
+          best_err = tot; best_mn = smn[k]; best_mx = smx[k];
+          if (pass == 0 && threadIdx.x == 0 && ((volatile int*)ctl)[1 + i0 + k] == 0) atomicOr(&ctl[1 + i0 + k], 1);
+        }
+      }
+    }
+    if (threadIdx.x == 0) {
+      ((T*)mn_out)[grp] = __float2bfloat16_rn(best_mn);
+      ((T*)mx_out)[grp] = __float2bfloat16_rn(best_mx);
+    }
+    __syncthreads();
+  }
+}
 #undef B200Q_BF2
+#undef B200Q_B
 
 // One CTA per group held in shared memory: a row (CHANNEL, bh = 1, bw = K) or a bh x bw block
 // (BLOCK; blocks that stick out of the matrix are completed with zeros, which take part in the
@@ -426,6 +565,32 @@ __global__ void clear_ctl_kernel(int* ctl, int n) {
   for (int i = threadIdx.x; i < n; i += blockDim.x) ctl[i] = 0;
 }
 
+// Blocks per SM of the table-driven kernels (the table takes 64 KiB of shared memory a block)
+constexpr int kTableBlocksPerSM = 3;
+
+template <int KIND, bool SYM>
+static int launch_group(const void* W, int64_t N, int64_t K, int64_t ldw, int g, const Cfg& c, const __nv_bfloat16* table,
+                        int* ctl, int pass, void* mn, void* mx, cudaStream_t st) {
+  const int chunks = g >> 3, r = chunks >= 4 ? 4 : chunks;
+  const int64_t slots = N * (K / g) * (chunks / r);
+  const int grid = grid_for((slots + 255) / 256, kTableBlocksPerSM);
+  auto kern = r == 4 ? mse_group_bf16_kernel<KIND, SYM, 4> : r == 2 ? mse_group_bf16_kernel<KIND, SYM, 2> : mse_group_bf16_kernel<KIND, SYM, 1>;
+  B200Q_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTableBytes));
+  kern<<<grid, 256, kTableBytes, st>>>(W, N, K, ldw, g, c, table, ctl, pass, mn, mx);
+  return B200Q_OK;
+}
+template <int KIND, bool SYM>
+static int launch_tile(const void* W, int64_t N, int64_t K, int64_t ldw, int bh, int bw, const Cfg& c,
+                       const __nv_bfloat16* table, int* ctl, int pass, void* mn, void* mx, cudaStream_t st) {
+  const size_t smem = kTableBytes + (size_t)bh * bw * 2;
+  const int64_t groups = ((N + bh - 1) / bh) * ((K + bw - 1) / bw);
+  const int per_sm = (int)(220 * 1024 / (smem + 1024));
+  auto kern = mse_tile_bf16_kernel<KIND, SYM>;
+  B200Q_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kern<<<grid_for(groups, per_sm < 1 ? 1 : per_sm), 256, smem, st>>>(W, N, K, ldw, bh, bw, c, table, ctl, pass, mn, mx);
+  return B200Q_OK;
+}
+
 }  // namespace mse
 }  // namespace b200q
 
@@ -440,16 +605,23 @@ int b200q_observe_mse_steps(double maxshrink, double grid) {
   return v > 2147483647.0 ? 2147483647 : (int)v;
 }
 
-size_t b200q_observe_mse_workspace_bytes(int64_t, int64_t, const b200q_qargs* qa, int steps) {
-  const size_t flags = sizeof(int) * (size_t)(steps + 1 > 1 ? steps + 1 : 1);
-  if (qa && qa->strategy == B200Q_TENSOR)   // search state and per-CTA partials
-    return flags + sizeof(float) * (size_t)(b200q::mse::kSpanState + 2 * 4 * b200q::kNumSMs);
-  return flags;
+static size_t mse_flag_bytes(int steps) {
+  return (sizeof(int) * (size_t)(steps + 1 > 1 ? steps + 1 : 1) + 255) / 256 * 256;
 }
 
-int b200q_observe_mse(const void* W, int wdtype, int64_t N, int64_t K, int64_t ldw, const b200q_qargs* qa,
-                      double maxshrink, int patience, double grid, float norm, float expand, void* mn_out,
-                      void* mx_out, void* scratch, void* stream) {
+size_t b200q_observe_mse_workspace_bytes(int64_t, int64_t, const b200q_qargs* qa, int steps) {
+  const size_t flags = mse_flag_bytes(steps);
+  if (qa && qa->strategy == B200Q_TENSOR)   // search state and per-CTA partials
+    return flags + sizeof(float) * (size_t)(b200q::mse::kSpanState + 2 * 4 * b200q::kNumSMs);
+  return flags + b200q::mse::kTableBytes + 256;   // (the table starts on a 16-byte boundary of whatever it is given)
+}
+
+}  // extern "C"
+
+// `table`: 64 KiB for the powers of bf16 errors, 16-byte aligned
+static int observe_mse(const void* W, int wdtype, int64_t N, int64_t K, int64_t ldw, const b200q_qargs* qa,
+                       double maxshrink, int patience, double grid, float norm, float expand, void* mn_out,
+                       void* mx_out, void* scratch, void* table_mem, void* stream) {
   using namespace b200q::mse;
   if (!W || !qa || !mn_out || !mx_out || !scratch || N <= 0 || K <= 0 || ldw < K) return B200Q_ERR_ARG;
   if (wdtype != B200Q_BF16 && wdtype != B200Q_F32) return B200Q_ERR_UNSUPPORTED;
@@ -459,6 +631,7 @@ int b200q_observe_mse(const void* W, int wdtype, int64_t N, int64_t K, int64_t l
   c.symmetric = qa->symmetric; c.scale_kind = qa->scale_kind; c.zp_kind = qa->zp_kind;
   c.mx_offset = (qa->num_bits == 4) ? 2 : 8;
   c.qmin = qr.qmin; c.qmax = qr.qmax; c.range = qr.qmax - qr.qmin; c.half_range = c.range / 2.0f; c.kind = qr.kind;
+  c.inv_half_range = 1.0f / c.half_range;
   if (!qa->symmetric && qr.kind == kFp4) return B200Q_ERR_UNSUPPORTED;
   if (qa->scale_kind == B200Q_SCALE_FP8) c.eps = 0.125f;
   else if (qa->scale_kind == B200Q_SCALE_E8M0) c.eps = 1.0f;
@@ -475,30 +648,41 @@ int b200q_observe_mse(const void* W, int wdtype, int64_t N, int64_t K, int64_t l
   if (c.steps < 0) return B200Q_ERR_ARG;
   cudaStream_t st = (cudaStream_t)stream;
   int* ctl = (int*)scratch;
-  clear_ctl_kernel<<<1, 128, 0, st>>>(ctl, c.steps + 1);
-  B200Q_LAUNCH_CHECK();
   const bool grp = qa->strategy == B200Q_GROUP || qa->strategy == B200Q_TENSOR_GROUP;
+  // bf16 weights in whole 16-byte pieces: the table-driven kernels
+  const bool blk = qa->strategy == B200Q_BLOCK;
+  const bool packed = wdtype == B200Q_BF16 && qa->strategy != B200Q_TENSOR && (K & 7) == 0 && (ldw & 7) == 0 &&
+                      (((uintptr_t)W) & 15) == 0 && (!blk || (qa->block_w > 0 && qa->block_w % 8 == 0)) &&
+                      (qr.kind != kInt || qa->num_bits == 4 || qa->num_bits == 8);
+  __nv_bfloat16* table = (__nv_bfloat16*)table_mem;
+  if (packed) make_table_kernel<<<kTable / 256, 256, 0, st>>>(table, c.norm, ctl, c.steps + 1);
+  else clear_ctl_kernel<<<1, 128, 0, st>>>(ctl, c.steps + 1);
+  B200Q_LAUNCH_CHECK();
+#define B200Q_MSE_PICK(fn, ...)                                                                                     \
+  do {                                                                                                              \
+    if (qr.kind == kFp8) rc = fn<kMseFp8, true>(__VA_ARGS__);                                                       \
+    else if (qr.kind == kFp4) rc = fn<kMseFp4, true>(__VA_ARGS__);                                                  \
+    else if (qa->num_bits == 4) rc = qa->symmetric ? fn<kMseInt4, true>(__VA_ARGS__) : fn<kMseInt4, false>(__VA_ARGS__); \
+    else rc = qa->symmetric ? fn<kMseInt8, true>(__VA_ARGS__) : fn<kMseInt8, false>(__VA_ARGS__);                    \
+    if (rc) return rc;                                                                                              \
+  } while (0)
   for (int pass = 0; pass < 2; ++pass) {
     if (grp) {
       int g = qa->group_size;
       if (!(g >= 8 && g <= 256 && (g & (g - 1)) == 0 && K % g == 0)) return B200Q_ERR_UNSUPPORTED;
       int grid_sz = grid_for((N * (K >> 3) + 255) / 256, 4);
-      const bool fast = wdtype == B200Q_BF16 && qr.kind == kInt && qa->scale_kind != B200Q_SCALE_FP8 &&
-                        qa->scale_kind != B200Q_SCALE_E8M0 && c.steps <= 1024 && (K & 7) == 0 && (ldw & 7) == 0 &&
-                        (((uintptr_t)W) & 15) == 0;
-      if (fast && qa->num_bits == 4) mse_group_bf16_int_kernel<true><<<grid_sz, 256, 0, st>>>(W, N, K, ldw, g, c, ctl, pass, mn_out, mx_out);
-      else if (fast) mse_group_bf16_int_kernel<false><<<grid_sz, 256, 0, st>>>(W, N, K, ldw, g, c, ctl, pass, mn_out, mx_out);
+      if (packed && (qa->symmetric || qr.kind == kInt)) B200Q_MSE_PICK(launch_group, W, N, K, ldw, g, c, table, ctl, pass, mn_out, mx_out, st);
       else if (wdtype == B200Q_BF16) mse_group_kernel<B200Q_BF16><<<grid_sz, 256, 0, st>>>(W, N, K, ldw, g, c, ctl, pass, mn_out, mx_out);
       else mse_group_kernel<B200Q_F32><<<grid_sz, 256, 0, st>>>(W, N, K, ldw, g, c, ctl, pass, mn_out, mx_out);
     } else if (qa->strategy == B200Q_CHANNEL || qa->strategy == B200Q_BLOCK) {
-      const bool blk = qa->strategy == B200Q_BLOCK;
       if (blk && (qa->block_h <= 0 || qa->block_w <= 0)) return B200Q_ERR_ARG;
       const int64_t bh = blk ? qa->block_h : 1, bw = blk ? qa->block_w : K;
       const size_t smem = (size_t)(bh * bw) * sizeof(float);
       if (bh * bw > (int64_t)50 * 1024) return B200Q_ERR_UNSUPPORTED;   // group does not fit in shared memory
       const int64_t groups = ((N + bh - 1) / bh) * ((K + bw - 1) / bw);
       int grid_sz = grid_for(groups, smem > 100 * 1024 ? 1 : 2);
-      if (wdtype == B200Q_BF16) {
+      if (packed && (qa->symmetric || qr.kind == kInt)) B200Q_MSE_PICK(launch_tile, W, N, K, ldw, (int)bh, (int)bw, c, table, ctl, pass, mn_out, mx_out, st);
+      else if (wdtype == B200Q_BF16) {
         B200Q_TRY(cudaFuncSetAttribute(mse_tile_kernel<B200Q_BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         mse_tile_kernel<B200Q_BF16><<<grid_sz, 256, smem, st>>>(W, N, K, ldw, (int)bh, (int)bw, c, ctl, pass, mn_out, mx_out);
       } else {
@@ -539,10 +723,20 @@ int b200q_observe_mse(const void* W, int wdtype, int64_t N, int64_t K, int64_t l
       B200Q_LAUNCH_CHECK();
     }
   }
+#undef B200Q_MSE_PICK
   return B200Q_OK;
 }
 
-}  // extern "C"
+extern "C" int b200q_observe_mse(const void* W, int wdtype, int64_t N, int64_t K, int64_t ldw, const b200q_qargs* qa,
+                                 double maxshrink, int patience, double grid, float norm, float expand, void* mn_out,
+                                 void* mx_out, void* scratch, void* stream) {
+  if (!scratch) return B200Q_ERR_ARG;
+  const int steps = b200q_observe_mse_steps(maxshrink, grid);
+  if (steps < 0) return B200Q_ERR_ARG;
+  const uintptr_t table = ((uintptr_t)scratch + mse_flag_bytes(steps) + 15) & ~(uintptr_t)15;
+  return observe_mse(W, wdtype, N, K, ldw, qa, maxshrink, patience, grid, norm, expand, mn_out, mx_out, scratch,
+                     (void*)table, stream);
+}
 
 // ---------------------------------------------------------------------------------------
 // Allocation-free variant of b200q_observe_mse.
@@ -558,14 +752,16 @@ namespace mse {
 
 constexpr int kStaticMaxSteps = 1023;  // candidates; the array holds kStaticMaxSteps + 1 ints (4 KiB)
 static __device__ __align__(256) int g_static_ctl[kStaticMaxSteps + 1];
+static __device__ __align__(256) __nv_bfloat16 g_static_table[kTable];   // powers of bf16 errors
 
 constexpr int kMaxDevices = 64;
 static int* g_static_ctl_ptr[kMaxDevices] = {nullptr};
+static void* g_static_table_ptr[kMaxDevices] = {nullptr};
 static std::mutex g_static_mutex;
 
-// Device address of the array on the current device.  In host code the symbol's name is only a
-// handle, not an address, so it is resolved once per device with cudaGetSymbolAddress.
-static int static_ctl_address(int** out) {
+// Device addresses of the arrays on the current device.  In host code the symbols' names are only
+// handles, not addresses, so they are resolved once per device with cudaGetSymbolAddress.
+static int static_addresses(int** out, void** table) {
   int dev = -1;
   B200Q_TRY(cudaGetDevice(&dev));
   if (dev < 0 || dev >= kMaxDevices) return B200Q_ERR_UNSUPPORTED;
@@ -574,9 +770,14 @@ static int static_ctl_address(int** out) {
     void* p = nullptr;
     B200Q_TRY(cudaGetSymbolAddress(&p, g_static_ctl));
     if (p == nullptr) return B200Q_ERR_CUDA;
+    void* t = nullptr;
+    B200Q_TRY(cudaGetSymbolAddress(&t, g_static_table));
+    if (t == nullptr) return B200Q_ERR_CUDA;
+    g_static_table_ptr[dev] = t;
     g_static_ctl_ptr[dev] = static_cast<int*>(p);
   }
   *out = g_static_ctl_ptr[dev];
+  *table = g_static_table_ptr[dev];
   return B200Q_OK;
 }
 
@@ -600,10 +801,11 @@ extern "C" int b200q_observe_mse_noalloc(const void* W, int wdtype, int64_t N, i
     return B200Q_ERR_UNSUPPORTED;
   }
   int* ctl = nullptr;
-  int rc = static_ctl_address(&ctl);
+  void* table = nullptr;
+  int rc = static_addresses(&ctl, &table);
   if (rc != B200Q_OK) return rc;
   // the search clears the flags it uses before its first pass, so the contents left by the
   // previous call do not matter
-  return b200q_observe_mse(W, wdtype, N, K, ldw, qa, maxshrink, patience, grid, norm, expand, mn_out, mx_out,
-                           ctl, stream);
+  return observe_mse(W, wdtype, N, K, ldw, qa, maxshrink, patience, grid, norm, expand, mn_out, mx_out, ctl, table,
+                     stream);
 }

@@ -200,37 +200,69 @@ static bool pow2(int v) { return v > 0 && (v & (v - 1)) == 0; }
 // ========================================================================================
 // observe_minmax (the streaming group kernels are in stream_kernels.cuh)
 // ========================================================================================
-// generic: one thread per qparam entry (group / block), any sizes
+// generic: one thread per group, any sizes
 template <int DT>
-__global__ void minmax_generic_kernel(const void* __restrict__ W, int64_t N, int64_t K, int64_t ldw,
-                                      int strategy, int g, int bh, int bw,
+__global__ void minmax_generic_kernel(const void* __restrict__ W, int64_t N, int64_t K, int64_t ldw, int g,
                                       void* __restrict__ mn_out, void* __restrict__ mx_out) {
   using E = Elem<DT>;
   using T = typename E::type;
-  int64_t gpr = (strategy == B200Q_BLOCK) ? (K + bw - 1) / bw : (K + g - 1) / g;
-  int64_t rows = (strategy == B200Q_BLOCK) ? (N + bh - 1) / bh : N;
-  int64_t total = rows * gpr;
+  const int64_t gpr = (K + g - 1) / g, total = N * gpr;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (int64_t)gridDim.x * blockDim.x) {
     int64_t r = i / gpr, c = i - r * gpr;
     float lo = INFINITY, hi = -INFINITY;
-    if (strategy == B200Q_BLOCK) {
-      // zero padding of ragged blocks takes part in the statistics
-      bool ragged = (r * bh + bh > N) || (c * bw + bw > K);
-      if (ragged) { lo = 0.0f; hi = 0.0f; }
-      for (int64_t y = r * bh; y < min((int64_t)(r * bh + bh), N); ++y)
-        for (int64_t x = c * bw; x < min((int64_t)(c * bw + bw), K); ++x) {
-          float v = E::load((const T*)W + y * ldw + x);
-          lo = fminf(lo, v); hi = fmaxf(hi, v);
-        }
-    } else {
-      for (int64_t x = c * g; x < min((int64_t)(c * g + g), K); ++x) {
-        float v = E::load((const T*)W + r * ldw + x);
-        lo = fminf(lo, v); hi = fmaxf(hi, v);
-      }
+    for (int64_t x = c * g; x < min((int64_t)(c * g + g), K); ++x) {
+      float v = E::load((const T*)W + r * ldw + x);
+      lo = fminf(lo, v); hi = fmaxf(hi, v);
     }
     E::store((T*)mn_out + i, lo);
     E::store((T*)mx_out + i, hi);
+  }
+}
+
+// BLOCK: a CTA per block (rows of the block over warps, 8 elements a lane, or an element a lane where the layout does
+// not allow more).  HBM-bound from a few hundred blocks on; a thread per block, which the generic kernel gives it, took
+// 1114 us for 128 x 128 blocks of 4096 x 4096.
+template <int DT, bool VEC>
+__global__ void __launch_bounds__(256) minmax_block_kernel(const void* __restrict__ W, int64_t N, int64_t K, int64_t ldw,
+                                                           int bh, int bw, int64_t blocks_per_row, int64_t blocks,
+                                                           void* __restrict__ mn_out, void* __restrict__ mx_out) {
+  using E = Elem<DT>;
+  using T = typename E::type;
+  __shared__ float s_lo[8], s_hi[8];
+  constexpr int PER = VEC ? 8 : 1;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int cw = bw / PER;
+  for (int64_t b = blockIdx.x; b < blocks; b += gridDim.x) {
+    const int64_t r0 = (b / blocks_per_row) * bh, c0 = (b % blocks_per_row) * bw;
+    const int rows = (int)min((int64_t)bh, N - r0), cols = (int)min((int64_t)bw, K - c0);
+    // zero padding of ragged blocks takes part in the statistics
+    const bool ragged = rows < bh || cols < bw;
+    float lo = ragged ? 0.0f : INFINITY, hi = ragged ? 0.0f : -INFINITY;
+    const T* base = (const T*)W + r0 * ldw + c0;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < rows * cw; i += 256) {
+      const int y = i / cw, x = (i - y * cw) * PER;
+      if (x >= cols) continue;
+      if constexpr (VEC) {
+        float v[8];
+        load8<DT>(base, (int64_t)y * ldw + x, v);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) { lo = fminf(lo, v[k]); hi = fmaxf(hi, v[k]); }
+      } else {
+        const float v = E::load(base + (int64_t)y * ldw + x);
+        lo = fminf(lo, v); hi = fmaxf(hi, v);
+      }
+    }
+    lo = warp_min(lo); hi = warp_max(hi);
+    if (lane == 0) { s_lo[warp] = lo; s_hi[warp] = hi; }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int w = 1; w < 8; ++w) { lo = fminf(lo, s_lo[w]); hi = fmaxf(hi, s_hi[w]); }
+      E::store((T*)mn_out + b, lo);
+      E::store((T*)mx_out + b, hi);
+    }
+    __syncthreads();
   }
 }
 
@@ -350,16 +382,19 @@ static int observe_minmax_impl(const void* W, int64_t N, int64_t K, int64_t ldw,
         }
       } else {
         int64_t total = N * ((K + g - 1) / g);
-        minmax_generic_kernel<DT><<<grid_for((total + 127) / 128, 8), 128, 0, st>>>(
-            W, N, K, ldw, qa->strategy, g, 1, 1, mn, mx);
+        minmax_generic_kernel<DT><<<grid_for((total + 127) / 128, 8), 128, 0, st>>>(W, N, K, ldw, g, mn, mx);
       }
       break;
     }
     case B200Q_BLOCK: {
       if (qa->block_h <= 0 || qa->block_w <= 0) return B200Q_ERR_ARG;
-      int64_t total = ((N + qa->block_h - 1) / qa->block_h) * ((K + qa->block_w - 1) / qa->block_w);
-      minmax_generic_kernel<DT><<<grid_for((total + 127) / 128, 8), 128, 0, st>>>(
-          W, N, K, ldw, qa->strategy, 1, qa->block_h, qa->block_w, mn, mx);
+      const int64_t per_row = (K + qa->block_w - 1) / qa->block_w;
+      const int64_t total = ((N + qa->block_h - 1) / qa->block_h) * per_row;
+      // (K % 8 == 0: a chunk of 8 is inside the matrix as a whole)
+      if (vec && qa->block_w % 8 == 0)
+        minmax_block_kernel<DT, true><<<grid_for(total, 8), 256, 0, st>>>(W, N, K, ldw, qa->block_h, qa->block_w, per_row, total, mn, mx);
+      else
+        minmax_block_kernel<DT, false><<<grid_for(total, 8), 256, 0, st>>>(W, N, K, ldw, qa->block_h, qa->block_w, per_row, total, mn, mx);
       break;
     }
     case B200Q_CHANNEL:
@@ -533,10 +568,10 @@ static int quant_launch(const void* W, int64_t N, int64_t K, int64_t ldw, const 
                           pm.g_idx == nullptr && (pm.group_size & 7) == 0) ||
                          (pm.strategy == B200Q_BLOCK && (pm.block_w & 7) == 0);
     // bf16 weights with per-group parameters in column order: lane / chunk split kernels.  The
-    // combinations that occur: a bf16 scale without a global scale, or a float32 scale with one
-    // (FP4 only); everything else takes the row kernel below.
-    if constexpr (XDT == B200Q_BF16 && MODE != kPackFake &&
-                  ((SDT == B200Q_BF16 && !GLOBAL) || (SDT == B200Q_F32 && GLOBAL && MODE == kPackFp4))) {
+    // combinations that occur: a bf16 scale without a global scale, or a scale with one (FP4 only: the
+    // observer's float32 scale, or the module's bf16 copy, with which the row kernel took 116 us for
+    // 14336 x 4096); everything else takes the row kernel below.
+    if constexpr (XDT == B200Q_BF16 && MODE != kPackFake && ((SDT == B200Q_BF16 && !GLOBAL) || (GLOBAL && MODE == kPackFp4))) {
       const int g = pm.group_size;
       if ((pm.strategy == B200Q_GROUP || pm.strategy == B200Q_TENSOR_GROUP) && pm.g_idx == nullptr && g >= 8 &&
           g <= 256 && (g & (g - 1)) == 0 && K % g == 0) {
@@ -752,6 +787,166 @@ __global__ void __launch_bounds__(256) rtn_channel_kernel(
   }
 }
 
+// ========================================================================================
+// Q(W * s) / s, one grid point of the AWQ search, for bf16 weights and integer codes
+// ========================================================================================
+// The chain of the element-wise formulation - scale and round to bf16, min / max of the group or row, qparams,
+// fake-quantise, divide by the scale in float32 and round - in one pass over the weight: 4 B of traffic an element
+// where the separate passes moved 30 (231 us for 4096 x 4096).
+struct ColScale { float s[8], rs[8]; };
+__device__ __forceinline__ void load_col_scale(const float* __restrict__ col, int64_t c, ColScale& k) {
+  const float4 a = __ldg(reinterpret_cast<const float4*>(col + c)), b = __ldg(reinterpret_cast<const float4*>(col + c) + 1);
+  k.s[0] = a.x; k.s[1] = a.y; k.s[2] = a.z; k.s[3] = a.w; k.s[4] = b.x; k.s[5] = b.y; k.s[6] = b.z; k.s[7] = b.w;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) k.rs[i] = __frcp_rn(k.s[i]);
+}
+__device__ __forceinline__ uint4 scale_chunk(const uint4& raw, const ColScale& k) {
+  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+  uint32_t o[4];
+#pragma unroll
+  for (int p = 0; p < 4; ++p)
+    o[p] = stream::cvt_bf16x2(__uint_as_float(w[p] & 0xFFFF0000u) * k.s[2 * p + 1], __uint_as_float(w[p] << 16) * k.s[2 * p]);
+  return make_uint4(o[0], o[1], o[2], o[3]);
+}
+// bf16(fq / s): the product with 1 / s is a few float32 ulps off the quotient, so it rounds to the same bf16 value
+// unless it lies within 16 ulps of a midpoint (or leaves the normal range): then the division is done
+__device__ __forceinline__ float unscale(float fq, float s, float rs) {
+  const float q = fq * rs, a = fabsf(q);
+  if (((__float_as_uint(q) & 0xFFFFu) - 0x7FF0u) > 0x20u && ((a < 1e30f && a > 1e-30f) || fq == 0.0f) && a == a) return q;
+  return __fdiv_rn(fq, s);
+}
+__device__ __forceinline__ uint32_t rint_bf16x2(uint32_t v, bool four_bit) {
+  if (four_bit) {   // integers are 1 apart in [128, 256)
+    const uint32_t magic = 0x43404340u;
+    const __nv_bfloat162 m = *reinterpret_cast<const __nv_bfloat162*>(&magic);
+    __nv_bfloat162 r = __hsub2_rn(__hadd2_rn(*reinterpret_cast<__nv_bfloat162*>(&v), m), m);
+    return *reinterpret_cast<uint32_t*>(&r);
+  }
+  __nv_bfloat162 r = h2rint(*reinterpret_cast<__nv_bfloat162*>(&v));
+  return *reinterpret_cast<uint32_t*>(&r);
+}
+__device__ __forceinline__ uint4 fake_quant_unscale(const uint4& ws, const stream::GroupQ& g, const QRange& qr, bool sym,
+                                                    bool four_bit, const ColScale& k) {
+  uint32_t fq[4];
+  if (g.slow) {
+    const uint32_t w[4] = {ws.x, ws.y, ws.z, ws.w};
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      float f[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float x = h ? __uint_as_float(w[p] & 0xFFFF0000u) : __uint_as_float(w[p] << 16);
+        f[h] = dequant_code<true>(quant_code<true>(x, g.se, g.z, qr), g.se, g.z);
+      }
+      fq[p] = stream::cvt_bf16x2(f[1], f[0]);
+    }
+  } else {
+    uint32_t v[4];
+    stream::quot8_bf16<false>(ws, g, v);
+    const uint32_t lo2 = stream::bf2_splat(qr.qmin), hi2 = stream::bf2_splat(qr.qmax), s2 = stream::bf2_splat(g.se);
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      if (!sym) v[p] = stream::bf2_add(v[p], g.z2);
+      const uint32_t sign = v[p] & 0x80008000u;     // rounding to zero keeps the sign
+      uint32_t q = rint_bf16x2(stream::bf2_min(stream::bf2_max(v[p], lo2), hi2), four_bit);
+      q = (q & 0x7FFF7FFFu) | sign;
+      __nv_bfloat162 d = *reinterpret_cast<__nv_bfloat162*>(&q);
+      if (!sym) d = __hsub2_rn(d, *reinterpret_cast<const __nv_bfloat162*>(&g.z2));
+      d = __hmul2_rn(d, *reinterpret_cast<const __nv_bfloat162*>(&s2));
+      fq[p] = *reinterpret_cast<uint32_t*>(&d);
+    }
+  }
+  uint32_t o[4];
+#pragma unroll
+  for (int p = 0; p < 4; ++p)
+    o[p] = stream::cvt_bf16x2(unscale(__uint_as_float(fq[p] & 0xFFFF0000u), k.s[2 * p + 1], k.rs[2 * p + 1]),
+                              unscale(__uint_as_float(fq[p] << 16), k.s[2 * p], k.rs[2 * p]));
+  return make_uint4(o[0], o[1], o[2], o[3]);
+}
+
+// GROUP: a thread owns a chunk of 8 columns and walks down the rows, so that its column scales and their reciprocals
+// stay in registers; the g / 8 lanes of a group shuffle.
+__global__ void __launch_bounds__(256) scaled_group_kernel(const void* __restrict__ W, int64_t N, int64_t K, int64_t ldw,
+                                                           int lanes, const float* __restrict__ col, QParamCfg qc, QRange qr,
+                                                           bool four_bit, void* __restrict__ out) {
+  using T = __nv_bfloat16;
+  const int64_t chunk = (int64_t)blockIdx.x * 32 + (threadIdx.x & 31), cpr = K >> 3;
+  const bool live = chunk < cpr;
+  ColScale k;
+  if (live) load_col_scale(col, chunk * 8, k);
+  const int64_t step = (int64_t)gridDim.y * 8;
+  int64_t row = (int64_t)blockIdx.y * 8 + (threadIdx.x >> 5);
+  uint4 next = make_uint4(0, 0, 0, 0);
+  if (live && row < N) next = stream::ldg_stream((const T*)W + row * ldw + chunk * 8);
+  for (; row < N; row += step) {
+    const uint4 raw = next;
+    if (live && row + step < N) next = stream::ldg_stream((const T*)W + (row + step) * ldw + chunk * 8);
+    uint4 ws = make_uint4(0, 0, 0, 0);
+    if (live) ws = scale_chunk(raw, k);
+    stream::RangeQ r;
+    r.first(ws);
+    float lo, hi;
+    r.finish(lo, hi);
+    for (int o = lanes >> 1; o > 0; o >>= 1) {
+      lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+      hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    float s, z;
+    qparams_one<true>(lo, hi, qc, 1.0f, s, z);
+    const stream::GroupQ gq = stream::make_group_q<true>(s, z + 0.0f);   // (a stored zero point has no -0)
+    if (live)
+      *reinterpret_cast<uint4*>((T*)out + row * K + chunk * 8) = fake_quant_unscale(ws, gq, qr, qc.symmetric != 0, four_bit, k);
+  }
+}
+// CHANNEL: a CTA per row, the scaled row in registers between the two halves (R chunks of 8 per thread)
+template <int R>
+__global__ void __launch_bounds__(256) scaled_channel_kernel(const void* __restrict__ W, int64_t N, int64_t K, int64_t ldw,
+                                                             const float* __restrict__ col, QParamCfg qc, QRange qr,
+                                                             bool four_bit, void* __restrict__ out) {
+  using T = __nv_bfloat16;
+  __shared__ float s_lo[2][8], s_hi[2][8];
+  const int cpr = (int)(K >> 3), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int par = 0;
+  for (int64_t row = blockIdx.x; row < N; row += gridDim.x, par ^= 1) {
+    uint4 ws[R];
+    stream::RangeQ r;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const int c = threadIdx.x + i * 256;
+      ws[i] = c < cpr ? stream::ldg_stream((const T*)W + row * ldw + (int64_t)c * 8) : make_uint4(0, 0, 0, 0);
+    }
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const int c = threadIdx.x + i * 256;
+      if (c < cpr) {
+        ColScale k;
+        load_col_scale(col, (int64_t)c * 8, k);
+        ws[i] = scale_chunk(ws[i], k);
+      }
+      if (i == 0) r.first(ws[0]); else r.add(ws[i]);
+    }
+    float lo, hi;
+    r.finish(lo, hi);
+    lo = warp_min(lo); hi = warp_max(hi);
+    if (lane == 0) { s_lo[par][warp] = lo; s_hi[par][warp] = hi; }
+    __syncthreads();   // one barrier per row: the buffers alternate
+#pragma unroll
+    for (int w = 0; w < 8; ++w) { lo = fminf(lo, s_lo[par][w]); hi = fmaxf(hi, s_hi[par][w]); }
+    float s, z;
+    qparams_one<true>(lo, hi, qc, 1.0f, s, z);
+    const stream::GroupQ gq = stream::make_group_q<true>(s, z + 0.0f);
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const int c = threadIdx.x + i * 256;
+      if (c < cpr) {
+        ColScale k;
+        load_col_scale(col, (int64_t)c * 8, k);
+        *reinterpret_cast<uint4*>((T*)out + row * K + (int64_t)c * 8) = fake_quant_unscale(ws[i], gq, qr, qc.symmetric != 0, four_bit, k);
+      }
+    }
+  }
+}
+
 }  // namespace b200q
 
 using namespace b200q;
@@ -862,6 +1057,41 @@ int b200q_quantize_pack(const void* W, int wdtype, int64_t N, int64_t K, int64_t
     return quant_dispatch<kPackFp4>(W, wdtype, N, K, ldw, scale, sdtype, zp, g_idx, gscale, qa, out, 0, st);
   }
   return B200Q_ERR_UNSUPPORTED;
+}
+
+int b200q_scaled_fake_quantize(const void* W, int wdtype, int64_t N, int64_t K, int64_t ldw, const float* col_scale,
+                               const b200q_qargs* qa, void* out, void* stream) {
+  if (!W || !col_scale || !qa || !out || N <= 0 || K <= 0 || ldw < K) return B200Q_ERR_ARG;
+  if (wdtype != B200Q_BF16 || qa->qtype != B200Q_QINT || (qa->num_bits != 4 && qa->num_bits != 8) ||
+      qa->scale_kind != B200Q_SCALE_PLAIN || !vec_ok(W, K, ldw, 2) || (((uintptr_t)out) % 16) || (((uintptr_t)col_scale) % 16))
+    return B200Q_ERR_UNSUPPORTED;
+  QParamCfg qc; QRange qr;
+  int rc = make_qparam_cfg(qa, true, false, &qc); if (rc) return rc;
+  rc = make_qrange(qa, &qr); if (rc) return rc;
+  cudaStream_t st = (cudaStream_t)stream;
+  const bool four = qa->num_bits == 4;
+  const int64_t cpr = K >> 3;
+  if (qa->strategy == B200Q_GROUP) {
+    const int g = qa->group_size;
+    if (!(pow2(g) && g >= 8 && g <= 256 && K % g == 0)) return B200Q_ERR_UNSUPPORTED;
+    const int64_t gx = (cpr + 31) / 32;
+    // enough CTAs to fill the machine, rows enough per CTA to earn the column scales' reciprocals
+    int64_t gy = (6 * kNumSMs + gx - 1) / gx;
+    if (gy > (N + 7) / 8) gy = (N + 7) / 8;
+    if (gx > 2147483647LL || gy > 65535) return B200Q_ERR_UNSUPPORTED;
+    scaled_group_kernel<<<dim3((unsigned)gx, (unsigned)gy), 256, 0, st>>>(W, N, K, ldw, g >> 3, col_scale, qc, qr, four, out);
+  } else if (qa->strategy == B200Q_CHANNEL) {
+    if (cpr > 8 * 256) return B200Q_ERR_UNSUPPORTED;
+    const int grid = grid_for(N, 6);
+    if (cpr <= 256) scaled_channel_kernel<1><<<grid, 256, 0, st>>>(W, N, K, ldw, col_scale, qc, qr, four, out);
+    else if (cpr <= 512) scaled_channel_kernel<2><<<grid, 256, 0, st>>>(W, N, K, ldw, col_scale, qc, qr, four, out);
+    else if (cpr <= 1024) scaled_channel_kernel<4><<<grid, 256, 0, st>>>(W, N, K, ldw, col_scale, qc, qr, four, out);
+    else scaled_channel_kernel<8><<<grid, 256, 0, st>>>(W, N, K, ldw, col_scale, qc, qr, four, out);
+  } else {
+    return B200Q_ERR_UNSUPPORTED;
+  }
+  B200Q_LAUNCH_CHECK();
+  return B200Q_OK;
 }
 
 int b200q_pack_zero_points(const int8_t* zp, int64_t N, int64_t G, int num_bits, int32_t* out, void* stream) {

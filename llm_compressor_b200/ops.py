@@ -152,6 +152,21 @@ def fake_quantize(w, scale, zp, args: QuantizationArgs, g_idx=None, global_scale
     return out
 
 
+def scaled_fake_quantize(w, col_scale: torch.Tensor, args: QuantizationArgs):
+    """Q(w * s) / s in one pass (see the header), or None for weights and schemes it does not take."""
+    _need_cuda(w, col_scale)
+    if w.dtype != torch.bfloat16 or col_scale.dtype != torch.float32 or not col_scale.is_contiguous():
+        return None
+    N, K, ld = _2d(w)
+    out = torch.empty((N, K), dtype=w.dtype, device=w.device)
+    rc = _lib.load().b200q_scaled_fake_quantize(ptr(w), _dt(w), N, K, ld, ptr(col_scale), args.c_struct(), ptr(out),
+                                                stream_ptr())
+    if rc == -2:
+        return None
+    check(rc, "b200q_scaled_fake_quantize")
+    return out
+
+
 def quantize_pack(w, scale, zp, args: QuantizationArgs, g_idx=None, global_scale=None,
                   pack_int8=False):
     """Storage codes: int32 words (int4, or int8 with pack_int8), int8 / float8 bytes, or
