@@ -83,6 +83,10 @@ size_t b200q_observe_minmax_workspace_bytes(int64_t N, int64_t K, const b200q_qa
 int b200q_observe_minmax(const void* W, int wdtype, int64_t N, int64_t K, int64_t ldw,
                          const b200q_qargs* qa, void* min_out, void* max_out, void* scratch,
                          void* stream);
+/* The same, and the weight's largest magnitude folded into *absmax (float, started at 0 by the caller): bf16 weights with
+ * grouped strategies (a power of two, 8..256); otherwise B200Q_ERR_UNSUPPORTED. */
+int b200q_observe_minmax_absmax(const void* W, int wdtype, int64_t N, int64_t K, int64_t ldw, const b200q_qargs* qa, void* mn,
+                                void* mx, void* scratch, float* absmax, void* stream);
 
 /* Largest magnitude over `count` min/max statistics, folded into *absmax (float, device);
  * call once per member of a fused q/k/v or gate/up group, with *absmax zeroed before the
@@ -142,6 +146,13 @@ int b200q_observe_mse_noalloc(const void* W, int wdtype, int64_t N, int64_t K, i
                               float norm, float expand, void* min_out, void* max_out, void* stream);
 
 /* ------------------------------------------------------------- quantize / pack */
+
+/* Statistics and parameters of a memoryless min-max observation in one pass: b200q_observe_minmax followed by
+ * b200q_qparams without a global scale, for one weight (W) or `count` weights of one shape (table: device array of
+ * pointers, 16-byte aligned).  bf16 weights in whole 16-byte pieces; GROUP (a power of two, 8..256), CHANNEL and
+ * BLOCK (width a multiple of 8); everything else returns B200Q_ERR_UNSUPPORTED.  scale_out: bf16 [count][entries]. */
+int b200q_minmax_qparams(const void* W, const void* const* table, int count, int wdtype, int64_t N, int64_t K, int64_t ldw,
+                         const b200q_qargs* qa, void* scale_out, void* zp_out, void* stream);
 
 /* Quantize-dequantize.  Replaces fake_quantize (CT/quantization/lifecycle/forward.py:149-181,
  * forward_helpers.py:113-210).  scale: [qparam shape] of dtype sdtype; zp may be NULL;
@@ -216,6 +227,8 @@ int b200q_hessian_syrk(const void* X, int64_t T, int64_t K, int64_t ldx, float* 
 /* H[i][j] = H[j][i] = H_lower[i][j] * scale for j <= i.  The division of
  * src/modifiers/gptq/base.py:336 (H / num_samples) is scale = 1/n. */
 int b200q_hessian_finalize(float* H, int64_t K, int64_t ldh, float scale, void* stream);
+/* The same for `count` matrices of one size: device arrays of pointers (16-byte aligned) and of scales. */
+int b200q_hessian_finalize_many(float* const* H, const float* scales, int count, int64_t K, int64_t ldh, void* stream);
 
 /* b200q_hessian_syrk splits long token ranges over several thread blocks per tile and adds the
  * partial tiles with floating-point atomics: H is then reproducible to rounding error (about 1e-7
@@ -247,6 +260,12 @@ int b200q_scatter_columns_cast(const float* Wf, int64_t N, int64_t K, int64_t ld
  * W[:,i]=0; then H_ii += percdamp * mean(diag H). */
 int b200q_gptq_prepare(float* H, int64_t K, int64_t ldh, float* Wf, int64_t N, int64_t ldf,
                        float percdamp, void* stream);
+/* What comes before `count` factorisations of one size (device array of pointers H): perm[i] (int32 [count][K],
+ * NULL: no reordering) = b200q_actorder_perm, diag[i] (float [count][K]) = the diagonal in that order, and
+ * out[i] (float [count][K][K]) = the permuted matrix with dead diagonal entries set to 1 and damping added; without
+ * perm that happens in place.  damp: float [count], scratch. */
+int b200q_gptq_prologue_many(float* const* H, int count, int64_t K, int64_t ldh, float percdamp, int32_t* perm, float* diag,
+                             float* damp, float* out, void* stream);
 /* W[:, i] = 0 where diag[i * diag_stride] == 0 (gptq_quantize.py:144-146), for modules that
  * share one Hessian (q/k/v, gate/up): `diag` is the diagonal saved before b200q_gptq_prepare. */
 int b200q_gptq_zero_dead_columns(const float* diag, int64_t diag_stride, int64_t K, float* Wf,

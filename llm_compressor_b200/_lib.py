@@ -49,6 +49,10 @@ SIGNATURES = {
     "b200q_take_wait_status": (_i, []),
     "b200q_observe_minmax_workspace_bytes": (C.c_size_t, [_i64, _i64, _qa]),
     "b200q_observe_minmax": (_i, [_p, _i, _i64, _i64, _i64, _qa, _p, _p, _p, _p]),
+    "b200q_observe_minmax_absmax": (_i, [_p, _i, _i64, _i64, _i64, _qa, _p, _p, _p, _p, _p]),
+    "b200q_minmax_qparams": (_i, [_p, _p, _i, _i, _i64, _i64, _i64, _qa, _p, _p, _p]),
+    "b200q_hessian_finalize_many": (_i, [_p, _p, _i, _i64, _i64, _p]),
+    "b200q_gptq_prologue_many": (_i, [_p, _i, _i64, _i64, _f, _p, _p, _p, _p, _p]),
     "b200q_absmax_accumulate": (_i, [_p, _p, _i, _i64, _p, _p]),
     "b200q_global_scale_finalize": (_i, [_p, _i, _p, _p]),
     "b200q_absmax_accumulate_weight": (_i, [_p, _i, _i64, _i64, _i64, _p, _p]),

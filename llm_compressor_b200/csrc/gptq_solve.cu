@@ -15,28 +15,38 @@ __device__ __forceinline__ uint32_t order_key(float d) {
   const uint32_t b = __float_as_uint(d + 0.0f);   // -0 + 0 = +0
   return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
 }
-__global__ void __launch_bounds__(256) perm_kernel(const float* __restrict__ H, int64_t K, int64_t ldh,
+// A CTA ranks 32 columns, its eight warps counting an eighth of the others each (one thread per column counted all
+// of them: 26 us at K = 1160).  blockIdx.y = problem.
+__global__ void __launch_bounds__(256) perm_kernel(const float* H0, const float* const* Hs, int64_t K, int64_t ldh,
                                                    int32_t* __restrict__ perm) {
   __shared__ uint32_t sd[1024];
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  __shared__ int s_rank[8][32];
+  const float* __restrict__ H = Hs ? Hs[blockIdx.y] : H0;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t i = (int64_t)blockIdx.x * 32 + lane;
   const uint32_t ki = (i < K) ? order_key(H[i * ldh + i]) : 0u;
   int rank = 0;
   for (int64_t j0 = 0; j0 < K; j0 += 1024) {
-    for (int t = threadIdx.x; t < 1024; t += blockDim.x) {
-      int64_t j = j0 + t;
+    for (int t = threadIdx.x; t < 1024; t += 256) {
+      const int64_t j = j0 + t;
       sd[t] = (j < K) ? order_key(H[j * ldh + j]) : 0u;
     }
     __syncthreads();
-    if (i < K) {
-      const int lim = (int)min((int64_t)1024, K - j0);
-      for (int t = 0; t < lim; ++t) {
-        const uint32_t kj = sd[t];
-        rank += (kj > ki) || (kj == ki && (j0 + t) < i);
-      }
+    const int lim = (int)min((int64_t)1024, K - j0);
+#pragma unroll 8
+    for (int t = warp; t < lim; t += 8) {
+      const uint32_t kj = sd[t];
+      rank += (kj > ki) || (kj == ki && (j0 + t) < i);
     }
     __syncthreads();
   }
-  if (i < K) perm[rank] = (int32_t)i;
+  s_rank[warp][lane] = rank;
+  __syncthreads();
+  if (warp == 0 && i < K) {
+#pragma unroll
+    for (int w = 1; w < 8; ++w) rank += s_rank[w][lane];
+    perm[blockIdx.y * K + rank] = (int32_t)i;
+  }
 }
 
 // column index taken from a caller-supplied permutation, kept inside the matrix
@@ -110,6 +120,55 @@ __global__ void permute_hessian_kernel(const float* __restrict__ H, int64_t K, i
   }
 }
 
+// The prologue of many factorisations of one size: per problem (blockIdx.y) the diagonal in the new order, the damping
+// (summed in that order, as damp_kernel does on the permuted matrix) ...
+__global__ void __launch_bounds__(1024) diag_damp_kernel(const float* const* __restrict__ Hs, int64_t K, int64_t ldh,
+                                                         const int32_t* __restrict__ perm, float percdamp,
+                                                         float* __restrict__ diag, float* __restrict__ damp) {
+  __shared__ float s_part[32];
+  const float* H = Hs[blockIdx.y];
+  const int32_t* pm = perm ? perm + blockIdx.y * K : nullptr;
+  float sum = 0.0f;
+  for (int64_t i = threadIdx.x; i < K; i += 1024) {
+    const int64_t r = pm ? pm[i] : i;
+    const float d = H[r * ldh + r];
+    diag[blockIdx.y * K + i] = d;
+    sum += d == 0.0f ? 1.0f : d;
+  }
+  sum = warp_sum(sum);
+  if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = sum;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const float v = warp_sum(s_part[threadIdx.x]);
+    if (threadIdx.x == 0) damp[blockIdx.y] = percdamp * (v / (float)K);
+  }
+}
+// ... and the matrix: out[r][c] = H[perm r][perm c], dead diagonal entries 1, damping added.  In place without a
+// permutation, where only the diagonal changes.
+__global__ void __launch_bounds__(256) permute_damp_kernel(float* const* __restrict__ Hs, int64_t K, int64_t ldh,
+                                                           const int32_t* __restrict__ perm, const float* __restrict__ damp,
+                                                           float* __restrict__ out) {
+  const float* H = Hs[blockIdx.y];
+  const float dm = damp[blockIdx.y];
+  if (!perm) {
+    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < K; i += (int64_t)gridDim.x * 256) {
+      const float d = H[i * ldh + i];
+      Hs[blockIdx.y][i * ldh + i] = (d == 0.0f ? 1.0f : d) + dm;
+    }
+    return;
+  }
+  const int32_t* pm = perm + blockIdx.y * K;
+  float* o = out + blockIdx.y * K * K;
+  for (int64_t r = blockIdx.x; r < K; r += gridDim.x) {
+    const float* row = H + (int64_t)pm[r] * ldh;
+    for (int64_t c = threadIdx.x; c < K; c += 256) {
+      float v = row[pm[c]];
+      if (c == r) v = (v == 0.0f ? 1.0f : v) + dm;
+      o[r * K + c] = v;
+    }
+  }
+}
+
 template <int DT>
 __global__ void scatter_cols_kernel(const float* __restrict__ Wf, int64_t N, int64_t K, int64_t ldf,
                                     const int32_t* __restrict__ perm, void* __restrict__ out, int64_t ldo) {
@@ -169,7 +228,23 @@ extern "C" {
 
 int b200q_actorder_perm(const float* H, int64_t K, int64_t ldh, int32_t* perm, void* stream) {
   if (!H || !perm || K <= 0 || ldh < K) return B200Q_ERR_ARG;
-  perm_kernel<<<(int)((K + 255) / 256), 256, 0, (cudaStream_t)stream>>>(H, K, ldh, perm);
+  perm_kernel<<<(int)((K + 31) / 32), 256, 0, (cudaStream_t)stream>>>(H, nullptr, K, ldh, perm);
+  B200Q_LAUNCH_CHECK();
+  return B200Q_OK;
+}
+
+int b200q_gptq_prologue_many(float* const* H, int count, int64_t K, int64_t ldh, float percdamp, int32_t* perm, float* diag,
+                             float* damp, float* out, void* stream) {
+  if (!H || !diag || !damp || count <= 0 || count > 65535 || K <= 0 || ldh < K || (perm && !out)) return B200Q_ERR_ARG;
+  cudaStream_t st = (cudaStream_t)stream;
+  if (perm) {
+    perm_kernel<<<dim3((unsigned)((K + 31) / 32), (unsigned)count), 256, 0, st>>>(nullptr, H, K, ldh, perm);
+    B200Q_LAUNCH_CHECK();
+  }
+  diag_damp_kernel<<<dim3(1, (unsigned)count), 1024, 0, st>>>(H, K, ldh, perm, percdamp, diag, damp);
+  B200Q_LAUNCH_CHECK();
+  const int64_t need = perm ? K : (K + 255) / 256, cap = 8 * kNumSMs / count + 1;
+  permute_damp_kernel<<<dim3((unsigned)(need < cap ? need : cap), (unsigned)count), 256, 0, st>>>(H, K, ldh, perm, damp, out);
   B200Q_LAUNCH_CHECK();
   return B200Q_OK;
 }

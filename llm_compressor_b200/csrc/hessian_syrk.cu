@@ -668,33 +668,72 @@ syrk_pair_kernel(const __grid_constant__ CUtensorMap xmap, Params p) {
   }
 }
 
-// H[i][j] = H[j][i] = scale * H[i][j] for j <= i, by 32x32 blocks through shared memory.
-__global__ void __launch_bounds__(256) finalize_kernel(float* __restrict__ H, int64_t K, int64_t ldh,
-                                                       float scale) {
-  __shared__ float tile[32][33];
-  const int nb = (int)((K + 31) / 32);
+// H[i][j] = H[j][i] = scale * H[i][j] for j <= i, by 64 x 64 blocks through shared memory (a quarter of the bytes of
+// a block row is one 128-byte line of the mirrored half as well).  HBM-bound: the lower half is read, the whole
+// matrix written.  For one matrix, or (Hs, scales) a batch: blockIdx.y = matrix.
+constexpr int kFinTile = 64;
+__global__ void __launch_bounds__(256) finalize_kernel(float* H0, float* const* Hs, const float* scales, int64_t K, int64_t ldh,
+                                                       float scale, bool vec) {
+  __shared__ float tile[kFinTile][kFinTile + 1];
+  float* H = Hs ? Hs[blockIdx.y] : H0;
+  if (scales) scale = scales[blockIdx.y];
+  const int nb = (int)((K + kFinTile - 1) / kFinTile);
   const int64_t nblk = (int64_t)nb * (nb + 1) / 2;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;   // 16 quads of columns x 16 rows
   for (int64_t blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
     // blk -> (bi >= bj)
-    int bi = (int)((sqrt(8.0 * (double)blk + 1.0) - 1.0) * 0.5);
+    int bi = (int)((sqrtf(8.0f * (float)blk + 1.0f) - 1.0f) * 0.5f);
     while ((int64_t)bi * (bi + 1) / 2 > blk) --bi;
     while ((int64_t)(bi + 1) * (bi + 2) / 2 <= blk) ++bi;
     const int bj = (int)(blk - (int64_t)bi * (bi + 1) / 2);
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    for (int r = ty; r < 32; r += 8) {
-      int64_t i = (int64_t)bi * 32 + r, j = (int64_t)bj * 32 + tx;
-      float v = 0.0f;
-      if (i < K && j < K) {
-        v = H[i * ldh + j] * scale;
-        if (bi != bj || j <= i) H[i * ldh + j] = v;
+    float4 v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int64_t i = (int64_t)bi * kFinTile + ty + 16 * k, j = (int64_t)bj * kFinTile + tx * 4;
+      v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (i < K) {
+        if (vec && j + 3 < K) v[k] = *reinterpret_cast<const float4*>(H + i * ldh + j);
+        else {
+          float* e = &v[k].x;
+          for (int q = 0; q < 4; ++q)
+            if (j + q < K) e[q] = H[i * ldh + j + q];
+        }
       }
-      tile[r][tx] = v;
+      v[k].x *= scale; v[k].y *= scale; v[k].z *= scale; v[k].w *= scale;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      float* t = &tile[ty + 16 * k][tx * 4];
+      t[0] = v[k].x; t[1] = v[k].y; t[2] = v[k].z; t[3] = v[k].w;
     }
     __syncthreads();
-    for (int r = ty; r < 32; r += 8) {
-      // element (j-block row r, i-block col tx) of the mirrored block
-      int64_t j = (int64_t)bj * 32 + r, i = (int64_t)bi * 32 + tx;
-      if (i < K && j < K && (bi != bj || j < i)) H[j * ldh + i] = tile[tx][r];
+    if (bi == bj) {   // what lies above the diagonal comes from below it
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        float* e = &v[k].x;
+        const int y = ty + 16 * k;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (tx * 4 + q > y) e[q] = tile[tx * 4 + q][y];
+      }
+    }
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      if (half == 1 && bi == bj) break;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int y = ty + 16 * k;
+        float4 o = v[k];
+        if (half == 1) o = make_float4(tile[tx * 4][y], tile[tx * 4 + 1][y], tile[tx * 4 + 2][y], tile[tx * 4 + 3][y]);
+        const int64_t i = (int64_t)(half ? bj : bi) * kFinTile + y, j = (int64_t)(half ? bi : bj) * kFinTile + tx * 4;
+        if (i >= K) continue;
+        if (vec && j + 3 < K) *reinterpret_cast<float4*>(H + i * ldh + j) = o;
+        else {
+          const float* e = &o.x;
+          for (int q = 0; q < 4; ++q)
+            if (j + q < K) H[i * ldh + j + q] = e[q];
+        }
+      }
     }
     __syncthreads();
   }
@@ -881,13 +920,25 @@ int b200q_hessian_syrk(const void* X, int64_t T, int64_t K, int64_t ldx, float* 
 void b200q_set_reproducible(int on) { g_reproducible.store(on ? 1 : 0, std::memory_order_relaxed); }
 int b200q_get_reproducible(void) { return g_reproducible.load(std::memory_order_relaxed); }
 
-int b200q_hessian_finalize(float* H, int64_t K, int64_t ldh, float scale, void* stream) {
-  if (!H || K <= 0 || ldh < K) return B200Q_ERR_ARG;
-  int64_t nb = (K + 31) / 32;
-  int64_t nblk = nb * (nb + 1) / 2;
-  b200q::syrk::finalize_kernel<<<grid_for(nblk, 8), 256, 0, (cudaStream_t)stream>>>(H, K, ldh, scale);
+static int finalize(float* H, float* const* Hs, const float* scales, int count, int64_t K, int64_t ldh, float scale,
+                    void* stream) {
+  using namespace b200q::syrk;
+  const int64_t nb = (K + kFinTile - 1) / kFinTile, nblk = nb * (nb + 1) / 2, cap = 8 * kNumSMs / count + 1;
+  const bool vec = (ldh & 3) == 0 && (Hs || (((uintptr_t)H) & 15) == 0);   // (a batch's matrices are whole allocations)
+  finalize_kernel<<<dim3((unsigned)(nblk < cap ? nblk : cap), (unsigned)count), 256, 0, (cudaStream_t)stream>>>(
+      H, Hs, scales, K, ldh, scale, vec);
   B200Q_LAUNCH_CHECK();
   return B200Q_OK;
+}
+
+int b200q_hessian_finalize(float* H, int64_t K, int64_t ldh, float scale, void* stream) {
+  if (!H || K <= 0 || ldh < K) return B200Q_ERR_ARG;
+  return finalize(H, nullptr, nullptr, 1, K, ldh, scale, stream);
+}
+
+int b200q_hessian_finalize_many(float* const* H, const float* scales, int count, int64_t K, int64_t ldh, void* stream) {
+  if (!H || !scales || count <= 0 || count > 65535 || K <= 0 || ldh < K) return B200Q_ERR_ARG;
+  return finalize(nullptr, H, scales, count, K, ldh, 1.0f, stream);
 }
 
 }  // extern "C"

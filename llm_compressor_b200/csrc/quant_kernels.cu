@@ -355,9 +355,10 @@ constexpr int kTensorPartialBlocks = kNumSMs * 4;
 
 template <int DT>
 static int observe_minmax_impl(const void* W, int64_t N, int64_t K, int64_t ldw,
-                               const b200q_qargs* qa, void* mn, void* mx, void* scratch,
+                               const b200q_qargs* qa, void* mn, void* mx, void* scratch, float* absmax,
                                cudaStream_t st) {
   const bool vec = vec_ok(W, K, ldw, 2);
+  if (absmax && qa->strategy != B200Q_GROUP && qa->strategy != B200Q_TENSOR_GROUP) return B200Q_ERR_UNSUPPORTED;
   switch (qa->strategy) {
     case B200Q_GROUP:
     case B200Q_TENSOR_GROUP: {
@@ -372,15 +373,17 @@ static int observe_minmax_impl(const void* W, int64_t N, int64_t K, int64_t ldw,
           const int rows2 = stream::kThreads / tx2;
           const int grid2 = grid_for((N + rows2 - 1) / rows2, 8);
           const int txl2 = __builtin_ctz(tx2), ll2 = __builtin_ctz(gsp.L);
-          if (gsp.R == 8) stream::minmax_group_bf16_kernel<8><<<grid2, stream::kThreads, 0, st>>>(W, (int)N, (int)K, ldw, g, ll2, txl2, mn, mx);
-          else if (gsp.R == 4) stream::minmax_group_bf16_kernel<4><<<grid2, stream::kThreads, 0, st>>>(W, (int)N, (int)K, ldw, g, ll2, txl2, mn, mx);
-          else if (gsp.R == 2) stream::minmax_group_bf16_kernel<2><<<grid2, stream::kThreads, 0, st>>>(W, (int)N, (int)K, ldw, g, ll2, txl2, mn, mx);
-          else stream::minmax_group_bf16_kernel<1><<<grid2, stream::kThreads, 0, st>>>(W, (int)N, (int)K, ldw, g, ll2, txl2, mn, mx);
+          if (gsp.R == 8) stream::minmax_group_bf16_kernel<8><<<grid2, stream::kThreads, 0, st>>>(W, (int)N, (int)K, ldw, g, ll2, txl2, mn, mx, absmax);
+          else if (gsp.R == 4) stream::minmax_group_bf16_kernel<4><<<grid2, stream::kThreads, 0, st>>>(W, (int)N, (int)K, ldw, g, ll2, txl2, mn, mx, absmax);
+          else if (gsp.R == 2) stream::minmax_group_bf16_kernel<2><<<grid2, stream::kThreads, 0, st>>>(W, (int)N, (int)K, ldw, g, ll2, txl2, mn, mx, absmax);
+          else stream::minmax_group_bf16_kernel<1><<<grid2, stream::kThreads, 0, st>>>(W, (int)N, (int)K, ldw, g, ll2, txl2, mn, mx, absmax);
         } else {
+          if (absmax) return B200Q_ERR_UNSUPPORTED;
           stream::RowTiling t = stream::make_tiling(N, K, 8);
           stream::minmax_group_kernel<DT><<<t.grid, stream::kThreads, 0, st>>>(W, (int)N, (int)K, ldw, g, __builtin_ctz(t.tx), mn, mx);
         }
       } else {
+        if (absmax) return B200Q_ERR_UNSUPPORTED;
         int64_t total = N * ((K + g - 1) / g);
         minmax_generic_kernel<DT><<<grid_for((total + 127) / 128, 8), 128, 0, st>>>(W, N, K, ldw, g, mn, mx);
       }
@@ -500,6 +503,89 @@ __global__ void qparams_kernel(const void* __restrict__ mn, const void* __restri
     if (GLOBAL) ((float*)scale_out)[i] = s;
     else E::store((T*)scale_out + i, s);
     if (zp_out) store_zp(zp_out, c.zp_kind, i, z);
+  }
+}
+
+// ========================================================================================
+// statistics -> qparams in one pass, for one weight or a batch of weights of one shape
+// ========================================================================================
+// What min / max and qparams kernels do one after the other for a memoryless min-max observer, without the statistics
+// in between: bf16 weights in 16-byte pieces, the scale in the weight's dtype.  blockIdx.y = weight.
+struct StatJob {
+  const void* one; const void* const* table;   // the weight, or a device array of them
+  void* scale; void* zp;                       // [count][entries], contiguous
+  int64_t entries;
+  __device__ __forceinline__ const __nv_bfloat16* weight() const { return (const __nv_bfloat16*)(table ? table[blockIdx.y] : one); }
+  __device__ __forceinline__ void put(int64_t i, float lo, float hi, const QParamCfg& c) const {
+    float s, z;
+    qparams_one<true>(lo, hi, c, 1.0f, s, z);
+    const int64_t at = blockIdx.y * entries + i;
+    ((__nv_bfloat16*)scale)[at] = __float2bfloat16_rn(s);
+    if (zp) store_zp(zp, c.zp_kind, at, z);
+  }
+};
+// groups of R * L chunks: the lane / chunk split of the fused round-to-nearest kernel
+template <int R>
+__global__ void __launch_bounds__(256) group_qparams_kernel(StatJob j, int N, int K, int64_t ldw, int l_log2, int tx_log2,
+                                                            QParamCfg qc) {
+  const int TX = 1 << tx_log2, rows = 256 >> tx_log2, L = 1 << l_log2;
+  const int tx = threadIdx.x & (TX - 1), ty = threadIdx.x >> tx_log2;
+  const int cpg = R << l_log2, gpr = (K >> 3) / cpg, slots = gpr << l_log2, send = (slots + 31) & ~31;
+  const __nv_bfloat16* W = j.weight();
+  for (int row = blockIdx.x * rows + ty; row < N; row += gridDim.x * rows) {
+    const __nv_bfloat16* wrow = W + (int64_t)row * ldw;
+    for (int t = tx; t < send; t += TX) {
+      const bool live = t < slots;
+      const int grp = t >> l_log2, ln = t & (L - 1);
+      const int c0 = grp * cpg + ln;
+      uint4 raw[R];
+#pragma unroll
+      for (int k = 0; k < R; ++k)
+        raw[k] = live ? stream::ldg_stream(wrow + (int64_t)(c0 + k * L) * 8) : make_uint4(0, 0, 0, 0);
+      stream::RangeQ r;
+      r.first(raw[0]);
+#pragma unroll
+      for (int k = 1; k < R; ++k) r.add(raw[k]);
+      float lo, hi;
+      r.finish(lo, hi);
+      for (int o = L >> 1; o > 0; o >>= 1) {
+        lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+      }
+      if (live && ln == 0) j.put((int64_t)row * gpr + grp, lo, hi, qc);
+    }
+  }
+}
+// rows (bh = 1, bw = K) or bh x bw blocks: a CTA each
+__global__ void __launch_bounds__(256) span_qparams_kernel(StatJob j, int64_t N, int64_t K, int64_t ldw, int bh, int bw,
+                                                           int64_t per_row, int64_t spans, QParamCfg qc) {
+  __shared__ float s_lo[2][8], s_hi[2][8];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, cw = bw >> 3;
+  const __nv_bfloat16* W = j.weight();
+  int par = 0;
+  for (int64_t b = blockIdx.x; b < spans; b += gridDim.x, par ^= 1) {
+    const int64_t br = b / per_row, r0 = br * bh, c0 = (b - br * per_row) * bw;
+    const int rows = (int)min((int64_t)bh, N - r0), cols = (int)min((int64_t)bw, K - c0);
+    const __nv_bfloat16* base = W + r0 * ldw + c0;
+    // (the zero padding of ragged blocks changes nothing: the range is made to contain zero anyway)
+    float lo = 0.0f, hi = 0.0f;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < rows * cw; i += 256) {
+      const int y = i / cw, x = (i - y * cw) * 8;
+      if (x >= cols) continue;
+      stream::RangeQ r;
+      r.first(stream::ldg_stream(base + (int64_t)y * ldw + x));
+      float l, h;
+      r.finish(l, h);
+      lo = fminf(lo, l); hi = fmaxf(hi, h);
+    }
+    lo = warp_min(lo); hi = warp_max(hi);
+    if (lane == 0) { s_lo[par][warp] = lo; s_hi[par][warp] = hi; }
+    __syncthreads();   // one barrier per span: the buffers alternate
+    if (threadIdx.x == 0) {
+      for (int w = 1; w < 8; ++w) { lo = fminf(lo, s_lo[par][w]); hi = fmaxf(hi, s_hi[par][w]); }
+      j.put(b, lo, hi, qc);
+    }
   }
 }
 
@@ -973,13 +1059,18 @@ size_t b200q_observe_minmax_workspace_bytes(int64_t, int64_t, const b200q_qargs*
   return (qa && qa->strategy == B200Q_TENSOR) ? sizeof(float) * 2 * kTensorPartialBlocks : 0;
 }
 
-int b200q_observe_minmax(const void* W, int wdtype, int64_t N, int64_t K, int64_t ldw,
-                         const b200q_qargs* qa, void* mn, void* mx, void* scratch, void* stream) {
+int b200q_observe_minmax_absmax(const void* W, int wdtype, int64_t N, int64_t K, int64_t ldw, const b200q_qargs* qa, void* mn,
+                                void* mx, void* scratch, float* absmax, void* stream) {
   if (!W || !qa || !mn || !mx || N <= 0 || K <= 0 || ldw < K) return B200Q_ERR_ARG;
   cudaStream_t st = (cudaStream_t)stream;
-  if (wdtype == B200Q_BF16) return observe_minmax_impl<B200Q_BF16>(W, N, K, ldw, qa, mn, mx, scratch, st);
-  if (wdtype == B200Q_F32) return observe_minmax_impl<B200Q_F32>(W, N, K, ldw, qa, mn, mx, scratch, st);
+  if (wdtype == B200Q_BF16) return observe_minmax_impl<B200Q_BF16>(W, N, K, ldw, qa, mn, mx, scratch, absmax, st);
+  if (wdtype == B200Q_F32) return observe_minmax_impl<B200Q_F32>(W, N, K, ldw, qa, mn, mx, scratch, absmax, st);
   return B200Q_ERR_UNSUPPORTED;
+}
+
+int b200q_observe_minmax(const void* W, int wdtype, int64_t N, int64_t K, int64_t ldw,
+                         const b200q_qargs* qa, void* mn, void* mx, void* scratch, void* stream) {
+  return b200q_observe_minmax_absmax(W, wdtype, N, K, ldw, qa, mn, mx, scratch, nullptr, stream);
 }
 
 int b200q_absmax_accumulate(const void* mn, const void* mx, int dtype, int64_t count, float* absmax,
@@ -1026,6 +1117,46 @@ int b200q_qparams(const void* mn, const void* mx, int stat_dtype, int64_t count,
     if (gscale) qparams_kernel<B200Q_F32, true><<<grid, 256, 0, st>>>(mn, mx, count, c, gscale, scale_out, zp_out);
     else qparams_kernel<B200Q_F32, false><<<grid, 256, 0, st>>>(mn, mx, count, c, gscale, scale_out, zp_out);
   } else return B200Q_ERR_UNSUPPORTED;
+  B200Q_LAUNCH_CHECK();
+  return B200Q_OK;
+}
+
+int b200q_minmax_qparams(const void* W, const void* const* table, int count, int wdtype, int64_t N, int64_t K, int64_t ldw,
+                         const b200q_qargs* qa, void* scale_out, void* zp_out, void* stream) {
+  if ((!W && !table) || !qa || !scale_out || count <= 0 || count > 65535 || N <= 0 || K <= 0 || ldw < K) return B200Q_ERR_ARG;
+  if (wdtype != B200Q_BF16 || !vec_ok(W, K, ldw, 2) || N >= (1 << 30) || K >= (1 << 30)) return B200Q_ERR_UNSUPPORTED;
+  QParamCfg qc;
+  int rc = make_qparam_cfg(qa, true, false, &qc); if (rc) return rc;
+  cudaStream_t st = (cudaStream_t)stream;
+  StatJob j;
+  j.one = W; j.table = table; j.scale = scale_out; j.zp = zp_out;
+  const int cap = count > 1 ? 8 * kNumSMs / count + 1 : 8 * kNumSMs;
+  auto grid = [&](int64_t need) { return dim3((unsigned)(need < cap ? need : cap), (unsigned)count, 1); };
+  if (qa->strategy == B200Q_GROUP) {
+    const int g = qa->group_size;
+    if (!(pow2(g) && g >= 8 && g <= 256 && K % g == 0)) return B200Q_ERR_UNSUPPORTED;
+    j.entries = N * (K / g);
+    const stream::GroupSplit gsp = stream::make_group_split(g);
+    const int64_t slots = (K / g) * gsp.L;
+    int tx = 32;
+    while (tx < 256 && tx < slots) tx <<= 1;
+    const dim3 gd = grid((N + 256 / tx - 1) / (256 / tx));
+    const int ll = __builtin_ctz(gsp.L), txl = __builtin_ctz(tx);
+    if (gsp.R == 8) group_qparams_kernel<8><<<gd, 256, 0, st>>>(j, (int)N, (int)K, ldw, ll, txl, qc);
+    else if (gsp.R == 4) group_qparams_kernel<4><<<gd, 256, 0, st>>>(j, (int)N, (int)K, ldw, ll, txl, qc);
+    else if (gsp.R == 2) group_qparams_kernel<2><<<gd, 256, 0, st>>>(j, (int)N, (int)K, ldw, ll, txl, qc);
+    else group_qparams_kernel<1><<<gd, 256, 0, st>>>(j, (int)N, (int)K, ldw, ll, txl, qc);
+  } else if (qa->strategy == B200Q_CHANNEL || qa->strategy == B200Q_BLOCK) {
+    const bool blk = qa->strategy == B200Q_BLOCK;
+    if (blk && (qa->block_h <= 0 || qa->block_w <= 0 || qa->block_w % 8)) return B200Q_ERR_UNSUPPORTED;
+    const int bh = blk ? qa->block_h : 1, bw = blk ? qa->block_w : (int)K;
+    if ((int64_t)bh * bw >= (1LL << 31)) return B200Q_ERR_UNSUPPORTED;
+    const int64_t per_row = (K + bw - 1) / bw;
+    j.entries = ((N + bh - 1) / bh) * per_row;
+    span_qparams_kernel<<<grid(j.entries), 256, 0, st>>>(j, N, K, ldw, bh, bw, per_row, j.entries, qc);
+  } else {
+    return B200Q_ERR_UNSUPPORTED;
+  }
   B200Q_LAUNCH_CHECK();
   return B200Q_OK;
 }

@@ -657,7 +657,10 @@ template <int R>
 __global__ void __launch_bounds__(kThreads) minmax_group_bf16_kernel(const void* __restrict__ W, int N, int K,
                                                                      int64_t ldw, int g, int l_log2, int tx_log2,
                                                                      void* __restrict__ mn_out,
-                                                                     void* __restrict__ mx_out) {
+                                                                     void* __restrict__ mx_out,
+                                                                     float* __restrict__ absmax) {
+  // absmax (optional): the largest magnitude of the whole weight is folded into it
+  float amax = 0.0f;
   using T = __nv_bfloat16;
   const int TX = 1 << tx_log2, rows = kThreads >> tx_log2;
   const int tx = threadIdx.x & (TX - 1), ty = threadIdx.x >> tx_log2;
@@ -691,7 +694,13 @@ __global__ void __launch_bounds__(kThreads) minmax_group_bf16_kernel(const void*
         ((T*)mn_out)[gi] = __float2bfloat16_rn(lo);
         ((T*)mx_out)[gi] = __float2bfloat16_rn(hi);
       }
+      if (live) amax = fmaxf(amax, fmaxf(fabsf(lo), fabsf(hi)));
     }
+  }
+  if (absmax) {
+    amax = warp_max(amax);
+    // non-negative floats order like their bit patterns
+    if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<int*>(absmax), __float_as_int(amax));
   }
 }
 
