@@ -260,9 +260,12 @@ int b200q_scatter_columns_cast(const float* Wf, int64_t N, int64_t K, int64_t ld
  * W[:,i]=0; then H_ii += percdamp * mean(diag H). */
 int b200q_gptq_prepare(float* H, int64_t K, int64_t ldh, float* Wf, int64_t N, int64_t ldf,
                        float percdamp, void* stream);
+/* `nbytes` (a multiple of 8) of host memory, read during the call, written to dst (8-byte aligned) in stream order.  For
+ * a few words at a time: they travel as kernel arguments. */
+int b200q_upload(const void* host, int64_t nbytes, void* dst, void* stream);
 /* What comes before `count` factorisations of one size (device array of pointers H): perm[i] (int32 [count][K],
  * NULL: no reordering) = b200q_actorder_perm, diag[i] (float [count][K]) = the diagonal in that order, and
- * out[i] (float [count][K][K]) = the permuted matrix with dead diagonal entries set to 1 and damping added; without
+ * out[i] (float [K][K], at every K * K floats rounded up to a multiple of 4) = the permuted matrix with dead diagonal entries set to 1 and damping added; without
  * perm that happens in place.  damp: float [count], scratch. */
 int b200q_gptq_prologue_many(float* const* H, int count, int64_t K, int64_t ldh, float percdamp, int32_t* perm, float* diag,
                              float* damp, float* out, void* stream);

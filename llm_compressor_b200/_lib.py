@@ -52,6 +52,7 @@ SIGNATURES = {
     "b200q_observe_minmax_absmax": (_i, [_p, _i, _i64, _i64, _i64, _qa, _p, _p, _p, _p, _p]),
     "b200q_minmax_qparams": (_i, [_p, _p, _i, _i, _i64, _i64, _i64, _qa, _p, _p, _p]),
     "b200q_hessian_finalize_many": (_i, [_p, _p, _i, _i64, _i64, _p]),
+    "b200q_upload": (_i, [_p, _i64, _p, _p]),
     "b200q_gptq_prologue_many": (_i, [_p, _i, _i64, _i64, _f, _p, _p, _p, _p, _p]),
     "b200q_absmax_accumulate": (_i, [_p, _p, _i, _i64, _p, _p]),
     "b200q_global_scale_finalize": (_i, [_p, _i, _p, _p]),
@@ -124,10 +125,19 @@ def check(rc: int, what: str) -> int:
 
 def ptr(t):
     """Device pointer of a torch tensor (or None)."""
-    return None if t is None else C.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
+
+
+_raw_stream = None
 
 
 def stream_ptr():
-    import torch
+    """The calling thread's current stream, without building a ``torch.cuda.Stream`` object on every call (6 us)."""
+    global _raw_stream
+    if _raw_stream is None:
+        import torch
 
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+        raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+        device = torch.cuda.current_device
+        _raw_stream = (lambda: raw(device())) if raw is not None else (lambda: torch.cuda.current_stream().cuda_stream)
+    return _raw_stream()

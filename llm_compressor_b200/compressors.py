@@ -96,7 +96,7 @@ def compress_state_dict(state_dict: dict, scheme, fmt: str | None = None) -> dic
     gs = sd.get("weight_global_scale")
     if fmt == "pack-quantized":
         sd["weight_packed"] = ops.quantize_pack(w, scale, zp, args, g_idx=g_idx, pack_int8=True)
-        sd["weight_shape"] = torch.tensor(list(w.shape), device=w.device)
+        sd["weight_shape"] = ops.upload_words(w.shape, w.device)
         if not args.symmetric and args.strategy in ("group", "channel"):
             assert zp is not None, "Asymmetric quant requires zero-point values"
             sd["weight_zero_point"] = ops.pack_zero_points(zp, args.num_bits)

@@ -120,6 +120,15 @@ __global__ void permute_hessian_kernel(const float* __restrict__ H, int64_t K, i
   }
 }
 
+// A few words of host data (pointer tables, shapes) as kernel arguments: ordered in the stream like any launch.  A copy
+// from pageable memory waited for everything queued before it (0.5 ms each in an epoch of 96 expert modules).
+constexpr int kUploadWords = 448;
+struct UploadWords { unsigned long long v[kUploadWords]; };
+__global__ void __launch_bounds__(kUploadWords) upload_kernel(const __grid_constant__ UploadWords w, int n,
+                                                              unsigned long long* __restrict__ dst) {
+  if ((int)threadIdx.x < n) dst[threadIdx.x] = w.v[threadIdx.x];
+}
+
 // The prologue of many factorisations of one size: per problem (blockIdx.y) the diagonal in the new order, the damping
 // (summed in that order, as damp_kernel does on the permuted matrix) ...
 __global__ void __launch_bounds__(1024) diag_damp_kernel(const float* const* __restrict__ Hs, int64_t K, int64_t ldh,
@@ -158,7 +167,7 @@ __global__ void __launch_bounds__(256) permute_damp_kernel(float* const* __restr
     return;
   }
   const int32_t* pm = perm + blockIdx.y * K;
-  float* o = out + blockIdx.y * K * K;
+  float* o = out + blockIdx.y * ((K * K + 3) & ~(int64_t)3);
   for (int64_t r = blockIdx.x; r < K; r += gridDim.x) {
     const float* row = H + (int64_t)pm[r] * ldh;
     for (int64_t c = threadIdx.x; c < K; c += 256) {
@@ -230,6 +239,18 @@ int b200q_actorder_perm(const float* H, int64_t K, int64_t ldh, int32_t* perm, v
   if (!H || !perm || K <= 0 || ldh < K) return B200Q_ERR_ARG;
   perm_kernel<<<(int)((K + 31) / 32), 256, 0, (cudaStream_t)stream>>>(H, nullptr, K, ldh, perm);
   B200Q_LAUNCH_CHECK();
+  return B200Q_OK;
+}
+
+int b200q_upload(const void* host, int64_t nbytes, void* dst, void* stream) {
+  if (!host || !dst || nbytes < 0 || nbytes % 8 || ((uintptr_t)dst) % 8) return B200Q_ERR_ARG;
+  for (int64_t at = 0; at < nbytes; at += (int64_t)sizeof(UploadWords)) {
+    UploadWords w;
+    const int64_t n = nbytes - at < (int64_t)sizeof(w) ? nbytes - at : (int64_t)sizeof(w);
+    memcpy(w.v, (const char*)host + at, (size_t)n);
+    upload_kernel<<<1, kUploadWords, 0, (cudaStream_t)stream>>>(w, (int)(n / 8), (unsigned long long*)((char*)dst + at));
+    B200Q_LAUNCH_CHECK();
+  }
   return B200Q_OK;
 }
 

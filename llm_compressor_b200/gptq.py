@@ -18,7 +18,7 @@ from typing import Optional
 import torch
 
 from . import _lib, ops
-from .observers import Observer
+from .observers import Observer, direct_qparams
 from .quant_args import QuantizationArgs
 
 __all__ = ["make_empty_hessian", "accumulate_hessian", "accumulate_hessian_lower",
@@ -154,14 +154,16 @@ def factor_hessians_batched(hessians, percdamp: float = 0.01, actorder=None):
     """``factor_hessian(..., defer=True)`` for a list of small Hessians of one size, with all the
     factorisations in one launch (one thread block per matrix).  The matrices are consumed.
     Returns the deferred factors; ``resolve_factors`` reads all their status words at once."""
-    parts = [_factor_prologue(H, percdamp, actorder) for H in hessians]
-    status = ops.gptq_factor_batched([H for H, _, _ in parts])
-    return [HessianFactor(H.shape[0], perm, diag, H, None, status[i]) for i, (H, perm, diag) in enumerate(parts)]
+    hessians, perms, diags = ops.gptq_prologue_batched(list(hessians), percdamp, bool(actorder))
+    status = ops.gptq_factor_batched(hessians)
+    perms = [None] * len(hessians) if perms is None else perms.unbind(0)
+    return [HessianFactor(H.shape[0], perm, diag, H, None, st)
+            for H, perm, diag, st in zip(hessians, perms, diags.unbind(0), status.unbind(0))]
 
 
 def resolve_factors(factors) -> None:
     """``HessianFactor.resolve`` for many factors with one wait for the device."""
-    pending = [f for f in factors if f.ok is None]
+    pending = list({id(f): f for f in factors if f.ok is None}.values())
     if not pending:
         return
     words = torch.stack([f.status.reshape(-1)[:4] for f in pending]).tolist()
@@ -189,9 +191,10 @@ class _SweepInput:
     final_dtype: torch.dtype
 
 
-def _sweep_input(module, quant_args, hessian, percdamp, factor, W=None) -> _SweepInput:
+def _sweep_input(module, quant_args, hessian, percdamp, factor, W=None, qparams=None, order=None) -> _SweepInput:
     """``W``: the float32 copy of the weight, already permuted and with its dead columns zeroed (the
-    batched path makes it for all modules at once); made here when not given."""
+    batched path makes it for all modules at once); made here when not given.  ``qparams`` (scale, zero point) and
+    ``order`` (column order of the groups) likewise."""
     args = QuantizationArgs.of(quant_args)
     strategy, actorder = args.strategy, args.actorder
     weight = module.weight.data if isinstance(module.weight, torch.nn.Parameter) else module.weight
@@ -217,26 +220,37 @@ def _sweep_input(module, quant_args, hessian, percdamp, factor, W=None) -> _Swee
     if not prepared:
         W = ops.gather_columns_f32(weight, perm)
 
-    if actorder == "group":
-        observer.delete_statistics(check_fused=False)
-        observer(W)
-    elif not observer.has_statistics:
-        observer(weight)     # memoryless: the statistics of the weight as it is now
+    global_scale = None
+    if qparams is None and actorder != "group":
+        qparams = direct_qparams([observer], [weight])
+        if qparams is not None:
+            qparams = (qparams[0][0], qparams[1][0])
+    if qparams is None:
+        if actorder == "group":
+            observer.delete_statistics(check_fused=False)
+            observer(W)
+        elif not observer.has_statistics:
+            observer(weight)     # memoryless: the statistics of the weight as it is now
+        qp = observer.get_qparams()
+        qparams, global_scale = (qp["scale"], qp["zero_point"]), qp["global_scale"]
 
-    col_group = None
+    # which group a column of the permuted weight belongs to: needed where the columns are out of order
     g_idx = None
-    if strategy in ("group", "tensor_group", "block"):
-        divisor = args.group_size if strategy != "block" else args.block_structure[1]
-        g_idx = torch.arange(K, device=W.device, dtype=torch.int32) // divisor
-        if actorder == "weight":
-            g_idx = g_idx[perm.long()]
-            col_group = g_idx
+    if actorder in ("weight", "group") and strategy in ("group", "tensor_group", "block"):
+        g_idx = order if order is not None else _column_groups(args, K, perm if actorder == "weight" else None, W.device)
+    col_group = g_idx if actorder == "weight" else None
 
-    qparams = observer.get_qparams()
     if not prepared:
         ops.gptq_zero_dead_columns(factor.diag, W)
-    return _SweepInput(args, actorder, factor, W, qparams["scale"], qparams["zero_point"], qparams["global_scale"],
-                       col_group, g_idx, weight.dtype)
+    return _SweepInput(args, actorder, factor, W, qparams[0], qparams[1], global_scale, col_group, g_idx, weight.dtype)
+
+
+def _column_groups(args, K: int, perm, device) -> torch.Tensor:
+    """Group of every column, in the order of ``perm`` ([K] or [count, K], int32; None: as they are)."""
+    divisor = args.group_size if args.strategy != "block" else args.block_structure[1]
+    if perm is None:
+        return torch.arange(K, device=device, dtype=torch.int32) // divisor
+    return torch.div(perm, divisor, rounding_mode="floor")
 
 
 def _sweep_output(inp: _SweepInput, weight=None) -> dict:
@@ -304,7 +318,16 @@ def quantize_weights_batched(modules, quant_args, factors, blocksize: int = 128,
         raise ValueError("the factors of a batch must all carry a permutation or none")
     # one launch: float32 copies, permuted, dead columns zeroed
     Wf = ops.gather_columns_f32_batched(weights, None if perms[0] is None else perms, [f.diag for f in factors])
-    inputs = [_sweep_input(m, quant_args, None, percdamp, f, W=Wf[k])
+    args = QuantizationArgs.of(quant_args)
+    count = len(weights)
+    qparams = order = None
+    if args.actorder != "group":
+        qparams = direct_qparams([m.weight_observer for m in modules], weights)
+    if args.actorder == "weight" and args.strategy in ("group", "tensor_group", "block"):
+        order = _column_groups(args, Wf.shape[2], torch.stack(perms), Wf.device).unbind(0)
+    Ws = Wf.unbind(0)
+    each = [None] * count if qparams is None else list(zip(qparams[0].unbind(0), qparams[1].unbind(0)))
+    inputs = [_sweep_input(m, args, None, percdamp, f, W=Ws[k], qparams=each[k], order=None if order is None else order[k])
               for k, (m, f) in enumerate(zip(modules, factors))]
     first = inputs[0]
 
@@ -314,13 +337,12 @@ def quantize_weights_batched(modules, quant_args, factors, blocksize: int = 128,
             raise ValueError(f"{name} must be present for all modules of a batch or for none")
         return None if vals[0] is None else vals
 
-    losses, status = ops.gptq_sweep_batched([i.W for i in inputs], [i.factor.U for i in inputs], column("scale"),
-                                    None if first.args.symmetric else column("zero_point"), first.args, col_groups=column("col_group"),
-                                    global_scales=column("global_scale"), blocksize=blocksize,
-                                            return_status=True)
-    sums = losses.sum(dim=1)
-    back = ops.scatter_columns_cast_batched([i.W for i in inputs], first.final_dtype,
-                                            None if perms[0] is None else perms)
+    losses, status = ops.gptq_sweep_batched(
+        Wf, [i.factor.U for i in inputs], column("scale") if qparams is None else qparams[0],
+        None if first.args.symmetric else (column("zero_point") if qparams is None else qparams[1]), first.args,
+        col_groups=column("col_group"), global_scales=column("global_scale"), blocksize=blocksize, return_status=True)
+    sums = losses.sum(dim=1).unbind(0)
+    back = ops.scatter_columns_cast_batched(Wf, first.final_dtype, None if perms[0] is None else perms).unbind(0)
     done = [(sums[k], _sweep_output(i, weight=back[k])) for k, i in enumerate(inputs)]
     done[0][1]["_status"] = status
     return done

@@ -22,7 +22,7 @@ import torch
 from . import dist as bdist
 from . import gptq
 from ._lib import B200QError
-from .observers import Observer, fuse_weight_observers
+from .observers import Observer, direct_qparams, fuse_weight_observers
 from .streams import run_concurrent
 from .quant_args import (PRESET_SCHEMES, QuantizationArgs, QuantizationScheme,
                          preset_name_to_scheme)
@@ -203,7 +203,8 @@ class QuantizationMixin(HooksMixin):
                 module.quantization_scheme = scheme
                 module.quantization_status = "initialized"   # "frozen" once its qparams are written
                 self._module_names[module] = name
-                dev, dt = module.weight.device, module.weight.dtype
+                weight = module.weight
+                dev, dt = weight.device, weight.dtype
                 shape = w.qparam_shape(N, K)
 
                 def reg(pname, t):
@@ -257,14 +258,15 @@ class QuantizationMixin(HooksMixin):
                 "bypass_divisibility_checks=True")
 
     def quantized_modules(self, model: torch.nn.Module):
-        return [(n, m) for n, m in model.named_modules() if hasattr(m, "quantization_scheme")
-                and m in self._module_names]
+        return [(n, m) for n, m in model.named_modules() if m in self._module_names and hasattr(m, "quantization_scheme")]
 
     def start_calibration(self, model: torch.nn.Module) -> None:
+        shared = False   # some weights have a global scale that siblings share
         for _, module in self.quantized_modules(model):
             w = module.quantization_scheme.weights
             module.weight_observer = Observer.load_from_registry(
                 w.observer or "memoryless_minmax", base_name="weight", args=w)
+            shared = shared or w.strategy == "tensor_group"
             a = module.quantization_scheme.input_activations
             if a is not None and a.dynamic is not True:
                 name = a.observer if a.observer not in (None, "memoryless_minmax") else "minmax"
@@ -276,7 +278,8 @@ class QuantizationMixin(HooksMixin):
             module.k_observer = Observer.load_from_registry(name, base_name="k", args=a)
             module.v_observer = Observer.load_from_registry(name, base_name="v", args=a)
             self.register_hook(module, _observing_cache_hook, "forward_pre", with_kwargs=True)
-        fuse_weight_observers(model)
+        if shared:
+            fuse_weight_observers(model)
 
     @property
     def calibrates_activations(self) -> bool:
@@ -310,7 +313,7 @@ class QuantizationMixin(HooksMixin):
         self.remove_hooks()
         for module in [m for _, m in self.quantized_modules(model)] + list(self._attention_names):
             for name in ("weight_observer", "input_observer", "k_observer", "v_observer"):
-                if hasattr(module, name):
+                if name in module.__dict__:
                     delattr(module, name)
 
 
@@ -372,15 +375,34 @@ def update_qparams(modules: Iterable[torch.nn.Module], base_name: str = "weight"
             warnings.warn(f"Observer of {type(m).__name__} has no statistics; qparams not updated")
             continue
         qp = obs.get_qparams()
-        if hasattr(m, f"{base_name}_scale"):    # absent for locally dynamic activations (global scale only)
-            getattr(m, f"{base_name}_scale").data.copy_(qp["scale"].reshape(getattr(m, f"{base_name}_scale").shape))
-            if hasattr(m, f"{base_name}_zero_point"):   # symmetric kv-cache scales carry none
-                getattr(m, f"{base_name}_zero_point").data.copy_(qp["zero_point"].reshape(
-                    getattr(m, f"{base_name}_zero_point").shape))
-        if qp["global_scale"] is not None and hasattr(m, f"{base_name}_global_scale"):
-            getattr(m, f"{base_name}_global_scale").data.copy_(qp["global_scale"])
-        if base_name == "weight":
-            m.quantization_status = "frozen"
+        _write_qparams(m, base_name, qp["scale"], qp["zero_point"], qp["global_scale"])
+
+
+def _write_qparams(m, base_name, scale, zero_point, global_scale) -> None:
+    # (the scale is absent for locally dynamic activations, which have a global scale only; symmetric kv-cache scales
+    # carry no zero point)
+    params = m._parameters
+    written = [("scale", scale)]
+    if params.get(base_name + "_scale") is not None:
+        written.append(("zero_point", zero_point))
+    if global_scale is not None:
+        written.append(("global_scale", global_scale))
+    for what, val in written:
+        p = params.get(f"{base_name}_{what}")
+        if p is not None:
+            _put(p, val)
+    if base_name == "weight":
+        m.quantization_status = "frozen"
+
+
+def _put(p: torch.Tensor, val: torch.Tensor) -> None:
+    """Give parameter ``p`` the values of ``val``, a fresh tensor nobody else writes: no copy where it can stand in."""
+    if val.shape != p.shape:
+        val = val.reshape(p.shape)
+    if val.dtype == p.dtype and val.device == p.device and val.is_contiguous():
+        p.data = val
+    else:
+        p.data.copy_(val)
 
 
 # ------------------------------------------------------------------------------------------
@@ -401,7 +423,8 @@ class QuantizationModifier(QuantizationMixin):
 
     def on_sequential_epoch_end(self, model, modules: Iterable[torch.nn.Module], **_):
         modules = list(modules)
-        self.update_activation_qparams(modules)
+        if self.calibrates_activations:
+            self.update_activation_qparams(modules)
         modules = [m for m in modules if hasattr(m, "weight_observer")
                    and getattr(m, "quantization_status", None) != "frozen"]
         if bdist.is_distributed():
@@ -416,8 +439,17 @@ class QuantizationModifier(QuantizationMixin):
             for m in items:
                 m.quantization_status = "frozen"
         else:
-            observe(modules)
-            update_qparams(modules)
+            # most weights: statistics and parameters in one launch
+            rest = []
+            for m in modules:
+                weight = m.weight.data
+                qp = direct_qparams([m.weight_observer], [weight]) if weight.is_cuda else None
+                if qp is None:
+                    rest.append(m)
+                else:
+                    _write_qparams(m, "weight", qp[0][0], qp[1][0], None)
+            observe(rest)
+            update_qparams(rest)
 
     def pending_modules(self):
         """Targeted modules whose parameters have not been written yet (modules behind the
@@ -468,6 +500,7 @@ class GPTQModifier(QuantizationMixin):
         self.batch_small_hessians = batch_small_hessians
         self.small_hessian_columns = small_hessian_columns
         self._groups: dict = {}        # module -> _HessianGroup
+        self._by_input: dict = {}      # _input_key of a batch of this epoch -> the group that took it last
         self._num_samples: dict = {}   # module -> None (membership: modules awaiting compression)
         self.trace = None              # optional callback(event: str, module | None) for instrumentation
         self._hooked: list = []        # every module that got a calibration hook
@@ -546,13 +579,18 @@ class GPTQModifier(QuantizationMixin):
         group = self._groups.get(module)
         if group is None:
             group = self._find_shared(inp) if self.share_hessians else None
-            if group is None:
-                group = _HessianGroup(module, offload=self.offload_hessians, stage_tokens=self.hessian_stage_tokens)
-            else:
+            if group is not None:
                 group.members.append(module)
+                self._groups[module] = group
+                self._num_samples[module] = None
+                return   # the batch is in the Hessian already
+            else:
+                group = _HessianGroup(module, offload=self.offload_hessians, stage_tokens=self.hessian_stage_tokens)
             self._groups[module] = group
             self._num_samples[module] = None
-        elif module is not group.members[0] and not group.same_input(inp):
+        elif group.same_input(inp):
+            return
+        elif module is not group.members[0]:
             # membership was decided on the first batch; the first member adds every batch and
             # the others must keep receiving that very tensor
             raise RuntimeError(
@@ -561,8 +599,15 @@ class GPTQModifier(QuantizationMixin):
                 "the same input on the first calibration batch, but its input differs on a later batch; "
                 "set GPTQModifier(share_hessians=False)")
         group.accumulate(inp)
+        self._by_input[_input_key(inp)] = group
 
     def _find_shared(self, inp):
+        # by address first: an epoch of 64 experts has 65 groups to look through for each new module
+        g = self._by_input.get(_input_key(inp))
+        if g is None:
+            return None
+        if g.same_input(inp):
+            return g
         for g in {id(g): g for g in self._groups.values()}.values():
             if g.same_input(inp):
                 return g
@@ -570,7 +615,8 @@ class GPTQModifier(QuantizationMixin):
 
     def on_sequential_epoch_end(self, model, modules: Iterable[torch.nn.Module], **_):
         modules = list(modules)
-        self.update_activation_qparams(modules)
+        if self.calibrates_activations:
+            self.update_activation_qparams(modules)
         mods = [m for m in modules if m in self._num_samples]
         # the weight observers are called by the solves themselves (gptq._sweep_input), on the rank
         # and stream that quantises the module, next to the rest of its work
@@ -582,6 +628,7 @@ class GPTQModifier(QuantizationMixin):
 
     def compress_modules(self, modules=None):
         modules = list(self._num_samples.keys()) if modules is None else list(modules)
+        self._by_input.clear()
         if not bdist.is_distributed():
             self._trace("solve")
             self.compress_module_list(modules)
@@ -712,13 +759,9 @@ class GPTQModifier(QuantizationMixin):
             for attr, val in out.items():
                 if attr == "weight":
                     continue
-                elif hasattr(module, attr):
-                    p = getattr(module, attr)
-                    val = val.reshape(p.shape)
-                    if val.dtype == p.dtype and val.device == p.device and val.is_contiguous():
-                        p.data = val        # a fresh tensor of the solve: no copy into the placeholder
-                    else:
-                        p.data.copy_(val)
+                p = getattr(module, attr, None)
+                if p is not None:
+                    _put(p, val)
                 else:
                     module.register_parameter(attr, torch.nn.Parameter(val, requires_grad=False))
             module.quantization_status = "frozen"
@@ -757,6 +800,7 @@ class GPTQModifier(QuantizationMixin):
             return holder
 
         taken, words = [], []
+        _finalize_groups([self._groups[mods[0]] for mods in jobs])
         for mods in jobs:
             part, status = self._queue_factors(mods, ask)
             taken += part
@@ -772,9 +816,11 @@ class GPTQModifier(QuantizationMixin):
             for (_, holder), factor in zip(items, factors):
                 holder.append(factor)
         del requests, by_kind
-        by_shape: dict = {}
+        by_shape, schemes = {}, {}
         for module, qargs, holder in taken:
-            key = (tuple(module.weight.shape), module.weight.dtype, repr(qargs))
+            if id(qargs) not in schemes:
+                schemes[id(qargs)] = repr(qargs)
+            key = (tuple(module.weight.shape), module.weight.dtype, schemes[id(qargs)])
             by_shape.setdefault(key, []).append((module, qargs, holder[0]))
         queued = []
         # the class with the most device work first: its sweep runs while the host prepares the others
@@ -850,6 +896,10 @@ def _with_actorder(qargs: QuantizationArgs, actorder):
     return a
 
 
+def _input_key(inp: torch.Tensor):
+    return inp.data_ptr(), inp.shape, inp.dtype
+
+
 class _HessianGroup:
     """One Hessian shared by the modules that see the same input.
 
@@ -862,10 +912,14 @@ class _HessianGroup:
         self.members = [module]
         K = module.weight.shape[1]
         self.device = module.weight.device
-        self.H = torch.zeros((K, K), dtype=torch.float32, device=self.device)
+        # one allocation (and one launch to clear it) for the sum and the word that a bounded wait running out sets
+        both = torch.zeros(K * K + 1, dtype=torch.float32, device=self.device)
+        self.H = both[:K * K].view(K, K)
         self.n = 0
         self._last = None  # (tensor kept alive, version) of the batch accumulated last
-        self.status = torch.zeros(1, dtype=torch.int32, device=self.device)   # bounded-wait expiry of any update
+        self.status = both[K * K:].view(torch.int32)
+        if offload:   # the sum moves to the host between batches: the word must not keep its place on the device
+            self.status = self.status.clone()
         self.offload = offload
         self._final = None
         self.stage_tokens = int(stage_tokens)
@@ -909,17 +963,35 @@ class _HessianGroup:
         self.n += added
         self._last = (inp, inp._version)
 
+    def take_sum(self) -> torch.Tensor:
+        """The lower triangle of the sum over all batches, handed over."""
+        self._last = None
+        self.flush()
+        self._stage = None
+        H, self.H = self.H.to(self.device), None
+        return H
+
     def finalized(self, keep: bool = False) -> torch.Tensor:
         """Full symmetric H / n.  The caller's factorisation consumes the matrix it gets;
         ``keep`` asks for a copy because another act-order setting still needs H."""
         self._last = None
         if self._final is None:
-            self.flush()
-            self._stage = None
-            H = self.H.to(self.device)
-            self.H = None
-            self._final = gptq.finalize_hessian(H, self.n)
+            self._final = gptq.finalize_hessian(self.take_sum(), self.n)
         out = self._final.clone() if keep else self._final
         if not keep:
             self._final = None
         return out
+
+
+def _finalize_groups(groups) -> None:
+    """``finalized`` for many groups: one launch for all the Hessians of a width."""
+    by_width: dict = {}
+    for g in groups:
+        if g._final is None:
+            by_width.setdefault(g.H.shape[0], []).append(g)
+    for gs in by_width.values():
+        if len(gs) > 1:
+            Hs = [g.take_sum() for g in gs]
+            gptq.ops.hessian_finalize_many(Hs, [1.0 / g.n if g.n else 1.0 for g in gs])
+            for g, H in zip(gs, Hs):
+                g._final = H

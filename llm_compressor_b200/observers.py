@@ -152,6 +152,21 @@ class Observer:
         return {"scale": scale, "zero_point": zero_point, "global_scale": global_scale}
 
 
+def direct_qparams(observers, weights):
+    """What observing ``weights[i]`` with ``observers[i]`` and asking for the parameters gives, in one launch and without
+    statistics in between: (scales, zero points) with a leading dimension, or None where the two steps are needed (other
+    observers, shared global scales, statistics that are already there, weights the kernel does not take)."""
+    first = observers[0]
+    for o in observers:
+        if type(o) is not MemorylessMinMaxObserver or o.has_statistics or o._fused or o.args.strategy == "tensor_group" \
+                or (o.args is not first.args and o.args != first.args):
+            return None
+    if len(weights) == 1:
+        qp = ops.minmax_qparams(weights[0], first.args)
+        return None if qp is None else (qp[0].unsqueeze(0), qp[1].unsqueeze(0))
+    return ops.minmax_qparams(list(weights), first.args)
+
+
 @Observer.register("memoryless_minmax")
 class MemorylessMinMaxObserver(Observer):
     def update_statistics_from_weight(self, weight):

@@ -5,6 +5,9 @@ into ``libb200q.so``.  All tensors must live on a CUDA device.
 """
 from __future__ import annotations
 
+import ctypes
+import struct
+
 import torch
 
 from . import _lib
@@ -52,6 +55,34 @@ def observe_minmax(w: torch.Tensor, args: QuantizationArgs):
     check(lib.b200q_observe_minmax(ptr(w), _dt(w), N, K, ld, qa, ptr(mn), ptr(mx), ptr(scratch),
                                    stream_ptr()), "b200q_observe_minmax")
     return mn, mx
+
+
+def minmax_qparams(w, args: QuantizationArgs):
+    """``qparams(*observe_minmax(w, args), args)`` in one launch: (scale, zero_point), or None for what it does not take.
+    ``w`` may be a list of weights of one shape and layout: the results then carry a leading dimension."""
+    many = not isinstance(w, torch.Tensor)
+    first = w[0] if many else w
+    if first.dtype != torch.bfloat16 or args.strategy == "tensor_group":
+        return None
+    N, K, ld = _2d(first)
+    count = len(w) if many else 1
+    if many:
+        for t in w:
+            if t.shape != (N, K) or t.stride() != (ld, 1) or t.dtype != first.dtype or t.data_ptr() % 16:
+                return None
+    _need_cuda(*w) if many else _need_cuda(w)
+    shape = args.qparam_shape(N, K)
+    if many:
+        shape = (count,) + tuple(shape)
+    scale = torch.empty(shape, dtype=first.dtype, device=first.device)
+    zp = torch.empty(shape, dtype=_zp_storage(args), device=first.device)
+    table = _pointer_table([w]) if many else None
+    rc = _lib.load().b200q_minmax_qparams(None if many else ptr(w), ptr(table), count, _dt(first), N, K, ld, args.c_struct(),
+                                          ptr(scale), ptr(zp), stream_ptr())
+    if rc == -2:
+        return None
+    check(rc, "b200q_minmax_qparams")
+    return scale, zp
 
 
 def observe_mse(w, args, maxshrink=0.20, patience=5, grid=100.0, norm=2.4, expand=1.0):
@@ -311,6 +342,21 @@ def hessian_finalize(H: torch.Tensor, scale: float = 1.0):
     return H
 
 
+def hessian_finalize_many(Hs, scales):
+    """``hessian_finalize`` of a list of Hessians of one size, each with its own scale, in one launch."""
+    _need_cuda(*Hs)
+    K, ld = Hs[0].shape[0], Hs[0].stride(0)
+    for H in Hs:
+        if H.shape != (K, K) or H.stride() != (ld, 1) or H.dtype != torch.float32 or H.data_ptr() % 16:
+            raise ValueError("batched finalisation needs float32 Hessians of one size and one layout")
+    count = len(Hs)
+    halves = [struct.unpack("<I", struct.pack("<f", float(s)))[0] for s in scales] + [0] * (count % 2)
+    words = upload_words([H.data_ptr() for H in Hs] + [lo | ((hi & 0x7fffffff) << 32) for lo, hi in
+                                                        zip(halves[::2], halves[1::2])], Hs[0].device)
+    check(_lib.load().b200q_hessian_finalize_many(ptr(words), ptr(words[count:]), count, K, ld, stream_ptr()),
+          "b200q_hessian_finalize_many")
+
+
 # ---------------------------------------------------------------------------- GPTQ solve
 def set_reproducible(on: bool) -> bool:
     """Bitwise reproducible Hessian accumulation (no atomics across token splits) for all later
@@ -428,12 +474,55 @@ def gptq_sweep(wf, U, scale, zp, args: QuantizationArgs, blocksize=128, col_grou
     return losses
 
 
+def upload_words(words, device) -> torch.Tensor:
+    """Device int64 tensor of a few python integers, in stream order and without waiting for the device."""
+    words = list(words)
+    out = torch.empty(len(words), dtype=torch.int64, device=device)
+    host = (ctypes.c_int64 * len(words))(*words)
+    check(_lib.load().b200q_upload(ctypes.addressof(host), 8 * len(words), ptr(out), stream_ptr()), "b200q_upload")
+    return out
+
+
 def _pointer_table(rows) -> torch.Tensor:
-    """Device int64 [len(rows), count]: row r holds the addresses of the tensors in rows[r]
-    (a row that is None becomes a row of zeros and is passed to the library as NULL)."""
+    """Device int64 [len(rows), count]: row r holds the addresses of the tensors in rows[r], a tensor standing for the
+    slices of its first dimension (a row that is None becomes a row of zeros and is passed to the library as NULL)."""
     first = next(r for r in rows if r is not None)
-    table = [[0] * len(first) if r is None else [t.data_ptr() for t in r] for r in rows]
-    return torch.tensor(table, dtype=torch.int64, device=first[0].device)
+    count, words = len(first), []
+    for r in rows:
+        if r is None:
+            words += [0] * count
+        elif isinstance(r, torch.Tensor):
+            step = r.stride(0) * r.element_size()
+            words += range(r.data_ptr(), r.data_ptr() + step * count, step)
+        else:
+            words += [t.data_ptr() for t in r]
+    return upload_words(words, first[0].device).view(len(rows), count)
+
+
+def _each_contiguous(ts, dtype):
+    """A list of tensors, or one tensor of them all, as contiguous tensors of ``dtype``."""
+    if isinstance(ts, torch.Tensor):
+        return ts.to(dtype).contiguous()
+    return [t.to(dtype).contiguous() for t in ts]
+
+
+def gptq_prologue_batched(Hs, percdamp: float, actorder: bool):
+    """Permutation, diagonal and damping of a list of Hessians of one size: (matrices ready to factor, permutations or
+    None, diagonals).  Without ``actorder`` the matrices are changed in place, otherwise they are left alone."""
+    _need_cuda(*Hs)
+    K, ld = Hs[0].shape[0], Hs[0].stride(0)
+    for H in Hs:
+        if H.shape != (K, K) or H.stride() != (ld, 1) or H.dtype != torch.float32:
+            raise ValueError("batched factorisation needs float32 Hessians of one size and one layout")
+    count, dev = len(Hs), Hs[0].device
+    perm = torch.empty((count, K), dtype=torch.int32, device=dev) if actorder else None
+    out = torch.empty((count, -(-K * K // 4) * 4), dtype=torch.float32, device=dev) if actorder else None
+    diag = torch.empty((count, K), dtype=torch.float32, device=dev)
+    damp = torch.empty(count, dtype=torch.float32, device=dev)
+    table = _pointer_table([Hs])
+    check(_lib.load().b200q_gptq_prologue_many(ptr(table), count, K, ld, float(percdamp), ptr(perm), ptr(diag), ptr(damp),
+                                               ptr(out), stream_ptr()), "b200q_gptq_prologue_many")
+    return [o[:K * K].view(K, K) for o in out] if actorder else Hs, perm, diag
 
 
 def gptq_factor_batched(Hs) -> torch.Tensor:
@@ -465,10 +554,10 @@ def gather_columns_f32_batched(ws, perms=None, dead_diags=None) -> torch.Tensor:
     _need_cuda(*ws)
     out = torch.empty((count, N, K), dtype=torch.float32, device=ws[0].device)
     if perms is not None:
-        perms = [p.to(torch.int32).contiguous() for p in perms]
+        perms = _each_contiguous(perms, torch.int32)
     if dead_diags is not None:
-        dead_diags = [d.to(torch.float32).contiguous() for d in dead_diags]
-    table = _pointer_table([ws, perms, dead_diags, list(out.unbind(0))])
+        dead_diags = _each_contiguous(dead_diags, torch.float32)
+    table = _pointer_table([ws, perms, dead_diags, out])
     check(_lib.load().b200q_gather_columns_f32_batched(
         ptr(table[0]), _dt(ws[0]), ptr(table[1]) if perms is not None else None,
         ptr(table[2]) if dead_diags is not None else None, ptr(table[3]), count, N, K, ld, K, stream_ptr()),
@@ -480,14 +569,14 @@ def scatter_columns_cast_batched(wfs, dtype: torch.dtype, perms=None) -> torch.T
     """The way back: [count, N, K] in ``dtype`` with ``out[i][:, perms[i][c]] = wfs[i][:, c]``."""
     count = len(wfs)
     N, K, ld = _2d(wfs[0])
-    for w in wfs:
+    for w in () if isinstance(wfs, torch.Tensor) else wfs:
         if _2d(w) != (N, K, ld) or w.dtype != torch.float32:
             raise ValueError("batched scatter needs float32 matrices of one shape and layout")
-    _need_cuda(*wfs)
+    _need_cuda(wfs[0])
     out = torch.empty((count, N, K), dtype=dtype, device=wfs[0].device)
     if perms is not None:
-        perms = [p.to(torch.int32).contiguous() for p in perms]
-    table = _pointer_table([wfs, perms, list(out.unbind(0))])
+        perms = _each_contiguous(perms, torch.int32)
+    table = _pointer_table([wfs, perms, out])
     check(_lib.load().b200q_scatter_columns_cast_batched(
         ptr(table[0]), ptr(table[1]) if perms is not None else None, ptr(table[2]), _DT[dtype], count, N, K, ld, K,
         stream_ptr()), "b200q_scatter_columns_cast_batched")
@@ -498,24 +587,24 @@ def gptq_sweep_batched(wfs, Us, scales, zps, args: QuantizationArgs, col_groups=
                        blocksize=128, return_status: bool = False):
     """The column sweep, in place, on a list of float32 weights of one shape that share the
     quantisation scheme, in one launch.  ``Us``, ``zps``, ``col_groups``, ``global_scales``: a list
-    with one tensor per weight, or None for all.  Returns the per-row losses [count, N], and with
+    with one tensor per weight (or, as ``wfs`` and ``scales``, one tensor of them all), or None for all.  Returns the per-row losses [count, N], and with
     ``return_status`` also the call's device status word (see ``gptq_sweep``)."""
     if blocksize != 128:
         raise ValueError("the batched sweep takes blocksize 128")
     count = len(wfs)
     N, K, ld = _2d(wfs[0])
     dev = wfs[0].device
-    scales = [s.contiguous() for s in scales]
+    scales = _each_contiguous(scales, scales[0].dtype)
     sdt = _dt(scales[0])
-    zps = None if zps is None else [z.contiguous() for z in zps]
-    col_groups = None if col_groups is None else [c.to(torch.int32).contiguous() for c in col_groups]
-    global_scales = None if global_scales is None else [g.to(torch.float32).contiguous() for g in global_scales]
+    zps = None if zps is None else _each_contiguous(zps, zps[0].dtype)
+    col_groups = None if col_groups is None else _each_contiguous(col_groups, torch.int32)
+    global_scales = None if global_scales is None else _each_contiguous(global_scales, torch.float32)
     for lst in (wfs, Us, scales, zps, col_groups, global_scales):
         if lst is not None:
             if len(lst) != count:
                 raise ValueError("one tensor per weight, or None for all")
-            _need_cuda(*lst)
-    for w in wfs:
+            _need_cuda(*((lst,) if isinstance(lst, torch.Tensor) else lst))
+    for w in () if isinstance(wfs, torch.Tensor) else wfs:
         if _2d(w) != (N, K, ld) or w.dtype != torch.float32:
             raise ValueError("batched sweep needs float32 weights of one shape and one layout")
     ldu = 0
@@ -524,10 +613,10 @@ def gptq_sweep_batched(wfs, Us, scales, zps, args: QuantizationArgs, col_groups=
         for U in Us:
             if U.shape != (K, K) or U.stride(0) != ldu or U.stride(1) != 1:
                 raise ValueError("batched sweep needs factors of one size and one layout")
-    if any(_dt(s) != sdt or s.numel() != scales[0].numel() for s in scales):
+    if not isinstance(scales, torch.Tensor) and any(_dt(s) != sdt or s.numel() != scales[0].numel() for s in scales):
         raise ValueError("batched sweep needs scales of one dtype and one shape")
     losses = torch.empty((count, N), dtype=torch.float32, device=dev)
-    table = _pointer_table([wfs, Us, scales, zps, col_groups, global_scales, list(losses.unbind(0))])
+    table = _pointer_table([wfs, Us, scales, zps, col_groups, global_scales, losses])
     distinct, index = table[1], None
     ndistinct = count if Us is not None else 1
     if Us is not None:
@@ -536,8 +625,10 @@ def gptq_sweep_batched(wfs, Us, scales, zps, args: QuantizationArgs, col_groups=
         order = [place.setdefault(U.data_ptr(), len(place)) for U in Us]
         ndistinct = len(place)
         if ndistinct < count:
-            distinct = torch.tensor(list(place), dtype=torch.int64, device=dev)
-            index = torch.tensor(order, dtype=torch.int32, device=dev)
+            padded = order + [0] * (count % 2)      # int32 pairs
+            pairs = [lo | (hi << 32) for lo, hi in zip(padded[::2], padded[1::2])]
+            tail = upload_words(list(place) + pairs, dev)
+            distinct, index = tail[:ndistinct], tail[ndistinct:].view(torch.int32)
     lib = _lib.load()
     ws = torch.empty(lib.b200q_gptq_sweep_many_workspace_bytes(N, K, count, ndistinct), dtype=torch.uint8, device=dev)
 

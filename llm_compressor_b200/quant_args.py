@@ -20,6 +20,9 @@ _STRATEGY = {"tensor": _lib.TENSOR, "channel": _lib.CHANNEL, "group": _lib.GROUP
              "tensor_group": _lib.TENSOR_GROUP, "block": _lib.BLOCK}
 
 
+_C_STRUCTS: dict = {}   # field values -> the structure the kernels read (never written to after it is made)
+
+
 def _plain(v):
     return v.value if hasattr(v, "value") else v
 
@@ -106,6 +109,16 @@ class QuantizationArgs:
                 and self.scale_dtype == torch.uint8)
 
     def c_struct(self) -> _lib.QArgs:
+        key = (self.num_bits, self.type, self.symmetric, self.strategy, self.group_size, self.scale_dtype, self.zp_dtype,
+               tuple(self.block_structure) if self.block_structure else None)
+        made = _C_STRUCTS.get(key)
+        if made is None:
+            if len(_C_STRUCTS) >= 256:
+                _C_STRUCTS.clear()
+            made = _C_STRUCTS[key] = self._make_c_struct()
+        return made
+
+    def _make_c_struct(self) -> _lib.QArgs:
         if self.scale_dtype is None:
             sk = _lib.SCALE_PLAIN
         elif self.scale_dtype == torch.float8_e4m3fn:
