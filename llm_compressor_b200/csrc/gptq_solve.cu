@@ -3,6 +3,8 @@
 #include "common.cuh"
 #include "tgemm_tf32.cuh"
 
+#include <cstring>
+
 namespace b200q {
 namespace solve {
 
@@ -55,69 +57,214 @@ __device__ __forceinline__ int64_t perm_at(const int32_t* __restrict__ perm, int
   return v < 0 ? 0 : (v >= K ? K - 1 : v);
 }
 
-template <int DT>
-__global__ void gather_cols_kernel(const void* __restrict__ W, int64_t N, int64_t K, int64_t ldw,
-                                   const int32_t* __restrict__ perm, float* __restrict__ out, int64_t ldo) {
+// ---------------------------------------------------------------------------------------
+// columns in another order, to and from float32
+// Both kernels are bound by HBM (the weight once in, once out).  One problem (src, dst), or a batch (tables of pointers,
+// blockIdx.y = problem; dst without a table: every dst_batch elements).
+struct Columns {
+  const void* src; const void* const* src_table;
+  void* dst; void* const* dst_table; int64_t dst_batch;
+  const int32_t* perm; const int32_t* const* perm_table; int64_t perm_batch;
+  const float* const* diag_table;     // gather: columns with a zero entry come out as zeros
+  const float* damp;                  // gather of a square matrix with `rows`: diagonal 0 -> 1, + damp[problem]
+  int64_t N, K, lds, ldd;
+  bool rows;                          // gather: rows in the order of perm too
+  bool vec;                           // sizes allow 16-byte pieces (whether the addresses do is seen per problem)
+  __device__ __forceinline__ const void* in() const { return src_table ? src_table[blockIdx.y] : src; }
+  template <typename T> __device__ __forceinline__ T* out() const {
+    return dst_table ? (T*)dst_table[blockIdx.y] : (T*)dst + blockIdx.y * dst_batch;
+  }
+  __device__ __forceinline__ const int32_t* order() const {
+    return perm_table ? perm_table[blockIdx.y] : (perm ? perm + blockIdx.y * perm_batch : nullptr);
+  }
+};
+// four rows of a column, next to each other in shared memory
+template <typename T> struct alignas(4 * sizeof(T)) Quad { T v[4]; };
+
+__device__ __forceinline__ bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
+
+// Columns as they are: a thread moves 8 (a 64-bit division per element took 48 us for 4096 x 4096 where HBM needs 16).
+// Also any order, element by element, where four rows do not fit in shared memory.
+template <int DT, bool GATHER>
+__global__ void __launch_bounds__(256) plain_columns_kernel(Columns j, int tx_log2) {
   using E = Elem<DT>;
-  const int64_t total = N * K;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    int64_t r = i / K, c = i - r * K;
-    int64_t src = perm ? perm_at(perm, c, K) : c;
-    out[r * ldo + c] = E::load((const typename E::type*)W + r * ldw + src);
+  using T = typename E::type;
+  const int TX = 1 << tx_log2, tx = threadIdx.x & (TX - 1), ty = threadIdx.x >> tx_log2, rows = 256 >> tx_log2;
+  const int32_t* perm = j.order();
+  const float* dg = GATHER && j.diag_table ? j.diag_table[blockIdx.y] : nullptr;
+  const void* in = j.in();
+  const bool vec = j.vec && !perm && aligned16(in) && aligned16(GATHER ? (void*)j.template out<float>() : (void*)j.template out<T>());
+  for (int64_t r = (int64_t)blockIdx.x * rows + ty; r < j.N; r += (int64_t)gridDim.x * rows) {
+    const int64_t from = GATHER && j.rows && perm ? perm_at(perm, r, j.K) : r;
+    if (vec) {
+      for (int64_t c = tx * 8; c < j.K; c += TX * 8) {
+        alignas(16) float v[8];
+        if constexpr (GATHER) {
+          const T* w = (const T*)in + from * j.lds + c;
+          alignas(16) T t[8];
+#pragma unroll
+          for (int e = 0; e < (int)sizeof(T) / 2; ++e) reinterpret_cast<uint4*>(t)[e] = reinterpret_cast<const uint4*>(w)[e];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) v[e] = E::load(t + e);
+          if (dg) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[e] = dg[c + e] == 0.0f ? 0.0f : v[e];
+          }
+          float4* o = reinterpret_cast<float4*>(j.template out<float>() + r * j.ldd + c);
+          o[0] = make_float4(v[0], v[1], v[2], v[3]);
+          o[1] = make_float4(v[4], v[5], v[6], v[7]);
+        } else {
+          const float4* w = reinterpret_cast<const float4*>((const float*)in + r * j.lds + c);
+          *reinterpret_cast<float4*>(v) = w[0];
+          *reinterpret_cast<float4*>(v + 4) = w[1];
+          alignas(16) T t[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) E::store(t + e, v[e]);
+          T* o = j.template out<T>() + r * j.ldd + c;
+#pragma unroll
+          for (int e = 0; e < (int)sizeof(T) / 2; ++e) reinterpret_cast<uint4*>(o)[e] = reinterpret_cast<const uint4*>(t)[e];
+        }
+      }
+    } else {
+      for (int64_t c = tx; c < j.K; c += TX) {
+        const int64_t at = perm ? perm_at(perm, c, j.K) : c;
+        if constexpr (GATHER) {
+          float v = (dg && dg[c] == 0.0f) ? 0.0f : E::load((const T*)in + from * j.lds + at);
+          if (j.damp && c == r) v = (v == 0.0f ? 1.0f : v) + j.damp[blockIdx.y];
+          j.template out<float>()[r * j.ldd + c] = v;
+        } else {
+          E::store(j.template out<T>() + r * j.ldd + at, ((const float*)in)[r * j.lds + c]);
+        }
+      }
+    }
   }
 }
 
-// Batched forms for many weights of one shape (device arrays of pointers, blockIdx.y = problem):
-// the gather also zeroes the columns whose Hessian diagonal entry (after the permutation) is zero.
+// Another order: four rows at a time go through shared memory, column by column, so that the scattered side is one
+// shared-memory access for four rows and both sides of device memory stay in order (experts, 64 x 768 x 2048:
+// gather 0.5 -> see below, scatter likewise).
 template <int DT>
-__global__ void gather_cols_batched_kernel(const void* const* __restrict__ W, int64_t N, int64_t K, int64_t ldw,
-                                           const int32_t* const* __restrict__ perm,
-                                           const float* const* __restrict__ diag, float* const* __restrict__ out,
-                                           int64_t ldo) {
+__global__ void __launch_bounds__(256) gather_columns_kernel(Columns j) {
   using E = Elem<DT>;
-  const int j = blockIdx.y;
-  const typename E::type* w = (const typename E::type*)W[j];
-  const int32_t* pm = perm ? perm[j] : nullptr;
-  const float* dg = diag ? diag[j] : nullptr;
-  float* o = out[j];
-  const int64_t total = N * K;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r = i / K, c = i - r * K;
-    const int64_t src = pm ? perm_at(pm, c, K) : c;
-    const bool dead = dg && dg[c] == 0.0f;
-    o[r * ldo + c] = dead ? 0.0f : E::load(w + r * ldw + src);
+  using T = typename E::type;
+  constexpr int V = 16 / sizeof(T);
+  extern __shared__ __align__(16) unsigned char smem[];
+  Quad<T>* s = reinterpret_cast<Quad<T>*>(smem);
+  const int32_t* perm = j.order();
+  const float* dg = j.diag_table ? j.diag_table[blockIdx.y] : nullptr;
+  const T* in = (const T*)j.in();
+  float* out = j.template out<float>();
+  const bool vec = j.vec && aligned16(in);
+  for (int64_t r0 = (int64_t)blockIdx.x * 4; r0 < j.N; r0 += (int64_t)gridDim.x * 4) {
+    const int nr = (int)min((int64_t)4, j.N - r0);
+    const T* row[4];
+#pragma unroll
+    for (int y = 0; y < 4; ++y) {
+      const int64_t r = r0 + (y < nr ? y : 0);
+      row[y] = in + (j.rows ? perm_at(perm, r, j.K) : r) * j.lds;
+    }
+    if (vec) {
+      for (int c = threadIdx.x * V; c < j.K; c += 256 * V) {
+        alignas(16) T v[4][V];
+#pragma unroll
+        for (int y = 0; y < 4; ++y) *reinterpret_cast<uint4*>(v[y]) = *reinterpret_cast<const uint4*>(row[y] + c);
+#pragma unroll
+        for (int e = 0; e < V; ++e) s[c + e] = Quad<T>{{v[0][e], v[1][e], v[2][e], v[3][e]}};
+      }
+    } else {
+      for (int c = threadIdx.x; c < j.K; c += 256) s[c] = Quad<T>{{row[0][c], row[1][c], row[2][c], row[3][c]}};
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int c = threadIdx.x; c < j.K; c += 256) {
+      const Quad<T> q = s[perm_at(perm, c, j.K)];
+      const bool dead = dg && dg[c] == 0.0f;
+#pragma unroll
+      for (int y = 0; y < 4; ++y) {
+        if (y >= nr) break;
+        float v = dead ? 0.0f : E::load(&q.v[y]);
+        if (j.damp && c == r0 + y) v = (v == 0.0f ? 1.0f : v) + j.damp[blockIdx.y];
+        out[(r0 + y) * j.ldd + c] = v;
+      }
+    }
+    __syncthreads();
+  }
+}
+template <int DT>
+__global__ void __launch_bounds__(256) scatter_columns_kernel(Columns j) {
+  using E = Elem<DT>;
+  using T = typename E::type;
+  constexpr int V = 16 / sizeof(T);
+  extern __shared__ __align__(16) unsigned char smem[];
+  Quad<T>* s = reinterpret_cast<Quad<T>*>(smem);
+  const int32_t* perm = j.order();
+  const float* in = (const float*)j.in();
+  T* out = j.template out<T>();
+  const bool vec = j.vec && aligned16(out);
+  for (int64_t r0 = (int64_t)blockIdx.x * 4; r0 < j.N; r0 += (int64_t)gridDim.x * 4) {
+    const int nr = (int)min((int64_t)4, j.N - r0);
+    const float* row[4];
+#pragma unroll
+    for (int y = 0; y < 4; ++y) row[y] = in + (r0 + (y < nr ? y : 0)) * j.lds;
+#pragma unroll 4
+    for (int c = threadIdx.x; c < j.K; c += 256) {
+      Quad<T> q;
+#pragma unroll
+      for (int y = 0; y < 4; ++y) E::store(&q.v[y], row[y][c]);
+      s[perm_at(perm, c, j.K)] = q;
+    }
+    __syncthreads();
+    if (vec) {
+      for (int c = threadIdx.x * V; c < j.K; c += 256 * V) {
+        alignas(16) T v[4][V];
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+          const Quad<T> q = s[c + e];
+#pragma unroll
+          for (int y = 0; y < 4; ++y) v[y][e] = q.v[y];
+        }
+#pragma unroll
+        for (int y = 0; y < 4; ++y)
+          if (y < nr) *reinterpret_cast<uint4*>(out + (r0 + y) * j.ldd + c) = *reinterpret_cast<const uint4*>(v[y]);
+      }
+    } else {
+      for (int c = threadIdx.x; c < j.K; c += 256) {
+        const Quad<T> q = s[c];
+#pragma unroll
+        for (int y = 0; y < 4; ++y)
+          if (y < nr) out[(r0 + y) * j.ldd + c] = q.v[y];
+      }
+    }
+    __syncthreads();
   }
 }
 
-template <int DT>
-__global__ void scatter_cols_batched_kernel(const float* const* __restrict__ Wf, int64_t N, int64_t K, int64_t ldf,
-                                            const int32_t* const* __restrict__ perm, void* const* __restrict__ out,
-                                            int64_t ldo) {
-  using E = Elem<DT>;
-  const int j = blockIdx.y;
-  const float* wf = Wf[j];
-  const int32_t* pm = perm ? perm[j] : nullptr;
-  typename E::type* o = (typename E::type*)out[j];
-  const int64_t total = N * K;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r = i / K, c = i - r * K;
-    const int64_t dst = pm ? perm_at(pm, c, K) : c;
-    E::store(o + r * ldo + dst, wf[r * ldf + c]);
-  }
-}
+static bool pieces_ok(const void* p, int64_t ld, int64_t K) { return K % 8 == 0 && ld % 8 == 0 && ((uintptr_t)p & 15) == 0; }
 
-__global__ void permute_hessian_kernel(const float* __restrict__ H, int64_t K, int64_t ldh,
-                                       const int32_t* __restrict__ perm, float* __restrict__ out,
-                                       int64_t ldo) {
-  const int64_t total = K * K;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    int64_t r = i / K, c = i - r * K;
-    out[r * ldo + c] = H[perm_at(perm, r, K) * ldh + perm_at(perm, c, K)];
+template <int DT, bool GATHER>
+static int launch_columns(const Columns& j, int count, cudaStream_t st) {
+  using T = typename Elem<DT>::type;
+  const int cap = count > 1 ? 8 * kNumSMs / count + 1 : 8 * kNumSMs;
+  auto grid = [&](int64_t need) { return dim3((unsigned)(need < cap ? need : cap), (unsigned)count, 1); };
+  const bool ordered = j.perm || j.perm_table;
+  const int64_t bytes = j.K * 4 * (int64_t)sizeof(T);
+  if (ordered && bytes <= 227 * 1024) {
+    auto kernel = GATHER ? gather_columns_kernel<DT> : scatter_columns_kernel<DT>;
+    static thread_local int attr_device = -1;
+    int dev = 0;
+    B200Q_TRY(cudaGetDevice(&dev));
+    if (attr_device != dev) {
+      B200Q_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+      attr_device = dev;
+    }
+    kernel<<<grid((j.N + 3) / 4), 256, (size_t)bytes, st>>>(j);
+  } else {
+    int tx = 5;
+    while (tx < 8 && (1 << tx) * 8 < j.K) ++tx;
+    plain_columns_kernel<DT, GATHER><<<grid((j.N + (256 >> tx) - 1) / (256 >> tx)), 256, 0, st>>>(j, tx);
   }
+  B200Q_LAUNCH_CHECK();
+  return B200Q_OK;
 }
 
 // A few words of host data (pointer tables, shapes) as kernel arguments: ordered in the stream like any launch.  A copy
@@ -152,43 +299,14 @@ __global__ void __launch_bounds__(1024) diag_damp_kernel(const float* const* __r
     if (threadIdx.x == 0) damp[blockIdx.y] = percdamp * (v / (float)K);
   }
 }
-// ... and the matrix: out[r][c] = H[perm r][perm c], dead diagonal entries 1, damping added.  In place without a
-// permutation, where only the diagonal changes.
-__global__ void __launch_bounds__(256) permute_damp_kernel(float* const* __restrict__ Hs, int64_t K, int64_t ldh,
-                                                           const int32_t* __restrict__ perm, const float* __restrict__ damp,
-                                                           float* __restrict__ out) {
-  const float* H = Hs[blockIdx.y];
-  const float dm = damp[blockIdx.y];
-  if (!perm) {
-    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < K; i += (int64_t)gridDim.x * 256) {
-      const float d = H[i * ldh + i];
-      Hs[blockIdx.y][i * ldh + i] = (d == 0.0f ? 1.0f : d) + dm;
-    }
-    return;
-  }
-  const int32_t* pm = perm + blockIdx.y * K;
-  float* o = out + blockIdx.y * ((K * K + 3) & ~(int64_t)3);
-  for (int64_t r = blockIdx.x; r < K; r += gridDim.x) {
-    const float* row = H + (int64_t)pm[r] * ldh;
-    for (int64_t c = threadIdx.x; c < K; c += 256) {
-      float v = row[pm[c]];
-      if (c == r) v = (v == 0.0f ? 1.0f : v) + dm;
-      o[r * K + c] = v;
-    }
-  }
-}
-
-template <int DT>
-__global__ void scatter_cols_kernel(const float* __restrict__ Wf, int64_t N, int64_t K, int64_t ldf,
-                                    const int32_t* __restrict__ perm, void* __restrict__ out, int64_t ldo) {
-  using E = Elem<DT>;
-  const int64_t total = N * K;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    int64_t r = i / K, c = i - r * K;
-    int64_t dst = perm ? perm_at(perm, c, K) : c;
-    E::store((typename E::type*)out + r * ldo + dst, Wf[r * ldf + c]);
-  }
+// ... and, without a permutation, dead diagonal entries set to 1 and the damping added, in place.
+__global__ void __launch_bounds__(256) damp_many_kernel(float* const* __restrict__ Hs, int64_t K, int64_t ldh,
+                                                        const float* __restrict__ damp) {
+  float* H = Hs[blockIdx.y];
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= K) return;
+  const float d = H[i * ldh + i];
+  H[i * ldh + i] = (d == 0.0f ? 1.0f : d) + damp[blockIdx.y];
 }
 
 // ---------------------------------------------------------------------------------------
@@ -264,74 +382,81 @@ int b200q_gptq_prologue_many(float* const* H, int count, int64_t K, int64_t ldh,
   }
   diag_damp_kernel<<<dim3(1, (unsigned)count), 1024, 0, st>>>(H, K, ldh, perm, percdamp, diag, damp);
   B200Q_LAUNCH_CHECK();
-  const int64_t need = perm ? K : (K + 255) / 256, cap = 8 * kNumSMs / count + 1;
-  permute_damp_kernel<<<dim3((unsigned)(need < cap ? need : cap), (unsigned)count), 256, 0, st>>>(H, K, ldh, perm, damp, out);
-  B200Q_LAUNCH_CHECK();
-  return B200Q_OK;
+  if (!perm) {
+    damp_many_kernel<<<dim3((unsigned)((K + 255) / 256), (unsigned)count), 256, 0, st>>>(H, K, ldh, damp);
+    B200Q_LAUNCH_CHECK();
+    return B200Q_OK;
+  }
+  Columns j = {};
+  j.src_table = (const void* const*)H;
+  j.dst = out; j.dst_batch = (K * K + 3) & ~(int64_t)3;
+  j.perm = perm; j.perm_batch = K;
+  j.damp = damp;
+  j.N = j.K = j.ldd = K; j.lds = ldh;
+  j.rows = true;
+  j.vec = pieces_ok(nullptr, ldh, K);
+  return launch_columns<B200Q_F32, true>(j, count, st);
 }
 
 int b200q_gather_columns_f32(const void* W, int wdtype, int64_t N, int64_t K, int64_t ldw, const int32_t* perm,
                              float* Wf, int64_t ldf, void* stream) {
   if (!W || !Wf || N <= 0 || K <= 0 || ldw < K || ldf < K) return B200Q_ERR_ARG;
-  int grid = grid_for((N * K + 255) / 256, 8);
-  cudaStream_t st = (cudaStream_t)stream;
-  if (wdtype == B200Q_BF16) gather_cols_kernel<B200Q_BF16><<<grid, 256, 0, st>>>(W, N, K, ldw, perm, Wf, ldf);
-  else if (wdtype == B200Q_F32) gather_cols_kernel<B200Q_F32><<<grid, 256, 0, st>>>(W, N, K, ldw, perm, Wf, ldf);
-  else return B200Q_ERR_UNSUPPORTED;
-  B200Q_LAUNCH_CHECK();
-  return B200Q_OK;
+  Columns j = {};
+  j.src = W; j.dst = Wf; j.perm = perm;
+  j.N = N; j.K = K; j.lds = ldw; j.ldd = ldf;
+  j.vec = pieces_ok(W, ldw, K) && (perm || pieces_ok(Wf, ldf, K));
+  if (wdtype == B200Q_BF16) return launch_columns<B200Q_BF16, true>(j, 1, (cudaStream_t)stream);
+  if (wdtype == B200Q_F32) return launch_columns<B200Q_F32, true>(j, 1, (cudaStream_t)stream);
+  return B200Q_ERR_UNSUPPORTED;
 }
 
 int b200q_permute_hessian(const float* H, int64_t K, int64_t ldh, const int32_t* perm, float* Hp, int64_t ldp,
                           void* stream) {
   if (!H || !perm || !Hp || K <= 0 || ldh < K || ldp < K || H == Hp) return B200Q_ERR_ARG;
-  permute_hessian_kernel<<<grid_for((K * K + 255) / 256, 8), 256, 0, (cudaStream_t)stream>>>(H, K, ldh, perm, Hp, ldp);
-  B200Q_LAUNCH_CHECK();
-  return B200Q_OK;
+  Columns j = {};
+  j.src = H; j.dst = Hp; j.perm = perm;
+  j.N = j.K = K; j.lds = ldh; j.ldd = ldp;
+  j.rows = true;
+  j.vec = pieces_ok(H, ldh, K);
+  return launch_columns<B200Q_F32, true>(j, 1, (cudaStream_t)stream);
 }
 
 int b200q_scatter_columns_cast(const float* Wf, int64_t N, int64_t K, int64_t ldf, const int32_t* perm, void* out,
                                int odtype, int64_t ldo, void* stream) {
   if (!Wf || !out || N <= 0 || K <= 0 || ldf < K || ldo < K) return B200Q_ERR_ARG;
-  int grid = grid_for((N * K + 255) / 256, 8);
-  cudaStream_t st = (cudaStream_t)stream;
-  if (odtype == B200Q_BF16) scatter_cols_kernel<B200Q_BF16><<<grid, 256, 0, st>>>(Wf, N, K, ldf, perm, out, ldo);
-  else if (odtype == B200Q_F32) scatter_cols_kernel<B200Q_F32><<<grid, 256, 0, st>>>(Wf, N, K, ldf, perm, out, ldo);
-  else return B200Q_ERR_UNSUPPORTED;
-  B200Q_LAUNCH_CHECK();
-  return B200Q_OK;
+  Columns j = {};
+  j.src = Wf; j.dst = out; j.perm = perm;
+  j.N = N; j.K = K; j.lds = ldf; j.ldd = ldo;
+  j.vec = pieces_ok(out, ldo, K) && (perm || pieces_ok(Wf, ldf, K));
+  if (odtype == B200Q_BF16) return launch_columns<B200Q_BF16, false>(j, 1, (cudaStream_t)stream);
+  if (odtype == B200Q_F32) return launch_columns<B200Q_F32, false>(j, 1, (cudaStream_t)stream);
+  return B200Q_ERR_UNSUPPORTED;
 }
 
 int b200q_gather_columns_f32_batched(const void* const* W, int wdtype, const int32_t* const* perm,
                                      const float* const* dead_diag, float* const* Wf, int count, int64_t N,
                                      int64_t K, int64_t ldw, int64_t ldf, void* stream) {
   if (!W || !Wf || count <= 0 || count > 65535 || N <= 0 || K <= 0 || ldw < K || ldf < K) return B200Q_ERR_ARG;
-  int gx = grid_for((N * K + 255) / 256, 8);
-  const int cap = 8 * kNumSMs / count + 1;          // enough blocks over all problems to fill the machine
-  if (gx > cap) gx = cap;
-  dim3 grid((unsigned)gx, (unsigned)count, 1);
-  cudaStream_t st = (cudaStream_t)stream;
-  if (wdtype == B200Q_BF16) gather_cols_batched_kernel<B200Q_BF16><<<grid, 256, 0, st>>>(W, N, K, ldw, perm, dead_diag, Wf, ldf);
-  else if (wdtype == B200Q_F32) gather_cols_batched_kernel<B200Q_F32><<<grid, 256, 0, st>>>(W, N, K, ldw, perm, dead_diag, Wf, ldf);
-  else return B200Q_ERR_UNSUPPORTED;
-  B200Q_LAUNCH_CHECK();
-  return B200Q_OK;
+  Columns j = {};
+  j.src_table = W; j.dst_table = (void* const*)Wf; j.perm_table = perm; j.diag_table = dead_diag;
+  j.N = N; j.K = K; j.lds = ldw; j.ldd = ldf;
+  j.vec = pieces_ok(nullptr, ldw, K) && (perm || pieces_ok(nullptr, ldf, K));
+  if (wdtype == B200Q_BF16) return launch_columns<B200Q_BF16, true>(j, count, (cudaStream_t)stream);
+  if (wdtype == B200Q_F32) return launch_columns<B200Q_F32, true>(j, count, (cudaStream_t)stream);
+  return B200Q_ERR_UNSUPPORTED;
 }
 
 int b200q_scatter_columns_cast_batched(const float* const* Wf, const int32_t* const* perm, void* const* out,
                                        int odtype, int count, int64_t N, int64_t K, int64_t ldf, int64_t ldo,
                                        void* stream) {
   if (!Wf || !out || count <= 0 || count > 65535 || N <= 0 || K <= 0 || ldf < K || ldo < K) return B200Q_ERR_ARG;
-  int gx = grid_for((N * K + 255) / 256, 8);
-  const int cap = 8 * kNumSMs / count + 1;
-  if (gx > cap) gx = cap;
-  dim3 grid((unsigned)gx, (unsigned)count, 1);
-  cudaStream_t st = (cudaStream_t)stream;
-  if (odtype == B200Q_BF16) scatter_cols_batched_kernel<B200Q_BF16><<<grid, 256, 0, st>>>(Wf, N, K, ldf, perm, out, ldo);
-  else if (odtype == B200Q_F32) scatter_cols_batched_kernel<B200Q_F32><<<grid, 256, 0, st>>>(Wf, N, K, ldf, perm, out, ldo);
-  else return B200Q_ERR_UNSUPPORTED;
-  B200Q_LAUNCH_CHECK();
-  return B200Q_OK;
+  Columns j = {};
+  j.src_table = (const void* const*)Wf; j.dst_table = out; j.perm_table = perm;
+  j.N = N; j.K = K; j.lds = ldf; j.ldd = ldo;
+  j.vec = pieces_ok(nullptr, ldo, K) && (perm || pieces_ok(nullptr, ldf, K));
+  if (odtype == B200Q_BF16) return launch_columns<B200Q_BF16, false>(j, count, (cudaStream_t)stream);
+  if (odtype == B200Q_F32) return launch_columns<B200Q_F32, false>(j, count, (cudaStream_t)stream);
+  return B200Q_ERR_UNSUPPORTED;
 }
 
 int b200q_gptq_prepare(float* H, int64_t K, int64_t ldh, float* Wf, int64_t N, int64_t ldf, float percdamp,
