@@ -35,6 +35,17 @@ void count_launch();
   } while (0)
 
 // Grid size for a grid-stride kernel: whole multiples of the SM count, capped by the work.
+// CTAs of a grid-stride kernel: what is resident at once, no more.  (A grid of six CTAs per SM where five fit ran a second
+// wave of one CTA per SM: 14336 x 4096 NVFP4 codes took 99 us.)
+template <auto Kernel> inline int resident_grid(int threads, size_t smem, int64_t blocks_needed) {
+  static const int per_sm = [&] {
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, Kernel, threads, smem) != cudaSuccess || n < 1) n = 1;
+    return n;
+  }();
+  const int64_t cap = (int64_t)kNumSMs * per_sm;
+  return (int)(blocks_needed < 1 ? 1 : (blocks_needed < cap ? blocks_needed : cap));
+}
 inline int grid_for(int64_t blocks_needed, int blocks_per_sm) {
   int64_t cap = (int64_t)kNumSMs * blocks_per_sm;
   if (blocks_needed >= cap) return (int)cap;

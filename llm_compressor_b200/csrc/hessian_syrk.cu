@@ -595,25 +595,47 @@ syrk_pair_kernel(const __grid_constant__ CUtensorMap xmap, Params p) {
       if (t_end <= t_begin) continue;
       const int buf = local & 1;
       const uint32_t acc_phase = (uint32_t)((local >> 1) & 1);
-      if (!mbar_wait(accf_bar(buf), acc_phase, &s_abort, p.status, 4)) { ok = false; break; }
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int row_blk = bi * kPairTile + (int)rank * 128;   // this CTA's 128 rows of the tile
       const int row0 = row_blk + q * 32;
       const int col_base = bj * kPairTile;
       const int row_blk_end = row_blk + 128;  // columns >= this belong to the upper part
-#pragma unroll 1
+      const bool add = p.splits > 1 && !p.tile_major;   // other pairs add to this tile: atomics
+      // 32-column chunks of this warp's rows that hold something (warp-uniform)
+      const int col_end = min(row_blk_end, p.K);
+      const int nchunk = row_blk >= p.K || col_end <= col_base ? 0 : min(kPairTile / 32, (col_end - col_base + 31) / 32);
+      // H is read two chunks ahead, the first two while the MMAs still run: with one chunk at a time the latency of
+      // H stood in the way eight times a tile (22.8 us for 512 tokens at K = 4096, where the MMAs take 5)
+      constexpr int kAhead = 2;
+      float4 h[kAhead + 1][8];
+      auto fetch = [&](int c, float4 (&to)[8]) {
+        const int cc = col_base + c * 32 + sub_col;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int row = row0 + i * 4 + sub_row;
+          to[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (row < p.K && cc < p.K) to[i] = *reinterpret_cast<const float4*>(p.H + (int64_t)row * p.ldh + cc);
+        }
+      };
+      if (!add) {
+#pragma unroll
+        for (int c = 0; c < kAhead; ++c)
+          if (c < nchunk) fetch(c, h[c]);
+      }
+      if (!mbar_wait(accf_bar(buf), acc_phase, &s_abort, p.status, 4)) { ok = false; break; }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
       for (int c = 0; c < kPairTile / 32; ++c) {
-        const int col0 = col_base + c * 32;
-        if (col0 >= row_blk_end || col0 >= p.K || row_blk >= p.K) break;  // warp-uniform
+        if (c >= nchunk) break;   // warp-uniform
+        if (!add && c + kAhead < nchunk) fetch(c + kAhead, h[(c + kAhead) % (kAhead + 1)]);
         uint32_t r[32];
         tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * kPairTile + c * 32), r);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
         for (int j = 0; j < 32; ++j) stage[lane * 33 + j] = __uint_as_float(r[j]) * p.alpha;
         __syncwarp();
-        const int cc = col0 + sub_col;
+        const int cc = col_base + c * 32 + sub_col;
         if (cc < p.K) {
-          if (p.splits > 1 && !p.tile_major) {
+          if (add) {
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               const int lr = i * 4 + sub_row, row = row0 + lr;
@@ -623,20 +645,14 @@ syrk_pair_kernel(const __grid_constant__ CUtensorMap xmap, Params p) {
               }
             }
           } else {
-            float4 h[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const int row = row0 + i * 4 + sub_row;
-              h[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-              if (row < p.K) h[i] = *reinterpret_cast<const float4*>(p.H + (int64_t)row * p.ldh + cc);
-            }
+            float4 (&o)[8] = h[c % (kAhead + 1)];
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               const int lr = i * 4 + sub_row, row = row0 + lr;
               if (row < p.K) {
                 const float* sp = stage + lr * 33 + sub_col;
-                h[i].x += sp[0]; h[i].y += sp[1]; h[i].z += sp[2]; h[i].w += sp[3];
-                *reinterpret_cast<float4*>(p.H + (int64_t)row * p.ldh + cc) = h[i];
+                o[i].x += sp[0]; o[i].y += sp[1]; o[i].z += sp[2]; o[i].w += sp[3];
+                *reinterpret_cast<float4*>(p.H + (int64_t)row * p.ldh + cc) = o[i];
               }
             }
           }

@@ -556,9 +556,35 @@ __global__ void __launch_bounds__(256) group_qparams_kernel(StatJob j, int N, in
     }
   }
 }
+// rows, a warp each: no barrier between the rows of a CTA, whose loads follow one another (25 us for 6001 x 7168 with a
+// CTA per row).  For fewer rows than a few warps per SM scheduler the CTA per row below.
+__global__ void __launch_bounds__(256) row_qparams_kernel(StatJob j, int64_t N, int64_t K, int64_t ldw, QParamCfg qc) {
+  const int lane = threadIdx.x & 31;
+  const __nv_bfloat16* W = j.weight();
+  const int64_t warps = (int64_t)gridDim.x * 8;
+  for (int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); r < N; r += warps) {
+    const __nv_bfloat16* row = W + r * ldw;
+    stream::RangeQ q;
+    q.umax = q.smax = 0;   // (zeros change nothing: the range is made to contain zero anyway)
+    int64_t c = lane * 8;
+    for (; c + 7 * 256 < K; c += 8 * 256) {
+      uint4 raw[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) raw[k] = stream::ldg_stream(row + c + k * 256);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) q.add(raw[k]);
+    }
+#pragma unroll 4
+    for (; c < K; c += 256) q.add(stream::ldg_stream(row + c));
+    float lo, hi;
+    q.finish(lo, hi);
+    lo = warp_min(lo); hi = warp_max(hi);
+    if (lane == 0) j.put(r, lo, hi, qc);
+  }
+}
 // rows (bh = 1, bw = K) or bh x bw blocks: a CTA each
 __global__ void __launch_bounds__(256) span_qparams_kernel(StatJob j, int64_t N, int64_t K, int64_t ldw, int bh, int bw,
-                                                           int64_t per_row, int64_t spans, QParamCfg qc) {
+                                                           int64_t per_row, int64_t spans, int cw_log2, QParamCfg qc) {
   __shared__ float s_lo[2][8], s_hi[2][8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, cw = bw >> 3;
   const __nv_bfloat16* W = j.weight();
@@ -571,7 +597,7 @@ __global__ void __launch_bounds__(256) span_qparams_kernel(StatJob j, int64_t N,
     float lo = 0.0f, hi = 0.0f;
 #pragma unroll 4
     for (int i = threadIdx.x; i < rows * cw; i += 256) {
-      const int y = i / cw, x = (i - y * cw) * 8;
+      const int y = cw_log2 >= 0 ? i >> cw_log2 : i / cw, x = (i - y * cw) * 8;
       if (x >= cols) continue;
       stream::RangeQ r;
       r.first(stream::ldg_stream(base + (int64_t)y * ldw + x));
@@ -666,25 +692,27 @@ static int quant_launch(const void* W, int64_t N, int64_t K, int64_t ldw, const 
         int tx2 = 32;
         while (tx2 < 256 && tx2 < slots) tx2 <<= 1;
         const int rows2 = stream::kThreads / tx2;
-        const int grid2 = grid_for((N + rows2 - 1) / rows2, 6);
         const int txl2 = __builtin_ctz(tx2);
-#define B200Q_QG(RR, LL) stream::quant_group_bf16_kernel<SDT, GLOBAL, MODE, RR, LL><<<grid2, stream::kThreads, 0, st>>>(W, (int)N, (int)K, ldw, txl2, scale, zp, zp_kind, gscale, qr, out)
+#define B200Q_QG(RR, LL) const int grid2 = resident_grid<stream::quant_group_bf16_kernel<SDT, GLOBAL, MODE, RR, LL>>(stream::kThreads, 0, (N + rows2 - 1) / rows2); stream::quant_group_bf16_kernel<SDT, GLOBAL, MODE, RR, LL><<<grid2, stream::kThreads, 0, st>>>(W, (int)N, (int)K, ldw, txl2, scale, zp, zp_kind, gscale, qr, out)
         switch (g) {
-          case 8: B200Q_QG(1, 1); break;
-          case 16: B200Q_QG(2, 1); break;
-          case 32: B200Q_QG(4, 1); break;
-          case 64: B200Q_QG(4, 2); break;
-          case 128: B200Q_QG(4, 4); break;
-          default: B200Q_QG(4, 8); break;
+          case 8: { B200Q_QG(1, 1); break; }
+          case 16: { B200Q_QG(2, 1); break; }
+          case 32: { B200Q_QG(4, 1); break; }
+          case 64: { B200Q_QG(4, 2); break; }
+          case 128: { B200Q_QG(4, 4); break; }
+          default: { B200Q_QG(4, 8); break; }
         }
 #undef B200Q_QG
         B200Q_LAUNCH_CHECK();
         return B200Q_OK;
       }
     }
-    stream::RowTiling t = stream::make_tiling(N, K, 6);
-    stream::quant_rows_kernel<XDT, SDT, GLOBAL, MODE><<<t.grid, stream::kThreads, 0, st>>>(
-        W, (int)N, (int)K, ldw, __builtin_ctz(t.tx), scale, zp, zp_kind, pm, uniform, gscale, qr, out, ldo);
+    const stream::RowTiling t = stream::make_tiling(N, K, 6);
+    const int grid = resident_grid<stream::quant_rows_kernel<XDT, SDT, GLOBAL, MODE>>(stream::kThreads, 0, (N + t.rows - 1) / t.rows);
+    const int width = pm.strategy == B200Q_BLOCK ? pm.block_w : pm.group_size;
+    const int width_log2 = width > 0 && (width & (width - 1)) == 0 ? __builtin_ctz((unsigned)width) : -1;
+    stream::quant_rows_kernel<XDT, SDT, GLOBAL, MODE><<<grid, stream::kThreads, 0, st>>>(
+        W, (int)N, (int)K, ldw, __builtin_ctz(t.tx), scale, zp, zp_kind, pm, uniform, width_log2, gscale, qr, out, ldo);
   } else {
     int64_t blocks = (N * K + 255) / 256;
     quant_scalar_kernel<XDT, SDT, GLOBAL, MODE><<<grid_for(blocks, 8), 256, 0, st>>>(
@@ -1109,7 +1137,7 @@ int b200q_qparams(const void* mn, const void* mx, int stat_dtype, int64_t count,
   int rc = make_qparam_cfg(qa, stat_dtype == B200Q_BF16, gscale != nullptr, &c);
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
-  int grid = grid_for((count + 255) / 256, 4);
+  int grid = grid_for((count + 255) / 256, 8);
   if (stat_dtype == B200Q_BF16) {
     if (gscale) qparams_kernel<B200Q_BF16, true><<<grid, 256, 0, st>>>(mn, mx, count, c, gscale, scale_out, zp_out);
     else qparams_kernel<B200Q_BF16, false><<<grid, 256, 0, st>>>(mn, mx, count, c, gscale, scale_out, zp_out);
@@ -1153,7 +1181,12 @@ int b200q_minmax_qparams(const void* W, const void* const* table, int count, int
     if ((int64_t)bh * bw >= (1LL << 31)) return B200Q_ERR_UNSUPPORTED;
     const int64_t per_row = (K + bw - 1) / bw;
     j.entries = ((N + bh - 1) / bh) * per_row;
-    span_qparams_kernel<<<grid(j.entries), 256, 0, st>>>(j, N, K, ldw, bh, bw, per_row, j.entries, qc);
+    const int cw = bw / 8;
+    if (!blk && N * count >= 16 * kNumSMs)
+      row_qparams_kernel<<<grid((N + 7) / 8), 256, 0, st>>>(j, N, K, ldw, qc);
+    else
+      span_qparams_kernel<<<grid(j.entries), 256, 0, st>>>(j, N, K, ldw, bh, bw, per_row, j.entries,
+                                                           (cw & (cw - 1)) == 0 ? __builtin_ctz((unsigned)cw) : -1, qc);
   } else {
     return B200Q_ERR_UNSUPPORTED;
   }
@@ -1237,7 +1270,7 @@ int b200q_compress_scale(const void* scale, int sdtype, int64_t count, int scale
   if (!scale || !out || count <= 0) return B200Q_ERR_ARG;
   if (scale_kind != B200Q_SCALE_FP8 && scale_kind != B200Q_SCALE_E8M0) return B200Q_ERR_ARG;
   cudaStream_t st = (cudaStream_t)stream;
-  int grid = grid_for((count + 255) / 256, 4);
+  int grid = grid_for((count + 255) / 256, 8);
   if (sdtype == B200Q_BF16) compress_scale_kernel<B200Q_BF16><<<grid, 256, 0, st>>>(scale, count, scale_kind, out);
   else if (sdtype == B200Q_F32) compress_scale_kernel<B200Q_F32><<<grid, 256, 0, st>>>(scale, count, scale_kind, out);
   else return B200Q_ERR_UNSUPPORTED;

@@ -710,8 +710,9 @@ __global__ void __launch_bounds__(kThreads) minmax_group_bf16_kernel(const void*
 template <int XDT, int SDT, bool GLOBAL, int MODE>
 __global__ void __launch_bounds__(kThreads) quant_rows_kernel(
     const void* __restrict__ W, int N, int K, int64_t ldw, int tx_log2, const void* __restrict__ scale,
-    const void* __restrict__ zp, int zp_kind, ParamMap pm, bool uniform, const float* __restrict__ gscale,
+    const void* __restrict__ zp, int zp_kind, ParamMap pm, bool uniform, int width_log2, const float* __restrict__ gscale,
     QRange qr, void* __restrict__ out, int64_t ldo) {
+  // (width_log2: log2 of the columns of a block or group, -1 if that is no power of two)
   using EX = Elem<XDT>;
   using TXT = typename EX::type;
   using ES = Elem<SDT>;
@@ -724,6 +725,17 @@ __global__ void __launch_bounds__(kThreads) quant_rows_kernel(
   const int cpr = K >> 3;
   for (int row = blockIdx.x * rows + ty; row < N; row += gridDim.x * rows) {
     const TXT* wrow = (const TXT*)W + (int64_t)row * ldw;
+    // parameters of the whole row, or where this row's begin
+    const bool per_row = pm.strategy == B200Q_CHANNEL || pm.strategy == B200Q_TENSOR;
+    const int64_t row_at = uniform ? pm.index(row, 0) : 0;
+    GroupQ row_q;
+    if constexpr (XB && MODE != kFake) {
+      if (per_row) {
+        float s = ES::load((const typename ES::type*)scale + row_at);
+        if (GLOBAL) s = __fdiv_rn(s, g);
+        row_q = make_group_q<ES::is_bf16 && !GLOBAL>(s, zp ? load_zp(zp, zp_kind, row_at) : 0.0f);
+      }
+    }
     for (int c = tx; c < cpr; c += 2 * TX) {
       const int c1 = c + TX;
       const bool l1 = c1 < cpr;
@@ -743,16 +755,20 @@ __global__ void __launch_bounds__(kThreads) quant_rows_kernel(
         const int col0 = cc * 8;
         float q[8];
         if (uniform) {
-          const int64_t pi = pm.index(row, col0);
-          float s = ES::load((const typename ES::type*)scale + pi);
-          if (GLOBAL) s = __fdiv_rn(s, g);
-          const float z = zp ? load_zp(zp, zp_kind, pi) : 0.0f;
+          const int64_t pi = per_row ? row_at : row_at + (width_log2 >= 0 ? col0 >> width_log2
+                                             : col0 / (pm.strategy == B200Q_BLOCK ? pm.block_w : pm.group_size));
+          float s = 0.0f, z = 0.0f;
+          if (!(per_row && XB && MODE != kFake)) {
+            s = ES::load((const typename ES::type*)scale + pi);
+            if (GLOBAL) s = __fdiv_rn(s, g);
+            z = zp ? load_zp(zp, zp_kind, pi) : 0.0f;
+          }
           if constexpr (XB && MODE != kFake) {
             uint32_t w0 = 0, w1 = 0;
             {
               const uint4 one[1] = {raw[h]};
               uint32_t a1[1], b1[1];
-              const GroupQ gq = make_group_q<ES::is_bf16 && !GLOBAL>(s, z);
+              const GroupQ gq = per_row ? row_q : make_group_q<ES::is_bf16 && !GLOBAL>(s, z);
               if (zp) lane_codes<MODE, GLOBAL, ES::is_bf16, 1, false, true, false>(one, gq, qr, a1, b1);
               else lane_codes<MODE, GLOBAL, ES::is_bf16, 1, false, false, false>(one, gq, qr, a1, b1);
               w0 = a1[0]; w1 = b1[0];
@@ -802,21 +818,39 @@ __global__ void __launch_bounds__(kThreads) quant_group_bf16_kernel(
   const int tx = threadIdx.x & (TX - 1), ty = threadIdx.x >> tx_log2;
   const int cpr = K >> 3, gpr = cpr / cpg;
   const int slots = gpr * L;
-  for (int row = blockIdx.x * rows + ty; row < N; row += gridDim.x * rows) {
-    const T* wrow = (const T*)W + (int64_t)row * ldw;
+  // the next slot's loads are asked for before this one's codes are made: a slot of 16 elements (R = 2) alone keeps too
+  // few bytes in flight
+  auto fetch = [&](int row, int t, uint4 (&to)[R], float& s, float& z) {
+    const int grp = t / L, c0 = grp * cpg + t % L;
+    const uint4* src = reinterpret_cast<const uint4*>((const T*)W + (int64_t)row * ldw) + c0;
+#pragma unroll
+    for (int k = 0; k < R; ++k) to[k] = ldg_stream(src + k * L);
+    const int64_t pi = (int64_t)row * gpr + grp;
+    s = ES::load((const typename ES::type*)scale + pi);
+    z = zp ? load_zp(zp, zp_kind, pi) : 0.0f;
+  };
+  constexpr bool kAhead = R <= 2;
+  uint4 nraw[R];
+  float ns = 0.0f, nz = 0.0f;
+  const int first = blockIdx.x * rows + ty;
+  if (kAhead && first < N && tx < slots) fetch(first, tx, nraw, ns, nz);
+  for (int row = first; row < N; row += gridDim.x * rows) {
     for (int t = tx; t < slots; t += TX) {
       const int grp = t / L, j = t % L;
       const int c0 = grp * cpg + j;
       uint4 raw[R];
-      {
-        const uint4* src = reinterpret_cast<const uint4*>(wrow) + c0;
+      float s, z;
+      if constexpr (kAhead) {
 #pragma unroll
-        for (int k = 0; k < R; ++k) raw[k] = ldg_stream(src + k * L);
+        for (int k = 0; k < R; ++k) raw[k] = nraw[k];
+        s = ns; z = nz;
+        const bool same = t + TX < slots;
+        const int nrow = same ? row : row + gridDim.x * rows;
+        if (nrow < N) fetch(nrow, same ? t + TX : tx, nraw, ns, nz);
+      } else {
+        fetch(row, t, raw, s, z);
       }
-      const int64_t pi = (int64_t)row * gpr + grp;
-      float s = ES::load((const typename ES::type*)scale + pi);
       if (GLOBAL) s = __fdiv_rn(s, gs);
-      const float z = zp ? load_zp(zp, zp_kind, pi) : 0.0f;
       const GroupQ gq = make_group_q<ES::is_bf16 && !GLOBAL>(s, z);
       uint32_t a[R], b[R];
       if (zp) lane_codes<MODE, GLOBAL, ES::is_bf16, R, false, true, false>(raw, gq, qr, a, b);

@@ -80,6 +80,46 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
       ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1) : "memory");
 }
+// CTA pairs (cta_group::2): the same location in CTA `rank` of the cluster, a load whose bytes count on a barrier of the
+// even CTA, an arrival there, and the commit that arrives in both CTAs
+__device__ __forceinline__ uint32_t cluster_ctarank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) {
+  uint32_t out;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(addr), "r"(rank));
+  return out;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar_cluster_addr,
+                                                 int c0, int c1) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4}], [%2];"
+      ::"r"(dst), "l"(map), "r"(bar_cluster_addr), "r"(c0), "r"(c1) : "memory");
+}
+__device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
+  const uint16_t both = 3;
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+      ::"r"(bar), "h"(both) : "memory");
+}
+__device__ __forceinline__ void mma_tf32_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                              uint32_t accumulate) {
+  const uint32_t z = 0;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(z) : "memory");
+}
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
@@ -109,47 +149,52 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t lbo_bytes
   d |= (uint64_t)2 << 61;
   return d;
 }
-// D fp32, A/B tf32, both K-major, M = 128, N = tn
-__host__ __device__ constexpr uint32_t instr_desc(int tn) {
-  return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(tn >> 3) << 17) | ((uint32_t)(kTile >> 4) << 24);
+// D fp32, A/B tf32, both K-major, M = tm, N = tn
+__host__ __device__ constexpr uint32_t instr_desc(int tm, int tn) {
+  return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(tn >> 3) << 17) | ((uint32_t)(tm >> 4) << 24);
 }
 
 struct Params {
   Job j;
-  int row_tiles, tn_log2;
+  int row_tiles, tm_rows, tn_log2;      // rows of a tile: 128, or 256 for a CTA pair
   int64_t num_tiles;                    // over all problems
-  uint16_t start[kNumSMs][3];           // (problem, row tile, column tile) each CTA starts at
+  uint16_t start[kNumSMs][3];           // (problem, row tile, column tile) each CTA or pair starts at
 };
 
-__host__ __device__ __forceinline__ int tile_row(const Job& j, int tm) {
-  int r = j.row_begin + tm * kTile;
+__host__ __device__ __forceinline__ int tile_row(const Job& j, int tm, int rows) {
+  int r = j.row_begin + tm * rows;
   if (j.set == kPanel && r >= j.skip0) r += j.skip1 - j.skip0;
   return r;
 }
 // column tiles of row tile tm (they are contiguous from column 0)
-__host__ __device__ __forceinline__ int col_tiles(const Job& j, int tm, int tn_log2) {
+__host__ __device__ __forceinline__ int col_tiles(const Job& j, int tm, int rows, int tn_log2) {
   int lim = j.N;
   if (j.set == kLower || j.set == kBulk) {
-    const int r = tile_row(j, tm);
-    const int diag = (j.set == kBulk && r < j.skip1) ? j.skip0 : r + kTile;
+    const int r = tile_row(j, tm, rows);
+    const int diag = (j.set == kBulk && r < j.skip1) ? j.skip0 : r + rows;
     lim = diag < lim ? diag : lim;
   }
   return (lim + (1 << tn_log2) - 1) >> tn_log2;
 }
-__host__ __device__ __forceinline__ void next_tile(const Params& p, int& b, int& tm, int& tn) {
+__device__ __forceinline__ void next_tile(const Params& p, int& b, int& tm, int& tn) {
   ++tn;
-  while (tn >= col_tiles(p.j, tm, p.tn_log2)) {   // a row tile may have no column at all
+  while (tn >= col_tiles(p.j, tm, p.tm_rows, p.tn_log2)) {   // a row tile may have no column at all
     tn = 0;
     if (++tm == p.row_tiles) { tm = 0; ++b; return; }
   }
 }
 
-template <int TN, bool SPLIT_OUT>
+// PAIR: two CTAs on neighbouring SMs (a cluster of 2) share a 256 x 256 tile.  One MMA issued by the even CTA runs on both
+// SMs; each stages its own 128 rows of A and its own 128 of B, 64 KiB a chunk instead of 96, and has its own half of the
+// accumulator and its own epilogue.  full[] and acc_empty[] live in the even CTA, empty[] and acc_full[] in both.
+template <int TN, bool SPLIT_OUT, bool PAIR>
 __global__ void __launch_bounds__(kThreads, 1)
 tgemm_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ CUtensorMap a_lo,
              const __grid_constant__ CUtensorMap b_hi, const __grid_constant__ CUtensorMap b_lo,
              const __grid_constant__ Params p) {
-  constexpr int kBPart = TN * kChunkK * 4;
+  constexpr int kRows = PAIR ? 2 * kTile : kTile;      // rows of a tile
+  constexpr int kBRows = PAIR ? TN / 2 : TN;           // rows of B that this CTA stages
+  constexpr int kBPart = kBRows * kChunkK * 4;
   constexpr int kStageBytes = 2 * kAPart + 2 * kBPart;
   constexpr int kStages = kRingBytes / kStageBytes;
   constexpr uint32_t kTmemCols = 2 * TN;
@@ -166,26 +211,35 @@ tgemm_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ C
   __shared__ uint32_t s_tmem_base;
   __shared__ volatile int s_abort;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = PAIR ? (int)cluster_ctarank() : 0;
+  const int unit = PAIR ? blockIdx.x >> 1 : blockIdx.x, units = PAIR ? gridDim.x >> 1 : gridDim.x;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(accf_bar(b), 1); mbar_init(acce_bar(b), kEpiWarps); }
+    for (int b = 0; b < 2; ++b) { mbar_init(accf_bar(b), 1); mbar_init(acce_bar(b), PAIR ? 2 * kEpiWarps : kEpiWarps); }
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem_base)),
-                 "r"(kTmemCols) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    if constexpr (PAIR) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem_base)),
+                   "r"(kTmemCols) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem_base)),
+                   "r"(kTmemCols) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (PAIR) cluster_sync_all();   // the peer's barriers are initialised before anything signals them
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = s_tmem_base;
   const Job& j = p.j;
   const int chunks = (j.Kd + kChunkK - 1) / kChunkK;
-  const int64_t count = p.num_tiles * (blockIdx.x + 1) / gridDim.x - p.num_tiles * blockIdx.x / gridDim.x;
-  int b = p.start[blockIdx.x][0], tm = p.start[blockIdx.x][1], tn = p.start[blockIdx.x][2];
+  const int64_t count = p.num_tiles * (unit + 1) / units - p.num_tiles * unit / units;
+  int b = p.start[unit][0], tm = p.start[unit][1], tn = p.start[unit][2];
 
   if (warp < kFirstEpiWarp) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kIssueRegs));
@@ -194,25 +248,34 @@ tgemm_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ C
       uint32_t phase = 0;
       bool ok = true;
       for (int64_t i = 0; i < count && ok; ++i, next_tile(p, b, tm, tn)) {
-        const int ra = (int)(b * j.A.batch_rows) + j.A.row0 + tile_row(j, tm);
-        const int rb = (int)((j.b_index ? j.b_index[b] : b) * j.B.batch_rows) + j.B.row0 + tn * TN;
+        const int ra = (int)(b * j.A.batch_rows) + j.A.row0 + tile_row(j, tm, kRows) + rank * kTile;
+        const int rb = (int)((j.b_index ? j.b_index[b] : b) * j.B.batch_rows) + j.B.row0 + tn * TN + rank * kBRows;
         for (int c = 0; c < chunks; ++c) {
           if (!mbar_wait(empty_bar(stage), phase ^ 1u, &s_abort)) { ok = false; break; }
-          mbar_expect_tx(full_bar(stage), kStageBytes);
           const uint32_t s = base + stage * kStageBytes;
+          if constexpr (PAIR) {
+            if (rank == 0) mbar_expect_tx(full_bar(stage), 2 * kStageBytes);
+            const uint32_t full = map_to_cta(full_bar(stage), 0);
+            tma_load_2d_pair(s, &a_hi, full, c * kChunkK, ra);
+            tma_load_2d_pair(s + 2 * kAPart, &b_hi, full, c * kChunkK, rb);
+            tma_load_2d_pair(s + 2 * kAPart + kBPart, &b_lo, full, c * kChunkK, rb);
+            tma_load_2d_pair(s + kAPart, &a_lo, full, c * kChunkK, ra);
+          } else {
+          mbar_expect_tx(full_bar(stage), kStageBytes);
           tma_load_2d(s, &a_hi, full_bar(stage), c * kChunkK, ra);
           tma_load_2d(s + 2 * kAPart, &b_hi, full_bar(stage), c * kChunkK, rb);
           tma_load_2d(s + 2 * kAPart + kBPart, &b_lo, full_bar(stage), c * kChunkK, rb);
           tma_load_2d(s + kAPart, &a_lo, full_bar(stage), c * kChunkK, ra);
+          }
           if (++stage == kStages) { stage = 0; phase ^= 1u; }
         }
       }
     }
-    if (warp == 1) {
+    if (warp == 1 && rank == 0) {
     int stage = 0, slice = 0;
     uint32_t phase = 0;
     bool ok = true;
-    constexpr uint32_t idesc = instr_desc(TN);
+    constexpr uint32_t idesc = instr_desc(kRows, TN);
     for (int64_t i = 0; i < count && ok; ++i) {
       for (int c = 0; c < chunks; ++c) {
         const int buf = slice & 1;
@@ -230,12 +293,23 @@ tgemm_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ C
             const uint64_t al = make_desc(sa + kAPart + kk * 32, 16, 1024);
             const uint64_t bh = make_desc(sb + kk * 32, 16, 1024);
             const uint64_t bl = make_desc(sb + kBPart + kk * 32, 16, 1024);
-            mma_tf32(d_tmem, ah, bh, idesc, (first && kk == 0) ? 0u : 1u);
-            mma_tf32(d_tmem, ah, bl, idesc, 1u);
-            mma_tf32(d_tmem, al, bh, idesc, 1u);
+            if constexpr (PAIR) {
+              mma_tf32_pair(d_tmem, ah, bh, idesc, (first && kk == 0) ? 0u : 1u);
+              mma_tf32_pair(d_tmem, ah, bl, idesc, 1u);
+              mma_tf32_pair(d_tmem, al, bh, idesc, 1u);
+            } else {
+              mma_tf32(d_tmem, ah, bh, idesc, (first && kk == 0) ? 0u : 1u);
+              mma_tf32(d_tmem, ah, bl, idesc, 1u);
+              mma_tf32(d_tmem, al, bh, idesc, 1u);
+            }
           }
-          tc_commit(empty_bar(stage));
-          if (last) tc_commit(accf_bar(buf));
+          if constexpr (PAIR) {
+            tc_commit_pair(empty_bar(stage));
+            if (last) tc_commit_pair(accf_bar(buf));
+          } else {
+            tc_commit(empty_bar(stage));
+            if (last) tc_commit(accf_bar(buf));
+          }
         }
         __syncwarp();
         if (last) ++slice;
@@ -254,7 +328,7 @@ tgemm_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ C
     int slice = 0;
     bool ok = true;
     for (int64_t i = 0; i < count && ok; ++i, next_tile(p, b, tm, tn)) {
-      const int row0 = tile_row(j, tm) + q * 32, colw = tn * TN + half * kHalf;
+      const int row0 = tile_row(j, tm, kRows) + rank * kTile + q * 32, colw = tn * TN + half * kHalf;
       float sum[kHalf];
       for (int c = 0; c < chunks; c += kSliceChunks, ++slice) {
         const int buf = slice & 1;
@@ -271,7 +345,10 @@ tgemm_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ C
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
-        if (lane == 0) mbar_arrive(acce_bar(buf));
+        if (lane == 0) {
+          if (rank == 0) mbar_arrive(acce_bar(buf));
+          else mbar_arrive_cluster(map_to_cta(acce_bar(buf), 0));
+        }
       }
       if (!ok) break;
       float* C = nullptr;
@@ -368,9 +445,13 @@ tgemm_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ C
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (PAIR) cluster_sync_all();   // nothing of the peer's is still on its way here
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
+    if constexpr (PAIR)
+      asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
+    else
+      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
   }
 }
 
@@ -505,50 +586,107 @@ inline MapCache& map_cache() {
   return c;
 }
 
-static int64_t count_tiles(const Job& j, int row_tiles, int tn_log2) {
-  if (j.set == kAll || j.set == kPanel) return (int64_t)row_tiles * col_tiles(j, 0, tn_log2);
+// Row tiles of `rows` rows: kPanel leaves out [skip0, skip1), which tiles of 256 rows can only do at multiples of 256.
+static int count_rows(const Job& j, int rows) {
+  if (j.set != kPanel) return j.M > j.row_begin ? (j.M - j.row_begin + rows - 1) / rows : 0;
+  return j.skip0 / rows + (j.M > j.skip1 ? (j.M - j.skip1 + rows - 1) / rows : 0);
+}
+static bool rows_fit(const Job& j, int rows) {
+  if (j.set == kPanel) return j.skip0 % rows == 0;
+  return j.set != kBulk || j.skip1 <= j.row_begin || (j.skip1 - j.row_begin) % rows == 0;
+}
+static int64_t count_tiles(const Job& j, int rows, int tn_log2) {
+  const int row_tiles = count_rows(j, rows);
+  if (j.set == kAll || j.set == kPanel) return row_tiles ? (int64_t)row_tiles * col_tiles(j, 0, rows, tn_log2) : 0;
   int64_t n = 0;
-  for (int tm = 0; tm < row_tiles; ++tm) n += col_tiles(j, tm, tn_log2);
+  for (int tm = 0; tm < row_tiles; ++tm) n += col_tiles(j, tm, rows, tn_log2);
   return n;
 }
 
-// Tile width: SM cycles of the busiest CTA.  A 32-deep chunk takes the longer of its MMAs (12 of 32 / 64 /
-// 128 cycles) and the arrival of its operands from L2 (about 64 B/clk and SM); the last tile's epilogue,
-// about 20 cycles per column, is not hidden.
-static int pick_width(const Job& j, int row_tiles, int ctas) {
-  const double chunk[3] = {800.0, 1150.0, 1700.0};
-  const int chunks = (j.Kd + kChunkK - 1) / kChunkK;
-  int best = 6;
-  double best_cost = 0.0;
-  for (int w = 6; w <= 8; ++w) {
-    const int64_t tiles = count_tiles(j, row_tiles, w) * j.batch;
-    const double cost = (double)((tiles + ctas - 1) / ctas) * chunks * chunk[w - 6] + 20.0 * (1 << w);
-    if (w == 6 || cost < best_cost) { best = w; best_cost = cost; }
+// CTA pairs that can be resident at once on the current device; 0 if a cluster of two cannot be launched
+static int pair_capacity() {
+  static std::mutex mu;
+  static int cached[64];
+  static bool have[64] = {false};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  std::lock_guard<std::mutex> lock(mu);
+  if (have[dev]) return cached[dev];
+  auto kernel = tgemm_kernel<256, false, true>;
+  int n = 0;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) == cudaSuccess) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * (kNumSMs / 2), 1, 1);
+    cfg.blockDim = dim3(kThreads, 1, 1);
+    cfg.dynamicSmemBytes = kSmemBytes;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) n = 0;
   }
-  return best;
+  (void)cudaGetLastError();
+  cached[dev] = n < 0 ? 0 : (n < kNumSMs / 2 ? n : kNumSMs / 2);
+  have[dev] = true;
+  return cached[dev];
 }
 
-template <int TN>
-static int launch_width(const Params& p, int grid, cudaStream_t st) {
+// Tile width, and whether CTA pairs take 256 x 256: SM cycles of the busiest CTA.  A 32-deep chunk takes the longer of its
+// MMAs (12 of 32 / 64 / 128 cycles) and the arrival of its operands from L2 (about 64 B/clk and SM); the last tile's
+// epilogue, about 20 cycles per column, is not hidden.
+static void pick_tiles(Params& p, int ctas, int pairs) {
+  const double chunk[3] = {800.0, 1150.0, 1700.0};
+  static const double pair_chunk = [] { const char* e = getenv("PAIR_CHUNK"); return e ? atof(e) : 1600.0; }();
   const Job& j = p.j;
+  const int chunks = (j.Kd + kChunkK - 1) / kChunkK;
+  double best_cost = 0.0;
+  for (int w = 6; w <= 8; ++w) {
+    const int64_t tiles = count_tiles(j, kTile, w) * j.batch;
+    const double cost = (double)((tiles + ctas - 1) / ctas) * chunks * chunk[w - 6] + 20.0 * (1 << w);
+    if (w == 6 || cost < best_cost) { p.tn_log2 = w; p.tm_rows = kTile; best_cost = cost; }
+  }
+  if (pairs > 0 && rows_fit(j, 2 * kTile)) {
+    const int64_t tiles = count_tiles(j, 2 * kTile, 8) * j.batch;
+    const double cost = (double)((tiles + pairs - 1) / pairs) * chunks * pair_chunk + 20.0 * 256;
+    if (cost < best_cost) { p.tn_log2 = 8; p.tm_rows = 2 * kTile; }
+  }
+}
+
+template <int TN, bool SPLIT_OUT, bool PAIR>
+static int launch_tiles(const Params& p, int units, cudaStream_t st) {
+  const Job& j = p.j;
+  constexpr int kBRows = PAIR ? TN / 2 : TN;
   MapCache& mc = map_cache();
   CUtensorMap mah, mal, mbh, mbl;
   if (!mc.get(j.A.hi, j.A.ld, j.A.rows, kTile, &mah) || !mc.get(j.A.lo, j.A.ld, j.A.rows, kTile, &mal) ||
-      !mc.get(j.B.hi, j.B.ld, j.B.rows, TN, &mbh) || !mc.get(j.B.lo, j.B.ld, j.B.rows, TN, &mbl)) {
+      !mc.get(j.B.hi, j.B.ld, j.B.rows, kBRows, &mbh) || !mc.get(j.B.lo, j.B.ld, j.B.rows, kBRows, &mbl)) {
     set_last_error("cuTensorMapEncodeTiled (tgemm)", cudaErrorInvalidValue);
     return B200Q_ERR_CUDA;
   }
-  const bool split_out = j.out_hi || j.X;
+  auto kernel = tgemm_kernel<TN, SPLIT_OUT, PAIR>;
   static thread_local int attr_device = -1;
   int dev = 0;
   B200Q_TRY(cudaGetDevice(&dev));
   if (attr_device != dev) {
-    B200Q_TRY(cudaFuncSetAttribute(tgemm_kernel<TN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-    B200Q_TRY(cudaFuncSetAttribute(tgemm_kernel<TN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
+    B200Q_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
     attr_device = dev;
   }
-  if (split_out) tgemm_kernel<TN, true><<<grid, kThreads, kSmemBytes, st>>>(mah, mal, mbh, mbl, p);
-  else tgemm_kernel<TN, false><<<grid, kThreads, kSmemBytes, st>>>(mah, mal, mbh, mbl, p);
+  if constexpr (PAIR) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(2 * units), 1, 1);
+    cfg.blockDim = dim3(kThreads, 1, 1);
+    cfg.dynamicSmemBytes = kSmemBytes;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    B200Q_TRY(cudaLaunchKernelEx(&cfg, kernel, mah, mal, mbh, mbl, p));
+  } else {
+    kernel<<<units, kThreads, kSmemBytes, st>>>(mah, mal, mbh, mbl, p);
+  }
   B200Q_LAUNCH_CHECK();
   return B200Q_OK;
 }
@@ -557,33 +695,34 @@ int launch(const Job& j, cudaStream_t st) {
   if (j.Kd <= 0 || j.batch <= 0) return B200Q_OK;
   if (j.Kd > kMaxDepth || j.batch > 65535 || (j.A.ld & 31) || (j.B.ld & 31) || j.A.ld < j.Kd || j.B.ld < j.Kd)
     return B200Q_ERR_ARG;
+  if (count_rows(j, kTile) <= 0 || j.N <= 0) return B200Q_OK;
   Params p;
   p.j = j;
-  if (j.set == kPanel) {
-    const int above = j.skip0 / kTile, below = j.M > j.skip1 ? (j.M - j.skip1 + kTile - 1) / kTile : 0;
-    p.row_tiles = above + below;
-  } else {
-    p.row_tiles = j.M > j.row_begin ? (j.M - j.row_begin + kTile - 1) / kTile : 0;
-  }
-  if (p.row_tiles <= 0 || j.N <= 0) return B200Q_OK;
   const int ctas = j.max_ctas > 0 && j.max_ctas < kNumSMs ? j.max_ctas : kNumSMs;
-  p.tn_log2 = pick_width(j, p.row_tiles, ctas);
-  const int64_t per_problem = count_tiles(j, p.row_tiles, p.tn_log2);
+  const int resident = pair_capacity(), pairs = ctas / 2 < resident ? ctas / 2 : resident;
+  pick_tiles(p, ctas, pairs);
+  p.row_tiles = count_rows(j, p.tm_rows);
+  const bool pair = p.tm_rows == 2 * kTile;
+  const int64_t per_problem = count_tiles(j, p.tm_rows, p.tn_log2);
   p.num_tiles = per_problem * j.batch;
-  const int grid = (int)(p.num_tiles < ctas ? p.num_tiles : ctas);
-  // where each CTA's range starts: problem, row tile, column tile
+  if (p.num_tiles <= 0) return B200Q_OK;
+  const int most = pair ? pairs : ctas;
+  const int units = (int)(p.num_tiles < most ? p.num_tiles : most);
+  // where each CTA's (pair's) range starts: problem, row tile, column tile
   int tm = 0;
   int64_t before = 0, of = 0;   // tiles before row tile tm of problem `of`
-  for (int i = 0; i < grid; ++i) {
-    const int64_t t = p.num_tiles * i / grid, b = t / per_problem, in = t - b * per_problem;
+  for (int i = 0; i < units; ++i) {
+    const int64_t t = p.num_tiles * i / units, b = t / per_problem, in = t - b * per_problem;
     if (b != of) { of = b; tm = 0; before = 0; }
     int64_t n;
-    while (in >= before + (n = col_tiles(j, tm, p.tn_log2))) { before += n; ++tm; }
+    while (in >= before + (n = col_tiles(j, tm, p.tm_rows, p.tn_log2))) { before += n; ++tm; }
     p.start[i][0] = (uint16_t)b; p.start[i][1] = (uint16_t)tm; p.start[i][2] = (uint16_t)(in - before);
   }
-  if (p.tn_log2 == 8) return launch_width<256>(p, grid, st);
-  if (p.tn_log2 == 7) return launch_width<128>(p, grid, st);
-  return launch_width<64>(p, grid, st);
+  const bool split_out = j.out_hi || j.X;
+  if (pair) return split_out ? launch_tiles<256, true, true>(p, units, st) : launch_tiles<256, false, true>(p, units, st);
+  if (p.tn_log2 == 8) return split_out ? launch_tiles<256, true, false>(p, units, st) : launch_tiles<256, false, false>(p, units, st);
+  if (p.tn_log2 == 7) return split_out ? launch_tiles<128, true, false>(p, units, st) : launch_tiles<128, false, false>(p, units, st);
+  return split_out ? launch_tiles<64, true, false>(p, units, st) : launch_tiles<64, false, false>(p, units, st);
 }
 
 SideStream* side_stream(cudaStream_t like) {

@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import collections
 import contextlib
+import math
 import re
 import time
 import warnings
@@ -185,7 +186,7 @@ class QuantizationMixin(HooksMixin):
         parameters to every targeted module (CT lifecycle/initialize.py:132-254)."""
         groups = self.resolve_quantization_config()
         self._resolved = groups
-        bad = []
+        bad, zero_points = [], {}
         for scheme in groups.values():
             for name, module in match_named_modules(model, scheme.targets, self.ignore):
                 if not hasattr(module, "weight") or module.weight is None or module.weight.ndim != 2:
@@ -200,8 +201,8 @@ class QuantizationMixin(HooksMixin):
                         and not self.bypass_divisibility_checks):
                     bad.append((name, K, w.group_size))
                     continue
-                module.quantization_scheme = scheme
-                module.quantization_status = "initialized"   # "frozen" once its qparams are written
+                _set_plain(module, "quantization_scheme", scheme)
+                _set_plain(module, "quantization_status", "initialized")   # "frozen" once its qparams are written
                 self._module_names[module] = name
                 weight = module.weight
                 dev, dt = weight.device, weight.dtype
@@ -213,7 +214,7 @@ class QuantizationMixin(HooksMixin):
                     reg("weight_global_scale", torch.empty(1, dtype=torch.float32, device=dev))
                 reg("weight_scale", torch.empty(shape, dtype=dt if dt.is_floating_point else torch.float16,
                                                 device=dev))
-                reg("weight_zero_point", torch.zeros(shape, dtype=w.zp_dtype, device=dev))
+                zero_points.setdefault(dev, []).append((module, shape, w.zp_dtype))
                 if w.actorder == "group":
                     reg("weight_g_idx", torch.full((K,), -1, dtype=torch.int32, device=dev))
                 a = scheme.input_activations
@@ -228,6 +229,12 @@ class QuantizationMixin(HooksMixin):
                         reg("input_scale", torch.empty(1, dtype=dt if dt.is_floating_point else torch.float16,
                                                        device=dev))
                         reg("input_zero_point", torch.zeros(1, dtype=a.zp_dtype, device=dev))
+        for dev, wanted in zero_points.items():
+            # one launch clears them all (a module's own tensor took 8 us of host time and a launch)
+            sizes = [-(-math.prod(shape) * dtype.itemsize // 16) * 16 for _, shape, dtype in wanted]
+            for (module, shape, dtype), piece in zip(wanted, torch.zeros(sum(sizes), dtype=torch.uint8, device=dev).split(sizes)):
+                zp = piece.view(dtype)[:math.prod(shape)].view(shape)
+                module.register_parameter("weight_zero_point", torch.nn.Parameter(zp, requires_grad=False))
         if self.kv_cache_scheme is not None:
             # attention modules get k_scale / v_scale (CT lifecycle/initialize.py:255-310); the scheme
             # sits on the module as its input_activations, as the reference's config resolution puts it
@@ -264,8 +271,8 @@ class QuantizationMixin(HooksMixin):
         shared = False   # some weights have a global scale that siblings share
         for _, module in self.quantized_modules(model):
             w = module.quantization_scheme.weights
-            module.weight_observer = Observer.load_from_registry(
-                w.observer or "memoryless_minmax", base_name="weight", args=w)
+            _set_plain(module, "weight_observer", Observer.load_from_registry(
+                w.observer or "memoryless_minmax", base_name="weight", args=w))
             shared = shared or w.strategy == "tensor_group"
             a = module.quantization_scheme.input_activations
             if a is not None and a.dynamic is not True:
@@ -392,7 +399,13 @@ def _write_qparams(m, base_name, scale, zero_point, global_scale) -> None:
         if p is not None:
             _put(p, val)
     if base_name == "weight":
-        m.quantization_status = "frozen"
+        _set_plain(m, "quantization_status", "frozen")
+
+
+def _set_plain(module, name, value) -> None:
+    """``setattr`` for a value that is no parameter, buffer or submodule: torch's own looks for all of these first, in
+    Python, at 4 us an attribute."""
+    object.__setattr__(module, name, value)
 
 
 def _put(p: torch.Tensor, val: torch.Tensor) -> None:
@@ -764,7 +777,7 @@ class GPTQModifier(QuantizationMixin):
                     _put(p, val)
                 else:
                     module.register_parameter(attr, torch.nn.Parameter(val, requires_grad=False))
-            module.quantization_status = "frozen"
+            _set_plain(module, "quantization_status", "frozen")
             self._done.add(module)
 
     def _compress_group(self, module_list):

@@ -44,6 +44,7 @@ class Observer:
         self._fused_weights: list = []  # callables returning the partner's weight
         self._own_weight = None
         self._deletion_called = False
+        self._absmax = None           # (min_vals, max_vals, their largest magnitude)
 
     # ---- registry (RegistryMixin-like) -------------------------------------------------
     @classmethod
@@ -138,9 +139,16 @@ class Observer:
             return None
         self._observe_partners()
         members = [self] + self._fused
-        absmax = torch.zeros(1, dtype=torch.float32, device=self.min_vals.device)
-        for m in members:
-            ops.absmax_accumulate(m.min_vals, m.max_vals, absmax)
+        known = [m._absmax[2] for m in members
+                 if m._absmax is not None and m._absmax[0] is m.min_vals and m._absmax[1] is m.max_vals]
+        if len(known) == len(members):   # found while the statistics were made
+            absmax = known[0]
+            for other in known[1:]:
+                absmax = torch.maximum(absmax, other)
+        else:
+            absmax = torch.zeros(1, dtype=torch.float32, device=self.min_vals.device)
+            for m in members:
+                ops.absmax_accumulate(m.min_vals, m.max_vals, absmax)
         return ops.global_scale_from_absmax(absmax, self.min_vals.dtype)
 
     @torch.no_grad()
@@ -170,6 +178,10 @@ def direct_qparams(observers, weights):
 @Observer.register("memoryless_minmax")
 class MemorylessMinMaxObserver(Observer):
     def update_statistics_from_weight(self, weight):
+        made = ops.observe_minmax_absmax(weight, self.args) if self.args.strategy == "tensor_group" else None
+        if made is not None:
+            self.min_vals, self.max_vals, _ = self._absmax = made
+            return
         self.min_vals, self.max_vals = ops.observe_minmax(weight, self.args)
 
 

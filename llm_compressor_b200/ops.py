@@ -57,6 +57,24 @@ def observe_minmax(w: torch.Tensor, args: QuantizationArgs):
     return mn, mx
 
 
+def observe_minmax_absmax(w: torch.Tensor, args: QuantizationArgs):
+    """(min_vals, max_vals, largest magnitude of w as float32 [1]) in one pass, or None for what it does not take."""
+    _need_cuda(w)
+    N, K, ld = _2d(w)
+    if w.dtype != torch.bfloat16:
+        return None
+    shape = args.qparam_shape(N, K)
+    mn = torch.empty(shape, dtype=w.dtype, device=w.device)
+    mx = torch.empty(shape, dtype=w.dtype, device=w.device)
+    absmax = torch.zeros(1, dtype=torch.float32, device=w.device)
+    rc = _lib.load().b200q_observe_minmax_absmax(ptr(w), _dt(w), N, K, ld, args.c_struct(), ptr(mn), ptr(mx), None,
+                                                 ptr(absmax), stream_ptr())
+    if rc == -2:
+        return None
+    check(rc, "b200q_observe_minmax_absmax")
+    return mn, mx, absmax
+
+
 def minmax_qparams(w, args: QuantizationArgs):
     """``qparams(*observe_minmax(w, args), args)`` in one launch: (scale, zero_point), or None for what it does not take.
     ``w`` may be a list of weights of one shape and layout: the results then carry a leading dimension."""
