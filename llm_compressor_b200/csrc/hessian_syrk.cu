@@ -176,6 +176,7 @@ struct Params {
                              // the other, and adds them into H without atomics (bitwise reproducible)
   float alpha;
   int* status;
+  int red;
 };
 
 __global__ void __launch_bounds__(kThreads, 1)
@@ -599,7 +600,7 @@ syrk_pair_kernel(const __grid_constant__ CUtensorMap xmap, Params p) {
       const int row0 = row_blk + q * 32;
       const int col_base = bj * kPairTile;
       const int row_blk_end = row_blk + 128;  // columns >= this belong to the upper part
-      const bool add = p.splits > 1 && !p.tile_major;   // other pairs add to this tile: atomics
+      const bool add = (p.splits > 1 && !p.tile_major) || p.red;   // other pairs add to this tile: atomics
       // 32-column chunks of this warp's rows that hold something (warp-uniform)
       const int col_end = min(row_blk_end, p.K);
       const int nchunk = row_blk >= p.K || col_end <= col_base ? 0 : min(kPairTile / 32, (col_end - col_base + 31) / 32);
@@ -858,6 +859,7 @@ int b200q_hessian_syrk(const void* X, int64_t T, int64_t K, int64_t ldx, float* 
   Params p;
   p.H = H; p.ldh = ldh; p.K = (int)K; p.T = T; p.alpha = alpha; p.status = status;
   p.tile_major = 0;
+  { static const int red = [] { const char* e = getenv("SYRK_RED"); return e ? atoi(e) : 0; }(); p.red = red; }
   cudaStream_t st = (cudaStream_t)stream;
   const int pairs = pair_capacity();
   if (pairs > 0) {

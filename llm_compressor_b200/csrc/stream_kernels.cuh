@@ -278,6 +278,20 @@ __device__ __forceinline__ uint32_t nvfp4_8(const uint4& raw, float rs, bool& un
   return c;
 }
 
+// The same with the division itself: the converter rounds like e2m1_round (to nearest, ties to the even code, the sign kept),
+// so only the quotients cost more (the general exact path, which also emulates the rounding, made a 14336 x 4096 weight
+// with outliers take 93 us instead of 35).
+__device__ __noinline__ uint32_t nvfp4_8_exact(uint4 raw, float se, float z) {
+  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+  float f[8];
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    f[2 * p] = __fdiv_rn(__uint_as_float(w[p] << 16), se) + z;
+    f[2 * p + 1] = __fdiv_rn(__uint_as_float(w[p] & 0xFFFF0000u), se) + z;
+  }
+  return cvt_e2m1x8(f);
+}
+
 // ---------------------------------------------------------------------------------------
 // per-group min / max
 template <int DT>
@@ -523,10 +537,8 @@ __device__ __forceinline__ void lane_codes(const uint4 (&raw)[R], const GroupQ& 
     for (int k = 0; k < R; ++k) {
       bool unsafe;
       a[k] = nvfp4_8(raw[k], g.rs, unsafe);
-      if (unsafe) {
-        const uint2 r = chunk_codes_exact<MODE, CB>(raw[k], g.se, g.z, qr);
-        a[k] = r.x; b[k] = r.y;
-      }
+      // (frequent where the global scale is a power of two: quotients then fall on rounding boundaries exactly)
+      if (unsafe) a[k] = nvfp4_8_exact(raw[k], g.se, g.z);
     }
   } else {
 #pragma unroll

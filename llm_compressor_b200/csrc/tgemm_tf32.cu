@@ -139,6 +139,11 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
         "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr) : "memory");
 }
+// x += v in L2: an update neither waits for C nor holds registers for it.  With loads and stores the epilogue (two waits
+// on C per 32 columns) was slower than the MMAs of its tile, and the tensor pipe stood at 53 %.
+__device__ __forceinline__ void red_add_v4(float* p, float a, float b, float c, float d) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
 // shared-memory matrix descriptor, 128-byte swizzle, descriptor version 1
 __device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
   uint64_t d = 0;
@@ -398,6 +403,16 @@ tgemm_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ C
           __syncwarp();
           if (fast) {
             float* c = C + (int64_t)(row0 + sub_row) * j.ldc + cc;
+            if (beta == 1.0f) {
+#pragma unroll
+              for (int s = 0; s < 8; ++s) {
+                const int lr = s * 4 + sub_row;
+                if (row0 + lr < j.M) {
+                  const float* sp = stage + lr * 33 + sub_col;
+                  red_add_v4(c + (int64_t)(s * 4) * j.ldc, sp[0], sp[1], sp[2], sp[3]);
+                }
+              }
+            } else {
 #pragma unroll
             for (int s0 = 0; s0 < 8; s0 += 4) {
               float4 h[4];
@@ -418,6 +433,7 @@ tgemm_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ C
                   *reinterpret_cast<float4*>(c + (int64_t)((s0 + s) * 4) * j.ldc) = o;
                 }
               }
+            }
             }
           } else {
             for (int s = 0; s < 8; ++s) {
