@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import collections
 import contextlib
+import functools
 import math
 import re
 import time
@@ -36,12 +37,15 @@ _UNSET = object()
 
 # ------------------------------------------------------------------------------------------
 # module matching (compressed-tensors utils/match.py:34-70,344-456)
+@functools.lru_cache(maxsize=1024)
+def _class_names(cls: type) -> frozenset:
+    return frozenset(c.__name__ for c in cls.__mro__)
+
+
 def _match_one(name: str, module: torch.nn.Module, target: str) -> bool:
     if target.startswith("re:"):
         return re.match(target[3:], name) is not None
-    if name == target:
-        return True
-    return any(cls.__name__ == target for cls in type(module).__mro__)
+    return name == target or target in _class_names(type(module))
 
 
 def match_named_modules(model: torch.nn.Module, targets: Iterable[str], ignore: Iterable[str] = ()):
@@ -51,11 +55,16 @@ def match_named_modules(model: torch.nn.Module, targets: Iterable[str], ignore: 
     targets, ignore = list(targets or []), list(ignore or [])
     out = []
     for name, module in model.named_modules():
-        if not any(_match_one(name, module, t) for t in targets):
+        for t in targets:
+            if _match_one(name, module, t):
+                break
+        else:
             continue
-        if any(_match_one(name, module, t) for t in ignore):
-            continue
-        out.append((name, module))
+        for t in ignore:
+            if _match_one(name, module, t):
+                break
+        else:
+            out.append((name, module))
     return out
 
 
@@ -189,14 +198,15 @@ class QuantizationMixin(HooksMixin):
         bad, zero_points = [], {}
         for scheme in groups.values():
             for name, module in match_named_modules(model, scheme.targets, self.ignore):
-                if not hasattr(module, "weight") or module.weight is None or module.weight.ndim != 2:
+                weight = getattr(module, "weight", None)
+                if weight is None or weight.ndim != 2:
                     continue
                 if isinstance(module, torch.nn.Embedding):
                     continue
                 w = scheme.weights
                 if w is None:
                     continue
-                N, K = module.weight.shape
+                N, K = weight.shape
                 if (w.strategy in ("group", "tensor_group") and K >= w.group_size and K % w.group_size
                         and not self.bypass_divisibility_checks):
                     bad.append((name, K, w.group_size))
@@ -204,7 +214,6 @@ class QuantizationMixin(HooksMixin):
                 _set_plain(module, "quantization_scheme", scheme)
                 _set_plain(module, "quantization_status", "initialized")   # "frozen" once its qparams are written
                 self._module_names[module] = name
-                weight = module.weight
                 dev, dt = weight.device, weight.dtype
                 shape = w.qparam_shape(N, K)
 
@@ -318,10 +327,9 @@ class QuantizationMixin(HooksMixin):
 
     def end_calibration(self, model: torch.nn.Module) -> None:
         self.remove_hooks()
-        for module in [m for _, m in self.quantized_modules(model)] + list(self._attention_names):
+        for module in list(self._module_names) + list(self._attention_names):
             for name in ("weight_observer", "input_observer", "k_observer", "v_observer"):
-                if name in module.__dict__:
-                    delattr(module, name)
+                module.__dict__.pop(name, None)
 
 
 KV_CACHE_TARGETS = ("re:.*self_attn$",)   # the reference's match for attention modules (mixin.py:216-218)
@@ -438,7 +446,7 @@ class QuantizationModifier(QuantizationMixin):
         modules = list(modules)
         if self.calibrates_activations:
             self.update_activation_qparams(modules)
-        modules = [m for m in modules if hasattr(m, "weight_observer")
+        modules = [m for m in modules if "weight_observer" in m.__dict__
                    and getattr(m, "quantization_status", None) != "frozen"]
         if bdist.is_distributed():
             # owners by weight size; each rank observes its share, scales are broadcast
@@ -455,14 +463,16 @@ class QuantizationModifier(QuantizationMixin):
             # most weights: statistics and parameters in one launch
             rest = []
             for m in modules:
-                weight = m.weight.data
-                qp = direct_qparams([m.weight_observer], [weight]) if weight.is_cuda else None
-                if qp is None:
-                    rest.append(m)
+                params = m._parameters
+                scale, zp = params.get("weight_scale"), params.get("weight_zero_point")
+                into = None if scale is None or zp is None else (scale.data, zp.data)
+                if into is not None and direct_qparams([m.weight_observer], [m.weight.data], into) is not None:
+                    _set_plain(m, "quantization_status", "frozen")
                 else:
-                    _write_qparams(m, "weight", qp[0][0], qp[1][0], None)
-            observe(rest)
-            update_qparams(rest)
+                    rest.append(m)
+            if rest:
+                observe(rest)
+                update_qparams(rest)
 
     def pending_modules(self):
         """Targeted modules whose parameters have not been written yet (modules behind the

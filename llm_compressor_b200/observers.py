@@ -160,17 +160,20 @@ class Observer:
         return {"scale": scale, "zero_point": zero_point, "global_scale": global_scale}
 
 
-def direct_qparams(observers, weights):
+def direct_qparams(observers, weights, into=None):
     """What observing ``weights[i]`` with ``observers[i]`` and asking for the parameters gives, in one launch and without
     statistics in between: (scales, zero points) with a leading dimension, or None where the two steps are needed (other
-    observers, shared global scales, statistics that are already there, weights the kernel does not take)."""
+    observers, shared global scales, statistics that are already there, weights the kernel does not take).  ``into`` (for one weight):
+    the scale and zero point to fill in."""
     first = observers[0]
     for o in observers:
         if type(o) is not MemorylessMinMaxObserver or o.has_statistics or o._fused or o.args.strategy == "tensor_group" \
                 or (o.args is not first.args and o.args != first.args):
             return None
     if len(weights) == 1:
-        qp = ops.minmax_qparams(weights[0], first.args)
+        qp = ops.minmax_qparams(weights[0], first.args, into)
+        if into is not None:
+            return qp
         return None if qp is None else (qp[0].unsqueeze(0), qp[1].unsqueeze(0))
     return ops.minmax_qparams(list(weights), first.args)
 

@@ -310,7 +310,8 @@ def oneshot(model, recipe=None, dataset=None, num_calibration_samples: int = 512
     if pipeline not in ("independent", "sequential", "datafree", "basic"):
         raise ValueError(f"unknown pipeline {pipeline}")
     device = next(model.parameters()).device
-    model.eval()
+    if any(m.training for m in model.modules()):
+        model.eval()
     for m in modifiers:
         m.on_initialize(model)
     # "independent": each modifier runs alone with the driver it needs (pipelines/independent)

@@ -75,9 +75,10 @@ def observe_minmax_absmax(w: torch.Tensor, args: QuantizationArgs):
     return mn, mx, absmax
 
 
-def minmax_qparams(w, args: QuantizationArgs):
+def minmax_qparams(w, args: QuantizationArgs, into=None):
     """``qparams(*observe_minmax(w, args), args)`` in one launch: (scale, zero_point), or None for what it does not take.
-    ``w`` may be a list of weights of one shape and layout: the results then carry a leading dimension."""
+    ``w`` may be a list of weights of one shape and layout: the results then carry a leading dimension.  ``into``: tensors
+    to write the results to (None comes back if their types or shapes are others)."""
     many = not isinstance(w, torch.Tensor)
     first = w[0] if many else w
     if first.dtype != torch.bfloat16 or args.strategy == "tensor_group":
@@ -92,8 +93,15 @@ def minmax_qparams(w, args: QuantizationArgs):
     shape = args.qparam_shape(N, K)
     if many:
         shape = (count,) + tuple(shape)
-    scale = torch.empty(shape, dtype=first.dtype, device=first.device)
-    zp = torch.empty(shape, dtype=_zp_storage(args), device=first.device)
+    if into is not None:
+        scale, zp = into
+        if (scale.dtype != first.dtype or zp.dtype != _zp_storage(args) or scale.shape != shape or zp.shape != shape
+                or not scale.is_contiguous() or not zp.is_contiguous() or scale.device != first.device
+                or zp.device != first.device):
+            return None
+    else:
+        scale = torch.empty(shape, dtype=first.dtype, device=first.device)
+        zp = torch.empty(shape, dtype=_zp_storage(args), device=first.device)
     table = _pointer_table([w]) if many else None
     rc = _lib.load().b200q_minmax_qparams(None if many else ptr(w), ptr(table), count, _dt(first), N, K, ld, args.c_struct(),
                                           ptr(scale), ptr(zp), stream_ptr())

@@ -7,7 +7,7 @@ compressed-tensors class is accepted wherever one of these is (``QuantizationArg
 """
 from __future__ import annotations
 
-from dataclasses import dataclass, field, replace
+from dataclasses import dataclass, field
 from typing import Any, Optional
 
 import torch
@@ -93,7 +93,12 @@ class QuantizationArgs:
         return cls(**{n: getattr(obj, n) for n in names if hasattr(obj, n)})
 
     def model_copy(self, update=None) -> "QuantizationArgs":
-        return replace(self, **(update or {}))
+        # (what dataclasses.replace does, without its walk over the fields)
+        out = object.__new__(type(self))
+        out.__dict__.update(self.__dict__)
+        out.__dict__.update(update or {})
+        out.__post_init__()
+        return out
 
     def pytorch_dtype(self) -> torch.dtype:
         if self.type == "float":
