@@ -154,6 +154,12 @@ int b200q_observe_mse_noalloc(const void* W, int wdtype, int64_t N, int64_t K, i
 int b200q_minmax_qparams(const void* W, const void* const* table, int count, int wdtype, int64_t N, int64_t K, int64_t ldw,
                          const b200q_qargs* qa, void* scale_out, void* zp_out, void* stream);
 
+/* The same for up to 8 contiguous bf16 weights [N[i]][K] that share one global scale (host arrays of device pointers,
+ * 16-byte aligned): symmetric TENSOR_GROUP schemes of group size 16 or 32; otherwise B200Q_ERR_UNSUPPORTED.  Writes
+ * scale[i] (bf16 [N[i]][K / g]), zp[i] (one byte each, zero) and *global_scale[i]; absmax: float, scratch. */
+int b200q_shared_qparams(const void* const* W, void* const* scale, void* const* zp, float* const* global_scale,
+                         const int64_t* N, int count, int64_t K, const b200q_qargs* qa, float* absmax, void* stream);
+
 /* Quantize-dequantize.  Replaces fake_quantize (CT/quantization/lifecycle/forward.py:149-181,
  * forward_helpers.py:113-210).  scale: [qparam shape] of dtype sdtype; zp may be NULL;
  * g_idx (int32 [K], group of each column) may be NULL; global_scale may be NULL.

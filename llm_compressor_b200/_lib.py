@@ -51,6 +51,7 @@ SIGNATURES = {
     "b200q_observe_minmax": (_i, [_p, _i, _i64, _i64, _i64, _qa, _p, _p, _p, _p]),
     "b200q_observe_minmax_absmax": (_i, [_p, _i, _i64, _i64, _i64, _qa, _p, _p, _p, _p, _p]),
     "b200q_minmax_qparams": (_i, [_p, _p, _i, _i, _i64, _i64, _i64, _qa, _p, _p, _p]),
+    "b200q_shared_qparams": (_i, [_p, _p, _p, _p, _p, _i, _i64, _qa, _p, _p]),
     "b200q_hessian_finalize_many": (_i, [_p, _p, _i, _i64, _i64, _p]),
     "b200q_upload": (_i, [_p, _i64, _p, _p]),
     "b200q_gptq_prologue_many": (_i, [_p, _i, _i64, _i64, _f, _p, _p, _p, _p, _p]),

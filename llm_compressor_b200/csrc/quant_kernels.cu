@@ -472,9 +472,7 @@ __global__ void __launch_bounds__(256) absmax_weight_bf16_kernel(const void* __r
   }
 }
 
-__global__ void global_scale_kernel(const float* __restrict__ absmax, int stat_bf16,
-                                    float* __restrict__ out) {
-  float a = *absmax;
+__device__ __forceinline__ float global_scale_of(float a, bool stat_bf16) {
   float tiny = 1.17549435e-38f;  // smallest normal of both bf16 and float32
   a = fmaxf(a, tiny);
   // "scalar / tensor" in torch is tensor.reciprocal() * scalar: two roundings in the statistics' dtype
@@ -483,7 +481,11 @@ __global__ void global_scale_kernel(const float* __restrict__ absmax, int stat_b
   float g = __fmul_rn(r, 448.0f * 6.0f);
   if (stat_bf16) g = bf16r(g);
   if (!(fabsf(g) <= 3.402823466e38f)) g = 1.0f;  // NaN / Inf -> 1
-  *out = g;
+  return g;
+}
+__global__ void global_scale_kernel(const float* __restrict__ absmax, int stat_bf16,
+                                    float* __restrict__ out) {
+  *out = global_scale_of(*absmax, stat_bf16 != 0);
 }
 
 // ========================================================================================
@@ -611,6 +613,78 @@ __global__ void __launch_bounds__(256) span_qparams_kernel(StatJob j, int64_t N,
     if (threadIdx.x == 0) {
       for (int w = 1; w < 8; ++w) { lo = fminf(lo, s_lo[par][w]); hi = fmaxf(hi, s_hi[par][w]); }
       j.put(b, lo, hi, qc);
+    }
+  }
+}
+
+// The same for symmetric schemes with a global scale that up to eight contiguous weights share: a symmetric scale needs only
+// the largest magnitude of its group, so that is what pass one leaves in the place of the scale (while it finds the
+// largest of all), and pass two turns it into the scale.  W is read once; the statistics of the separate kernels
+// (min, max, float32 scale, copy) moved another 66 bytes a group.  blockIdx.y = weight.
+constexpr int kMaxShared = 8;
+struct SharedJob {
+  const __nv_bfloat16* w[kMaxShared];
+  __nv_bfloat16* scale[kMaxShared];
+  void* zp[kMaxShared];
+  float* global_scale[kMaxShared];
+  int64_t groups[kMaxShared];
+  float* absmax;
+};
+template <int R>
+__global__ void __launch_bounds__(256) shared_absmax_kernel(const __grid_constant__ SharedJob j) {
+  const int64_t n = j.groups[blockIdx.y], step = (int64_t)gridDim.x * 256;
+  const uint4* w = reinterpret_cast<const uint4*>(j.w[blockIdx.y]);
+  __nv_bfloat16* out = j.scale[blockIdx.y];
+  constexpr int U = 8 / R;      // groups of a thread whose loads are in flight together
+  float top = 0.0f;
+  for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += U * step) {
+    uint4 raw[U][R];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        raw[u][r] = i + u * step < n ? stream::ldg_stream(w + (i + u * step) * R + r) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      __nv_bfloat162 m = __float2bfloat162_rn(0.0f);
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const __nv_bfloat162* e = reinterpret_cast<const __nv_bfloat162*>(&raw[u][r]);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) m = __hmax2(m, __habs2(e[q]));
+      }
+      const __nv_bfloat16 a = __hmax(m.x, m.y);
+      if (i + u * step < n) out[i + u * step] = a;
+      top = fmaxf(top, __bfloat162float(a));
+    }
+  }
+  top = warp_max(top);
+  if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<int*>(j.absmax), __float_as_int(top));
+}
+__global__ void __launch_bounds__(256) shared_qparams_kernel(const __grid_constant__ SharedJob j, QParamCfg qc) {
+  const float g = global_scale_of(*j.absmax, true);
+  const int64_t n = j.groups[blockIdx.y];
+  __nv_bfloat16* scale = j.scale[blockIdx.y];
+  void* zp = j.zp[blockIdx.y];
+  if (blockIdx.x == 0 && threadIdx.x == 0) *j.global_scale[blockIdx.y] = g;
+  for (int64_t i = ((int64_t)blockIdx.x * 256 + threadIdx.x) * 8; i < n; i += (int64_t)gridDim.x * 2048) {
+    const int m = (int)(n - i < 8 ? n - i : 8);
+    alignas(16) __nv_bfloat16 v[8];
+    if (m == 8) *reinterpret_cast<uint4*>(v) = *reinterpret_cast<const uint4*>(scale + i);
+    else for (int e = 0; e < m; ++e) v[e] = scale[i + e];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      if (e >= m) break;
+      float s, z;
+      const float a = __bfloat162float(v[e]);
+      qparams_one<true>(-a, a, qc, g, s, z);
+      v[e] = __float2bfloat16_rn(s);
+    }
+    if (m == 8) {
+      *reinterpret_cast<uint4*>(scale + i) = *reinterpret_cast<const uint4*>(v);
+      *reinterpret_cast<uint2*>((uint8_t*)zp + i) = make_uint2(0u, 0u);   // (zero in every storage type)
+    } else {
+      for (int e = 0; e < m; ++e) { scale[i + e] = v[e]; ((uint8_t*)zp)[i + e] = 0; }
     }
   }
 }
@@ -1190,6 +1264,37 @@ int b200q_minmax_qparams(const void* W, const void* const* table, int count, int
   } else {
     return B200Q_ERR_UNSUPPORTED;
   }
+  B200Q_LAUNCH_CHECK();
+  return B200Q_OK;
+}
+
+int b200q_shared_qparams(const void* const* W, void* const* scale, void* const* zp, float* const* global_scale,
+                         const int64_t* N, int count, int64_t K, const b200q_qargs* qa, float* absmax, void* stream) {
+  if (!W || !scale || !zp || !global_scale || !N || count <= 0 || K <= 0 || !qa || !absmax) return B200Q_ERR_ARG;
+  const int g = qa->group_size;
+  if (count > kMaxShared || qa->strategy != B200Q_TENSOR_GROUP || !qa->symmetric || (g != 16 && g != 32) || K % g)
+    return B200Q_ERR_UNSUPPORTED;
+  QParamCfg qc;
+  int rc = make_qparam_cfg(qa, true, true, &qc); if (rc) return rc;
+  SharedJob j = {};
+  int64_t most = 0;
+  for (int i = 0; i < count; ++i) {
+    if (!W[i] || !scale[i] || !zp[i] || !global_scale[i] || N[i] <= 0) return B200Q_ERR_ARG;
+    if ((((uintptr_t)W[i]) | ((uintptr_t)scale[i]) | ((uintptr_t)zp[i])) & 15) return B200Q_ERR_UNSUPPORTED;
+    j.w[i] = (const __nv_bfloat16*)W[i]; j.scale[i] = (__nv_bfloat16*)scale[i]; j.zp[i] = zp[i];
+    j.global_scale[i] = global_scale[i];
+    j.groups[i] = N[i] * (K / g);
+    most = most > j.groups[i] ? most : j.groups[i];
+  }
+  j.absmax = absmax;
+  cudaStream_t st = (cudaStream_t)stream;
+  B200Q_TRY(cudaMemsetAsync(absmax, 0, sizeof(float), st));
+  const int cap = (8 * kNumSMs + count - 1) / count;
+  auto grid = [&](int64_t need) { return dim3((unsigned)(need < cap ? need : cap), (unsigned)count, 1); };
+  if (g == 16) shared_absmax_kernel<2><<<grid((most + 255) / 256), 256, 0, st>>>(j);
+  else shared_absmax_kernel<4><<<grid((most + 255) / 256), 256, 0, st>>>(j);
+  B200Q_LAUNCH_CHECK();
+  shared_qparams_kernel<<<grid((most + 2047) / 2048), 256, 0, st>>>(j, qc);
   B200Q_LAUNCH_CHECK();
   return B200Q_OK;
 }

@@ -22,9 +22,9 @@ from typing import Any, Iterable, Optional
 import torch
 
 from . import dist as bdist
-from . import gptq
+from . import gptq, ops
 from ._lib import B200QError
-from .observers import Observer, direct_qparams, fuse_weight_observers
+from .observers import MemorylessMinMaxObserver, Observer, direct_qparams, fuse_weight_observers
 from .streams import run_concurrent
 from .quant_args import (PRESET_SCHEMES, QuantizationArgs, QuantizationScheme,
                          preset_name_to_scheme)
@@ -410,6 +410,32 @@ def _write_qparams(m, base_name, scale, zero_point, global_scale) -> None:
         _set_plain(m, "quantization_status", "frozen")
 
 
+def _write_shared_qparams(modules):
+    """Parameters of the weights that share a global scale (and of single ones with a global scale), all of a group in two
+    launches; returns the modules that are left."""
+    by_observer = {id(m.weight_observer): m for m in modules if m.weight_observer.args.strategy == "tensor_group"}
+    if not by_observer:
+        return modules
+    done = set()
+    for m in modules:
+        obs = m.weight_observer
+        if id(obs) not in by_observer or id(m) in done:
+            continue
+        observers = [obs] + obs._fused
+        group = [by_observer.get(id(o)) for o in observers]
+        if any(g is None or type(o) is not MemorylessMinMaxObserver or o.has_statistics or o.args != obs.args
+               for o, g in zip(observers, group)):
+            continue
+        into = [[g._parameters.get("weight_" + name) for g in group] for name in ("scale", "zero_point", "global_scale")]
+        if any(p is None for ps in into for p in ps):
+            continue
+        if ops.shared_qparams([g.weight.data for g in group], obs.args, *[[p.data for p in ps] for ps in into]):
+            for g in group:
+                done.add(id(g))
+                _set_plain(g, "quantization_status", "frozen")
+    return [m for m in modules if id(m) not in done]
+
+
 def _set_plain(module, name, value) -> None:
     """``setattr`` for a value that is no parameter, buffer or submodule: torch's own looks for all of these first, in
     Python, at 4 us an attribute."""
@@ -462,6 +488,7 @@ class QuantizationModifier(QuantizationMixin):
         else:
             # most weights: statistics and parameters in one launch
             rest = []
+            modules = _write_shared_qparams(modules)
             for m in modules:
                 params = m._parameters
                 scale, zp = params.get("weight_scale"), params.get("weight_zero_point")

@@ -111,6 +111,29 @@ def minmax_qparams(w, args: QuantizationArgs, into=None):
     return scale, zp
 
 
+def shared_qparams(weights, args: QuantizationArgs, scales, zps, global_scales) -> bool:
+    """Fills in the parameters of weights that share one global scale; False for what the kernel does not take."""
+    K, dev = weights[0].shape[1], weights[0].device
+    for w, s, z, g in zip(weights, scales, zps, global_scales):
+        shape = args.qparam_shape(w.shape[0], K)
+        if (w.dtype != torch.bfloat16 or w.shape[1] != K or s.dtype != torch.bfloat16 or z.dtype != _zp_storage(args)
+                or g.dtype != torch.float32 or s.shape != shape or z.shape != shape or g.numel() != 1
+                or not (w.is_contiguous() and s.is_contiguous() and z.is_contiguous())
+                or not (w.device == s.device == z.device == g.device == dev)):
+            return False
+    _need_cuda(weights[0])
+    n = len(weights)
+    ptrs = ctypes.c_void_p * n
+    absmax = torch.empty(1, dtype=torch.float32, device=dev)
+    rc = _lib.load().b200q_shared_qparams(
+        ptrs(*map(ptr, weights)), ptrs(*map(ptr, scales)), ptrs(*map(ptr, zps)), ptrs(*map(ptr, global_scales)),
+        (ctypes.c_int64 * n)(*(w.shape[0] for w in weights)), n, K, args.c_struct(), ptr(absmax), stream_ptr())
+    if rc == -2:
+        return False
+    check(rc, "b200q_shared_qparams")
+    return True
+
+
 def observe_mse(w, args, maxshrink=0.20, patience=5, grid=100.0, norm=2.4, expand=1.0):
     _need_cuda(w)
     lib = _lib.load()
