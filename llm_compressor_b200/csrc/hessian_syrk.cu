@@ -176,7 +176,6 @@ struct Params {
                              // the other, and adds them into H without atomics (bitwise reproducible)
   float alpha;
   int* status;
-  int red;
 };
 
 __global__ void __launch_bounds__(kThreads, 1)
@@ -600,34 +599,13 @@ syrk_pair_kernel(const __grid_constant__ CUtensorMap xmap, Params p) {
       const int row0 = row_blk + q * 32;
       const int col_base = bj * kPairTile;
       const int row_blk_end = row_blk + 128;  // columns >= this belong to the upper part
-      const bool add = (p.splits > 1 && !p.tile_major) || p.red;   // other pairs add to this tile: atomics
       // 32-column chunks of this warp's rows that hold something (warp-uniform)
       const int col_end = min(row_blk_end, p.K);
       const int nchunk = row_blk >= p.K || col_end <= col_base ? 0 : min(kPairTile / 32, (col_end - col_base + 31) / 32);
-      // H is read two chunks ahead, the first two while the MMAs still run: with one chunk at a time the latency of
-      // H stood in the way eight times a tile (22.8 us for 512 tokens at K = 4096, where the MMAs take 5)
-      constexpr int kAhead = 2;
-      float4 h[kAhead + 1][8];
-      auto fetch = [&](int c, float4 (&to)[8]) {
-        const int cc = col_base + c * 32 + sub_col;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int row = row0 + i * 4 + sub_row;
-          to[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (row < p.K && cc < p.K) to[i] = *reinterpret_cast<const float4*>(p.H + (int64_t)row * p.ldh + cc);
-        }
-      };
-      if (!add) {
-#pragma unroll
-        for (int c = 0; c < kAhead; ++c)
-          if (c < nchunk) fetch(c, h[c]);
-      }
       if (!mbar_wait(accf_bar(buf), acc_phase, &s_abort, p.status, 4)) { ok = false; break; }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-      for (int c = 0; c < kPairTile / 32; ++c) {
-        if (c >= nchunk) break;   // warp-uniform
-        if (!add && c + kAhead < nchunk) fetch(c + kAhead, h[(c + kAhead) % (kAhead + 1)]);
+#pragma unroll 1
+      for (int c = 0; c < nchunk; ++c) {
         uint32_t r[32];
         tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * kPairTile + c * 32), r);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -636,7 +614,9 @@ syrk_pair_kernel(const __grid_constant__ CUtensorMap xmap, Params p) {
         __syncwarp();
         const int cc = col_base + c * 32 + sub_col;
         if (cc < p.K) {
-          if (add) {
+          if (!p.tile_major) {
+            // reductions in L2, also where this pair alone adds to the tile: nothing waits for H (a load and a store
+            // per element: 22.8 us for 512 tokens at K = 4096 against 18.9)
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               const int lr = i * 4 + sub_row, row = row0 + lr;
@@ -646,14 +626,20 @@ syrk_pair_kernel(const __grid_constant__ CUtensorMap xmap, Params p) {
               }
             }
           } else {
-            float4 (&o)[8] = h[c % (kAhead + 1)];
+            float4 h[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const int row = row0 + i * 4 + sub_row;
+              h[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+              if (row < p.K) h[i] = *reinterpret_cast<const float4*>(p.H + (int64_t)row * p.ldh + cc);
+            }
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
               const int lr = i * 4 + sub_row, row = row0 + lr;
               if (row < p.K) {
                 const float* sp = stage + lr * 33 + sub_col;
-                o[i].x += sp[0]; o[i].y += sp[1]; o[i].z += sp[2]; o[i].w += sp[3];
-                *reinterpret_cast<float4*>(p.H + (int64_t)row * p.ldh + cc) = o[i];
+                h[i].x += sp[0]; h[i].y += sp[1]; h[i].z += sp[2]; h[i].w += sp[3];
+                *reinterpret_cast<float4*>(p.H + (int64_t)row * p.ldh + cc) = h[i];
               }
             }
           }
@@ -859,7 +845,6 @@ int b200q_hessian_syrk(const void* X, int64_t T, int64_t K, int64_t ldx, float* 
   Params p;
   p.H = H; p.ldh = ldh; p.K = (int)K; p.T = T; p.alpha = alpha; p.status = status;
   p.tile_major = 0;
-  { static const int red = [] { const char* e = getenv("SYRK_RED"); return e ? atoi(e) : 0; }(); p.red = red; }
   cudaStream_t st = (cudaStream_t)stream;
   const int pairs = pair_capacity();
   if (pairs > 0) {
