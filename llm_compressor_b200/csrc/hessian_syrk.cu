@@ -680,15 +680,20 @@ __global__ void __launch_bounds__(256) finalize_kernel(float* H0, float* const* 
   __shared__ float tile[kFinTile][kFinTile + 1];
   float* H = Hs ? Hs[blockIdx.y] : H0;
   if (scales) scale = scales[blockIdx.y];
-  const int nb = (int)((K + kFinTile - 1) / kFinTile);
-  const int64_t nblk = (int64_t)nb * (nb + 1) / 2;
+  // patches of 8 x 8 blocks: what the CTAs write at the same time makes whole 2 KB pieces of rows on both sides of the
+  // diagonal (row by row of blocks, the mirrored side got 256-byte pieces 57 KB apart: 316 us at K = 14336)
+  const int nb = (int)((K + kFinTile - 1) / kFinTile), np = (nb + 7) / 8;
+  const int64_t nblk = (int64_t)np * (np + 1) / 2 * 64;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;   // 16 quads of columns x 16 rows
   for (int64_t blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
     // blk -> (bi >= bj)
-    int bi = (int)((sqrtf(8.0f * (float)blk + 1.0f) - 1.0f) * 0.5f);
-    while ((int64_t)bi * (bi + 1) / 2 > blk) --bi;
-    while ((int64_t)(bi + 1) * (bi + 2) / 2 <= blk) ++bi;
-    const int bj = (int)(blk - (int64_t)bi * (bi + 1) / 2);
+    const int patch = (int)(blk >> 6), in = (int)blk & 63;
+    int bi = (int)((sqrtf(8.0f * (float)patch + 1.0f) - 1.0f) * 0.5f);
+    while (bi * (bi + 1) / 2 > patch) --bi;
+    while ((bi + 1) * (bi + 2) / 2 <= patch) ++bi;
+    const int bj = (patch - bi * (bi + 1) / 2) * 8 + (in & 7);
+    bi = bi * 8 + (in >> 3);
+    if (bi < bj || bi >= nb) continue;   // CTA-uniform
     float4 v[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -853,13 +858,20 @@ int b200q_hessian_syrk(const void* X, int64_t T, int64_t K, int64_t ldx, float* 
     p.tiles = nb2 * (nb2 + 1) / 2;
     p.nb = nb2;
     const int64_t max_splits = (T + 511) / 512;
+    // Token splits: SM cycles of the busiest pair.  A unit takes the longer of its MMAs (8 cycles a token) and its
+    // addition to H, which the whole GPU does at about 3 TB/s while H stays in L2 and 2.2 TB/s beyond it (12 and 17
+    // thousand cycles a tile with all pairs at it); what ends last, the other of the two, is not hidden.  Filling the
+    // waves alone, as the rule was, split 4096 tokens of K = 4096 seven ways: 84 us where one split takes 60.
+    const double add = (double)K * (double)K * 2.0 > 60e6 ? 17000.0 : 12000.0;
     int best = 1;
-    double best_eff = 0.0;
+    double best_cost = 0.0;
     for (int s = 1; s <= (int)(max_splits < 64 ? max_splits : 64); ++s) {
-      const int64_t units = (int64_t)p.tiles * s;
-      const int64_t waves = (units + pairs - 1) / pairs;
-      const double eff = (double)units / (double)(waves * pairs);
-      if (eff > best_eff + 0.02) { best_eff = eff; best = s; }
+      const int64_t waves = ((int64_t)p.tiles * s + pairs - 1) / pairs;
+      const double mma = 8.0 * (double)((T + s - 1) / s);
+      const double together = (double)p.tiles * s < pairs ? (double)p.tiles * s / pairs : 1.0;
+      const double tile_add = add * together < 3000.0 ? 3000.0 : add * together;
+      const double cost = (double)waves * (mma > tile_add ? mma : tile_add) + (mma > tile_add ? tile_add : mma);
+      if (s == 1 || cost < 0.98 * best_cost) { best_cost = cost; best = s; }
     }
     {
       // bound the length of one tensor-core accumulation chain: its float32 error grows with it
@@ -926,7 +938,7 @@ int b200q_get_reproducible(void) { return g_reproducible.load(std::memory_order_
 static int finalize(float* H, float* const* Hs, const float* scales, int count, int64_t K, int64_t ldh, float scale,
                     void* stream) {
   using namespace b200q::syrk;
-  const int64_t nb = (K + kFinTile - 1) / kFinTile, nblk = nb * (nb + 1) / 2, cap = 8 * kNumSMs / count + 1;
+  const int64_t np = (K + 8 * kFinTile - 1) / (8 * kFinTile), nblk = np * (np + 1) / 2 * 64, cap = 8 * kNumSMs / count + 1;
   const bool vec = (ldh & 3) == 0 && (Hs || (((uintptr_t)H) & 15) == 0);   // (a batch's matrices are whole allocations)
   finalize_kernel<<<dim3((unsigned)(nblk < cap ? nblk : cap), (unsigned)count), 256, 0, (cudaStream_t)stream>>>(
       H, Hs, scales, K, ldh, scale, vec);
