@@ -862,15 +862,14 @@ int b200q_hessian_syrk(const void* X, int64_t T, int64_t K, int64_t ldx, float* 
     // addition to H, which the whole GPU does at about 3 TB/s while H stays in L2 and 2.2 TB/s beyond it (12 and 17
     // thousand cycles a tile with all pairs at it); what ends last, the other of the two, is not hidden.  Filling the
     // waves alone, as the rule was, split 4096 tokens of K = 4096 seven ways: 84 us where one split takes 60.
+    // (A single round of tiles leaves its additions behind in about 4 thousand.)
     const double add = (double)K * (double)K * 2.0 > 60e6 ? 17000.0 : 12000.0;
     int best = 1;
     double best_cost = 0.0;
     for (int s = 1; s <= (int)(max_splits < 64 ? max_splits : 64); ++s) {
-      const int64_t waves = ((int64_t)p.tiles * s + pairs - 1) / pairs;
-      const double mma = 8.0 * (double)((T + s - 1) / s);
-      const double together = (double)p.tiles * s < pairs ? (double)p.tiles * s / pairs : 1.0;
-      const double tile_add = add * together < 3000.0 ? 3000.0 : add * together;
-      const double cost = (double)waves * (mma > tile_add ? mma : tile_add) + (mma > tile_add ? tile_add : mma);
+      const int64_t rounds = ((int64_t)p.tiles * s + pairs - 1) / pairs;
+      const double mma = 8.0 * (double)((T + s - 1) / s), tile_add = rounds == 1 ? 4000.0 : add;
+      const double cost = (double)rounds * (mma > tile_add ? mma : tile_add) + (mma > tile_add ? tile_add : mma);
       if (s == 1 || cost < 0.98 * best_cost) { best_cost = cost; best = s; }
     }
     {
