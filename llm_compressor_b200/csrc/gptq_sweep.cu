@@ -22,8 +22,8 @@ constexpr int kMaxBlock = 128;               // largest block size callers may a
 constexpr size_t kSweepHeaderBytes = 256;    // status word at the start of the workspace
 constexpr int kRows = 32;                    // rows of a CTA: a lane each
 constexpr int kMicro = 16;                   // columns a lane keeps in registers at a time
-// 12 warps where a CTA has its SM to itself, 4 where three share one
-constexpr int warps_of(int width) { return width == 512 ? 12 : 4; }
+// 12 warps where a CTA has its SM to itself, 8 where two share one
+constexpr int warps_of(int superblock) { return superblock == 512 ? 12 : 8; }
 constexpr int WLD = kRows + 4, ELD = kRows + 8;   // columns of W and of the errors in shared memory: the strides
                                                   // make the MMA fragments' accesses conflict-free
 __host__ __device__ constexpr int u_stride(int superblock) { return superblock + 8; }   // likewise
@@ -190,18 +190,17 @@ __device__ __forceinline__ void apply_errors(const ErrFrag& f, const float* u, f
 // from a counter.  The columns next in line take the first twelve errors from a warp that waits for them while the chain
 // is on the last four, and those four from the chain warp.  Duties beside that: the warps that share the chain warp's
 // scheduler ask for rows of U by bulk copies (as per-thread copies they block the warps that issue them: all CTAs want
-// the same rows at the same time), and take tasks only while these, not the chain, decide; one warp fetches parameters,
-// one writes the errors out as the operand of the trailing product.  One barrier per micro-block.  Every role is a
+// the same rows at the same time), and take tasks only while these, not the chain, decide; warp 5 fetches parameters,
+// warp 6 writes the errors out as the operand of the trailing product.  One barrier per micro-block.  Every role is a
 // latency-bound stream of instructions, a quarter of its stalls instruction fetch, hence short loops rather than
 // unrolled code off the chain.
 template <int SBLK, bool SB, int KIND, bool ZP>
-__global__ void __launch_bounds__(32 * warps_of(SBLK), SBLK == 512 ? 1 : 3) sweep_block_kernel(const __grid_constant__ Params p) {
+__global__ void __launch_bounds__(32 * warps_of(SBLK), SBLK == 512 ? 1 : 2) sweep_block_kernel(const __grid_constant__ Params p) {
   const float qmin = p.qr.qmin, qmax = p.qr.qmax;
   extern __shared__ __align__(16) float sm[];
   constexpr int ULD = u_stride(SBLK);
   constexpr int NW = warps_of(SBLK), NT = 32 * NW;
   constexpr int kNextWarp = NW > 8 ? 9 : 1;            // brings the next micro-block's columns up to date
-  constexpr int kParamWarp = NW > 8 ? 5 : 2, kErrorWarp = NW > 8 ? 6 : 3;
   constexpr int kHead = 12;                            // its share of a micro-block's errors
   float* sU = sm;                                      // [3][kMicro][ULD]
   float* sP = sU + 3 * kMicro * ULD;                   // [2][scale, low and high 1 / scale, zero point][kMicro][kRows]
@@ -213,11 +212,7 @@ __global__ void __launch_bounds__(32 * warps_of(SBLK), SBLK == 512 ? 1 : 3) swee
   __shared__ int s_odd;                                // some scale is outside the range the low / high test covers
   __shared__ int s_next[2];                            // next task of the helpers
   __shared__ __align__(8) uint64_t s_bar[3];           // rows of U of a micro-block have arrived
-  // (the roles of a CTA of four warps are turned by one from one round of CTAs to the next: the chain warps of an SM
-  // should not all sit on one scheduler)
-  const int turn = NW == 4 ? (int)((blockIdx.y * gridDim.x + blockIdx.x) / kNumSMs) * 32 : 0;
-  const int job = blockIdx.y, tid = NW == 4 ? (int)((threadIdx.x + turn) & (NT - 1)) : (int)threadIdx.x;
-  const int warp = tid >> 5, lane = tid & 31;
+  const int job = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int sb = p.sb, micros = (sb + kMicro - 1) / kMicro;
   float* __restrict__ W = p.W.at(job) + p.i1;
   const float* __restrict__ U = p.U.at(job);
@@ -253,7 +248,7 @@ __global__ void __launch_bounds__(32 * warps_of(SBLK), SBLK == 512 ? 1 : 3) swee
       }
     }
   };
-  // of twelve warps, two ask for half of a micro-block's rows each, of four one for all
+  // a warp of twelve asks for half of a micro-block's rows, of eight for all
   constexpr std::integral_constant<int, NW == 12 ? kMicro / 2 : kMicro> kAskRows;
   auto wait_u = [&](int m) {
     if (!bulk) return;
@@ -372,11 +367,11 @@ __global__ void __launch_bounds__(32 * warps_of(SBLK), SBLK == 512 ? 1 : 3) swee
     sSame[tid] = same ? 1 : 0;
   }
   __syncthreads();
-  if (warp == kParamWarp) fetch_params(0);
+  if (warp == 5) fetch_params(0);
   wait_u(0);
   __syncthreads();
 
-  float loss = 0.0f;   // of the error warp's rows, a lane each
+  float loss = 0.0f;   // of warp 6's rows, a lane each
   // the errors of micro-block `of`: their squares into the loss, and out as operand rows
   auto finish_errors = [&](int of) {
     const float* ei = sE + (of & 1) * kMicro * ELD + lane;
@@ -500,11 +495,10 @@ __global__ void __launch_bounds__(32 * warps_of(SBLK), SBLK == 512 ? 1 : 3) swee
       }
     } else if (m + 1 < micros) {
       const bool beside = (warp & 3) == 0;   // the chain warp's scheduler
-      if ((NW == 12 ? beside : warp == kParamWarp) && m > 0)   // into the buffer of micro-block m - 2
-        fetch_u(m + 1, NW == 12 ? (warp - 4) * (kAskRows / 4) : 0, kAskRows);
+      if (beside && m > 0) fetch_u(m + 1, (warp - 4) * (kAskRows / 4), kAskRows);   // into the buffer of micro-block m - 2
       if (tid == 32) s_next[(m + 1) & 1] = 0;   // (nobody takes from it before the barrier)
-      if (warp == kParamWarp) fetch_params(m + 1);
-      if (warp == kErrorWarp && m > 0) finish_errors(m - 1);
+      if (warp == 5) fetch_params(m + 1);
+      if (warp == 6 && m > 0) finish_errors(m - 1);
       ErrFrag f;
       if (m > 0 && (!beside || micros - m > 16)) {
         load_errors(sE + ((m - 1) & 1) * kMicro * ELD, lane, false, f);
@@ -526,13 +520,13 @@ __global__ void __launch_bounds__(32 * warps_of(SBLK), SBLK == 512 ? 1 : 3) swee
         load_errors(sE + (m & 1) * kMicro * ELD, lane, true, f);
         apply_errors<ULD>(f, u + kMicro, sW + (c0 + kMicro) * WLD, lane);
       }
-    } else if (warp == kErrorWarp && m > 0) {
+    } else if (warp == 6 && m > 0) {
       finish_errors(m - 1);
     }
     if (m + 1 < micros) wait_u(m + 1);
     __syncthreads();
   }
-  if (warp == kErrorWarp) finish_errors(micros - 1);   // (a superblock with columns after it is a whole one)
+  if (warp == 6) finish_errors(micros - 1);   // (a superblock with columns after it is a whole one)
   // tile out
   if (vecw) {
 #pragma unroll 2
@@ -551,38 +545,34 @@ __global__ void __launch_bounds__(32 * warps_of(SBLK), SBLK == 512 ? 1 : 3) swee
       for (int c = lane; c < sb; c += 32) dst[c] = sW[c * WLD + r];
     }
   }
-  if (warp == kErrorWarp && live) {
+  if (warp == 6 && live) {
     float* lo = p.losses.at(job);
     const float half = loss * 0.5f;
     lo[row] = p.i1 == 0 ? half : lo[row] + half;
   }
 }
 
-// Columns of a launch.  With at most one CTA per SM the chain decides and 512 columns halve the launches and the traffic of
-// the products between them.  With more rows than that what counts is how many chains an SM carries at once and how much
-// of the updates the CTAs do themselves (width / 2 multiply-adds per element, by warp-level MMAs): 128 columns and four
-// warps let three CTAs share an SM, and a launch takes the errors of the launches before it in its superblock from one
-// product of depth 128, 256 or 384.  (256 columns with eight warps, two CTAs to an SM: 274 us for 256 columns of
-// 64 x 768 rows.)
-static int width_of(int64_t ctas) { return ctas <= kNumSMs ? 512 : 128; }
-constexpr int kSuper = 512;   // columns whose errors the rest of the matrix takes in one product
+// Superblock width.  With at most one CTA per SM the chain decides and 512 columns halve the launches and the traffic
+// of the trailing products; with more rows than that the CTA's own updates (width / 2 multiply-adds per element) do,
+// and 256 columns leave room for two CTAs per SM.
+static int superblock_of(int64_t ctas) { return ctas <= kNumSMs ? 512 : 256; }
 // The trailing product is split in the columns the next superblock needs and the rest on a helper stream only while
 // a superblock's CTAs leave half of the GPU idle.
 static bool look_ahead(int64_t ctas) { return ctas <= kNumSMs / 2; }
 
 struct Layout {
-  int sb, width, sets;
+  int sb, sets;
   int64_t rows_n, rows_k, err, ub;   // rows per problem of the operands; floats of one hi or lo array
   size_t bytes;
 };
 static Layout layout_of(int64_t N, int64_t K, int batch, int distinct_u, bool may_overlap) {
   const int64_t ctas = (N + kRows - 1) / kRows * batch;
   Layout l;
-  l.sb = kSuper; l.width = width_of(ctas);
+  l.sb = superblock_of(ctas);
   l.sets = may_overlap && look_ahead(ctas) ? 2 : 1;
   l.rows_n = (N + 127) / 128 * 128; l.rows_k = (K + 127) / 128 * 128;
   l.err = l.rows_n * l.sb * batch; l.ub = l.rows_k * l.sb * distinct_u;
-  l.bytes = kSweepHeaderBytes + (K > l.width ? (size_t)(2 * l.sets * (l.err + l.ub)) * sizeof(float) : 0) + 64;
+  l.bytes = kSweepHeaderBytes + (K > l.sb ? (size_t)(2 * l.sets * (l.err + l.ub)) * sizeof(float) : 0) + 64;
   return l;
 }
 
@@ -610,22 +600,21 @@ static int sweep(Params p, int sdtype, bool global, int batch, const float* cons
     else if (p.qr.kind == kFp8) B200Q_SWEEP_SB(S, kFp8); \
     else B200Q_SWEEP_SB(S, kFp4);                        \
   } while (0)
-  if (l.width == 512) B200Q_SWEEP_PICK(512); else B200Q_SWEEP_PICK(128);
+  if (l.sb == 512) B200Q_SWEEP_PICK(512); else B200Q_SWEEP_PICK(256);
 #undef B200Q_SWEEP_PICK
 #undef B200Q_SWEEP_SB
 #undef B200Q_SWEEP_ZP
-  B200Q_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(l.width)));
+  B200Q_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(l.sb)));
   const int ctas = (int)((N + kRows - 1) / kRows);
   tgemm::SideStream* side = l.sets == 2 && has_u && K > 2 * l.sb ? tgemm::side_stream(st) : nullptr;
   bool side_busy = false;
   int rc;
   auto split_u = [&](int64_t i1, int which, cudaStream_t on) -> int {
-    // operand form of U[i1 : i1 + sb, i1 + width :] (independent of the sweep: kept off its chain)
-    const int64_t i2 = i1 + l.width;
+    // operand form of U[i1 : i1 + sb, i1 + sb :] (independent of the sweep: kept off its chain)
+    const int64_t i2 = i1 + l.sb;
     if (i2 >= K) return B200Q_OK;
-    const int rows = (int)(K - i1 < l.sb ? K - i1 : l.sb);
     float* hi = ub + (int64_t)which * 2 * l.ub;
-    return tgemm::split_transposed(p.U.one ? p.U.one + i1 * p.ldu + i2 : nullptr, Ud, i1 * p.ldu + i2, p.ldu, rows,
+    return tgemm::split_transposed(p.U.one ? p.U.one + i1 * p.ldu + i2 : nullptr, Ud, i1 * p.ldu + i2, p.ldu, l.sb,
                                    (int)(K - i2), hi, hi + l.ub, l.sb, l.rows_k * l.sb, distinct_u, on);
   };
   if (has_u && (rc = split_u(0, 0, st))) return rc;
@@ -634,32 +623,22 @@ static int sweep(Params p, int sdtype, bool global, int batch, const float* cons
     const int w = (int)(K - i1 < l.sb ? K - i1 : l.sb), which = l.sets == 2 ? blk & 1 : 0;
     const int64_t i2 = i1 + w;
     const bool trailing = i2 < K && has_u;
-    float* ehi = err + (int64_t)which * 2 * l.err;
-    float* bhi = ub + (int64_t)which * 2 * l.ub;
-    // W[:, c0 : c0 + n] -= Err[N, depth] * U[i1 : i1 + depth, c0 : c0 + n]
-    auto product = [&](int64_t c0, int64_t n, int depth) {
-      tgemm::Job j;
-      j.A = tgemm::Operand{ehi, ehi + l.err, l.sb, l.rows_n * batch, l.rows_n, 0};
-      j.B = tgemm::Operand{bhi, bhi + l.ub, l.sb, l.rows_k * distinct_u, l.rows_k, (int)(c0 - i1 - l.width)};
-      j.b_index = u_index;
-      j.M = (int)N; j.N = (int)n; j.Kd = depth; j.batch = batch; j.alpha = -1.0f; j.beta = 1.0f;
-      if (p.W.one) j.C = p.W.one + c0;
-      j.c_table = p.W.table; j.c_offset = c0; j.ldc = p.ldw; j.status = status;
-      return j;
-    };
+    p.i1 = (int)i1; p.sb = w;
+    p.err_hi = trailing ? err + (int64_t)which * 2 * l.err : nullptr;
+    p.err_lo = trailing ? p.err_hi + l.err : nullptr;
     p.lde = l.sb; p.err_batch = l.rows_n * l.sb;
-    for (int in = 0; in < w; in += l.width) {
-      const int wi = w - in < l.width ? w - in : l.width;
-      if (in > 0 && has_u && (rc = tgemm::launch(product(i1 + in, wi, in), st))) return rc;
-      const bool errors = i1 + in + wi < K && has_u;   // somebody after these columns takes them
-      p.i1 = (int)i1 + in; p.sb = wi;
-      p.err_hi = errors ? ehi + in : nullptr;
-      p.err_lo = errors ? ehi + l.err + in : nullptr;
-      kern<<<dim3(ctas, batch), 32 * warps_of(l.width), smem_bytes(l.width), st>>>(p);
-      B200Q_LAUNCH_CHECK();
-    }
+    kern<<<dim3(ctas, batch), 32 * warps_of(l.sb), smem_bytes(l.sb), st>>>(p);
+    B200Q_LAUNCH_CHECK();
     if (!trailing) continue;
-    tgemm::Job j = product(i2, K - i2, w);
+    // W[:, i2:] -= Err[N, w] * U[i1:i2, i2:]
+    float* bhi = ub + (int64_t)which * 2 * l.ub;
+    tgemm::Job j;
+    j.A = tgemm::Operand{p.err_hi, p.err_lo, l.sb, l.rows_n * batch, l.rows_n, 0};
+    j.B = tgemm::Operand{bhi, bhi + l.ub, l.sb, l.rows_k * distinct_u, l.rows_k, 0};
+    j.b_index = u_index;
+    j.M = (int)N; j.N = (int)(K - i2); j.Kd = w; j.batch = batch; j.alpha = -1.0f; j.beta = 1.0f;
+    if (p.W.one) j.C = p.W.one + i2;
+    j.c_table = p.W.table; j.c_offset = i2; j.ldc = p.ldw; j.status = status;
     if (!side) {
       if ((rc = tgemm::launch(j, st))) return rc;
       if ((rc = split_u(i2, l.sets == 2 ? which ^ 1 : 0, st))) return rc;
@@ -673,7 +652,7 @@ static int sweep(Params p, int sdtype, bool global, int batch, const float* cons
     if (side_busy) B200Q_TRY(cudaStreamWaitEvent(st, side->done, 0));
     if ((rc = tgemm::launch(j, st))) return rc;
     if (far.N > l.sb) {
-      far.B.row0 += l.sb; far.N -= l.sb; far.max_ctas = kNumSMs - ctas * batch;
+      far.B.row0 = l.sb; far.N -= l.sb; far.max_ctas = kNumSMs - ctas * batch;
       if (p.W.one) far.C = p.W.one + i2 + l.sb;
       far.c_offset = i2 + l.sb;
       if ((rc = tgemm::launch(far, side->stream))) return rc;
