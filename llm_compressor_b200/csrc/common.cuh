@@ -46,6 +46,27 @@ template <auto Kernel> inline int resident_grid(int threads, size_t smem, int64_
   const int64_t cap = (int64_t)kNumSMs * per_sm;
   return (int)(blocks_needed < 1 ? 1 : (blocks_needed < cap ? blocks_needed : cap));
 }
+// ---- chains of short kernels ------------------------------------------------------------------
+// Programmatic dependent launch: the next kernel of the stream is set up while this one ends (about 1.5 us each of a solve
+// of 190 launches).  A kernel launched by launch_chained begins with chain_wait(), before it touches device memory: it
+// returns once everything the kernels before it wrote is there.  chain_go(), late in a kernel, lets the next one start
+// to be set up; its CTAs then take room on the SMs, so not earlier than they are needed.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename... P, typename... A>
+inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
 inline int grid_for(int64_t blocks_needed, int blocks_per_sm) {
   int64_t cap = (int64_t)kNumSMs * blocks_per_sm;
   if (blocks_needed >= cap) return (int)cap;

@@ -116,6 +116,7 @@ __device__ __forceinline__ float* active_row(float* R, int ar, int kb) {
 }
 
 __global__ void __launch_bounds__(kThreads, 1) chol_diag_kernel(Mat mt, int k0, int n) {
+  chain_wait();
   extern __shared__ __align__(16) float sm[];
   float* R = sm;                    // rows 0..127: the block, then L; rows 128..255: the identity, then L^-T
   float* Lt = R + 2 * NB * LD;      // [16][20] transposed diagonal block of the step
@@ -259,6 +260,7 @@ __global__ void __launch_bounds__(kThreads, 1) chol_diag_kernel(Mat mt, int k0, 
     }
     __syncthreads();
   }
+  chain_go();
   if (tid == 0 && bad) {
     int* status = mt.status + 4 * blockIdx.x;
     if (atomicCAS(status, 0, B200Q_NOT_POSITIVE_DEFINITE) == 0) status[1] = k0 + bad;
@@ -297,6 +299,7 @@ constexpr int kVec = 16;
 constexpr int kPanelSmemFloats = (NB / 2 + kVec) * LD;
 
 __global__ void __launch_bounds__(kThreads) panel_kernel(Mat mt, float* P0, int K0, int n, int k) {
+  chain_wait();
   extern __shared__ __align__(16) float sm[];
   float* D = sm;                   // [64][LD] rows of D
   float* V = D + NB / 2 * LD;      // [16][LD] the vectors, contraction contiguous
@@ -332,6 +335,7 @@ __global__ void __launch_bounds__(kThreads) panel_kernel(Mat mt, float* P0, int 
       V[(idx & 15) * LD + (idx >> 4)] = x[i];
     }
   }
+  chain_go();
   cp_async_wait_all();
   __syncthreads();
   // a warp: 16 vectors x 8 outputs
@@ -354,6 +358,7 @@ __global__ void __launch_bounds__(kThreads) panel_kernel(Mat mt, float* P0, int 
 constexpr int kUpdSmemFloats = 32 * LD + NB * 40;
 
 __global__ void __launch_bounds__(kThreads) square_update_kernel(Mat mt, const float* P0, int K0, int n, int k, int tiles) {
+  chain_wait();
   extern __shared__ __align__(16) float sm[];
   float* Ps = sm;                // [32][LD]
   float* Qs = Ps + 32 * LD;      // second operand: [32][LD] contraction contiguous, or [128][40] column contiguous
@@ -402,6 +407,7 @@ __global__ void __launch_bounds__(kThreads) square_update_kernel(Mat mt, const f
     const int rr = r + (e >> 1) * 8, cc = c + (e & 1);
     old[e] = (!own && rr < n && cc < n) ? A[(int64_t)rr * mt.lda + cc] : 0.0f;
   }
+  chain_go();
   cp_async_wait_all();
   __syncthreads();
   float acc[1][4] = {};
@@ -419,6 +425,8 @@ __global__ void __launch_bounds__(kThreads) square_update_kernel(Mat mt, const f
 // update's second operand.
 __global__ void __launch_bounds__(256) split_square_kernel(Mat mt, int K0, int n, float* d_hi, float* d_lo,
                                                            float* t_hi, float* t_lo, int64_t t_batch) {
+  chain_wait();
+  chain_go();
   __shared__ float tile[32][33];
   const float* A = mt.A + blockIdx.y * mt.batch + (int64_t)K0 * mt.lda + K0;
   const int64_t db = (int64_t)blockIdx.y * OB * OB, tb = blockIdx.y * t_batch + (int64_t)K0 * OB;
@@ -448,6 +456,8 @@ __global__ void __launch_bounds__(256) split_square_kernel(Mat mt, int K0, int n
 // transposed; operand row = matrix row or column, zero-padded to 32.
 __global__ void __launch_bounds__(256) split_panel_kernel(Mat mt, int K0, int n, int r0, int r1, int tcols, float* hi,
                                                           float* lo, int64_t dst_batch) {
+  chain_wait();
+  chain_go();
   __shared__ float tile[32][33];
   const float* A = mt.A + blockIdx.y * mt.batch;
   hi += blockIdx.y * dst_batch;
@@ -548,15 +558,15 @@ static int factor(float* H, float* const* Hs, int batch, int64_t K, int64_t ldh,
     const bool last = K1 >= K;
     for (int k = 0; k < blocks; ++k) {
       const int bn = n - k * NB < NB ? n - k * NB : NB, below = n - k * NB - bn;
-      chol_diag_kernel<<<batch, kThreads, chol_smem, st>>>(mt, (int)K0 + k * NB, bn);
+      B200Q_TRY(launch_chained(chol_diag_kernel, dim3(batch), kThreads, chol_smem, st, mt, (int)K0 + k * NB, bn));
       B200Q_LAUNCH_CHECK();
       const int units = (below + kVec - 1) / kVec + k * NB / kVec;
       if (units == 0) continue;
-      panel_kernel<<<dim3(2 * units, batch), kThreads, panel_smem, st>>>(mt, P, (int)K0, n, k);
+      B200Q_TRY(launch_chained(panel_kernel, dim3(2 * units, batch), kThreads, panel_smem, st, mt, P, (int)K0, n, k));
       B200Q_LAUNCH_CHECK();
       const int rt = (below + 31) / 32, base = (k + 1) * (NB / 32), tiles = rt * base + rt * (rt + 1) / 2;
-      square_update_kernel<<<dim3(tiles + k * 16, batch), kThreads, kUpdSmemFloats * sizeof(float), st>>>(
-          mt, P, (int)K0, n, k, tiles);
+      B200Q_TRY(launch_chained(square_update_kernel, dim3(tiles + k * 16, batch), kThreads, kUpdSmemFloats * sizeof(float), st,
+                               mt, P, (int)K0, n, k, tiles));
       B200Q_LAUNCH_CHECK();
     }
     if (K0 == 0 && last) break;
@@ -566,13 +576,14 @@ static int factor(float* H, float* const* Hs, int batch, int64_t K, int64_t ldh,
         Q{q_hi, q_lo, OB, (int64_t)batch * rows, rows, 0};
     const int n2 = last ? 0 : (int)(K - K1 < OB ? K - K1 : OB);
     if (side_busy) B200Q_TRY(cudaStreamWaitEvent(st, side->done, 0));   // products of the step before
-    split_square_kernel<<<dim3(OB / 32 * (OB / 32), batch), 256, 0, st>>>(mt, (int)K0, n, d_hi, d_lo, last ? nullptr : q_hi,
-                                                                          q_lo, pb);
+    B200Q_TRY(launch_chained(split_square_kernel, dim3(OB / 32 * (OB / 32), batch), 256, 0, st, mt, (int)K0, n, d_hi, d_lo,
+                             last ? nullptr : q_hi, q_lo, pb));
     B200Q_LAUNCH_CHECK();
     auto split_panel = [&](int64_t r0, int64_t r1, int64_t tcols, cudaStream_t on) -> int {
       const int64_t tiles = ((r1 - r0 + 31) / 32 + tcols / 32) * ((n + 31) / 32);
       if (tiles == 0) return B200Q_OK;
-      split_panel_kernel<<<grid(tiles, row_ctas), 256, 0, on>>>(mt, (int)K0, n, (int)r0, (int)r1, (int)tcols, a_hi, a_lo, pb);
+      B200Q_TRY(launch_chained(split_panel_kernel, grid(tiles, row_ctas), 256, 0, on, mt, (int)K0, n, (int)r0, (int)r1, (int)tcols, a_hi,
+                               a_lo, pb));
       B200Q_LAUNCH_CHECK();
       return B200Q_OK;
     };

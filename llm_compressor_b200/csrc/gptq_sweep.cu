@@ -197,6 +197,7 @@ __device__ __forceinline__ void apply_errors(const ErrFrag& f, const float* u, f
 template <int SBLK, bool SB, int KIND, bool ZP>
 __global__ void __launch_bounds__(32 * warps_of(SBLK), SBLK == 512 ? 1 : 2) sweep_block_kernel(const __grid_constant__ Params p) {
   const float qmin = p.qr.qmin, qmax = p.qr.qmax;
+  chain_wait();
   extern __shared__ __align__(16) float sm[];
   constexpr int ULD = u_stride(SBLK);
   constexpr int NW = warps_of(SBLK), NT = 32 * NW;
@@ -526,6 +527,7 @@ __global__ void __launch_bounds__(32 * warps_of(SBLK), SBLK == 512 ? 1 : 2) swee
     if (m + 1 < micros) wait_u(m + 1);
     __syncthreads();
   }
+  chain_go();
   if (warp == 6) finish_errors(micros - 1);   // (a superblock with columns after it is a whole one)
   // tile out
   if (vecw) {
@@ -627,7 +629,7 @@ static int sweep(Params p, int sdtype, bool global, int batch, const float* cons
     p.err_hi = trailing ? err + (int64_t)which * 2 * l.err : nullptr;
     p.err_lo = trailing ? p.err_hi + l.err : nullptr;
     p.lde = l.sb; p.err_batch = l.rows_n * l.sb;
-    kern<<<dim3(ctas, batch), 32 * warps_of(l.sb), smem_bytes(l.sb), st>>>(p);
+    B200Q_TRY(launch_chained(kern, dim3(ctas, batch), 32 * warps_of(l.sb), smem_bytes(l.sb), st, p));
     B200Q_LAUNCH_CHECK();
     if (!trailing) continue;
     // W[:, i2:] -= Err[N, w] * U[i1:i2, i2:]

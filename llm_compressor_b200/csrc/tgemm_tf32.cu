@@ -241,6 +241,7 @@ tgemm_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ C
   if (PAIR) cluster_sync_all();   // the peer's barriers are initialised before anything signals them
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = s_tmem_base;
+  chain_wait();
   const Job& j = p.j;
   const int chunks = (j.Kd + kChunkK - 1) / kChunkK;
   const int64_t count = p.num_tiles * (unit + 1) / units - p.num_tiles * unit / units;
@@ -453,6 +454,7 @@ tgemm_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ C
     }
   }
 
+  chain_go();
   if (s_abort) {
     if (threadIdx.x == 0 && j.status)
       for (int k = 0; k < j.batch; ++k) atomicCAS(j.status + k * j.status_stride, 0, B200Q_ERR_DEVICE);
@@ -497,6 +499,8 @@ __global__ void __launch_bounds__(256) split_transposed_kernel(const float* __re
                                                                float* __restrict__ hi, float* __restrict__ lo,
                                                                int64_t ld_dst, int64_t dst_batch) {
   __shared__ float tile[32][33];
+  chain_wait();
+  chain_go();
   const float* __restrict__ src = table ? table[blockIdx.y] + src_offset : src0;
   hi += (int64_t)blockIdx.y * dst_batch;
   lo += (int64_t)blockIdx.y * dst_batch;
@@ -571,7 +575,8 @@ int split_transposed(const float* src, const float* const* table, int64_t src_of
   const int64_t tiles = (int64_t)((cols + 31) / 32) * (ld_dst / 32);
   const int cap = batch > 1 ? 8 * kNumSMs / batch + 1 : 8 * kNumSMs;
   dim3 grid((unsigned)(tiles < cap ? tiles : cap), (unsigned)batch, 1);
-  split_transposed_kernel<<<grid, 256, 0, st>>>(src, table, src_offset, ld_src, rows, cols, hi, lo, ld_dst, dst_batch);
+  B200Q_TRY(launch_chained(split_transposed_kernel, grid, 256, 0, st, src, table, src_offset, ld_src, rows, cols, hi, lo, ld_dst,
+                           dst_batch));
   B200Q_LAUNCH_CHECK();
   return B200Q_OK;
 }
@@ -694,14 +699,16 @@ static int launch_tiles(const Params& p, int units, cudaStream_t st) {
     cfg.blockDim = dim3(kThreads, 1, 1);
     cfg.dynamicSmemBytes = kSmemBytes;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     B200Q_TRY(cudaLaunchKernelEx(&cfg, kernel, mah, mal, mbh, mbl, p));
   } else {
-    kernel<<<units, kThreads, kSmemBytes, st>>>(mah, mal, mbh, mbl, p);
+    B200Q_TRY(launch_chained(kernel, dim3((unsigned)units), kThreads, kSmemBytes, st, mah, mal, mbh, mbl, p));
   }
   B200Q_LAUNCH_CHECK();
   return B200Q_OK;
