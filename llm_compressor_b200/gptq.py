@@ -11,6 +11,7 @@ all-expert calibration) share one permutation and one factor U instead of recomp
 """
 from __future__ import annotations
 
+import struct
 import warnings
 from dataclasses import dataclass
 from typing import Optional
@@ -117,12 +118,17 @@ class HessianFactor:
 
     def resolve(self) -> "HessianFactor":
         if self.ok is None:
-            st = ops.gptq_factor_status(self.status)
-            self.ok = st != _lib.NOT_POSITIVE_DEFINITE
-            if not self.ok:
-                warnings.warn(_NOT_PD_MESSAGE)
-                self.U = None
+            self.settle(self.status.reshape(-1)[:4].tolist())
         return self
+
+    def settle(self, words) -> None:
+        """``words``: the four status words, read from the device."""
+        if words[2] != 0:
+            raise _lib.B200QError("b200q_gptq_factor: a bounded wait inside the GEMM kernel expired")
+        self.ok = words[0] != _lib.NOT_POSITIVE_DEFINITE
+        if not self.ok:
+            warnings.warn(_NOT_PD_MESSAGE)
+            self.U = None
 
 
 def factor_hessian(hessian: torch.Tensor, percdamp: float = 0.01, actorder=None,
@@ -168,12 +174,7 @@ def resolve_factors(factors) -> None:
         return
     words = torch.stack([f.status.reshape(-1)[:4] for f in pending]).tolist()
     for f, st in zip(pending, words):
-        if st[2] != 0:
-            raise _lib.B200QError("b200q_gptq_factor: a bounded wait inside the GEMM kernel expired")
-        f.ok = st[0] != _lib.NOT_POSITIVE_DEFINITE
-        if not f.ok:
-            warnings.warn(_NOT_PD_MESSAGE)
-            f.U = None
+        f.settle(st)
 
 
 @dataclass
@@ -197,7 +198,7 @@ def _sweep_input(module, quant_args, hessian, percdamp, factor, W=None, qparams=
     ``order`` (column order of the groups) likewise."""
     args = QuantizationArgs.of(quant_args)
     strategy, actorder = args.strategy, args.actorder
-    weight = module.weight.data if isinstance(module.weight, torch.nn.Parameter) else module.weight
+    weight = _weight_of(module)
     observer: Observer = module.weight_observer
     N, K = weight.shape
     if strategy not in ("tensor", "channel", "group", "tensor_group", "block"):
@@ -211,7 +212,7 @@ def _sweep_input(module, quant_args, hessian, percdamp, factor, W=None, qparams=
     if factor is None:
         if hessian is None or hessian.shape != (K, K):
             raise ValueError("hessian must be float32 [in_features, in_features]")
-        factor = factor_hessian(hessian, percdamp, actorder)
+        factor = factor_hessian(hessian, percdamp, actorder, defer=True)
     elif factor.K != K or (factor.perm is not None) != bool(actorder):
         raise ValueError("factor does not match this module / act-order setting")
     perm = factor.perm
@@ -298,11 +299,29 @@ def quantize_weight(module, quant_args, hessian: Optional[torch.Tensor], blocksi
     if defer:
         loss = losses.sum()
         out["_status"] = status   # the sweep's device status word; the caller checks and removes it
-    else:
-        loss, st = torch.stack([losses.sum(), status[0].to(torch.float32)]).tolist()
-        if st != 0:
-            raise _lib.B200QError("b200q_gptq_sweep: a bounded wait inside the GEMM kernel expired")
-    return loss, out
+        return loss, out
+    # one wait for everything: the loss, the sweep's status and, of a factorisation that nobody has waited for yet
+    # (the sweep was queued behind it without asking), the factor's
+    waiting = inp.factor.ok is None
+    words = [losses.sum().reshape(1).view(torch.int32), status] + ([inp.factor.status.reshape(-1)[:4]] if waiting else [])
+    words = torch.cat(words).tolist()
+    if waiting:
+        inp.factor.settle(words[2:])
+        if not inp.factor.ok:   # round to nearest with the parameters that are there already
+            W = ops.gather_columns_f32(_weight_of(module), inp.factor.perm)
+            ops.gptq_zero_dead_columns(inp.factor.diag, W)
+            inp.W = W
+            losses, status = ops.gptq_sweep(W, None, inp.scale, zero_point, inp.args, blocksize=blocksize,
+                                            col_group=inp.col_group, global_scale=inp.global_scale, return_status=True)
+            out = _sweep_output(inp)
+            words = torch.cat([losses.sum().reshape(1).view(torch.int32), status]).tolist()
+    if words[1] != 0:
+        raise _lib.B200QError("b200q_gptq_sweep: a bounded wait inside the GEMM kernel expired")
+    return struct.unpack("<f", struct.pack("<i", words[0]))[0], out
+
+
+def _weight_of(module) -> torch.Tensor:
+    return module.weight.data if isinstance(module.weight, torch.nn.Parameter) else module.weight
 
 
 def quantize_weights_batched(modules, quant_args, factors, blocksize: int = 128, percdamp: float = 0.01):
@@ -312,7 +331,7 @@ def quantize_weights_batched(modules, quant_args, factors, blocksize: int = 128,
     device tensors and the first dict carries the sweep's ``"_status"`` for all of them.
     As with the deferred single call, the caller resolves the factors afterwards and redoes the
     modules whose factorisation failed."""
-    weights = [m.weight.data if isinstance(m.weight, torch.nn.Parameter) else m.weight for m in modules]
+    weights = [_weight_of(m) for m in modules]
     perms = [f.perm for f in factors]
     if any((p is None) != (perms[0] is None) for p in perms):
         raise ValueError("the factors of a batch must all carry a permutation or none")
