@@ -1,0 +1,241 @@
+"""Kernels and dispatch branches at the sizes where they can go wrong: edges of tiles and blocks, remainders, misaligned
+rows, the smallest and largest of a branch's range.  Bytes and scales exact against the CPU oracle or the element-wise
+chain; float32 solves against float64 with the tolerances of the other GPU tests."""
+import pytest
+import torch
+
+import oracle
+from helpers import args_from, bits_equal, mismatch, synth_acts, synth_weight
+from llm_compressor_b200 import QuantizationModifier, compress_state_dict, gptq, observers, oneshot, ops
+from llm_compressor_b200.awq import scaled_fake_quantize
+from llm_compressor_b200.quant_args import QuantizationArgs, preset_name_to_scheme
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _spd(K, seed):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    X = torch.randn(2 * K + 64, K, generator=g, device=DEV, dtype=torch.float64)
+    H = X.t() @ X / K
+    H.diagonal().add_(0.05)
+    return H
+
+
+def _inverse_residual(U, H):
+    """U^T U = H^-1, seen as U H U^T = I (float64, on the device)."""
+    U = U.double()
+    return float((U @ H @ U.t() - torch.eye(H.shape[0], device=DEV, dtype=torch.float64)).abs().max())
+
+
+# one, two and three outer blocks of 512, their remainders, odd widths, and tile widths of the products
+@pytest.mark.parametrize("K", [1, 16, 127, 129, 511, 512, 513, 640, 1030, 1536, 2500])
+def test_factor_at_block_edges(K):
+    H = _spd(K, K)
+    one = H.float()
+    assert ops.gptq_factor(one) == 0
+    assert float(one.tril(-1).abs().max()) == 0.0 if K > 1 else True
+    assert _inverse_residual(one, H) < 2e-4
+    if K <= 1030:
+        many = [H.float() for _ in range(3)]
+        assert int(ops.gptq_factor_batched(many).abs().max()) == 0
+        assert all(_inverse_residual(u, H) < 2e-4 for u in many)
+
+
+# rows: one CTA, part of one, more CTAs than SMs (narrow superblocks); columns: superblock and micro-block remainders
+@pytest.mark.parametrize("N,K,scheme", [(1, 16, "FP8_DYNAMIC"), (33, 520, "FP8_DYNAMIC"), (64, 1032, "W8A16"),
+                                        (31, 513, "W8A16"), (4768, 264, "FP8_DYNAMIC"), (5000, 640, "W4A16")])
+def test_sweep_at_superblock_edges(N, K, scheme):
+    args = preset_name_to_scheme(scheme, ["Linear"]).weights
+    w = (torch.randn(N, K, generator=torch.Generator().manual_seed(K)) * 0.02).bfloat16().to(DEV)
+    H = _spd(K, 3)
+    U = torch.linalg.cholesky(torch.linalg.inv(H), upper=True)
+    scale, zp = ops.qparams(*ops.observe_minmax(w, args), args)
+    wf = w.float()
+    losses = ops.gptq_sweep(wf, U.float(), scale, None, args)
+    # the recursion in float64 with the same codes' rules, column by column
+    ref, Ud = w.double(), U
+    spread = scale.float() if scale.shape[1] == 1 else scale.float().repeat_interleave(args.group_size, 1)
+    qmin, qmax = (-448.0, 448.0) if args.type == "float" else (-(1 << (args.num_bits - 1)), (1 << (args.num_bits - 1)) - 1)
+    out, total = torch.empty_like(wf), torch.zeros(N, device=DEV, dtype=torch.float64)
+    for i in range(K):
+        s = spread[:, min(i, spread.shape[1] - 1)]
+        v = (ref[:, i].float() / s).clamp(qmin, qmax)
+        q = v.to(torch.float8_e4m3fn).float() if args.type == "float" else v.round()
+        q = (q * s).bfloat16().float()
+        err = (ref[:, i] - q.double()) / Ud[i, i]
+        out[:, i], total = q, total + err * err / 2
+        ref[:, i + 1:] -= err[:, None] * Ud[i, i + 1:]
+    assert mismatch(wf, out) <= 0.005
+    assert torch.allclose(losses.double(), total, rtol=0.02, atol=1e-9)
+
+
+def test_sweep_exact_pass_at_rounding_boundaries():
+    """Every quotient on a rounding boundary: the fast test of a code fails in every micro-block."""
+    args = preset_name_to_scheme("W8A16", ["Linear"]).weights
+    N, K = 40, 96
+    w = (torch.randint(-100, 100, (N, K), generator=torch.Generator().manual_seed(0)).float() + 0.5) * 0.0078125
+    wf = w.to(DEV)
+    scale = torch.full((N, 1), 0.0078125, device=DEV).bfloat16()
+    ops.gptq_sweep(wf, None, scale, None, args)
+    assert bits_equal(wf, (w / 0.0078125).round() * 0.0078125)
+
+
+@pytest.mark.parametrize("count,N,K,scheme", [(5, 96, 520, "FP8_DYNAMIC"), (3, 70, 640, "W4A16")])
+def test_batched_sweep_with_shared_factors(count, N, K, scheme):
+    args = preset_name_to_scheme(scheme, ["Linear"]).weights
+    Us = [torch.linalg.cholesky(torch.linalg.inv(_spd(K, i)), upper=True).float() for i in range(2)]
+    pick = [Us[i % 2] for i in range(count)]
+    ws = [(torch.randn(N, K, generator=torch.Generator().manual_seed(i)) * 0.02).bfloat16().to(DEV) for i in range(count)]
+    qp = [ops.qparams(*ops.observe_minmax(w, args), args) for w in ws]
+    got = [w.float() for w in ws]
+    losses = ops.gptq_sweep_batched(got, pick, [s for s, _ in qp], None, args)
+    for k in range(count):
+        ref = ws[k].float()
+        ref_losses = ops.gptq_sweep(ref, pick[k], qp[k][0], None, args)
+        assert mismatch(got[k], ref) <= 0.005
+        assert torch.allclose(losses[k], ref_losses, rtol=0.01)
+
+
+# columns in order and permuted, whole 16-byte pieces and not, rows that are no multiple of four, K too wide for four
+# rows in shared memory
+@pytest.mark.parametrize("N,K", [(1, 1), (3, 40), (5, 37), (130, 1160), (2, 30000)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_column_gathers_and_scatters(N, K, dtype):
+    g = torch.Generator(device=DEV).manual_seed(K)
+    w = torch.randn(N, K, generator=g, device=DEV).to(dtype)
+    perm = torch.randperm(K, generator=g, device=DEV).int()
+    diag = (torch.rand(K, generator=g, device=DEV) > 0.3).float()
+    for p in (None, perm):
+        ref = w.float() if p is None else w.float()[:, p.long()]
+        assert torch.equal(ops.gather_columns_f32(w, p), ref)
+        assert torch.equal(ops.scatter_columns_cast(ref, dtype, p), w)
+        ws = [w, w.flip(0).contiguous()]
+        many = ops.gather_columns_f32_batched(ws, None if p is None else [p, p], [diag, diag])
+        assert torch.equal(many[0], ref * diag)
+        back = ops.scatter_columns_cast_batched(torch.stack([ref, ref]), dtype, None if p is None else [p, p])
+        assert torch.equal(back[1], w)
+
+
+@pytest.mark.parametrize("K", [3, 40, 129, 700])
+def test_batched_prologue_and_mirror(K):
+    Hs = [torch.randn(K, K, generator=torch.Generator(device=DEV).manual_seed(i), device=DEV) for i in range(3)]
+    for H in Hs:
+        H.diagonal().abs_()
+        H[K // 2, K // 2] = 0.0   # a dead column
+    full = [H.clone() for H in Hs]
+    ops.hessian_finalize_many(full, [0.5, 1.0, 2.0])
+    for H, f, s in zip(Hs, full, (0.5, 1.0, 2.0)):
+        one = H.clone()
+        ops.hessian_finalize(one, s)
+        low = (H * s).tril()
+        assert torch.equal(f, low + low.tril(-1).t()) and torch.equal(f, one)
+    for actorder in (False, True):
+        mats, perm, diag = ops.gptq_prologue_batched([f.clone() for f in full], 0.01, actorder)
+        for i, f in enumerate(full):
+            H, p, d = gptq._factor_prologue(f.clone(), 0.01, "weight" if actorder else None)
+            assert torch.equal(diag[i], d)
+            assert not actorder or torch.equal(perm[i], p)
+            assert torch.allclose(mats[i], H, rtol=1e-6, atol=0)
+
+
+# short and long accumulation, widths with a ragged last tile, one split and many
+@pytest.mark.parametrize("T,K", [(8, 8), (64, 264), (513, 1160), (1024, 4104), (2048, 2056)])
+def test_hessian_update_adds_to_what_is_there(T, K):
+    g = torch.Generator(device=DEV).manual_seed(T)
+    xs = [torch.randn(T, K, generator=g, device=DEV).bfloat16() for _ in range(2)]
+    H = torch.zeros(K, K, device=DEV)
+    for x in xs:
+        ops.hessian_syrk(x, H)
+    ops.hessian_finalize(H, 0.5)
+    ref = sum(x.double().t() @ x.double() for x in xs)
+    assert float((H.double() - ref).norm() / ref.norm()) < 1e-5
+
+
+SCHEMES = ["W4A16", "W4A16_ASYM", "W8A16", "FP8_DYNAMIC", "FP8_BLOCK", "NVFP4A16", "MXFP4A16", "MXFP8A16"]
+
+
+# a row or block each per warp, lane or CTA; ragged blocks; rows misaligned to 16 bytes; too many rows for a CTA each
+@pytest.mark.parametrize("scheme", SCHEMES)
+@pytest.mark.parametrize("N,K", [(1, 128), (130, 384), (129, 1152), (2400, 256), (67, 200)])
+def test_one_pass_parameters_and_codes(scheme, N, K):
+    s = preset_name_to_scheme(scheme, ["Linear"])
+    args = s.weights
+    if args.group_size and K % args.group_size:
+        pytest.skip("group size does not divide K")
+    names = ["gate_proj", "up_proj"] if scheme == "NVFP4A16" else ["o_proj"]
+    model = torch.nn.Module()
+    for i, name in enumerate(names):
+        lin = torch.nn.Linear(K, N, bias=False, dtype=torch.bfloat16, device=DEV)
+        lin.weight.data = (synth_weight(N, K, seed=N + K + i) * (1 + 3 * i)).to(DEV)
+        model.add_module(name, lin)
+    oneshot(model, recipe=QuantizationModifier(targets="Linear", scheme=scheme))
+    spec = oracle.preset(scheme)
+    obs = [oracle.WeightObserver(spec) for _ in names]
+    if len(obs) > 1:
+        top = max(float(model.get_submodule(n).weight.abs().max()) for n in names)
+    for name, o in zip(names, obs):
+        lin = model.get_submodule(name)
+        w = lin.weight.data.cpu()
+        if len(obs) > 1:   # the global scale of the larger of the two: an element of that size in a copy of the weight
+            lift = torch.cat([w, torch.full((1, K), top, dtype=w.dtype)])
+            qp = o(lift).get_qparams()
+            qp = dict(qp, scale=qp["scale"][:N], zero_point=qp["zero_point"][:N])
+            assert bits_equal(lin.weight_global_scale.data, qp["global_scale"])
+        else:
+            qp = o(w).get_qparams()
+        assert bits_equal(lin.weight_scale.data, qp["scale"].to(w.dtype))
+        assert bits_equal(lin.weight_zero_point.data, qp["zero_point"])
+        sd = {"weight": w, "weight_scale": qp["scale"].to(w.dtype), "weight_zero_point": qp["zero_point"]}
+        if qp["global_scale"] is not None:
+            sd["weight_global_scale"] = qp["global_scale"]
+        ref = oracle.compress_weight(sd, spec)
+        out = compress_state_dict({k: v.to(DEV) for k, v in sd.items()}, s, "pack-quantized" if args.type == "int" else None)
+        for k in ("weight_packed", "weight"):
+            if k in ref and k in out:
+                assert bits_equal(out[k], ref[k]), (k, mismatch(out[k], ref[k]))
+
+
+def test_batched_parameters_equal_the_single_ones():
+    for scheme in ("W4A16_ASYM", "W8A16", "FP8_BLOCK", "MXFP4A16"):
+        args = preset_name_to_scheme(scheme, ["Linear"]).weights
+        ws = [synth_weight(200, 256, seed=i).to(DEV) for i in range(5)]
+        scales, zps = ops.minmax_qparams(ws, args)
+        for w, s, z in zip(ws, scales, zps):
+            ref_s, ref_z = ops.qparams(*ops.observe_minmax(w, args), args)
+            assert bits_equal(s, ref_s) and bits_equal(z, ref_z)
+
+
+# groups and channels, symmetric or not, odd rows, channels of one and of many pieces per lane
+@pytest.mark.parametrize("kw", [dict(num_bits=4, symmetric=True, strategy="group", group_size=128),
+                                dict(num_bits=4, symmetric=False, strategy="group", group_size=32),
+                                dict(num_bits=8, symmetric=False, strategy="channel"),
+                                dict(num_bits=8, symmetric=True, strategy="channel")])
+@pytest.mark.parametrize("N,K", [(1, 128), (33, 384), (7, 4096), (130, 6144)])
+def test_scale_search_step_equals_the_element_wise_chain(kw, N, K):
+    args = QuantizationArgs(type="int", **kw)
+    w = synth_weight(N, K, seed=N + K).to(DEV)
+    s = torch.exp(0.5 * torch.randn(K, generator=torch.Generator(device=DEV).manual_seed(1), device=DEV))
+    got = ops.scaled_fake_quantize(w, s, args)
+    assert got is not None
+    scaled = (w * s.view(1, -1)).to(w.dtype)
+    qp = ops.qparams(*ops.observe_minmax(scaled, args), args)
+    ref = (ops.fake_quantize(scaled, qp[0], qp[1], args) / s.view(1, -1)).to(w.dtype)
+    assert bits_equal(got, ref), mismatch(got, ref)
+
+
+# table of powers: every code type, groups and whole rows, symmetric or not, rows that are no multiple of a CTA's
+@pytest.mark.parametrize("scheme", SCHEMES)
+@pytest.mark.parametrize("N,K", [(3, 128), (130, 640)])
+def test_grid_search_against_the_oracle(scheme, N, K):
+    args = preset_name_to_scheme(scheme, ["Linear"]).weights
+    w = synth_weight(N, K, seed=5 * N + K)
+    spec = oracle.preset(scheme)
+    o = oracle.WeightObserver(spec, "memoryless_mse")
+    o(w)
+    mn, mx = ops.observe_mse(w.to(DEV), args)
+    # two candidates whose errors are equal to rounding may swap: compare all but a few groups
+    for got, ref in ((mn, o.min_vals), (mx, o.max_vals)):
+        differ = (got.cpu().float() != ref.float()).float().mean()
+        assert float(differ) <= 0.02, float(differ)
+        assert float((got.cpu().float() - ref.float()).norm() / ref.float().norm()) < 0.02
