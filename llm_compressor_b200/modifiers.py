@@ -743,6 +743,13 @@ class GPTQModifier(QuantizationMixin):
         if jobs:
             run_concurrent([lambda mods=mods: self._compress_group(mods) for mods in jobs], device,
                            max_streams=self.parallel_streams)
+            # the jobs end in an order that varies from run to run: the losses are kept in that of the jobs' lengths (a
+            # chain of columns for the factor and one for each sweep)
+            for mods in sorted(jobs, key=lambda mods: mods[0].weight.shape[1] * (1 + len(mods))):
+                for m in mods:
+                    name = self._module_names.get(m, type(m).__name__)
+                    if name in self.losses:
+                        self.losses[name] = self.losses.pop(name)
 
     def _queue_factors(self, module_list, make_factor):
         """Take the modules of one Hessian out of the pending tables and give each the factor of its

@@ -14,6 +14,12 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 
 
+def _spec(scheme):
+    if scheme == "FP8_BLOCK":
+        return oracle.preset("FP8_DYNAMIC", strategy="block", block_structure=[128, 128])
+    return oracle.preset(scheme)
+
+
 def _spd(K, seed):
     g = torch.Generator(device=DEV).manual_seed(seed)
     X = torch.randn(2 * K + 64, K, generator=g, device=DEV, dtype=torch.float64)
@@ -170,10 +176,10 @@ def test_one_pass_parameters_and_codes(scheme, N, K):
         lin.weight.data = (synth_weight(N, K, seed=N + K + i) * (1 + 3 * i)).to(DEV)
         model.add_module(name, lin)
     oneshot(model, recipe=QuantizationModifier(targets="Linear", scheme=scheme))
-    spec = oracle.preset(scheme)
+    spec = _spec(scheme)
     obs = [oracle.WeightObserver(spec) for _ in names]
     if len(obs) > 1:
-        top = max(float(model.get_submodule(n).weight.abs().max()) for n in names)
+        top = max(float(model.get_submodule(n).weight.data.abs().max()) for n in names)
     for name, o in zip(names, obs):
         lin = model.get_submodule(name)
         w = lin.weight.data.cpu()
@@ -230,7 +236,7 @@ def test_scale_search_step_equals_the_element_wise_chain(kw, N, K):
 def test_grid_search_against_the_oracle(scheme, N, K):
     args = preset_name_to_scheme(scheme, ["Linear"]).weights
     w = synth_weight(N, K, seed=5 * N + K)
-    spec = oracle.preset(scheme)
+    spec = _spec(scheme)
     o = oracle.WeightObserver(spec, "memoryless_mse")
     o(w)
     mn, mx = ops.observe_mse(w.to(DEV), args)
