@@ -148,11 +148,16 @@ __global__ void __launch_bounds__(256) mse_group_kernel(const void* __restrict__
 constexpr int kTable = 32768;
 constexpr size_t kTableBytes = kTable * 2;
 
+// Where entry i stands.  An error is a difference of two close numbers with few significant bits left, so the low bits of
+// its pattern are mostly zero: in plain order the look-ups of a warp meet in a few banks (FP8 errors use 16 of 128
+// patterns of an exponent).  Both halves of a pair at once.
+__device__ __forceinline__ uint32_t table_place(uint32_t i) { return i ^ ((i >> 4) & 0x07FF07FFu); }
+
 __global__ void __launch_bounds__(256) make_table_kernel(__nv_bfloat16* __restrict__ table, float norm, int* __restrict__ ctl,
                                                          int n) {
   const int i = blockIdx.x * 256 + threadIdx.x;
   const float d = __uint_as_float((uint32_t)i << 16);
-  if (i < kTable) table[i] = __float2bfloat16_rn(d == 0.0f ? 0.0f : powf(d, norm));
+  if (i < kTable) table[table_place((uint32_t)i)] = __float2bfloat16_rn(d == 0.0f ? 0.0f : powf(d, norm));
   if (blockIdx.x == 0)
     for (int k = threadIdx.x; k < n; k += 256) ctl[k] = 0;
 }
@@ -231,7 +236,7 @@ __device__ __forceinline__ float chunk_error(const uint32_t (&w)[4], const Cand&
   }
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    const uint32_t d = pair_error<KIND, SYM>(w[k], q, qmin2, qmax2);
+    const uint32_t d = table_place(pair_error<KIND, SYM>(w[k], q, qmin2, qmax2));
     err += __uint_as_float((uint32_t)tab[d & 0xFFFFu] << 16);
     err += __uint_as_float((uint32_t)tab[d >> 16] << 16);
   }

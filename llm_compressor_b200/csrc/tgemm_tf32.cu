@@ -658,7 +658,7 @@ static int pair_capacity() {
 // epilogue, about 20 cycles per column, is not hidden.
 static void pick_tiles(Params& p, int ctas, int pairs) {
   const double chunk[3] = {800.0, 1150.0, 1700.0};
-  static const double pair_chunk = [] { const char* e = getenv("PAIR_CHUNK"); return e ? atof(e) : 1600.0; }();
+  const double pair_chunk = 1600.0;   // K = 14336: factor 13.2 -> 11.7 ms against single CTAs of 128 x 256
   const Job& j = p.j;
   const int chunks = (j.Kd + kChunkK - 1) / kChunkK;
   double best_cost = 0.0;
