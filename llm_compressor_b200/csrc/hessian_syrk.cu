@@ -510,6 +510,7 @@ syrk_pair_kernel(const __grid_constant__ CUtensorMap xmap, Params p) {
   cluster_sync_all();   // the peer's barriers are initialised before anything signals them
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = s_tmem_base;
+  chain_wait();   // (setting up overlaps the end of the kernel before: hidden in calls of a few hundred tokens)
 
   const int total_units = p.tiles * p.splits;
 
@@ -656,6 +657,7 @@ syrk_pair_kernel(const __grid_constant__ CUtensorMap xmap, Params p) {
   }
 
   // ---------------------------------------------------------------------- teardown
+  chain_go();
   if (s_abort) {
     const long long t0 = clock64();
     while (clock64() - t0 < 2000000LL) __nanosleep(1000);
@@ -678,6 +680,8 @@ constexpr int kFinTile = 64;
 __global__ void __launch_bounds__(256) finalize_kernel(float* H0, float* const* Hs, const float* scales, int64_t K, int64_t ldh,
                                                        float scale, bool vec) {
   __shared__ float tile[kFinTile][kFinTile + 1];
+  chain_wait();
+  chain_go();
   float* H = Hs ? Hs[blockIdx.y] : H0;
   if (scales) scale = scales[blockIdx.y];
   // patches of 8 x 8 blocks: what the CTAs write at the same time makes whole 2 KB pieces of rows on both sides of the
@@ -895,11 +899,13 @@ int b200q_hessian_syrk(const void* X, int64_t T, int64_t K, int64_t ldx, float* 
     cfg.blockDim = dim3(kThreads, 1, 1);
     cfg.dynamicSmemBytes = kPairSmemBytes;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     B200Q_TRY(cudaLaunchKernelEx(&cfg, syrk_pair_kernel, map, p));
     B200Q_LAUNCH_CHECK();
     return B200Q_OK;
@@ -939,8 +945,8 @@ static int finalize(float* H, float* const* Hs, const float* scales, int count, 
   using namespace b200q::syrk;
   const int64_t np = (K + 8 * kFinTile - 1) / (8 * kFinTile), nblk = np * (np + 1) / 2 * 64, cap = 8 * kNumSMs / count + 1;
   const bool vec = (ldh & 3) == 0 && (Hs || (((uintptr_t)H) & 15) == 0);   // (a batch's matrices are whole allocations)
-  finalize_kernel<<<dim3((unsigned)(nblk < cap ? nblk : cap), (unsigned)count), 256, 0, (cudaStream_t)stream>>>(
-      H, Hs, scales, K, ldh, scale, vec);
+  B200Q_TRY(launch_chained(finalize_kernel, dim3((unsigned)(nblk < cap ? nblk : cap), (unsigned)count), 256, 0,
+                           (cudaStream_t)stream, H, Hs, scales, K, ldh, scale, vec));
   B200Q_LAUNCH_CHECK();
   return B200Q_OK;
 }

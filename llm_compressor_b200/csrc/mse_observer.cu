@@ -259,10 +259,10 @@ __device__ __forceinline__ void chunk_range(const uint4& raw, float& lo, float& 
 // are derived once per R * 8 elements.  The chunk sums are added in the order of a butterfly over all chunks of the
 // group, whatever R is.
 template <int KIND, bool SYM, int R>
-__global__ void __launch_bounds__(256) mse_group_bf16_kernel(const void* __restrict__ W, int64_t N, int64_t K, int64_t ldw,
+__global__ void __launch_bounds__(256, 3) mse_group_bf16_kernel(const void* __restrict__ W, int64_t N, int64_t K, int64_t ldw,
                                                              int g, Cfg c, const __nv_bfloat16* __restrict__ table,
                                                              int* __restrict__ ctl, int pass, void* __restrict__ mn_out,
-                                                             void* __restrict__ mx_out) {
+                                                             void* __restrict__ mx_out, uint32_t* __restrict__ better) {
   using T = __nv_bfloat16;
   extern __shared__ __align__(16) unsigned short s_table[];
   __shared__ float s_shrink[1024];
@@ -298,6 +298,8 @@ __global__ void __launch_bounds__(256) mse_group_bf16_kernel(const void* __restr
     const float mn = bf16r(lo * c.expand), mx = bf16r(hi * c.expand);
     float best_err = 3.3895313892515355e38f;  // finfo(bfloat16).max
     float best_mn = mn, best_mx = mx;
+    uint32_t mask = 0;
+#pragma unroll 1   // (unrolled, the candidates outgrow the instruction cache: 188 us instead of 136 for int4, 3000 x 3840)
     for (int i = 0; i < limit; ++i) {
       const float p = i < 1024 ? s_shrink[i] : shrink_factor(i, c.grid);
       const float smn = bf16r(mn * p), smx = bf16r(mx * p);
@@ -309,13 +311,14 @@ __global__ void __launch_bounds__(256) mse_group_bf16_kernel(const void* __restr
       for (int o = L >> 1; o > 0; o >>= 1) err += __shfl_xor_sync(0xffffffffu, err, o);
       err = bf16r(err);
       if (live && err < best_err) {
-        best_err = err; best_mn = smn; best_mx = smx;
+        best_err = err; best_mn = smn; best_mx = smx; mask |= 1u << (i & 31);
         if (pass == 0 && j == 0 && ((volatile int*)ctl)[1 + i] == 0) atomicOr(&ctl[1 + i], 1);
       }
     }
     if (live && j == 0) {
-      ((T*)mn_out)[gi] = __float2bfloat16_rn(best_mn);
-      ((T*)mx_out)[gi] = __float2bfloat16_rn(best_mx);
+      if (better) better[gi] = mask;
+      ((T*)mn_out)[gi] = __float2bfloat16_rn(better ? mn : best_mn);
+      ((T*)mx_out)[gi] = __float2bfloat16_rn(better ? mx : best_mx);
     }
   }
 }
@@ -327,7 +330,7 @@ template <int KIND, bool SYM>
 __global__ void __launch_bounds__(256) mse_tile_bf16_kernel(const void* __restrict__ W, int64_t N, int64_t K, int64_t ldw,
                                                             int bh, int bw, Cfg c, const __nv_bfloat16* __restrict__ table,
                                                             int* __restrict__ ctl, int pass, void* __restrict__ mn_out,
-                                                            void* __restrict__ mx_out) {
+                                                            void* __restrict__ mx_out, uint32_t* __restrict__ better) {
   using T = __nv_bfloat16;
   extern __shared__ __align__(16) unsigned short s_table[];
   uint4* data = reinterpret_cast<uint4*>(s_table + kTable);
@@ -356,6 +359,7 @@ __global__ void __launch_bounds__(256) mse_tile_bf16_kernel(const void* __restri
     for (int w = 0; w < 8; ++w) { lo = fminf(lo, s_lo[w]); hi = fmaxf(hi, s_hi[w]); }
     const float mn = bf16r(lo * c.expand), mx = bf16r(hi * c.expand);
     float best_err = 3.3895313892515355e38f, best_mn = mn, best_mx = mx;
+    uint32_t mask = 0;
     for (int i0 = 0, turn = 0; i0 < limit; i0 += 4, turn ^= 1) {
       Cand q[4];
       float smn[4], smx[4], err[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -383,14 +387,15 @@ __global__ void __launch_bounds__(256) mse_tile_bf16_kernel(const void* __restri
         for (int w = 0; w < 8; ++w) tot += s_part[turn][w][k];
         tot = bf16r(tot);
         if (i0 + k < limit && tot < best_err) {
-          best_err = tot; best_mn = smn[k]; best_mx = smx[k];
+          best_err = tot; best_mn = smn[k]; best_mx = smx[k]; mask |= 1u << ((i0 + k) & 31);
           if (pass == 0 && threadIdx.x == 0 && ((volatile int*)ctl)[1 + i0 + k] == 0) atomicOr(&ctl[1 + i0 + k], 1);
         }
       }
     }
     if (threadIdx.x == 0) {
-      ((T*)mn_out)[grp] = __float2bfloat16_rn(best_mn);
-      ((T*)mx_out)[grp] = __float2bfloat16_rn(best_mx);
+      if (better) better[grp] = mask;
+      ((T*)mn_out)[grp] = __float2bfloat16_rn(better ? mn : best_mn);
+      ((T*)mx_out)[grp] = __float2bfloat16_rn(better ? mx : best_mx);
     }
     __syncthreads();
   }
@@ -557,6 +562,28 @@ __global__ void mse_span_store_kernel(const float* __restrict__ state, void* __r
   E::store((T*)mx_out, state[4]);
 }
 
+// Which candidate counts is known once every group has been through all of them: the search ends for all groups at once,
+// when no group has found a better one for `patience` candidates.  Groups with up to 32 candidates note which ones were
+// better than all before (`better`, bit i), and the last of these before the end is taken here; with more, the search is
+// run a second time up to the end (half as long again where it ends early: FP8 per channel 365 us, 205 without).
+__global__ void __launch_bounds__(256) pick_kernel(const int* __restrict__ ctl, const uint32_t* __restrict__ better,
+                                                   int64_t groups, Cfg c, __nv_bfloat16* __restrict__ mn,
+                                                   __nv_bfloat16* __restrict__ mx) {
+  int stale = 0, run = c.steps;
+  for (int i = 0; i < c.steps; ++i) {
+    if (ctl[1 + i]) stale = 0;
+    else if (++stale >= c.patience) { run = i + 1; break; }
+  }
+  const uint32_t before = run >= 32 ? 0xFFFFFFFFu : (1u << run) - 1u;
+  for (int64_t g = (int64_t)blockIdx.x * 256 + threadIdx.x; g < groups; g += (int64_t)gridDim.x * 256) {
+    const uint32_t m = better[g] & before;
+    if (m == 0) continue;   // none: the range as it is
+    const float p = shrink_factor(31 - __clz(m), c.grid);
+    mn[g] = __float2bfloat16_rn(__bfloat162float(mn[g]) * p);
+    mx[g] = __float2bfloat16_rn(__bfloat162float(mx[g]) * p);
+  }
+}
+
 // ctl[0] <- number of candidates the reference's loop evaluates before it breaks
 __global__ void stop_step_kernel(int* ctl, int steps, int patience) {
   int stale = 0, run = steps;
@@ -575,24 +602,25 @@ constexpr int kTableBlocksPerSM = 3;
 
 template <int KIND, bool SYM>
 static int launch_group(const void* W, int64_t N, int64_t K, int64_t ldw, int g, const Cfg& c, const __nv_bfloat16* table,
-                        int* ctl, int pass, void* mn, void* mx, cudaStream_t st) {
+                        int* ctl, int pass, void* mn, void* mx, uint32_t* better, cudaStream_t st) {
   const int chunks = g >> 3, r = chunks >= 4 ? 4 : chunks;
   const int64_t slots = N * (K / g) * (chunks / r);
   const int grid = grid_for((slots + 255) / 256, kTableBlocksPerSM);
   auto kern = r == 4 ? mse_group_bf16_kernel<KIND, SYM, 4> : r == 2 ? mse_group_bf16_kernel<KIND, SYM, 2> : mse_group_bf16_kernel<KIND, SYM, 1>;
   B200Q_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTableBytes));
-  kern<<<grid, 256, kTableBytes, st>>>(W, N, K, ldw, g, c, table, ctl, pass, mn, mx);
+  kern<<<grid, 256, kTableBytes, st>>>(W, N, K, ldw, g, c, table, ctl, pass, mn, mx, better);
   return B200Q_OK;
 }
 template <int KIND, bool SYM>
 static int launch_tile(const void* W, int64_t N, int64_t K, int64_t ldw, int bh, int bw, const Cfg& c,
-                       const __nv_bfloat16* table, int* ctl, int pass, void* mn, void* mx, cudaStream_t st) {
+                       const __nv_bfloat16* table, int* ctl, int pass, void* mn, void* mx, uint32_t* better,
+                       cudaStream_t st) {
   const size_t smem = kTableBytes + (size_t)bh * bw * 2;
   const int64_t groups = ((N + bh - 1) / bh) * ((K + bw - 1) / bw);
   const int per_sm = (int)(220 * 1024 / (smem + 1024));
   auto kern = mse_tile_bf16_kernel<KIND, SYM>;
   B200Q_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kern<<<grid_for(groups, per_sm < 1 ? 1 : per_sm), 256, smem, st>>>(W, N, K, ldw, bh, bw, c, table, ctl, pass, mn, mx);
+  kern<<<grid_for(groups, per_sm < 1 ? 1 : per_sm), 256, smem, st>>>(W, N, K, ldw, bh, bw, c, table, ctl, pass, mn, mx, better);
   return B200Q_OK;
 }
 
@@ -614,19 +642,31 @@ static size_t mse_flag_bytes(int steps) {
   return (sizeof(int) * (size_t)(steps + 1 > 1 ? steps + 1 : 1) + 255) / 256 * 256;
 }
 
-size_t b200q_observe_mse_workspace_bytes(int64_t, int64_t, const b200q_qargs* qa, int steps) {
+// groups that a packed search notes its better candidates for
+static int64_t mse_groups(int64_t N, int64_t K, const b200q_qargs* qa) {
+  if (N <= 0 || K <= 0 || !qa) return 0;
+  switch (qa->strategy) {
+    case B200Q_GROUP: case B200Q_TENSOR_GROUP: return qa->group_size > 0 ? N * ((K + qa->group_size - 1) / qa->group_size) : 0;
+    case B200Q_CHANNEL: return N;
+    case B200Q_BLOCK:
+      return qa->block_h > 0 && qa->block_w > 0 ? ((N + qa->block_h - 1) / qa->block_h) * ((K + qa->block_w - 1) / qa->block_w) : 0;
+    default: return 0;
+  }
+}
+
+size_t b200q_observe_mse_workspace_bytes(int64_t N, int64_t K, const b200q_qargs* qa, int steps) {
   const size_t flags = mse_flag_bytes(steps);
   if (qa && qa->strategy == B200Q_TENSOR)   // search state and per-CTA partials
     return flags + sizeof(float) * (size_t)(b200q::mse::kSpanState + 2 * 4 * b200q::kNumSMs);
-  return flags + b200q::mse::kTableBytes + 256;   // (the table starts on a 16-byte boundary of whatever it is given)
+  return flags + b200q::mse::kTableBytes + 256 + (steps <= 32 ? sizeof(uint32_t) * (size_t)mse_groups(N, K, qa) : 0);   // (the table starts on a 16-byte boundary of whatever it is given)
 }
 
 }  // extern "C"
 
-// `table`: 64 KiB for the powers of bf16 errors, 16-byte aligned
+// `table`: 64 KiB for the powers of bf16 errors, 16-byte aligned; `notes`: 4 bytes a group (null: the search runs twice)
 static int observe_mse(const void* W, int wdtype, int64_t N, int64_t K, int64_t ldw, const b200q_qargs* qa,
                        double maxshrink, int patience, double grid, float norm, float expand, void* mn_out,
-                       void* mx_out, void* scratch, void* table_mem, void* stream) {
+                       void* mx_out, void* scratch, void* table_mem, void* notes, void* stream) {
   using namespace b200q::mse;
   if (!W || !qa || !mn_out || !mx_out || !scratch || N <= 0 || K <= 0 || ldw < K) return B200Q_ERR_ARG;
   if (wdtype != B200Q_BF16 && wdtype != B200Q_F32) return B200Q_ERR_UNSUPPORTED;
@@ -660,6 +700,7 @@ static int observe_mse(const void* W, int wdtype, int64_t N, int64_t K, int64_t 
                       (((uintptr_t)W) & 15) == 0 && (!blk || (qa->block_w > 0 && qa->block_w % 8 == 0)) &&
                       (qr.kind != kInt || qa->num_bits == 4 || qa->num_bits == 8);
   __nv_bfloat16* table = (__nv_bfloat16*)table_mem;
+  uint32_t* better = packed && (qa->symmetric || qr.kind == kInt) && c.steps <= 32 ? (uint32_t*)notes : nullptr;
   if (packed) make_table_kernel<<<kTable / 256, 256, 0, st>>>(table, c.norm, ctl, c.steps + 1);
   else clear_ctl_kernel<<<1, 128, 0, st>>>(ctl, c.steps + 1);
   B200Q_LAUNCH_CHECK();
@@ -676,7 +717,7 @@ static int observe_mse(const void* W, int wdtype, int64_t N, int64_t K, int64_t 
       int g = qa->group_size;
       if (!(g >= 8 && g <= 256 && (g & (g - 1)) == 0 && K % g == 0)) return B200Q_ERR_UNSUPPORTED;
       int grid_sz = grid_for((N * (K >> 3) + 255) / 256, 4);
-      if (packed && (qa->symmetric || qr.kind == kInt)) B200Q_MSE_PICK(launch_group, W, N, K, ldw, g, c, table, ctl, pass, mn_out, mx_out, st);
+      if (packed && (qa->symmetric || qr.kind == kInt)) B200Q_MSE_PICK(launch_group, W, N, K, ldw, g, c, table, ctl, pass, mn_out, mx_out, better, st);
       else if (wdtype == B200Q_BF16) mse_group_kernel<B200Q_BF16><<<grid_sz, 256, 0, st>>>(W, N, K, ldw, g, c, ctl, pass, mn_out, mx_out);
       else mse_group_kernel<B200Q_F32><<<grid_sz, 256, 0, st>>>(W, N, K, ldw, g, c, ctl, pass, mn_out, mx_out);
     } else if (qa->strategy == B200Q_CHANNEL || qa->strategy == B200Q_BLOCK) {
@@ -686,7 +727,7 @@ static int observe_mse(const void* W, int wdtype, int64_t N, int64_t K, int64_t 
       if (bh * bw > (int64_t)50 * 1024) return B200Q_ERR_UNSUPPORTED;   // group does not fit in shared memory
       const int64_t groups = ((N + bh - 1) / bh) * ((K + bw - 1) / bw);
       int grid_sz = grid_for(groups, smem > 100 * 1024 ? 1 : 2);
-      if (packed && (qa->symmetric || qr.kind == kInt)) B200Q_MSE_PICK(launch_tile, W, N, K, ldw, (int)bh, (int)bw, c, table, ctl, pass, mn_out, mx_out, st);
+      if (packed && (qa->symmetric || qr.kind == kInt)) B200Q_MSE_PICK(launch_tile, W, N, K, ldw, (int)bh, (int)bw, c, table, ctl, pass, mn_out, mx_out, better, st);
       else if (wdtype == B200Q_BF16) {
         B200Q_TRY(cudaFuncSetAttribute(mse_tile_kernel<B200Q_BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         mse_tile_kernel<B200Q_BF16><<<grid_sz, 256, smem, st>>>(W, N, K, ldw, (int)bh, (int)bw, c, ctl, pass, mn_out, mx_out);
@@ -723,6 +764,13 @@ static int observe_mse(const void* W, int wdtype, int64_t N, int64_t K, int64_t 
       return B200Q_ERR_UNSUPPORTED;
     }
     B200Q_LAUNCH_CHECK();
+    if (better) {
+      const int64_t groups = mse_groups(N, K, qa);
+      pick_kernel<<<grid_for((groups + 255) / 256, 4), 256, 0, st>>>(ctl, better, groups, c, (__nv_bfloat16*)mn_out,
+                                                                     (__nv_bfloat16*)mx_out);
+      B200Q_LAUNCH_CHECK();
+      break;
+    }
     if (pass == 0) {
       stop_step_kernel<<<1, 1, 0, st>>>(ctl, c.steps, c.patience);
       B200Q_LAUNCH_CHECK();
@@ -740,7 +788,7 @@ extern "C" int b200q_observe_mse(const void* W, int wdtype, int64_t N, int64_t K
   if (steps < 0) return B200Q_ERR_ARG;
   const uintptr_t table = ((uintptr_t)scratch + mse_flag_bytes(steps) + 15) & ~(uintptr_t)15;
   return observe_mse(W, wdtype, N, K, ldw, qa, maxshrink, patience, grid, norm, expand, mn_out, mx_out, scratch,
-                     (void*)table, stream);
+                     (void*)table, (void*)(table + b200q::mse::kTableBytes), stream);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -811,6 +859,6 @@ extern "C" int b200q_observe_mse_noalloc(const void* W, int wdtype, int64_t N, i
   if (rc != B200Q_OK) return rc;
   // the search clears the flags it uses before its first pass, so the contents left by the
   // previous call do not matter
-  return observe_mse(W, wdtype, N, K, ldw, qa, maxshrink, patience, grid, norm, expand, mn_out, mx_out, ctl, table,
+  return observe_mse(W, wdtype, N, K, ldw, qa, maxshrink, patience, grid, norm, expand, mn_out, mx_out, ctl, table, nullptr,
                      stream);
 }

@@ -957,6 +957,12 @@ def _input_key(inp: torch.Tensor):
     return inp.data_ptr(), inp.shape, inp.dtype
 
 
+# Batches of this many tokens go to the Hessian as they are: the update is bound by its MMAs from about there on, and the
+# copy into the staging buffer costs what the larger calls save (4096 tokens: K = 4096 59 us against 10 + 53, K = 2048 21
+# against 5 + 17, K = 1024 13 against 3 + 9; 2048 tokens: K = 4096 35 against 5 + 13 to 26).
+_DIRECT_TOKENS = 4096
+
+
 class _HessianGroup:
     """One Hessian shared by the modules that see the same input.
 
@@ -1007,8 +1013,7 @@ class _HessianGroup:
             return  # another member already added this batch
         x, added = gptq._tokens_2d(inp, self.device)
         t = x.shape[0]
-        if self.stage_tokens <= 0 or t >= self.stage_tokens:
-            self.flush()
+        if t >= min(self.stage_tokens, _DIRECT_TOKENS):
             self._syrk(x)
         else:
             if self._stage is None:
