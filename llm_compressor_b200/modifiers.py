@@ -966,10 +966,9 @@ _DIRECT_TOKENS = 4096
 class _HessianGroup:
     """One Hessian shared by the modules that see the same input.
 
-    Small calibration batches are gathered in a bf16 staging buffer and added with one kernel
-    call per ``stage_tokens`` tokens: the symmetric rank-k update re-reads and re-writes the lower
-    triangle of H on every call and fills the machine in whole waves of 256x256 tiles, so a call
-    over 2048 tokens runs at about half the rate of a call over 32768 (K = 4096)."""
+    Small calibration batches (below ``stage_tokens`` and ``_DIRECT_TOKENS``) are gathered in a bf16
+    staging buffer and added with one kernel call per ``stage_tokens`` tokens: the symmetric rank-k
+    update re-reads and re-writes the lower triangle of H on every call."""
 
     def __init__(self, module, offload=False, stage_tokens: int = 0):
         self.members = [module]
@@ -1013,7 +1012,8 @@ class _HessianGroup:
             return  # another member already added this batch
         x, added = gptq._tokens_2d(inp, self.device)
         t = x.shape[0]
-        if t >= min(self.stage_tokens, _DIRECT_TOKENS):
+        # (a sum that lives on the host between calls is worth fewer calls)
+        if t >= (self.stage_tokens if self.offload else min(self.stage_tokens, _DIRECT_TOKENS)):
             self._syrk(x)
         else:
             if self._stage is None:

@@ -14,6 +14,12 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 
 
+@pytest.fixture(autouse=True, scope="module")
+def _leave_the_allocator_as_it_was():
+    yield
+    torch.cuda.empty_cache()
+
+
 def _spec(scheme):
     if scheme == "FP8_BLOCK":
         return oracle.preset("FP8_DYNAMIC", strategy="block", block_structure=[128, 128])
