@@ -299,7 +299,7 @@ int b200q_gptq_factor(float* H, int64_t K, int64_t ldh, void* workspace, int* st
                       void* stream);
 
 /* The float32-accurate tensor-core GEMM that the factorisation and the sweep use for their
- * rank-128 updates (tcgen05 kind::tf32, three MMAs per product on hi/lo splits of the operands):
+ * updates (tcgen05 kind::tf32, three MMAs per product on hi/lo splits of the operands):
  *   C[M,N] = beta*C + alpha * A[M,Kd] * (trans_b ? B[N,Kd]^T : B[Kd,N]),   Kd <= 128.
  * Stands in for the torch.matmul calls of gptq_quantize.py:236,244 and the cuSOLVER updates
  * behind :153-155.  lower_tiles != 0 restricts the update to 128x128 tiles with column block <=
@@ -310,8 +310,8 @@ int b200q_gemm_tf32x3(int trans_b, const float* A, int64_t lda, const float* B, 
                       int64_t ldc, int64_t M, int64_t N, int64_t Kd, float alpha, float beta,
                       int lower_tiles, void* workspace, int* status, void* stream);
 
-/* Blockwise column sweep (gptq_quantize.py:166-245): for each block of `blocksize` columns,
- * column by column: q = fake_quantize(w); loss += (w-q)^2/d^2/2; err = (w-q)/d;
+/* Blockwise column sweep (gptq_quantize.py:166-245); `blocksize` (at most 128) only orders float32
+ * operations in the reference and does not decide the blocks here.  Column by column: q = fake_quantize(w); loss += (w-q)^2/d^2/2; err = (w-q)/d;
  * W_block[:, i:] -= err x U[i, i:]; then W[:, after] -= Err @ U[block, after].
  * Wf fp32 [N,K] in/out (ends as the fake-quantised weight); U from b200q_gptq_factor
  * (NULL = identity: round to nearest); scale [N,G] / [N,1] / [1] of dtype sdtype; zp may be

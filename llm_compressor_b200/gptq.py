@@ -158,7 +158,7 @@ def _factor_prologue(hessian: torch.Tensor, percdamp: float, actorder):
 
 def factor_hessians_batched(hessians, percdamp: float = 0.01, actorder=None):
     """``factor_hessian(..., defer=True)`` for a list of small Hessians of one size, with all the
-    factorisations in one launch (one thread block per matrix).  The matrices are consumed.
+    factorisations in the same launches.  The matrices are consumed.
     Returns the deferred factors; ``resolve_factors`` reads all their status words at once."""
     hessians, perms, diags = ops.gptq_prologue_batched(list(hessians), percdamp, bool(actorder))
     status = ops.gptq_factor_batched(hessians)

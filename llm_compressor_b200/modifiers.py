@@ -524,10 +524,10 @@ class GPTQModifier(QuantizationMixin):
     ``share_hessians=False`` to keep one per module like the reference.  The solves of different
     Hessians run concurrently on up to ``parallel_streams`` CUDA streams (1: one after another
     on the current stream, like the reference).  Calibration batches smaller than
-    ``hessian_stage_tokens`` tokens are gathered and added to the Hessian together (0: one kernel
+    ``hessian_stage_tokens`` (and than ``_DIRECT_TOKENS``) tokens are gathered and added to the Hessian together (0: one kernel
     call per batch).  When an epoch holds ``batch_small_hessians`` or more Hessians of one width of
     at most ``small_hessian_columns`` columns (the experts of a mixture-of-experts layer), their
-    factorisations and sweeps run as batched launches, one thread block per problem, instead of
+    factorisations and sweeps run as batched launches that serve all of them, instead of
     dozens of launches per module (0 switches this off).
     """
 
@@ -846,7 +846,7 @@ class GPTQModifier(QuantizationMixin):
     def _compress_small_jobs(self, jobs):
         """Many Hessians of few columns: the same steps as ``_compress_group`` for every job, but the
         factorisations of one width and the sweeps of one weight shape and scheme are gathered
-        into batched launches (one thread block per problem) on the current stream."""
+        into batched launches on the current stream."""
         t0 = time.perf_counter()
         self._trace("job_start", jobs[0][0])
         requests = []   # (H, actorder, holder): the holder receives the factor once it exists
