@@ -981,12 +981,13 @@ __global__ void __launch_bounds__(256) rtn_channel_kernel(
 // The chain of the element-wise formulation - scale and round to bf16, min / max of the group or row, qparams,
 // fake-quantise, divide by the scale in float32 and round - in one pass over the weight: 4 B of traffic an element
 // where the separate passes moved 30 (231 us for 4096 x 4096).
-struct ColScale { float s[8], rs[8]; };
+struct ColScale { float s[8], rs[8]; bool plain; };   // plain: all of them within 2^-24 .. 2^24
 __device__ __forceinline__ void load_col_scale(const float* __restrict__ col, int64_t c, ColScale& k) {
   const float4 a = __ldg(reinterpret_cast<const float4*>(col + c)), b = __ldg(reinterpret_cast<const float4*>(col + c) + 1);
   k.s[0] = a.x; k.s[1] = a.y; k.s[2] = a.z; k.s[3] = a.w; k.s[4] = b.x; k.s[5] = b.y; k.s[6] = b.z; k.s[7] = b.w;
+  k.plain = true;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) k.rs[i] = __frcp_rn(k.s[i]);
+  for (int i = 0; i < 8; ++i) { k.rs[i] = __frcp_rn(k.s[i]); k.plain = k.plain && k.s[i] >= 0x1p-24f && k.s[i] <= 0x1p24f; }
 }
 __device__ __forceinline__ uint4 scale_chunk(const uint4& raw, const ColScale& k) {
   const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
@@ -996,12 +997,12 @@ __device__ __forceinline__ uint4 scale_chunk(const uint4& raw, const ColScale& k
     o[p] = stream::cvt_bf16x2(__uint_as_float(w[p] & 0xFFFF0000u) * k.s[2 * p + 1], __uint_as_float(w[p] << 16) * k.s[2 * p]);
   return make_uint4(o[0], o[1], o[2], o[3]);
 }
-// bf16(fq / s): the product with 1 / s is a few float32 ulps off the quotient, so it rounds to the same bf16 value
-// unless it lies within 16 ulps of a midpoint (or leaves the normal range): then the division is done
-__device__ __forceinline__ float unscale(float fq, float s, float rs) {
-  const float q = fq * rs, a = fabsf(q);
-  if (((__float_as_uint(q) & 0xFFFFu) - 0x7FF0u) > 0x20u && ((a < 1e30f && a > 1e-30f) || fq == 0.0f) && a == a) return q;
-  return __fdiv_rn(fq, s);
+// bf16(fq / s) of a chunk by the division itself (arguments by value and out of line: rarely needed)
+__device__ __noinline__ uint4 unscale_exact(uint4 fq, float4 s0, float4 s1) {
+  auto one = [](uint32_t w, float lo, float hi) {
+    return stream::cvt_bf16x2(__fdiv_rn(__uint_as_float(w & 0xFFFF0000u), hi), __fdiv_rn(__uint_as_float(w << 16), lo));
+  };
+  return make_uint4(one(fq.x, s0.x, s0.y), one(fq.y, s0.z, s0.w), one(fq.z, s1.x, s1.y), one(fq.w, s1.z, s1.w));
 }
 __device__ __forceinline__ uint32_t rint_bf16x2(uint32_t v, bool four_bit) {
   if (four_bit) {   // integers are 1 apart in [128, 256)
@@ -1044,12 +1045,19 @@ __device__ __forceinline__ uint4 fake_quant_unscale(const uint4& ws, const strea
       fq[p] = *reinterpret_cast<uint32_t*>(&d);
     }
   }
-  uint32_t o[4];
+  // The product with 1 / s is a few float32 ulps off the quotient, so it rounds to the same bf16 value unless it lies
+  // within 16 ulps of a midpoint, which one test settles for the chunk.  The scales' ranges keep every product that is
+  // not zero a normal number.
+  uint32_t o[4], near = 0xFFFFFFFFu;
 #pragma unroll
-  for (int p = 0; p < 4; ++p)
-    o[p] = stream::cvt_bf16x2(unscale(__uint_as_float(fq[p] & 0xFFFF0000u), k.s[2 * p + 1], k.rs[2 * p + 1]),
-                              unscale(__uint_as_float(fq[p] << 16), k.s[2 * p], k.rs[2 * p]));
-  return make_uint4(o[0], o[1], o[2], o[3]);
+  for (int p = 0; p < 4; ++p) {
+    const float lo = __uint_as_float(fq[p] << 16) * k.rs[2 * p], hi = __uint_as_float(fq[p] & 0xFFFF0000u) * k.rs[2 * p + 1];
+    near = min(near, min((__float_as_uint(lo) & 0xFFFFu) - 0x7FF0u, (__float_as_uint(hi) & 0xFFFFu) - 0x7FF0u));
+    o[p] = stream::cvt_bf16x2(hi, lo);
+  }
+  if (near > 0x20u && k.plain && g.se >= 0x1p-60f && g.se <= 0x1p60f) return make_uint4(o[0], o[1], o[2], o[3]);
+  return unscale_exact(make_uint4(fq[0], fq[1], fq[2], fq[3]), make_float4(k.s[0], k.s[1], k.s[2], k.s[3]),
+                       make_float4(k.s[4], k.s[5], k.s[6], k.s[7]));
 }
 
 // GROUP: a thread owns a chunk of 8 columns and walks down the rows, so that its column scales and their reciprocals
@@ -1344,18 +1352,21 @@ int b200q_scaled_fake_quantize(const void* W, int wdtype, int64_t N, int64_t K, 
     const int g = qa->group_size;
     if (!(pow2(g) && g >= 8 && g <= 256 && K % g == 0)) return B200Q_ERR_UNSUPPORTED;
     const int64_t gx = (cpr + 31) / 32;
-    // enough CTAs to fill the machine, rows enough per CTA to earn the column scales' reciprocals
-    int64_t gy = (6 * kNumSMs + gx - 1) / gx;
+    // as many CTAs as are resident at once: each walks down its share of the rows, which earns the column scales'
+    // reciprocals (six per SM where four fit: 33 us for 4096 x 4096)
+    int64_t gy = resident_grid<scaled_group_kernel>(256, 0, (int64_t)1 << 40) / gx;
+    if (gy < 1) gy = 1;
     if (gy > (N + 7) / 8) gy = (N + 7) / 8;
     if (gx > 2147483647LL || gy > 65535) return B200Q_ERR_UNSUPPORTED;
     scaled_group_kernel<<<dim3((unsigned)gx, (unsigned)gy), 256, 0, st>>>(W, N, K, ldw, g >> 3, col_scale, qc, qr, four, out);
   } else if (qa->strategy == B200Q_CHANNEL) {
     if (cpr > 8 * 256) return B200Q_ERR_UNSUPPORTED;
-    const int grid = grid_for(N, 6);
-    if (cpr <= 256) scaled_channel_kernel<1><<<grid, 256, 0, st>>>(W, N, K, ldw, col_scale, qc, qr, four, out);
-    else if (cpr <= 512) scaled_channel_kernel<2><<<grid, 256, 0, st>>>(W, N, K, ldw, col_scale, qc, qr, four, out);
-    else if (cpr <= 1024) scaled_channel_kernel<4><<<grid, 256, 0, st>>>(W, N, K, ldw, col_scale, qc, qr, four, out);
-    else scaled_channel_kernel<8><<<grid, 256, 0, st>>>(W, N, K, ldw, col_scale, qc, qr, four, out);
+#define B200Q_SC(R) scaled_channel_kernel<R><<<resident_grid<scaled_channel_kernel<R>>(256, 0, N), 256, 0, st>>>(W, N, K, ldw, col_scale, qc, qr, four, out)
+    if (cpr <= 256) B200Q_SC(1);
+    else if (cpr <= 512) B200Q_SC(2);
+    else if (cpr <= 1024) B200Q_SC(4);
+    else B200Q_SC(8);
+#undef B200Q_SC
   } else {
     return B200Q_ERR_UNSUPPORTED;
   }
