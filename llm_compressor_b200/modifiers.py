@@ -743,9 +743,16 @@ class GPTQModifier(QuantizationMixin):
         if jobs:
             run_concurrent([lambda mods=mods: self._compress_group(mods) for mods in jobs], device,
                            max_streams=self.parallel_streams)
-            # the jobs end in an order that varies from run to run: the losses are kept in that of the jobs' lengths (a
-            # chain of columns for the factor and one for each sweep)
-            for mods in sorted(jobs, key=lambda mods: mods[0].weight.shape[1] * (1 + len(mods))):
+            # The jobs end in an order that varies from run to run; the losses are kept in the one they mostly end in: by
+            # the columns of their chains (one for the factor and one for each sweep), or, where Hessians are so narrow
+            # that queueing the launches takes longer, by the modules.
+            narrow = min(mods[0].weight.shape[1] for mods in jobs) < 1024
+
+            def length(mods):
+                width = mods[0].weight.shape[1]
+                return (len(mods) if narrow else width * (1 + len(mods)), width)
+
+            for mods in sorted(jobs, key=length):
                 for m in mods:
                     name = self._module_names.get(m, type(m).__name__)
                     if name in self.losses:
