@@ -63,9 +63,12 @@ __device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], 
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
-// acc[j] += A[16 x depth] B_j[8 x depth]^T, B_j = rows 8 j .. 8 j + 7 of B.  Lane (g, t) = (lane / 4, lane % 4) ends
+// acc[j] = A[16 x depth] B_j[8 x depth]^T, B_j = rows 8 j .. 8 j + 7 of B.  Lane (g, t) = (lane / 4, lane % 4) ends
 // with rows g, g + 8 and columns 2 t, 2 t + 1.  A: contraction contiguous, row stride lda; B: element (n, k) at
 // n * sn + k * sk.
+// An MMA's addition to its accumulator cuts off instead of rounding, so the large products run over 16 terms at most and
+// the runs are added by float32 additions (all 128 in one accumulator: relative error of the factor 3.5e-7 at K = 256
+// and 4.4e-7 at 512 against 1.9e-7 and 2.1e-7).
 template <int NT, int UNROLL>
 __device__ __forceinline__ void mma_block(const float* A, int lda, const float* B, int sn, int sk, int depth, int lane,
                                           float (&acc)[NT][4]) {
@@ -73,7 +76,7 @@ __device__ __forceinline__ void mma_block(const float* A, int lda, const float* 
   const float* b0 = B + (lane >> 2) * sn + (lane & 3) * sk;
   // the three products accumulate apart: a warp issues in order, and an MMA whose accumulator the one before it
   // still has stalls everything behind it for some 35 cycles
-  float part[2][NT][4] = {};
+  float part[2][NT][4] = {}, run[NT][4] = {}, sum[NT][4] = {};
 #pragma unroll UNROLL
   for (int k = 0; k < depth; k += 8) {
     const float x[4] = {a0[k], a0[k + 8 * lda], a0[k + 4], a0[k + 8 * lda + 4]};
@@ -85,16 +88,25 @@ __device__ __forceinline__ void mma_block(const float* A, int lda, const float* 
 #pragma unroll
     for (int j = 0; j < NT; ++j) split_frag(y[j], bh[j], bl[j]);
 #pragma unroll
-    for (int j = 0; j < NT; ++j) mma_tf32(acc[j], ah, bh[j]);
+    for (int j = 0; j < NT; ++j) mma_tf32(run[j], ah, bh[j]);
 #pragma unroll
     for (int j = 0; j < NT; ++j) mma_tf32(part[0][j], ah, bl[j]);
 #pragma unroll
     for (int j = 0; j < NT; ++j) mma_tf32(part[1][j], al, bh[j]);
+    if (depth > 16 && (k & 8)) {
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { sum[j][e] += run[j][e]; run[j][e] = 0.0f; }
+    }
   }
 #pragma unroll
   for (int j = 0; j < NT; ++j)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) acc[j][e] += part[0][j][e] + part[1][j][e];
+    for (int e = 0; e < 4; ++e) {
+      acc[j][e] = run[j][e] + (part[0][j][e] + part[1][j][e]);
+      if (depth > 16) acc[j][e] += sum[j][e];
+    }
 }
 
 // ---------------------------------------------------------------------------------------
@@ -146,7 +158,7 @@ __global__ void __launch_bounds__(kThreads, 1) chol_diag_kernel(Mat mt, int k0, 
     const int c0 = kb * W16, p0 = c0 - W16;
     if (warp == 0) {
       if (kb > 0) {   // the diagonal block takes the step before
-        float acc[2][4] = {};
+        float acc[2][4];
         float* o = R + (c0 + (lane >> 2)) * LD + c0 + 2 * (lane & 3);
         float2 old[2][2];
 #pragma unroll
@@ -211,7 +223,7 @@ __global__ void __launch_bounds__(kThreads, 1) chol_diag_kernel(Mat mt, int k0, 
           const bool matrix = s >= kb;
           float* rows = R + ((matrix ? 0 : NB) + s * W16) * LD;
           const int cc = c0 + g * 32;
-          float acc[4][4] = {};
+          float acc[4][4];
           float* o = rows + (lane >> 2) * LD + cc + 2 * (lane & 3);
           float2 old[4][2];   // (all of them before the products: loads cannot pass the stores below)
 #pragma unroll
@@ -340,7 +352,7 @@ __global__ void __launch_bounds__(kThreads) panel_kernel(Mat mt, float* P0, int 
   __syncthreads();
   // a warp: 16 vectors x 8 outputs
   const int warp = tid >> 5, lane = tid & 31, j0 = warp * 8;
-  float acc[1][4] = {};
+  float acc[1][4];
   mma_block<1, 4>(V, LD, D + j0 * LD, LD, 1, half + j0 + 8, lane, acc);
   const int v = v0 + (lane >> 2), j = half + j0 + 2 * (lane & 3);
 #pragma unroll
@@ -410,7 +422,7 @@ __global__ void __launch_bounds__(kThreads) square_update_kernel(Mat mt, const f
   chain_go();
   cp_async_wait_all();
   __syncthreads();
-  float acc[1][4] = {};
+  float acc[1][4];
   if (right) mma_block<1, 4>(Ps + tr * LD, LD, Qs + tc * LD, LD, 1, NB, lane, acc);
   else mma_block<1, 4>(Ps + tr * LD, LD, Qs + tc, 1, 40, NB, lane, acc);
 #pragma unroll
@@ -527,6 +539,7 @@ static int factor(float* H, float* const* Hs, int batch, int64_t K, int64_t ldh,
                   cudaStream_t st) {
   using tgemm::Job;
   using tgemm::Operand;
+  const int slice = Hs ? tgemm::kShortestSlice : tgemm::kLongSlice;   // (measured where they are defined)
   int rc;
 #define B200Q_RC(expr) do { rc = (expr); if (rc != B200Q_OK) return rc; } while (0)
   const int64_t lda = round_up(K, 32), rows = round_up(K, NB);
@@ -589,7 +602,7 @@ static int factor(float* H, float* const* Hs, int batch, int64_t K, int64_t ldh,
     };
     Job j;
     j.A = Pan; j.B = D; j.Kd = n; j.N = n; j.batch = batch; j.status = status + 2; j.status_stride = 4;
-    j.out_ld = OB; j.out_batch = pb;
+    j.out_ld = OB; j.out_batch = pb; j.slice = slice;
     if (!last) {
       // the next block's rows of P and its square: all the chain needs
       B200Q_RC(split_panel(K1, K1 + n2, 0, st));
@@ -604,7 +617,7 @@ static int factor(float* H, float* const* Hs, int batch, int64_t K, int64_t ldh,
       Job d;
       d.A = d.B = Q; d.A.row0 = d.B.row0 = (int)K1; d.M = d.N = n2; d.Kd = n; d.set = tgemm::kLower; d.batch = batch;
       d.alpha = -1.0f; d.beta = 1.0f; d.C = mt.A + K1 * (lda + 1); d.c_batch = mt.batch; d.ldc = lda;
-      d.status = status + 2; d.status_stride = 4;
+      d.status = status + 2; d.status_stride = 4; d.slice = slice;
       B200Q_RC(tgemm::launch(d, st));
     } else {
       bulk = st;
@@ -624,7 +637,7 @@ static int factor(float* H, float* const* Hs, int batch, int64_t K, int64_t ldh,
     u.A = Q; u.B = Q; u.A.row0 = 0; u.M = u.N = (int)K; u.Kd = n; u.set = tgemm::kBulk; u.batch = batch;
     u.row_begin = (int)K1; u.skip0 = (int)K1; u.skip1 = (int)(K1 + n2);
     u.alpha = -1.0f; u.beta = 1.0f; u.C = mt.A; u.c_batch = mt.batch; u.ldc = lda; u.fresh0 = (int)K0; u.fresh1 = (int)K1;
-    u.status = status + 2; u.status_stride = 4; u.max_ctas = r.max_ctas;
+    u.status = status + 2; u.status_stride = 4; u.max_ctas = r.max_ctas; u.slice = slice;
     B200Q_RC(tgemm::launch(u, bulk));
     if (side) {
       B200Q_TRY(cudaEventRecord(side->done, bulk));

@@ -214,3 +214,47 @@ def test_modifier_takes_the_batched_path_for_many_small_hessians(fail_one):
         assert mismatch(a.weight.data, b.weight.data) <= 1 - CODE_MATCH, name
     for name, loss in mod.losses.items():
         assert loss == pytest.approx(base.losses[name], rel=LOSS_RTOL, abs=1e-9), name
+
+
+def _spd_factor64(K, tokens):
+    """(H as a calibration of so many tokens leaves it, damped; its factor in float64)"""
+    g = torch.Generator(device=DEV).manual_seed(K + tokens)
+    scale = 0.25 + 2.0 * torch.rand(K, generator=g, device=DEV)
+    H = torch.zeros(K, K, device=DEV, dtype=torch.float64)
+    for t in range(0, tokens, 4096):
+        x = (torch.randn(min(4096, tokens - t), K, generator=g, device=DEV) * scale).bfloat16().double()
+        H.addmm_(x.t(), x, alpha=2.0)
+    H = H.float()
+    H.diagonal().add_(0.01 * H.diagonal().mean())
+    L = torch.linalg.cholesky(H.double().flip(0, 1))
+    return H, torch.linalg.solve_triangular(L, torch.eye(K, device=DEV, dtype=torch.float64), upper=False).flip(0, 1)
+
+
+# `limit`: the same error of an elimination by float32 multiply-adds, one thread block a problem (relative, 2-norm)
+@pytest.mark.parametrize("K,tokens,limit", [(256, 600, 2.4e-7), (520, 1500, 1.9e-7), (768, 4096, 1.5e-7),
+                                            (1160, 6933, 1.4e-7), (2048, 8192, 1.7e-7)])
+def test_batched_factor_is_as_accurate_as_float32_multiply_adds(K, tokens, limit):
+    H, ref = _spd_factor64(K, tokens)
+    Hs = [H.clone() for _ in range(3)]
+    ops.gptq_factor_batched(Hs)
+    for U in Hs:
+        assert float((U.double() - ref).norm() / ref.norm()) <= limit
+
+
+# the last column after all the corrections: the earlier rows of U times 2^20 keep their errors out of the loss, every
+# code is zero (a huge scale), so the loss is half the square of that column's error.  `limit` as above, relative to the
+# column's root mean square
+@pytest.mark.parametrize("N,K,tokens,limit", [(1001, 520, 1500, 2.8e-7), (6000, 520, 1500, 3.2e-7),
+                                              (1001, 2048, 8192, 4.0e-7)])
+def test_batched_sweep_is_as_accurate_as_float32_multiply_adds(N, K, tokens, limit):
+    _, ref = _spd_factor64(K, tokens)
+    U = ref.float().contiguous()
+    U[:-1] *= 2.0 ** 20
+    w = (torch.randn(N, K, generator=torch.Generator(device=DEV).manual_seed(N), device=DEV) * 0.02).bfloat16()
+    last = torch.linalg.solve_triangular(U.double(), w.double(), upper=True, left=False)[:, -1].abs()
+    args = args_from(SCHEMES["W8_CHANNEL"])
+    scale = torch.full((N, 1), 1e4, device=DEV).bfloat16()
+    losses = ops.gptq_sweep_batched([w.float() for _ in range(3)], [U] * 3, [scale] * 3, None, args)
+    for row in losses:
+        error = (2.0 * row.double()).sqrt() - last
+        assert float(error.pow(2).mean().sqrt() / last.pow(2).mean().sqrt()) <= limit
