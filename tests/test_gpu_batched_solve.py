@@ -258,3 +258,17 @@ def test_batched_sweep_is_as_accurate_as_float32_multiply_adds(N, K, tokens, lim
     for row in losses:
         error = (2.0 * row.double()).sqrt() - last
         assert float(error.pow(2).mean().sqrt() / last.pow(2).mean().sqrt()) <= limit
+
+
+# every code zero: the errors of a row are W U^-1, their sum of squares the loss.  `limit`: the same error (relative, root
+# mean square over the rows) with sums of 128 terms
+@pytest.mark.parametrize("N,K,tokens,limit", [(1001, 520, 1500, 2.3e-7), (1001, 1160, 6933, 1.6e-7), (6000, 1160, 6933, 1.6e-7)])
+def test_sweep_losses_are_summed_in_short_runs(N, K, tokens, limit):
+    _, ref = _spd_factor64(K, tokens)
+    U = ref.float().contiguous()
+    w = (torch.randn(N, K, generator=torch.Generator(device=DEV).manual_seed(N), device=DEV) * 0.02).bfloat16()
+    errors = torch.linalg.solve_triangular(U.double(), w.double(), upper=True, left=False)
+    total = 0.5 * (errors * errors).sum(1)
+    scale = torch.full((N, 1), 1e4, device=DEV).bfloat16()
+    losses = ops.gptq_sweep(w.float(), U, scale, None, args_from(SCHEMES["W8_CHANNEL"]))
+    assert float(((losses.double() - total) / total).pow(2).mean().sqrt()) <= limit
