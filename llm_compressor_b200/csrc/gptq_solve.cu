@@ -511,6 +511,6 @@ extern "C" int b200q_gemm_tf32x3(int trans_b, const float* A, int64_t lda, const
   j.A = tgemm::Operand{a_hi, a_lo, kp, (M + 127) / 128 * 128, 0, 0};
   j.B = tgemm::Operand{b_hi, b_lo, kp, (N + 127) / 128 * 128, 0, 0};
   j.M = (int)M; j.N = (int)N; j.Kd = (int)Kd; j.alpha = alpha; j.beta = beta; j.C = C; j.ldc = ldc; j.status = status;
-  j.set = lower_tiles ? tgemm::kLower : tgemm::kAll;
+  j.set = lower_tiles ? tgemm::kLowerBlocks : tgemm::kAll;
   return tgemm::launch(j, st);
 }

@@ -175,7 +175,7 @@ __host__ __device__ __forceinline__ int tile_row(const Job& j, int tm, int rows)
 // column tiles of row tile tm (they are contiguous from column 0)
 __host__ __device__ __forceinline__ int col_tiles(const Job& j, int tm, int rows, int tn_log2) {
   int lim = j.N;
-  if (j.set == kLower || j.set == kBulk) {
+  if (j.set == kLower || j.set == kBulk || j.set == kLowerBlocks) {
     const int r = tile_row(j, tm, rows);
     const int diag = (j.set == kBulk && r < j.skip1) ? j.skip0 : r + rows;
     lim = diag < lim ? diag : lim;
@@ -621,6 +621,7 @@ static int count_rows(const Job& j, int rows) {
   return j.skip0 / rows + (j.M > j.skip1 ? (j.M - j.skip1 + rows - 1) / rows : 0);
 }
 static bool rows_fit(const Job& j, int rows) {
+  if (j.set == kLowerBlocks) return rows <= kTile;
   if (j.set == kPanel) return j.skip0 % rows == 0;
   return j.set != kBulk || j.skip1 <= j.row_begin || (j.skip1 - j.row_begin) % rows == 0;
 }
@@ -670,7 +671,7 @@ static void pick_tiles(Params& p, int ctas, int pairs) {
   const Job& j = p.j;
   const int chunks = (j.Kd + kChunkK - 1) / kChunkK;
   double best_cost = 0.0;
-  for (int w = 6; w <= 8; ++w) {
+  for (int w = 6; w <= (j.set == kLowerBlocks ? 7 : 8); ++w) {
     const int64_t tiles = count_tiles(j, kTile, w) * j.batch;
     const double cost = (double)((tiles + ctas - 1) / ctas) * chunks * chunk[w - 6] + 20.0 * (1 << w);
     if (w == 6 || cost < best_cost) { p.tn_log2 = w; p.tm_rows = kTile; best_cost = cost; }

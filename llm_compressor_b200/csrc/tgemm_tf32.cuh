@@ -39,12 +39,13 @@ __device__ __forceinline__ float tf32_rn(float x) {
   return __uint_as_float(b);
 }
 
-// Which 128-row x TN-column tiles of the output a launch computes:
+// Which tiles of the output a launch computes:
 //   kAll    every tile
 //   kLower  tiles that hold something on or below the diagonal
 //   kPanel  all columns of every row outside [skip0, skip1)
 //   kBulk   rows from row_begin on: columns below skip0 for rows below skip1, else everything on or below the diagonal
-enum TileSet { kAll = 0, kLower = 1, kPanel = 2, kBulk = 3 };
+//   kLowerBlocks   as kLower, and nothing outside the 128 x 128 blocks on or below the diagonal: tiles no larger than these
+enum TileSet { kAll = 0, kLower = 1, kPanel = 2, kBulk = 3, kLowerBlocks = 4 };
 
 struct Job {
   Operand A, B;

@@ -372,6 +372,20 @@ def test_gemm_tf32x3_lower_tiles_only():
                 assert float(blk.abs().max()) == 0.0
 
 
+# sizes at which wider tiles would be the quicker choice: pairs of 256 x 256, 128 x 256, and a rest of a block
+@pytest.mark.parametrize("M,N", [(4096, 4096), (2560, 2560), (4000, 3000), (1300, 2100)])
+def test_gemm_tf32x3_lower_tiles_leaves_the_other_blocks_alone(M, N):
+    g = torch.Generator(device=DEV).manual_seed(M)
+    a, b = torch.randn(M, 128, generator=g, device=DEV), torch.randn(N, 128, generator=g, device=DEV)
+    c0 = torch.randn(M, N, generator=g, device=DEV)
+    c = c0.clone()
+    ops.gemm_tf32x3(a, b, c, True, alpha=1.0, beta=1.0, lower_tiles=True)
+    lower = (torch.arange(N, device=DEV)[None, :] // 128) <= (torch.arange(M, device=DEV)[:, None] // 128)
+    assert torch.equal(c[~lower], c0[~lower])
+    ref = c0.double() + a.double() @ b.double().t()
+    assert float((c.double() - ref)[lower].norm() / ref[lower].norm()) < 3e-6
+
+
 def _solve_fingerprint(K, N, out_path=None):
     """Factor a seeded Hessian and sweep a seeded weight on the GPU; returns (U, Wq) on the CPU."""
     g = torch.Generator(device=DEV).manual_seed(K)
