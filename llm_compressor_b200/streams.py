@@ -2,8 +2,9 @@
 
 The Hessian factorisation and the column sweep of one module are long chains of small,
 dependent kernel launches that leave most of the GPU idle; the chains of different Hessians
-are independent of each other.  Each job gets a host thread (the C library releases the
-interpreter lock during its calls and keeps its caches per thread) and a side stream.
+are independent of each other.  Each job gets a side stream; the jobs are queued by a host thread
+per stream (``run_concurrent``; the C library releases the interpreter lock during its calls and
+keeps its caches per thread) or all by the calling thread (``run_queued``).
 
 Ordering contract: side streams start after everything already queued on the caller's
 current stream and the caller's stream waits for every side stream before this function
@@ -80,7 +81,9 @@ def run_queued(jobs: Sequence[Callable[[], Callable[[], object]]], device) -> li
     """``run_concurrent`` for jobs, a stream each, that queue their work without waiting for the device and return a
     callable that waits for it and ends the job.  The calling thread queues them all (longest first), then ends them:
     with a host thread each, the jobs of a decoder layer spent as long waiting for the interpreter as queueing
-    (hidden 768 / intermediate 2048: 4.9 ms, 3.2 this way; hidden 2048 / intermediate 5632, bound by the device: 6.3)."""
+    (hidden 768 / intermediate 2048: 4.9 ms, 3.2 this way; hidden 2048 / intermediate 5632, bound by the device: 6.3).
+    A job that raises, when it is queued or when it is ended, keeps none of the others from being ended; the first
+    exception is re-raised after that."""
     jobs = list(jobs)
     device = torch.device(device)
     if len(jobs) <= 1 or device.type != "cuda":
@@ -91,17 +94,24 @@ def run_queued(jobs: Sequence[Callable[[], Callable[[], object]]], device) -> li
     main = torch.cuda.current_stream(device)
     ready = torch.cuda.Event()
     ready.record(main)
-    ends = []
+    errors: list = []
+
+    def attempt(stream, call):
+        with torch.cuda.stream(stream):
+            try:
+                return call()
+            except Exception as e:  # noqa: BLE001 - re-raised below
+                errors.append(e)
+                return None
+
     try:
-        for job, stream in zip(jobs, streams):
-            with torch.cuda.stream(stream):
-                stream.wait_event(ready)
-                ends.append(job())
-        results = []
-        for end, stream in zip(ends, streams):
-            with torch.cuda.stream(stream):
-                results.append(end())
-        return results
+        for stream in streams:
+            stream.wait_event(ready)
+        ends = [attempt(stream, job) for job, stream in zip(jobs, streams)]
+        results = [None if end is None else attempt(stream, end) for end, stream in zip(ends, streams)]
     finally:
         for stream in streams:
             main.wait_stream(stream)
+    if errors:
+        raise errors[0]
+    return results

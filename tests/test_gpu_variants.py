@@ -6,7 +6,7 @@ import torch
 
 import oracle
 from helpers import args_from, bits_equal, mismatch, synth_acts, synth_weight
-from llm_compressor_b200 import QuantizationModifier, compress_state_dict, gptq, observers, oneshot, ops
+from llm_compressor_b200 import GPTQModifier, QuantizationModifier, compress_state_dict, gptq, observers, oneshot, ops
 from llm_compressor_b200.awq import scaled_fake_quantize
 from llm_compressor_b200.quant_args import QuantizationArgs, preset_name_to_scheme
 
@@ -251,3 +251,29 @@ def test_grid_search_against_the_oracle(scheme, N, K):
         differ = (got.cpu().float() != ref.float()).float().mean()
         assert float(differ) <= 0.02, float(differ)
         assert float((got.cpu().float() - ref.float()).norm() / ref.float().norm()) < 0.02
+
+
+def test_a_solve_that_raises_leaves_the_others_quantised():
+    parent = torch.nn.Module()
+    for k in range(3):
+        lin = torch.nn.Linear(256, 64, bias=False, device=DEV, dtype=torch.bfloat16)
+        lin.weight.data = synth_weight(64, 256, k).to(DEV)
+        parent.add_module(f"p{k}", lin)
+    mod = GPTQModifier(targets="Linear", scheme="W4A16", actorder=None)
+    mod.on_initialize(parent)
+    mod.on_calibration_start(parent)
+    for k, lin in enumerate(parent.children()):
+        mod.calibrate_module(lin, (synth_acts(2, 512, 256, k).to(DEV),), None)
+    before = [lin.weight.data.clone() for lin in parent.children()]
+
+    class Broken(observers.MemorylessMinMaxObserver):
+        def update_statistics_from_weight(self, weight):
+            raise RuntimeError("no statistics today")
+    parent.p0.weight_observer = Broken("weight", parent.p0.quantization_scheme.weights)
+    with pytest.raises(RuntimeError, match="no statistics today"):
+        mod.on_sequential_epoch_end(parent, list(parent.modules()))
+    assert torch.equal(parent.p0.weight.data, before[0]) and parent.p0.quantization_status != "frozen"
+    for k in (1, 2):
+        lin = getattr(parent, f"p{k}")
+        assert not torch.equal(lin.weight.data, before[k]) and lin.quantization_status == "frozen"
+    assert sorted(mod.losses) == ["p1", "p2"]

@@ -161,3 +161,59 @@ def test_converter_config_merge():
     assert _merge_configs(old, None)["format"] == "int-quantized"
     same = _merge_configs({"format": "float-quantized", "config_groups": {}}, new)
     assert same["format"] == "float-quantized" and list(same["config_groups"]) == ["group_0"]
+
+
+class _FakeStream:
+    def __init__(self):
+        self.waited = []
+
+    def wait_event(self, event):
+        self.waited.append(event)
+
+    def wait_stream(self, stream):
+        self.waited.append(stream)
+
+
+class _FakeEvent:
+    def record(self, stream):
+        pass
+
+
+@pytest.fixture
+def fake_streams(monkeypatch):
+    import contextlib
+
+    from llm_compressor_b200 import streams
+    main, side = _FakeStream(), [_FakeStream() for _ in range(4)]
+    monkeypatch.setattr(streams, "_side_streams", lambda device, n: side[:n])
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: main)
+    monkeypatch.setattr(torch.cuda, "Event", _FakeEvent)
+    monkeypatch.setattr(torch.cuda, "stream", lambda s: contextlib.nullcontext())
+    return streams, main, side
+
+
+# a job of three that raises: when it is queued, when it is ended, or not at all
+@pytest.mark.parametrize("bad_queue,bad_end", [(None, None), (0, None), (1, None), (None, 0), (None, 2), (2, 0)])
+def test_queued_jobs_end_although_one_raises(fake_streams, bad_queue, bad_end):
+    streams, main, side = fake_streams
+    done = []
+
+    def job(k):
+        def end():
+            if k == bad_end:
+                raise RuntimeError(f"end {k}")
+            done.append(k)
+            return 10 * k
+        if k == bad_queue:
+            raise RuntimeError(f"queue {k}")
+        return end
+
+    jobs = [lambda k=k: job(k) for k in range(3)]
+    if bad_queue is None and bad_end is None:
+        assert streams.run_queued(jobs, "cuda:0") == [0, 10, 20]
+    else:
+        first = f"queue {bad_queue}" if bad_queue is not None else f"end {bad_end}"
+        with pytest.raises(RuntimeError, match=first):
+            streams.run_queued(jobs, "cuda:0")
+    assert done == [k for k in range(3) if k not in (bad_queue, bad_end)]
+    assert main.waited == side[:3] and all(len(s.waited) == 1 for s in side[:3])
