@@ -94,9 +94,13 @@ class QuantizationArgs:
 
     def model_copy(self, update=None) -> "QuantizationArgs":
         # (what dataclasses.replace does, without its walk over the fields)
+        update = update or {}
+        for name in update:
+            if name not in self.__dataclass_fields__:
+                raise TypeError(f"{type(self).__name__} has no field {name!r}")
         out = object.__new__(type(self))
         out.__dict__.update(self.__dict__)
-        out.__dict__.update(update or {})
+        out.__dict__.update(update)
         out.__post_init__()
         return out
 

@@ -217,3 +217,11 @@ def test_queued_jobs_end_although_one_raises(fake_streams, bad_queue, bad_end):
             streams.run_queued(jobs, "cuda:0")
     assert done == [k for k in range(3) if k not in (bad_queue, bad_end)]
     assert main.waited == side[:3] and all(len(s.waited) == 1 for s in side[:3])
+
+
+def test_model_copy_takes_fields_only():
+    args = QuantizationArgs(num_bits=4, group_size=128)
+    copy = args.model_copy(update={"num_bits": 8, "actorder": "static"})
+    assert (copy.num_bits, copy.actorder, copy.group_size) == (8, "weight", 128) and args.num_bits == 4
+    with pytest.raises(TypeError, match="group_sise"):
+        args.model_copy(update={"group_sise": 64})
