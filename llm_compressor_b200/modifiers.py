@@ -770,7 +770,6 @@ class GPTQModifier(QuantizationMixin):
         taken, status = [], None
         for module in module_list:
             group = self._groups.pop(module)
-            status = group.status
             self._num_samples.pop(module, None)
             qargs = module.quantization_scheme.weights
             if qargs.actorder not in factors:
@@ -778,6 +777,7 @@ class GPTQModifier(QuantizationMixin):
                 H = group.finalized(keep=bool(left))  # the factorisation consumes its argument
                 factors[qargs.actorder] = make_factor(H, qargs.actorder)
                 self._trace("job_factored", module)
+            status = group.status   # (after the sum has been handed over)
             taken.append((module, qargs, factors[qargs.actorder]))
         return taken, status
 
@@ -1043,11 +1043,13 @@ class _HessianGroup:
         self.n += added
         self._last = (inp, inp._version)
 
-    def take_sum(self) -> torch.Tensor:
-        """The lower triangle of the sum over all batches, handed over."""
+    def take_sum(self, status=None) -> torch.Tensor:
+        """The lower triangle of the sum over all batches, handed over.  The status word leaves the sum's allocation, for
+        ``status`` if the caller has copied it already: who reads it must not keep the matrix from being freed."""
         self._last = None
         self.flush()
         self._stage = None
+        self.status = self.status.clone() if status is None else status
         H, self.H = self.H.to(self.device), None
         return H
 
@@ -1071,7 +1073,10 @@ def _finalize_groups(groups) -> None:
             by_width.setdefault(g.H.shape[0], []).append(g)
     for gs in by_width.values():
         if len(gs) > 1:
-            Hs = [g.take_sum() for g in gs]
+            for g in gs:
+                g.flush()
+            words = torch.cat([g.status for g in gs]).split(1)
+            Hs = [g.take_sum(status) for g, status in zip(gs, words)]
             gptq.ops.hessian_finalize_many(Hs, [1.0 / g.n if g.n else 1.0 for g in gs])
             for g, H in zip(gs, Hs):
                 g._final = H

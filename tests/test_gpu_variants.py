@@ -6,7 +6,7 @@ import torch
 
 import oracle
 from helpers import args_from, bits_equal, mismatch, synth_acts, synth_weight
-from llm_compressor_b200 import GPTQModifier, QuantizationModifier, compress_state_dict, gptq, observers, oneshot, ops
+from llm_compressor_b200 import GPTQModifier, QuantizationModifier, compress_state_dict, gptq, modifiers, observers, oneshot, ops
 from llm_compressor_b200.awq import scaled_fake_quantize
 from llm_compressor_b200.quant_args import QuantizationArgs, preset_name_to_scheme
 
@@ -277,3 +277,20 @@ def test_a_solve_that_raises_leaves_the_others_quantised():
         lin = getattr(parent, f"p{k}")
         assert not torch.equal(lin.weight.data, before[k]) and lin.quantization_status == "frozen"
     assert sorted(mod.losses) == ["p1", "p2"]
+
+
+@pytest.mark.parametrize("many", [False, True])
+def test_status_word_does_not_keep_the_hessian(many):
+    K = 1024
+    lin = torch.nn.Linear(K, 8, bias=False, device=DEV, dtype=torch.bfloat16)
+    groups = [modifiers._HessianGroup(lin) for _ in range(2)]
+    for g in groups:
+        g.accumulate(synth_acts(1, 256, K, 0).to(DEV))
+        g.flush()
+    if many:
+        modifiers._finalize_groups(groups)
+    Hs = [g.finalized() for g in groups]
+    before = torch.cuda.memory_allocated()
+    del Hs
+    assert torch.cuda.memory_allocated() <= before - 2 * 4 * K * K
+    assert [int(g.status) for g in groups] == [0, 0]
