@@ -298,7 +298,7 @@ def quantize_weight(module, quant_args, hessian: Optional[torch.Tensor], blocksi
     out = _sweep_output(inp)
     if defer:
         loss = losses.sum()
-        out["_status"] = status   # the sweep's device status word; the caller checks and removes it
+        out["_status"] = status.clone()   # the caller checks and removes it; it must not keep the workspace it came from
         return loss, out
     # one wait for everything: the loss, the sweep's status and, of a factorisation that nobody has waited for yet
     # (the sweep was queued behind it without asking), the factor's
@@ -363,5 +363,5 @@ def quantize_weights_batched(modules, quant_args, factors, blocksize: int = 128,
     sums = losses.sum(dim=1).unbind(0)
     back = ops.scatter_columns_cast_batched(Wf, first.final_dtype, None if perms[0] is None else perms).unbind(0)
     done = [(sums[k], _sweep_output(i, weight=back[k])) for k, i in enumerate(inputs)]
-    done[0][1]["_status"] = status
+    done[0][1]["_status"] = status.clone()   # (not a view of the workspace)
     return done

@@ -272,3 +272,14 @@ def test_sweep_losses_are_summed_in_short_runs(N, K, tokens, limit):
     scale = torch.full((N, 1), 1e4, device=DEV).bfloat16()
     losses = ops.gptq_sweep(w.float(), U, scale, None, args_from(SCHEMES["W8_CHANNEL"]))
     assert float(((losses.double() - total) / total).pow(2).mean().sqrt()) <= limit
+
+
+def test_status_of_a_deferred_sweep_does_not_keep_its_workspace():
+    args = args_from(SCHEMES["W4A16"])
+    problems = [_problem(64, 640, seed=i) for i in range(2)]
+    mods = [_lin(w, args) for w, _ in problems]
+    factors = gptq.factor_hessians_batched([H.clone().to(DEV) for _, H in problems], 0.01, None)
+    words = [gptq.quantize_weights_batched(mods, args, factors)[0][1]["_status"]]
+    words.append(gptq.quantize_weight(mods[0], args, None, factor=factors[0], defer=True)[1]["_status"])
+    for w in words:
+        assert int(w) == 0 and w.untyped_storage().nbytes() == 4
