@@ -13,7 +13,6 @@ from __future__ import annotations
 import collections
 import contextlib
 import functools
-import math
 import re
 import time
 import warnings
@@ -223,7 +222,9 @@ class QuantizationMixin(HooksMixin):
                     reg("weight_global_scale", torch.empty(1, dtype=torch.float32, device=dev))
                 reg("weight_scale", torch.empty(shape, dtype=dt if dt.is_floating_point else torch.float16,
                                                 device=dev))
-                zero_points.setdefault(dev, []).append((module, shape, w.zp_dtype))
+                zero_point = torch.empty(shape, dtype=w.zp_dtype, device=dev)
+                reg("weight_zero_point", zero_point)
+                zero_points.setdefault(dev, []).append(zero_point)
                 if w.actorder == "group":
                     reg("weight_g_idx", torch.full((K,), -1, dtype=torch.int32, device=dev))
                 a = scheme.input_activations
@@ -238,12 +239,9 @@ class QuantizationMixin(HooksMixin):
                         reg("input_scale", torch.empty(1, dtype=dt if dt.is_floating_point else torch.float16,
                                                        device=dev))
                         reg("input_zero_point", torch.zeros(1, dtype=a.zp_dtype, device=dev))
-        for dev, wanted in zero_points.items():
-            # one launch clears them all (a module's own tensor took 8 us of host time and a launch)
-            sizes = [-(-math.prod(shape) * dtype.itemsize // 16) * 16 for _, shape, dtype in wanted]
-            for (module, shape, dtype), piece in zip(wanted, torch.zeros(sum(sizes), dtype=torch.uint8, device=dev).split(sizes)):
-                zp = piece.view(dtype)[:math.prod(shape)].view(shape)
-                module.register_parameter("weight_zero_point", torch.nn.Parameter(zp, requires_grad=False))
+        for tensors in zero_points.values():
+            # one launch clears them all (each by itself took 8 us of host time and a launch)
+            torch._foreach_zero_([t.view(torch.int8) for t in tensors])
         if self.kv_cache_scheme is not None:
             # attention modules get k_scale / v_scale (CT lifecycle/initialize.py:255-310); the scheme
             # sits on the module as its input_activations, as the reference's config resolution puts it

@@ -74,6 +74,18 @@ def test_initialize_attaches_params_and_checks_divisibility():
     assert m3.attn.q_proj.weight_global_scale.dtype == torch.float32
 
 
+@pytest.mark.parametrize("scheme", ["W4A16", "FP8_DYNAMIC", "NVFP4A16"])
+def test_every_parameter_owns_its_storage(scheme):
+    """Saving or dropping one module must not take the others' parameters along."""
+    m = Tiny().to(torch.bfloat16)
+    QuantizationModifier(targets="Linear", scheme=scheme, ignore=["lm_head"]).on_initialize(m)
+    for name in ("q_proj", "k_proj", "v_proj"):
+        lin = getattr(m.attn, name)
+        for p in lin.parameters():
+            assert p.untyped_storage().nbytes() == p.numel() * p.element_size(), name
+        assert not lin.weight_zero_point.float().any()
+
+
 def test_gptq_requires_targets():
     m = Tiny()
     mod = GPTQModifier(targets="Conv2d", scheme="W4A16")
