@@ -816,6 +816,7 @@ class GPTQModifier(QuantizationMixin):
         if results:
             torch._foreach_copy_([module.weight.data for module, _, _ in results],
                                  [out["weight"] for _, _, out in results])
+        shared = {}   # dtype -> ([parameters], [values]) of values that are slices of a batch's buffer
         for module, loss, out in results:
             loss = float(loss)
             name = self._module_names.get(module, type(module).__name__)
@@ -825,12 +826,21 @@ class GPTQModifier(QuantizationMixin):
                 if attr == "weight":
                     continue
                 p = getattr(module, attr, None)
-                if p is not None:
+                whole = val.untyped_storage().nbytes() == val.numel() * val.element_size()
+                if p is None:
+                    module.register_parameter(attr, torch.nn.Parameter(val if whole else val.clone(), requires_grad=False))
+                elif whole or p.dtype != val.dtype or p.device != val.device:
                     _put(p, val)
                 else:
-                    module.register_parameter(attr, torch.nn.Parameter(val, requires_grad=False))
+                    into, values = shared.setdefault(val.dtype, ([], []))
+                    into.append(p.data)
+                    values.append(val.reshape(p.shape))
             _set_plain(module, "quantization_status", "frozen")
             self._done.add(module)
+        for dtype, (into, values) in shared.items():
+            if dtype.itemsize == 1:   # (the one-launch copy takes no float8)
+                into, values = [t.view(torch.uint8) for t in into], [t.view(torch.uint8) for t in values]
+            torch._foreach_copy_(into, values)
 
     def _compress_group(self, module_list):
         """Factor and sweep the modules of one Hessian."""

@@ -283,3 +283,29 @@ def test_status_of_a_deferred_sweep_does_not_keep_its_workspace():
     words.append(gptq.quantize_weight(mods[0], args, None, factor=factors[0], defer=True)[1]["_status"])
     for w in words:
         assert int(w) == 0 and w.untyped_storage().nbytes() == 4
+
+
+@pytest.mark.parametrize("scheme", ["FP8_DYNAMIC", "W4A16_ASYM"])
+def test_parameters_of_a_batch_own_their_storage(scheme):
+    """Saving or dropping one expert must not take the others' parameters along; values as a module by itself gets them."""
+    K, N, count = 256, 64, 16
+    parent = torch.nn.Module()
+    for k in range(count):
+        lin = torch.nn.Linear(K, N, bias=False, device=DEV, dtype=torch.bfloat16)
+        lin.weight.data = synth_weight(N, K, k).to(DEV)
+        parent.add_module(f"expert_{k}", lin)
+    mod = GPTQModifier(targets="Linear", scheme=scheme, actorder=None)
+    mod.on_initialize(parent)
+    mod.on_calibration_start(parent)
+    x = synth_acts(2, 512, K, 0).to(DEV)
+    expected = []
+    for lin in parent.children():
+        args = lin.quantization_scheme.weights
+        expected.append(ops.qparams(*ops.observe_minmax(lin.weight.data, args), args))
+        mod.calibrate_module(lin, (x,), None)
+    mod.on_sequential_epoch_end(parent, list(parent.modules()))
+    for lin, (scale, zp) in zip(parent.children(), expected):
+        assert lin.quantization_status == "frozen"
+        for p in lin.parameters():
+            assert p.untyped_storage().nbytes() == p.numel() * p.element_size()
+        assert bits_equal(lin.weight_scale, scale) and bits_equal(lin.weight_zero_point, zp)
