@@ -65,11 +65,15 @@ const char* b200q_last_error(void);
 /* Number of kernels this library has launched in the process so far (diagnostic; no
  * counterpart in the reference). */
 long long b200q_launch_count(void);
-/* The streaming quantize / pack kernels that are fed by TMA copies wait for them with a bound.  If
- * such a wait ever ran out on the current device since the last call, this returns
- * B200Q_ERR_DEVICE once (the affected launch left its output incomplete), otherwise B200Q_OK.
+/* The streaming quantize / pack kernels that are fed by TMA copies, and b200q_gptq_sweep_batched,
+ * have no status word to give back.  If one of their bounded waits ever ran out on the current
+ * device since the last call, this returns B200Q_ERR_DEVICE once (the affected launch left its
+ * output incomplete), otherwise B200Q_OK.
  * Synchronises the device.  No counterpart in the reference. */
 int b200q_take_wait_status(void);
+/* Hands the status word of another call (a device int32 that is non-zero after a wait that ran
+ * out) over to b200q_take_wait_status, in stream order and without waiting. */
+int b200q_note_wait_status(const int* status, void* stream);
 
 /* ------------------------------------------------------------------ observers */
 
@@ -347,7 +351,8 @@ int b200q_gptq_sweep(float* Wf, int64_t N, int64_t K, int64_t ldf, const float* 
  *
  * b200q_gptq_factor_batched / b200q_gptq_sweep_batched: the same two calls without a workspace
  * argument (scratch[i], K*K floats each, is accepted and not used; blocksize must be 128): what
- * they need is taken from the stream's memory pool and given back before they return. */
+ * they need is taken from the stream's memory pool and given back in stream order.  A wait of the
+ * sweep that ran out is reported by b200q_take_wait_status. */
 size_t b200q_gptq_factor_many_workspace_bytes(int64_t K, int count);
 int b200q_gptq_factor_many(float* const* H, int count, int64_t K, int64_t ldh, void* workspace, int* status,
                            void* stream);

@@ -746,8 +746,10 @@ int b200q_gptq_sweep_batched(float* const* W, const float* const* U, const void*
   void* ws = nullptr;
   cudaStream_t st = (cudaStream_t)stream;
   B200Q_TRY(cudaMallocAsync(&ws, b200q_gptq_sweep_many_workspace_bytes(N, K, count, count), st));
-  const int rc = b200q_gptq_sweep_many(W, U, U, count, nullptr, scale, sdtype, zp, col_group, gscale, losses, count, N, K,
-                                       ldw, ldu, qa, ws, stream);
+  int rc = b200q_gptq_sweep_many(W, U, U, count, nullptr, scale, sdtype, zp, col_group, gscale, losses, count, N, K,
+                                 ldw, ldu, qa, ws, stream);
+  // the status word goes with the workspace: whatever it says by then is kept for b200q_take_wait_status
+  if (rc == B200Q_OK) rc = b200q_note_wait_status((const int*)ws, stream);
   B200Q_TRY(cudaFreeAsync(ws, st));
   return rc;
 }

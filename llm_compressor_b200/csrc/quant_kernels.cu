@@ -1143,6 +1143,10 @@ __global__ void __launch_bounds__(256) scaled_channel_kernel(const void* __restr
   }
 }
 
+__global__ void note_wait_kernel(const int* status) {
+  if (*status != 0) atomicExch(&tma::g_wait_expired, 1);
+}
+
 }  // namespace b200q
 
 using namespace b200q;
@@ -1158,11 +1162,19 @@ long long b200q_launch_count(void) { return g_launches.load(std::memory_order_re
 
 int b200q_take_wait_status(void) {
   int v = 0;
+  B200Q_TRY(cudaDeviceSynchronize());   // (the copy alone does not wait for non-blocking streams)
   B200Q_TRY(cudaMemcpyFromSymbol(&v, tma::g_wait_expired, sizeof(int)));
   if (v == 0) return B200Q_OK;
   v = 0;
   B200Q_TRY(cudaMemcpyToSymbol(tma::g_wait_expired, &v, sizeof(int)));
   return B200Q_ERR_DEVICE;
+}
+
+int b200q_note_wait_status(const int* status, void* stream) {
+  if (!status) return B200Q_ERR_ARG;
+  note_wait_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(status);
+  B200Q_LAUNCH_CHECK();
+  return B200Q_OK;
 }
 
 size_t b200q_observe_minmax_workspace_bytes(int64_t, int64_t, const b200q_qargs* qa) {

@@ -10,7 +10,7 @@ import torch
 
 import oracle
 from helpers import args_from, bits_equal, mismatch, synth_acts, synth_weight
-from llm_compressor_b200 import GPTQModifier, gptq, observers, ops
+from llm_compressor_b200 import GPTQModifier, _lib, gptq, observers, ops
 from test_oracle_golden import spec_from
 
 pytestmark = pytest.mark.gpu
@@ -309,3 +309,36 @@ def test_parameters_of_a_batch_own_their_storage(scheme):
         for p in lin.parameters():
             assert p.untyped_storage().nbytes() == p.numel() * p.element_size()
         assert bits_equal(lin.weight_scale, scale) and bits_equal(lin.weight_zero_point, zp)
+
+
+def test_entry_points_without_workspace():
+    """b200q_gptq_factor_batched and b200q_gptq_sweep_batched give what the calls with a workspace give."""
+    lib, args, K, N, count = _lib.load(), args_from(SCHEMES["W4A16"]), 640, 96, 3
+    Hs = [_spd(K, i).to(DEV) for i in range(count)]
+    many, batched = [H.clone() for H in Hs], [H.clone() for H in Hs]
+    ops.gptq_factor_batched(many)
+    scratch = [torch.empty(lib.b200q_gptq_factor_batched_workspace_bytes(K, 1) // 4, device=DEV) for _ in range(count)]
+    status = torch.full((count, 4), 7, dtype=torch.int32, device=DEV)
+    table = ops._pointer_table([batched, scratch])
+    _lib.check(lib.b200q_gptq_factor_batched(table[0].data_ptr(), table[1].data_ptr(), count, K, K, status.data_ptr(),
+                                             _lib.stream_ptr()), "factor")
+    assert int(status.abs().max()) == 0 and all(bits_equal(a, b) for a, b in zip(many, batched))
+    ws = [synth_weight(N, K, seed=i).to(DEV) for i in range(count)]
+    scales = [ops.qparams(*ops.observe_minmax(w, args), args)[0] for w in ws]
+    a, b = [w.float() for w in ws], [w.float() for w in ws]
+    losses = ops.gptq_sweep_batched(a, many, scales, None, args)
+    got = torch.empty_like(losses)
+    table = ops._pointer_table([b, many, scales, got])
+    _lib.check(lib.b200q_gptq_sweep_batched(table[0].data_ptr(), table[1].data_ptr(), table[2].data_ptr(), _lib.BF16, None,
+                                            None, None, table[3].data_ptr(), count, N, K, K, K, args.c_struct(), 128,
+                                            _lib.stream_ptr()), "sweep")
+    assert bits_equal(got, losses) and all(bits_equal(x, y) for x, y in zip(a, b))
+    assert lib.b200q_take_wait_status() == 0
+
+
+def test_noted_status_word_is_reported_once():
+    lib = _lib.load()
+    for word, expected in ((0, 0), (-4, -4)):
+        _lib.check(lib.b200q_note_wait_status(torch.full((1,), word, dtype=torch.int32, device=DEV).data_ptr(),
+                                              _lib.stream_ptr()), "note")
+        assert lib.b200q_take_wait_status() == expected and lib.b200q_take_wait_status() == 0
