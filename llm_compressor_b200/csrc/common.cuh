@@ -34,7 +34,6 @@ void count_launch();
     B200Q_TRY(cudaGetLastError());    \
   } while (0)
 
-// Grid size for a grid-stride kernel: whole multiples of the SM count, capped by the work.
 // CTAs of a grid-stride kernel: what is resident at once, no more.  (A grid of six CTAs per SM where five fit ran a second
 // wave of one CTA per SM: 14336 x 4096 NVFP4 codes took 99 us.)
 template <auto Kernel> inline int resident_grid(int threads, size_t smem, int64_t blocks_needed) {
@@ -67,6 +66,7 @@ inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, int threads, 
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
+// Grid size for a grid-stride kernel: whole multiples of the SM count, capped by the work.
 inline int grid_for(int64_t blocks_needed, int blocks_per_sm) {
   int64_t cap = (int64_t)kNumSMs * blocks_per_sm;
   if (blocks_needed >= cap) return (int)cap;
@@ -207,27 +207,6 @@ template <bool SB>
 __device__ __forceinline__ float dequant_code(float q, float s, float zp) {
   float d = rnd_if<SB>(q - zp);
   return rnd_if<SB>(d * s);
-}
-
-// Fake-quantised value of a float32 weight, as the GPTQ sweep needs it once per column on its
-// critical path: the same result as dequant_code<SB>(quant_code<false>(x, s, zp, r), s, zp), with
-// the code type a compile-time constant and the division replaced by the product with rs = 1/s
-// whenever both ends of a 2^-20 interval around it give the same code (else the division is redone).
-template <int KIND, bool SB>
-__device__ __forceinline__ float fake_quant_f32(float x, float s, float rs, float zp, float qmin, float qmax) {
-  const float qa = x * rs;
-  const float aq = fabsf(qa);
-  const float a = round_code_k<KIND>(fmaf(qa, 1.0f - 0x1p-20f, zp), qmin, qmax);
-  const float b = round_code_k<KIND>(fmaf(qa, 1.0f + 0x1p-20f, zp), qmin, qmax);
-  float q = a;   // both ends have the sign of qa, so this is also the code's sign of zero
-  if (!((aq < 1e30f) && (aq > 1e-30f || aq == 0.0f) && (a == b)))
-    q = round_code_k<KIND>(__fdiv_rn(x, s) + zp, qmin, qmax);
-  if constexpr (KIND == kInt) {
-    // an integer code minus an integer zero point is at most 255 in magnitude: exact in bf16 too,
-    // so only the product with the scale is rounded
-    return rnd_if<SB>((q - zp) * s);
-  }
-  return dequant_code<SB>(q, s, zp);
 }
 
 __device__ __forceinline__ float load_zp(const void* zp, int zp_kind, int64_t i) {

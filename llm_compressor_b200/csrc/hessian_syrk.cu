@@ -512,8 +512,6 @@ syrk_pair_kernel(const __grid_constant__ CUtensorMap xmap, Params p) {
   const uint32_t tmem_base = s_tmem_base;
   chain_wait();   // (setting up overlaps the end of the kernel before: hidden in calls of a few hundred tokens)
 
-  const int total_units = p.tiles * p.splits;
-
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (both CTAs)
     if (lane == 0) {

@@ -400,14 +400,7 @@ __global__ void __launch_bounds__(kThreads) rtn_group_kernel(
   }
 }
 
-// bf16 weights: same as rtn_group_kernel<B200Q_BF16, ...> with the packed fast paths.
-__device__ __forceinline__ void minmax8_bf16(const uint4& raw, float& lo, float& hi) {
-  const __nv_bfloat162* w = reinterpret_cast<const __nv_bfloat162*>(&raw);
-  __nv_bfloat162 mx = __hmax2(__hmax2(w[0], w[1]), __hmax2(w[2], w[3]));
-  __nv_bfloat162 mn = __hmin2(__hmin2(w[0], w[1]), __hmin2(w[2], w[3]));
-  hi = fmaxf(__bfloat162float(mx.x), __bfloat162float(mx.y));
-  lo = fminf(__bfloat162float(mn.x), __bfloat162float(mn.y));
-}
+// ---- bf16 weights: the packed paths ----
 // Range of a group for calculate_qparams, which clamps it to contain zero first: bf16 bit
 // patterns order like unsigned integers among negative values (the larger pattern is the more
 // negative number, and every negative pattern is above every positive one) and like signed
