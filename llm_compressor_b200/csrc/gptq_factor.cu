@@ -20,6 +20,8 @@
 // The last three are one launch: the rows of its second operand are X[o,:o]^T, D^T and P, indexed by absolute column.
 //
 // A pivot <= 0 (or NaN) sets the problem's status; the host then takes the reference's identity fallback.
+#include <type_traits>
+
 #include "common.cuh"
 #include "tgemm_tf32.cuh"
 
@@ -174,28 +176,46 @@ __global__ void __launch_bounds__(kThreads, 1) chol_diag_kernel(Mat mt, int k0, 
                 make_float2(old[j][h].x - acc[j][2 * h], old[j][h].y - acc[j][2 * h + 1]);
         __syncwarp();
       }
-      float a[W16];
+      float a[W16], ri;
       const float* src = R + (c0 + (lane & 15)) * LD + c0;
+      // the first pivot that `Exact` does not accept, + 1: the quick form takes positive normal numbers, the exact one
+      // (rare, so out of the way) everything above zero.  Garbage from that pivot on.
+      auto eliminate = [&](auto Exact) -> int {
+        int first = 0;
+        ri = 0.0f;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const float4 v = *reinterpret_cast<const float4*>(src + 4 * q);
-        a[4 * q] = v.x; a[4 * q + 1] = v.y; a[4 * q + 2] = v.z; a[4 * q + 3] = v.w;
-      }
-      float piv = __shfl_sync(0xffffffffu, a[0], 0), ri = 0.0f;
+        for (int q = 0; q < 4; ++q) {
+          const float4 v = *reinterpret_cast<const float4*>(src + 4 * q);
+          a[4 * q] = v.x; a[4 * q + 1] = v.y; a[4 * q + 2] = v.z; a[4 * q + 3] = v.w;
+        }
+        float piv = __shfl_sync(0xffffffffu, a[0], 0);
 #pragma unroll
-      for (int j = 0; j < W16; ++j) {
-        // (a pivot that is not a positive normal number makes garbage from here on, and is reported)
-        bad = (!(piv >= 1.17549435e-38f) && bad == 0) ? c0 + j + 1 : bad;
-        float r;
-        asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(piv));
-        // one Newton step r (1.5 - piv r^2 / 2), within an ulp of 1 / sqrt, folded into the column's scaling
-        const float u = fmaf(-(0.5f * piv) * r, r, 1.5f);
-        const float l = (a[j] * r) * u;
-        if (j + 1 < W16) piv = __shfl_sync(0xffffffffu, fmaf(-l, l, a[j + 1]), j + 1);
-        a[j] = l;
-        ri = (lane == j) ? r * u : ri;
+        for (int j = 0; j < W16; ++j) {
+          float l, root;   // 1 / sqrt(piv)
+          if constexpr (Exact) {
+            first = (!(piv > 0.0f) && first == 0) ? j + 1 : first;
+            root = __fdiv_rn(1.0f, __fsqrt_rn(piv));
+            l = a[j] * root;
+          } else {
+            first = (!(piv >= 1.17549435e-38f) && first == 0) ? j + 1 : first;
+            float r;
+            asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(piv));
+            // one Newton step r (1.5 - piv r^2 / 2), within an ulp of 1 / sqrt, folded into the column's scaling
+            const float u = fmaf(-(0.5f * piv) * r, r, 1.5f);
+            l = (a[j] * r) * u;
+            root = r * u;
+          }
+          if (j + 1 < W16) piv = __shfl_sync(0xffffffffu, fmaf(-l, l, a[j + 1]), j + 1);
+          a[j] = l;
+          ri = (lane == j) ? root : ri;
 #pragma unroll
-        for (int c = j + 1; c < W16; ++c) a[c] = fmaf(-l, __shfl_sync(0xffffffffu, l, c), a[c]);
+          for (int c = j + 1; c < W16; ++c) a[c] = fmaf(-l, __shfl_sync(0xffffffffu, l, c), a[c]);
+        }
+        return first;
+      };
+      if (eliminate(std::false_type())) {
+        const int first = eliminate(std::true_type());
+        bad = (first && bad == 0) ? c0 + first : bad;
       }
       if (lane < W16) {
 #pragma unroll

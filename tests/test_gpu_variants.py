@@ -6,7 +6,7 @@ import torch
 
 import oracle
 from helpers import args_from, bits_equal, mismatch, synth_acts, synth_weight
-from llm_compressor_b200 import GPTQModifier, QuantizationModifier, compress_state_dict, gptq, modifiers, observers, oneshot, ops
+from llm_compressor_b200 import GPTQModifier, QuantizationModifier, _lib, compress_state_dict, gptq, modifiers, observers, oneshot, ops
 from llm_compressor_b200.awq import scaled_fake_quantize
 from llm_compressor_b200.quant_args import QuantizationArgs, preset_name_to_scheme
 
@@ -294,3 +294,27 @@ def test_status_word_does_not_keep_the_hessian(many):
     del Hs
     assert torch.cuda.memory_allocated() <= before - 2 * 4 * K * K
     assert [int(g.status) for g in groups] == [0, 0]
+
+
+# pivots below the smallest normal float32 (1.2e-38): alone, and one among normal ones in the middle of a 16-column step
+@pytest.mark.parametrize("K,tiny", [(1, [0]), (16, range(16)), (130, range(130)), (200, [77])])
+def test_factor_accepts_subnormal_pivots(K, tiny):
+    d = torch.full((K,), 4.0, dtype=torch.float64)
+    for i in tiny:
+        d[i] = 1e-39 * (1 + i % 7)
+    H = torch.diag(d).float().to(DEV)
+    ref = 1.0 / H.diagonal().double().sqrt()
+    many = [H.clone() for _ in range(2)]
+    assert ops.gptq_factor(H) == 0
+    assert int(ops.gptq_factor_batched(many).abs().max()) == 0
+    for U in [H] + many:
+        assert torch.allclose(U.diagonal().double(), ref, rtol=2e-7)
+        assert float((U - torch.diag(U.diagonal())).abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("K,column,value", [(16, 3, 0.0), (200, 150, -1e-39), (200, 77, float("nan")), (640, 600, -0.0)])
+def test_factor_reports_the_first_bad_pivot(K, column, value):
+    H = torch.diag(torch.full((K,), 4.0)).to(DEV)
+    H[column, column] = value
+    status = ops.gptq_factor_async(H).tolist()
+    assert status == [_lib.NOT_POSITIVE_DEFINITE, K - column, 0, 0]   # (columns are counted in reversed order)
