@@ -744,16 +744,7 @@ class GPTQModifier(QuantizationMixin):
             else:
                 run_concurrent([lambda mods=mods: self._compress_group(mods) for mods in jobs], device,
                                max_streams=self.parallel_streams)
-            # The jobs end in an order that varies from run to run; the losses are kept in the one they mostly end in: by
-            # the columns of their chains (one for the factor and one for each sweep), or, where Hessians are so narrow
-            # that queueing the launches takes longer, by the modules.
-            narrow = min(mods[0].weight.shape[1] for mods in jobs) < 1024
-
-            def length(mods):
-                width = mods[0].weight.shape[1]
-                return (len(mods) if narrow else width * (1 + len(mods)), width)
-
-            for mods in sorted(jobs, key=length):
+            for mods in _loss_order(jobs):
                 for m in mods:
                     name = self._module_names.get(m, type(m).__name__)
                     if name in self.losses:
@@ -944,6 +935,20 @@ class GPTQModifier(QuantizationMixin):
                              f"compressed: {names}{' ...' if len(missed) > 8 else ''}")
         self._groups, self._num_samples, self._hooked = {}, {}, []
         return True
+
+
+def _loss_order(jobs) -> list:
+    """The order in which the losses of one ``compress_module_list`` call stand in ``losses``, whichever job ended first:
+    by the columns of a job's chain (one for the factor, one for each sweep), or, if some Hessian has fewer than 1024
+    columns, by its number of modules; then by width.  The order means nothing, and callers should look losses up by name;
+    it is fixed so that callers that go through ``losses.values()`` meet the same places on every run."""
+    narrow = min(mods[0].weight.shape[1] for mods in jobs) < 1024
+
+    def length(mods):
+        width = mods[0].weight.shape[1]
+        return (len(mods) if narrow else width * (1 + len(mods)), width)
+
+    return sorted(jobs, key=length)
 
 
 def _plain_args(a: QuantizationArgs) -> dict:

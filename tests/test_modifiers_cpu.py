@@ -7,7 +7,8 @@ import torch
 import torch.multiprocessing as mp
 
 from llm_compressor_b200 import dist as bdist
-from llm_compressor_b200.modifiers import GPTQModifier, QuantizationModifier, match_named_modules
+from llm_compressor_b200 import modifiers
+from llm_compressor_b200.modifiers import GPTQModifier, QuantizationModifier, _loss_order, match_named_modules
 
 
 class Attn(torch.nn.Module):
@@ -84,6 +85,83 @@ def test_every_parameter_owns_its_storage(scheme):
         for p in lin.parameters():
             assert p.untyped_storage().nbytes() == p.numel() * p.element_size(), name
         assert not lin.weight_zero_point.float().any()
+
+
+@pytest.mark.parametrize("hidden,inter,expected", [(2048, 5632, "o gate up q k v down"), (768, 2048, "o down gate up q k v")])
+@pytest.mark.parametrize("reverse", [False, True])
+def test_losses_stand_in_one_order(hidden, inter, expected, reverse):
+    """A decoder layer's jobs (a Hessian each), ended in whatever order."""
+    jobs = []
+    for names, width in ((["q", "k", "v"], hidden), (["o"], hidden), (["gate", "up"], hidden), (["down"], inter)):
+        job = [torch.nn.Linear(width, 8, bias=False, device="meta") for _ in names]
+        for name, lin in zip(names, job):
+            lin.name = name
+        jobs.append(job)
+    order = _loss_order(jobs[::-1] if reverse else jobs)
+    assert [lin.name for job in order for lin in job] == expected.split()
+
+
+def _stub_group(monkeypatch):
+    made = []
+
+    class Group(modifiers._HessianGroup):
+        def __init__(self, module, offload=False, stage_tokens=0):
+            self.members, self._last, self.taken = [module], None, []
+            made.append(self)
+
+        def accumulate(self, inp):
+            self.taken.append(inp)
+            self._last = (inp, inp._version)
+    monkeypatch.setattr(modifiers, "_HessianGroup", Group)
+    return made
+
+
+def test_modules_of_one_input_share_a_hessian(monkeypatch):
+    made = _stub_group(monkeypatch)
+    m = Tiny()
+    mod = GPTQModifier(targets="Linear", scheme="W4A16", ignore=["lm_head", "gate"])
+    q, k, v = m.attn.q_proj, m.attn.k_proj, m.attn.v_proj
+    x = torch.randn(4, 256)
+    for lin in (q, k):
+        mod.calibrate_module(lin, (x,), None)
+    mod.calibrate_module(v, (x.clone(),), None)          # equal values elsewhere: another input
+    assert [g.members for g in made] == [[q, k], [v]] and [len(g.taken) for g in made] == [1, 1]
+    # the same buffer with other contents (an allocator that hands the block out again) is another batch
+    x.add_(1.0)
+    for lin in (q, k):
+        mod.calibrate_module(lin, (x,), None)
+    assert [len(g.taken) for g in made] == [2, 1]
+    # a view of the same address that reads it another way is another input, so k's membership no longer holds
+    with pytest.raises(RuntimeError, match="shared a Hessian"):
+        mod.calibrate_module(k, (x.as_strided((4, 256), (1, 4)),), None)
+
+
+def test_a_module_that_joins_late_finds_its_hessian(monkeypatch):
+    """Two groups whose batches had one address in turn: the table by address points at the later one."""
+    made = _stub_group(monkeypatch)
+    m = Tiny()
+    mod = GPTQModifier(targets="Linear", scheme="W4A16", ignore=["lm_head", "gate"])
+    q, k, v = m.attn.q_proj, m.attn.k_proj, m.attn.v_proj
+    x = torch.randn(4, 256)
+    mod.calibrate_module(q, (x,), None)
+    x.add_(1.0)
+    mod.calibrate_module(k, (x,), None)                   # q's group holds the older version: a group of its own
+    mod.calibrate_module(v, (x,), None)
+    assert [g.members for g in made] == [[q], [k, v]] and len(made[1].taken) == 1
+
+
+@pytest.mark.parametrize("value,stands_in", [
+    (torch.tensor([[1.0], [2.0]], dtype=torch.bfloat16), True),
+    (torch.tensor([1.0, 2.0], dtype=torch.bfloat16), True),                    # another shape of as many
+    (torch.tensor([[1.0], [2.0]]), False),                                     # another type
+    (torch.tensor([[1.0, 9.0], [2.0, 9.0]], dtype=torch.bfloat16)[:, :1], False),   # strided
+])
+def test_put_gives_a_parameter_its_values(value, stands_in):
+    p = torch.nn.Parameter(torch.zeros(2, 1, dtype=torch.bfloat16), requires_grad=False)
+    before = p.data_ptr()
+    modifiers._put(p, value)
+    assert p.dtype == torch.bfloat16 and p.shape == (2, 1) and p.is_contiguous() and p.reshape(-1).tolist() == [1.0, 2.0]
+    assert (p.data_ptr() == value.data_ptr()) == stands_in and (p.data_ptr() == before) != stands_in
 
 
 def test_gptq_requires_targets():
