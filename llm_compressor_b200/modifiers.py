@@ -777,10 +777,11 @@ class GPTQModifier(QuantizationMixin):
             raise B200QError("a bounded wait inside the Hessian or GEMM kernels of this job expired; "
                              "its results are incomplete")
 
-    def _finish_queued(self, queued, t0):
+    def _finish_queued(self, queued, t0, batch=(), copies={}):
         """``queued``: [(module, qargs, factor, loss, out)] of deferred solves whose factors have been
-        resolved.  Redo the modules whose Hessian was not positive definite with the identity, as
-        the reference falls back (gptq_quantize.py:157-164), then write every result to its module."""
+        resolved; ``batch``: those of them whose values are slices of a batch's buffers, and ``copies`` what
+        ``_gather_copies`` makes of them all.  Redo the modules whose Hessian was not positive definite with the
+        identity, as the reference falls back (gptq_quantize.py:157-164), then write every result to its module."""
         redo = [q for q in queued if not q[2].ok]
         # the deferred call consumed the observers' statistics: observe again before the
         # round-to-nearest redo (act-order "group" re-observes the permuted weight itself)
@@ -807,30 +808,26 @@ class GPTQModifier(QuantizationMixin):
         if results:
             torch._foreach_copy_([module.weight.data for module, _, _ in results],
                                  [out["weight"] for _, _, out in results])
-        shared = {}   # dtype -> ([parameters], [values]) of values that are slices of a batch's buffer
+        sliced = {id(q[0]) for q in batch if q[2].ok}
         for module, loss, out in results:
             loss = float(loss)
             name = self._module_names.get(module, type(module).__name__)
             self.losses[name] = loss
             self._log_metric(name, time.perf_counter() - t0, loss)
-            for attr, val in out.items():
-                if attr == "weight":
-                    continue
-                p = getattr(module, attr, None)
-                whole = val.untyped_storage().nbytes() == val.numel() * val.element_size()
-                if p is None:
-                    module.register_parameter(attr, torch.nn.Parameter(val if whole else val.clone(), requires_grad=False))
-                elif whole or p.dtype != val.dtype or p.device != val.device:
-                    _put(p, val)
-                else:
-                    into, values = shared.setdefault(val.dtype, ([], []))
-                    into.append(p.data)
-                    values.append(val.reshape(p.shape))
+            if id(module) not in sliced:
+                for attr, val in out.items():
+                    if attr == "weight":
+                        continue
+                    p = getattr(module, attr, None)
+                    if p is not None:
+                        _put(p, val)
+                    else:
+                        module.register_parameter(attr, torch.nn.Parameter(val, requires_grad=False))
             _set_plain(module, "quantization_status", "frozen")
             self._done.add(module)
-        for dtype, (into, values) in shared.items():
-            if dtype.itemsize == 1:   # (the one-launch copy takes no float8)
-                into, values = [t.view(torch.uint8) for t in into], [t.view(torch.uint8) for t in values]
+        if redo and batch:
+            copies = _gather_copies([(q[0], q[4]) for q in batch if q[2].ok])
+        for into, values in copies.values():
             torch._foreach_copy_(into, values)
 
     def _compress_group(self, module_list):
@@ -896,7 +893,7 @@ class GPTQModifier(QuantizationMixin):
                 schemes[id(qargs)] = repr(qargs)
             key = (tuple(module.weight.shape), module.weight.dtype, schemes[id(qargs)])
             by_shape.setdefault(key, []).append((module, qargs, holder[0]))
-        queued = []
+        queued, batch = [], []
         # the class with the most device work first: its sweep runs while the host prepares the others
         classes = sorted(by_shape.values(), key=lambda it: -len(it) * it[0][0].weight.shape[0]
                          * it[0][0].weight.shape[1] ** 2)
@@ -911,10 +908,13 @@ class GPTQModifier(QuantizationMixin):
                                                  factor=f, defer=True) for m, q, f in items]
                 words += [out.pop("_status", None) for _, out in done]
             queued += [(m, q, f, loss, out) for (m, q, f), (loss, out) in zip(items, done)]
+            if len(items) >= 4:
+                batch += queued[-len(items):]
         self._trace("job_swept", jobs[0][0])
+        copies = _gather_copies([(q[0], q[4]) for q in batch])   # (while the device is at work)
         self._check_status_words(words)
         gptq.resolve_factors([q[2] for q in queued])
-        self._finish_queued(queued, t0)
+        self._finish_queued(queued, t0, batch, copies)
 
     @staticmethod
     def _log_metric(name, seconds, loss):
@@ -949,6 +949,31 @@ def _loss_order(jobs) -> list:
         return (len(mods) if narrow else width * (1 + len(mods)), width)
 
     return sorted(jobs, key=length)
+
+
+def _gather_copies(solved) -> dict:
+    """{(types, device): ([parameters], [values])} of [(module, out)] whose values are slices of buffers that many modules share, for
+    one copy a type.  Put in as they are, the slices would keep the buffer alive, and saving one module would write all of
+    it."""
+    copies: dict = {}
+    for module, out in solved:
+        params = module._parameters
+        for attr, val in out.items():
+            if attr == "weight":
+                continue
+            p = params.get(attr)
+            if p is None:
+                p = torch.nn.Parameter(torch.empty_like(val, memory_format=torch.contiguous_format), requires_grad=False)
+                module.register_parameter(attr, p)
+            p = p.data
+            if val.shape != p.shape:
+                val = val.reshape(p.shape)
+            if val.dtype.itemsize == 1 and p.dtype == val.dtype:   # (the one-launch copy takes no float8)
+                p, val = p.view(torch.uint8), val.view(torch.uint8)
+            into, values = copies.setdefault((p.dtype, val.dtype, p.device), ([], []))
+            into.append(p)
+            values.append(val)
+    return copies
 
 
 def _plain_args(a: QuantizationArgs) -> dict:
