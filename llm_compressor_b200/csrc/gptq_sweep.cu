@@ -182,9 +182,10 @@ __device__ __forceinline__ void apply_errors(const ErrFrag& f, const float* u, f
         o[(x * 8 + (k & 1)) * WLD + y * 16 + (k >> 1) * 8] = old[y][x][k] - (acc[y][x][k] + part[y][x][k]);
 }
 
-// What bounds it: the chain of columns, some 60 cycles each for the quantisation (product with 1 / s, clamp, round,
-// dequantise, difference, product with the reciprocal pivot, correction of the next column).  So one warp of the CTA
-// does nothing but the chain: 16 columns at a time in registers, a lane per row.  Others apply a finished micro-block's
+// What bounds it: the chain of columns.  Its dependent instructions (product with 1 / s, clamp, round, dequantise,
+// difference, product with the reciprocal pivot, correction of the next column) come to some 60 cycles a column by their
+// latencies; measured it takes 308 (512 columns in 86.5 us at 1.82 GHz, 4096 rows), and where the rest goes has not been
+// measured.  So one warp of the CTA does nothing but the chain: 16 columns at a time in registers, a lane per row.  Others apply a finished micro-block's
 // 16 errors to the columns two micro-blocks on and later as warp-level tensor-core products (a float32 FMA formulation
 // spends its time on the broadcast loads of U: 480 cycles a column against the chain's own), taking tasks of 16 columns
 // from a counter.  The columns next in line take the first twelve errors from a warp that waits for them while the chain

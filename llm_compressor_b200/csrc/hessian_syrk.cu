@@ -865,6 +865,10 @@ int b200q_hessian_syrk(const void* X, int64_t T, int64_t K, int64_t ldx, float* 
     // thousand cycles a tile with all pairs at it); what ends last, the other of the two, is not hidden.  Filling the
     // waves alone, as the rule was, split 4096 tokens of K = 4096 seven ways: 84 us where one split takes 60.
     // (A single round of tiles leaves its additions behind in about 4 thousand.)
+    // The change of rate is gradual: 512 tokens, additions alone, take 15 thousand cycles a tile from K = 5120 to 6144
+    // (the lower half of H is 52 to 75 MB of the 126 MB L2), 16.5 at 7168, 17 to 18 from 8192 on.  With the line at
+    // 110 MB the splits that come out differently (K = 5504 to 7168) took as long or up to 14 % longer, 3000 tokens of
+    // K = 5632 4 % less.
     const double add = (double)K * (double)K * 2.0 > 60e6 ? 17000.0 : 12000.0;
     int best = 1;
     double best_cost = 0.0;

@@ -798,8 +798,9 @@ extern "C" int b200q_observe_mse(const void* W, int wdtype, int64_t N, int64_t K
 // serving process that has handed its whole memory budget to a KV-cache pool and re-calibrates
 // a layer in place, code running inside a framework callback where the caching allocator must
 // not be re-entered, or a C program that links this library without any allocator of its own.
-// For them the search's scratch (one flag per shrink candidate plus the stop step) lives in a
-// fixed array inside the library image instead of a caller-supplied buffer.
+// For them the search's scratch (one flag per shrink candidate plus the stop step, 4 KiB, and the 64 KiB
+// table of powers of bf16 errors) lives in fixed arrays inside the library image instead of a
+// caller-supplied buffer.  Calls that overlap on the GPU would share both: the caller keeps them on one stream.
 namespace b200q {
 namespace mse {
 

@@ -19,9 +19,9 @@
 // At rank 512 the C traffic per flop is a quarter and the launch count drops with it.
 // Why three tile widths: the operands of a chunk come from L2 at 64 B/clk and SM for TN = 256, 85 for
 // 128 and 128 for 64, so wide tiles run closer to the tensor pipe, narrow ones spread a small update
-// over more SMs; pick_width() takes whatever finishes its waves first.
+// over more SMs; pick_tiles() takes whatever finishes its waves first, CTA pairs of 256 x 256 among them.
 //
-// All mbarrier waits are bounded; no cluster launch, no multicast.
+// All mbarrier waits are bounded.  CTA pairs are clusters of two; no load is multicast.
 #include <cuda.h>
 
 #include <cstdlib>
@@ -667,7 +667,10 @@ static int pair_capacity() {
 // epilogue, about 20 cycles per column, is not hidden.
 static void pick_tiles(Params& p, int ctas, int pairs) {
   const double chunk[3] = {800.0, 1150.0, 1700.0};
-  const double pair_chunk = 1600.0;   // K = 14336: factor 13.2 -> 11.7 ms against single CTAs of 128 x 256
+  // Anything from 1000 to 1600 gives the same times; above 1700 pairs are never taken.  Without / with pairs, us: factor
+  // K = 4096 1198 / 1196, 8192 3340 / 3115, 14336 13353 / 11398; sweep 4096 x 4096 1035 / 984, 14336 x 4096 2829 / 2681,
+  // 4096 x 14336 6545 / 5879; 1024 rows and K = 2048 the same either way.
+  const double pair_chunk = 1600.0;
   const Job& j = p.j;
   const int chunks = (j.Kd + kChunkK - 1) / kChunkK;
   double best_cost = 0.0;

@@ -1014,8 +1014,12 @@ def _input_key(inp: torch.Tensor):
 
 
 # Batches of this many tokens go to the Hessian as they are: the update is bound by its MMAs from about there on, and the
-# copy into the staging buffer costs what the larger calls save (4096 tokens: K = 4096 59 us against 10 + 53, K = 2048 21
-# against 5 + 17, K = 1024 13 against 3 + 9; 2048 tokens: K = 4096 35 against 5 + 13 to 26).
+# copy into the staging buffer costs what the larger calls save.  Microseconds a batch, direct / staged:
+#   columns        256       1024      2048      4096      5632       8192       14336
+#   2048 tokens  10 / 8    11 / 8    14 / 13   34 / 34   67 / 59   136 / 115   433 / 365
+#   4096         10 / 9    11 / 11   19 / 21   56 / 65  112 / 116  248 / 229   759 / 748
+#   8192         10 / 10   15 / 17   31 / 39  108 / 127 199 / 250  526 / 531  1524 / 1542
+# One line for all widths is within 8 % of the better side at 4096 tokens, 15 % (1.5 us) below 512 columns.
 _DIRECT_TOKENS = 4096
 
 
