@@ -559,7 +559,7 @@ static int factor(float* H, float* const* Hs, int batch, int64_t K, int64_t ldh,
                   cudaStream_t st) {
   using tgemm::Job;
   using tgemm::Operand;
-  const int slice = Hs ? tgemm::kShortestSlice : tgemm::kLongSlice;   // (measured where they are defined)
+  const int slice = Hs ? tgemm::kShortSlice : tgemm::kLongSlice;   // (measured where they are defined)
   int rc;
 #define B200Q_RC(expr) do { rc = (expr); if (rc != B200Q_OK) return rc; } while (0)
   const int64_t lda = round_up(K, 32), rows = round_up(K, NB);

@@ -644,7 +644,7 @@ static int sweep(Params p, int sdtype, bool global, int batch, const float* cons
     if (p.W.one) j.C = p.W.one + i2;
     j.c_table = p.W.table; j.c_offset = i2; j.ldc = p.ldw; j.status = status;
     // a batch: error of the last of 2048 columns 2.6e-7 of its root mean square, with long slices 7.5e-7, by float32
-    // multiply-adds 4.1e-7; 64 weights of 768 x 2048: 4.05 ms, 3.91 with long slices.  The single weight keeps the long
+    // multiply-adds 4.1e-7; 64 weights of 768 x 2048: 4.0 ms, 3.8 with long slices.  The single weight keeps the long
     // ones (6.4e-7; 8.8e-7 when its products had rank 128).
     j.slice = p.W.table ? tgemm::kShortSlice : tgemm::kLongSlice;
     if (!side) {

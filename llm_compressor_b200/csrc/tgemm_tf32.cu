@@ -9,7 +9,7 @@
 //
 // Structure: persistent CTAs, each with a contiguous range of the tile list (128 x TN tiles).  Warp 0
 // streams 32-deep chunks of both operands (A_hi, A_lo, B_hi, B_lo) through a shared-memory ring by
-// TMA.  Warp 1 issues the MMAs and owns TMEM.  A contraction is cut into slices of 128, 32 or 16 terms:
+// TMA.  Warp 1 issues the MMAs and owns TMEM.  A contraction is cut into slices of 128 or 32 terms:
 // each slice accumulates in its own TMEM buffer (two, used in turn) and the epilogue (warps 4-11) adds
 // the slices in registers, so no tensor-core accumulation chain is longer than that whatever Kd is, and
 // C is read and written once per launch.
@@ -26,7 +26,6 @@
 
 #include <cstdlib>
 #include <mutex>
-#include <type_traits>
 
 #include "common.cuh"
 #include "tgemm_tf32.cuh"
@@ -35,7 +34,6 @@ namespace b200q {
 namespace tgemm {
 
 constexpr int kChunkK = 32;                          // fp32 elements per 128-byte row
-constexpr int kChunkSteps = kChunkK / 8;             // MMAs are 8 deep
 constexpr int kAPart = kTile * kChunkK * 4;          // A_hi or A_lo of a chunk: 16 KiB
 constexpr int kRingBytes = 196608;                   // 2, 3 or 4 stages for TN = 256, 128, 64
 constexpr int kEpiWarps = 8;                         // two per TMEM lane quarter, each half of the columns
@@ -283,50 +281,39 @@ tgemm_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ C
     uint32_t phase = 0;
     bool ok = true;
     constexpr uint32_t idesc = instr_desc(kRows, TN);
-    const int whole = j.slice < kChunkSteps ? 1 : j.slice / kChunkSteps;   // chunks of a slice
-    uint32_t sa = 0;                                                       // of the chunk
-    // steps [K0, K1) of the chunk; false if the accumulator did not become free
-    auto issue = [&](auto K0, auto K1, bool first, bool last) -> bool {
-      const int buf = slice & 1;
-      if (first && !mbar_wait(acce_bar(buf), (uint32_t)(((slice >> 1) & 1) ^ 1), &s_abort)) return false;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if (lane == 0) {
-        const uint32_t d_tmem = tmem_base + (uint32_t)(buf * TN), sb = sa + 2 * kAPart;
-        // K-major, 128-byte rows: 8-row groups 1024 bytes apart; a k-step of 8 tf32 is 32 bytes
-        auto mma = [&](uint32_t x, uint32_t y, uint32_t accumulate) {
-          if constexpr (PAIR) mma_tf32_pair(d_tmem, make_desc(x, 16, 1024), make_desc(y, 16, 1024), idesc, accumulate);
-          else mma_tf32(d_tmem, make_desc(x, 16, 1024), make_desc(y, 16, 1024), idesc, accumulate);
-        };
-        // the small products first: in a short slice they lose next to nothing, the sum being as small as they are
-#pragma unroll
-        for (int kk = K0; kk < K1; ++kk) {
-          mma(sa + kk * 32, sb + kBPart + kk * 32, (first && kk == K0) ? 0u : 1u);
-          mma(sa + kAPart + kk * 32, sb + kk * 32, 1u);
-        }
-#pragma unroll
-        for (int kk = K0; kk < K1; ++kk) mma(sa + kk * 32, sb + kk * 32, 1u);
-        if (K1 == kChunkSteps) {
-          if constexpr (PAIR) tc_commit_pair(empty_bar(stage));
-          else tc_commit(empty_bar(stage));
-        }
-        if (last) {
-          if constexpr (PAIR) tc_commit_pair(accf_bar(buf));
-          else tc_commit(accf_bar(buf));
-        }
-      }
-      __syncwarp();
-      if (last) ++slice;
-      return true;
-    };
-    const std::integral_constant<int, 0> begin;
-    const std::integral_constant<int, kChunkSteps / 2> middle;
-    const std::integral_constant<int, kChunkSteps> end;
     for (int64_t i = 0; i < count && ok; ++i) {
-      for (int c = 0; c < chunks && ok; ++c) {
+      for (int c = 0; c < chunks; ++c) {
+        const int buf = slice & 1;
+        const bool first = c % j.slice == 0, last = c % j.slice == j.slice - 1 || c == chunks - 1;
+        if (first && !mbar_wait(acce_bar(buf), (uint32_t)(((slice >> 1) & 1) ^ 1), &s_abort)) { ok = false; break; }
         if (!mbar_wait(full_bar(stage), phase, &s_abort)) { ok = false; break; }
-        sa = base + stage * kStageBytes;
-        if (j.slice < kChunkSteps) ok = issue(begin, middle, true, true) && issue(middle, end, true, true);
-        else ok = issue(begin, end, c % whole == 0, c % whole == whole - 1 || c == chunks - 1);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (lane == 0) {
+          const uint32_t d_tmem = tmem_base + (uint32_t)(buf * TN);
+          const uint32_t sa = base + stage * kStageBytes, sb = sa + 2 * kAPart;
+          // K-major, 128-byte rows: 8-row groups 1024 bytes apart; a k-step of 8 tf32 is 32 bytes
+          auto mma = [&](uint32_t x, uint32_t y, uint32_t accumulate) {
+            if constexpr (PAIR) mma_tf32_pair(d_tmem, make_desc(x, 16, 1024), make_desc(y, 16, 1024), idesc, accumulate);
+            else mma_tf32(d_tmem, make_desc(x, 16, 1024), make_desc(y, 16, 1024), idesc, accumulate);
+          };
+          // the small products first: in a short slice they lose next to nothing, the sum being as small as they are
+#pragma unroll
+          for (int kk = 0; kk < kChunkK / 8; ++kk) {
+            mma(sa + kk * 32, sb + kBPart + kk * 32, (first && kk == 0) ? 0u : 1u);
+            mma(sa + kAPart + kk * 32, sb + kk * 32, 1u);
+          }
+#pragma unroll
+          for (int kk = 0; kk < kChunkK / 8; ++kk) mma(sa + kk * 32, sb + kk * 32, 1u);
+          if constexpr (PAIR) {
+            tc_commit_pair(empty_bar(stage));
+            if (last) tc_commit_pair(accf_bar(buf));
+          } else {
+            tc_commit(empty_bar(stage));
+            if (last) tc_commit(accf_bar(buf));
+          }
+        }
+        __syncwarp();
+        if (last) ++slice;
         if (++stage == kStages) { stage = 0; phase ^= 1u; }
       }
     }
@@ -344,7 +331,7 @@ tgemm_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ C
     for (int64_t i = 0; i < count && ok; ++i, next_tile(p, b, tm, tn)) {
       const int row0 = tile_row(j, tm, kRows) + rank * kTile + q * 32, colw = tn * TN + half * kHalf;
       float sum[kHalf];
-      for (int c = 0; c < chunks * kChunkSteps; c += j.slice, ++slice) {
+      for (int c = 0; c < chunks; c += j.slice, ++slice) {
         const int buf = slice & 1;
         if (!mbar_wait(accf_bar(buf), (uint32_t)((slice >> 1) & 1), &s_abort)) { ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");

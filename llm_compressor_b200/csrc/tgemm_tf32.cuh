@@ -10,12 +10,13 @@ namespace tgemm {
 
 constexpr int kTile = 128;      // rows of a tile
 constexpr int kMaxDepth = 512;  // largest contraction of one launch
-// Steps of 8 terms that one tensor-core accumulation runs over, before float32 additions take the sums up.  The tensor core
-// cuts off at every addition, always downwards, so a long run drifts.  Relative error of a batch's factor against float64
-// at K = 2048 (8192 tokens): 5.6e-7 with 16 steps, 1.5e-7 with 4, 1.4e-7 with 2; elimination by float32 multiply-adds has
-// 1.7e-7.  Time of four such: 0.86, 0.93, 1.00 ms.  The single problem keeps 16 (K = 14336: 11.3 ms, 15.5 with 4): 4.2e-7
-// there, where rank-128 updates had 6.1e-7.
-constexpr int kLongSlice = 16, kShortSlice = 4, kShortestSlice = 2;
+// Chunks of 32 terms that one tensor-core accumulation runs over, before float32 additions take the sums up.  The tensor
+// core cuts off at every addition, always downwards, so a long run drifts.  Relative error of a batch's factors against
+// float64, 2048 columns of 8192 tokens: 5.6e-7 with four chunks, 1.5e-7 with one; elimination by float32 multiply-adds has
+// 1.7e-7 (768 columns of 4096: 3.5e-7, 1.1e-7, 1.5e-7).  Half a chunk gives 1.4e-7.  64 factors of K = 2048 take 8.3, 9.0
+// and 10.1 ms with four, one and half a chunk, 32 of K = 768 0.65, 0.68 and 0.71.  The single problem keeps four (K = 14336:
+// 11.3 ms, 15.5 with one): 4.2e-7 where rank-128 updates had 6.1e-7.
+constexpr int kLongSlice = 4, kShortSlice = 1;
 
 // One side of a product: float32 values x as hi = tf32_rn(x), lo = tf32_rn(x - hi), K-major (row r holds
 // the values of output row / column r), zero-padded to `ld`.  `rows`: rows the two arrays hold, reads
@@ -71,7 +72,7 @@ struct Job {
   int* status = nullptr;        // problem b: status + b * status_stride
   int status_stride = 0;
   int max_ctas = 0;             // 0: the whole GPU
-  int slice = kLongSlice;       // 8-deep steps that one tensor-core accumulation runs over
+  int slice = kLongSlice;       // chunks that one tensor-core accumulation runs over
 };
 int launch(const Job& j, cudaStream_t st);
 
