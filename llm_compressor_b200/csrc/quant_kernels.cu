@@ -512,7 +512,8 @@ __global__ void qparams_kernel(const void* __restrict__ mn, const void* __restri
 // statistics -> qparams in one pass, for one weight or a batch of weights of one shape
 // ========================================================================================
 // What min / max and qparams kernels do one after the other for a memoryless min-max observer, without the statistics
-// in between: bf16 weights in 16-byte pieces, the scale in the weight's dtype.  blockIdx.y = weight.
+// in between: bf16 weights in 16-byte pieces, the scale in the weight's dtype.  blockIdx.y = weight.  (By MinMax2, which
+// leaves a NaN out as the separate kernels do; RangeQ loses the chunk's other values with it.)
 struct StatJob {
   const void* one; const void* const* table;   // the weight, or a device array of them
   void* scale; void* zp;                       // [count][entries], contiguous
@@ -544,7 +545,7 @@ __global__ void __launch_bounds__(256) group_qparams_kernel(StatJob j, int N, in
 #pragma unroll
       for (int k = 0; k < R; ++k)
         raw[k] = live ? stream::ldg_stream(wrow + (int64_t)(c0 + k * L) * 8) : make_uint4(0, 0, 0, 0);
-      stream::RangeQ r;
+      stream::MinMax2 r;
       r.first(raw[0]);
 #pragma unroll
       for (int k = 1; k < R; ++k) r.add(raw[k]);
@@ -566,8 +567,8 @@ __global__ void __launch_bounds__(256) row_qparams_kernel(StatJob j, int64_t N, 
   const int64_t warps = (int64_t)gridDim.x * 8;
   for (int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); r < N; r += warps) {
     const __nv_bfloat16* row = W + r * ldw;
-    stream::RangeQ q;
-    q.umax = q.smax = 0;   // (zeros change nothing: the range is made to contain zero anyway)
+    stream::MinMax2 q;
+    q.mn = q.mx = __nv_bfloat162(0.0f, 0.0f);   // (zeros change nothing: the range is made to contain zero anyway)
     int64_t c = lane * 8;
     for (; c + 7 * 256 < K; c += 8 * 256) {
       uint4 raw[8];
@@ -601,7 +602,7 @@ __global__ void __launch_bounds__(256) span_qparams_kernel(StatJob j, int64_t N,
     for (int i = threadIdx.x; i < rows * cw; i += 256) {
       const int y = cw_log2 >= 0 ? i >> cw_log2 : i / cw, x = (i - y * cw) * 8;
       if (x >= cols) continue;
-      stream::RangeQ r;
+      stream::MinMax2 r;
       r.first(stream::ldg_stream(base + (int64_t)y * ldw + x));
       float l, h;
       r.finish(l, h);

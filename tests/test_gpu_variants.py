@@ -318,3 +318,22 @@ def test_factor_reports_the_first_bad_pivot(K, column, value):
     H[column, column] = value
     status = ops.gptq_factor_async(H).tolist()
     assert status == [_lib.NOT_POSITIVE_DEFINITE, K - column, 0, 0]   # (columns are counted in reversed order)
+
+
+@pytest.mark.parametrize("scheme", ["W4A16", "W4A16_ASYM", "W8A16", "FP8_DYNAMIC", "FP8_BLOCK", "MXFP4A16", "MXFP8A16"])
+@pytest.mark.parametrize("N,K", [(8, 2048), (2400, 384), (130, 256)])
+def test_one_launch_parameters_of_unusual_values(scheme, N, K):
+    """Statistics and parameters in one launch leave a NaN of either sign out as the two launches do."""
+    args = preset_name_to_scheme(scheme, ["Linear"]).weights
+    w = synth_weight(N, K, seed=N + K)
+    nan, inf = float("nan"), float("inf")
+    for row, col, value in ((1, 5, nan), (2, 6, -nan), (3, K - 1, -nan), (4, 0, inf), (5, 7, -inf), (6, 9, 3.3e38), (6, 10, nan)):
+        w[row, col] = value
+    w[0, 16:180] = -nan
+    w[7] = torch.where(w[7] > 0, torch.tensor(-0.0, dtype=w.dtype), w[7])
+    w = w.to(DEV)
+    scale, zp = ops.qparams(*ops.observe_minmax(w, args), args)
+    one = ops.minmax_qparams(w, args)
+    many = ops.minmax_qparams([w.clone(), w], args)
+    for s, z in (one, (many[0][0], many[1][0]), (many[0][1], many[1][1])):
+        assert bits_equal(s, scale) and bits_equal(z, zp)
