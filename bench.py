@@ -45,10 +45,10 @@ GROUP_K = {"attn_in": HIDDEN, "o_in": HIDDEN, "mlp_in": HIDDEN, "down_in": INTER
 # K = 14336 (four token splits per tile: 8.7 GB read, 1.6 GB written).  A step runs 96 launches of
 # width 4096 and 32 of width 14336.
 SYRK_TRAFFIC = {
-    "K4096": 0.62e9, "K14336": 10.3e9,
-    "per_launch_weighted": (96 * 0.62e9 + 32 * 10.3e9) / 128,
-    "note": "mean bytes per launch over a step's 96 K=4096 launches (0.62e9 each, algorithmic 0.34e9) and 32 "
-            "K=14336 launches (10.3e9 each, algorithmic 1.76e9): X panels are re-read by every band of 8 block "
+    "K4096": 0.61e9, "K14336": 11.4e9,
+    "per_launch_weighted": (96 * 0.61e9 + 32 * 11.4e9) / 128,
+    "note": "mean bytes per launch over a step's 96 K=4096 launches (0.61e9 each, algorithmic 0.34e9) and 32 "
+            "K=14336 launches (11.4e9 each, algorithmic 1.76e9): X panels are re-read by every band of 8 block "
             "rows and the partial tiles of the four token splits are added into H; DRAM stays at 19-27 % of its "
             "peak, the kernel is tensor bound",
 }
