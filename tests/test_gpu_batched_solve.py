@@ -342,3 +342,25 @@ def test_noted_status_word_is_reported_once():
         _lib.check(lib.b200q_note_wait_status(torch.full((1,), word, dtype=torch.int32, device=DEV).data_ptr(),
                                               _lib.stream_ptr()), "note")
         assert lib.b200q_take_wait_status() == expected and lib.b200q_take_wait_status() == 0
+
+
+# one problem: `limit` is the error of the same solve with rank-128 tensor-core updates and float32 multiply-adds inside a block
+@pytest.mark.parametrize("K,tokens,limit", [(256, 600, 7.3e-7), (768, 4096, 4.3e-7), (2048, 8192, 6.0e-7), (4096, 9000, 1.28e-6)])
+def test_factor_is_as_accurate_as_rank_128_updates(K, tokens, limit):
+    H, ref = _spd_factor64(K, tokens)
+    assert ops.gptq_factor(H) == 0
+    assert float((H.double() - ref).norm() / ref.norm()) <= limit
+
+
+@pytest.mark.parametrize("N,K,tokens,limit", [(1001, 256, 600, 3.7e-7), (1001, 520, 1500, 9.2e-7), (6000, 1160, 6933, 4.8e-7),
+                                              (1001, 4096, 9000, 7.0e-7)])
+def test_sweep_is_as_accurate_as_rank_128_updates(N, K, tokens, limit):
+    _, ref = _spd_factor64(K, tokens)
+    U = ref.float().contiguous()
+    U[:-1] *= 2.0 ** 20
+    w = (torch.randn(N, K, generator=torch.Generator(device=DEV).manual_seed(N), device=DEV) * 0.02).bfloat16()
+    last = torch.linalg.solve_triangular(U.double(), w.double(), upper=True, left=False)[:, -1].abs()
+    scale = torch.full((N, 1), 1e4, device=DEV).bfloat16()
+    losses = ops.gptq_sweep(w.float(), U, scale, None, args_from(SCHEMES["W8_CHANNEL"]))
+    error = (2.0 * losses.double()).sqrt() - last
+    assert float(error.pow(2).mean().sqrt() / last.pow(2).mean().sqrt()) <= limit
