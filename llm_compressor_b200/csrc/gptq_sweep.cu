@@ -2,7 +2,7 @@
 //
 // Rows of W are independent and the columns of a row form one dependent chain: quantise column i, divide the error
 // by U[i,i], subtract its multiple of U[i, i+1:] from the rest of the row.  The columns are taken in superblocks of
-// up to 512.  Inside one, a CTA carries 32 rows through all columns with everything in shared memory
+// up to 512.  Inside one, a CTA carries 32 or 64 rows through all columns without touching device memory for them
 // (sweep_block_kernel); between superblocks the rest of the matrix takes W[:, after] -= Err * U[block, after] as one
 // fp32-accurate tensor-core product (tgemm).  What the reference calls its block size only orders float32 operations
 // and does not change the result otherwise, so it does not decide the split here.
@@ -20,13 +20,17 @@ namespace sweep {
 
 constexpr int kMaxBlock = 128;               // largest block size callers may ask for
 constexpr size_t kSweepHeaderBytes = 256;    // status word at the start of the workspace
-constexpr int kRows = 32;                    // rows of a CTA: a lane each
-constexpr int kMicro = 16;                   // columns a lane keeps in registers at a time
-// 12 warps where a CTA has its SM to itself, 8 where two share one
-constexpr int warps_of(int superblock) { return superblock == 512 ? 12 : 8; }
-constexpr int WLD = kRows + 4, ELD = kRows + 8;   // columns of W and of the errors in shared memory: the strides
-                                                  // make the MMA fragments' accesses conflict-free
-__host__ __device__ constexpr int u_stride(int superblock) { return superblock + 8; }   // likewise
+constexpr int kMicro = 16;                   // columns whose errors make one operand of the MMAs
+constexpr int kHalf = 8;                     // columns the chain takes at a time
+constexpr int kSlots = 4;                    // micro-blocks whose parameters and band of U are in shared memory
+constexpr int kBlockCols = 128;              // columns of W that one MMA corrects
+constexpr int kRowBytes = 4 * kMicro;        // operand row of a micro-block: 16 hi and 16 lo halves
+constexpr int kTileBytes = kBlockCols * kRowBytes;   // a block's columns of U for a micro-block's errors
+constexpr int kLag = 3;                      // errors of micro-block m reach columns from m + kLag on by MMAs
+constexpr int kBandCols = kLag * kMicro;     // columns of U that chain and feeder need of a micro-block's rows (8 rows at
+                                             // most reach 5 half-blocks on)
+constexpr int kErrSlots = 4;                 // micro-blocks whose errors are kept
+constexpr int kBandFloats = kMicro * kBandCols + kMicro;   // and the reciprocals of the pivots
 
 // One pointer per operand, or (table set) a device array with one per problem.
 template <class T> struct Ptr {
@@ -44,22 +48,46 @@ struct Params {
   float* err_hi; float* err_lo; int64_t lde, err_batch;   // operand form of the superblock's errors (null: nothing after it)
   int i1, sb;                                             // superblock: first column, width
   int sdtype;                                             // of the scales
+  const unsigned char* tiles; int64_t tiles_batch;        // operand form of U[i1 : i1 + sb, i1 : i1 + sb], one a factor
+  const int32_t* u_index;                                 // factor of problem b (null: one each)
   int* status;                                            // set if a bounded wait expires
 };
 
-__host__ __device__ constexpr size_t smem_bytes(int superblock) {
-  return (size_t)(3 * kMicro * u_stride(superblock)   // rows of U of three micro-blocks
-                  + 2 * 4 * kMicro * kRows            // parameters of two micro-blocks
-                  + 2 * superblock                    // 1 / U[i,i], parameter column
-                  + 32                                // one parameter column for all of a micro-block?
-                  + 2 * kMicro * ELD                  // errors of two micro-blocks
-                  + superblock * WLD) * sizeof(float);   // W, column-major
-}
+// What a CTA of ROWS rows and SBLK columns holds, and where.
+template <int ROWS, int SBLK> struct Shape {
+  static constexpr int kChains = ROWS / 32;            // chain warps: a lane per row
+  static constexpr int kBlocks = SBLK / kBlockCols;
+  static constexpr int kHelpers = 4 * kBlocks;         // warps with 32 columns each
+  // first warp of each role; two feeders per chain, one of each other kind of 32 rows, one for the MMAs and one for
+  // the parameters
+  static constexpr int kErrors = ROWS == 32 ? 3 : 2, kFeeder = ROWS == 32 ? 1 : 4, kMma = ROWS == 32 ? 4 : 8,
+                       kOut = kMma + 1, kParams = kOut + kChains;
+  static constexpr int kFirstHelper = ROWS == 32 ? 8 : 12;
+  static constexpr int kThreads = 32 * (kFirstHelper + kHelpers);
+  static constexpr int kStages = 3, kStageBytes = kBlocks * kTileBytes;   // ring of the tiles of a micro-block's errors
+  static constexpr int kErrBytes = ROWS * kRowBytes;   // errors of a micro-block as operand
+  static constexpr int kWld = ROWS + 4;                // stride of a column of W: float4 accesses conflict-free
+  static constexpr int kRing = 0, kErr = kRing + kStages * kStageBytes, kW = kErr + 2 * kErrBytes,
+                       kE = kW + SBLK * kWld * 4, kPar = kE + kErrSlots * kMicro * ROWS * 4,
+                       kZ = kPar + kSlots * kMicro * ROWS * 8, kBand = kZ + kSlots * kMicro * ROWS * 4,
+                       kSe = kBand + kSlots * kBandFloats * 4,
+                       kNext = kSe + 4 * ROWS * 4, kEnd = kNext + 2 * kHalf * ROWS * 4;
+  static constexpr size_t kSmem = kEnd + 1024;
+  static constexpr int kMicros = SBLK / kMicro;
+};
+static_assert(Shape<32, 512>::kSmem <= 232448 - 2048 && Shape<64, 256>::kSmem <= 232448 - 2048, "shared memory");
+// Registers a thread of the warpgroups, as many as at the launch: 32 rows 768 threads at 80 (160 + 64 + 4 * 64), 64 rows 640 at
+// 96 (144 + 64 + 48 + 2 * 112).
+template <int ROWS> struct Regs {
+  static constexpr int kChain = ROWS == 32 ? 160 : 144, kFeeder = 64, kOther = ROWS == 32 ? 64 : 48, kHelper = ROWS == 32 ? 64 : 112;
+};
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void bulk_copy(float* dst, const float* src, uint32_t bytes, uint32_t bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(bar) : "memory");
+__device__ __forceinline__ void bar_init(uint32_t bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ bool bar_ready(uint32_t bar, uint32_t parity) {
   uint32_t ok;
@@ -68,8 +96,153 @@ __device__ __forceinline__ bool bar_ready(uint32_t bar, uint32_t parity) {
       : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
   return ok != 0;
 }
-__device__ __forceinline__ void fma2(uint64_t& d, uint64_t a, uint64_t b) {
-  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+// (try_wait above may suspend the thread for thousands of cycles, this one never does)
+__device__ __forceinline__ bool bar_test(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred P1;\n\tmbarrier.test_wait.parity.shared::cta.b64 P1, [%1], %2;\n\tselp.b32 %0, 1, 0, P1;\n\t}"
+      : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+  return ok != 0;
+}
+// After a wait has run out nothing waits any more: the CTA ends with garbage and the status says so.
+__device__ __forceinline__ void bar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  if (bar_ready(bar, parity)) return;
+  const long long t0 = clock64();
+  while (!bar_ready(bar, parity)) {
+    if (*abort_flag) return;
+    if (clock64() - t0 > 4000000000LL) { *abort_flag = 1; return; }
+  }
+}
+// the same for warps that nobody waits for soon: they leave the issue slots and the barrier unit to the others
+__device__ __forceinline__ void bar_sleep(uint32_t bar, uint32_t parity, unsigned ns, volatile int* abort_flag) {
+  if (bar_test(bar, parity)) return;
+  const long long t0 = clock64();
+  while (!bar_test(bar, parity)) {
+    __nanosleep(ns);
+    if (*abort_flag) return;
+    if (clock64() - t0 > 4000000000LL) { *abort_flag = 1; return; }
+  }
+}
+// the same without suspending: for the few warps whose reaction the chain waits for
+__device__ __forceinline__ void bar_spin(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  for (uint32_t tries = 0; !bar_test(bar, parity);)
+    if ((++tries & 1023u) == 0 && (*abort_flag || tries > (1u << 26))) { *abort_flag = 1; return; }
+}
+__device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void tc_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                         uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+}
+// K-major operand in rows of 64 bytes, 64-byte swizzle: groups of eight rows are 512 bytes apart
+__device__ __forceinline__ uint64_t make_desc(uint32_t saddr) {
+  return (uint64_t)((saddr >> 4) & 0x3FFFu) | (uint64_t)1 << 16 | (uint64_t)(512 >> 4) << 32 | (uint64_t)1 << 46 |
+         (uint64_t)4 << 61;
+}
+// D fp32, A / B f16, both K-major, M = 128
+__host__ __device__ constexpr uint32_t instr_desc(int n) {
+  return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((128u >> 4) << 24);
+}
+// ---- operands of the products inside a superblock: float32 values as two halves
+// x * 2^k = hi + lo with |x| * 2^k < 2^15: eleven bits each, as the tf32 halves of tgemm have, at half their bytes and
+// twice their rate.  k belongs to a row of U^T (a column of the superblock) or to a row of a micro-block's errors, so
+// that values down to 2^-18 of the row's largest keep all 22 bits, and smaller ones are off by 2^-40 of it at most.
+// (float of 2^k, exponent field of the row's largest value) -> the scale, its inverse
+__device__ __forceinline__ void row_scale(float largest, float& scale, float& inverse) {
+  int k = 141 - (int)(__float_as_uint(largest) >> 23);
+  k = min(max(k, -112), 126);
+  scale = __uint_as_float((uint32_t)(127 + k) << 23);
+  inverse = __uint_as_float((uint32_t)(127 - k) << 23);
+}
+// the hi halves of two neighbours and their lo halves
+__device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi, uint32_t& lo) {
+  const __half2 h = __floats2half2_rn(a, b);
+  const float2 f = __half22float2(h);
+  const __half2 l = __floats2half2_rn(a - f.x, b - f.y);
+  hi = *reinterpret_cast<const uint32_t*>(&h);
+  lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+
+// U[i1 : i1 + sb, i1 : i1 + sb] as the tiles that the sweep copies into shared memory: tile (micro-block m, block b) holds
+// for each of the block's 128 columns 16 hi and 16 lo halves of the micro-block's rows of U, in 64-byte rows swizzled as
+// the MMA reads them.  Behind the tiles the inverse scale of every column, and then for every micro-block its rows of U
+// from the diagonal on (the identity beyond sb) and the reciprocals of its pivots.  A CTA takes 32 columns.
+constexpr int kTileThreads = 256;
+constexpr int64_t band_offset(int sblk) { return (int64_t)(sblk / kMicro) * (sblk / kBlockCols) * kTileBytes + sblk * 4; }
+constexpr int64_t tiles_bytes(int sblk) { return band_offset(sblk) + sblk / kMicro * kBandFloats * 4; }   // of one factor
+template <int SBLK>
+__global__ void __launch_bounds__(kTileThreads) square_tiles_kernel(Ptr<const float> Us, int64_t ldu, int i1, int sb,
+                                                                   unsigned char* tiles, int64_t batch_bytes) {
+  chain_wait();
+  chain_go();
+  extern __shared__ float stage[];   // [32][SBLK + 1]
+  __shared__ float s_max[kTileThreads / 32][32];
+  constexpr int kWarps = kTileThreads / 32, kBlocks = SBLK / kBlockCols;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = blockIdx.x * 32 + lane;
+  const float* U = Us.at(blockIdx.y) + (int64_t)i1 * ldu + i1;
+  tiles += blockIdx.y * batch_bytes;
+  float v[SBLK / kWarps], largest = 0.0f;
+#pragma unroll
+  for (int i = 0; i < SBLK / kWarps; ++i) {
+    const int p = warp + i * kWarps;
+    v[i] = (p <= c && c < sb) ? U[(int64_t)p * ldu + c] : 0.0f;
+  }
+  float* bands = reinterpret_cast<float*>(tiles + band_offset(SBLK));
+#pragma unroll
+  for (int i = 0; i < SBLK / kWarps; ++i) {
+    const int p = warp + i * kWarps, c0 = p / kMicro * kMicro;
+    largest = fmaxf(largest, fabsf(v[i]));
+    const float x = (p == c && c >= sb) ? 1.0f : v[i];
+    if (c >= c0 && c < c0 + kBandCols) bands[p / kMicro * kBandFloats + (p - c0) * kBandCols + c - c0] = x;
+    if (c == p) bands[p / kMicro * kBandFloats + kMicro * kBandCols + p - c0] = __frcp_rn(x);
+  }
+  s_max[warp][lane] = largest;
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kWarps; ++k) largest = fmaxf(largest, s_max[k][lane]);
+  float scale, inverse;
+  row_scale(largest, scale, inverse);
+  if (warp == 0) reinterpret_cast<float*>(tiles + SBLK / kMicro * kBlocks * kTileBytes)[c] = inverse;
+#pragma unroll
+  for (int i = 0; i < SBLK / kWarps; ++i) stage[lane * (SBLK + 1) + warp + i * kWarps] = v[i] * scale;
+  __syncthreads();
+  const int b = c / kBlockCols, row = c % kBlockCols;
+  for (int m = warp; (m + kLag) * kMicro <= c; m += kWarps) {
+    const float* x = stage + lane * (SBLK + 1) + m * kMicro;
+    unsigned char* d = tiles + (int64_t)(m * kBlocks + b) * kTileBytes + row * kRowBytes;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      uint32_t hi[4], lo[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) split_pair(x[8 * j + 2 * k], x[8 * j + 2 * k + 1], hi[k], lo[k]);
+      *reinterpret_cast<uint4*>(d + ((j ^ ((row >> 1) & 3)) << 4)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+      *reinterpret_cast<uint4*>(d + (((j + 2) ^ ((row >> 1) & 3)) << 4)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    }
+  }
+}
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
 }
 __device__ __forceinline__ uint64_t pair(float lo, float hi) {
   uint64_t r;
@@ -85,18 +258,25 @@ __device__ __forceinline__ void unpair(uint64_t v, float& lo, float& hi) {
 // the product and the reference's division cannot matter.  Whether they are equal is not waited for column by column:
 // a micro-block whose flags show a difference anywhere (some per mille of them) is swept again by the exact rules.
 constexpr float kMargin = 0x1p-21f;   // > the 2^-22 by which reciprocal, product and division can differ in all
+constexpr float kMagic = 12582912.0f; // 1.5 * 2^23: a float32 sum with it is rounded to the nearest integer, ties to even
 
-template <int KIND>
-__device__ __forceinline__ float code_of(float v, float qmin, float qmax) {
-  v = fminf(fmaxf(v, qmin), qmax);
-  if constexpr (KIND == kInt) {
-    return (v + 12582912.0f) - 12582912.0f;   // 1.5 * 2^23: rounds to nearest even (the sign of a zero is put back later)
-  } else if constexpr (KIND == kFp8) {
-    return e4m3_round(v);
+// code of x * r + zz (the sign of a zero is put back later)
+template <int KIND, bool ZP>
+__device__ __forceinline__ float code_of(float x, float r, float zz, float qmin, float qmax) {
+  if constexpr (KIND == kInt && !ZP) {
+    // product and rounding to an integer in one: beyond 2^22, where the sum's ulp grows, only the clamp matters
+    return fminf(fmaxf(fmaf(x, r, kMagic), kMagic + qmin), kMagic + qmax) - kMagic;
   } else {
-    uint32_t h;   // through the hardware's E2M1 pair and back
-    asm("{\n\t.reg .b8 b;\n\tcvt.rn.satfinite.e2m1x2.f32 b, %1, %1;\n\tcvt.rn.f16x2.e2m1x2 %0, b;\n\t}" : "=r"(h) : "f"(v));
-    return __half2float(__ushort_as_half((unsigned short)(h & 0xFFFFu)));
+    const float v = fminf(fmaxf(fmaf(x, r, zz), qmin), qmax);
+    if constexpr (KIND == kInt) {
+      return (v + kMagic) - kMagic;
+    } else if constexpr (KIND == kFp8) {
+      return e4m3_round(v);
+    } else {
+      uint32_t h;   // through the hardware's E2M1 pair and back
+      asm("{\n\t.reg .b8 b;\n\tcvt.rn.satfinite.e2m1x2.f32 b, %1, %1;\n\tcvt.rn.f16x2.e2m1x2 %0, b;\n\t}" : "=r"(h) : "f"(v));
+      return __half2float(__ushort_as_half((unsigned short)(h & 0xFFFFu)));
+    }
   }
 }
 // bf16 rounding with the result already in place as a float
@@ -115,469 +295,576 @@ __device__ __forceinline__ float dequant(float q, float s, float z) {
   return SB ? bf16_in_place(q) : q;
 }
 
-// three tf32 MMAs per product of hi / lo splits, as in tgemm
-__device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) {
-  hi = (__float_as_uint(x) + 0x1000u) & 0xFFFFE000u;
-  lo = (__float_as_uint(x - __uint_as_float(hi)) + 0x1000u) & 0xFFFFE000u;
-}
-__device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
-  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
-}
+// What bounds it: the chain of columns, one warp of 32 rows.  Eight columns take it some 600 cycles on its own (the
+// dependent instructions of a column are about 45, the 26 16-byte loads of U and 56 packed FMAs of its half-block the
+// rest), and 900 to 1100 beside the other roles.  What it costs most is instruction fetch: all roles together ran from
+// 35 KB of unrolled code at first, 3000 fetches a CTA went to the GPC's cache and the kernel took 140 us for 4096 rows x
+// 512 columns; with eight columns unrolled instead of sixteen and short loops everywhere else it takes 64 (81 when
+// warp-level MMAs on 16-column tiles in shared memory did the corrections, ncu, warm caches; the whole 4096 x 4096 sweep
+// 0.92 ms, 1.04 before).  So: nothing is unrolled further than the registers demand.
+//
+// Roles, all of them warps of one CTA that hand over by one-shot mbarriers, so that nobody waits for all:
+//   chain    codes and errors of eight columns; applies them to these columns and sums what they are to the next eight
+//   feeders  give the eight after these the errors of up to four half-blocks (even and odd ones a warp each)
+//   errors   turn the errors of 16 columns into an MMA operand
+//   MMA      U^T[128 columns, 16] E[16, rows] for everything from kLag micro-blocks on, accumulators in TMEM (two sets)
+//   helpers  hold the columns of W in registers (a lane each, all rows), add the products to them, hand them over
+//            when their turn comes and write the codes out when the chain is past, while it goes on
+//   out      errors out as operand of the trailing product, losses;  params  scales and zero points, copies of U
+// U comes as tiles that one bulk copy brings in (as 64-byte rows of a tensor map it arrived at 18 bytes a clock and SM).
+template <int ROWS, int SBLK, bool SB, int KIND, bool ZP>
+__global__ void __launch_bounds__(Shape<ROWS, SBLK>::kThreads, 1)
+sweep_block_kernel(const __grid_constant__ Params p) {
+  using S = Shape<ROWS, SBLK>;
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* sm = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  float* sW = reinterpret_cast<float*>(sm + S::kW);         // [SBLK][kWld]
+  float* sE = reinterpret_cast<float*>(sm + S::kE);         // [kErrSlots][kMicro][ROWS] negated errors
+  float2* sPar = reinterpret_cast<float2*>(sm + S::kPar);   // [kSlots][kMicro][ROWS] scale, 1 / scale
+  float* sZ = reinterpret_cast<float*>(sm + S::kZ);         // [kSlots][kMicro][ROWS] zero point
+  float* sBand = reinterpret_cast<float*>(sm + S::kBand);   // [kSlots][kMicro][kBandCols] U[c0 + t, c0 ...], [kMicro] 1 / U[i,i]
+  float* sSe = reinterpret_cast<float*>(sm + S::kSe);       // [4][ROWS] inverse scales of a micro-block's errors
+  float* sNext = reinterpret_cast<float*>(sm + S::kNext);   // [2][kHalf][ROWS] columns that the chain takes next
+  // One-shot barriers.  Of a micro-block m: parameters and band are there; its columns have the errors up to m - kLag
+  // (helpers); its errors are there as operand; its errors are out.  Of half a micro-block n: its columns have the errors up to n - 2 (feeder);
+  // its errors and codes are there (chain).
+  __shared__ __align__(8) uint64_t s_par[S::kMicros], s_raw[S::kMicros], s_opr[S::kMicros], s_out[S::kMicros], s_ready[2 * S::kMicros],
+      s_done[2 * S::kMicros];
+  __shared__ __align__(8) uint64_t s_full[S::kStages], s_empty[S::kStages];
+  __shared__ __align__(8) uint64_t s_accf[2][S::kBlocks], s_acce[2][S::kBlocks];
+  __shared__ int s_odd[S::kChains][kSlots];                        // some scale is outside the range the low / high test covers
+  __shared__ uint32_t s_tmem;
+  __shared__ volatile int s_abort;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-// A micro-block's errors as MMA operand: rows of the CTA x columns of the micro-block, [row tile][k step]
-struct ErrFrag { uint32_t hi[2][2][4], lo[2][2][4]; };
-// `upto12`: only the first twelve columns exist yet
-__device__ __forceinline__ void load_errors(const float* e, int lane, bool upto12, ErrFrag& f) {
-  const float* ei = e + (lane & 3) * ELD + (lane >> 2);
-#pragma unroll
-  for (int y = 0; y < 2; ++y)
-#pragma unroll
-    for (int ks = 0; ks < 2; ++ks)
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const bool out = upto12 && ks == 1 && k >= 2;
-        split_tf32(out ? 0.0f : ei[(ks * 8 + (k >> 1) * 4) * ELD + y * 16 + (k & 1) * 8], f.hi[y][ks][k], f.lo[y][ks][k]);
-      }
-}
-// W[32 rows, 16 columns] -= E[32, 16] U[16, 16 columns]; `w`, `u`: the first of the columns
-template <int ULD>
-__device__ __forceinline__ void apply_errors(const ErrFrag& f, const float* u, float* w, int lane) {
-  float* o = w + 2 * (lane & 3) * WLD + (lane >> 2);
-  const float* ub = u + (lane & 3) * ULD + (lane >> 2);
-  float old[2][2][4], acc[2][2][4] = {}, part[2][2][4] = {};   // [row tile][column tile]
-#pragma unroll
-  for (int y = 0; y < 2; ++y)
-#pragma unroll
-    for (int x = 0; x < 2; ++x)
-#pragma unroll
-      for (int k = 0; k < 4; ++k) old[y][x][k] = o[(x * 8 + (k & 1)) * WLD + y * 16 + (k >> 1) * 8];
-#pragma unroll
-  for (int ks = 0; ks < 2; ++ks) {
-    uint32_t bh[2][2], bl[2][2];
-#pragma unroll
-    for (int x = 0; x < 2; ++x)
-#pragma unroll
-      for (int k = 0; k < 2; ++k) split_tf32(ub[(ks * 8 + k * 4) * ULD + x * 8], bh[x][k], bl[x][k]);
-#pragma unroll
-    for (int y = 0; y < 2; ++y)
-#pragma unroll
-      for (int x = 0; x < 2; ++x) mma_tf32(acc[y][x], f.hi[y][ks], bh[x]);
-#pragma unroll
-    for (int y = 0; y < 2; ++y)
-#pragma unroll
-      for (int x = 0; x < 2; ++x) mma_tf32(part[y][x], f.hi[y][ks], bl[x]);
-#pragma unroll
-    for (int y = 0; y < 2; ++y)
-#pragma unroll
-      for (int x = 0; x < 2; ++x) mma_tf32(part[y][x], f.lo[y][ks], bh[x]);
-  }
-#pragma unroll
-  for (int y = 0; y < 2; ++y)
-#pragma unroll
-    for (int x = 0; x < 2; ++x)
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-        o[(x * 8 + (k & 1)) * WLD + y * 16 + (k >> 1) * 8] = old[y][x][k] - (acc[y][x][k] + part[y][x][k]);
-}
-
-// What bounds it: the chain of columns.  Its dependent instructions (product with 1 / s, clamp, round, dequantise,
-// difference, product with the reciprocal pivot, correction of the next column) come to some 60 cycles a column by their
-// latencies; measured it takes 308 (512 columns in 86.5 us at 1.82 GHz, 4096 rows), and where the rest goes has not been
-// measured.  So one warp of the CTA does nothing but the chain: 16 columns at a time in registers, a lane per row.  Others apply a finished micro-block's
-// 16 errors to the columns two micro-blocks on and later as warp-level tensor-core products (a float32 FMA formulation
-// spends its time on the broadcast loads of U: 480 cycles a column against the chain's own), taking tasks of 16 columns
-// from a counter.  The columns next in line take the first twelve errors from a warp that waits for them while the chain
-// is on the last four, and those four from the chain warp.  Duties beside that: the warps that share the chain warp's
-// scheduler ask for rows of U by bulk copies (as per-thread copies they block the warps that issue them: all CTAs want
-// the same rows at the same time), and take tasks only while these, not the chain, decide; warp 5 fetches parameters,
-// warp 6 writes the errors out as the operand of the trailing product.  One barrier per micro-block.  Every role is a
-// latency-bound stream of instructions, a quarter of its stalls instruction fetch, hence short loops rather than
-// unrolled code off the chain.
-template <int SBLK, bool SB, int KIND, bool ZP>
-__global__ void __launch_bounds__(32 * warps_of(SBLK), SBLK == 512 ? 1 : 2) sweep_block_kernel(const __grid_constant__ Params p) {
-  const float qmin = p.qr.qmin, qmax = p.qr.qmax;
-  chain_wait();
-  extern __shared__ __align__(16) float sm[];
-  constexpr int ULD = u_stride(SBLK);
-  constexpr int NW = warps_of(SBLK), NT = 32 * NW;
-  constexpr int kNextWarp = NW > 8 ? 9 : 1;            // brings the next micro-block's columns up to date
-  constexpr int kHead = 12;                            // its share of a micro-block's errors
-  float* sU = sm;                                      // [3][kMicro][ULD]
-  float* sP = sU + 3 * kMicro * ULD;                   // [2][scale, low and high 1 / scale, zero point][kMicro][kRows]
-  float* sRd = sP + 2 * 4 * kMicro * kRows;            // [SBLK]
-  int* sGrp = reinterpret_cast<int*>(sRd + SBLK);      // [SBLK]
-  int* sSame = sGrp + SBLK;                            // [32]
-  float* sE = sRd + 2 * SBLK + 32;                     // [2][kMicro][ELD]
-  float* sW = sE + 2 * kMicro * ELD;                   // [SBLK][WLD]
-  __shared__ int s_odd;                                // some scale is outside the range the low / high test covers
-  __shared__ int s_next[2];                            // next task of the helpers
-  __shared__ __align__(8) uint64_t s_bar[3];           // rows of U of a micro-block have arrived
-  const int job = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int sb = p.sb, micros = (sb + kMicro - 1) / kMicro;
-  float* __restrict__ W = p.W.at(job) + p.i1;
-  const float* __restrict__ U = p.U.at(job);
-  if (U) U += (int64_t)p.i1 * p.ldu + p.i1;
-  const int64_t row0 = (int64_t)blockIdx.x * kRows, row = row0 + lane;
-  const bool live = row < p.N;
-  const bool bulk = U && ((p.ldu & 3) == 0) && ((((uintptr_t)U) & 15) == 0) && (sb % kMicro) == 0;
-  const bool vecw = ((p.ldw & 3) == 0) && ((((uintptr_t)W) & 15) == 0) && (sb & 3) == 0;
-  // `ROWS` rows from t0 on of U's micro-block m, columns from its own first one on (columns beyond sb are zero).
-  // Called by whole warps; with bulk copies one lane of each works, the one with t0 = 0 announces the bytes.
-  auto fetch_u = [&](int m, int t0, auto ROWS) {
-    float* dst = sU + (m % 3) * kMicro * ULD;
-    const int c0 = m * kMicro, c_end = micros * kMicro;
-    if (bulk) {
-      if (lane == 0) {
-        const uint32_t bytes = (uint32_t)(c_end - c0) * 4, bar = smem_u32(&s_bar[m % 3]);
-        if (t0 == 0)
-          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes * kMicro) : "memory");
-#pragma unroll
-        for (int t = 0; t < ROWS; ++t)
-          bulk_copy(dst + (t0 + t) * ULD + c0, U + (int64_t)(c0 + t0 + t) * p.ldu + c0, bytes, bar);
-      }
-      return;
+  if (tid == 0) {
+    for (int m = 0; m < S::kMicros; ++m) {
+      bar_init(smem_u32(&s_par[m]), 2); bar_init(smem_u32(&s_raw[m]), 1); bar_init(smem_u32(&s_opr[m]), S::kChains);
+      bar_init(smem_u32(&s_out[m]), S::kChains);
     }
-#pragma unroll 1
-    for (int t = t0; t < t0 + ROWS; ++t) {
-      const int i = c0 + t;
-#pragma unroll 1
-      for (int c = c0 + lane; c < c_end; c += 32) {
-        float v = (i == c) ? 1.0f : 0.0f;
-        if (U) v = (i < sb && c < sb) ? U[(int64_t)i * p.ldu + c] : 0.0f;
-        dst[t * ULD + c] = v;
-      }
+    for (int n = 0; n < 2 * S::kMicros; ++n) {
+      bar_init(smem_u32(&s_ready[n]), S::kChains); bar_init(smem_u32(&s_done[n]), S::kChains);
     }
-  };
-  // a warp of twelve asks for half of a micro-block's rows, of eight for all
-  constexpr std::integral_constant<int, NW == 12 ? kMicro / 2 : kMicro> kAskRows;
-  auto wait_u = [&](int m) {
-    if (!bulk) return;
-    const uint32_t bar = smem_u32(&s_bar[m % 3]), parity = (uint32_t)(m / 3) & 1u;
-    if (bar_ready(bar, parity)) return;
-    const long long t0 = clock64();
-    while (!bar_ready(bar, parity))
-      if (clock64() - t0 > 4000000000LL) { atomicCAS(p.status, 0, B200Q_ERR_DEVICE); break; }
-  };
-  // parameters of micro-block m's columns for the CTA's rows, by one warp (columns beyond sb: unit scale)
-  const void* scale = p.scale.at(job);
-  const void* zp = p.zp.at(job);
-  const float* gs = p.gscale.at(job);
-  int64_t pbase;
-  switch (p.strategy) {
-    case B200Q_TENSOR: pbase = 0; break;
-    case B200Q_CHANNEL: pbase = row; break;
-    case B200Q_BLOCK: pbase = (row / p.block_h) * p.groups_per_row; break;
-    default: pbase = row * p.groups_per_row; break;
-  }
-  auto fetch_params = [&](int m) {
-    float* dst = sP + (m & 1) * 4 * kMicro * kRows + lane;
-    const int c0 = m * kMicro;
-    const bool same = sSame[m] != 0;
-    const float g = gs ? *gs : 1.0f;
-    auto put = [&](int t, float s) {
-      if (gs) s = __fdiv_rn(s, g);
-      const float rs = __frcp_rn(s);
-      if (!(s >= 0x1p-100f && s <= 0x1p100f)) s_odd = 1;
-      dst[t * kRows] = s;
-      dst[(kMicro + t) * kRows] = rs * (1.0f - kMargin);
-      dst[(2 * kMicro + t) * kRows] = rs * (1.0f + kMargin);
-    };
-    auto load = [&](int t, float& s, float& z) {
-      s = 1.0f; z = 0.0f;
-      if (c0 + t < sb && live) {
-        const int64_t pi = pbase + sGrp[c0 + t];
-        s = p.sdtype == B200Q_BF16 ? __bfloat162float(((const __nv_bfloat16*)scale)[pi]) : ((const float*)scale)[pi];
-        if (ZP) z = load_zp(zp, p.zp_kind, pi);
-      }
-    };
-    if (same) {
-      float s, z;
-      load(0, s, z);
-      put(0, s);
-      s = dst[0];
-      const float lo = dst[kMicro * kRows], hi = dst[2 * kMicro * kRows];
-#pragma unroll 4
-      for (int t = 0; t < kMicro; ++t) {
-        dst[t * kRows] = s;
-        dst[(kMicro + t) * kRows] = lo;
-        dst[(2 * kMicro + t) * kRows] = hi;
-        if (ZP) dst[(3 * kMicro + t) * kRows] = z;
-      }
-    } else {
-      float s[kMicro], z[kMicro];
-#pragma unroll
-      for (int t = 0; t < kMicro; ++t) load(t, s[t], z[t]);   // all of them on their way before the first is used
-#pragma unroll
-      for (int t = 0; t < kMicro; ++t) {
-        dst[t * kRows] = s[t];
-        if (ZP) dst[(3 * kMicro + t) * kRows] = z[t];
-      }
-#pragma unroll 1
-      for (int t = 0; t < kMicro; ++t) put(t, dst[t * kRows]);
-    }
-  };
-  if (tid == 32) {
-    s_odd = 0; s_next[0] = s_next[1] = 0;
-    for (int k = 0; k < 3; ++k) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&s_bar[k])) : "memory");
+    for (int k = 0; k < S::kStages; ++k) { bar_init(smem_u32(&s_full[k]), 1); bar_init(smem_u32(&s_empty[k]), 1); }
+    for (int k = 0; k < 2; ++k)
+      for (int b = 0; b < S::kBlocks; ++b) { bar_init(smem_u32(&s_accf[k][b]), 1); bar_init(smem_u32(&s_acce[k][b]), 4); }
+    s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) {
-    __syncwarp();
-#pragma unroll 1
-    for (int m = 0; m < micros && m < 2; ++m) fetch_u(m, 0, std::integral_constant<int, kMicro>());
+  if (warp == S::kMma) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(512) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  const int32_t* col_group = p.col_group.at(job);
-  for (int c = tid; c < micros * kMicro; c += NT) {
-    float d = 1.0f;
-    int grp = 0;
-    if (c < sb) {
-      if (U) d = U[(int64_t)c * p.ldu + c];
-      const int col = p.i1 + c;
-      grp = (p.strategy == B200Q_TENSOR || p.strategy == B200Q_CHANNEL) ? 0 : (col_group ? col_group[col] : col / p.group_size);
-    }
-    sRd[c] = __frcp_rn(d);
-    sGrp[c] = grp;
-  }
-  // tile in: a lane per row, eight columns (a whole sector) at a time
-  if (vecw) {
-#pragma unroll 4
-    for (int c = warp * 8; c < micros * kMicro; c += 8 * (NW)) {
-      float4 v[2];
-#pragma unroll
-      for (int h = 0; h < 2; ++h)
-        v[h] = (live && c + 4 * h < sb) ? *reinterpret_cast<const float4*>(W + row * p.ldw + c + 4 * h)
-                                        : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        float* d = sW + (c + 4 * h) * WLD + lane;
-        d[0] = v[h].x; d[WLD] = v[h].y; d[2 * WLD] = v[h].z; d[3 * WLD] = v[h].w;
-      }
-    }
-  } else {
-    for (int r = warp; r < kRows; r += NW) {
-      const bool in = row0 + r < p.N;
-      const float* src = W + (row0 + r) * p.ldw;
-      for (int c = lane; c < micros * kMicro; c += 32) sW[c * WLD + r] = (in && c < sb) ? src[c] : 0.0f;
-    }
-  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (tid < micros) {
-    bool same = true;
-    for (int t = 1; t < kMicro; ++t) same = same && (tid * kMicro + t >= sb || sGrp[tid * kMicro + t] == sGrp[tid * kMicro]);
-    sSame[tid] = same ? 1 : 0;
-  }
-  __syncthreads();
-  if (warp == 5) fetch_params(0);
-  wait_u(0);
-  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = s_tmem;
+  chain_wait();
 
-  float loss = 0.0f;   // of warp 6's rows, a lane each
-  // the errors of micro-block `of`: their squares into the loss, and out as operand rows
-  auto finish_errors = [&](int of) {
-    const float* ei = sE + (of & 1) * kMicro * ELD + lane;
-    float x[kMicro], sum = 0.0f;
+  const int job = blockIdx.y, sb = p.sb, micros = (sb + kMicro - 1) / kMicro, blocks = (sb + kBlockCols - 1) / kBlockCols;
+  const int64_t row0 = (int64_t)blockIdx.x * ROWS;
+  const float* __restrict__ U = p.U.at(job);
+  const bool has_u = U != nullptr;
+  const unsigned char* tiles = p.tiles + (p.u_index ? p.u_index[job] : job) * p.tiles_batch;
+  const float qmin = p.qr.qmin, qmax = p.qr.qmax;
+  const int steps = micros - kLag;   // micro-blocks whose errors go anywhere by MMAs
+  auto first_block = [](int m) { return (m + kLag) * kMicro / kBlockCols; };
+
+  auto helper_role = [&] {
+    // ---- helpers: warp (block b, quarter q) has columns 128 b + 32 q + lane in registers, all rows of them
+    const int b = (warp - S::kFirstHelper) >> 2, q = warp & 3, own = 4 * b + q, col = own * 32 + lane;
+    float* __restrict__ W = p.W.at(job) + p.i1 + col;
+    float v[ROWS];
 #pragma unroll
-    for (int t = 0; t < kMicro; ++t) { x[t] = ei[t * ELD]; sum = fmaf(x[t], x[t], sum); }
-    loss += sum;   // (512 terms one after the other: 3.0e-7 off at K = 520, this way 0.9e-7)
-    if (!p.err_hi || !live) return;
-    const int64_t at = job * p.err_batch + row * p.lde + of * kMicro;
+    for (int r = 0; r < ROWS; ++r) v[r] = (col < sb && row0 + r < p.N) ? W[(row0 + r) * p.ldw] : 0.0f;
+    // columns of micro-block `m`, one of this warp's two, for the feeder
+    auto hand_over = [&](int m) {
+      if ((lane >> 4) == (m & 1)) {
+        float4* d = reinterpret_cast<float4*>(sW + col * S::kWld);
 #pragma unroll
-    for (int q = 0; q < kMicro; q += 4) {
-      float h[4], l[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        h[k] = tgemm::tf32_rn(x[q + k]);
-        l[k] = tgemm::tf32_rn(x[q + k] - h[k]);
+        for (int r = 0; r < ROWS; r += 4) d[r / 4] = make_float4(v[r], v[r + 1], v[r + 2], v[r + 3]);
       }
-      *reinterpret_cast<float4*>(p.err_hi + at + q) = make_float4(h[0], h[1], h[2], h[3]);
-      *reinterpret_cast<float4*>(p.err_lo + at + q) = make_float4(l[0], l[1], l[2], l[3]);
-    }
-  };
-  float e[kMicro];
-#pragma unroll
-  for (int t = 0; t < kMicro; ++t) e[t] = 0.0f;
+      __syncwarp();
+      if (lane == 0) bar_arrive(smem_u32(&s_raw[m]));
+    };
+    if (own == 0) { hand_over(0); hand_over(1); }
+    if (own == 1) hand_over(2);
+    const int last_step = min(2 * own + 1 - kLag, steps - 1);         // the last whose errors this warp's columns take
+    const int last_mma = min(8 * b + 7 - kLag, steps - 1);            // the last that its block takes part in
+    const float su = has_u && col < sb ? reinterpret_cast<const float*>(tiles + S::kMicros * S::kBlocks * kTileBytes)[col] : 0.0f;
+    if (b < blocks) {
 #pragma unroll 1
-  for (int m = 0; m < micros; ++m) {
-    const int c0 = m * kMicro;
-    const float* u_prev = sU + ((m + 2) % 3) * kMicro * ULD;
-    const float* u = sU + (m % 3) * kMicro * ULD + c0;
-    if (warp == 0) {
-      float* wcol = sW + c0 * WLD + lane;
-      float* eo = sE + (m & 1) * kMicro * ELD + lane;
-      const float* par = sP + (m & 1) * 4 * kMicro * kRows + lane;
-      float w[kMicro];
-      {
-        // the last errors of the micro-block before this one
-        uint64_t v[kMicro / 2];
+      for (int m = 0; m <= last_mma; ++m) {
+        const uint32_t acc = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)((m & 1) * 256 + b * 2 * ROWS);
+        bar_sleep(smem_u32(&s_accf[m & 1][b]), (uint32_t)(m >> 1) & 1u, m + kLag + 2 >= 2 * own ? 20 : 100, &s_abort);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (has_u && m <= last_step) {
 #pragma unroll
-        for (int k = 0; k < kMicro / 2; ++k) v[k] = pair(wcol[2 * k * WLD], wcol[(2 * k + 1) * WLD]);
-        if (m > 0) {
+          for (int r0 = 0; r0 < ROWS; r0 += 8) {
+            uint32_t x[8], y[8];
+            tmem_ld8(acc + r0, x);
+            tmem_ld8(acc + ROWS + r0, y);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-          for (int t = kHead; t < kMicro; ++t) {
-            const uint64_t ne = pair(-e[t], -e[t]);
+            for (int r = 0; r < 8; r += 4) {
+              const float4 se = *reinterpret_cast<const float4*>(sSe + (m & 3) * ROWS + r0 + r);
+              const float f[4] = {se.x, se.y, se.z, se.w};
 #pragma unroll
-            for (int k = 0; k < kMicro / 4; ++k) {
-              const ulonglong2 uu = *reinterpret_cast<const ulonglong2*>(u_prev + t * ULD + c0 + 4 * k);
-              fma2(v[2 * k], ne, uu.x);
-              fma2(v[2 * k + 1], ne, uu.y);
+              for (int k = 0; k < 4; ++k)
+                v[r0 + r + k] = fmaf((__uint_as_float(x[r + k]) + __uint_as_float(y[r + k])) * su, f[k], v[r0 + r + k]);
             }
           }
         }
-#pragma unroll
-        for (int k = 0; k < kMicro / 2; ++k) unpair(v[k], w[2 * k], w[2 * k + 1]);
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) bar_arrive(smem_u32(&s_acce[m & 1][b]));
+        if (m + kLag == 2 * own || m + kLag == 2 * own + 1) hand_over(m + kLag);
       }
-      // columns [begin, end) in registers; true if the test of some code failed
-      auto chain = [&](auto begin, auto end) -> bool {
-        bool differ = false;
+      // the columns as the chain leaves them
+      bar_sleep(smem_u32(&s_done[2 * min(2 * own + 1, micros - 1) + 1]), 0, 200, &s_abort);
+      if (col < sb) {
+        const float4* d = reinterpret_cast<const float4*>(sW + col * S::kWld);
 #pragma unroll
-        for (int t = begin; t < end; ++t) {
-          const float s = par[t * kRows], rlo = par[(kMicro + t) * kRows], rhi = par[(2 * kMicro + t) * kRows];
-          const float z = ZP ? par[(3 * kMicro + t) * kRows] : 0.0f, mz = ZP ? fabsf(z) * (0.5f * kMargin) : 0.0f;
-          const float wi = w[t], lo = fmaf(wi, rlo, z - mz);
-          const float qc = code_of<KIND>(lo, qmin, qmax);
-          differ |= qc != code_of<KIND>(fmaf(wi, rhi, z + mz), qmin, qmax);
-          const float q = dequant<KIND, SB, ZP>(qc, s, z);
-          // loss and error use the reciprocal of the pivot (an ulp from the reference's divisions)
-          const float tt = __fmul_rn(__fsub_rn(wi, q), sRd[c0 + t]);
-          e[t] = tt;
-          // a zero has the sign of the quotient: x / s + 0 is -0 for a small negative x, and stays it
-          w[t] = (KIND == kInt && (!ZP || (q == 0.0f && z == 0.0f))) ? copysignf(q, lo) : q;
-#pragma unroll
-          for (int k4 = (t + 1) / 4; k4 < kMicro / 4; ++k4) {
-            const float4 uu = *reinterpret_cast<const float4*>(u + t * ULD + 4 * k4);
-            if (4 * k4 + 0 > t) w[4 * k4 + 0] = fmaf(-tt, uu.x, w[4 * k4 + 0]);
-            if (4 * k4 + 1 > t) w[4 * k4 + 1] = fmaf(-tt, uu.y, w[4 * k4 + 1]);
-            if (4 * k4 + 2 > t) w[4 * k4 + 2] = fmaf(-tt, uu.z, w[4 * k4 + 2]);
-            if (4 * k4 + 3 > t) w[4 * k4 + 3] = fmaf(-tt, uu.w, w[4 * k4 + 3]);
-          }
-        }
-        return __any_sync(0xffffffffu, differ);
-      };
-      // columns from `begin` on by the exact rules, one by one in shared memory
-      auto exact = [&](int begin) {
-#pragma unroll 1
-        for (int t = begin; t < kMicro; ++t) {
-          const float wi = wcol[t * WLD], s = par[t * kRows], z = ZP ? par[(3 * kMicro + t) * kRows] : 0.0f;
-          const float q = dequant_code<SB>(round_code_k<KIND>(__fdiv_rn(wi, s) + z, qmin, qmax), s, z);
-          const float tt = __fmul_rn(__fsub_rn(wi, q), sRd[c0 + t]);
-          wcol[t * WLD] = q;
-          eo[t * ELD] = tt;
-          for (int k = t + 1; k < kMicro; ++k) wcol[k * WLD] = fmaf(-tt, u[t * ULD + k], wcol[k * WLD]);
+        for (int r = 0; r < ROWS; r += 4) {
+          const float4 x = d[r / 4];
+          v[r] = x.x; v[r + 1] = x.y; v[r + 2] = x.z; v[r + 3] = x.w;
         }
 #pragma unroll
-        for (int t = kHead; t < kMicro; ++t) e[t] = eo[t * ELD];
-      };
-      auto announce = [&] {   // the first errors are there
-        if (m + 1 < micros) asm volatile("bar.arrive 1, 64;" ::: "memory");
-      };
-      if (!chain(std::integral_constant<int, 0>(), std::integral_constant<int, kHead>()) && !s_odd) {
-#pragma unroll
-        for (int t = 0; t < kHead; ++t) eo[t * ELD] = e[t];
-        announce();
-#pragma unroll
-        for (int t = 0; t < kMicro; ++t) wcol[t * WLD] = w[t];
-        if (!chain(std::integral_constant<int, kHead>(), std::integral_constant<int, kMicro>())) {
-#pragma unroll
-          for (int t = kHead; t < kMicro; ++t) { wcol[t * WLD] = w[t]; eo[t * ELD] = e[t]; }
-        } else {
-          exact(kHead);
-        }
-      } else {
-        // (the tile still is as the micro-block found it, without the last errors of the one before)
-#pragma unroll 1
-        for (int k = 0; k < kMicro && m > 0; ++k) {
-          float v = wcol[k * WLD];
-          for (int t = kHead; t < kMicro; ++t)
-            v = fmaf(-sE[((m + 1) & 1) * kMicro * ELD + t * ELD + lane], u_prev[t * ULD + c0 + k], v);
-          wcol[k * WLD] = v;
-        }
-        exact(0);
-        announce();
+        for (int r = 0; r < ROWS; ++r)
+          if (row0 + r < p.N) W[(row0 + r) * p.ldw] = v[r];
       }
-    } else if (m + 1 < micros) {
-      const bool beside = (warp & 3) == 0;   // the chain warp's scheduler
-      if (beside && m > 0) fetch_u(m + 1, (warp - 4) * (kAskRows / 4), kAskRows);   // into the buffer of micro-block m - 2
-      if (tid == 32) s_next[(m + 1) & 1] = 0;   // (nobody takes from it before the barrier)
-      if (warp == 5) fetch_params(m + 1);
-      if (warp == 6 && m > 0) finish_errors(m - 1);
-      ErrFrag f;
-      if (m > 0 && (!beside || micros - m > 16)) {
-        load_errors(sE + ((m - 1) & 1) * kMicro * ELD, lane, false, f);
-        if (warp == kNextWarp) {
-          apply_errors<ULD>(f, u_prev + c0 + kMicro, sW + (c0 + kMicro) * WLD, lane);
-        } else {
-#pragma unroll 1
-          while (true) {
-            int task = 0;
-            if (lane == 0) task = atomicAdd(&s_next[m & 1], 1);
-            const int c = c0 + (2 + __shfl_sync(0xffffffffu, task, 0)) * kMicro;
-            if (c >= micros * kMicro) break;
-            apply_errors<ULD>(f, u_prev + c, sW + c * WLD, lane);
-          }
-        }
-      }
-      if (warp == kNextWarp) {
-        asm volatile("bar.sync 1, 64;" ::: "memory");
-        load_errors(sE + (m & 1) * kMicro * ELD, lane, true, f);
-        apply_errors<ULD>(f, u + kMicro, sW + (c0 + kMicro) * WLD, lane);
-      }
-    } else if (warp == 6 && m > 0) {
-      finish_errors(m - 1);
     }
-    if (m + 1 < micros) wait_u(m + 1);
-    __syncthreads();
+  };
+  auto chain_role = [&] {
+    // ---- the chain, a lane per row: eight columns at a time
+    const int r = warp * 32 + lane;
+    uint64_t x[kHalf / 2];    // columns of half-block n, all corrections up to it done
+    bar_wait(smem_u32(&s_raw[0]), 0, &s_abort);
+    bar_wait(smem_u32(&s_par[0]), 0, &s_abort);
+#pragma unroll
+    for (int k = 0; k < kHalf / 2; ++k) x[k] = pair(sW[2 * k * S::kWld + r], sW[(2 * k + 1) * S::kWld + r]);
+#pragma unroll 1
+    for (int n = 0; n < 2 * micros; ++n) {
+      const int slot = (n >> 1) & (kSlots - 1), t0 = (n & 1) * kHalf;
+      float* wcol = sW + n * kHalf * S::kWld + r;
+      float* eo = sE + (((n >> 1) & (kErrSlots - 1)) * kMicro + t0) * ROWS + r;
+      const float* band = sBand + slot * kBandFloats + t0 * kBandCols + t0;
+      const float2* par = sPar + (slot * kMicro + t0) * ROWS + r;
+      const float* zero = sZ + (slot * kMicro + t0) * ROWS + r;
+      uint64_t y[kHalf / 2] = {0, 0, 0, 0};   // what its errors are to the columns of n + 1
+      const uint64_t x0[kHalf / 2] = {x[0], x[1], x[2], x[3]};
+      uint64_t ne[kHalf];                     // negated errors, twice each
+      bool differ = s_odd[warp][slot] != 0;
+      float q[kHalf];
+#pragma unroll
+      for (int t = 0; t < kHalf; ++t) {
+        float a, c;
+        unpair(x[t / 2], a, c);
+        const float2 sr = par[t * ROWS];
+        const float wi = (t & 1) ? c : a, s = sr.x, z = ZP ? zero[t * ROWS] : 0.0f;
+        const float mz = ZP ? fabsf(z) * (0.5f * kMargin) : 0.0f;
+        const float rlo = sr.y * (1.0f - kMargin), rhi = sr.y * (1.0f + kMargin);
+        const float qc = code_of<KIND, ZP>(wi, rlo, z - mz, qmin, qmax);
+        differ |= qc != code_of<KIND, ZP>(wi, rhi, z + mz, qmin, qmax);
+        const float dq = dequant<KIND, SB, ZP>(qc, s, z);
+        // loss and error use the reciprocal of the pivot (an ulp from the reference's divisions)
+        const float e = __fmul_rn(__fsub_rn(dq, wi), sBand[slot * kBandFloats + kMicro * kBandCols + t0 + t]);
+        ne[t] = pair(e, e);
+        // a zero has the sign of the quotient: x / s + 0 is -0 for a small negative x, and stays it
+        q[t] = (KIND == kInt && (!ZP || (dq == 0.0f && z == 0.0f))) ? copysignf(dq, fmaf(wi, rlo, z - mz)) : dq;
+#pragma unroll
+        for (int k = (t + 1) / 4; k < 4; ++k) {
+          const ulonglong2 u = *reinterpret_cast<const ulonglong2*>(band + t * kBandCols + 4 * k);
+          if (k < 2) {
+            if (4 * k + 1 > t) x[2 * k] = fma2(ne[t], u.x, x[2 * k]);
+            x[2 * k + 1] = fma2(ne[t], u.y, x[2 * k + 1]);
+          } else {
+            y[2 * k - 4] = fma2(ne[t], u.x, y[2 * k - 4]);
+            y[2 * k - 3] = fma2(ne[t], u.y, y[2 * k - 3]);
+          }
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < kHalf; ++t) {
+        float e, f;
+        unpair(ne[t], e, f);
+        eo[t * ROWS] = e;
+        wcol[t * S::kWld] = q[t];
+      }
+      if (__any_sync(0xffffffffu, differ)) {
+        // again by the exact rules, column by column in shared memory
+#pragma unroll
+        for (int k = 0; k < kHalf / 2; ++k) {
+          float a, c;
+          unpair(x0[k], a, c);
+          wcol[2 * k * S::kWld] = a;
+          wcol[(2 * k + 1) * S::kWld] = c;
+          y[k] = 0;
+        }
+#pragma unroll 1
+        for (int t = 0; t < kHalf; ++t) {
+          const float wi = wcol[t * S::kWld], s = par[t * ROWS].x, z = ZP ? zero[t * ROWS] : 0.0f;
+          const float v = dequant_code<SB>(round_code_k<KIND>(__fdiv_rn(wi, s) + z, qmin, qmax), s, z);
+          const float e = __fmul_rn(__fsub_rn(v, wi), sBand[slot * kBandFloats + kMicro * kBandCols + t0 + t]);
+          wcol[t * S::kWld] = v;
+          eo[t * ROWS] = e;
+#pragma unroll 1
+          for (int k = t + 1; k < kHalf; ++k) wcol[k * S::kWld] = fmaf(e, band[t * kBandCols + k], wcol[k * S::kWld]);
+          const uint64_t ee = pair(e, e);
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const ulonglong2 u = *reinterpret_cast<const ulonglong2*>(band + t * kBandCols + kHalf + 4 * k);
+            y[2 * k] = fma2(ee, u.x, y[2 * k]);
+            y[2 * k + 1] = fma2(ee, u.y, y[2 * k + 1]);
+          }
+        }
+      }
+      __syncwarp();
+      if (lane == 0) bar_arrive(smem_u32(&s_done[n]));
+      if (n + 1 == 2 * micros) break;
+      if (n > 0) bar_spin(smem_u32(&s_ready[n + 1]), 0, &s_abort);
+      const float* next = n > 0 ? sNext + ((n + 1) & 1) * kHalf * ROWS + r : wcol + kHalf * S::kWld;
+      const int ld = n > 0 ? ROWS : S::kWld;
+#pragma unroll
+      for (int k = 0; k < kHalf / 2; ++k) x[k] = add2(pair(next[2 * k * ld], next[(2 * k + 1) * ld]), y[k]);
+    }
+  };
+  auto feeder_role = [&] {
+    // ---- feeders (of even and of odd half-blocks), a lane per row: half-block n takes the errors that no MMA gives it, up to those of n - 2
+    const int r = ((warp - S::kFeeder) >> 1) * 32 + lane;
+#pragma unroll 1
+    for (int n = 2 + ((warp - S::kFeeder) & 1); n < 2 * micros; n += 2) {
+      const int m = n >> 1;
+      const float* wcol = sW + n * kHalf * S::kWld + r;
+      uint64_t x[kHalf / 2] = {0, 0, 0, 0};   // summed apart: one rounding at the weight's magnitude
+#pragma unroll 1
+      for (int h = max(2 * (m - kLag + 1), 0); h <= n - 2; ++h) {
+        bar_spin(smem_u32(&s_done[h]), 0, &s_abort);
+        const int t0 = (h & 1) * kHalf;
+        const float* e = sE + (((h >> 1) & (kErrSlots - 1)) * kMicro + t0) * ROWS + r;
+        const float* band = sBand + ((h >> 1) & (kSlots - 1)) * kBandFloats + t0 * (kBandCols + 1) + (n - h) * kHalf;
+#pragma unroll
+        for (int t = 0; t < kHalf; ++t) {
+          const float f = e[t * ROWS];
+          const uint64_t ee = pair(f, f);
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const ulonglong2 u = *reinterpret_cast<const ulonglong2*>(band + t * kBandCols + 4 * k);
+            x[2 * k] = fma2(ee, u.x, x[2 * k]);
+            x[2 * k + 1] = fma2(ee, u.y, x[2 * k + 1]);
+          }
+        }
+      }
+      float* next = sNext + (n & 1) * kHalf * ROWS + r;
+      bar_spin(smem_u32(&s_raw[m]), 0, &s_abort);
+      // (the chain has taken n - 2 out of `next`)
+#pragma unroll
+      for (int k = 0; k < kHalf / 2; ++k) {
+        float a, c;
+        unpair(add2(x[k], pair(wcol[2 * k * S::kWld], wcol[(2 * k + 1) * S::kWld])), a, c);
+        next[2 * k * ROWS] = a;
+        next[(2 * k + 1) * ROWS] = c;
+      }
+      if ((n & 1) == 0) bar_spin(smem_u32(&s_par[m]), 0, &s_abort);
+      __syncwarp();
+      if (lane == 0) bar_arrive(smem_u32(&s_ready[n]));
+    }
+  };
+  auto error_role = [&] {
+    // ---- errors of 32 rows as operand of the MMAs
+    const int r = (warp - S::kErrors) * 32 + lane;
+#pragma unroll 1
+    for (int m = 0; m < steps; ++m) {
+      if (m >= 2)   // the operand buffer's last readers are done
+        bar_spin(smem_u32(&s_accf[m & 1][blocks - 1]), (uint32_t)((m - 2) >> 1) & 1u, &s_abort);
+      bar_spin(smem_u32(&s_done[2 * m + 1]), 0, &s_abort);
+      const float* es = sE + (m & (kErrSlots - 1)) * kMicro * ROWS + r;
+      const uint32_t eop = smem_u32(sm + S::kErr + (m & 1) * S::kErrBytes) + (uint32_t)(r * kRowBytes);
+      float largest[4] = {0.0f, 0.0f, 0.0f, 0.0f}, to, back;
+#pragma unroll
+      for (int t = 0; t < kMicro; ++t) largest[t & 3] = fmaxf(largest[t & 3], fabsf(es[t * ROWS]));
+      row_scale(fmaxf(fmaxf(largest[0], largest[1]), fmaxf(largest[2], largest[3])), to, back);
+      sSe[(m & 3) * ROWS + r] = back;
+#pragma unroll 1
+      for (int j = 0; j < 2; ++j) {   // 16 bytes of hi halves and of lo halves each; 64-byte swizzle
+        uint32_t hi[4], lo[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) split_pair(es[(8 * j + 2 * k) * ROWS] * to, es[(8 * j + 2 * k + 1) * ROWS] * to, hi[k], lo[k]);
+        const uint32_t at = eop + ((uint32_t)(j ^ ((r >> 1) & 3)) << 4), at2 = eop + ((uint32_t)((j + 2) ^ ((r >> 1) & 3)) << 4);
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(hi[0]), "r"(hi[1]), "r"(hi[2]), "r"(hi[3]) : "memory");
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at2), "r"(lo[0]), "r"(lo[1]), "r"(lo[2]), "r"(lo[3]) : "memory");
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) bar_arrive(smem_u32(&s_opr[m]));
+    }
+  };
+  auto out_role = [&] {
+    // ---- errors of 32 rows: out as operand of the trailing product, into the losses
+    const int r = (warp - S::kOut) * 32 + lane;
+    const int64_t row = row0 + r;
+    const bool live = row < p.N, out = p.err_hi && live;   // (a superblock with columns after it is a whole one)
+    float loss = 0.0f;
+#pragma unroll 1
+    for (int m = 0; m < micros; ++m) {
+      bar_wait(smem_u32(&s_done[2 * m + 1]), 0, &s_abort);
+      const float* es = sE + (m & (kErrSlots - 1)) * kMicro * ROWS + r;
+      const int64_t at = job * p.err_batch + row * p.lde + m * kMicro;
+      float sum = 0.0f;
+#pragma unroll 1
+      for (int t = 0; t < kMicro; t += 4) {
+        float hi[4], lo[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const float x = es[(t + k) * ROWS];
+          sum = fmaf(x, x, sum);
+          hi[k] = tgemm::tf32_rn(-x);
+          lo[k] = tgemm::tf32_rn(-x - hi[k]);
+        }
+        if (out) {
+          *reinterpret_cast<float4*>(p.err_hi + at + t) = make_float4(hi[0], hi[1], hi[2], hi[3]);
+          *reinterpret_cast<float4*>(p.err_lo + at + t) = make_float4(lo[0], lo[1], lo[2], lo[3]);
+        }
+      }
+      __syncwarp();
+      if (lane == 0) bar_arrive(smem_u32(&s_out[m]));
+      loss += sum;   // (512 terms one after the other: 3.0e-7 off at K = 520, this way 0.9e-7)
+    }
+    if (live) {
+      float* losses = p.losses.at(job);
+      const float half = loss * 0.5f;
+      losses[row] = p.i1 == 0 ? half : losses[row] + half;
+    }
+  };
+  auto param_role = [&] {
+    // ---- parameters of the rows, up to four micro-blocks ahead; copies of U: tiles (a stage per micro-block), bands
+    const void* scale = p.scale.at(job);
+    const void* zp = p.zp.at(job);
+    const float* gs = p.gscale.at(job);
+    const int32_t* col_group = p.col_group.at(job);
+    const float g = gs ? *gs : 1.0f;
+    const bool per_column = p.strategy != B200Q_TENSOR && p.strategy != B200Q_CHANNEL;
+    int64_t pbase[S::kChains];
+#pragma unroll
+    for (int h = 0; h < S::kChains; ++h) {
+      const int64_t row = min(row0 + h * 32 + lane, p.N - 1);
+      pbase[h] = p.strategy == B200Q_CHANNEL ? row : p.strategy == B200Q_BLOCK ? (row / p.block_h) * p.groups_per_row
+                 : p.strategy == B200Q_TENSOR ? 0 : row * p.groups_per_row;
+    }
+    auto load = [&](int64_t pi, float& s, float& z) {
+      s = p.sdtype == B200Q_BF16 ? __bfloat162float(((const __nv_bfloat16*)scale)[pi]) : ((const float*)scale)[pi];
+      z = ZP ? load_zp(zp, p.zp_kind, pi) : 0.0f;
+    };
+    auto groups = [&](int k) -> int {   // of column lane % 16 of micro-block k (columns beyond the superblock: of the last)
+      if (!per_column) return 0;
+      const int col = p.i1 + min(k * kMicro + (lane & 15), sb - 1);
+      return col_group ? col_group[col] : col / p.group_size;
+    };
+    // asked for a micro-block ahead: the groups, and scale and zero point at the group of the first column
+    int grp = groups(0), now = 0;
+    float s1[S::kChains], z1[S::kChains];
+    auto ask = [&](int k) {
+      now = grp;
+#pragma unroll
+      for (int h = 0; h < S::kChains; ++h) load(pbase[h] + __shfl_sync(0xffffffffu, now, 0), s1[h], z1[h]);
+      grp = groups(k + 1);
+    };
+    auto load_step = [&](int m) {
+      if (!has_u || m >= steps) return;
+      const int stage = m % S::kStages;
+      if (m >= S::kStages) bar_wait(smem_u32(&s_empty[stage]), (uint32_t)(m / S::kStages - 1) & 1u, &s_abort);
+      if (lane == 0 && !s_abort) {
+        // (rows of columns that are past stay as they are: nobody takes their sums)
+        const int first = first_block(m);
+        const uint32_t bar = smem_u32(&s_full[stage]), skip = ((m + kLag) * kMicro - first * kBlockCols) * kRowBytes;
+        const uint32_t dst = smem_u32(sm + S::kRing + stage * S::kStageBytes);
+        const unsigned char* src = tiles + m * S::kStageBytes;
+        const uint32_t begin = first * kTileBytes + skip, bytes = blocks * kTileBytes - begin;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+        bulk_copy(dst + begin, src + begin, bytes, bar);
+      }
+      __syncwarp();
+    };
+    auto load_band = [&](int k) {
+      if (k >= micros) return;
+      if (k >= kSlots) {   // the feeders are through with the slot
+        bar_wait(smem_u32(&s_ready[2 * k - 4]), 0, &s_abort);
+        bar_wait(smem_u32(&s_ready[2 * k - 3]), 0, &s_abort);
+      }
+      if (lane == 0 && !s_abort) {
+        const uint32_t bar = smem_u32(&s_par[k]);
+        if (has_u) {
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(kBandFloats * 4) : "memory");
+          bulk_copy(smem_u32(sBand + (k & (kSlots - 1)) * kBandFloats),
+                    tiles + band_offset(SBLK) + (int64_t)k * kBandFloats * 4, kBandFloats * 4, bar);
+        } else {
+          bar_arrive(bar);
+        }
+      }
+      __syncwarp();
+    };
+    if (!has_u)
+      for (int i = lane; i < kSlots * kBandFloats; i += 32) {
+        const int k = i % kBandFloats;
+        sBand[i] = k >= kMicro * kBandCols || k / kBandCols == k % kBandCols ? 1.0f : 0.0f;
+      }
+    __syncwarp();
+    for (int k = 0; k < kSlots - 1; ++k) load_band(k);
+    for (int k = 0; k < S::kStages; ++k) load_step(k);
+    ask(0);
+#pragma unroll 1
+    for (int k = 0; k < micros; ++k) {
+      const int slot = k & (kSlots - 1);
+      if (k >= kSlots) {   // the chain and the other readers of the slots are through with them
+        bar_wait(smem_u32(&s_done[2 * (k - kSlots) + 1]), 0, &s_abort);
+        bar_wait(smem_u32(&s_out[k - kSlots]), 0, &s_abort);
+      }
+      const bool same = __all_sync(0xffffffffu, now == __shfl_sync(0xffffffffu, now, 0));
+#pragma unroll
+      for (int h = 0; h < S::kChains; ++h) {
+        const int r = h * 32 + lane;
+        const bool live = row0 + r < p.N;
+        bool odd = false;
+        auto put = [&](int t, float s, float z) {   // the effective scale and its reciprocal
+          if (!live) { s = 1.0f; z = 0.0f; }
+          else if (gs) s = __fdiv_rn(s, g);
+          odd |= !(s >= 0x1p-100f && s <= 0x1p100f);
+          sPar[(slot * kMicro + t) * ROWS + r] = make_float2(s, __frcp_rn(s));
+          if (ZP) sZ[(slot * kMicro + t) * ROWS + r] = z;
+        };
+        if (same) {
+          put(0, s1[h], z1[h]);
+          const float2 sr = sPar[slot * kMicro * ROWS + r];
+          const float z = ZP ? sZ[slot * kMicro * ROWS + r] : 0.0f;
+#pragma unroll 5
+          for (int t = 1; t < kMicro; ++t) {
+            sPar[(slot * kMicro + t) * ROWS + r] = sr;
+            if (ZP) sZ[(slot * kMicro + t) * ROWS + r] = z;
+          }
+        } else {
+#pragma unroll 1
+          for (int t0 = 0; t0 < kMicro; t0 += 4) {
+            float s[4], z[4];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) load(pbase[h] + __shfl_sync(0xffffffffu, now, t0 + t), s[t], z[t]);
+#pragma unroll 1
+            for (int t = 0; t < 4; ++t) put(t0 + t, t == 0 ? s[0] : t == 1 ? s[1] : t == 2 ? s[2] : s[3],
+                                            t == 0 ? z[0] : t == 1 ? z[1] : t == 2 ? z[2] : z[3]);
+          }
+        }
+        odd = __any_sync(0xffffffffu, odd);
+        if (lane == 0) s_odd[h][slot] = odd;
+      }
+      __syncwarp();
+      if (lane == 0) bar_arrive(smem_u32(&s_par[k]));
+      ask(k + 1);
+      if (k - 1 >= S::kStages) load_step(k - 1);
+      if (k - 1 >= kSlots - 1) load_band(k - 1);
+    }
+    if (micros - 1 >= kSlots - 1) load_band(micros - 1);
+  };
+  auto mma_role = [&] {
+    // ---- MMAs
+#pragma unroll 1
+    for (int m = 0; m < steps; ++m) {
+      {
+        const int first = first_block(m);
+        for (int b = first; b < blocks; ++b) bar_spin(smem_u32(&s_acce[m & 1][b]), ((uint32_t)(m >> 1) & 1u) ^ 1u, &s_abort);
+        if (has_u) bar_spin(smem_u32(&s_full[m % S::kStages]), (uint32_t)(m / S::kStages) & 1u, &s_abort);
+        bar_spin(smem_u32(&s_opr[m]), 0, &s_abort);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (lane == 0) {
+          constexpr uint32_t lo = kRowBytes / 2;
+          const uint64_t e_hi = make_desc(smem_u32(sm + S::kErr + (m & 1) * S::kErrBytes)), e_lo = e_hi + (lo >> 4);
+          uint64_t u_hi = make_desc(smem_u32(sm + S::kRing + (m % S::kStages) * S::kStageBytes + first * kTileBytes));
+          uint32_t d = tmem + (uint32_t)((m & 1) * 256 + first * 2 * ROWS);
+#pragma unroll 1
+          for (int b = first; b < blocks; ++b, d += 2 * ROWS, u_hi += kTileBytes >> 4) {
+            if (has_u) {   // hi * hi, and beside it hi * lo + lo * hi
+              mma_f16(d, u_hi, e_hi, instr_desc(ROWS), 0u);
+              mma_f16(d + ROWS, u_hi, e_lo, instr_desc(ROWS), 0u);
+              mma_f16(d + ROWS, u_hi + (lo >> 4), e_hi, instr_desc(ROWS), 1u);
+              tc_commit(smem_u32(&s_accf[m & 1][b]));
+            } else {       // (nothing to add: the helpers still follow the steps)
+              bar_arrive(smem_u32(&s_accf[m & 1][b]));
+            }
+          }
+          if (has_u) tc_commit(smem_u32(&s_empty[m % S::kStages]));
+        }
+        __syncwarp();
+      }
+    }
+  };
+  if (warp >= S::kFirstHelper) {
+    if constexpr (ROWS == 32) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Regs<ROWS>::kHelper));
+    else asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Regs<ROWS>::kHelper));
+    helper_role();
+  } else if (warp < 4) {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Regs<ROWS>::kChain));
+    if (warp < S::kChains) chain_role();
+    else if (warp >= S::kErrors && warp < S::kErrors + S::kChains) error_role();
+    else if (ROWS == 32) feeder_role();
+  } else if (ROWS == 64 && warp < 8) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Regs<ROWS>::kFeeder));
+    feeder_role();
+  } else {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Regs<ROWS>::kOther));
+    if (warp == S::kMma) mma_role();
+    else if (warp >= S::kOut && warp < S::kParams) out_role();
+    else if (warp == S::kParams) param_role();
   }
   chain_go();
-  if (warp == 6) finish_errors(micros - 1);   // (a superblock with columns after it is a whole one)
-  // tile out
-  if (vecw) {
-#pragma unroll 2
-    for (int c = warp * 8; c < sb; c += 8 * (NW)) {
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const float* d = sW + (c + 4 * h) * WLD + lane;
-        if (live && c + 4 * h < sb)
-          *reinterpret_cast<float4*>(W + row * p.ldw + c + 4 * h) = make_float4(d[0], d[WLD], d[2 * WLD], d[3 * WLD]);
-      }
-    }
-  } else {
-    for (int r = warp; r < kRows; r += NW) {
-      if (row0 + r >= p.N) break;
-      float* dst = W + (row0 + r) * p.ldw;
-      for (int c = lane; c < sb; c += 32) dst[c] = sW[c * WLD + r];
-    }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (s_abort) {
+    if (tid == 0 && p.status) atomicCAS(p.status, 0, B200Q_ERR_DEVICE);
+    const long long t0 = clock64();
+    while (clock64() - t0 < 2000000LL) __nanosleep(1000);   // copies in flight land
   }
-  if (warp == 6 && live) {
-    float* lo = p.losses.at(job);
-    const float half = loss * 0.5f;
-    lo[row] = p.i1 == 0 ? half : lo[row] + half;
+  if (warp == S::kMma) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
   }
 }
 
-// Superblock width.  With at most one CTA per SM the chain decides and 512 columns halve the launches and the traffic
-// of the trailing products; with more rows than that the CTA's own updates (width / 2 multiply-adds per element) do,
-// and 256 columns leave room for two CTAs per SM.
-static int superblock_of(int64_t ctas) { return ctas <= kNumSMs ? 512 : 256; }
+// Superblock width, rows of a CTA.  32 rows a CTA and 512 columns while that gives every CTA an SM of its own; more rows
+// are carried 64 a CTA (two chains, the operand tiles of U read once for both), whose share of the superblock fits the
+// helpers' registers up to 256 columns.
+static bool wide(int64_t N, int batch) { return (N + 31) / 32 * batch <= kNumSMs; }
 // The trailing product is split in the columns the next superblock needs and the rest on a helper stream only while
 // a superblock's CTAs leave half of the GPU idle.
 static bool look_ahead(int64_t ctas) { return ctas <= kNumSMs / 2; }
 
 struct Layout {
-  int sb, sets;
-  int64_t rows_n, rows_k, err, ub;   // rows per problem of the operands; floats of one hi or lo array
+  int rows, sb, sets;
+  int64_t ctas, rows_n, rows_k, err, ub;   // CTAs, rows per problem of the operands; floats of one hi or lo array
+  int64_t tiles;                           // bytes of the tiles of all factors
   size_t bytes;
 };
 static Layout layout_of(int64_t N, int64_t K, int batch, int distinct_u, bool may_overlap) {
-  const int64_t ctas = (N + kRows - 1) / kRows * batch;
   Layout l;
-  l.sb = superblock_of(ctas);
-  l.sets = may_overlap && look_ahead(ctas) ? 2 : 1;
+  l.rows = wide(N, batch) ? 32 : 64;
+  l.sb = l.rows == 32 ? 512 : 256;
+  l.ctas = (N + l.rows - 1) / l.rows;
+  l.sets = may_overlap && K > l.sb ? 2 : 1;
   l.rows_n = (N + 127) / 128 * 128; l.rows_k = (K + 127) / 128 * 128;
-  l.err = l.rows_n * l.sb * batch; l.ub = l.rows_k * l.sb * distinct_u;
-  l.bytes = kSweepHeaderBytes + (K > l.sb ? (size_t)(2 * l.sets * (l.err + l.ub)) * sizeof(float) : 0) + 64;
+  l.err = K > l.sb ? l.rows_n * l.sb * batch : 0; l.ub = K > l.sb ? l.rows_k * l.sb * distinct_u : 0;
+  l.tiles = tiles_bytes(l.sb) * distinct_u;
+  l.bytes = kSweepHeaderBytes + (size_t)(2 * l.sets * (l.err + l.ub)) * sizeof(float) + (size_t)(l.sets * l.tiles) + 64;
   return l;
+}
+
+typedef void (*Kernel)(const Params);
+template <int ROWS, int SBLK, bool SB, int KIND> static Kernel pick_zp(bool zp) {
+  return zp ? sweep_block_kernel<ROWS, SBLK, SB, KIND, true> : sweep_block_kernel<ROWS, SBLK, SB, KIND, false>;
+}
+template <int ROWS, int SBLK, bool SB> static Kernel pick_kind(int kind, bool zp) {
+  return kind == kInt ? pick_zp<ROWS, SBLK, SB, kInt>(zp)
+                      : kind == kFp8 ? pick_zp<ROWS, SBLK, SB, kFp8>(zp) : pick_zp<ROWS, SBLK, SB, kFp4>(zp);
+}
+static Kernel pick_kernel(int rows, bool bf16_values, int kind, bool zp) {
+  if (rows == 32) return bf16_values ? pick_kind<32, 512, true>(kind, zp) : pick_kind<32, 512, false>(kind, zp);
+  return bf16_values ? pick_kind<64, 256, true>(kind, zp) : pick_kind<64, 256, false>(kind, zp);
 }
 
 // `Ud` / `u_index`: the distinct factors of a batch and the one each problem uses (null: the single U, or one each)
@@ -586,39 +873,40 @@ static int sweep(Params p, int sdtype, bool global, int batch, const float* cons
   const int64_t N = p.N, K = p.K;
   const bool has_u = p.U.one || p.U.table;
   const Layout l = layout_of(N, K, batch, distinct_u, may_overlap);
-  // header of the workspace: a status word that a bounded wait expiring inside one of the trailing products sets to
+  // header of the workspace: a status word that a bounded wait expiring in a sweep or a trailing product sets to
   // B200Q_ERR_DEVICE (cleared here, read by the caller afterwards)
   int* status = (int*)workspace;
   float* err = (float*)((char*)workspace + kSweepHeaderBytes);   // [sets][hi, lo]
   float* ub = err + 2 * l.sets * l.err;                          // [sets][hi, lo]
+  unsigned char* tiles = (unsigned char*)(ub + 2 * l.sets * l.ub);   // [sets][factor]
   B200Q_TRY(cudaMemsetAsync(status, 0, sizeof(int), st));
   if (sdtype != B200Q_BF16 && sdtype != B200Q_F32) return B200Q_ERR_UNSUPPORTED;
-  p.sdtype = sdtype; p.status = status;
+  p.sdtype = sdtype; p.status = status; p.u_index = u_index; p.tiles_batch = tiles_bytes(l.sb);
   const bool with_zp = p.zp.one || p.zp.table, bf16_values = sdtype == B200Q_BF16 && !global;
-  void (*kern)(const Params) = nullptr;
-#define B200Q_SWEEP_ZP(S, B, K) kern = with_zp ? sweep_block_kernel<S, B, K, true> : sweep_block_kernel<S, B, K, false>
-#define B200Q_SWEEP_SB(S, K) do { if (bf16_values) B200Q_SWEEP_ZP(S, true, K); else B200Q_SWEEP_ZP(S, false, K); } while (0)
-#define B200Q_SWEEP_PICK(S)                            \
-  do {                                                 \
-    if (p.qr.kind == kInt) B200Q_SWEEP_SB(S, kInt);      \
-    else if (p.qr.kind == kFp8) B200Q_SWEEP_SB(S, kFp8); \
-    else B200Q_SWEEP_SB(S, kFp4);                        \
-  } while (0)
-  if (l.sb == 512) B200Q_SWEEP_PICK(512); else B200Q_SWEEP_PICK(256);
-#undef B200Q_SWEEP_PICK
-#undef B200Q_SWEEP_SB
-#undef B200Q_SWEEP_ZP
-  B200Q_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(l.sb)));
-  const int ctas = (int)((N + kRows - 1) / kRows);
-  tgemm::SideStream* side = l.sets == 2 && has_u && K > 2 * l.sb ? tgemm::side_stream(st) : nullptr;
-  bool side_busy = false;
+  const Kernel kern = pick_kernel(l.rows, bf16_values, p.qr.kind, with_zp);
+  const size_t smem = l.rows == 32 ? Shape<32, 512>::kSmem : Shape<64, 256>::kSmem;
+  const int threads = l.rows == 32 ? Shape<32, 512>::kThreads : Shape<64, 256>::kThreads;
+  B200Q_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // A single weight makes the next superblock's slice of U beside the sweep, and with few rows the far columns'
+  // product beside the sweep after it.
+  tgemm::SideStream* side = l.sets == 2 && has_u ? tgemm::side_stream(st) : nullptr;
+  const bool far_beside = side && look_ahead(l.ctas * batch);
   int rc;
+  // the operand forms of U that superblock i1 needs: of its square, and of U[i1 : i1 + sb, i1 + sb :] for the trailing
+  // product (row = column, contraction contiguous)
+  Ptr<const float> factors = p.U;
+  if (Ud) factors = {nullptr, Ud};
+  auto square = l.sb == 512 ? square_tiles_kernel<512> : square_tiles_kernel<256>;
+  const size_t square_smem = 32 * (l.sb + 1) * sizeof(uint32_t);
+  B200Q_TRY(cudaFuncSetAttribute(square, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)square_smem));
   auto split_u = [&](int64_t i1, int which, cudaStream_t on) -> int {
-    // operand form of U[i1 : i1 + sb, i1 + sb :] (independent of the sweep: kept off its chain)
-    const int64_t i2 = i1 + l.sb;
-    if (i2 >= K) return B200Q_OK;
+    const int w = (int)(K - i1 < l.sb ? K - i1 : l.sb);
+    const int64_t i2 = i1 + w;
     float* hi = ub + (int64_t)which * 2 * l.ub;
-    return tgemm::split_transposed(p.U.one ? p.U.one + i1 * p.ldu + i2 : nullptr, Ud, i1 * p.ldu + i2, p.ldu, l.sb,
+    B200Q_TRY(launch_chained(square, dim3((w + 31) / 32, distinct_u), kTileThreads, square_smem, on, factors, p.ldu, (int)i1,
+                             w, tiles + which * l.tiles, p.tiles_batch));
+    B200Q_LAUNCH_CHECK();
+    return tgemm::split_transposed(p.U.one ? p.U.one + i1 * p.ldu + i2 : nullptr, Ud, i1 * p.ldu + i2, p.ldu, w,
                                    (int)(K - i2), hi, hi + l.ub, l.sb, l.rows_k * l.sb, distinct_u, on);
   };
   if (has_u && (rc = split_u(0, 0, st))) return rc;
@@ -627,15 +915,22 @@ static int sweep(Params p, int sdtype, bool global, int batch, const float* cons
     const int w = (int)(K - i1 < l.sb ? K - i1 : l.sb), which = l.sets == 2 ? blk & 1 : 0;
     const int64_t i2 = i1 + w;
     const bool trailing = i2 < K && has_u;
+    float* bhi = ub + (int64_t)which * 2 * l.ub;
     p.i1 = (int)i1; p.sb = w;
     p.err_hi = trailing ? err + (int64_t)which * 2 * l.err : nullptr;
     p.err_lo = trailing ? p.err_hi + l.err : nullptr;
-    p.lde = l.sb; p.err_batch = l.rows_n * l.sb;
-    B200Q_TRY(launch_chained(kern, dim3(ctas, batch), 32 * warps_of(l.sb), smem_bytes(l.sb), st, p));
+    p.tiles = tiles + which * l.tiles; p.lde = l.sb; p.err_batch = l.rows_n * l.sb;
+    if (trailing && side) {
+      // the next superblock's slice of U: its buffer was last read by the products of the superblock before this one
+      B200Q_TRY(cudaEventRecord(side->next, st));
+      B200Q_TRY(cudaStreamWaitEvent(side->stream, side->next, 0));
+      if ((rc = split_u(i2, which ^ 1, side->stream))) return rc;
+      B200Q_TRY(cudaEventRecord(side->done, side->stream));
+    }
+    B200Q_TRY(launch_chained(kern, dim3((unsigned)l.ctas, batch), threads, smem, st, p));
     B200Q_LAUNCH_CHECK();
     if (!trailing) continue;
     // W[:, i2:] -= Err[N, w] * U[i1:i2, i2:]
-    float* bhi = ub + (int64_t)which * 2 * l.ub;
     tgemm::Job j;
     j.A = tgemm::Operand{p.err_hi, p.err_lo, l.sb, l.rows_n * batch, l.rows_n, 0};
     j.B = tgemm::Operand{bhi, bhi + l.ub, l.sb, l.rows_k * distinct_u, l.rows_k, 0};
@@ -653,24 +948,21 @@ static int sweep(Params p, int sdtype, bool global, int batch, const float* cons
       continue;
     }
     tgemm::Job far = j;
-    if (j.N > l.sb) j.N = l.sb;
-    B200Q_TRY(cudaEventRecord(side->ready, st));
-    B200Q_TRY(cudaStreamWaitEvent(side->stream, side->ready, 0));
-    // the far columns of the superblock before, and this one's operand form of U made behind them
-    if (side_busy) B200Q_TRY(cudaStreamWaitEvent(st, side->done, 0));
+    if (far_beside) {
+      if (j.N > l.sb) j.N = l.sb;
+      B200Q_TRY(cudaEventRecord(side->ready, st));
+      B200Q_TRY(cudaStreamWaitEvent(side->stream, side->ready, 0));
+    }
+    // the far columns of the superblock before, and the next slice of U, made behind them
+    B200Q_TRY(cudaStreamWaitEvent(st, side->done, 0));
     if ((rc = tgemm::launch(j, st))) return rc;
-    if (far.N > l.sb) {
-      far.B.row0 = l.sb; far.N -= l.sb; far.max_ctas = kNumSMs - ctas * batch;
+    if (far_beside && far.N > l.sb) {   // (waited for with the slice of U that the next round makes)
+      far.B.row0 += l.sb; far.N -= l.sb; far.max_ctas = kNumSMs - (int)l.ctas * batch;
       if (p.W.one) far.C = p.W.one + i2 + l.sb;
       far.c_offset = i2 + l.sb;
       if ((rc = tgemm::launch(far, side->stream))) return rc;
     }
-    // the next superblock's slice of U: its buffer was last read by the superblock before this one
-    if ((rc = split_u(i2, which ^ 1, side->stream))) return rc;
-    B200Q_TRY(cudaEventRecord(side->done, side->stream));
-    side_busy = true;
   }
-  if (side_busy) B200Q_TRY(cudaStreamWaitEvent(st, side->done, 0));
   return B200Q_OK;
 }
 

@@ -337,3 +337,38 @@ def test_one_launch_parameters_of_unusual_values(scheme, N, K):
     many = ops.minmax_qparams([w.clone(), w], args)
     for s, z in (one, (many[0][0], many[1][0]), (many[0][1], many[1][1])):
         assert bits_equal(s, scale) and bits_equal(z, zp)
+
+
+@pytest.mark.parametrize("N,K", [(1, 1), (31, 7), (33, 17), (64, 47), (65, 49), (32, 129), (40, 511), (33, 520),
+                                 (4736, 40), (4737, 136), (4801, 264)])
+@pytest.mark.parametrize("scheme", ["W8_CHANNEL", "W4_ASYM"])
+def test_sweep_at_edges_of_blocks(N, K, scheme):
+    """Half-blocks of 8 columns, operands of 16, tiles of 128, superblocks of 512 (32 rows a CTA) and 256 (64)."""
+    g = torch.Generator().manual_seed(N * 1000 + K)
+    a = torch.randn(3 * K + 8, K, generator=g, dtype=torch.float64)
+    U = torch.linalg.cholesky(torch.linalg.inv(a.T @ a / len(a) + 0.05 * torch.eye(K, dtype=torch.float64)), upper=True)
+    w = (torch.randn(N, K, generator=g) * 0.02).to(torch.float64)
+    asym = scheme == "W4_ASYM"
+    scale = torch.full((N, 1), 0.01 if asym else 5e-4).bfloat16()
+    zp = (torch.arange(N) % 5 - 2).to(torch.int8).view(N, 1) if asym else None
+    args = QuantizationArgs(num_bits=4 if asym else 8, type="int", symmetric=not asym, strategy="channel")
+    lo, hi = (-8, 7) if asym else (-128, 127)
+    x, s, z = w.clone(), scale.double(), zp.double() if asym else torch.zeros(N, 1, dtype=torch.float64)
+    q, loss, close = torch.zeros_like(w), torch.zeros(N, dtype=torch.float64), torch.zeros(N, dtype=torch.bool)
+    for i in range(K):
+        v = x[:, i:i + 1] / s + z
+        c = v.clamp(lo, hi)
+        # float32 sums (errors below 1e-6 of the weights' size) may turn a code this close to a boundary, and with it
+        # everything later in the row
+        close |= ((c - c.floor() - 0.5).abs() < 1e-3)[:, 0]
+        q[:, i] = ((c.round() - z) * s).bfloat16().double()[:, 0]
+        e = (x[:, i] - q[:, i]) / U[i, i]
+        loss += e * e / 2
+        x[:, i:] -= e[:, None] * U[i, i:]
+    W = w.float().cuda()
+    losses = ops.gptq_sweep(W, U.float().cuda().contiguous(), scale.cuda(), None if zp is None else zp.cuda(), args)
+    torch.cuda.synchronize()
+    sure = ~close
+    assert torch.equal(W.cpu().double()[sure], q[sure])
+    assert torch.allclose(losses.cpu().double()[sure], loss[sure], rtol=1e-4)
+    assert float((W.cpu().double() != q).double().mean()) < 0.05
