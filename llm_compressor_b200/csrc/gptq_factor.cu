@@ -17,7 +17,8 @@
 // Schur complement.  Outer step o with D = L_oo^-1:
 //     X[o,:o] = D S[o,:o]      P = A[below,o] D^T (= L[below,o])      S[below,o] = -P D
 //     S[i,:o] -= P_i X[o,:o]   and   A[i,j] -= P_i P_j^T (o < j <= i)
-// The last three are one launch: the rows of its second operand are X[o,:o]^T, D^T and P, indexed by absolute column.
+// The last three are one launch on halves with a scale per row: the rows of its second operand are X[o,:o]^T, D^T and P,
+// indexed by absolute column.
 //
 // A pivot <= 0 (or NaN) sets the problem's status; the host then takes the reference's identity fallback.
 #include <type_traits>
@@ -453,15 +454,12 @@ __global__ void __launch_bounds__(kThreads) square_update_kernel(Mat mt, const f
 }
 
 // ---------------------------------------------------------------------------------------
-// Operand forms.  D (the square's inverse, zero above the diagonal) as rows, and D^T as the rows K0.. of the
-// update's second operand.
-__global__ void __launch_bounds__(256) split_square_kernel(Mat mt, int K0, int n, float* d_hi, float* d_lo,
-                                                           float* t_hi, float* t_lo, int64_t t_batch) {
+// Operand form of D (the square's inverse, zero above the diagonal) as rows.
+__global__ void __launch_bounds__(256) split_square_kernel(Mat mt, int K0, int n, float* d_hi, float* d_lo) {
   chain_wait();
   chain_go();
-  __shared__ float tile[32][33];
   const float* A = mt.A + blockIdx.y * mt.batch + (int64_t)K0 * mt.lda + K0;
-  const int64_t db = (int64_t)blockIdx.y * OB * OB, tb = blockIdx.y * t_batch + (int64_t)K0 * OB;
+  const int64_t db = (int64_t)blockIdx.y * OB * OB;
   const int tr = blockIdx.x >> 4, tc = blockIdx.x & 15, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -470,17 +468,6 @@ __global__ void __launch_bounds__(256) split_square_kernel(Mat mt, int K0, int n
     const float h = tgemm::tf32_rn(x);
     d_hi[db + (int64_t)r * OB + c] = h;
     d_lo[db + (int64_t)r * OB + c] = tgemm::tf32_rn(x - h);
-    tile[ty + 8 * i][tx] = x;
-  }
-  if (!t_hi) return;
-  __syncthreads();
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int c = tc * 32 + ty + 8 * i, r = tr * 32 + tx;
-    const float x = tile[tx][ty + 8 * i];
-    const float h = tgemm::tf32_rn(x);
-    t_hi[tb + (int64_t)c * OB + r] = h;
-    t_lo[tb + (int64_t)c * OB + r] = tgemm::tf32_rn(x - h);
   }
 }
 
@@ -544,11 +531,12 @@ __global__ void __launch_bounds__(256) reverse_out_kernel(float* H0, float* cons
 
 static int64_t round_up(int64_t v, int64_t m) { return (v + m - 1) / m * m; }
 
-// floats of workspace per problem: the matrix, the scratch panel of the square, the square's operand form and (for
-// more than one outer block) three operand panels with a row per matrix row
+// floats of workspace per problem: the matrix, the scratch panel of the square, and (for more than one outer block) the
+// operand forms: of the square, of the next block's rows of P (two copies), of the panel before its product with D; P; and
+// two copies of the update's operand of halves with its scales, a row per matrix row
 static int64_t problem_floats(int64_t K) {
   const int64_t rows = round_up(K, NB);
-  return K * round_up(K, 32) + kScratchFloats + (K > OB ? 2 * OB * OB + 6 * rows * OB : 0);
+  return K * round_up(K, 32) + kScratchFloats + (K > OB ? 6 * OB * OB + 5 * rows * OB + 2 * rows : 0);
 }
 
 // SMs the bulk of an update leaves to the chain beside it: the square's kernels are small (24 to 120 CTAs of which
@@ -560,6 +548,7 @@ static int factor(float* H, float* const* Hs, int batch, int64_t K, int64_t ldh,
   using tgemm::Job;
   using tgemm::Operand;
   const int slice = Hs ? tgemm::kShortSlice : tgemm::kLongSlice;   // (measured where they are defined)
+  const int slice16 = Hs ? tgemm::kShortestSlice16 : tgemm::kLongSlice16;
   int rc;
 #define B200Q_RC(expr) do { rc = (expr); if (rc != B200Q_OK) return rc; } while (0)
   const int64_t lda = round_up(K, 32), rows = round_up(K, NB);
@@ -568,10 +557,13 @@ static int factor(float* H, float* const* Hs, int batch, int64_t K, int64_t ldh,
   float* P = ws + (int64_t)batch * K * lda;
   float* d_hi = P + (int64_t)batch * kScratchFloats;
   float* d_lo = d_hi + (int64_t)batch * OB * OB;
-  float* a_hi = d_lo + (int64_t)batch * OB * OB;          // panel before its product with D, and S[o,:o]^T
+  float* f_base = d_lo + (int64_t)batch * OB * OB;        // next block's rows of P, two copies used in turn
+  float* a_hi = f_base + (int64_t)batch * 4 * OB * OB;    // panel before its product with D, and S[o,:o]^T
   const int64_t cap = (int64_t)batch * rows * OB, pb = rows * OB;
   float* a_lo = a_hi + cap;
-  float* q_base = a_lo + cap;                             // the update's second operand, two copies used in turn
+  float* p_all = a_lo + cap;                              // the other rows of P
+  __half* q_base = (__half*)(p_all + cap);                // the update's operand, two copies used in turn
+  float* q_scales = (float*)(q_base + 4 * cap);
   const size_t chol_smem = kCholSmemFloats * sizeof(float), panel_smem = kPanelSmemFloats * sizeof(float);
   B200Q_TRY(cudaFuncSetAttribute(chol_diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)chol_smem));
   B200Q_TRY(cudaFuncSetAttribute(panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)panel_smem));
@@ -603,14 +595,16 @@ static int factor(float* H, float* const* Hs, int batch, int64_t K, int64_t ldh,
       B200Q_LAUNCH_CHECK();
     }
     if (K0 == 0 && last) break;
-    float* q_hi = q_base + (step & 1) * 2 * cap;
-    float* q_lo = q_hi + cap;
+    float* f_hi = f_base + (step & 1) * 2 * batch * (int64_t)OB * OB;
+    float* f_lo = f_hi + batch * (int64_t)OB * OB;
+    __half* q_hi = q_base + (step & 1) * 2 * cap;
+    __half* q_lo = q_hi + cap;
+    float* q_scale = q_scales + (step & 1) * (int64_t)batch * rows;
     const Operand D{d_hi, d_lo, OB, (int64_t)batch * OB, OB, 0}, Pan{a_hi, a_lo, OB, (int64_t)batch * rows, rows, 0},
-        Q{q_hi, q_lo, OB, (int64_t)batch * rows, rows, 0};
+        F{f_hi, f_lo, OB, (int64_t)batch * OB, OB, 0}, Q{q_hi, q_lo, OB, (int64_t)batch * rows, rows, 0, q_scale};
     const int n2 = last ? 0 : (int)(K - K1 < OB ? K - K1 : OB);
     if (side_busy) B200Q_TRY(cudaStreamWaitEvent(st, side->done, 0));   // products of the step before
-    B200Q_TRY(launch_chained(split_square_kernel, dim3(OB / 32 * (OB / 32), batch), 256, 0, st, mt, (int)K0, n, d_hi, d_lo,
-                             last ? nullptr : q_hi, q_lo, pb));
+    B200Q_TRY(launch_chained(split_square_kernel, dim3(OB / 32 * (OB / 32), batch), 256, 0, st, mt, (int)K0, n, d_hi, d_lo));
     B200Q_LAUNCH_CHECK();
     auto split_panel = [&](int64_t r0, int64_t r1, int64_t tcols, cudaStream_t on) -> int {
       const int64_t tiles = ((r1 - r0 + 31) / 32 + tcols / 32) * ((n + 31) / 32);
@@ -631,11 +625,11 @@ static int factor(float* H, float* const* Hs, int batch, int64_t K, int64_t ldh,
         B200Q_TRY(cudaStreamWaitEvent(bulk, side->ready, 0));
       }
       Job f = j;
-      f.A.row0 = (int)K1; f.M = n2; f.out_hi = q_hi; f.out_lo = q_lo; f.out_row0 = (int)K1;
+      f.A.row0 = (int)K1; f.M = n2; f.out_hi = f_hi; f.out_lo = f_lo; f.out_batch = (int64_t)OB * OB;
       B200Q_RC(tgemm::launch(f, st));
       if (side) B200Q_TRY(cudaEventRecord(side->next, st));
       Job d;
-      d.A = d.B = Q; d.A.row0 = d.B.row0 = (int)K1; d.M = d.N = n2; d.Kd = n; d.set = tgemm::kLower; d.batch = batch;
+      d.A = d.B = F; d.M = d.N = n2; d.Kd = n; d.set = tgemm::kLower; d.batch = batch;
       d.alpha = -1.0f; d.beta = 1.0f; d.C = mt.A + K1 * (lda + 1); d.c_batch = mt.batch; d.ldc = lda;
       d.status = status + 2; d.status_stride = 4; d.slice = slice;
       B200Q_RC(tgemm::launch(d, st));
@@ -646,18 +640,25 @@ static int factor(float* H, float* const* Hs, int batch, int64_t K, int64_t ldh,
     B200Q_RC(split_panel(K1 + n2, K, K0, bulk));
     Job r = j;
     r.set = tgemm::kPanel; r.skip0 = (int)K0; r.skip1 = (int)(K1 + n2); r.M = (int)K;
-    if (!last) { r.out_hi = q_hi; r.out_lo = q_lo; }
+    if (!last) r.out_hi = p_all;
     r.X = mt.A + K0 * lda; r.x_batch = mt.batch; r.ldx = lda; r.xt_rows = (int)K0;
     r.max_ctas = side && !last ? kNumSMs - chain_reserve(K) : 0;
     B200Q_RC(tgemm::launch(r, bulk));
     if (last) break;
     if (side) B200Q_TRY(cudaStreamWaitEvent(bulk, side->next, 0));
+    // the update's operand: X[o,:o]^T and D^T, P (of the next block's rows from its operand form)
+    B200Q_RC(tgemm::split_transposed16(mt.A + K0 * lda, nullptr, 0, mt.batch, lda, n, K1, K0, q_hi, q_lo, q_scale, OB, rows, batch,
+                                       bulk));
+    B200Q_RC(tgemm::split_rows16(f_hi, f_lo, OB, (int64_t)OB * OB, n2, n, q_hi + K1 * OB, q_lo + K1 * OB, q_scale + K1, OB, rows,
+                                 batch, bulk));
+    B200Q_RC(tgemm::split_rows16(p_all + (K1 + n2) * OB, nullptr, OB, pb, K - K1 - n2, n, q_hi + (K1 + n2) * OB,
+                                 q_lo + (K1 + n2) * OB, q_scale + K1 + n2, OB, rows, batch, bulk));
     // S[below,o] = -P D, S[i,:o] -= P_i X[o,:o], A[i,j] -= P_i P_j^T, without the next square
     Job u;
     u.A = Q; u.B = Q; u.A.row0 = 0; u.M = u.N = (int)K; u.Kd = n; u.set = tgemm::kBulk; u.batch = batch;
     u.row_begin = (int)K1; u.skip0 = (int)K1; u.skip1 = (int)(K1 + n2);
     u.alpha = -1.0f; u.beta = 1.0f; u.C = mt.A; u.c_batch = mt.batch; u.ldc = lda; u.fresh0 = (int)K0; u.fresh1 = (int)K1;
-    u.status = status + 2; u.status_stride = 4; u.max_ctas = r.max_ctas; u.slice = slice;
+    u.status = status + 2; u.status_stride = 4; u.max_ctas = r.max_ctas; u.slice = slice16;
     B200Q_RC(tgemm::launch(u, bulk));
     if (side) {
       B200Q_TRY(cudaEventRecord(side->done, bulk));

@@ -45,7 +45,7 @@ struct Params {
   int strategy, group_size, block_h, zp_kind;
   int64_t groups_per_row;
   QRange qr;
-  float* err_hi; float* err_lo; int64_t lde, err_batch;   // operand form of the superblock's errors (null: nothing after it)
+  float* err; int64_t lde, err_batch;                     // the superblock's errors (null: nothing after it)
   int i1, sb;                                             // superblock: first column, width
   int sdtype;                                             // of the scales
   const unsigned char* tiles; int64_t tiles_batch;        // operand form of U[i1 : i1 + sb, i1 : i1 + sb], one a factor
@@ -152,25 +152,11 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t saddr) {
 __host__ __device__ constexpr uint32_t instr_desc(int n) {
   return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((128u >> 4) << 24);
 }
-// ---- operands of the products inside a superblock: float32 values as two halves
-// x * 2^k = hi + lo with |x| * 2^k < 2^15: eleven bits each, as the tf32 halves of tgemm have, at half their bytes and
-// twice their rate.  k belongs to a row of U^T (a column of the superblock) or to a row of a micro-block's errors, so
-// that values down to 2^-18 of the row's largest keep all 22 bits, and smaller ones are off by 2^-40 of it at most.
-// (float of 2^k, exponent field of the row's largest value) -> the scale, its inverse
-__device__ __forceinline__ void row_scale(float largest, float& scale, float& inverse) {
-  int k = 141 - (int)(__float_as_uint(largest) >> 23);
-  k = min(max(k, -112), 126);
-  scale = __uint_as_float((uint32_t)(127 + k) << 23);
-  inverse = __uint_as_float((uint32_t)(127 - k) << 23);
-}
-// the hi halves of two neighbours and their lo halves
-__device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi, uint32_t& lo) {
-  const __half2 h = __floats2half2_rn(a, b);
-  const float2 f = __half22float2(h);
-  const __half2 l = __floats2half2_rn(a - f.x, b - f.y);
-  hi = *reinterpret_cast<const uint32_t*>(&h);
-  lo = *reinterpret_cast<const uint32_t*>(&l);
-}
+// ---- operands of the products inside a superblock
+// Float32 values as two halves with a scale per operand row, as tgemm has them: a row is a column of the superblock (of
+// U^T), or a row of a micro-block's errors.
+using tgemm::row_scale;
+using tgemm::split_pair;
 
 // U[i1 : i1 + sb, i1 : i1 + sb] as the tiles that the sweep copies into shared memory: tile (micro-block m, block b) holds
 // for each of the block's 128 columns 16 hi and 16 lo halves of the micro-block's rows of U, in 64-byte rows swizzled as
@@ -310,7 +296,7 @@ __device__ __forceinline__ float dequant(float q, float s, float z) {
 //   MMA      U^T[128 columns, 16] E[16, rows] for everything from kLag micro-blocks on, accumulators in TMEM (two sets)
 //   helpers  hold the columns of W in registers (a lane each, all rows), add the products to them, hand them over
 //            when their turn comes and write the codes out when the chain is past, while it goes on
-//   out      errors out as operand of the trailing product, losses;  params  scales and zero points, copies of U
+//   out      errors out for the trailing product, losses;  params  scales and zero points, copies of U
 // U comes as tiles that one bulk copy brings in (as 64-byte rows of a tensor map it arrived at 18 bytes a clock and SM).
 template <int ROWS, int SBLK, bool SB, int KIND, bool ZP>
 __global__ void __launch_bounds__(Shape<ROWS, SBLK>::kThreads, 1)
@@ -600,10 +586,10 @@ sweep_block_kernel(const __grid_constant__ Params p) {
     }
   };
   auto out_role = [&] {
-    // ---- errors of 32 rows: out as operand of the trailing product, into the losses
+    // ---- errors of 32 rows: out for the trailing product, into the losses
     const int r = (warp - S::kOut) * 32 + lane;
     const int64_t row = row0 + r;
-    const bool live = row < p.N, out = p.err_hi && live;   // (a superblock with columns after it is a whole one)
+    const bool live = row < p.N, out = p.err && live;   // (a superblock with columns after it is a whole one)
     float loss = 0.0f;
 #pragma unroll 1
     for (int m = 0; m < micros; ++m) {
@@ -613,18 +599,13 @@ sweep_block_kernel(const __grid_constant__ Params p) {
       float sum = 0.0f;
 #pragma unroll 1
       for (int t = 0; t < kMicro; t += 4) {
-        float hi[4], lo[4];
+        float x[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          const float x = es[(t + k) * ROWS];
-          sum = fmaf(x, x, sum);
-          hi[k] = tgemm::tf32_rn(-x);
-          lo[k] = tgemm::tf32_rn(-x - hi[k]);
+          x[k] = -es[(t + k) * ROWS];
+          sum = fmaf(x[k], x[k], sum);
         }
-        if (out) {
-          *reinterpret_cast<float4*>(p.err_hi + at + t) = make_float4(hi[0], hi[1], hi[2], hi[3]);
-          *reinterpret_cast<float4*>(p.err_lo + at + t) = make_float4(lo[0], lo[1], lo[2], lo[3]);
-        }
+        if (out) *reinterpret_cast<float4*>(p.err + at + t) = make_float4(x[0], x[1], x[2], x[3]);
       }
       __syncwarp();
       if (lane == 0) bar_arrive(smem_u32(&s_out[m]));
@@ -837,8 +818,9 @@ static bool look_ahead(int64_t ctas) { return ctas <= kNumSMs / 2; }
 
 struct Layout {
   int rows, sb, sets;
-  int64_t ctas, rows_n, rows_k, err, ub;   // CTAs, rows per problem of the operands; floats of one hi or lo array
+  int64_t ctas, rows_n, rows_k, err, ub;   // CTAs, rows per problem of the operands; elements of the errors and of U's slice
   int64_t tiles;                           // bytes of the tiles of all factors
+  size_t set;                              // bytes of a set: errors, their halves and scales, the slice's, the tiles
   size_t bytes;
 };
 static Layout layout_of(int64_t N, int64_t K, int batch, int distinct_u, bool may_overlap) {
@@ -850,7 +832,8 @@ static Layout layout_of(int64_t N, int64_t K, int batch, int distinct_u, bool ma
   l.rows_n = (N + 127) / 128 * 128; l.rows_k = (K + 127) / 128 * 128;
   l.err = K > l.sb ? l.rows_n * l.sb * batch : 0; l.ub = K > l.sb ? l.rows_k * l.sb * distinct_u : 0;
   l.tiles = tiles_bytes(l.sb) * distinct_u;
-  l.bytes = kSweepHeaderBytes + (size_t)(2 * l.sets * (l.err + l.ub)) * sizeof(float) + (size_t)(l.sets * l.tiles) + 64;
+  l.set = (size_t)(2 * l.err + l.ub) * sizeof(float) + (size_t)(l.err + l.ub) / l.sb * sizeof(float) + (size_t)l.tiles;
+  l.bytes = kSweepHeaderBytes + l.sets * l.set + 64;
   return l;
 }
 
@@ -876,9 +859,16 @@ static int sweep(Params p, int sdtype, bool global, int batch, const float* cons
   // header of the workspace: a status word that a bounded wait expiring in a sweep or a trailing product sets to
   // B200Q_ERR_DEVICE (cleared here, read by the caller afterwards)
   int* status = (int*)workspace;
-  float* err = (float*)((char*)workspace + kSweepHeaderBytes);   // [sets][hi, lo]
-  float* ub = err + 2 * l.sets * l.err;                          // [sets][hi, lo]
-  unsigned char* tiles = (unsigned char*)(ub + 2 * l.sets * l.ub);   // [sets][factor]
+  struct Set { float* err; __half *e_hi, *e_lo, *u_hi, *u_lo; float *e_scale, *u_scale; unsigned char* tiles; };
+  auto set = [&](int which) {
+    Set t;
+    t.err = (float*)((char*)workspace + kSweepHeaderBytes + which * l.set);
+    t.e_hi = (__half*)(t.err + l.err); t.e_lo = t.e_hi + l.err;
+    t.u_hi = t.e_lo + l.err; t.u_lo = t.u_hi + l.ub;
+    t.e_scale = (float*)(t.u_lo + l.ub); t.u_scale = t.e_scale + l.err / l.sb;
+    t.tiles = (unsigned char*)(t.u_scale + l.ub / l.sb);
+    return t;
+  };
   B200Q_TRY(cudaMemsetAsync(status, 0, sizeof(int), st));
   if (sdtype != B200Q_BF16 && sdtype != B200Q_F32) return B200Q_ERR_UNSUPPORTED;
   p.sdtype = sdtype; p.status = status; p.u_index = u_index; p.tiles_batch = tiles_bytes(l.sb);
@@ -902,12 +892,12 @@ static int sweep(Params p, int sdtype, bool global, int batch, const float* cons
   auto split_u = [&](int64_t i1, int which, cudaStream_t on) -> int {
     const int w = (int)(K - i1 < l.sb ? K - i1 : l.sb);
     const int64_t i2 = i1 + w;
-    float* hi = ub + (int64_t)which * 2 * l.ub;
+    const Set t = set(which);
     B200Q_TRY(launch_chained(square, dim3((w + 31) / 32, distinct_u), kTileThreads, square_smem, on, factors, p.ldu, (int)i1,
-                             w, tiles + which * l.tiles, p.tiles_batch));
+                             w, t.tiles, p.tiles_batch));
     B200Q_LAUNCH_CHECK();
-    return tgemm::split_transposed(p.U.one ? p.U.one + i1 * p.ldu + i2 : nullptr, Ud, i1 * p.ldu + i2, p.ldu, w,
-                                   (int)(K - i2), hi, hi + l.ub, l.sb, l.rows_k * l.sb, distinct_u, on);
+    return tgemm::split_transposed16(p.U.one ? p.U.one + i1 * p.ldu + i2 : nullptr, Ud, i1 * p.ldu + i2, 0, p.ldu, w, K - i2,
+                                     INT64_MAX / 2, t.u_hi, t.u_lo, t.u_scale, l.sb, l.rows_k, distinct_u, on);
   };
   if (has_u && (rc = split_u(0, 0, st))) return rc;
   int blk = 0;
@@ -915,11 +905,10 @@ static int sweep(Params p, int sdtype, bool global, int batch, const float* cons
     const int w = (int)(K - i1 < l.sb ? K - i1 : l.sb), which = l.sets == 2 ? blk & 1 : 0;
     const int64_t i2 = i1 + w;
     const bool trailing = i2 < K && has_u;
-    float* bhi = ub + (int64_t)which * 2 * l.ub;
+    const Set t = set(which);
     p.i1 = (int)i1; p.sb = w;
-    p.err_hi = trailing ? err + (int64_t)which * 2 * l.err : nullptr;
-    p.err_lo = trailing ? p.err_hi + l.err : nullptr;
-    p.tiles = tiles + which * l.tiles; p.lde = l.sb; p.err_batch = l.rows_n * l.sb;
+    p.err = trailing ? t.err : nullptr;
+    p.tiles = t.tiles; p.lde = l.sb; p.err_batch = l.rows_n * l.sb;
     if (trailing && side) {
       // the next superblock's slice of U: its buffer was last read by the products of the superblock before this one
       B200Q_TRY(cudaEventRecord(side->next, st));
@@ -931,9 +920,11 @@ static int sweep(Params p, int sdtype, bool global, int batch, const float* cons
     B200Q_LAUNCH_CHECK();
     if (!trailing) continue;
     // W[:, i2:] -= Err[N, w] * U[i1:i2, i2:]
+    if ((rc = tgemm::split_rows16(t.err, nullptr, l.sb, p.err_batch, N, w, t.e_hi, t.e_lo, t.e_scale, l.sb, l.rows_n, batch, st)))
+      return rc;
     tgemm::Job j;
-    j.A = tgemm::Operand{p.err_hi, p.err_lo, l.sb, l.rows_n * batch, l.rows_n, 0};
-    j.B = tgemm::Operand{bhi, bhi + l.ub, l.sb, l.rows_k * distinct_u, l.rows_k, 0};
+    j.A = tgemm::Operand{t.e_hi, t.e_lo, l.sb, l.rows_n * batch, l.rows_n, 0, t.e_scale};
+    j.B = tgemm::Operand{t.u_hi, t.u_lo, l.sb, l.rows_k * distinct_u, l.rows_k, 0, t.u_scale};
     j.b_index = u_index;
     j.M = (int)N; j.N = (int)(K - i2); j.Kd = w; j.batch = batch; j.alpha = -1.0f; j.beta = 1.0f;
     if (p.W.one) j.C = p.W.one + i2;
@@ -941,7 +932,7 @@ static int sweep(Params p, int sdtype, bool global, int batch, const float* cons
     // a batch: error of the last of 2048 columns 2.6e-7 of its root mean square, with long slices 7.5e-7, by float32
     // multiply-adds 4.1e-7; 64 weights of 768 x 2048: 4.0 ms, 3.8 with long slices.  The single weight keeps the long
     // ones (6.4e-7; 8.8e-7 when its products had rank 128).
-    j.slice = p.W.table ? tgemm::kShortSlice : tgemm::kLongSlice;
+    j.slice = p.W.table ? tgemm::kShortSlice16 : tgemm::kLongSlice16;
     if (!side) {
       if ((rc = tgemm::launch(j, st))) return rc;
       if ((rc = split_u(i2, l.sets == 2 ? which ^ 1 : 0, st))) return rc;

@@ -9,7 +9,7 @@
 //
 // Structure: persistent CTAs, each with a contiguous range of the tile list (128 x TN tiles).  Warp 0
 // streams 32-deep chunks of both operands (A_hi, A_lo, B_hi, B_lo) through a shared-memory ring by
-// TMA.  Warp 1 issues the MMAs and owns TMEM.  A contraction is cut into slices of 128 or 32 terms:
+// TMA.  Warp 1 issues the MMAs and owns TMEM.  A contraction is cut into slices of 32 to 128 terms:
 // each slice accumulates in its own TMEM buffer (two, used in turn) and the epilogue (warps 4-11) adds
 // the slices in registers, so no tensor-core accumulation chain is longer than that whatever Kd is, and
 // C is read and written once per launch.
@@ -20,6 +20,9 @@
 // Why three tile widths: the operands of a chunk come from L2 at 64 B/clk and SM for TN = 256, 85 for
 // 128 and 128 for 64, so wide tiles run closer to the tensor pipe, narrow ones spread a small update
 // over more SMs; pick_tiles() takes whatever finishes its waves first, CTA pairs of 256 x 256 among them.
+//
+// Operands of halves (kind::f16, "3xFP16" with a power-of-two scale per operand row) run the same way with chunks of 64
+// terms: half the bytes and half the MMAs for as many bits.  The scales go onto the finished sums.
 //
 // All mbarrier waits are bounded.  CTA pairs are clusters of two; no load is multicast.
 #include <cuda.h>
@@ -33,8 +36,9 @@
 namespace b200q {
 namespace tgemm {
 
-constexpr int kChunkK = 32;                          // fp32 elements per 128-byte row
-constexpr int kAPart = kTile * kChunkK * 4;          // A_hi or A_lo of a chunk: 16 KiB
+constexpr int kChunkBytes = 128;                     // of an operand row: 32 floats or 64 halves
+constexpr int kChunkK = kChunkBytes / 4, kChunkK16 = kChunkBytes / 2;
+constexpr int kAPart = kTile * kChunkBytes;          // A_hi or A_lo of a chunk: 16 KiB
 constexpr int kRingBytes = 196608;                   // 2, 3 or 4 stages for TN = 256, 128, 64
 constexpr int kEpiWarps = 8;                         // two per TMEM lane quarter, each half of the columns
 constexpr int kEpiBytes = kEpiWarps * 32 * 33 * 4;   // per-warp staging tiles of the epilogue
@@ -110,25 +114,41 @@ __device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
       "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
       ::"r"(bar), "h"(both) : "memory");
 }
-__device__ __forceinline__ void mma_tf32_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+template <bool F16>
+__device__ __forceinline__ void mma_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                               uint32_t accumulate) {
   const uint32_t z = 0;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(z) : "memory");
+  if constexpr (F16)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(z) : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(z) : "memory");
 }
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ void mma_tf32(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                         uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+template <bool F16>
+__device__ __forceinline__ void mma_one(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                        uint32_t accumulate) {
+  if constexpr (F16)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
@@ -153,9 +173,9 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t lbo_bytes
   d |= (uint64_t)2 << 61;
   return d;
 }
-// D fp32, A/B tf32, both K-major, M = tm, N = tn
-__host__ __device__ constexpr uint32_t instr_desc(int tm, int tn) {
-  return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(tn >> 3) << 17) | ((uint32_t)(tm >> 4) << 24);
+// D fp32, A/B tf32 or f16, both K-major, M = tm, N = tn
+__host__ __device__ constexpr uint32_t instr_desc(int tm, int tn, bool f16) {
+  return (1u << 4) | (f16 ? 0u : (2u << 7) | (2u << 10)) | ((uint32_t)(tn >> 3) << 17) | ((uint32_t)(tm >> 4) << 24);
 }
 
 struct Params {
@@ -191,14 +211,15 @@ __device__ __forceinline__ void next_tile(const Params& p, int& b, int& tm, int&
 // PAIR: two CTAs on neighbouring SMs (a cluster of 2) share a 256 x 256 tile.  One MMA issued by the even CTA runs on both
 // SMs; each stages its own 128 rows of A and its own 128 of B, 64 KiB a chunk instead of 96, and has its own half of the
 // accumulator and its own epilogue.  full[] and acc_empty[] live in the even CTA, empty[] and acc_full[] in both.
-template <int TN, bool SPLIT_OUT, bool PAIR>
+template <int TN, bool SPLIT_OUT, bool PAIR, bool F16>
 __global__ void __launch_bounds__(kThreads, 1)
 tgemm_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ CUtensorMap a_lo,
              const __grid_constant__ CUtensorMap b_hi, const __grid_constant__ CUtensorMap b_lo,
              const __grid_constant__ Params p) {
   constexpr int kRows = PAIR ? 2 * kTile : kTile;      // rows of a tile
   constexpr int kBRows = PAIR ? TN / 2 : TN;           // rows of B that this CTA stages
-  constexpr int kBPart = kBRows * kChunkK * 4;
+  constexpr int kBPart = kBRows * kChunkBytes, kChunk = F16 ? kChunkK16 : kChunkK;
+  static_assert(!(F16 && SPLIT_OUT), "");
   constexpr int kStageBytes = 2 * kAPart + 2 * kBPart;
   constexpr int kStages = kRingBytes / kStageBytes;
   constexpr uint32_t kTmemCols = 2 * TN;
@@ -242,7 +263,8 @@ tgemm_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ C
   const uint32_t tmem_base = s_tmem_base;
   chain_wait();
   const Job& j = p.j;
-  const int chunks = (j.Kd + kChunkK - 1) / kChunkK;
+  constexpr int kSteps = kChunkBytes / 32;   // k-steps of a chunk
+  const int chunks = (j.Kd + kChunk - 1) / kChunk;
   const int64_t count = p.num_tiles * (unit + 1) / units - p.num_tiles * unit / units;
   int b = p.start[unit][0], tm = p.start[unit][1], tn = p.start[unit][2];
 
@@ -261,16 +283,16 @@ tgemm_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ C
           if constexpr (PAIR) {
             if (rank == 0) mbar_expect_tx(full_bar(stage), 2 * kStageBytes);
             const uint32_t full = map_to_cta(full_bar(stage), 0);
-            tma_load_2d_pair(s, &a_hi, full, c * kChunkK, ra);
-            tma_load_2d_pair(s + 2 * kAPart, &b_hi, full, c * kChunkK, rb);
-            tma_load_2d_pair(s + 2 * kAPart + kBPart, &b_lo, full, c * kChunkK, rb);
-            tma_load_2d_pair(s + kAPart, &a_lo, full, c * kChunkK, ra);
+            tma_load_2d_pair(s, &a_hi, full, c * kChunk, ra);
+            tma_load_2d_pair(s + 2 * kAPart, &b_hi, full, c * kChunk, rb);
+            tma_load_2d_pair(s + 2 * kAPart + kBPart, &b_lo, full, c * kChunk, rb);
+            tma_load_2d_pair(s + kAPart, &a_lo, full, c * kChunk, ra);
           } else {
           mbar_expect_tx(full_bar(stage), kStageBytes);
-          tma_load_2d(s, &a_hi, full_bar(stage), c * kChunkK, ra);
-          tma_load_2d(s + 2 * kAPart, &b_hi, full_bar(stage), c * kChunkK, rb);
-          tma_load_2d(s + 2 * kAPart + kBPart, &b_lo, full_bar(stage), c * kChunkK, rb);
-          tma_load_2d(s + kAPart, &a_lo, full_bar(stage), c * kChunkK, ra);
+          tma_load_2d(s, &a_hi, full_bar(stage), c * kChunk, ra);
+          tma_load_2d(s + 2 * kAPart, &b_hi, full_bar(stage), c * kChunk, rb);
+          tma_load_2d(s + 2 * kAPart + kBPart, &b_lo, full_bar(stage), c * kChunk, rb);
+          tma_load_2d(s + kAPart, &a_lo, full_bar(stage), c * kChunk, ra);
           }
           if (++stage == kStages) { stage = 0; phase ^= 1u; }
         }
@@ -280,40 +302,42 @@ tgemm_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ C
     int stage = 0, slice = 0;
     uint32_t phase = 0;
     bool ok = true;
-    constexpr uint32_t idesc = instr_desc(kRows, TN);
+    constexpr uint32_t idesc = instr_desc(kRows, TN, F16);
     for (int64_t i = 0; i < count && ok; ++i) {
       for (int c = 0; c < chunks; ++c) {
-        const int buf = slice & 1;
-        const bool first = c % j.slice == 0, last = c % j.slice == j.slice - 1 || c == chunks - 1;
-        if (first && !mbar_wait(acce_bar(buf), (uint32_t)(((slice >> 1) & 1) ^ 1), &s_abort)) { ok = false; break; }
         if (!mbar_wait(full_bar(stage), phase, &s_abort)) { ok = false; break; }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (lane == 0) {
-          const uint32_t d_tmem = tmem_base + (uint32_t)(buf * TN);
-          const uint32_t sa = base + stage * kStageBytes, sb = sa + 2 * kAPart;
-          // K-major, 128-byte rows: 8-row groups 1024 bytes apart; a k-step of 8 tf32 is 32 bytes
-          auto mma = [&](uint32_t x, uint32_t y, uint32_t accumulate) {
-            if constexpr (PAIR) mma_tf32_pair(d_tmem, make_desc(x, 16, 1024), make_desc(y, 16, 1024), idesc, accumulate);
-            else mma_tf32(d_tmem, make_desc(x, 16, 1024), make_desc(y, 16, 1024), idesc, accumulate);
-          };
-          // the small products first: in a short slice they lose next to nothing, the sum being as small as they are
-#pragma unroll
-          for (int kk = 0; kk < kChunkK / 8; ++kk) {
-            mma(sa + kk * 32, sb + kBPart + kk * 32, (first && kk == 0) ? 0u : 1u);
-            mma(sa + kAPart + kk * 32, sb + kk * 32, 1u);
+        const uint32_t sa = base + stage * kStageBytes, sb = sa + 2 * kAPart;
+        const int part = j.slice < kSteps ? j.slice : kSteps;   // k-steps of this chunk that one slice takes
+        for (int k0 = 0; k0 < kSteps && ok; k0 += part) {
+          const int buf = slice & 1, at = c * kSteps + k0;
+          const bool first = at % j.slice == 0, last = (at + part) % j.slice == 0 || (c == chunks - 1 && k0 + part == kSteps);
+          if (first && !mbar_wait(acce_bar(buf), (uint32_t)(((slice >> 1) & 1) ^ 1), &s_abort)) { ok = false; break; }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          if (lane == 0) {
+            const uint32_t d_tmem = tmem_base + (uint32_t)(buf * TN);
+            // K-major, 128-byte rows: 8-row groups 1024 bytes apart; a k-step of 8 tf32 or 16 halves is 32 bytes
+            auto mma = [&](uint32_t x, uint32_t y, uint32_t accumulate) {
+              if constexpr (PAIR) mma_pair<F16>(d_tmem, make_desc(x, 16, 1024), make_desc(y, 16, 1024), idesc, accumulate);
+              else mma_one<F16>(d_tmem, make_desc(x, 16, 1024), make_desc(y, 16, 1024), idesc, accumulate);
+            };
+            // the small products first: in a short slice they lose next to nothing, the sum being as small as they are
+            for (int kk = k0; kk < k0 + part; ++kk) {
+              mma(sa + kk * 32, sb + kBPart + kk * 32, (first && kk == k0) ? 0u : 1u);
+              mma(sa + kAPart + kk * 32, sb + kk * 32, 1u);
+            }
+            for (int kk = k0; kk < k0 + part; ++kk) mma(sa + kk * 32, sb + kk * 32, 1u);
+            if (k0 + part == kSteps) {
+              if constexpr (PAIR) tc_commit_pair(empty_bar(stage));
+              else tc_commit(empty_bar(stage));
+            }
+            if (last) {
+              if constexpr (PAIR) tc_commit_pair(accf_bar(buf));
+              else tc_commit(accf_bar(buf));
+            }
           }
-#pragma unroll
-          for (int kk = 0; kk < kChunkK / 8; ++kk) mma(sa + kk * 32, sb + kk * 32, 1u);
-          if constexpr (PAIR) {
-            tc_commit_pair(empty_bar(stage));
-            if (last) tc_commit_pair(accf_bar(buf));
-          } else {
-            tc_commit(empty_bar(stage));
-            if (last) tc_commit(accf_bar(buf));
-          }
+          __syncwarp();
+          if (last) ++slice;
         }
-        __syncwarp();
-        if (last) ++slice;
         if (++stage == kStages) { stage = 0; phase ^= 1u; }
       }
     }
@@ -331,7 +355,15 @@ tgemm_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ C
     for (int64_t i = 0; i < count && ok; ++i, next_tile(p, b, tm, tn)) {
       const int row0 = tile_row(j, tm, kRows) + rank * kTile + q * 32, colw = tn * TN + half * kHalf;
       float sum[kHalf];
-      for (int c = 0; c < chunks; c += j.slice, ++slice) {
+      // scales of halves: the lane's row, a column of every 32 (asked for now, they are needed when the sums are there)
+      float row_factor = j.alpha, col_factor[kHalf / 32];
+      if constexpr (F16) {
+        row_factor *= row0 + lane < j.M ? j.A.scale[(int64_t)b * j.A.batch_rows + j.A.row0 + row0 + lane] : 0.0f;
+        const float* cf = j.B.scale + (j.b_index ? j.b_index[b] : b) * j.B.batch_rows + j.B.row0;
+#pragma unroll
+        for (int k = 0; k < kHalf / 32; ++k) col_factor[k] = colw + k * 32 + lane < j.N ? cf[colw + k * 32 + lane] : 0.0f;
+      }
+      for (int c = 0; c < chunks * kSteps; c += j.slice, ++slice) {
         const int buf = slice & 1;
         if (!mbar_wait(accf_bar(buf), (uint32_t)((slice >> 1) & 1), &s_abort)) { ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -378,13 +410,17 @@ tgemm_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ C
 #pragma unroll
             for (int s = 0; s < 8; ++s) {
               const int lr = s * 4 + sub_row, row = row0 + lr;
-              if (row < j.M) {
+              if (row < j.M && (j.out_lo || row >= j.xt_rows)) {
                 const float* sp = stage + lr * 33 + sub_col;
+                const int64_t at = (int64_t)b * j.out_batch + (int64_t)(row + j.out_row0) * j.out_ld + cc;
+                if (!j.out_lo) {
+                  *reinterpret_cast<float4*>(j.out_hi + at) = make_float4(sp[0], sp[1], sp[2], sp[3]);
+                  continue;
+                }
                 float4 h, l;
                 h.x = tf32_rn(sp[0]); h.y = tf32_rn(sp[1]); h.z = tf32_rn(sp[2]); h.w = tf32_rn(sp[3]);
                 l.x = tf32_rn(sp[0] - h.x); l.y = tf32_rn(sp[1] - h.y);
                 l.z = tf32_rn(sp[2] - h.z); l.w = tf32_rn(sp[3] - h.w);
-                const int64_t at = (int64_t)b * j.out_batch + (int64_t)(row + j.out_row0) * j.out_ld + cc;
                 *reinterpret_cast<float4*>(j.out_hi + at) = h;
                 *reinterpret_cast<float4*>(j.out_lo + at) = l;
               }
@@ -394,8 +430,14 @@ tgemm_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ C
         } else {
           const float beta = (col0 >= j.fresh0 && col0 < j.fresh1) ? 0.0f : j.beta;
           const bool fast = vec && col0 + 31 < j.N;
+          float4 f = make_float4(1.f, 1.f, 1.f, 1.f);   // of the four columns that this lane writes
+          if constexpr (F16) {
+            f.x = __shfl_sync(0xffffffffu, col_factor[k], sub_col); f.y = __shfl_sync(0xffffffffu, col_factor[k], sub_col + 1);
+            f.z = __shfl_sync(0xffffffffu, col_factor[k], sub_col + 2); f.w = __shfl_sync(0xffffffffu, col_factor[k], sub_col + 3);
+          }
+          const float fs[4] = {f.x, f.y, f.z, f.w};
 #pragma unroll
-          for (int e = 0; e < 32; ++e) stage[lane * 33 + e] = sum[k * 32 + e] * j.alpha;
+          for (int e = 0; e < 32; ++e) stage[lane * 33 + e] = sum[k * 32 + e] * row_factor;
           __syncwarp();
           if (fast) {
             float* c = C + (int64_t)(row0 + sub_row) * j.ldc + cc;
@@ -405,7 +447,7 @@ tgemm_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ C
                 const int lr = s * 4 + sub_row;
                 if (row0 + lr < j.M) {
                   const float* sp = stage + lr * 33 + sub_col;
-                  red_add_v4(c + (int64_t)(s * 4) * j.ldc, sp[0], sp[1], sp[2], sp[3]);
+                  red_add_v4(c + (int64_t)(s * 4) * j.ldc, sp[0] * f.x, sp[1] * f.y, sp[2] * f.z, sp[3] * f.w);
                 }
               }
             } else {
@@ -424,8 +466,8 @@ tgemm_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ C
                 if (row0 + lr < j.M) {
                   const float* sp = stage + lr * 33 + sub_col;
                   float4 o;
-                  o.x = beta * h[s].x + sp[0]; o.y = beta * h[s].y + sp[1];
-                  o.z = beta * h[s].z + sp[2]; o.w = beta * h[s].w + sp[3];
+                  o.x = beta * h[s].x + sp[0] * f.x; o.y = beta * h[s].y + sp[1] * f.y;
+                  o.z = beta * h[s].z + sp[2] * f.z; o.w = beta * h[s].w + sp[3] * f.w;
                   *reinterpret_cast<float4*>(c + (int64_t)((s0 + s) * 4) * j.ldc) = o;
                 }
               }
@@ -439,7 +481,7 @@ tgemm_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ C
                 if (cc + e < j.N) {
                   float* d = C + (int64_t)row * j.ldc + cc + e;
                   const float old = (beta != 0.0f) ? *d : 0.0f;
-                  *d = beta * old + stage[lr * 33 + sub_col + e];
+                  *d = beta * old + stage[lr * 33 + sub_col + e] * fs[e];
                 }
             }
           }
@@ -526,6 +568,100 @@ __global__ void __launch_bounds__(256) split_transposed_kernel(const float* __re
   }
 }
 
+// Halves of rows: a warp takes a row, kept in registers between the search for its largest value and the split.
+template <int LD>
+__global__ void __launch_bounds__(256) split_rows16_kernel(const float* __restrict__ src, const float* __restrict__ src2,
+                                                           int64_t ld_src, int64_t src_batch, int64_t rows, int cols,
+                                                           __half* hi, __half* lo, float* scale, int64_t dst_rows) {
+  chain_wait();
+  chain_go();
+  constexpr int kParts = LD / 128;
+  const int lane = threadIdx.x & 31;
+  src += blockIdx.y * src_batch;
+  if (src2) src2 += blockIdx.y * src_batch;
+  for (int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); r < rows; r += (int64_t)gridDim.x * 8) {
+    float4 x[kParts], y[kParts];
+    const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < kParts; ++i) x[i] = *reinterpret_cast<const float4*>(src + r * ld_src + i * 128 + lane * 4);
+#pragma unroll
+    for (int i = 0; i < kParts; ++i) y[i] = src2 ? *reinterpret_cast<const float4*>(src2 + r * ld_src + i * 128 + lane * 4) : none;
+    float largest = 0.0f;
+#pragma unroll
+    for (int i = 0; i < kParts; ++i) {
+      x[i].x += y[i].x; x[i].y += y[i].y; x[i].z += y[i].z; x[i].w += y[i].w;
+      float* e = &x[i].x;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (i * 128 + lane * 4 + k >= cols) e[k] = 0.0f;
+        largest = fmaxf(largest, fabsf(e[k]));
+      }
+    }
+    largest = warp_max(largest);
+    float to, back;
+    row_scale(largest, to, back);
+    const int64_t row = blockIdx.y * dst_rows + r;
+    if (lane == 0) scale[row] = back;
+#pragma unroll
+    for (int i = 0; i < kParts; ++i) {
+      uint2 h, l;
+      split_pair(x[i].x * to, x[i].y * to, h.x, l.x);
+      split_pair(x[i].z * to, x[i].w * to, h.y, l.y);
+      *reinterpret_cast<uint2*>(hi + row * LD + i * 128 + lane * 4) = h;
+      *reinterpret_cast<uint2*>(lo + row * LD + i * 128 + lane * 4) = l;
+    }
+  }
+}
+// Halves of columns, as operand rows: a CTA takes 32 of them.
+template <int LD>
+__global__ void __launch_bounds__(256) split_transposed16_kernel(const float* __restrict__ src0,
+                                                                 const float* const* __restrict__ table, int64_t src_offset,
+                                                                 int64_t src_batch, int64_t ld_src, int rows, int64_t cols,
+                                                                 int64_t diagonal, __half* hi, __half* lo, float* scale,
+                                                                 int64_t dst_rows) {
+  chain_wait();
+  chain_go();
+  extern __shared__ float stage16[];   // [32][LD + 2]
+  __shared__ float s_max[8][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const float* src = table ? table[blockIdx.y] + src_offset : src0 + blockIdx.y * src_batch;
+  const int64_t c = (int64_t)blockIdx.x * 32 + lane, last = c < cols ? c : cols - 1;
+  float v[LD / 8], largest = 0.0f;
+  // (no load depends on a condition: they go out together)
+#pragma unroll
+  for (int i = 0; i < LD / 8; ++i) v[i] = src[(int64_t)min(warp + i * 8, rows - 1) * ld_src + last];
+#pragma unroll
+  for (int i = 0; i < LD / 8; ++i) {
+    const int p = warp + i * 8;
+    if (p >= rows || c >= cols || c > diagonal + p) v[i] = 0.0f;
+    largest = fmaxf(largest, fabsf(v[i]));
+  }
+  s_max[warp][lane] = largest;
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < 8; ++k) largest = fmaxf(largest, s_max[k][lane]);
+  float to, back;
+  row_scale(largest, to, back);
+  const int64_t row0 = blockIdx.y * dst_rows + (int64_t)blockIdx.x * 32;
+  if (warp == 0 && c < cols) scale[row0 + lane] = back;
+#pragma unroll
+  for (int i = 0; i < LD / 8; ++i) stage16[lane * (LD + 2) + warp + i * 8] = v[i] * to;
+  __syncthreads();
+  for (int k = warp; k < 32; k += 8) {
+    if ((int64_t)blockIdx.x * 32 + k >= cols) break;
+    uint32_t* h = reinterpret_cast<uint32_t*>(hi + (row0 + k) * LD);
+    uint32_t* l = reinterpret_cast<uint32_t*>(lo + (row0 + k) * LD);
+#pragma unroll
+    for (int i = 0; i < LD / 64; ++i) {
+      const float2 x = *reinterpret_cast<const float2*>(stage16 + k * (LD + 2) + i * 64 + lane * 2);
+      uint32_t a, b;
+      split_pair(x.x, x.y, a, b);
+      h[i * 32 + lane] = a;
+      l[i * 32 + lane] = b;
+    }
+  }
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -542,15 +678,15 @@ inline EncodeTiledFn encode_fn() {
   }();
   return fn;
 }
-// fp32 matrix [rows][ld], boxes of [box_rows][32 columns]
-inline bool make_map(CUtensorMap* m, const float* base, int64_t rows, int64_t ld, int box_rows) {
+// matrix [rows][ld] of floats or halves, boxes of box_rows rows of 128 bytes
+inline bool make_map(CUtensorMap* m, const void* base, int64_t rows, int64_t ld, int box_rows, bool f16) {
   EncodeTiledFn enc = encode_fn();
   if (!enc) return false;
   cuuint64_t dims[2] = {(cuuint64_t)ld, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)ld * 4};
-  cuuint32_t box[2] = {32u, (cuuint32_t)box_rows};
+  cuuint64_t strides[1] = {(cuuint64_t)ld * (f16 ? 2 : 4)};
+  cuuint32_t box[2] = {f16 ? (cuuint32_t)kChunkK16 : (cuuint32_t)kChunkK, (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1, 1};
-  return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base), dims, strides, box, estr,
+  return enc(m, f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box, estr,
              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
@@ -576,23 +712,46 @@ int split_transposed(const float* src, const float* const* table, int64_t src_of
   return B200Q_OK;
 }
 
+int split_rows16(const float* src, const float* src2, int64_t ld_src, int64_t src_batch, int64_t rows, int cols, __half* hi,
+                 __half* lo, float* scale, int ld, int64_t dst_rows, int batch, cudaStream_t st) {
+  if (rows <= 0 || cols <= 0) return B200Q_OK;
+  auto kernel = ld == 512 ? split_rows16_kernel<512> : split_rows16_kernel<256>;
+  const int64_t blocks = (rows + 7) / 8, cap = 8 * kNumSMs / batch + 1;
+  B200Q_TRY(launch_chained(kernel, dim3((unsigned)(blocks < cap ? blocks : cap), (unsigned)batch), 256, 0, st, src, src2, ld_src,
+                           src_batch, rows, cols, hi, lo, scale, dst_rows));
+  B200Q_LAUNCH_CHECK();
+  return B200Q_OK;
+}
+int split_transposed16(const float* src, const float* const* table, int64_t src_offset, int64_t src_batch, int64_t ld_src,
+                       int rows, int64_t cols, int64_t diagonal, __half* hi, __half* lo, float* scale, int ld, int64_t dst_rows,
+                       int batch, cudaStream_t st) {
+  if (rows <= 0 || cols <= 0) return B200Q_OK;
+  auto kernel = ld == 512 ? split_transposed16_kernel<512> : split_transposed16_kernel<256>;
+  const size_t smem = 32 * (ld + 2) * sizeof(float);
+  B200Q_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  B200Q_TRY(launch_chained(kernel, dim3((unsigned)((cols + 31) / 32), (unsigned)batch), 256, smem, st, src, table, src_offset,
+                           src_batch, ld_src, rows, cols, diagonal, hi, lo, scale, dst_rows));
+  B200Q_LAUNCH_CHECK();
+  return B200Q_OK;
+}
+
 // Tensor maps are cached per (array, shape, box): one encode serves every launch that reads an operand
 // buffer.  Rows beyond an operand's extent inside its buffer may hold anything; they only reach
 // output rows / columns that the epilogue masks.  Columns beyond Kd are zero (the splits pad them).
-struct MapKey { const float* base; int64_t ld, rows; int box; };
+struct MapKey { const void* base; int64_t ld, rows; int box; bool f16; };
 struct MapCache {
   static constexpr int kSlots = 32;
   MapKey key[kSlots];
   CUtensorMap map[kSlots];
   int used = 0, next = 0;
   // Copies the map out: a later get() may evict the slot it came from.
-  bool get(const float* base, int64_t ld, int64_t rows, int box, CUtensorMap* out) {
+  bool get(const void* base, int64_t ld, int64_t rows, int box, bool f16, CUtensorMap* out) {
     for (int i = 0; i < used; ++i)
-      if (key[i].base == base && key[i].ld == ld && key[i].rows == rows && key[i].box == box) { *out = map[i]; return true; }
+      if (key[i].base == base && key[i].ld == ld && key[i].rows == rows && key[i].box == box && key[i].f16 == f16) { *out = map[i]; return true; }
     int slot = (used < kSlots) ? used++ : (next++ % kSlots);
-    key[slot] = MapKey{nullptr, 0, 0, 0};
-    if (!make_map(&map[slot], base, rows, ld, box)) return false;
-    key[slot] = MapKey{base, ld, rows, box};
+    key[slot] = MapKey{nullptr, 0, 0, 0, false};
+    if (!make_map(&map[slot], base, rows, ld, box, f16)) return false;
+    key[slot] = MapKey{base, ld, rows, box, f16};
     *out = map[slot];
     return true;
   }
@@ -629,7 +788,7 @@ static int pair_capacity() {
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
   std::lock_guard<std::mutex> lock(mu);
   if (have[dev]) return cached[dev];
-  auto kernel = tgemm_kernel<256, false, true>;
+  auto kernel = tgemm_kernel<256, false, true, false>;
   int n = 0;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) == cudaSuccess) {
     cudaLaunchConfig_t cfg = {};
@@ -649,7 +808,7 @@ static int pair_capacity() {
   return cached[dev];
 }
 
-// Tile width, and whether CTA pairs take 256 x 256: SM cycles of the busiest CTA.  A 32-deep chunk takes the longer of its
+// Tile width, and whether CTA pairs take 256 x 256: SM cycles of the busiest CTA.  A chunk of 128 bytes takes the longer of its
 // MMAs (12 of 32 / 64 / 128 cycles) and the arrival of its operands from L2 (about 64 B/clk and SM); the last tile's
 // epilogue, about 20 cycles per column, is not hidden.
 static void pick_tiles(Params& p, int ctas, int pairs) {
@@ -659,7 +818,7 @@ static void pick_tiles(Params& p, int ctas, int pairs) {
   // 4096 x 14336 6545 / 5879; 1024 rows and K = 2048 the same either way.
   const double pair_chunk = 1600.0;
   const Job& j = p.j;
-  const int chunks = (j.Kd + kChunkK - 1) / kChunkK;
+  const int depth = j.A.scale ? kChunkK16 : kChunkK, chunks = (j.Kd + depth - 1) / depth;
   double best_cost = 0.0;
   for (int w = 6; w <= (j.set == kLowerBlocks ? 7 : 8); ++w) {
     const int64_t tiles = count_tiles(j, kTile, w) * j.batch;
@@ -673,18 +832,18 @@ static void pick_tiles(Params& p, int ctas, int pairs) {
   }
 }
 
-template <int TN, bool SPLIT_OUT, bool PAIR>
+template <int TN, bool SPLIT_OUT, bool PAIR, bool F16>
 static int launch_tiles(const Params& p, int units, cudaStream_t st) {
   const Job& j = p.j;
   constexpr int kBRows = PAIR ? TN / 2 : TN;
   MapCache& mc = map_cache();
   CUtensorMap mah, mal, mbh, mbl;
-  if (!mc.get(j.A.hi, j.A.ld, j.A.rows, kTile, &mah) || !mc.get(j.A.lo, j.A.ld, j.A.rows, kTile, &mal) ||
-      !mc.get(j.B.hi, j.B.ld, j.B.rows, kBRows, &mbh) || !mc.get(j.B.lo, j.B.ld, j.B.rows, kBRows, &mbl)) {
+  if (!mc.get(j.A.hi, j.A.ld, j.A.rows, kTile, F16, &mah) || !mc.get(j.A.lo, j.A.ld, j.A.rows, kTile, F16, &mal) ||
+      !mc.get(j.B.hi, j.B.ld, j.B.rows, kBRows, F16, &mbh) || !mc.get(j.B.lo, j.B.ld, j.B.rows, kBRows, F16, &mbl)) {
     set_last_error("cuTensorMapEncodeTiled (tgemm)", cudaErrorInvalidValue);
     return B200Q_ERR_CUDA;
   }
-  auto kernel = tgemm_kernel<TN, SPLIT_OUT, PAIR>;
+  auto kernel = tgemm_kernel<TN, SPLIT_OUT, PAIR, F16>;
   static thread_local int attr_device = -1;
   int dev = 0;
   B200Q_TRY(cudaGetDevice(&dev));
@@ -715,6 +874,8 @@ static int launch_tiles(const Params& p, int units, cudaStream_t st) {
 
 int launch(const Job& j, cudaStream_t st) {
   if (j.Kd <= 0 || j.batch <= 0) return B200Q_OK;
+  const bool f16 = j.A.scale != nullptr;
+  if (f16 != (j.B.scale != nullptr) || (f16 && ((j.A.ld | j.B.ld) & 63 || j.out_hi || j.X))) return B200Q_ERR_ARG;
   if (j.Kd > kMaxDepth || j.batch > 65535 || (j.A.ld & 31) || (j.B.ld & 31) || j.A.ld < j.Kd || j.B.ld < j.Kd)
     return B200Q_ERR_ARG;
   if (count_rows(j, kTile) <= 0 || j.N <= 0) return B200Q_OK;
@@ -741,10 +902,14 @@ int launch(const Job& j, cudaStream_t st) {
     p.start[i][0] = (uint16_t)b; p.start[i][1] = (uint16_t)tm; p.start[i][2] = (uint16_t)(in - before);
   }
   const bool split_out = j.out_hi || j.X;
-  if (pair) return split_out ? launch_tiles<256, true, true>(p, units, st) : launch_tiles<256, false, true>(p, units, st);
-  if (p.tn_log2 == 8) return split_out ? launch_tiles<256, true, false>(p, units, st) : launch_tiles<256, false, false>(p, units, st);
-  if (p.tn_log2 == 7) return split_out ? launch_tiles<128, true, false>(p, units, st) : launch_tiles<128, false, false>(p, units, st);
-  return split_out ? launch_tiles<64, true, false>(p, units, st) : launch_tiles<64, false, false>(p, units, st);
+#define B200Q_TILES(TN, PAIR)                                                                             \
+  (f16 ? launch_tiles<TN, false, PAIR, true>(p, units, st)                                                \
+       : split_out ? launch_tiles<TN, true, PAIR, false>(p, units, st) : launch_tiles<TN, false, PAIR, false>(p, units, st))
+  if (pair) return B200Q_TILES(256, true);
+  if (p.tn_log2 == 8) return B200Q_TILES(256, false);
+  if (p.tn_log2 == 7) return B200Q_TILES(128, false);
+  return B200Q_TILES(64, false);
+#undef B200Q_TILES
 }
 
 SideStream* side_stream(cudaStream_t like) {

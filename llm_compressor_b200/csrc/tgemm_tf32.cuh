@@ -10,27 +10,50 @@ namespace tgemm {
 
 constexpr int kTile = 128;      // rows of a tile
 constexpr int kMaxDepth = 512;  // largest contraction of one launch
-// Chunks of 32 terms that one tensor-core accumulation runs over, before float32 additions take the sums up.  The tensor
-// core cuts off at every addition, always downwards, so a long run drifts.  Relative error of a batch's factors against
-// float64, 2048 columns of 8192 tokens: 5.6e-7 with four chunks, 1.5e-7 with one; elimination by float32 multiply-adds has
-// 1.7e-7 (768 columns of 4096: 3.5e-7, 1.1e-7, 1.5e-7).  Half a chunk gives 1.4e-7.  64 factors of K = 2048 take 8.3, 9.0
-// and 10.1 ms with four, one and half a chunk, 32 of K = 768 0.65, 0.68 and 0.71.  The single problem keeps four (K = 14336:
-// 11.3 ms, 15.5 with one): 4.2e-7 where rank-128 updates had 6.1e-7.
-constexpr int kLongSlice = 4, kShortSlice = 1;
+// How long one tensor-core accumulation runs before float32 additions take the sums up, in k-steps (an MMA each: 8 terms of
+// tf32, 16 of halves).  The tensor core cuts off at every addition, always downwards, so a long run drifts.
+//   tf32: relative error of a batch's factors against float64, 2048 columns of 8192 tokens: 5.6e-7 with 16 steps, 1.5e-7 with
+//   four; elimination by float32 multiply-adds has 1.7e-7.  64 factors of K = 2048 take 8.3 and 9.0 ms.  The single problem
+//   keeps 16 (K = 14336: 11.3 ms, 15.5 with four).
+//   halves: the factor's update with eight steps leaves 3.3e-7 where tf32 with 16 left 5.0e-7 (K = 2048, 4873 tokens; 4096:
+//   3.6e-7 and 5.8e-7), 14336 columns take 10.1 ms instead of 11.3; the sweep's products 2.9e-7 instead of 5.4e-7 (last of
+//   4096 columns).  In a batch's factors four steps are 1 to 2 % worse than tf32 with four, two are not.
+constexpr int kLongSlice = 16, kShortSlice = 4;
+constexpr int kLongSlice16 = 8, kShortSlice16 = 4, kShortestSlice16 = 2;
 
 // One side of a product: float32 values x as hi = tf32_rn(x), lo = tf32_rn(x - hi), K-major (row r holds
 // the values of output row / column r), zero-padded to `ld`.  `rows`: rows the two arrays hold, reads
 // beyond give zeros.  Problem b of a batch starts at row b * batch_rows.
+// Or (`scale` set, on both sides) as halves: x * 2^k = hi + lo, eleven bits each like tf32, at half the bytes and twice
+// the rate of the tensor cores; scale[row] = 2^-k brings the row's largest value below 2^15, so that values down to 2^-18
+// of it keep all 22 bits and smaller ones are off by 2^-40 of it at most.
 struct Operand {
-  const float* hi;
-  const float* lo;
+  const void* hi;
+  const void* lo;
   int64_t ld;
   int64_t rows;
   int64_t batch_rows;
   int row0;            // operand row of output row / column 0
+  const float* scale = nullptr;
 };
 
 inline int64_t split_ld(int64_t cols) { return (cols + 31) / 32 * 32; }
+
+// 2^k for a row whose largest magnitude is `largest`, and its inverse
+__device__ __forceinline__ void row_scale(float largest, float& scale, float& inverse) {
+  int k = 141 - (int)(__float_as_uint(largest) >> 23);
+  k = min(max(k, -112), 126);
+  scale = __uint_as_float((uint32_t)(127 + k) << 23);
+  inverse = __uint_as_float((uint32_t)(127 - k) << 23);
+}
+// the hi halves of two neighbours and their lo halves
+__device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi, uint32_t& lo) {
+  const __half2 h = __floats2half2_rn(a, b);
+  const float2 f = __half22float2(h);
+  const __half2 l = __floats2half2_rn(a - f.x, b - f.y);
+  hi = *reinterpret_cast<const uint32_t*>(&h);
+  lo = *reinterpret_cast<const uint32_t*>(&l);
+}
 
 // One half of an operand split: x rounded to nearest even on 10 mantissa bits, as a float32 word
 // whose low 13 mantissa bits are zero.
@@ -60,8 +83,8 @@ struct Job {
   float* const* c_table = nullptr;
   int64_t c_offset = 0, c_batch = 0, ldc = 0;
   int fresh0 = 0, fresh1 = 0;
-  // ... or (out_hi set) the operand form of alpha * product, and for rows below xt_rows also
-  // X[column][row] = alpha * product in float32
+  // ... or (out_hi set) the operand form of alpha * product (out_lo null: its float32 values, from row xt_rows on), and
+  // for rows below xt_rows also X[column][row] = alpha * product in float32
   float* out_hi = nullptr;
   float* out_lo = nullptr;
   int64_t out_ld = 0, out_batch = 0;
@@ -72,7 +95,7 @@ struct Job {
   int* status = nullptr;        // problem b: status + b * status_stride
   int status_stride = 0;
   int max_ctas = 0;             // 0: the whole GPU
-  int slice = kLongSlice;       // chunks that one tensor-core accumulation runs over
+  int slice = kLongSlice;       // k-steps that one tensor-core accumulation runs over
 };
 int launch(const Job& j, cudaStream_t st);
 
@@ -82,6 +105,16 @@ int split(const float* src, int64_t ld_src, int rows, int cols, float* hi, float
 // table of pointers (src + src_offset each) or, without one, a single matrix
 int split_transposed(const float* src, const float* const* table, int64_t src_offset, int64_t ld_src, int rows, int cols,
                      float* hi, float* lo, int64_t ld_dst, int64_t dst_batch, int batch, cudaStream_t st);
+
+// Operands of halves, rows of 512 or 256 (`ld`) zero-padded beyond `cols`.
+// src (src2 set: src + src2) [rows][ld_src] -> hi / lo [rows][ld], scale[row]; `batch` problems src_batch, dst_rows apart
+int split_rows16(const float* src, const float* src2, int64_t ld_src, int64_t src_batch, int64_t rows, int cols, __half* hi,
+                 __half* lo, float* scale, int ld, int64_t dst_rows, int batch, cudaStream_t st);
+// src [rows][cols] -> row c = column c of src.  Problems as with split_transposed, or (table null) src_batch apart.  Entries
+// whose column is above `diagonal` + their row count as zero.
+int split_transposed16(const float* src, const float* const* table, int64_t src_offset, int64_t src_batch, int64_t ld_src,
+                       int rows, int64_t cols, int64_t diagonal, __half* hi, __half* lo, float* scale, int ld, int64_t dst_rows,
+                       int batch, cudaStream_t st);
 
 // A helper stream of the calling host thread (same priority as `like`), with events, for the look-ahead of the
 // blocked solves: the bulk of an update runs there while the caller's stream goes on with the next block.

@@ -372,3 +372,25 @@ def test_sweep_at_edges_of_blocks(N, K, scheme):
     assert torch.equal(W.cpu().double()[sure], q[sure])
     assert torch.allclose(losses.cpu().double()[sure], loss[sure], rtol=1e-4)
     assert float((W.cpu().double() != q).double().mean()) < 0.05
+
+
+@pytest.mark.parametrize("K", [640, 1100, 1664])
+def test_factor_and_sweep_of_badly_scaled_problems(K):
+    """Operands of halves have a scale per row: columns 2^40 apart in size give the factor and the codes of equal ones."""
+    H = _spd(K, K).float()
+    e = torch.randint(-20, 21, (K,), generator=torch.Generator().manual_seed(K)).to(DEV)
+    s = torch.ldexp(torch.ones(K, device=DEV), e)
+    U, V = H.clone(), H * s[:, None] * s[None, :]
+    assert ops.gptq_factor(U) == 0 and ops.gptq_factor(V) == 0
+    W = V * s[None, :]   # (S H S)^-1 = S^-1 U^T U S^-1
+    ref = torch.linalg.cholesky(torch.linalg.inv(H.double()), upper=True)
+    for got in (U, W):   # float32 at this conditioning: about 1e-6
+        assert float((torch.triu(got).double() - ref).norm() / ref.norm()) < 5e-6
+    w = torch.randn(96, K, generator=torch.Generator().manual_seed(1)).to(DEV)
+    scale = torch.full((96, 1), 0.5, device=DEV).bfloat16()
+    args = QuantizationArgs(num_bits=8, type="int", strategy="channel")
+    a, b = w.clone(), w.clone()
+    ops.gptq_sweep(a, torch.triu(U).contiguous(), scale, None, args)
+    # rows of U scaled alike scale the errors inversely and leave the corrections as they are
+    ops.gptq_sweep(b, (torch.triu(U) * s[:, None]).contiguous(), scale, None, args)
+    assert mismatch(a, b) < 0.005
