@@ -71,7 +71,7 @@ template <int ROWS, int SBLK> struct Shape {
                        kE = kW + SBLK * kWld * 4, kPar = kE + kErrSlots * kMicro * ROWS * 4,
                        kZ = kPar + kSlots * kMicro * ROWS * 8, kBand = kZ + kSlots * kMicro * ROWS * 4,
                        kSe = kBand + kSlots * kBandFloats * 4,
-                       kNext = kSe + 4 * ROWS * 4, kEnd = kNext + 2 * kHalf * ROWS * 4;
+                       kNext = kSe + 4 * ROWS * 4, kPow = kNext + 2 * kHalf * ROWS * 4, kEnd = kPow + SBLK * 4;
   static constexpr size_t kSmem = kEnd + 1024;
   static constexpr int kMicros = SBLK / kMicro;
 };
@@ -160,10 +160,11 @@ using tgemm::split_pair;
 
 // U[i1 : i1 + sb, i1 : i1 + sb] as the tiles that the sweep copies into shared memory: tile (micro-block m, block b) holds
 // for each of the block's 128 columns 16 hi and 16 lo halves of the micro-block's rows of U, in 64-byte rows swizzled as
-// the MMA reads them.  Behind the tiles the inverse scale of every column, and then for every micro-block its rows of U
+// the MMA reads them, rows taken times the power of their pivot.  Behind the tiles the inverse scale of every column, the
+// inverses of the pivots' powers (the errors are taken times these), and then for every micro-block its rows of U
 // from the diagonal on (the identity beyond sb) and the reciprocals of its pivots.  A CTA takes 32 columns.
 constexpr int kTileThreads = 256;
-constexpr int64_t band_offset(int sblk) { return (int64_t)(sblk / kMicro) * (sblk / kBlockCols) * kTileBytes + sblk * 4; }
+constexpr int64_t band_offset(int sblk) { return (int64_t)(sblk / kMicro) * (sblk / kBlockCols) * kTileBytes + 2 * sblk * 4; }
 constexpr int64_t tiles_bytes(int sblk) { return band_offset(sblk) + sblk / kMicro * kBandFloats * 4; }   // of one factor
 template <int SBLK>
 __global__ void __launch_bounds__(kTileThreads) square_tiles_kernel(Ptr<const float> Us, int64_t ldu, int i1, int sb,
@@ -183,13 +184,22 @@ __global__ void __launch_bounds__(kTileThreads) square_tiles_kernel(Ptr<const fl
     v[i] = (p <= c && c < sb) ? U[(int64_t)p * ldu + c] : 0.0f;
   }
   float* bands = reinterpret_cast<float*>(tiles + band_offset(SBLK));
+  __shared__ float s_power[SBLK];   // of the rows' pivots
+  for (int p = threadIdx.x; p < SBLK; p += kTileThreads) {
+    const float reciprocal = __frcp_rn(p < sb ? U[(int64_t)p * ldu + p] : 1.0f);
+    s_power[p] = tgemm::pivot_power(reciprocal);
+    if (blockIdx.x == 0)
+      reinterpret_cast<float*>(tiles + SBLK / kMicro * kBlocks * kTileBytes)[SBLK + p] = tgemm::pivot_inverse(reciprocal);
+  }
+  __syncthreads();
 #pragma unroll
   for (int i = 0; i < SBLK / kWarps; ++i) {
     const int p = warp + i * kWarps, c0 = p / kMicro * kMicro;
-    largest = fmaxf(largest, fabsf(v[i]));
     const float x = (p == c && c >= sb) ? 1.0f : v[i];
     if (c >= c0 && c < c0 + kBandCols) bands[p / kMicro * kBandFloats + (p - c0) * kBandCols + c - c0] = x;
     if (c == p) bands[p / kMicro * kBandFloats + kMicro * kBandCols + p - c0] = __frcp_rn(x);
+    v[i] *= s_power[p];
+    largest = fmaxf(largest, fabsf(v[i]));
   }
   s_max[warp][lane] = largest;
   __syncthreads();
@@ -559,6 +569,11 @@ sweep_block_kernel(const __grid_constant__ Params p) {
   auto error_role = [&] {
     // ---- errors of 32 rows as operand of the MMAs
     const int r = (warp - S::kErrors) * 32 + lane;
+    float* power = reinterpret_cast<float*>(sm + S::kPow);   // of the pivots, inverted (every one of these warps writes all)
+    for (int i = lane; i < SBLK / 4; i += 32)
+      reinterpret_cast<float4*>(power)[i] = has_u ? reinterpret_cast<const float4*>(tiles + S::kMicros * S::kBlocks * kTileBytes)[SBLK / 4 + i]
+                                                  : make_float4(1.f, 1.f, 1.f, 1.f);
+    __syncwarp();
 #pragma unroll 1
     for (int m = 0; m < steps; ++m) {
       if (m >= 2)   // the operand buffer's last readers are done
@@ -567,15 +582,19 @@ sweep_block_kernel(const __grid_constant__ Params p) {
       const float* es = sE + (m & (kErrSlots - 1)) * kMicro * ROWS + r;
       const uint32_t eop = smem_u32(sm + S::kErr + (m & 1) * S::kErrBytes) + (uint32_t)(r * kRowBytes);
       float largest[4] = {0.0f, 0.0f, 0.0f, 0.0f}, to, back;
-#pragma unroll
-      for (int t = 0; t < kMicro; ++t) largest[t & 3] = fmaxf(largest[t & 3], fabsf(es[t * ROWS]));
+      const float* pw = power + m * kMicro;
+#pragma unroll 8
+      for (int t = 0; t < kMicro; ++t) largest[t & 3] = fmaxf(largest[t & 3], fabsf(es[t * ROWS] * pw[t]));
       row_scale(fmaxf(fmaxf(largest[0], largest[1]), fmaxf(largest[2], largest[3])), to, back);
       sSe[(m & 3) * ROWS + r] = back;
 #pragma unroll 1
       for (int j = 0; j < 2; ++j) {   // 16 bytes of hi halves and of lo halves each; 64-byte swizzle
         uint32_t hi[4], lo[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) split_pair(es[(8 * j + 2 * k) * ROWS] * to, es[(8 * j + 2 * k + 1) * ROWS] * to, hi[k], lo[k]);
+        for (int k = 0; k < 4; ++k) {
+          const int t = 8 * j + 2 * k;
+          split_pair(es[t * ROWS] * pw[t] * to, es[(t + 1) * ROWS] * pw[t + 1] * to, hi[k], lo[k]);
+        }
         const uint32_t at = eop + ((uint32_t)(j ^ ((r >> 1) & 3)) << 4), at2 = eop + ((uint32_t)((j + 2) ^ ((r >> 1) & 3)) << 4);
         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(hi[0]), "r"(hi[1]), "r"(hi[2]), "r"(hi[3]) : "memory");
         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at2), "r"(lo[0]), "r"(lo[1]), "r"(lo[2]), "r"(lo[3]) : "memory");
@@ -820,7 +839,8 @@ struct Layout {
   int rows, sb, sets;
   int64_t ctas, rows_n, rows_k, err, ub;   // CTAs, rows per problem of the operands; elements of the errors and of U's slice
   int64_t tiles;                           // bytes of the tiles of all factors
-  size_t set;                              // bytes of a set: errors, their halves and scales, the slice's, the tiles
+  int64_t pivots;                          // powers of the pivots of all factors
+  size_t set;                              // bytes of a set: errors, their halves and scales, the slice's, these, the tiles
   size_t bytes;
 };
 static Layout layout_of(int64_t N, int64_t K, int batch, int distinct_u, bool may_overlap) {
@@ -832,7 +852,8 @@ static Layout layout_of(int64_t N, int64_t K, int batch, int distinct_u, bool ma
   l.rows_n = (N + 127) / 128 * 128; l.rows_k = (K + 127) / 128 * 128;
   l.err = K > l.sb ? l.rows_n * l.sb * batch : 0; l.ub = K > l.sb ? l.rows_k * l.sb * distinct_u : 0;
   l.tiles = tiles_bytes(l.sb) * distinct_u;
-  l.set = (size_t)(2 * l.err + l.ub) * sizeof(float) + (size_t)(l.err + l.ub) / l.sb * sizeof(float) + (size_t)l.tiles;
+  l.pivots = (int64_t)l.sb * distinct_u;
+  l.set = (size_t)(2 * l.err + l.ub + (l.err + l.ub) / l.sb + l.pivots) * sizeof(float) + (size_t)l.tiles;
   l.bytes = kSweepHeaderBytes + l.sets * l.set + 64;
   return l;
 }
@@ -859,14 +880,15 @@ static int sweep(Params p, int sdtype, bool global, int batch, const float* cons
   // header of the workspace: a status word that a bounded wait expiring in a sweep or a trailing product sets to
   // B200Q_ERR_DEVICE (cleared here, read by the caller afterwards)
   int* status = (int*)workspace;
-  struct Set { float* err; __half *e_hi, *e_lo, *u_hi, *u_lo; float *e_scale, *u_scale; unsigned char* tiles; };
+  struct Set { float* err; __half *e_hi, *e_lo, *u_hi, *u_lo; float *e_scale, *u_scale, *pivots; unsigned char* tiles; };
   auto set = [&](int which) {
     Set t;
     t.err = (float*)((char*)workspace + kSweepHeaderBytes + which * l.set);
     t.e_hi = (__half*)(t.err + l.err); t.e_lo = t.e_hi + l.err;
     t.u_hi = t.e_lo + l.err; t.u_lo = t.u_hi + l.ub;
     t.e_scale = (float*)(t.u_lo + l.ub); t.u_scale = t.e_scale + l.err / l.sb;
-    t.tiles = (unsigned char*)(t.u_scale + l.ub / l.sb);
+    t.pivots = t.u_scale + l.ub / l.sb;
+    t.tiles = (unsigned char*)(t.pivots + l.pivots);
     return t;
   };
   B200Q_TRY(cudaMemsetAsync(status, 0, sizeof(int), st));
@@ -897,7 +919,7 @@ static int sweep(Params p, int sdtype, bool global, int batch, const float* cons
                              w, t.tiles, p.tiles_batch));
     B200Q_LAUNCH_CHECK();
     return tgemm::split_transposed16(p.U.one ? p.U.one + i1 * p.ldu + i2 : nullptr, Ud, i1 * p.ldu + i2, 0, p.ldu, w, K - i2,
-                                     INT64_MAX / 2, t.u_hi, t.u_lo, t.u_scale, l.sb, l.rows_k, distinct_u, on);
+                                     INT64_MAX / 2, t.u_hi, t.u_lo, t.u_scale, l.sb, l.rows_k, distinct_u, t.pivots, on);
   };
   if (has_u && (rc = split_u(0, 0, st))) return rc;
   int blk = 0;
@@ -920,7 +942,8 @@ static int sweep(Params p, int sdtype, bool global, int batch, const float* cons
     B200Q_LAUNCH_CHECK();
     if (!trailing) continue;
     // W[:, i2:] -= Err[N, w] * U[i1:i2, i2:]
-    if ((rc = tgemm::split_rows16(t.err, nullptr, l.sb, p.err_batch, N, w, t.e_hi, t.e_lo, t.e_scale, l.sb, l.rows_n, batch, st)))
+    if ((rc = tgemm::split_rows16(t.err, nullptr, l.sb, p.err_batch, N, w, t.e_hi, t.e_lo, t.e_scale, l.sb, l.rows_n, batch,
+                                  t.pivots, u_index, st)))
       return rc;
     tgemm::Job j;
     j.A = tgemm::Operand{t.e_hi, t.e_lo, l.sb, l.rows_n * batch, l.rows_n, 0, t.e_scale};

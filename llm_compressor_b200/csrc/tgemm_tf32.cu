@@ -29,6 +29,7 @@
 
 #include <cstdlib>
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 #include "tgemm_tf32.cuh"
@@ -307,26 +308,27 @@ tgemm_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ C
       for (int c = 0; c < chunks; ++c) {
         if (!mbar_wait(full_bar(stage), phase, &s_abort)) { ok = false; break; }
         const uint32_t sa = base + stage * kStageBytes, sb = sa + 2 * kAPart;
-        const int part = j.slice < kSteps ? j.slice : kSteps;   // k-steps of this chunk that one slice takes
-        for (int k0 = 0; k0 < kSteps && ok; k0 += part) {
-          const int buf = slice & 1, at = c * kSteps + k0;
-          const bool first = at % j.slice == 0, last = (at + part) % j.slice == 0 || (c == chunks - 1 && k0 + part == kSteps);
-          if (first && !mbar_wait(acce_bar(buf), (uint32_t)(((slice >> 1) & 1) ^ 1), &s_abort)) { ok = false; break; }
+        // k-steps k0 .. k0 + N of the chunk, to the slice under way (unrolled: descriptors made in a loop cost 5 us a launch)
+        auto issue = [&](int k0, auto N, bool first, bool last) {
+          const int buf = slice & 1;
+          if (first && !mbar_wait(acce_bar(buf), (uint32_t)(((slice >> 1) & 1) ^ 1), &s_abort)) { ok = false; return; }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           if (lane == 0) {
-            const uint32_t d_tmem = tmem_base + (uint32_t)(buf * TN);
+            const uint32_t d_tmem = tmem_base + (uint32_t)(buf * TN), a = sa + k0 * 32, b = sb + k0 * 32;
             // K-major, 128-byte rows: 8-row groups 1024 bytes apart; a k-step of 8 tf32 or 16 halves is 32 bytes
             auto mma = [&](uint32_t x, uint32_t y, uint32_t accumulate) {
               if constexpr (PAIR) mma_pair<F16>(d_tmem, make_desc(x, 16, 1024), make_desc(y, 16, 1024), idesc, accumulate);
               else mma_one<F16>(d_tmem, make_desc(x, 16, 1024), make_desc(y, 16, 1024), idesc, accumulate);
             };
             // the small products first: in a short slice they lose next to nothing, the sum being as small as they are
-            for (int kk = k0; kk < k0 + part; ++kk) {
-              mma(sa + kk * 32, sb + kBPart + kk * 32, (first && kk == k0) ? 0u : 1u);
-              mma(sa + kAPart + kk * 32, sb + kk * 32, 1u);
+#pragma unroll
+            for (int kk = 0; kk < N; ++kk) {
+              mma(a + kk * 32, b + kBPart + kk * 32, (first && kk == 0) ? 0u : 1u);
+              mma(a + kAPart + kk * 32, b + kk * 32, 1u);
             }
-            for (int kk = k0; kk < k0 + part; ++kk) mma(sa + kk * 32, sb + kk * 32, 1u);
-            if (k0 + part == kSteps) {
+#pragma unroll
+            for (int kk = 0; kk < N; ++kk) mma(a + kk * 32, b + kk * 32, 1u);
+            if (k0 + N == kSteps) {
               if constexpr (PAIR) tc_commit_pair(empty_bar(stage));
               else tc_commit(empty_bar(stage));
             }
@@ -337,7 +339,15 @@ tgemm_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ C
           }
           __syncwarp();
           if (last) ++slice;
+        };
+        if (!F16 || j.slice >= kSteps) {
+          const int whole = j.slice / kSteps;
+          issue(0, std::integral_constant<int, kSteps>(), c % whole == 0, c % whole == whole - 1 || c == chunks - 1);
+        } else {
+          issue(0, std::integral_constant<int, kSteps / 2>(), true, true);
+          if (ok) issue(kSteps / 2, std::integral_constant<int, kSteps / 2>(), true, true);
         }
+        if (!ok) break;
         if (++stage == kStages) { stage = 0; phase ^= 1u; }
       }
     }
@@ -572,11 +582,17 @@ __global__ void __launch_bounds__(256) split_transposed_kernel(const float* __re
 template <int LD>
 __global__ void __launch_bounds__(256) split_rows16_kernel(const float* __restrict__ src, const float* __restrict__ src2,
                                                            int64_t ld_src, int64_t src_batch, int64_t rows, int cols,
-                                                           __half* hi, __half* lo, float* scale, int64_t dst_rows) {
+                                                           __half* hi, __half* lo, float* scale, int64_t dst_rows,
+                                                           const float* __restrict__ columns, const int32_t* __restrict__ index) {
   chain_wait();
   chain_go();
   constexpr int kParts = LD / 128;
   const int lane = threadIdx.x & 31;
+  float4 f[kParts];
+#pragma unroll
+  for (int i = 0; i < kParts; ++i)
+    f[i] = columns ? *reinterpret_cast<const float4*>(columns + (int64_t)(index ? index[blockIdx.y] : blockIdx.y) * LD + i * 128 + lane * 4)
+                   : make_float4(1.f, 1.f, 1.f, 1.f);
   src += blockIdx.y * src_batch;
   if (src2) src2 += blockIdx.y * src_batch;
   for (int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); r < rows; r += (int64_t)gridDim.x * 8) {
@@ -589,7 +605,8 @@ __global__ void __launch_bounds__(256) split_rows16_kernel(const float* __restri
     float largest = 0.0f;
 #pragma unroll
     for (int i = 0; i < kParts; ++i) {
-      x[i].x += y[i].x; x[i].y += y[i].y; x[i].z += y[i].z; x[i].w += y[i].w;
+      x[i].x = (x[i].x + y[i].x) * f[i].x; x[i].y = (x[i].y + y[i].y) * f[i].y;
+      x[i].z = (x[i].z + y[i].z) * f[i].z; x[i].w = (x[i].w + y[i].w) * f[i].w;
       float* e = &x[i].x;
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
@@ -618,7 +635,7 @@ __global__ void __launch_bounds__(256) split_transposed16_kernel(const float* __
                                                                  const float* const* __restrict__ table, int64_t src_offset,
                                                                  int64_t src_batch, int64_t ld_src, int rows, int64_t cols,
                                                                  int64_t diagonal, __half* hi, __half* lo, float* scale,
-                                                                 int64_t dst_rows) {
+                                                                 int64_t dst_rows, float* columns) {
   chain_wait();
   chain_go();
   extern __shared__ float stage16[];   // [32][LD + 2]
@@ -630,10 +647,20 @@ __global__ void __launch_bounds__(256) split_transposed16_kernel(const float* __
   // (no load depends on a condition: they go out together)
 #pragma unroll
   for (int i = 0; i < LD / 8; ++i) v[i] = src[(int64_t)min(warp + i * 8, rows - 1) * ld_src + last];
+  __shared__ float s_power[LD];
+  if (columns) {
+    for (int p = threadIdx.x; p < LD; p += 256) {
+      const float reciprocal = p < rows ? __frcp_rn(src[(int64_t)p * ld_src + p - rows]) : 1.0f;
+      s_power[p] = pivot_power(reciprocal);
+      if (blockIdx.x == 0) columns[(int64_t)blockIdx.y * LD + p] = pivot_inverse(reciprocal);
+    }
+    __syncthreads();
+  }
 #pragma unroll
   for (int i = 0; i < LD / 8; ++i) {
     const int p = warp + i * 8;
     if (p >= rows || c >= cols || c > diagonal + p) v[i] = 0.0f;
+    if (columns) v[i] *= s_power[p];
     largest = fmaxf(largest, fabsf(v[i]));
   }
   s_max[warp][lane] = largest;
@@ -713,24 +740,25 @@ int split_transposed(const float* src, const float* const* table, int64_t src_of
 }
 
 int split_rows16(const float* src, const float* src2, int64_t ld_src, int64_t src_batch, int64_t rows, int cols, __half* hi,
-                 __half* lo, float* scale, int ld, int64_t dst_rows, int batch, cudaStream_t st) {
+                 __half* lo, float* scale, int ld, int64_t dst_rows, int batch, const float* columns, const int32_t* index,
+                 cudaStream_t st) {
   if (rows <= 0 || cols <= 0) return B200Q_OK;
   auto kernel = ld == 512 ? split_rows16_kernel<512> : split_rows16_kernel<256>;
   const int64_t blocks = (rows + 7) / 8, cap = 8 * kNumSMs / batch + 1;
   B200Q_TRY(launch_chained(kernel, dim3((unsigned)(blocks < cap ? blocks : cap), (unsigned)batch), 256, 0, st, src, src2, ld_src,
-                           src_batch, rows, cols, hi, lo, scale, dst_rows));
+                           src_batch, rows, cols, hi, lo, scale, dst_rows, columns, index));
   B200Q_LAUNCH_CHECK();
   return B200Q_OK;
 }
 int split_transposed16(const float* src, const float* const* table, int64_t src_offset, int64_t src_batch, int64_t ld_src,
                        int rows, int64_t cols, int64_t diagonal, __half* hi, __half* lo, float* scale, int ld, int64_t dst_rows,
-                       int batch, cudaStream_t st) {
+                       int batch, float* columns, cudaStream_t st) {
   if (rows <= 0 || cols <= 0) return B200Q_OK;
   auto kernel = ld == 512 ? split_transposed16_kernel<512> : split_transposed16_kernel<256>;
   const size_t smem = 32 * (ld + 2) * sizeof(float);
   B200Q_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   B200Q_TRY(launch_chained(kernel, dim3((unsigned)((cols + 31) / 32), (unsigned)batch), 256, smem, st, src, table, src_offset,
-                           src_batch, ld_src, rows, cols, diagonal, hi, lo, scale, dst_rows));
+                           src_batch, ld_src, rows, cols, diagonal, hi, lo, scale, dst_rows, columns));
   B200Q_LAUNCH_CHECK();
   return B200Q_OK;
 }

@@ -106,15 +106,29 @@ int split(const float* src, int64_t ld_src, int rows, int cols, float* hi, float
 int split_transposed(const float* src, const float* const* table, int64_t src_offset, int64_t ld_src, int rows, int cols,
                      float* hi, float* lo, int64_t ld_dst, int64_t dst_batch, int batch, cudaStream_t st);
 
+// The power of two in the reciprocal of a pivot U[p,p], and its inverse.  An error (w - q) / U[p,p] times the inverse has the
+// size of the weights whatever the size of the column's activations, a row U[p,:] times the power that of its pivot: with
+// them both sides of the sweep's products fit one scale per operand row.
+__device__ __forceinline__ int pivot_exponent(float reciprocal) {
+  return min(max((int)(__float_as_uint(reciprocal) >> 23) & 255, 1), 253);
+}
+__device__ __forceinline__ float pivot_power(float reciprocal) { return __uint_as_float((uint32_t)pivot_exponent(reciprocal) << 23); }
+__device__ __forceinline__ float pivot_inverse(float reciprocal) {
+  return __uint_as_float((uint32_t)(254 - pivot_exponent(reciprocal)) << 23);
+}
+
 // Operands of halves, rows of 512 or 256 (`ld`) zero-padded beyond `cols`.
-// src (src2 set: src + src2) [rows][ld_src] -> hi / lo [rows][ld], scale[row]; `batch` problems src_batch, dst_rows apart
+// src (src2 set: src + src2) [rows][ld_src] -> hi / lo [rows][ld], scale[row]; `batch` problems src_batch, dst_rows apart.
+// `columns` (optional): factors of the columns, ld of them per factor, problem b with those of factor index[b] (null: b).
 int split_rows16(const float* src, const float* src2, int64_t ld_src, int64_t src_batch, int64_t rows, int cols, __half* hi,
-                 __half* lo, float* scale, int ld, int64_t dst_rows, int batch, cudaStream_t st);
+                 __half* lo, float* scale, int ld, int64_t dst_rows, int batch, const float* columns, const int32_t* index,
+                 cudaStream_t st);
 // src [rows][cols] -> row c = column c of src.  Problems as with split_transposed, or (table null) src_batch apart.  Entries
-// whose column is above `diagonal` + their row count as zero.
+// whose column is above `diagonal` + their row count as zero.  `columns` (optional): row p is taken times pivot_power of the
+// pivot `rows` columns before src[p, p], whose pivot_inverse goes into columns[p] (ld of them per problem).
 int split_transposed16(const float* src, const float* const* table, int64_t src_offset, int64_t src_batch, int64_t ld_src,
                        int rows, int64_t cols, int64_t diagonal, __half* hi, __half* lo, float* scale, int ld, int64_t dst_rows,
-                       int batch, cudaStream_t st);
+                       int batch, float* columns, cudaStream_t st);
 
 // A helper stream of the calling host thread (same priority as `like`), with events, for the look-ahead of the
 // blocked solves: the bulk of an update runs there while the caller's stream goes on with the next block.
