@@ -911,17 +911,31 @@ static int sweep(Params p, int sdtype, bool global, int batch, const float* cons
   auto square = l.sb == 512 ? square_tiles_kernel<512> : square_tiles_kernel<256>;
   const size_t square_smem = 32 * (l.sb + 1) * sizeof(uint32_t);
   B200Q_TRY(cudaFuncSetAttribute(square, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)square_smem));
-  auto split_u = [&](int64_t i1, int which, cudaStream_t on) -> int {
+  auto split_square = [&](int64_t i1, int which, cudaStream_t on) -> int {
+    const int w = (int)(K - i1 < l.sb ? K - i1 : l.sb);
+    B200Q_TRY(launch_chained(square, dim3((w + 31) / 32, distinct_u), kTileThreads, square_smem, on, factors, p.ldu, (int)i1,
+                             w, set(which).tiles, p.tiles_batch));
+    B200Q_LAUNCH_CHECK();
+    return B200Q_OK;
+  };
+  auto split_rest = [&](int64_t i1, int which, cudaStream_t on) -> int {
     const int w = (int)(K - i1 < l.sb ? K - i1 : l.sb);
     const int64_t i2 = i1 + w;
     const Set t = set(which);
-    B200Q_TRY(launch_chained(square, dim3((w + 31) / 32, distinct_u), kTileThreads, square_smem, on, factors, p.ldu, (int)i1,
-                             w, t.tiles, p.tiles_batch));
-    B200Q_LAUNCH_CHECK();
     return tgemm::split_transposed16(p.U.one ? p.U.one + i1 * p.ldu + i2 : nullptr, Ud, i1 * p.ldu + i2, 0, p.ldu, w, K - i2,
                                      INT64_MAX / 2, t.u_hi, t.u_lo, t.u_scale, l.sb, l.rows_k, distinct_u, t.pivots, on);
   };
-  if (has_u && (rc = split_u(0, 0, st))) return rc;
+  auto split_u = [&](int64_t i1, int which, cudaStream_t on) -> int {
+    const int rc = split_square(i1, which, on);
+    return rc ? rc : split_rest(i1, which, on);
+  };
+  if (has_u && side) {   // the first slice beside the first superblock, which needs its square only
+    B200Q_TRY(cudaEventRecord(side->next, st));
+    B200Q_TRY(cudaStreamWaitEvent(side->stream, side->next, 0));
+    if ((rc = split_square(0, 0, st)) || (rc = split_rest(0, 0, side->stream))) return rc;
+  } else if (has_u && (rc = split_u(0, 0, st))) {
+    return rc;
+  }
   int blk = 0;
   for (int64_t i1 = 0; i1 < K; i1 += l.sb, ++blk) {
     const int w = (int)(K - i1 < l.sb ? K - i1 : l.sb), which = l.sets == 2 ? blk & 1 : 0;
@@ -952,9 +966,7 @@ static int sweep(Params p, int sdtype, bool global, int batch, const float* cons
     j.M = (int)N; j.N = (int)(K - i2); j.Kd = w; j.batch = batch; j.alpha = -1.0f; j.beta = 1.0f;
     if (p.W.one) j.C = p.W.one + i2;
     j.c_table = p.W.table; j.c_offset = i2; j.ldc = p.ldw; j.status = status;
-    // a batch: error of the last of 2048 columns 2.6e-7 of its root mean square, with long slices 7.5e-7, by float32
-    // multiply-adds 4.1e-7; 64 weights of 768 x 2048: 4.0 ms, 3.8 with long slices.  The single weight keeps the long
-    // ones (6.4e-7; 8.8e-7 when its products had rank 128).
+    // (measured where they are defined)
     j.slice = p.W.table ? tgemm::kShortSlice16 : tgemm::kLongSlice16;
     if (!side) {
       if ((rc = tgemm::launch(j, st))) return rc;

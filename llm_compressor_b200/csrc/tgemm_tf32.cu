@@ -768,18 +768,19 @@ int split_transposed16(const float* src, const float* const* table, int64_t src_
 // output rows / columns that the epilogue masks.  Columns beyond Kd are zero (the splits pad them).
 struct MapKey { const void* base; int64_t ld, rows; int box; bool f16; };
 struct MapCache {
-  static constexpr int kSlots = 32;
-  MapKey key[kSlots];
+  // one place per key: a solve has some 25 operand buffers, and one host thread queues several solves at a time
+  static constexpr uint32_t kSlots = 512;
+  MapKey key[kSlots] = {};
   CUtensorMap map[kSlots];
-  int used = 0, next = 0;
-  // Copies the map out: a later get() may evict the slot it came from.
   bool get(const void* base, int64_t ld, int64_t rows, int box, bool f16, CUtensorMap* out) {
-    for (int i = 0; i < used; ++i)
-      if (key[i].base == base && key[i].ld == ld && key[i].rows == rows && key[i].box == box && key[i].f16 == f16) { *out = map[i]; return true; }
-    int slot = (used < kSlots) ? used++ : (next++ % kSlots);
-    key[slot] = MapKey{nullptr, 0, 0, 0, false};
-    if (!make_map(&map[slot], base, rows, ld, box, f16)) return false;
-    key[slot] = MapKey{base, ld, rows, box, f16};
+    const uint64_t mixed = ((uint64_t)(uintptr_t)base / 128 * 64 + (uint64_t)box + (f16 ? 1 : 0)) * 0x9E3779B97F4A7C15ull;
+    const uint32_t slot = (uint32_t)(mixed >> 40) % kSlots;
+    MapKey& k = key[slot];
+    if (!(k.base == base && k.ld == ld && k.rows == rows && k.box == box && k.f16 == f16)) {
+      k = MapKey{nullptr, 0, 0, 0, false};
+      if (!make_map(&map[slot], base, rows, ld, box, f16)) return false;
+      k = MapKey{base, ld, rows, box, f16};
+    }
     *out = map[slot];
     return true;
   }
