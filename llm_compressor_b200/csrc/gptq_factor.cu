@@ -647,12 +647,9 @@ static int factor(float* H, float* const* Hs, int batch, int64_t K, int64_t ldh,
     if (last) break;
     if (side) B200Q_TRY(cudaStreamWaitEvent(bulk, side->next, 0));
     // the update's operand: X[o,:o]^T and D^T, P (of the next block's rows from its operand form)
-    B200Q_RC(tgemm::split_transposed16(mt.A + K0 * lda, nullptr, 0, mt.batch, lda, n, K1, K0, q_hi, q_lo, q_scale, OB, rows, batch,
-                                       nullptr, bulk));
-    B200Q_RC(tgemm::split_rows16(f_hi, f_lo, OB, (int64_t)OB * OB, n2, n, q_hi + K1 * OB, q_lo + K1 * OB, q_scale + K1, OB, rows,
-                                 batch, nullptr, nullptr, bulk));
-    B200Q_RC(tgemm::split_rows16(p_all + (K1 + n2) * OB, nullptr, OB, pb, K - K1 - n2, n, q_hi + (K1 + n2) * OB,
-                                 q_lo + (K1 + n2) * OB, q_scale + K1 + n2, OB, rows, batch, nullptr, nullptr, bulk));
+    B200Q_RC(tgemm::split_update16(tgemm::UpdateOperand{mt.A + K0 * lda, lda, mt.batch, n, K1, f_hi, f_lo, (int64_t)OB * OB, n2,
+                                                        p_all + (K1 + n2) * OB, pb, K - K1 - n2, q_hi, q_lo, q_scale, rows},
+                                   batch, bulk));
     // S[below,o] = -P D, S[i,:o] -= P_i X[o,:o], A[i,j] -= P_i P_j^T, without the next square
     Job u;
     u.A = Q; u.B = Q; u.A.row0 = 0; u.M = u.N = (int)K; u.Kd = n; u.set = tgemm::kBulk; u.batch = batch;

@@ -166,32 +166,42 @@ using tgemm::split_pair;
 constexpr int kTileThreads = 256;
 constexpr int64_t band_offset(int sblk) { return (int64_t)(sblk / kMicro) * (sblk / kBlockCols) * kTileBytes + 2 * sblk * 4; }
 constexpr int64_t tiles_bytes(int sblk) { return band_offset(sblk) + sblk / kMicro * kBandFloats * 4; }   // of one factor
+// Further CTAs (from `squares` on) make the operand of the trailing product: the columns behind the square.
+struct Slice { __half *hi, *lo; float *scale, *pivots; int64_t cols, rows; };   // rows of the operand per factor
 template <int SBLK>
 __global__ void __launch_bounds__(kTileThreads) square_tiles_kernel(Ptr<const float> Us, int64_t ldu, int i1, int sb,
-                                                                   unsigned char* tiles, int64_t batch_bytes) {
+                                                                   unsigned char* tiles, int64_t batch_bytes, int squares,
+                                                                   const Slice slice) {
   chain_wait();
   chain_go();
-  extern __shared__ float stage[];   // [32][SBLK + 1]
+  extern __shared__ float stage[];   // [32][SBLK + 2]
   __shared__ float s_max[kTileThreads / 32][32];
+  __shared__ float s_power[SBLK];   // of the rows' pivots
   constexpr int kWarps = kTileThreads / 32, kBlocks = SBLK / kBlockCols;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = blockIdx.x * 32 + lane;
   const float* U = Us.at(blockIdx.y) + (int64_t)i1 * ldu + i1;
+  if ((int)blockIdx.x >= squares) {
+    const int64_t at = blockIdx.y * slice.rows;
+    tgemm::split_columns16<SBLK>(U + sb, ldu, sb, slice.cols, INT64_MAX / 2, slice.hi + at * SBLK, slice.lo + at * SBLK,
+                                 slice.scale + at, slice.pivots + blockIdx.y * SBLK, blockIdx.x - squares, stage);
+    return;
+  }
   tiles += blockIdx.y * batch_bytes;
   float v[SBLK / kWarps], largest = 0.0f;
+  // (no load depends on a condition: they go out together)
 #pragma unroll
-  for (int i = 0; i < SBLK / kWarps; ++i) {
-    const int p = warp + i * kWarps;
-    v[i] = (p <= c && c < sb) ? U[(int64_t)p * ldu + c] : 0.0f;
-  }
-  float* bands = reinterpret_cast<float*>(tiles + band_offset(SBLK));
-  __shared__ float s_power[SBLK];   // of the rows' pivots
+  for (int i = 0; i < SBLK / kWarps; ++i) v[i] = U[(int64_t)min(warp + i * kWarps, sb - 1) * ldu + min(c, sb - 1)];
   for (int p = threadIdx.x; p < SBLK; p += kTileThreads) {
     const float reciprocal = __frcp_rn(p < sb ? U[(int64_t)p * ldu + p] : 1.0f);
     s_power[p] = tgemm::pivot_power(reciprocal);
     if (blockIdx.x == 0)
       reinterpret_cast<float*>(tiles + SBLK / kMicro * kBlocks * kTileBytes)[SBLK + p] = tgemm::pivot_inverse(reciprocal);
   }
+#pragma unroll
+  for (int i = 0; i < SBLK / kWarps; ++i)
+    if (warp + i * kWarps > c || c >= sb) v[i] = 0.0f;
   __syncthreads();
+  float* bands = reinterpret_cast<float*>(tiles + band_offset(SBLK));
 #pragma unroll
   for (int i = 0; i < SBLK / kWarps; ++i) {
     const int p = warp + i * kWarps, c0 = p / kMicro * kMicro;
@@ -209,11 +219,11 @@ __global__ void __launch_bounds__(kTileThreads) square_tiles_kernel(Ptr<const fl
   row_scale(largest, scale, inverse);
   if (warp == 0) reinterpret_cast<float*>(tiles + SBLK / kMicro * kBlocks * kTileBytes)[c] = inverse;
 #pragma unroll
-  for (int i = 0; i < SBLK / kWarps; ++i) stage[lane * (SBLK + 1) + warp + i * kWarps] = v[i] * scale;
+  for (int i = 0; i < SBLK / kWarps; ++i) stage[lane * (SBLK + 2) + warp + i * kWarps] = v[i] * scale;
   __syncthreads();
   const int b = c / kBlockCols, row = c % kBlockCols;
   for (int m = warp; (m + kLag) * kMicro <= c; m += kWarps) {
-    const float* x = stage + lane * (SBLK + 1) + m * kMicro;
+    const float* x = stage + lane * (SBLK + 2) + m * kMicro;
     unsigned char* d = tiles + (int64_t)(m * kBlocks + b) * kTileBytes + row * kRowBytes;
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
@@ -909,31 +919,24 @@ static int sweep(Params p, int sdtype, bool global, int batch, const float* cons
   Ptr<const float> factors = p.U;
   if (Ud) factors = {nullptr, Ud};
   auto square = l.sb == 512 ? square_tiles_kernel<512> : square_tiles_kernel<256>;
-  const size_t square_smem = 32 * (l.sb + 1) * sizeof(uint32_t);
+  const size_t square_smem = tgemm::split_columns16_smem(l.sb);
   B200Q_TRY(cudaFuncSetAttribute(square, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)square_smem));
-  auto split_square = [&](int64_t i1, int which, cudaStream_t on) -> int {
-    const int w = (int)(K - i1 < l.sb ? K - i1 : l.sb);
-    B200Q_TRY(launch_chained(square, dim3((w + 31) / 32, distinct_u), kTileThreads, square_smem, on, factors, p.ldu, (int)i1,
-                             w, set(which).tiles, p.tiles_batch));
+  auto split_u = [&](int64_t i1, int which, bool tiles, bool rest, cudaStream_t on) -> int {
+    const int w = (int)(K - i1 < l.sb ? K - i1 : l.sb), squares = tiles ? (w + 31) / 32 : 0;
+    const int64_t cols = rest ? K - i1 - w : 0;
+    const Set t = set(which);
+    if (squares + cols == 0) return B200Q_OK;
+    B200Q_TRY(launch_chained(square, dim3((unsigned)(squares + (cols + 31) / 32), distinct_u), kTileThreads, square_smem, on, factors,
+                             p.ldu, (int)i1, w, t.tiles, p.tiles_batch, squares,
+                             Slice{t.u_hi, t.u_lo, t.u_scale, t.pivots, cols, l.rows_k}));
     B200Q_LAUNCH_CHECK();
     return B200Q_OK;
-  };
-  auto split_rest = [&](int64_t i1, int which, cudaStream_t on) -> int {
-    const int w = (int)(K - i1 < l.sb ? K - i1 : l.sb);
-    const int64_t i2 = i1 + w;
-    const Set t = set(which);
-    return tgemm::split_transposed16(p.U.one ? p.U.one + i1 * p.ldu + i2 : nullptr, Ud, i1 * p.ldu + i2, 0, p.ldu, w, K - i2,
-                                     INT64_MAX / 2, t.u_hi, t.u_lo, t.u_scale, l.sb, l.rows_k, distinct_u, t.pivots, on);
-  };
-  auto split_u = [&](int64_t i1, int which, cudaStream_t on) -> int {
-    const int rc = split_square(i1, which, on);
-    return rc ? rc : split_rest(i1, which, on);
   };
   if (has_u && side) {   // the first slice beside the first superblock, which needs its square only
     B200Q_TRY(cudaEventRecord(side->next, st));
     B200Q_TRY(cudaStreamWaitEvent(side->stream, side->next, 0));
-    if ((rc = split_square(0, 0, st)) || (rc = split_rest(0, 0, side->stream))) return rc;
-  } else if (has_u && (rc = split_u(0, 0, st))) {
+    if ((rc = split_u(0, 0, true, false, st)) || (rc = split_u(0, 0, false, true, side->stream))) return rc;
+  } else if (has_u && (rc = split_u(0, 0, true, true, st))) {
     return rc;
   }
   int blk = 0;
@@ -949,14 +952,14 @@ static int sweep(Params p, int sdtype, bool global, int batch, const float* cons
       // the next superblock's slice of U: its buffer was last read by the products of the superblock before this one
       B200Q_TRY(cudaEventRecord(side->next, st));
       B200Q_TRY(cudaStreamWaitEvent(side->stream, side->next, 0));
-      if ((rc = split_u(i2, which ^ 1, side->stream))) return rc;
+      if ((rc = split_u(i2, which ^ 1, true, true, side->stream))) return rc;
       B200Q_TRY(cudaEventRecord(side->done, side->stream));
     }
     B200Q_TRY(launch_chained(kern, dim3((unsigned)l.ctas, batch), threads, smem, st, p));
     B200Q_LAUNCH_CHECK();
     if (!trailing) continue;
     // W[:, i2:] -= Err[N, w] * U[i1:i2, i2:]
-    if ((rc = tgemm::split_rows16(t.err, nullptr, l.sb, p.err_batch, N, w, t.e_hi, t.e_lo, t.e_scale, l.sb, l.rows_n, batch,
+    if ((rc = tgemm::split_rows16(t.err, l.sb, p.err_batch, N, w, t.e_hi, t.e_lo, t.e_scale, l.sb, l.rows_n, batch,
                                   t.pivots, u_index, st)))
       return rc;
     tgemm::Job j;
@@ -970,7 +973,7 @@ static int sweep(Params p, int sdtype, bool global, int batch, const float* cons
     j.slice = p.W.table ? tgemm::kShortSlice16 : tgemm::kLongSlice16;
     if (!side) {
       if ((rc = tgemm::launch(j, st))) return rc;
-      if ((rc = split_u(i2, l.sets == 2 ? which ^ 1 : 0, st))) return rc;
+      if ((rc = split_u(i2, l.sets == 2 ? which ^ 1 : 0, true, true, st))) return rc;
       continue;
     }
     tgemm::Job far = j;

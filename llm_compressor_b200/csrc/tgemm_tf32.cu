@@ -578,115 +578,37 @@ __global__ void __launch_bounds__(256) split_transposed_kernel(const float* __re
   }
 }
 
-// Halves of rows: a warp takes a row, kept in registers between the search for its largest value and the split.
 template <int LD>
-__global__ void __launch_bounds__(256) split_rows16_kernel(const float* __restrict__ src, const float* __restrict__ src2,
-                                                           int64_t ld_src, int64_t src_batch, int64_t rows, int cols,
-                                                           __half* hi, __half* lo, float* scale, int64_t dst_rows,
-                                                           const float* __restrict__ columns, const int32_t* __restrict__ index) {
+__global__ void __launch_bounds__(256) split_rows16_kernel(const float* __restrict__ src, int64_t ld_src, int64_t src_batch,
+                                                           int64_t rows, int cols, __half* hi, __half* lo, float* scale,
+                                                           int64_t dst_rows, const float* __restrict__ columns,
+                                                           const int32_t* __restrict__ index) {
   chain_wait();
   chain_go();
-  constexpr int kParts = LD / 128;
-  const int lane = threadIdx.x & 31;
-  float4 f[kParts];
-#pragma unroll
-  for (int i = 0; i < kParts; ++i)
-    f[i] = columns ? *reinterpret_cast<const float4*>(columns + (int64_t)(index ? index[blockIdx.y] : blockIdx.y) * LD + i * 128 + lane * 4)
-                   : make_float4(1.f, 1.f, 1.f, 1.f);
-  src += blockIdx.y * src_batch;
-  if (src2) src2 += blockIdx.y * src_batch;
-  for (int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); r < rows; r += (int64_t)gridDim.x * 8) {
-    float4 x[kParts], y[kParts];
-    const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-    for (int i = 0; i < kParts; ++i) x[i] = *reinterpret_cast<const float4*>(src + r * ld_src + i * 128 + lane * 4);
-#pragma unroll
-    for (int i = 0; i < kParts; ++i) y[i] = src2 ? *reinterpret_cast<const float4*>(src2 + r * ld_src + i * 128 + lane * 4) : none;
-    float largest = 0.0f;
-#pragma unroll
-    for (int i = 0; i < kParts; ++i) {
-      x[i].x = (x[i].x + y[i].x) * f[i].x; x[i].y = (x[i].y + y[i].y) * f[i].y;
-      x[i].z = (x[i].z + y[i].z) * f[i].z; x[i].w = (x[i].w + y[i].w) * f[i].w;
-      float* e = &x[i].x;
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        if (i * 128 + lane * 4 + k >= cols) e[k] = 0.0f;
-        largest = fmaxf(largest, fabsf(e[k]));
-      }
-    }
-    largest = warp_max(largest);
-    float to, back;
-    row_scale(largest, to, back);
-    const int64_t row = blockIdx.y * dst_rows + r;
-    if (lane == 0) scale[row] = back;
-#pragma unroll
-    for (int i = 0; i < kParts; ++i) {
-      uint2 h, l;
-      split_pair(x[i].x * to, x[i].y * to, h.x, l.x);
-      split_pair(x[i].z * to, x[i].w * to, h.y, l.y);
-      *reinterpret_cast<uint2*>(hi + row * LD + i * 128 + lane * 4) = h;
-      *reinterpret_cast<uint2*>(lo + row * LD + i * 128 + lane * 4) = l;
-    }
-  }
+  const int64_t at = blockIdx.y * dst_rows;
+  split_rows16<LD>(src + blockIdx.y * src_batch, nullptr, ld_src, rows, cols, hi + at * LD, lo + at * LD, scale + at,
+                   columns ? columns + (int64_t)(index ? index[blockIdx.y] : blockIdx.y) * LD : nullptr, blockIdx.x, gridDim.x);
 }
-// Halves of columns, as operand rows: a CTA takes 32 of them.
-template <int LD>
-__global__ void __launch_bounds__(256) split_transposed16_kernel(const float* __restrict__ src0,
-                                                                 const float* const* __restrict__ table, int64_t src_offset,
-                                                                 int64_t src_batch, int64_t ld_src, int rows, int64_t cols,
-                                                                 int64_t diagonal, __half* hi, __half* lo, float* scale,
-                                                                 int64_t dst_rows, float* columns) {
+// The operand of an update of the factor in one launch: `transposed` CTAs take the columns of the block row, the others rows
+// from its end on, `first` of them from a tf32 operand form.
+__global__ void __launch_bounds__(256) split_update16_kernel(const UpdateOperand u, int transposed) {
   chain_wait();
   chain_go();
-  extern __shared__ float stage16[];   // [32][LD + 2]
-  __shared__ float s_max[8][32];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const float* src = table ? table[blockIdx.y] + src_offset : src0 + blockIdx.y * src_batch;
-  const int64_t c = (int64_t)blockIdx.x * 32 + lane, last = c < cols ? c : cols - 1;
-  float v[LD / 8], largest = 0.0f;
-  // (no load depends on a condition: they go out together)
-#pragma unroll
-  for (int i = 0; i < LD / 8; ++i) v[i] = src[(int64_t)min(warp + i * 8, rows - 1) * ld_src + last];
-  __shared__ float s_power[LD];
-  if (columns) {
-    for (int p = threadIdx.x; p < LD; p += 256) {
-      const float reciprocal = p < rows ? __frcp_rn(src[(int64_t)p * ld_src + p - rows]) : 1.0f;
-      s_power[p] = pivot_power(reciprocal);
-      if (blockIdx.x == 0) columns[(int64_t)blockIdx.y * LD + p] = pivot_inverse(reciprocal);
-    }
-    __syncthreads();
+  extern __shared__ float stage16[];
+  const int64_t at = blockIdx.y * u.dst_rows;
+  __half *hi = u.hi + at * kMaxDepth, *lo = u.lo + at * kMaxDepth;
+  float* scale = u.scale + at;
+  if ((int)blockIdx.x < transposed) {
+    split_columns16<kMaxDepth>(u.row + blockIdx.y * u.row_batch, u.row_ld, u.n, u.end, u.end - u.n, hi, lo, scale, nullptr, blockIdx.x,
+                               stage16);
+    return;
   }
-#pragma unroll
-  for (int i = 0; i < LD / 8; ++i) {
-    const int p = warp + i * 8;
-    if (p >= rows || c >= cols || c > diagonal + p) v[i] = 0.0f;
-    if (columns) v[i] *= s_power[p];
-    largest = fmaxf(largest, fabsf(v[i]));
-  }
-  s_max[warp][lane] = largest;
-  __syncthreads();
-#pragma unroll
-  for (int k = 0; k < 8; ++k) largest = fmaxf(largest, s_max[k][lane]);
-  float to, back;
-  row_scale(largest, to, back);
-  const int64_t row0 = blockIdx.y * dst_rows + (int64_t)blockIdx.x * 32;
-  if (warp == 0 && c < cols) scale[row0 + lane] = back;
-#pragma unroll
-  for (int i = 0; i < LD / 8; ++i) stage16[lane * (LD + 2) + warp + i * 8] = v[i] * to;
-  __syncthreads();
-  for (int k = warp; k < 32; k += 8) {
-    if ((int64_t)blockIdx.x * 32 + k >= cols) break;
-    uint32_t* h = reinterpret_cast<uint32_t*>(hi + (row0 + k) * LD);
-    uint32_t* l = reinterpret_cast<uint32_t*>(lo + (row0 + k) * LD);
-#pragma unroll
-    for (int i = 0; i < LD / 64; ++i) {
-      const float2 x = *reinterpret_cast<const float2*>(stage16 + k * (LD + 2) + i * 64 + lane * 2);
-      uint32_t a, b;
-      split_pair(x.x, x.y, a, b);
-      h[i * 32 + lane] = a;
-      l[i * 32 + lane] = b;
-    }
-  }
+  const int64_t cta = blockIdx.x - transposed, ctas = gridDim.x - transposed;
+  hi += u.end * kMaxDepth; lo += u.end * kMaxDepth; scale += u.end;
+  split_rows16<kMaxDepth>(u.f_hi + blockIdx.y * u.f_batch, u.f_lo + blockIdx.y * u.f_batch, kMaxDepth, u.first, u.n, hi, lo, scale,
+                          nullptr, cta, ctas);
+  hi += u.first * kMaxDepth; lo += u.first * kMaxDepth; scale += u.first;
+  split_rows16<kMaxDepth>(u.p + blockIdx.y * u.p_batch, nullptr, kMaxDepth, u.rows, u.n, hi, lo, scale, nullptr, cta, ctas);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -739,26 +661,23 @@ int split_transposed(const float* src, const float* const* table, int64_t src_of
   return B200Q_OK;
 }
 
-int split_rows16(const float* src, const float* src2, int64_t ld_src, int64_t src_batch, int64_t rows, int cols, __half* hi,
-                 __half* lo, float* scale, int ld, int64_t dst_rows, int batch, const float* columns, const int32_t* index,
-                 cudaStream_t st) {
+int split_rows16(const float* src, int64_t ld_src, int64_t src_batch, int64_t rows, int cols, __half* hi, __half* lo, float* scale,
+                 int ld, int64_t dst_rows, int batch, const float* columns, const int32_t* index, cudaStream_t st) {
   if (rows <= 0 || cols <= 0) return B200Q_OK;
   auto kernel = ld == 512 ? split_rows16_kernel<512> : split_rows16_kernel<256>;
   const int64_t blocks = (rows + 7) / 8, cap = 8 * kNumSMs / batch + 1;
-  B200Q_TRY(launch_chained(kernel, dim3((unsigned)(blocks < cap ? blocks : cap), (unsigned)batch), 256, 0, st, src, src2, ld_src,
+  B200Q_TRY(launch_chained(kernel, dim3((unsigned)(blocks < cap ? blocks : cap), (unsigned)batch), 256, 0, st, src, ld_src,
                            src_batch, rows, cols, hi, lo, scale, dst_rows, columns, index));
   B200Q_LAUNCH_CHECK();
   return B200Q_OK;
 }
-int split_transposed16(const float* src, const float* const* table, int64_t src_offset, int64_t src_batch, int64_t ld_src,
-                       int rows, int64_t cols, int64_t diagonal, __half* hi, __half* lo, float* scale, int ld, int64_t dst_rows,
-                       int batch, float* columns, cudaStream_t st) {
-  if (rows <= 0 || cols <= 0) return B200Q_OK;
-  auto kernel = ld == 512 ? split_transposed16_kernel<512> : split_transposed16_kernel<256>;
-  const size_t smem = 32 * (ld + 2) * sizeof(float);
-  B200Q_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  B200Q_TRY(launch_chained(kernel, dim3((unsigned)((cols + 31) / 32), (unsigned)batch), 256, smem, st, src, table, src_offset,
-                           src_batch, ld_src, rows, cols, diagonal, hi, lo, scale, dst_rows, columns));
+int split_update16(const UpdateOperand& u, int batch, cudaStream_t st) {
+  const size_t smem = split_columns16_smem(kMaxDepth);
+  B200Q_TRY(cudaFuncSetAttribute(split_update16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int transposed = (int)((u.end + 31) / 32);
+  const int64_t blocks = (u.first + u.rows + 7) / 8, cap = 3 * kNumSMs / batch + 1;
+  B200Q_TRY(launch_chained(split_update16_kernel, dim3((unsigned)(transposed + (blocks < cap ? blocks : cap)), (unsigned)batch), 256,
+                           smem, st, u, transposed));
   B200Q_LAUNCH_CHECK();
   return B200Q_OK;
 }

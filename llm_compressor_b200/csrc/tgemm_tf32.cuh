@@ -117,18 +117,121 @@ __device__ __forceinline__ float pivot_inverse(float reciprocal) {
   return __uint_as_float((uint32_t)(254 - pivot_exponent(reciprocal)) << 23);
 }
 
-// Operands of halves, rows of 512 or 256 (`ld`) zero-padded beyond `cols`.
-// src (src2 set: src + src2) [rows][ld_src] -> hi / lo [rows][ld], scale[row]; `batch` problems src_batch, dst_rows apart.
-// `columns` (optional): factors of the columns, ld of them per factor, problem b with those of factor index[b] (null: b).
-int split_rows16(const float* src, const float* src2, int64_t ld_src, int64_t src_batch, int64_t rows, int cols, __half* hi,
-                 __half* lo, float* scale, int ld, int64_t dst_rows, int batch, const float* columns, const int32_t* index,
-                 cudaStream_t st);
-// src [rows][cols] -> row c = column c of src.  Problems as with split_transposed, or (table null) src_batch apart.  Entries
-// whose column is above `diagonal` + their row count as zero.  `columns` (optional): row p is taken times pivot_power of the
-// pivot `rows` columns before src[p, p], whose pivot_inverse goes into columns[p] (ld of them per problem).
-int split_transposed16(const float* src, const float* const* table, int64_t src_offset, int64_t src_batch, int64_t ld_src,
-                       int rows, int64_t cols, int64_t diagonal, __half* hi, __half* lo, float* scale, int ld, int64_t dst_rows,
-                       int batch, float* columns, cudaStream_t st);
+// Operands of halves, rows of LD = 512 or 256 zero-padded beyond `cols`.
+// Rows of src (src2 set: src + src2) -> hi / lo [rows][LD], scale[row], by CTA `cta` of `ctas` (256 threads): a warp takes a row,
+// kept in registers between the search for its largest value and the split.  `columns` (optional): factors of the columns.
+template <int LD>
+__device__ __forceinline__ void split_rows16(const float* __restrict__ src, const float* __restrict__ src2, int64_t ld_src,
+                                             int64_t rows, int cols, __half* hi, __half* lo, float* scale,
+                                             const float* __restrict__ columns, int64_t cta, int64_t ctas) {
+  constexpr int kParts = LD / 128;
+  const int lane = threadIdx.x & 31;
+  float4 f[kParts];
+#pragma unroll
+  for (int i = 0; i < kParts; ++i)
+    f[i] = columns ? *reinterpret_cast<const float4*>(columns + i * 128 + lane * 4) : make_float4(1.f, 1.f, 1.f, 1.f);
+  for (int64_t r = cta * 8 + (threadIdx.x >> 5); r < rows; r += ctas * 8) {
+    float4 x[kParts], y[kParts];
+#pragma unroll
+    for (int i = 0; i < kParts; ++i) x[i] = *reinterpret_cast<const float4*>(src + r * ld_src + i * 128 + lane * 4);
+#pragma unroll
+    for (int i = 0; i < kParts; ++i)
+      y[i] = src2 ? *reinterpret_cast<const float4*>(src2 + r * ld_src + i * 128 + lane * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+    float largest = 0.0f;
+#pragma unroll
+    for (int i = 0; i < kParts; ++i) {
+      x[i].x = (x[i].x + y[i].x) * f[i].x; x[i].y = (x[i].y + y[i].y) * f[i].y;
+      x[i].z = (x[i].z + y[i].z) * f[i].z; x[i].w = (x[i].w + y[i].w) * f[i].w;
+      float* e = &x[i].x;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (i * 128 + lane * 4 + k >= cols) e[k] = 0.0f;
+        largest = fmaxf(largest, fabsf(e[k]));
+      }
+    }
+    largest = warp_max(largest);
+    float to, back;
+    row_scale(largest, to, back);
+    if (lane == 0) scale[r] = back;
+#pragma unroll
+    for (int i = 0; i < kParts; ++i) {
+      uint2 h, l;
+      split_pair(x[i].x * to, x[i].y * to, h.x, l.x);
+      split_pair(x[i].z * to, x[i].w * to, h.y, l.y);
+      *reinterpret_cast<uint2*>(hi + r * LD + i * 128 + lane * 4) = h;
+      *reinterpret_cast<uint2*>(lo + r * LD + i * 128 + lane * 4) = l;
+    }
+  }
+}
+// Columns 32 `cta` .. + 31 of src [rows][cols] -> operand rows of those numbers, by a CTA of 256 threads with
+// split_columns16_smem(LD) bytes of shared memory.  Entries whose column is above `diagonal` + their row count as zero.
+// `pivots` (optional): row p is taken times pivot_power of the pivot `rows` columns before src[p, p], whose pivot_inverse goes
+// into pivots[p].
+constexpr size_t split_columns16_smem(int ld) { return 32 * (ld + 2) * sizeof(float); }
+template <int LD>
+__device__ __forceinline__ void split_columns16(const float* __restrict__ src, int64_t ld_src, int rows, int64_t cols,
+                                                int64_t diagonal, __half* hi, __half* lo, float* scale, float* pivots,
+                                                int64_t cta, float* stage) {   // stage [32][LD + 2]
+  __shared__ float s_max[8][32];
+  __shared__ float s_power[LD];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t c = cta * 32 + lane, last = c < cols ? c : cols - 1;
+  float v[LD / 8], largest = 0.0f;
+  // (no load depends on a condition: they go out together)
+#pragma unroll
+  for (int i = 0; i < LD / 8; ++i) v[i] = src[(int64_t)min(warp + i * 8, rows - 1) * ld_src + last];
+  if (pivots) {
+    for (int p = threadIdx.x; p < LD; p += 256) {
+      const float reciprocal = p < rows ? __frcp_rn(src[(int64_t)p * ld_src + p - rows]) : 1.0f;
+      s_power[p] = pivot_power(reciprocal);
+      if (cta == 0) pivots[p] = pivot_inverse(reciprocal);
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < LD / 8; ++i) {
+    const int p = warp + i * 8;
+    if (p >= rows || c >= cols || c > diagonal + p) v[i] = 0.0f;
+    if (pivots) v[i] *= s_power[p];
+    largest = fmaxf(largest, fabsf(v[i]));
+  }
+  s_max[warp][lane] = largest;
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < 8; ++k) largest = fmaxf(largest, s_max[k][lane]);
+  float to, back;
+  row_scale(largest, to, back);
+  if (warp == 0 && c < cols) scale[c] = back;
+#pragma unroll
+  for (int i = 0; i < LD / 8; ++i) stage[lane * (LD + 2) + warp + i * 8] = v[i] * to;
+  __syncthreads();
+  for (int k = warp; k < 32; k += 8) {
+    if (cta * 32 + k >= cols) break;
+    uint32_t* h = reinterpret_cast<uint32_t*>(hi + (cta * 32 + k) * LD);
+    uint32_t* l = reinterpret_cast<uint32_t*>(lo + (cta * 32 + k) * LD);
+#pragma unroll
+    for (int i = 0; i < LD / 64; ++i) {
+      const float2 x = *reinterpret_cast<const float2*>(stage + k * (LD + 2) + i * 64 + lane * 2);
+      uint32_t a, b;
+      split_pair(x.x, x.y, a, b);
+      h[i * 32 + lane] = a;
+      l[i * 32 + lane] = b;
+    }
+  }
+}
+// src [rows][ld_src] -> operand; `batch` problems src_batch, dst_rows apart, problem b with the column factors (ld of them) of
+// index[b] (null: b)
+int split_rows16(const float* src, int64_t ld_src, int64_t src_batch, int64_t rows, int cols, __half* hi, __half* lo, float* scale,
+                 int ld, int64_t dst_rows, int batch, const float* columns, const int32_t* index, cudaStream_t st);
+// The operand of an update of the factor: rows [0, end) are the columns of the block row `row` [n][end] (its last n columns
+// lower triangular), rows [end, end + first) f_hi + f_lo, then `rows` rows of p.
+struct UpdateOperand {
+  const float* row; int64_t row_ld, row_batch; int n; int64_t end;
+  const float *f_hi, *f_lo; int64_t f_batch, first;
+  const float* p; int64_t p_batch, rows;
+  __half *hi, *lo; float* scale; int64_t dst_rows;
+};
+int split_update16(const UpdateOperand& u, int batch, cudaStream_t st);
 
 // A helper stream of the calling host thread (same priority as `like`), with events, for the look-ahead of the
 // blocked solves: the bulk of an update runs there while the caller's stream goes on with the next block.
