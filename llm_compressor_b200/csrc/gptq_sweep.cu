@@ -307,7 +307,7 @@ __device__ __forceinline__ float dequant(float q, float s, float z) {
 // 35 KB of unrolled code at first, 3000 fetches a CTA went to the GPC's cache and the kernel took 140 us for 4096 rows x
 // 512 columns; with eight columns unrolled instead of sixteen and short loops everywhere else it takes 64 (81 when
 // warp-level MMAs on 16-column tiles in shared memory did the corrections, ncu, warm caches; the whole 4096 x 4096 sweep
-// 0.92 ms, 1.04 before).  So: nothing is unrolled further than the registers demand.
+// 0.90 ms, 1.04 before).  So: nothing is unrolled further than the registers demand.
 //
 // Roles, all of them warps of one CTA that hand over by one-shot mbarriers, so that nobody waits for all:
 //   chain    codes and errors of eight columns; applies them to these columns and sums what they are to the next eight
