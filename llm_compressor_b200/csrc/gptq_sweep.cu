@@ -164,10 +164,12 @@ using tgemm::split_pair;
 // inverses of the pivots' powers (the errors are taken times these), and then for every micro-block its rows of U
 // from the diagonal on (the identity beyond sb) and the reciprocals of its pivots.  A CTA takes 32 columns.
 constexpr int kTileThreads = 256;
-constexpr int64_t band_offset(int sblk) { return (int64_t)(sblk / kMicro) * (sblk / kBlockCols) * kTileBytes + 2 * sblk * 4; }
+constexpr int64_t scales_offset(int sblk) { return (int64_t)(sblk / kMicro) * (sblk / kBlockCols) * kTileBytes; }
+constexpr int64_t powers_offset(int sblk) { return scales_offset(sblk) + sblk * 4; }
+constexpr int64_t band_offset(int sblk) { return powers_offset(sblk) + sblk * 4; }
 constexpr int64_t tiles_bytes(int sblk) { return band_offset(sblk) + sblk / kMicro * kBandFloats * 4; }   // of one factor
 // Further CTAs (from `squares` on) make the operand of the trailing product: the columns behind the square.
-struct Slice { __half *hi, *lo; float *scale, *pivots; int64_t cols, rows; };   // rows of the operand per factor
+struct Slice { __half *hi, *lo; float* scale; int64_t cols, rows; };   // rows of the operand per factor
 template <int SBLK>
 __global__ void __launch_bounds__(kTileThreads) square_tiles_kernel(Ptr<const float> Us, int64_t ldu, int i1, int sb,
                                                                    unsigned char* tiles, int64_t batch_bytes, int squares,
@@ -183,7 +185,7 @@ __global__ void __launch_bounds__(kTileThreads) square_tiles_kernel(Ptr<const fl
   if ((int)blockIdx.x >= squares) {
     const int64_t at = blockIdx.y * slice.rows;
     tgemm::split_columns16<SBLK>(U + sb, ldu, sb, slice.cols, INT64_MAX / 2, slice.hi + at * SBLK, slice.lo + at * SBLK,
-                                 slice.scale + at, slice.pivots + blockIdx.y * SBLK, blockIdx.x - squares, stage);
+                                 slice.scale + at, true, blockIdx.x - squares, stage);
     return;
   }
   tiles += blockIdx.y * batch_bytes;
@@ -194,8 +196,7 @@ __global__ void __launch_bounds__(kTileThreads) square_tiles_kernel(Ptr<const fl
   for (int p = threadIdx.x; p < SBLK; p += kTileThreads) {
     const float reciprocal = __frcp_rn(p < sb ? U[(int64_t)p * ldu + p] : 1.0f);
     s_power[p] = tgemm::pivot_power(reciprocal);
-    if (blockIdx.x == 0)
-      reinterpret_cast<float*>(tiles + SBLK / kMicro * kBlocks * kTileBytes)[SBLK + p] = tgemm::pivot_inverse(reciprocal);
+    if (blockIdx.x == 0) reinterpret_cast<float*>(tiles + powers_offset(SBLK))[p] = tgemm::pivot_inverse(reciprocal);
   }
 #pragma unroll
   for (int i = 0; i < SBLK / kWarps; ++i)
@@ -217,7 +218,7 @@ __global__ void __launch_bounds__(kTileThreads) square_tiles_kernel(Ptr<const fl
   for (int k = 0; k < kWarps; ++k) largest = fmaxf(largest, s_max[k][lane]);
   float scale, inverse;
   row_scale(largest, scale, inverse);
-  if (warp == 0) reinterpret_cast<float*>(tiles + SBLK / kMicro * kBlocks * kTileBytes)[c] = inverse;
+  if (warp == 0) reinterpret_cast<float*>(tiles + scales_offset(SBLK))[c] = inverse;
 #pragma unroll
   for (int i = 0; i < SBLK / kWarps; ++i) stage[lane * (SBLK + 2) + warp + i * kWarps] = v[i] * scale;
   __syncthreads();
@@ -397,7 +398,7 @@ sweep_block_kernel(const __grid_constant__ Params p) {
     if (own == 1) hand_over(2);
     const int last_step = min(2 * own + 1 - kLag, steps - 1);         // the last whose errors this warp's columns take
     const int last_mma = min(8 * b + 7 - kLag, steps - 1);            // the last that its block takes part in
-    const float su = has_u && col < sb ? reinterpret_cast<const float*>(tiles + S::kMicros * S::kBlocks * kTileBytes)[col] : 0.0f;
+    const float su = has_u && col < sb ? reinterpret_cast<const float*>(tiles + scales_offset(SBLK))[col] : 0.0f;
     if (b < blocks) {
 #pragma unroll 1
       for (int m = 0; m <= last_mma; ++m) {
@@ -581,7 +582,7 @@ sweep_block_kernel(const __grid_constant__ Params p) {
     const int r = (warp - S::kErrors) * 32 + lane;
     float* power = reinterpret_cast<float*>(sm + S::kPow);   // of the pivots, inverted (every one of these warps writes all)
     for (int i = lane; i < SBLK / 4; i += 32)
-      reinterpret_cast<float4*>(power)[i] = has_u ? reinterpret_cast<const float4*>(tiles + S::kMicros * S::kBlocks * kTileBytes)[SBLK / 4 + i]
+      reinterpret_cast<float4*>(power)[i] = has_u ? reinterpret_cast<const float4*>(tiles + powers_offset(SBLK))[i]
                                                   : make_float4(1.f, 1.f, 1.f, 1.f);
     __syncwarp();
 #pragma unroll 1
@@ -849,8 +850,7 @@ struct Layout {
   int rows, sb, sets;
   int64_t ctas, rows_n, rows_k, err, ub;   // CTAs, rows per problem of the operands; elements of the errors and of U's slice
   int64_t tiles;                           // bytes of the tiles of all factors
-  int64_t pivots;                          // powers of the pivots of all factors
-  size_t set;                              // bytes of a set: errors, their halves and scales, the slice's, these, the tiles
+  size_t set;                              // bytes of a set: errors, their halves and scales, the slice's, the tiles
   size_t bytes;
 };
 static Layout layout_of(int64_t N, int64_t K, int batch, int distinct_u, bool may_overlap) {
@@ -862,8 +862,7 @@ static Layout layout_of(int64_t N, int64_t K, int batch, int distinct_u, bool ma
   l.rows_n = (N + 127) / 128 * 128; l.rows_k = (K + 127) / 128 * 128;
   l.err = K > l.sb ? l.rows_n * l.sb * batch : 0; l.ub = K > l.sb ? l.rows_k * l.sb * distinct_u : 0;
   l.tiles = tiles_bytes(l.sb) * distinct_u;
-  l.pivots = (int64_t)l.sb * distinct_u;
-  l.set = (size_t)(2 * l.err + l.ub + (l.err + l.ub) / l.sb + l.pivots) * sizeof(float) + (size_t)l.tiles;
+  l.set = (size_t)(2 * l.err + l.ub + (l.err + l.ub) / l.sb) * sizeof(float) + (size_t)l.tiles;
   l.bytes = kSweepHeaderBytes + l.sets * l.set + 64;
   return l;
 }
@@ -890,15 +889,14 @@ static int sweep(Params p, int sdtype, bool global, int batch, const float* cons
   // header of the workspace: a status word that a bounded wait expiring in a sweep or a trailing product sets to
   // B200Q_ERR_DEVICE (cleared here, read by the caller afterwards)
   int* status = (int*)workspace;
-  struct Set { float* err; __half *e_hi, *e_lo, *u_hi, *u_lo; float *e_scale, *u_scale, *pivots; unsigned char* tiles; };
+  struct Set { float* err; __half *e_hi, *e_lo, *u_hi, *u_lo; float *e_scale, *u_scale; unsigned char* tiles; };
   auto set = [&](int which) {
     Set t;
     t.err = (float*)((char*)workspace + kSweepHeaderBytes + which * l.set);
     t.e_hi = (__half*)(t.err + l.err); t.e_lo = t.e_hi + l.err;
     t.u_hi = t.e_lo + l.err; t.u_lo = t.u_hi + l.ub;
     t.e_scale = (float*)(t.u_lo + l.ub); t.u_scale = t.e_scale + l.err / l.sb;
-    t.pivots = t.u_scale + l.ub / l.sb;
-    t.tiles = (unsigned char*)(t.pivots + l.pivots);
+    t.tiles = (unsigned char*)(t.u_scale + l.ub / l.sb);
     return t;
   };
   B200Q_TRY(cudaMemsetAsync(status, 0, sizeof(int), st));
@@ -928,7 +926,7 @@ static int sweep(Params p, int sdtype, bool global, int batch, const float* cons
     if (squares + cols == 0) return B200Q_OK;
     B200Q_TRY(launch_chained(square, dim3((unsigned)(squares + (cols + 31) / 32), distinct_u), kTileThreads, square_smem, on, factors,
                              p.ldu, (int)i1, w, t.tiles, p.tiles_batch, squares,
-                             Slice{t.u_hi, t.u_lo, t.u_scale, t.pivots, cols, l.rows_k}));
+                             Slice{t.u_hi, t.u_lo, t.u_scale, cols, l.rows_k}));
     B200Q_LAUNCH_CHECK();
     return B200Q_OK;
   };
@@ -958,9 +956,11 @@ static int sweep(Params p, int sdtype, bool global, int batch, const float* cons
     B200Q_TRY(launch_chained(kern, dim3((unsigned)l.ctas, batch), threads, smem, st, p));
     B200Q_LAUNCH_CHECK();
     if (!trailing) continue;
-    // W[:, i2:] -= Err[N, w] * U[i1:i2, i2:]
+    // W[:, i2:] -= Err[N, w] * U[i1:i2, i2:].  What of this superblock's U the helper stream made, this stream may read
+    // behind its wait for side->done only: the slice below.  The powers of the pivots come with the square's tiles, the
+    // first of which are this stream's own; the others were waited for before the product of the superblock before.
     if ((rc = tgemm::split_rows16(t.err, l.sb, p.err_batch, N, w, t.e_hi, t.e_lo, t.e_scale, l.sb, l.rows_n, batch,
-                                  t.pivots, u_index, st)))
+                                  (const float*)(t.tiles + powers_offset(l.sb)), p.tiles_batch / 4, u_index, st)))
       return rc;
     tgemm::Job j;
     j.A = tgemm::Operand{t.e_hi, t.e_lo, l.sb, l.rows_n * batch, l.rows_n, 0, t.e_scale};

@@ -582,12 +582,12 @@ template <int LD>
 __global__ void __launch_bounds__(256) split_rows16_kernel(const float* __restrict__ src, int64_t ld_src, int64_t src_batch,
                                                            int64_t rows, int cols, __half* hi, __half* lo, float* scale,
                                                            int64_t dst_rows, const float* __restrict__ columns,
-                                                           const int32_t* __restrict__ index) {
+                                                           int64_t columns_batch, const int32_t* __restrict__ index) {
   chain_wait();
   chain_go();
   const int64_t at = blockIdx.y * dst_rows;
   split_rows16<LD>(src + blockIdx.y * src_batch, nullptr, ld_src, rows, cols, hi + at * LD, lo + at * LD, scale + at,
-                   columns ? columns + (int64_t)(index ? index[blockIdx.y] : blockIdx.y) * LD : nullptr, blockIdx.x, gridDim.x);
+                   columns ? columns + (index ? index[blockIdx.y] : blockIdx.y) * columns_batch : nullptr, blockIdx.x, gridDim.x);
 }
 // The operand of an update of the factor in one launch: `transposed` CTAs take the columns of the block row, the others rows
 // from its end on, `first` of them from a tf32 operand form.
@@ -599,7 +599,7 @@ __global__ void __launch_bounds__(256) split_update16_kernel(const UpdateOperand
   __half *hi = u.hi + at * kMaxDepth, *lo = u.lo + at * kMaxDepth;
   float* scale = u.scale + at;
   if ((int)blockIdx.x < transposed) {
-    split_columns16<kMaxDepth>(u.row + blockIdx.y * u.row_batch, u.row_ld, u.n, u.end, u.end - u.n, hi, lo, scale, nullptr, blockIdx.x,
+    split_columns16<kMaxDepth>(u.row + blockIdx.y * u.row_batch, u.row_ld, u.n, u.end, u.end - u.n, hi, lo, scale, false, blockIdx.x,
                                stage16);
     return;
   }
@@ -662,12 +662,13 @@ int split_transposed(const float* src, const float* const* table, int64_t src_of
 }
 
 int split_rows16(const float* src, int64_t ld_src, int64_t src_batch, int64_t rows, int cols, __half* hi, __half* lo, float* scale,
-                 int ld, int64_t dst_rows, int batch, const float* columns, const int32_t* index, cudaStream_t st) {
+                 int ld, int64_t dst_rows, int batch, const float* columns, int64_t columns_batch, const int32_t* index,
+                 cudaStream_t st) {
   if (rows <= 0 || cols <= 0) return B200Q_OK;
   auto kernel = ld == 512 ? split_rows16_kernel<512> : split_rows16_kernel<256>;
   const int64_t blocks = (rows + 7) / 8, cap = 8 * kNumSMs / batch + 1;
   B200Q_TRY(launch_chained(kernel, dim3((unsigned)(blocks < cap ? blocks : cap), (unsigned)batch), 256, 0, st, src, ld_src,
-                           src_batch, rows, cols, hi, lo, scale, dst_rows, columns, index));
+                           src_batch, rows, cols, hi, lo, scale, dst_rows, columns, columns_batch, index));
   B200Q_LAUNCH_CHECK();
   return B200Q_OK;
 }

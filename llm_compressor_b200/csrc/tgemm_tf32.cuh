@@ -165,12 +165,11 @@ __device__ __forceinline__ void split_rows16(const float* __restrict__ src, cons
 }
 // Columns 32 `cta` .. + 31 of src [rows][cols] -> operand rows of those numbers, by a CTA of 256 threads with
 // split_columns16_smem(LD) bytes of shared memory.  Entries whose column is above `diagonal` + their row count as zero.
-// `pivots` (optional): row p is taken times pivot_power of the pivot `rows` columns before src[p, p], whose pivot_inverse goes
-// into pivots[p].
+// `pivots`: row p is taken times pivot_power of the pivot `rows` columns before src[p, p].
 constexpr size_t split_columns16_smem(int ld) { return 32 * (ld + 2) * sizeof(float); }
 template <int LD>
 __device__ __forceinline__ void split_columns16(const float* __restrict__ src, int64_t ld_src, int rows, int64_t cols,
-                                                int64_t diagonal, __half* hi, __half* lo, float* scale, float* pivots,
+                                                int64_t diagonal, __half* hi, __half* lo, float* scale, bool pivots,
                                                 int64_t cta, float* stage) {   // stage [32][LD + 2]
   __shared__ float s_max[8][32];
   __shared__ float s_power[LD];
@@ -184,7 +183,6 @@ __device__ __forceinline__ void split_columns16(const float* __restrict__ src, i
     for (int p = threadIdx.x; p < LD; p += 256) {
       const float reciprocal = p < rows ? __frcp_rn(src[(int64_t)p * ld_src + p - rows]) : 1.0f;
       s_power[p] = pivot_power(reciprocal);
-      if (cta == 0) pivots[p] = pivot_inverse(reciprocal);
     }
     __syncthreads();
   }
@@ -219,10 +217,11 @@ __device__ __forceinline__ void split_columns16(const float* __restrict__ src, i
     }
   }
 }
-// src [rows][ld_src] -> operand; `batch` problems src_batch, dst_rows apart, problem b with the column factors (ld of them) of
-// index[b] (null: b)
+// src [rows][ld_src] -> operand; `batch` problems src_batch, dst_rows apart, problem b with the column factors (ld of them)
+// at columns + columns_batch * index[b] (null: b)
 int split_rows16(const float* src, int64_t ld_src, int64_t src_batch, int64_t rows, int cols, __half* hi, __half* lo, float* scale,
-                 int ld, int64_t dst_rows, int batch, const float* columns, const int32_t* index, cudaStream_t st);
+                 int ld, int64_t dst_rows, int batch, const float* columns, int64_t columns_batch, const int32_t* index,
+                 cudaStream_t st);
 // The operand of an update of the factor: rows [0, end) are the columns of the block row `row` [n][end] (its last n columns
 // lower triangular), rows [end, end + first) f_hi + f_lo, then `rows` rows of p.
 struct UpdateOperand {

@@ -394,3 +394,36 @@ def test_factor_and_sweep_of_badly_scaled_problems(K):
     # rows of U scaled alike scale the errors inversely and leave the corrections as they are
     ops.gptq_sweep(b, (torch.triu(U) * s[:, None]).contiguous(), scale, None, args)
     assert mismatch(a, b) < 0.005
+
+
+@pytest.mark.parametrize("N,K", [(64, 1024), (64, 4096), (4736, 1024), (4736, 4096)])
+def test_concurrent_sweeps_read_nothing_before_it_is_written(N, K):
+    """Superblocks' operands are made on helper streams: one problem alone and as one of nine that crowd the GPU, each on a
+    stream of its own with a workspace of NaN, give the same bits."""
+    lib, count = _lib.load(), 9
+    g = torch.Generator(device=DEV).manual_seed(N + K)
+    U = torch.triu(torch.randn(K, K, generator=g, device=DEV) / K ** 0.5, 1)
+    U.diagonal().copy_(torch.exp2(torch.randint(-3, 4, (K,), generator=g, device=DEV).float()))
+    w = torch.randn(N, K, generator=g, device=DEV) * 0.02
+    scale = torch.full((N, 1), 5e-4, device=DEV).bfloat16()
+    args = QuantizationArgs(num_bits=8, type="int", strategy="channel")
+
+    def problem():
+        ws = torch.full((lib.b200q_gptq_sweep_workspace_bytes(N, K, 128),), 0xFF, dtype=torch.uint8, device=DEV)
+        return w.clone(), torch.empty(N, device=DEV), ws
+
+    def run(W, losses, ws):
+        _lib.check(lib.b200q_gptq_sweep(W.data_ptr(), N, K, K, U.data_ptr(), K, scale.data_ptr(), _lib.BF16, None, None, None,
+                                        args.c_struct(), 128, losses.data_ptr(), ws.data_ptr(), _lib.stream_ptr()), "sweep")
+
+    alone, many = problem(), [problem() for _ in range(count)]
+    run(*alone)
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(count)]
+    for stream, p in zip(streams, many):
+        with torch.cuda.stream(stream):
+            run(*p)
+    torch.cuda.synchronize()
+    assert bool(torch.isfinite(alone[1]).all()) and int(alone[2][:4].view(torch.int32)) == 0
+    for W, losses, ws in many:
+        assert bits_equal(W, alone[0]) and bits_equal(losses, alone[1]) and int(ws[:4].view(torch.int32)) == 0
