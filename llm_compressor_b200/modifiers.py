@@ -1090,9 +1090,16 @@ class _HessianGroup:
 
     def take_sum(self, status=None) -> torch.Tensor:
         """The lower triangle of the sum over all batches, handed over.  The status word leaves the sum's allocation, for
-        ``status`` if the caller has copied it already: who reads it must not keep the matrix from being freed."""
+        ``status`` if the caller has copied it already: who reads it must not keep the matrix from being freed.
+        A solve takes the sum on a stream of its own: what calibration allocated on another is not to be given out there
+        before this stream has read it."""
         self._last = None
         self.flush()
+        if self.device.type == "cuda":
+            stream = torch.cuda.current_stream(self.device)
+            for t in (self.H, self.status, self._stage):
+                if t is not None and t.is_cuda:
+                    t.record_stream(stream)
         self._stage = None
         self.status = self.status.clone() if status is None else status
         H, self.H = self.H.to(self.device), None

@@ -427,3 +427,25 @@ def test_concurrent_sweeps_read_nothing_before_it_is_written(N, K):
     assert bool(torch.isfinite(alone[1]).all()) and int(alone[2][:4].view(torch.int32)) == 0
     for W, losses, ws in many:
         assert bits_equal(W, alone[0]) and bits_equal(losses, alone[1]) and int(ws[:4].view(torch.int32)) == 0
+
+
+def test_a_sum_taken_on_another_stream_is_not_given_out_before_it_is_read():
+    K, tokens = 1536, 2048
+    lin = torch.nn.Linear(K, 8, bias=False, device=DEV, dtype=torch.bfloat16)
+    torch.cuda.empty_cache()
+    x = torch.randn(1, 64, K, device=DEV).bfloat16()
+    modifiers._HessianGroup(lin).accumulate(x)   # (loads the kernels)
+    torch.cuda.synchronize()
+    group = modifiers._HessianGroup(lin, stage_tokens=tokens)
+    group.accumulate(x)
+    taken = [(t.untyped_storage().data_ptr(), t.untyped_storage().nbytes()) for t in (group.H, group._stage)]
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        torch.cuda._sleep(200_000_000)   # (about a tenth of a second, the readers behind it)
+        group.take_sum()                 # (and dropped)
+    given = [torch.empty(n, dtype=torch.uint8, device=DEV) for _, n in taken]
+    assert not stream.query()
+    for (at, n), t in zip(taken, given):
+        assert all(t.data_ptr() >= a + m or t.data_ptr() + t.nbytes <= a for a, m in taken)
+    torch.cuda.synchronize()
