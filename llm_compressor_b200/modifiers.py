@@ -964,7 +964,9 @@ def _gather_copies(solved) -> dict:
         for attr, val in out.items():
             if attr == "weight":
                 continue
-            p = params.get(attr)
+            p = params.get(attr)   # (nearly always; a buffer or plain tensor of that name is written as well)
+            if p is None:
+                p = getattr(module, attr, None)
             if p is None:
                 p = torch.nn.Parameter(torch.empty_like(val, memory_format=torch.contiguous_format), requires_grad=False)
                 module.register_parameter(attr, p)

@@ -1,10 +1,12 @@
 """Host logic that needs no GPU: AWQ mapping resolution and grid, the activation store of the
 sequential driver, the kv-cache plumbing, the merge of a converter's config."""
+import types
+
 import pytest
 import torch
 
 import oracle
-from llm_compressor_b200 import awq
+from llm_compressor_b200 import awq, modifiers
 from llm_compressor_b200.model_free import _merge_configs
 from llm_compressor_b200.modifiers import QuantizationModifier, _ObservingCache, _observing_cache_hook
 from llm_compressor_b200.oneshot import _ActivationStore, _tree_map, _with_hidden
@@ -225,3 +227,29 @@ def test_model_copy_takes_fields_only():
     assert (copy.num_bits, copy.actorder, copy.group_size) == (8, "weight", 128) and args.num_bits == 4
     with pytest.raises(TypeError, match="group_sise"):
         args.model_copy(update={"group_sise": 64})
+
+
+@pytest.mark.parametrize("kind", ["parameter", "buffer", "attribute", "none"])
+def test_values_of_a_batch_go_where_the_module_has_them(kind):
+    """Slices of a batch's buffers are copied into whatever the module holds under that name."""
+    batch = torch.rand(3, 4, 1)
+    mods = [torch.nn.Linear(4, 4, bias=False) for _ in range(3)]
+    targets = []
+    for lin in mods:
+        t = torch.full((4, 1), float("nan"))
+        if kind == "parameter":
+            t = torch.nn.Parameter(t, requires_grad=False)
+            lin.register_parameter("weight_scale", t)
+        elif kind == "buffer":
+            lin.register_buffer("weight_scale", t)
+        elif kind == "attribute":
+            lin.weight_scale = t
+        targets.append(t)
+    solved = [(lin, {"weight": lin.weight.data.clone(), "weight_scale": v}) for lin, v in zip(mods, batch)]
+    queued = [(lin, None, types.SimpleNamespace(ok=True), 0.25, out) for lin, out in solved]
+    modifier = modifiers.GPTQModifier(targets="Linear", scheme="W4A16")
+    modifier._finish_queued(queued, 0.0, queued, modifiers._gather_copies(solved))
+    for lin, v, t in zip(mods, batch, targets):
+        assert torch.equal(lin.weight_scale, v)
+        assert lin.weight_scale.untyped_storage().nbytes() == v.numel() * 4
+        assert kind == "none" or lin.weight_scale is t
