@@ -780,10 +780,10 @@ class GPTQModifier(QuantizationMixin):
             raise B200QError("a bounded wait inside the Hessian or GEMM kernels of this job expired; "
                              "its results are incomplete")
 
-    def _finish_queued(self, queued, t0, batch=(), copies={}):
+    def _finish_queued(self, queued, t0, batch=(), gathered=None):
         """``queued``: [(module, qargs, factor, loss, out)] of deferred solves whose factors have been
-        resolved; ``batch``: those of them whose values are slices of a batch's buffers, and ``copies`` what
-        ``_gather_copies`` makes of them all.  Redo the modules whose Hessian was not positive definite with the
+        resolved; ``batch``: those of them whose values are slices of a batch's buffers, and ``gathered``
+        what ``_gather_copies`` makes of them all.  Redo the modules whose Hessian was not positive definite with the
         identity, as the reference falls back (gptq_quantize.py:157-164), then write every result to its module."""
         redo = [q for q in queued if not q[2].ok]
         # the deferred call consumed the observers' statistics: observe again before the
@@ -829,9 +829,13 @@ class GPTQModifier(QuantizationMixin):
             _set_plain(module, "quantization_status", "frozen")
             self._done.add(module)
         if redo and batch:
-            copies = _gather_copies([(q[0], q[4]) for q in batch if q[2].ok])
-        for into, values in copies.values():
-            torch._foreach_copy_(into, values)
+            gathered = _gather_copies([(q[0], q[4]) for q in batch if q[2].ok])
+        if gathered:
+            copies, unset = gathered
+            for module, attr, p in unset:
+                module.register_parameter(attr, p)
+            for into, values in copies.values():
+                torch._foreach_copy_(into, values)
 
     def _compress_group(self, module_list):
         """Factor and sweep the modules of one Hessian."""
@@ -914,10 +918,10 @@ class GPTQModifier(QuantizationMixin):
             if len(items) >= 4:
                 batch += queued[-len(items):]
         self._trace("job_swept", jobs[0][0])
-        copies = _gather_copies([(q[0], q[4]) for q in batch])   # (while the device is at work)
+        gathered = _gather_copies([(q[0], q[4]) for q in batch])   # (while the device is at work)
         self._check_status_words(words)
         gptq.resolve_factors([q[2] for q in queued])
-        self._finish_queued(queued, t0, batch, copies)
+        self._finish_queued(queued, t0, batch, gathered)
 
     @staticmethod
     def _log_metric(name, seconds, loss):
@@ -954,11 +958,13 @@ def _loss_order(jobs) -> list:
     return sorted(jobs, key=length)
 
 
-def _gather_copies(solved) -> dict:
+def _gather_copies(solved):
     """{(types, device): ([parameters], [values])} of [(module, out)] whose values are slices of buffers that many modules share, for
-    one copy a type.  Put in as they are, the slices would keep the buffer alive, and saving one module would write all of
-    it."""
+    one copy a type, and the parameters [(module, name, parameter)] that the modules do not have yet: they get them with
+    their values, no sooner (a solve that fails leaves its modules as they were).  Put in as they are, the slices would keep
+    the buffer alive, and saving one module would write all of it."""
     copies: dict = {}
+    unset = []
     for module, out in solved:
         params = module._parameters
         for attr, val in out.items():
@@ -969,7 +975,7 @@ def _gather_copies(solved) -> dict:
                 p = getattr(module, attr, None)
             if p is None:
                 p = torch.nn.Parameter(torch.empty_like(val, memory_format=torch.contiguous_format), requires_grad=False)
-                module.register_parameter(attr, p)
+                unset.append((module, attr, p))
             p = p.data
             if val.shape != p.shape:
                 val = val.reshape(p.shape)
@@ -978,7 +984,7 @@ def _gather_copies(solved) -> dict:
             into, values = copies.setdefault((p.dtype, val.dtype, p.device), ([], []))
             into.append(p)
             values.append(val)
-    return copies
+    return copies, unset
 
 
 def _plain_args(a: QuantizationArgs) -> dict:

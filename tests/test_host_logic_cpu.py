@@ -253,3 +253,11 @@ def test_values_of_a_batch_go_where_the_module_has_them(kind):
         assert torch.equal(lin.weight_scale, v)
         assert lin.weight_scale.untyped_storage().nbytes() == v.numel() * 4
         assert kind == "none" or lin.weight_scale is t
+
+
+def test_a_batched_solve_that_fails_leaves_its_modules_as_they_were():
+    """Nothing is registered while the values are gathered: the device's status words are read after that."""
+    lin = torch.nn.Linear(4, 4, bias=False)
+    before = dict(lin.named_parameters())
+    modifiers._gather_copies([(lin, {"weight": lin.weight.data, "weight_g_idx": torch.zeros(2, 4, dtype=torch.int32)[0]})])
+    assert dict(lin.named_parameters()) == before
