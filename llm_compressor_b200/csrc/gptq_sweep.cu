@@ -160,7 +160,7 @@ using tgemm::split_pair;
 
 // U[i1 : i1 + sb, i1 : i1 + sb] as the tiles that the sweep copies into shared memory: tile (micro-block m, block b) holds
 // for each of the block's 128 columns 16 hi and 16 lo halves of the micro-block's rows of U, in 64-byte rows swizzled as
-// the MMA reads them, rows taken times the power of their pivot.  Behind the tiles the inverse scale of every column, the
+// the MMA reads them, rows taken times the power of their pivot (tgemm::pivot_power).  Behind the tiles the inverse scale of every column, the
 // inverses of the pivots' powers (the errors are taken times these), and then for every micro-block its rows of U
 // from the diagonal on (the identity beyond sb) and the reciprocals of its pivots.  A CTA takes 32 columns.
 constexpr int kTileThreads = 256;

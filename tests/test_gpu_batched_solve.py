@@ -364,3 +364,30 @@ def test_sweep_is_as_accurate_as_rank_128_updates(N, K, tokens, limit):
     losses = ops.gptq_sweep(w.float(), U, scale, None, args_from(SCHEMES["W8_CHANNEL"]))
     error = (2.0 * losses.double()).sqrt() - last
     assert float(error.pow(2).mean().sqrt() / last.pow(2).mean().sqrt()) <= limit
+
+
+# every code zero and the last column alone in the loss, as above, with columns of activations 2^-18 .. 2^18 in size: even
+# weights; weights that go the other way, so that all columns' errors count alike; even weights and every second column tiny
+# and without correlation to the others, so that only the smallest errors reach the last column.  Three times the limit of
+# equal sizes: either side of a product spans 2^18, and of its smallest values 21 to 22 bits are kept
+@pytest.mark.parametrize("N,K,tokens", [(1001, 520, 1500), (1001, 1160, 6933), (6000, 520, 1500)])
+@pytest.mark.parametrize("grading", ["activations", "weights", "groups"])
+def test_sweep_of_columns_graded_in_size(grading, N, K, tokens):
+    H, ref = _spd_factor64(K, tokens)
+    e = torch.randint(-18, 19, (K,), generator=torch.Generator().manual_seed(K)).to(DEV)
+    w = (torch.randn(N, K, generator=torch.Generator(device=DEV).manual_seed(N), device=DEV) * 0.02).bfloat16().float()
+    if grading == "groups":
+        odd = torch.arange(K, device=DEV) % 2 == (K - 1) % 2
+        e = torch.where(odd, -18, 18)
+        H = torch.where(odd[:, None] == odd[None, :], H, 0.0).double()
+        L = torch.linalg.cholesky(H.flip(0, 1))
+        ref = torch.linalg.solve_triangular(L, torch.eye(K, device=DEV, dtype=torch.float64), upper=False).flip(0, 1)
+    U = torch.ldexp(ref, -e).float().contiguous()   # H = S R S has U S^-1
+    if grading == "weights":
+        w = torch.ldexp(w, -e)
+    U[:-1] *= 2.0 ** 60
+    last = torch.linalg.solve_triangular(U.double(), w.double(), upper=True, left=False)[:, -1].abs()
+    scale = torch.full((N, 1), 2.0 ** 40, device=DEV).bfloat16()
+    losses = ops.gptq_sweep(w.clone(), U, scale, None, args_from(SCHEMES["W8_CHANNEL"]))
+    error = (2.0 * losses.double()).sqrt() - last
+    assert float(error.pow(2).mean().sqrt() / last.pow(2).mean().sqrt()) <= 3 * (9.2e-7 if K == 520 else 4.8e-7)
