@@ -505,7 +505,7 @@ extern "C" int b200q_gemm_tf32x3(int trans_b, const float* A, int64_t lda, const
   int rc = tgemm::split(A, lda, (int)M, (int)Kd, a_hi, a_lo, st);
   if (rc) return rc;
   if (trans_b) rc = tgemm::split(B, ldb, (int)N, (int)Kd, b_hi, b_lo, st);
-  else rc = tgemm::split_transposed(B, nullptr, 0, ldb, (int)Kd, (int)N, b_hi, b_lo, kp, 0, 1, st);
+  else rc = tgemm::split_transposed(B, ldb, (int)Kd, (int)N, b_hi, b_lo, kp, st);
   if (rc) return rc;
   tgemm::Job j;
   j.A = tgemm::Operand{a_hi, a_lo, kp, (M + 127) / 128 * 128, 0, 0};

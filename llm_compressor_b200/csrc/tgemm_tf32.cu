@@ -539,18 +539,14 @@ __global__ void split_kernel(const float* __restrict__ src, int64_t ld_src, int 
 }
 
 // Transposing variant: row c of hi/lo (ld_dst floats) holds column c of src, zero-padded.  Turns a
-// [Kd][N] operand into the K-major [N][Kd] form the MMA reads.  blockIdx.y = problem.
-__global__ void __launch_bounds__(256) split_transposed_kernel(const float* __restrict__ src0,
-                                                               const float* const* __restrict__ table,
-                                                               int64_t src_offset, int64_t ld_src, int rows, int cols,
+// [Kd][N] operand into the K-major [N][Kd] form the MMA reads.
+__global__ void __launch_bounds__(256) split_transposed_kernel(const float* __restrict__ src,
+                                                               int64_t ld_src, int rows, int cols,
                                                                float* __restrict__ hi, float* __restrict__ lo,
-                                                               int64_t ld_dst, int64_t dst_batch) {
+                                                               int64_t ld_dst) {
   __shared__ float tile[32][33];
   chain_wait();
   chain_go();
-  const float* __restrict__ src = table ? table[blockIdx.y] + src_offset : src0;
-  hi += (int64_t)blockIdx.y * dst_batch;
-  lo += (int64_t)blockIdx.y * dst_batch;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
   const int tiles_c = (cols + 31) / 32, tiles_r = (int)(ld_dst / 32);
   for (int t = blockIdx.x; t < tiles_c * tiles_r; t += gridDim.x) {
@@ -649,14 +645,12 @@ int split(const float* src, int64_t ld_src, int rows, int cols, float* hi, float
   return B200Q_OK;
 }
 
-int split_transposed(const float* src, const float* const* table, int64_t src_offset, int64_t ld_src, int rows, int cols,
-                     float* hi, float* lo, int64_t ld_dst, int64_t dst_batch, int batch, cudaStream_t st) {
+int split_transposed(const float* src, int64_t ld_src, int rows, int cols, float* hi, float* lo, int64_t ld_dst, cudaStream_t st) {
   if (rows <= 0 || cols <= 0) return B200Q_OK;
   const int64_t tiles = (int64_t)((cols + 31) / 32) * (ld_dst / 32);
-  const int cap = batch > 1 ? 8 * kNumSMs / batch + 1 : 8 * kNumSMs;
-  dim3 grid((unsigned)(tiles < cap ? tiles : cap), (unsigned)batch, 1);
-  B200Q_TRY(launch_chained(split_transposed_kernel, grid, 256, 0, st, src, table, src_offset, ld_src, rows, cols, hi, lo, ld_dst,
-                           dst_batch));
+  const int64_t cap = 8 * kNumSMs;
+  B200Q_TRY(launch_chained(split_transposed_kernel, dim3((unsigned)(tiles < cap ? tiles : cap)), 256, 0, st, src, ld_src, rows, cols,
+                           hi, lo, ld_dst));
   B200Q_LAUNCH_CHECK();
   return B200Q_OK;
 }
@@ -762,9 +756,11 @@ static int pair_capacity() {
 // epilogue, about 20 cycles per column, is not hidden.
 static void pick_tiles(Params& p, int ctas, int pairs) {
   const double chunk[3] = {800.0, 1150.0, 1700.0};
-  // Anything from 1000 to 1600 gives the same times; above 1700 pairs are never taken.  Without / with pairs, us: factor
-  // K = 4096 1198 / 1196, 8192 3340 / 3115, 14336 13353 / 11398; sweep 4096 x 4096 1035 / 984, 14336 x 4096 2829 / 2681,
-  // 4096 x 14336 6545 / 5879; 1024 rows and K = 2048 the same either way.
+  // Above 1700 pairs are never taken.  A chunk of halves holds twice the terms at the same bytes and MMA cycles, so the
+  // same line serves both, but it decides less for halves, whose additions to C are the larger part.  Without / with pairs, us:
+  // factor (halves) K = 4096 1215 / 1212, 8192 2903 / 2911, 14336 9830 to 10380 / 9670 to 10330; sweep (halves) 4096 x 4096
+  // 821 / 809, 14336 x 4096 2417 / 2430, 4096 x 14336 4627 / 4606, 32 weights of 768 x 2048 1820 / 1834; from 1000 to 2200, and
+  // with an epilogue of 10 to 40 cycles a column, within 2 % of these.  With products of tf32 14336 columns took 13353 / 11398.
   const double pair_chunk = 1600.0;
   const Job& j = p.j;
   const int depth = j.A.scale ? kChunkK16 : kChunkK, chunks = (j.Kd + depth - 1) / depth;

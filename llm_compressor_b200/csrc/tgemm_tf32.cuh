@@ -103,10 +103,8 @@ int launch(const Job& j, cudaStream_t st);
 
 // src [rows][cols] -> hi/lo [rows][split_ld(cols)]
 int split(const float* src, int64_t ld_src, int rows, int cols, float* hi, float* lo, cudaStream_t st);
-// src [rows][cols] -> hi/lo [cols][ld_dst], row c = column c of src zero-padded; `batch` problems given by a device
-// table of pointers (src + src_offset each) or, without one, a single matrix
-int split_transposed(const float* src, const float* const* table, int64_t src_offset, int64_t ld_src, int rows, int cols,
-                     float* hi, float* lo, int64_t ld_dst, int64_t dst_batch, int batch, cudaStream_t st);
+// src [rows][cols] -> hi/lo [cols][ld_dst], row c = column c of src zero-padded
+int split_transposed(const float* src, int64_t ld_src, int rows, int cols, float* hi, float* lo, int64_t ld_dst, cudaStream_t st);
 
 // The sweep's products are sums over p of an error (w - q) / U[p,p] and U[p,j], one scale per row on either side.  Where the
 // activations of column p have size s_p, pivots are of size 1 / s_p, rows of U as even as the correlations (with H = S R S,
