@@ -302,8 +302,10 @@ size_t b200q_gptq_factor_workspace_bytes(int64_t K);
 int b200q_gptq_factor(float* H, int64_t K, int64_t ldh, void* workspace, int* status,
                       void* stream);
 
-/* The float32-accurate tensor-core GEMM that the factorisation and the sweep use for their
- * updates (tcgen05 kind::tf32, three MMAs per product on hi/lo splits of the operands):
+/* A float32-accurate tensor-core GEMM (tcgen05 kind::tf32, three MMAs per product on hi/lo splits
+ * of the operands): the template that makes P and the next square in the factorisation.  Its
+ * rank-512 updates and the sweep's products run another instance, on pairs of halves
+ * (kind::f16), which no entry point exposes by itself.
  *   C[M,N] = beta*C + alpha * A[M,Kd] * (trans_b ? B[N,Kd]^T : B[Kd,N]),   Kd <= 128.
  * Stands in for the torch.matmul calls of gptq_quantize.py:236,244 and the cuSOLVER updates
  * behind :153-155.  lower_tiles != 0 restricts the update to 128x128 tiles with column block <=

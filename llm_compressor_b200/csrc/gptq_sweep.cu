@@ -304,13 +304,15 @@ __device__ __forceinline__ float dequant(float q, float s, float z) {
   return SB ? bf16_in_place(q) : q;
 }
 
-// What bounds it: the chain of columns, one warp of 32 rows.  Eight columns take it some 600 cycles on its own (the
-// dependent instructions of a column are about 45, the 26 16-byte loads of U and 56 packed FMAs of its half-block the
-// rest), and 900 to 1100 beside the other roles.  What it costs most is instruction fetch: all roles together ran from
-// 35 KB of unrolled code at first, 3000 fetches a CTA went to the GPC's cache and the kernel took 140 us for 4096 rows x
-// 512 columns; with eight columns unrolled instead of sixteen and short loops everywhere else it takes 64 (81 when
-// warp-level MMAs on 16-column tiles in shared memory did the corrections, ncu, warm caches; the whole 4096 x 4096 sweep
-// 0.90 ms, 1.04 before).  So: nothing is unrolled further than the registers demand.
+// What bounds it: the chain of columns, one warp of 32 rows.  Cycles of a CTA's launch, 4096 rows x 512 columns, clocks read
+// in the chain's warp: 2100 setting up, 6000 until the first columns of W are there, 500 their parameters, 83000 the
+// chain, 900 after it.  Eight columns of the chain take 1300, of which 210 are the hand-over from the feeder (180 where it has
+// long been through: the chain hardly ever waits), 1060 at the end of the superblock where few other roles still run.
+// What the roles cost one another is instruction fetch: from 35 KB of unrolled code, as they were at first, 3000 fetches a
+// CTA went to the GPC's cache and the kernel took 140 us; with eight columns unrolled instead of sixteen and short loops
+// everywhere else it takes 65 (81 when warp-level MMAs on 16-column tiles in shared memory did the corrections; ncu, warm
+// caches).  The whole 4096 x 4096 sweep takes 0.82 ms, 0.88 with zero points (1.04).  So: nothing is unrolled further than the
+// registers demand.
 //
 // Roles, all of them warps of one CTA that hand over by one-shot mbarriers, so that nobody waits for all:
 //   chain    codes and errors of eight columns; applies them to these columns and sums what they are to the next eight

@@ -757,7 +757,7 @@ static int pair_capacity() {
 static void pick_tiles(Params& p, int ctas, int pairs) {
   const double chunk[3] = {800.0, 1150.0, 1700.0};
   // Above 1700 pairs are never taken.  A chunk of halves holds twice the terms at the same bytes and MMA cycles, so the
-  // same line serves both, but it decides less for halves, whose additions to C are the larger part.  Without / with pairs, us:
+  // same line serves both, but with halves it decides next to nothing.  Without / with pairs, us:
   // factor (halves) K = 4096 1215 / 1212, 8192 2903 / 2911, 14336 9830 to 10380 / 9670 to 10330; sweep (halves) 4096 x 4096
   // 821 / 809, 14336 x 4096 2417 / 2430, 4096 x 14336 4627 / 4606, 32 weights of 768 x 2048 1820 / 1834; from 1000 to 2200, and
   // with an epilogue of 10 to 40 cycles a column, within 2 % of these.  With products of tf32 14336 columns took 13353 / 11398.
