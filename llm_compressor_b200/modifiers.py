@@ -22,7 +22,7 @@ import torch
 
 from . import dist as bdist
 from . import gptq, ops
-from ._lib import B200QError, stream_ptr
+from ._lib import B200QError, stream_of
 from .observers import MemorylessMinMaxObserver, Observer, direct_qparams, fuse_weight_observers
 from .streams import run_concurrent, run_queued
 from .quant_args import (PRESET_SCHEMES, QuantizationArgs, QuantizationScheme,
@@ -1045,7 +1045,7 @@ class _HessianGroup:
         self.members = [module]
         K = module.weight.shape[1]
         self.device = module.weight.device
-        self._streams = {self._stream()}   # that something of the group was allocated on
+        self._home = self._stage_home = self._stream()   # that sum and staging buffer were allocated on
         # one allocation (and one launch to clear it) for the sum and the word that a bounded wait running out sets
         both = torch.zeros(K * K + 1, dtype=torch.float32, device=self.device)
         self.H = both[:K * K].view(K, K)
@@ -1061,7 +1061,7 @@ class _HessianGroup:
         self._fill = 0
 
     def _stream(self):
-        return stream_ptr(self.device.index) if self.device.type == "cuda" else None
+        return stream_of(self.device.index) if self.device.type == "cuda" else None
 
     def same_input(self, inp: torch.Tensor) -> bool:
         if self._last is None:
@@ -1093,7 +1093,7 @@ class _HessianGroup:
         else:
             if self._stage is None:
                 self._stage = torch.empty((self.stage_tokens, x.shape[1]), dtype=torch.bfloat16, device=self.device)
-                self._streams.add(self._stream())
+                self._stage_home = self._stream()
             if self._fill + t > self.stage_tokens:
                 self.flush()
             self._stage[self._fill: self._fill + t].copy_(x)
@@ -1108,7 +1108,8 @@ class _HessianGroup:
         before this stream has read it."""
         self._last = None
         self.flush()
-        if self._streams - {self._stream()}:
+        here = self._stream()
+        if here != self._home or here != self._stage_home:
             stream = torch.cuda.current_stream(self.device)
             for t in (self.H, self.status, self._stage):
                 if t is not None and t.is_cuda:
