@@ -284,6 +284,13 @@ int b200q_gptq_prologue_many(float* const* H, int count, int64_t K, int64_t ldh,
 int b200q_gptq_zero_dead_columns(const float* diag, int64_t diag_stride, int64_t K, float* Wf,
                                  int64_t N, int64_t ldf, void* stream);
 
+/* b200q_gather_columns_f32 and b200q_gptq_zero_dead_columns in one launch (zero != 0; diag fp32 [K] in the new
+ * order), and, with keep, the same columns in W's type with those of a zero entry of diag as zeros
+ * (the W0 of b200q_gptq_sweep_blocks). */
+int b200q_gather_columns_keep(const void* W, int wdtype, int64_t N, int64_t K, int64_t ldw,
+                              const int32_t* perm, const float* diag, int zero, float* Wf, int64_t ldf,
+                              void* keep, int64_t ldk, void* stream);
+
 /* In place: H (symmetric positive definite, full storage) -> upper-triangular U with
  * U^T U = H^-1, strictly-lower part zeroed.  Stands in for cholesky -> cholesky_inverse ->
  * cholesky(upper=True) (gptq_quantize.py:153-156).  status: four device ints, zeroed by the
@@ -301,6 +308,12 @@ int b200q_gptq_zero_dead_columns(const float* diag, int64_t diag_stride, int64_t
 size_t b200q_gptq_factor_workspace_bytes(int64_t K);
 int b200q_gptq_factor(float* H, int64_t K, int64_t ldh, void* workspace, int* status,
                       void* stream);
+
+/* The same for b200q_gptq_sweep_blocks, at half the work: with H = V V^T (V upper) and the columns in
+ * blocks of 512 from column 0 on, block (b, b) of H ends as U_bb = V_bb^-1 and block (a, b), a < b, as
+ * -V[a, b] U_bb.  What is below the diagonal is left undefined. */
+int b200q_gptq_factor_blocks(float* H, int64_t K, int64_t ldh, void* workspace, int* status,
+                             void* stream);
 
 /* A float32-accurate tensor-core GEMM (tcgen05 kind::tf32, three MMAs per product on hi/lo splits
  * of the operands): the template that makes P and the next square in the factorisation.  Its
@@ -331,6 +344,17 @@ int b200q_gptq_sweep(float* Wf, int64_t N, int64_t K, int64_t ldf, const float* 
                      const void* scale, int sdtype, const void* zp, const int32_t* col_group,
                      const float* global_scale, const b200q_qargs* qa, int blocksize,
                      float* losses, void* workspace, void* stream);
+
+/* The same sweep with what b200q_gptq_factor_blocks has made of the Hessian: the same values up to
+ * rounding.  W0: the weights that Wf holds at first, bf16 or fp32, not written to; its rows 16-byte
+ * aligned (ld0 a multiple of 8).  For K > 512 and as many rows as leave every 32 of them an SM of their own;
+ * b200q_gptq_sweep_takes_blocks says whether (1 or 0), other sizes are B200Q_ERR_ARG.  workspace:
+ * as above. */
+int b200q_gptq_sweep_takes_blocks(int64_t N, int64_t K);
+int b200q_gptq_sweep_blocks(float* Wf, int64_t N, int64_t K, int64_t ldf, const void* W0, int w0dtype,
+                            int64_t ld0, const float* F, int64_t ldu, const void* scale, int sdtype, const void* zp, const int32_t* col_group,
+                            const float* global_scale, const b200q_qargs* qa, int blocksize,
+                            float* losses, void* workspace, void* stream);
 
 /* Many small problems of one shape per launch (the experts of a mixture-of-experts layer, whose
  * per-module calls of gptq_quantize.py:67-264 are otherwise bound by launch overhead).  Every

@@ -86,6 +86,10 @@ SIGNATURES = {
     "b200q_gemm_tf32x3_workspace_bytes": (C.c_size_t, [_i64, _i64, _i64]),
     "b200q_gemm_tf32x3": (_i, [_i, _p, _i64, _p, _i64, _p, _i64, _i64, _i64, _i64, _f, _f, _i, _p, _p, _p]),
     "b200q_gptq_sweep_workspace_bytes": (C.c_size_t, [_i64, _i64, _i]),
+    "b200q_gptq_factor_blocks": (_i, [_p, _i64, _i64, _p, _p, _p]),
+    "b200q_gptq_sweep_takes_blocks": (_i, [_i64, _i64]),
+    "b200q_gather_columns_keep": (_i, [_p, _i, _i64, _i64, _i64, _p, _p, _i, _p, _i64, _p, _i64, _p]),
+    "b200q_gptq_sweep_blocks": (_i, [_p, _i64, _i64, _i64, _p, _i, _i64, _p, _i64, _p, _i, _p, _p, _p, _qa, _i, _p, _p, _p]),
     "b200q_gptq_sweep": (_i, [_p, _i64, _i64, _i64, _p, _i64, _p, _i, _p, _p, _p, _qa, _i, _p, _p, _p]),
     "b200q_gptq_factor_batched_workspace_bytes": (C.c_size_t, [_i64, _i]),
     "b200q_gptq_factor_batched": (_i, [_p, _p, _i, _i64, _i64, _p, _p]),

@@ -20,6 +20,13 @@
 // The last three are one launch on halves with a scale per row: the rows of its second operand are X[o,:o]^T, D^T and P,
 // indexed by absolute column.
 //
+// The blocked form is what the sweep of a single weight needs and half of the work: the squares of U on the diagonal, and
+// beside them S as step o leaves it, -V[:o,o] U_oo, which no later step touches.  Then neither X[o,:o] nor S[i,:o] -= P_i X
+// is computed, 1/3 K^3 instead of 2/3 K^3 (gptq_sweep.cu: products across superblocks take w - q in place of the errors).
+// Its squares are the superblocks of the sweep, so the short one comes first, and the matrix begins with as many rows of the
+// identity as make its order a multiple of 32.  K = 14336: 6.6 ms (U: 9.7), 8192: 2.62 (2.92), 4096: 1.16 (1.22), 768: 0.215
+// (0.245).
+//
 // A pivot <= 0 (or NaN) sets the problem's status; the host then takes the reference's identity fallback.
 #include <type_traits>
 
@@ -39,6 +46,7 @@ constexpr int64_t kScratchFloats = 2LL * OB * NB;   // of the square: P [512][12
 struct Mat {                     // the batch's work matrices and status words
   float* A; int64_t batch, lda;
   int* status;
+  int pad;                       // rows of the identity before the matrix
 };
 
 __device__ __forceinline__ void cp_async16(float* dst, const float* src, int src_bytes) {
@@ -296,7 +304,7 @@ __global__ void __launch_bounds__(kThreads, 1) chol_diag_kernel(Mat mt, int k0, 
   chain_go();
   if (tid == 0 && bad) {
     int* status = mt.status + 4 * blockIdx.x;
-    if (atomicCAS(status, 0, B200Q_NOT_POSITIVE_DEFINITE) == 0) status[1] = k0 + bad;
+    if (atomicCAS(status, 0, B200Q_NOT_POSITIVE_DEFINITE) == 0) status[1] = k0 + bad - mt.pad;
   }
   // D[j][i] = (L^-T)[i][j], zero above the diagonal; a thread turns 4 x 4 entries round
 #pragma unroll
@@ -518,15 +526,19 @@ __global__ void __launch_bounds__(256) split_panel_kernel(Mat mt, int K0, int n,
 __global__ void __launch_bounds__(256) reverse_in_kernel(const float* H0, float* const* Hs, int64_t K, int64_t ldh, Mat mt) {
   const float* H = Hs ? Hs[blockIdx.y] : H0;
   float* A = mt.A + blockIdx.y * mt.batch;
-  for (int64_t r = blockIdx.x; r < K; r += gridDim.x)
-    for (int64_t c = threadIdx.x; c <= r; c += 256) A[r * mt.lda + c] = H[(K - 1 - r) * ldh + (K - 1 - c)];
+  const int64_t end = K + mt.pad;
+  for (int64_t r = blockIdx.x; r < end; r += gridDim.x)
+    for (int64_t c = threadIdx.x; c <= r; c += 256)
+      A[r * mt.lda + c] = c < mt.pad ? (c == r ? 1.0f : 0.0f) : H[(end - 1 - r) * ldh + (end - 1 - c)];
 }
-__global__ void __launch_bounds__(256) reverse_out_kernel(float* H0, float* const* Hs, int64_t K, int64_t ldh, Mat mt) {
+// (`zeros`: the lower part of U; nothing reads it of the blocked form)
+__global__ void __launch_bounds__(256) reverse_out_kernel(float* H0, float* const* Hs, int64_t K, int64_t ldh, Mat mt, bool zeros) {
   float* U = Hs ? Hs[blockIdx.y] : H0;
   const float* A = mt.A + blockIdx.y * mt.batch;
+  const int64_t end = K + mt.pad;
   for (int64_t r = blockIdx.x; r < K; r += gridDim.x)
-    for (int64_t c = threadIdx.x; c < K; c += 256)
-      U[r * ldh + c] = (c >= r) ? A[(K - 1 - r) * mt.lda + (K - 1 - c)] : 0.0f;
+    for (int64_t c = (zeros ? 0 : r / 32 * 32) + threadIdx.x; c < K; c += 256)
+      U[r * ldh + c] = (c >= r) ? A[(end - 1 - r) * mt.lda + (end - 1 - c)] : 0.0f;
 }
 
 static int64_t round_up(int64_t v, int64_t m) { return (v + m - 1) / m * m; }
@@ -536,24 +548,25 @@ static int64_t round_up(int64_t v, int64_t m) { return (v + m - 1) / m * m; }
 // two copies of the update's operand of halves with its scales, a row per matrix row
 static int64_t problem_floats(int64_t K) {
   const int64_t rows = round_up(K, NB);
-  return K * round_up(K, 32) + kScratchFloats + (K > OB ? 6 * OB * OB + 5 * rows * OB + 2 * rows : 0);
+  return round_up(K, 32) * round_up(K, 32) + kScratchFloats + (K > OB ? 6 * OB * OB + 5 * rows * OB + 2 * rows : 0);
 }
 
 // SMs the bulk of an update leaves to the chain beside it: the square's kernels are small (24 to 120 CTAs of which
 // several fit an SM), and while the matrix is narrow the chain is the longer of the two
 static int chain_reserve(int64_t K) { return K <= 6144 ? 40 : 20; }
 
-static int factor(float* H, float* const* Hs, int batch, int64_t K, int64_t ldh, float* ws, int* status, bool lookahead,
-                  cudaStream_t st) {
+// `blocks`: the blocked form in place of U
+static int factor(float* H, float* const* Hs, int batch, int64_t order, int64_t ldh, float* ws, int* status, bool lookahead,
+                  bool blocks, cudaStream_t st) {
   using tgemm::Job;
   using tgemm::Operand;
   const int slice = Hs ? tgemm::kShortSlice : tgemm::kLongSlice;   // (measured where they are defined)
   const int slice16 = Hs ? tgemm::kShortestSlice16 : tgemm::kLongSlice16;
   int rc;
 #define B200Q_RC(expr) do { rc = (expr); if (rc != B200Q_OK) return rc; } while (0)
-  const int64_t lda = round_up(K, 32), rows = round_up(K, NB);
+  const int64_t lda = round_up(order, 32), K = blocks ? lda : order, rows = round_up(K, NB);
   Mat mt;
-  mt.A = ws; mt.batch = K * lda; mt.lda = lda; mt.status = status;
+  mt.A = ws; mt.batch = K * lda; mt.lda = lda; mt.status = status; mt.pad = (int)(K - order);
   float* P = ws + (int64_t)batch * K * lda;
   float* d_hi = P + (int64_t)batch * kScratchFloats;
   float* d_lo = d_hi + (int64_t)batch * OB * OB;
@@ -570,18 +583,19 @@ static int factor(float* H, float* const* Hs, int batch, int64_t K, int64_t ldh,
   auto grid = [&](int64_t x, int64_t cap_x) { return dim3((unsigned)(x < cap_x ? x : cap_x), (unsigned)batch, 1); };
   const int64_t row_ctas = batch > 8 ? 2 * kNumSMs / batch + 1 : 8 * kNumSMs;
 
-  reverse_in_kernel<<<grid(K, row_ctas), 256, 0, st>>>(H, Hs, K, ldh, mt);
+  reverse_in_kernel<<<grid(K, row_ctas), 256, 0, st>>>(H, Hs, order, ldh, mt);
   B200Q_LAUNCH_CHECK();
   // Look-ahead: the chain (caller's stream) works on the next square while the products of this step that the next
   // square does not need run on a helper stream.  Arithmetic and its order do not depend on it.
   tgemm::SideStream* side = lookahead && K > 2 * OB ? tgemm::side_stream(st) : nullptr;
   cudaStream_t bulk = side ? side->stream : st;
   bool side_busy = false;
-  for (int64_t K0 = 0, step = 0; K0 < K; K0 += OB, ++step) {
-    const int n = (int)(K - K0 < OB ? K - K0 : OB), blocks = (n + NB - 1) / NB;
-    const int64_t K1 = K0 + n;
+  const int64_t first = blocks && K % OB ? K % OB : OB;
+  for (int64_t K0 = 0, K1 = 0, step = 0; K0 < K; K0 = K1, ++step) {
+    const int whole = (int)(step == 0 ? first : OB), n = (int)(K - K0 < whole ? K - K0 : whole), inner = (n + NB - 1) / NB;
+    K1 = K0 + n;
     const bool last = K1 >= K;
-    for (int k = 0; k < blocks; ++k) {
+    for (int k = 0; k < inner; ++k) {
       const int bn = n - k * NB < NB ? n - k * NB : NB, below = n - k * NB - bn;
       B200Q_TRY(launch_chained(chol_diag_kernel, dim3(batch), kThreads, chol_smem, st, mt, (int)K0 + k * NB, bn));
       B200Q_LAUNCH_CHECK();
@@ -594,7 +608,10 @@ static int factor(float* H, float* const* Hs, int batch, int64_t K, int64_t ldh,
                                mt, P, (int)K0, n, k, tiles));
       B200Q_LAUNCH_CHECK();
     }
-    if (K0 == 0 && last) break;
+    if (last && (K0 == 0 || blocks)) {
+      if (side_busy) B200Q_TRY(cudaStreamWaitEvent(st, side->done, 0));
+      break;
+    }
     float* f_hi = f_base + (step & 1) * 2 * batch * (int64_t)OB * OB;
     float* f_lo = f_hi + batch * (int64_t)OB * OB;
     __half* q_hi = q_base + (step & 1) * 2 * cap;
@@ -637,24 +654,27 @@ static int factor(float* H, float* const* Hs, int batch, int64_t K, int64_t ldh,
       bulk = st;
     }
     // the other rows of P, and X[o,:o] with its transpose
-    B200Q_RC(split_panel(K1 + n2, K, K0, bulk));
+    const int64_t left = blocks ? 0 : K0;   // columns before the square that take part
+    B200Q_RC(split_panel(K1 + n2, K, left, bulk));
     Job r = j;
-    r.set = tgemm::kPanel; r.skip0 = (int)K0; r.skip1 = (int)(K1 + n2); r.M = (int)K;
+    r.set = tgemm::kPanel; r.skip0 = (int)left; r.skip1 = (int)(K1 + n2); r.M = (int)K;
     if (!last) r.out_hi = p_all;
-    r.X = mt.A + K0 * lda; r.x_batch = mt.batch; r.ldx = lda; r.xt_rows = (int)K0;
+    if (left) { r.X = mt.A + K0 * lda; r.x_batch = mt.batch; r.ldx = lda; r.xt_rows = (int)K0; }
     r.max_ctas = side && !last ? kNumSMs - chain_reserve(K) : 0;
     B200Q_RC(tgemm::launch(r, bulk));
     if (last) break;
     if (side) B200Q_TRY(cudaStreamWaitEvent(bulk, side->next, 0));
-    // the update's operand: X[o,:o]^T and D^T, P (of the next block's rows from its operand form)
-    B200Q_RC(tgemm::split_update16(tgemm::UpdateOperand{mt.A + K0 * lda, lda, mt.batch, n, K1, f_hi, f_lo, (int64_t)OB * OB, n2,
-                                                        p_all + (K1 + n2) * OB, pb, K - K1 - n2, q_hi, q_lo, q_scale, rows},
-                                   batch, bulk));
+    // the update's operand: X[o,:o]^T and D^T, P (of the next block's rows from its operand form); everything from column c0 on
+    const int64_t c0 = K0 - left;
+    B200Q_RC(tgemm::split_update16(tgemm::UpdateOperand{mt.A + K0 * lda + c0, lda, mt.batch, n, K1 - c0, f_hi, f_lo,
+                                                        (int64_t)OB * OB, n2, p_all + (K1 + n2) * OB, pb, K - K1 - n2,
+                                                        q_hi + c0 * OB, q_lo + c0 * OB, q_scale + c0, rows}, batch, bulk));
     // S[below,o] = -P D, S[i,:o] -= P_i X[o,:o], A[i,j] -= P_i P_j^T, without the next square
     Job u;
-    u.A = Q; u.B = Q; u.A.row0 = 0; u.M = u.N = (int)K; u.Kd = n; u.set = tgemm::kBulk; u.batch = batch;
-    u.row_begin = (int)K1; u.skip0 = (int)K1; u.skip1 = (int)(K1 + n2);
-    u.alpha = -1.0f; u.beta = 1.0f; u.C = mt.A; u.c_batch = mt.batch; u.ldc = lda; u.fresh0 = (int)K0; u.fresh1 = (int)K1;
+    u.A = u.B = Q; u.A.row0 = u.B.row0 = (int)c0; u.M = u.N = (int)(K - c0); u.Kd = n; u.set = tgemm::kBulk; u.batch = batch;
+    u.row_begin = u.skip0 = (int)(K1 - c0); u.skip1 = (int)(K1 + n2 - c0);
+    u.alpha = -1.0f; u.beta = 1.0f; u.C = mt.A + c0 * (lda + 1); u.c_batch = mt.batch; u.ldc = lda;
+    u.fresh0 = (int)(K0 - c0); u.fresh1 = (int)(K1 - c0);
     u.status = status + 2; u.status_stride = 4; u.max_ctas = r.max_ctas; u.slice = slice16;
     B200Q_RC(tgemm::launch(u, bulk));
     if (side) {
@@ -663,7 +683,7 @@ static int factor(float* H, float* const* Hs, int batch, int64_t K, int64_t ldh,
     }
   }
 #undef B200Q_RC
-  reverse_out_kernel<<<grid(K, row_ctas), 256, 0, st>>>(H, Hs, K, ldh, mt);
+  reverse_out_kernel<<<grid(K, row_ctas), 256, 0, st>>>(H, Hs, order, ldh, mt, !blocks);
   B200Q_LAUNCH_CHECK();
   return B200Q_OK;
 }
@@ -681,7 +701,12 @@ size_t b200q_gptq_factor_workspace_bytes(int64_t K) {
 
 int b200q_gptq_factor(float* H, int64_t K, int64_t ldh, void* workspace, int* status, void* stream) {
   if (!H || !workspace || !status || K <= 0 || ldh < K || K > (1 << 24)) return B200Q_ERR_ARG;
-  return factor::factor(H, nullptr, 1, K, ldh, (float*)workspace, status, true, (cudaStream_t)stream);
+  return factor::factor(H, nullptr, 1, K, ldh, (float*)workspace, status, true, false, (cudaStream_t)stream);
+}
+
+int b200q_gptq_factor_blocks(float* H, int64_t K, int64_t ldh, void* workspace, int* status, void* stream) {
+  if (!H || !workspace || !status || K <= 0 || ldh < K || K > (1 << 24)) return B200Q_ERR_ARG;
+  return factor::factor(H, nullptr, 1, K, ldh, (float*)workspace, status, true, true, (cudaStream_t)stream);
 }
 
 size_t b200q_gptq_factor_batched_workspace_bytes(int64_t K, int count) {
@@ -698,7 +723,7 @@ int b200q_gptq_factor_many(float* const* H, int count, int64_t K, int64_t ldh, v
   if (K > 4096) return B200Q_ERR_UNSUPPORTED;
   cudaStream_t st = (cudaStream_t)stream;
   B200Q_TRY(cudaMemsetAsync(status, 0, sizeof(int) * 4 * (size_t)count, st));
-  return factor::factor(nullptr, H, count, K, ldh, (float*)workspace, status, false, st);
+  return factor::factor(nullptr, H, count, K, ldh, (float*)workspace, status, false, false, st);
 }
 
 int b200q_gptq_factor_batched(float* const* H, float* const* scratch, int count, int64_t K, int64_t ldh, int* status,

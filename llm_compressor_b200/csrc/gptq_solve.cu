@@ -66,6 +66,9 @@ struct Columns {
   void* dst; void* const* dst_table; int64_t dst_batch;
   const int32_t* perm; const int32_t* const* perm_table; int64_t perm_batch;
   const float* const* diag_table;     // gather: columns with a zero entry come out as zeros
+  const float* diag;                  // the same of a single problem
+  void* keep; int64_t ldk;            // gather: the values in the source's type as well, columns with a zero entry of
+  const float* keep_diag;             // this as zeros
   const float* damp;                  // gather of a square matrix with `rows`: diagonal 0 -> 1, + damp[problem]
   int64_t N, K, lds, ldd;
   bool rows;                          // gather: rows in the order of perm too
@@ -91,7 +94,8 @@ __global__ void __launch_bounds__(256) plain_columns_kernel(Columns j, int tx_lo
   using T = typename E::type;
   const int TX = 1 << tx_log2, tx = threadIdx.x & (TX - 1), ty = threadIdx.x >> tx_log2, rows = 256 >> tx_log2;
   const int32_t* perm = j.order();
-  const float* dg = GATHER && j.diag_table ? j.diag_table[blockIdx.y] : nullptr;
+  const float* dg = GATHER ? (j.diag_table ? j.diag_table[blockIdx.y] : j.diag) : nullptr;
+  T* keep = GATHER ? (T*)j.keep : nullptr;
   const void* in = j.in();
   const bool vec = j.vec && !perm && aligned16(in) && aligned16(GATHER ? (void*)j.template out<float>() : (void*)j.template out<T>());
   for (int64_t r = (int64_t)blockIdx.x * rows + ty; r < j.N; r += (int64_t)gridDim.x * rows) {
@@ -113,6 +117,14 @@ __global__ void __launch_bounds__(256) plain_columns_kernel(Columns j, int tx_lo
           float4* o = reinterpret_cast<float4*>(j.template out<float>() + r * j.ldd + c);
           o[0] = make_float4(v[0], v[1], v[2], v[3]);
           o[1] = make_float4(v[4], v[5], v[6], v[7]);
+          if (keep) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+              if (j.keep_diag[c + e] == 0.0f) E::store(t + e, 0.0f);
+            T* k = keep + r * j.ldk + c;
+#pragma unroll
+            for (int e = 0; e < (int)sizeof(T) / 2; ++e) reinterpret_cast<uint4*>(k)[e] = reinterpret_cast<const uint4*>(t)[e];
+          }
         } else {
           const float4* w = reinterpret_cast<const float4*>((const float*)in + r * j.lds + c);
           *reinterpret_cast<float4*>(v) = w[0];
@@ -130,6 +142,7 @@ __global__ void __launch_bounds__(256) plain_columns_kernel(Columns j, int tx_lo
         const int64_t at = perm ? perm_at(perm, c, j.K) : c;
         if constexpr (GATHER) {
           float v = (dg && dg[c] == 0.0f) ? 0.0f : E::load((const T*)in + from * j.lds + at);
+          if (keep) keep[r * j.ldk + c] = j.keep_diag[c] == 0.0f ? T(0.0f) : ((const T*)in)[from * j.lds + at];
           if (j.damp && c == r) v = (v == 0.0f ? 1.0f : v) + j.damp[blockIdx.y];
           j.template out<float>()[r * j.ldd + c] = v;
         } else {
@@ -151,8 +164,9 @@ __global__ void __launch_bounds__(256) gather_columns_kernel(Columns j) {
   extern __shared__ __align__(16) unsigned char smem[];
   Quad<T>* s = reinterpret_cast<Quad<T>*>(smem);
   const int32_t* perm = j.order();
-  const float* dg = j.diag_table ? j.diag_table[blockIdx.y] : nullptr;
+  const float* dg = j.diag_table ? j.diag_table[blockIdx.y] : j.diag;
   const T* in = (const T*)j.in();
+  T* keep = (T*)j.keep;
   float* out = j.template out<float>();
   const bool vec = j.vec && aligned16(in);
   for (int64_t r0 = (int64_t)blockIdx.x * 4; r0 < j.N; r0 += (int64_t)gridDim.x * 4) {
@@ -178,11 +192,12 @@ __global__ void __launch_bounds__(256) gather_columns_kernel(Columns j) {
 #pragma unroll 4
     for (int c = threadIdx.x; c < j.K; c += 256) {
       const Quad<T> q = s[perm_at(perm, c, j.K)];
-      const bool dead = dg && dg[c] == 0.0f;
+      const bool dead = dg && dg[c] == 0.0f, none = keep && j.keep_diag[c] == 0.0f;
 #pragma unroll
       for (int y = 0; y < 4; ++y) {
         if (y >= nr) break;
         float v = dead ? 0.0f : E::load(&q.v[y]);
+        if (keep) keep[(r0 + y) * j.ldk + c] = none ? T(0.0f) : q.v[y];
         if (j.damp && c == r0 + y) v = (v == 0.0f ? 1.0f : v) + j.damp[blockIdx.y];
         out[(r0 + y) * j.ldd + c] = v;
       }
@@ -405,6 +420,19 @@ int b200q_gather_columns_f32(const void* W, int wdtype, int64_t N, int64_t K, in
   j.src = W; j.dst = Wf; j.perm = perm;
   j.N = N; j.K = K; j.lds = ldw; j.ldd = ldf;
   j.vec = pieces_ok(W, ldw, K) && (perm || pieces_ok(Wf, ldf, K));
+  if (wdtype == B200Q_BF16) return launch_columns<B200Q_BF16, true>(j, 1, (cudaStream_t)stream);
+  if (wdtype == B200Q_F32) return launch_columns<B200Q_F32, true>(j, 1, (cudaStream_t)stream);
+  return B200Q_ERR_UNSUPPORTED;
+}
+
+int b200q_gather_columns_keep(const void* W, int wdtype, int64_t N, int64_t K, int64_t ldw, const int32_t* perm,
+                              const float* diag, int zero, float* Wf, int64_t ldf, void* keep, int64_t ldk, void* stream) {
+  if (!W || !Wf || N <= 0 || K <= 0 || ldw < K || ldf < K || (keep && ldk < K) || ((zero || keep) && !diag)) return B200Q_ERR_ARG;
+  Columns j = {};
+  j.src = W; j.dst = Wf; j.perm = perm; j.diag = zero ? diag : nullptr;
+  j.keep = keep; j.ldk = ldk; j.keep_diag = diag;
+  j.N = N; j.K = K; j.lds = ldw; j.ldd = ldf;
+  j.vec = pieces_ok(W, ldw, K) && (perm || (pieces_ok(Wf, ldf, K) && (!keep || pieces_ok(keep, ldk, K))));
   if (wdtype == B200Q_BF16) return launch_columns<B200Q_BF16, true>(j, 1, (cudaStream_t)stream);
   if (wdtype == B200Q_F32) return launch_columns<B200Q_F32, true>(j, 1, (cudaStream_t)stream);
   return B200Q_ERR_UNSUPPORTED;

@@ -7,6 +7,13 @@
 // fp32-accurate tensor-core product (tgemm).  What the reference calls its block size only orders float32 operations
 // and does not change the result otherwise, so it does not decide the split here.
 //
+// With the factor's blocked form (V upper, H = V V^T, U = V^-1; b200q_gptq_factor_blocks) the products across superblocks
+// use Err U = W - Q, that is Err = (W - Q) V: what the columns of superblock b get from those before it is
+// (W - Q)[:, :b] V[:b, b] U_bb.  The same product with W - Q in place of the errors and -V U_bb in place of U, without the
+// triangular inverse, half of the factor's work; W as it was is needed for it.  Error of the last column against float64, all
+// codes zero, 4096 columns: 2.3e-7 of its root mean square.  Reading W again costs the sweep 2 to 5 % (4096 x 4096: 757 us with
+// U, 787; 4096 x 14336: 4376, 4483), the factor saves more.
+//
 // Each correction is one fused multiply-add (the reference rounds the product first), true divisions decide a code
 // wherever an ulp could matter.
 #include <cstdlib>
@@ -45,7 +52,8 @@ struct Params {
   int strategy, group_size, block_h, zp_kind;
   int64_t groups_per_row;
   QRange qr;
-  float* err; int64_t lde, err_batch;                     // the superblock's errors (null: nothing after it)
+  float* err; int64_t lde, err_batch;                     // the superblock's errors (null: nothing after it), or
+  const void* W0; int64_t ld0; int w0dtype;               // (set) what its columns differ from these by
   int i1, sb;                                             // superblock: first column, width
   int sdtype;                                             // of the scales
   const unsigned char* tiles; int64_t tiles_batch;        // operand form of U[i1 : i1 + sb, i1 : i1 + sb], one a factor
@@ -171,7 +179,7 @@ constexpr int64_t powers_offset(int sblk) { return scales_offset(sblk) + sblk * 
 constexpr int64_t band_offset(int sblk) { return powers_offset(sblk) + sblk * 4; }
 constexpr int64_t tiles_bytes(int sblk) { return band_offset(sblk) + sblk / kMicro * kBandFloats * 4; }   // of one factor
 // Further CTAs (from `squares` on) make the operand of the trailing product: the columns behind the square.
-struct Slice { __half *hi, *lo; float* scale; int64_t cols, rows; };   // rows of the operand per factor
+struct Slice { __half *hi, *lo; float* scale; int64_t cols, rows; bool inverse; };   // rows of the operand per factor
 template <int SBLK>
 __global__ void __launch_bounds__(kTileThreads) square_tiles_kernel(Ptr<const float> Us, int64_t ldu, int i1, int sb,
                                                                    unsigned char* tiles, int64_t batch_bytes, int squares,
@@ -187,7 +195,7 @@ __global__ void __launch_bounds__(kTileThreads) square_tiles_kernel(Ptr<const fl
   if ((int)blockIdx.x >= squares) {
     const int64_t at = blockIdx.y * slice.rows;
     tgemm::split_columns16<SBLK>(U + sb, ldu, sb, slice.cols, INT64_MAX / 2, slice.hi + at * SBLK, slice.lo + at * SBLK,
-                                 slice.scale + at, true, blockIdx.x - squares, stage);
+                                 slice.scale + at, slice.inverse ? tgemm::kInverses : tgemm::kPowers, blockIdx.x - squares, stage);
     return;
   }
   tiles += blockIdx.y * batch_bytes;
@@ -627,6 +635,21 @@ sweep_block_kernel(const __grid_constant__ Params p) {
     float loss = 0.0f;
 #pragma unroll 1
     for (int m = 0; m < micros; ++m) {
+      const bool from = ROWS == 32 && p.W0 && out;   // (wider CTAs are never given the blocked form)
+      uint4 w0[kMicro / 4];   // asked for before the wait
+      if (from) {
+        const bool half = p.w0dtype == B200Q_BF16;
+        const int64_t col = row * p.ld0 + p.i1 + m * kMicro;
+        const uint4* src = reinterpret_cast<const uint4*>((const char*)p.W0 + (half ? 2 : 4) * col);
+        w0[0] = src[0]; w0[1] = src[1];
+        if (!half) {
+          w0[2] = src[2]; w0[3] = src[3];
+        } else {
+          auto wide = [](uint32_t a, uint32_t b) { return make_uint4(a << 16, a & 0xFFFF0000u, b << 16, b & 0xFFFF0000u); };
+          const uint4 a = w0[0], b = w0[1];
+          w0[0] = wide(a.x, a.y); w0[1] = wide(a.z, a.w); w0[2] = wide(b.x, b.y); w0[3] = wide(b.z, b.w);
+        }
+      }
       bar_wait(smem_u32(&s_done[2 * m + 1]), 0, &s_abort);
       const float* es = sE + (m & (kErrSlots - 1)) * kMicro * ROWS + r;
       const int64_t at = job * p.err_batch + row * p.lde + m * kMicro;
@@ -639,7 +662,15 @@ sweep_block_kernel(const __grid_constant__ Params p) {
           x[k] = -es[(t + k) * ROWS];
           sum = fmaf(x[k], x[k], sum);
         }
-        if (out) *reinterpret_cast<float4*>(p.err + at + t) = make_float4(x[0], x[1], x[2], x[3]);
+        if (out && !from) *reinterpret_cast<float4*>(p.err + at + t) = make_float4(x[0], x[1], x[2], x[3]);
+      }
+      if (from) {
+        const float* q = sW + m * kMicro * S::kWld + r;
+#pragma unroll
+        for (int k = 0; k < kMicro / 4; ++k)
+          *reinterpret_cast<float4*>(p.err + at + 4 * k) =
+              make_float4(__uint_as_float(w0[k].x) - q[4 * k * S::kWld], __uint_as_float(w0[k].y) - q[(4 * k + 1) * S::kWld],
+                          __uint_as_float(w0[k].z) - q[(4 * k + 2) * S::kWld], __uint_as_float(w0[k].w) - q[(4 * k + 3) * S::kWld]);
       }
       __syncwarp();
       if (lane == 0) bar_arrive(smem_u32(&s_out[m]));
@@ -890,6 +921,7 @@ static int sweep(Params p, int sdtype, bool global, int batch, const float* cons
   const int64_t N = p.N, K = p.K;
   const bool has_u = p.U.one || p.U.table;
   const Layout l = layout_of(N, K, batch, distinct_u, may_overlap);
+  const bool blocks = p.W0 != nullptr;
   // header of the workspace: a status word that a bounded wait expiring in a sweep or a trailing product sets to
   // B200Q_ERR_DEVICE (cleared here, read by the caller afterwards)
   int* status = (int*)workspace;
@@ -930,7 +962,7 @@ static int sweep(Params p, int sdtype, bool global, int batch, const float* cons
     if (squares + cols == 0) return B200Q_OK;
     B200Q_TRY(launch_chained(square, dim3((unsigned)(squares + (cols + 31) / 32), distinct_u), kTileThreads, square_smem, on, factors,
                              p.ldu, (int)i1, w, t.tiles, p.tiles_batch, squares,
-                             Slice{t.u_hi, t.u_lo, t.u_scale, cols, l.rows_k}));
+                             Slice{t.u_hi, t.u_lo, t.u_scale, cols, l.rows_k, blocks}));
     B200Q_LAUNCH_CHECK();
     return B200Q_OK;
   };
@@ -964,7 +996,7 @@ static int sweep(Params p, int sdtype, bool global, int batch, const float* cons
     // behind its wait for side->done only: the slice below.  The powers of the pivots come with the square's tiles, the
     // first of which are this stream's own; the others were waited for before the product of the superblock before.
     if ((rc = tgemm::split_rows16(t.err, l.sb, p.err_batch, N, w, t.e_hi, t.e_lo, t.e_scale, l.sb, l.rows_n, batch,
-                                  (const float*)(t.tiles + powers_offset(l.sb)), p.tiles_batch / 4, u_index, st)))
+                                  (const float*)(t.tiles + powers_offset(l.sb)), blocks, p.tiles_batch / 4, u_index, st)))
       return rc;
     tgemm::Job j;
     j.A = tgemm::Operand{t.e_hi, t.e_lo, l.sb, l.rows_n * batch, l.rows_n, 0, t.e_scale};
@@ -1024,9 +1056,12 @@ size_t b200q_gptq_sweep_workspace_bytes(int64_t N, int64_t K, int blocksize) {
   return sweep::layout_of(N, K, 1, 1, true).bytes;
 }
 
-int b200q_gptq_sweep(float* Wf, int64_t N, int64_t K, int64_t ldf, const float* U, int64_t ldu, const void* scale,
+int b200q_gptq_sweep_takes_blocks(int64_t N, int64_t K) { return N > 0 && sweep::wide(N, 1) && K > 512; }
+
+static int sweep_one(float* Wf, int64_t N, int64_t K, int64_t ldf, const float* U, int64_t ldu, const void* scale,
                      int sdtype, const void* zp, const int32_t* col_group, const float* gscale,
-                     const b200q_qargs* qa, int blocksize, float* losses, void* workspace, void* stream) {
+                     const b200q_qargs* qa, int blocksize, float* losses, const void* W0, int w0dtype, int64_t ld0,
+                     void* workspace, void* stream) {
   using namespace b200q::sweep;
   if (!Wf || !scale || !qa || !losses || !workspace || N <= 0 || K <= 0 || ldf < K) return B200Q_ERR_ARG;
   if (U && ldu < K) return B200Q_ERR_ARG;
@@ -1036,8 +1071,23 @@ int b200q_gptq_sweep(float* Wf, int64_t N, int64_t K, int64_t ldf, const float* 
   int rc = fill_scheme(&p, qa, N, K, col_group); if (rc) return rc;
   p.W = {Wf, nullptr}; p.U = {U, nullptr}; p.scale = {scale, nullptr}; p.zp = {zp, nullptr};
   p.col_group = {col_group, nullptr}; p.gscale = {gscale, nullptr}; p.losses = {losses, nullptr};
-  p.N = N; p.K = K; p.ldw = ldf; p.ldu = ldu;
+  p.N = N; p.K = K; p.ldw = ldf; p.ldu = ldu; p.W0 = W0; p.w0dtype = w0dtype; p.ld0 = ld0;
   return sweep::sweep(p, sdtype, gscale != nullptr, 1, nullptr, 1, nullptr, true, workspace, (cudaStream_t)stream);
+}
+
+int b200q_gptq_sweep(float* Wf, int64_t N, int64_t K, int64_t ldf, const float* U, int64_t ldu, const void* scale,
+                     int sdtype, const void* zp, const int32_t* col_group, const float* gscale,
+                     const b200q_qargs* qa, int blocksize, float* losses, void* workspace, void* stream) {
+  return sweep_one(Wf, N, K, ldf, U, ldu, scale, sdtype, zp, col_group, gscale, qa, blocksize, losses, nullptr, 0, 0, workspace, stream);
+}
+
+int b200q_gptq_sweep_blocks(float* Wf, int64_t N, int64_t K, int64_t ldf, const void* W0, int w0dtype, int64_t ld0,
+                            const float* F, int64_t ldu, const void* scale, int sdtype, const void* zp, const int32_t* col_group, const float* gscale,
+                            const b200q_qargs* qa, int blocksize, float* losses, void* workspace, void* stream) {
+  if (!F || !W0 || !b200q_gptq_sweep_takes_blocks(N, K) || ld0 < K || (ld0 & 7) || ((uintptr_t)W0 & 15)) return B200Q_ERR_ARG;
+  if (w0dtype != B200Q_BF16 && w0dtype != B200Q_F32) return B200Q_ERR_UNSUPPORTED;
+  return sweep_one(Wf, N, K, ldf, F, ldu, scale, sdtype, zp, col_group, gscale, qa, blocksize, losses, W0, w0dtype, ld0,
+                   workspace, stream);
 }
 
 size_t b200q_gptq_sweep_many_workspace_bytes(int64_t N, int64_t K, int count, int distinct) {
@@ -1055,6 +1105,7 @@ int b200q_gptq_sweep_many(float* const* W, const float* const* U, const float* c
   if (count > 65535 || (U && (!distinct_u || distinct <= 0 || distinct > 65535)) || ((uintptr_t)workspace) & 15) return B200Q_ERR_ARG;
   Params p;
   int rc = fill_scheme(&p, qa, N, K, nullptr); if (rc) return rc;
+  p.W0 = nullptr;
   p.W = {nullptr, W}; p.U = {nullptr, U}; p.scale = {nullptr, scale}; p.zp = {nullptr, zp};
   p.col_group = {nullptr, col_group}; p.gscale = {nullptr, gscale}; p.losses = {nullptr, losses};
   p.N = N; p.K = K; p.ldw = ldw; p.ldu = ldu;

@@ -400,10 +400,11 @@ tgemm_kernel(const __grid_constant__ CUtensorMap a_hi, const __grid_constant__ C
         C = j.c_table ? j.c_table[b] + j.c_offset : j.C + (int64_t)b * j.c_batch;
         vec = ((j.ldc & 3) == 0) && ((((uintptr_t)C) & 15) == 0);
       }
+      const int cols = j.set == kBulk && row0 < j.skip1 ? j.skip0 : j.N;   // (a tile may reach beyond skip0)
 #pragma unroll
       for (int k = 0; k < kHalf / 32; ++k) {
         const int col0 = colw + k * 32;
-        if (col0 >= j.N) break;   // warp-uniform
+        if (col0 >= cols) break;   // warp-uniform
         const int cc = col0 + sub_col;
         if constexpr (SPLIT_OUT) {
           if (j.X && row0 < j.xt_rows && row0 + lane < j.M) {
@@ -578,12 +579,12 @@ template <int LD>
 __global__ void __launch_bounds__(256) split_rows16_kernel(const float* __restrict__ src, int64_t ld_src, int64_t src_batch,
                                                            int64_t rows, int cols, __half* hi, __half* lo, float* scale,
                                                            int64_t dst_rows, const float* __restrict__ columns,
-                                                           int64_t columns_batch, const int32_t* __restrict__ index) {
+                                                           bool inverse, int64_t columns_batch, const int32_t* __restrict__ index) {
   chain_wait();
   chain_go();
   const int64_t at = blockIdx.y * dst_rows;
   split_rows16<LD>(src + blockIdx.y * src_batch, nullptr, ld_src, rows, cols, hi + at * LD, lo + at * LD, scale + at,
-                   columns ? columns + (index ? index[blockIdx.y] : blockIdx.y) * columns_batch : nullptr, blockIdx.x, gridDim.x);
+                   columns ? columns + (index ? index[blockIdx.y] : blockIdx.y) * columns_batch : nullptr, inverse, blockIdx.x, gridDim.x);
 }
 // The operand of an update of the factor in one launch: `transposed` CTAs take the columns of the block row, the others rows
 // from its end on, `first` of them from a tf32 operand form.
@@ -595,16 +596,16 @@ __global__ void __launch_bounds__(256) split_update16_kernel(const UpdateOperand
   __half *hi = u.hi + at * kMaxDepth, *lo = u.lo + at * kMaxDepth;
   float* scale = u.scale + at;
   if ((int)blockIdx.x < transposed) {
-    split_columns16<kMaxDepth>(u.row + blockIdx.y * u.row_batch, u.row_ld, u.n, u.end, u.end - u.n, hi, lo, scale, false, blockIdx.x,
+    split_columns16<kMaxDepth>(u.row + blockIdx.y * u.row_batch, u.row_ld, u.n, u.end, u.end - u.n, hi, lo, scale, kNoPivots, blockIdx.x,
                                stage16);
     return;
   }
   const int64_t cta = blockIdx.x - transposed, ctas = gridDim.x - transposed;
   hi += u.end * kMaxDepth; lo += u.end * kMaxDepth; scale += u.end;
   split_rows16<kMaxDepth>(u.f_hi + blockIdx.y * u.f_batch, u.f_lo + blockIdx.y * u.f_batch, kMaxDepth, u.first, u.n, hi, lo, scale,
-                          nullptr, cta, ctas);
+                          nullptr, false, cta, ctas);
   hi += u.first * kMaxDepth; lo += u.first * kMaxDepth; scale += u.first;
-  split_rows16<kMaxDepth>(u.p + blockIdx.y * u.p_batch, nullptr, kMaxDepth, u.rows, u.n, hi, lo, scale, nullptr, cta, ctas);
+  split_rows16<kMaxDepth>(u.p + blockIdx.y * u.p_batch, nullptr, kMaxDepth, u.rows, u.n, hi, lo, scale, nullptr, false, cta, ctas);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -656,13 +657,13 @@ int split_transposed(const float* src, int64_t ld_src, int rows, int cols, float
 }
 
 int split_rows16(const float* src, int64_t ld_src, int64_t src_batch, int64_t rows, int cols, __half* hi, __half* lo, float* scale,
-                 int ld, int64_t dst_rows, int batch, const float* columns, int64_t columns_batch, const int32_t* index,
+                 int ld, int64_t dst_rows, int batch, const float* columns, bool inverse, int64_t columns_batch, const int32_t* index,
                  cudaStream_t st) {
   if (rows <= 0 || cols <= 0) return B200Q_OK;
   auto kernel = ld == 512 ? split_rows16_kernel<512> : split_rows16_kernel<256>;
   const int64_t blocks = (rows + 7) / 8, cap = 8 * kNumSMs / batch + 1;
   B200Q_TRY(launch_chained(kernel, dim3((unsigned)(blocks < cap ? blocks : cap), (unsigned)batch), 256, 0, st, src, ld_src,
-                           src_batch, rows, cols, hi, lo, scale, dst_rows, columns, columns_batch, index));
+                           src_batch, rows, cols, hi, lo, scale, dst_rows, columns, inverse, columns_batch, index));
   B200Q_LAUNCH_CHECK();
   return B200Q_OK;
 }

@@ -117,6 +117,8 @@ int split_transposed(const float* src, int64_t ld_src, int rows, int cols, float
 // Error of the last column of a sweep with all codes zero, 1001 x 1160, sizes 2^-18 .. 2^18: even weights 4.4e-7, weights
 // that go as 1 / s_p 2.3e-7, rows of U in any sizes 2.3e-7 (2.4e-2, 2.2e-2 and 2.1e-7 with the whole grading on U's side);
 // equal sizes 2.1e-7 either way.
+// With w - q in place of the errors and -V U_bb in place of U it is the other way round: V is R's factor with its rows times
+// s_p, so w - q are taken times the root's inverse and the rows times the root.
 // (The factor needs none of this: in A - P P^T, P D and P X the contraction index has the columns of L = S L', whose rows
 // are graded, and the rows of L^-1, whose columns are; what is left are the pivots of L', the factor of a matrix with unit
 // diagonal, and where one of these is below 2^-12 float32 elimination fails.)
@@ -130,17 +132,20 @@ __device__ __forceinline__ float pivot_inverse(float reciprocal) {
 
 // Operands of halves, rows of LD = 512 or 256 zero-padded beyond `cols`.
 // Rows of src (src2 set: src + src2) -> hi / lo [rows][LD], scale[row], by CTA `cta` of `ctas` (256 threads): a warp takes a row,
-// kept in registers between the search for its largest value and the split.  `columns` (optional): factors of the columns.
+// kept in registers between the search for its largest value and the split.  `columns` (optional): factors of the columns,
+// `inverse`: powers of two whose inverses are.
 template <int LD>
 __device__ __forceinline__ void split_rows16(const float* __restrict__ src, const float* __restrict__ src2, int64_t ld_src,
                                              int64_t rows, int cols, __half* hi, __half* lo, float* scale,
-                                             const float* __restrict__ columns, int64_t cta, int64_t ctas) {
+                                             const float* __restrict__ columns, bool inverse, int64_t cta, int64_t ctas) {
   constexpr int kParts = LD / 128;
   const int lane = threadIdx.x & 31;
   float4 f[kParts];
 #pragma unroll
-  for (int i = 0; i < kParts; ++i)
+  for (int i = 0; i < kParts; ++i) {
     f[i] = columns ? *reinterpret_cast<const float4*>(columns + i * 128 + lane * 4) : make_float4(1.f, 1.f, 1.f, 1.f);
+    if (inverse) f[i] = make_float4(__frcp_rn(f[i].x), __frcp_rn(f[i].y), __frcp_rn(f[i].z), __frcp_rn(f[i].w));
+  }
   for (int64_t r = cta * 8 + (threadIdx.x >> 5); r < rows; r += ctas * 8) {
     float4 x[kParts], y[kParts];
 #pragma unroll
@@ -176,11 +181,12 @@ __device__ __forceinline__ void split_rows16(const float* __restrict__ src, cons
 }
 // Columns 32 `cta` .. + 31 of src [rows][cols] -> operand rows of those numbers, by a CTA of 256 threads with
 // split_columns16_smem(LD) bytes of shared memory.  Entries whose column is above `diagonal` + their row count as zero.
-// `pivots`: row p is taken times pivot_power of the pivot `rows` columns before src[p, p].
+// `pivots`: row p is taken times pivot_power, or its inverse, of the pivot `rows` columns before src[p, p].
+enum Pivots { kNoPivots = 0, kPowers = 1, kInverses = 2 };
 constexpr size_t split_columns16_smem(int ld) { return 32 * (ld + 2) * sizeof(float); }
 template <int LD>
 __device__ __forceinline__ void split_columns16(const float* __restrict__ src, int64_t ld_src, int rows, int64_t cols,
-                                                int64_t diagonal, __half* hi, __half* lo, float* scale, bool pivots,
+                                                int64_t diagonal, __half* hi, __half* lo, float* scale, int pivots,
                                                 int64_t cta, float* stage) {   // stage [32][LD + 2]
   __shared__ float s_max[8][32];
   __shared__ float s_power[LD];
@@ -193,7 +199,7 @@ __device__ __forceinline__ void split_columns16(const float* __restrict__ src, i
   if (pivots) {
     for (int p = threadIdx.x; p < LD; p += 256) {
       const float reciprocal = p < rows ? __frcp_rn(src[(int64_t)p * ld_src + p - rows]) : 1.0f;
-      s_power[p] = pivot_power(reciprocal);
+      s_power[p] = pivots == kInverses ? pivot_inverse(reciprocal) : pivot_power(reciprocal);
     }
     __syncthreads();
   }
@@ -229,9 +235,9 @@ __device__ __forceinline__ void split_columns16(const float* __restrict__ src, i
   }
 }
 // src [rows][ld_src] -> operand; `batch` problems src_batch, dst_rows apart, problem b with the column factors (ld of them)
-// at columns + columns_batch * index[b] (null: b)
+// (or the inverses of these) at columns + columns_batch * index[b] (null: b)
 int split_rows16(const float* src, int64_t ld_src, int64_t src_batch, int64_t rows, int cols, __half* hi, __half* lo, float* scale,
-                 int ld, int64_t dst_rows, int batch, const float* columns, int64_t columns_batch, const int32_t* index,
+                 int ld, int64_t dst_rows, int batch, const float* columns, bool inverse, int64_t columns_batch, const int32_t* index,
                  cudaStream_t st);
 // The operand of an update of the factor: rows [0, end) are the columns of the block row `row` [n][end] (its last n columns
 // lower triangular), rows [end, end + first) f_hi + f_lo, then `rows` rows of p.

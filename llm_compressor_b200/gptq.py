@@ -115,6 +115,7 @@ class HessianFactor:
     U: Optional[torch.Tensor]
     ok: Optional[bool]
     status: Optional[torch.Tensor] = None
+    blocked: bool = False   # U holds the blocked form (``ops.gptq_factor_async``)
 
     def resolve(self) -> "HessianFactor":
         if self.ok is None:
@@ -135,9 +136,19 @@ def factor_hessian(hessian: torch.Tensor, percdamp: float = 0.01, actorder=None,
                    defer: bool = False) -> HessianFactor:
     """Permute (act-order), patch dead columns, dampen and factor ``hessian`` (consumed).
     ``defer``: do not wait for the factorisation's status (see ``HessianFactor.resolve``)."""
-    H, perm, diag = _factor_prologue(hessian, percdamp, actorder)
-    factor = HessianFactor(H.shape[0], perm, diag, H, None, ops.gptq_factor_async(H))
+    factor = _factor_for(hessian, percdamp, actorder, False)
     return factor if defer else factor.resolve()
+
+
+def _factor_for(hessian, percdamp, actorder, blocks: bool) -> HessianFactor:
+    H, perm, diag = _factor_prologue(hessian, percdamp, actorder)
+    return HessianFactor(H.shape[0], perm, diag, H, None, ops.gptq_factor_async(H, blocks), blocks)
+
+
+def factor_for_modules(hessian, modules, percdamp: float = 0.01, actorder=None) -> HessianFactor:
+    """A deferred ``factor_hessian`` in the form that the sweeps of ``modules``, one at a time, take in least time: blocked
+    where every one of them can."""
+    return _factor_for(hessian, percdamp, actorder, all(ops.gptq_sweep_takes_blocks(*_weight_of(m).shape) for m in modules))
 
 
 def _factor_prologue(hessian: torch.Tensor, percdamp: float, actorder):
@@ -190,6 +201,7 @@ class _SweepInput:
     col_group: Optional[torch.Tensor]
     g_idx: Optional[torch.Tensor]
     final_dtype: torch.dtype
+    original: Optional[torch.Tensor] = None   # of W, where the factor is blocked
 
 
 def _sweep_input(module, quant_args, hessian, percdamp, factor, W=None, qparams=None, order=None) -> _SweepInput:
@@ -212,14 +224,16 @@ def _sweep_input(module, quant_args, hessian, percdamp, factor, W=None, qparams=
     if factor is None:
         if hessian is None or hessian.shape != (K, K):
             raise ValueError("hessian must be float32 [in_features, in_features]")
-        factor = factor_hessian(hessian, percdamp, actorder, defer=True)
+        factor = factor_for_modules(hessian, [module], percdamp, actorder)
     elif factor.K != K or (factor.perm is not None) != bool(actorder):
         raise ValueError("factor does not match this module / act-order setting")
     perm = factor.perm
 
     prepared = W is not None
-    if not prepared:
-        W = ops.gather_columns_f32(weight, perm)
+    original = None
+    if not prepared:   # (act-order "group" observes the weight with its dead columns)
+        W, original = ops.gather_columns_keep(weight, perm, factor.diag, actorder != "group",
+                                              factor.blocked and factor.U is not None)
 
     global_scale = None
     if qparams is None and actorder != "group":
@@ -241,9 +255,9 @@ def _sweep_input(module, quant_args, hessian, percdamp, factor, W=None, qparams=
         g_idx = order if order is not None else _column_groups(args, K, perm if actorder == "weight" else None, W.device)
     col_group = g_idx if actorder == "weight" else None
 
-    if not prepared:
+    if not prepared and actorder == "group":
         ops.gptq_zero_dead_columns(factor.diag, W)
-    return _SweepInput(args, actorder, factor, W, qparams[0], qparams[1], global_scale, col_group, g_idx, weight.dtype)
+    return _SweepInput(args, actorder, factor, W, qparams[0], qparams[1], global_scale, col_group, g_idx, weight.dtype, original)
 
 
 def _column_groups(args, K: int, perm, device) -> torch.Tensor:
@@ -294,7 +308,8 @@ def quantize_weight(module, quant_args, hessian: Optional[torch.Tensor], blocksi
     # (a symmetric scheme's zero points are all zero: the sweep does without them)
     zero_point = None if inp.args.symmetric else inp.zero_point
     losses, status = ops.gptq_sweep(inp.W, inp.factor.U, inp.scale, zero_point, inp.args, blocksize=blocksize,
-                                    col_group=inp.col_group, global_scale=inp.global_scale, return_status=True)
+                                    col_group=inp.col_group, global_scale=inp.global_scale, return_status=True,
+                                    original=inp.original)
     out = _sweep_output(inp)
     if defer:
         loss = losses.sum()
@@ -308,9 +323,7 @@ def quantize_weight(module, quant_args, hessian: Optional[torch.Tensor], blocksi
     if waiting:
         inp.factor.settle(words[2:])
         if not inp.factor.ok:   # round to nearest with the parameters that are there already
-            W = ops.gather_columns_f32(_weight_of(module), inp.factor.perm)
-            ops.gptq_zero_dead_columns(inp.factor.diag, W)
-            inp.W = W
+            W = inp.W = ops.gather_columns_keep(_weight_of(module), inp.factor.perm, inp.factor.diag, True, False)[0]
             losses, status = ops.gptq_sweep(W, None, inp.scale, zero_point, inp.args, blocksize=blocksize,
                                             col_group=inp.col_group, global_scale=inp.global_scale, return_status=True)
             out = _sweep_output(inp)

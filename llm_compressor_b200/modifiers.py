@@ -848,7 +848,7 @@ class GPTQModifier(QuantizationMixin):
         t0 = time.perf_counter()
         self._trace("job_start", module_list[0])
         taken, hess_status = self._queue_factors(
-            module_list, lambda H, actorder: gptq.factor_hessian(H, self.dampening_frac, actorder, defer=True))
+            module_list, lambda H, actorder: gptq.factor_for_modules(H, module_list, self.dampening_frac, actorder))
         queued = []
         for module, qargs, factor in taken:
             with torch.no_grad():

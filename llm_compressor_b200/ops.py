@@ -435,6 +435,20 @@ def gather_columns_f32(w: torch.Tensor, perm=None) -> torch.Tensor:
     return out
 
 
+def gather_columns_keep(w: torch.Tensor, perm, diag: torch.Tensor, zero: bool, keep: bool):
+    """``gather_columns_f32``, with ``zero`` as ``gptq_zero_dead_columns(diag, ...)`` leaves it; and, with ``keep``, the columns
+    in the weight's own dtype too, dead ones zeroed in any case (``original`` of ``gptq_sweep``), else None."""
+    _need_cuda(w, perm, diag)
+    assert diag.dtype == torch.float32 and diag.is_contiguous()
+    N, K, ld = _2d(w)
+    out = torch.empty((N, K), dtype=torch.float32, device=w.device)
+    kept = torch.empty((N, (K + 7) // 8 * 8), dtype=w.dtype, device=w.device)[:, :K] if keep else None
+    check(_lib.load().b200q_gather_columns_keep(ptr(w), _dt(w), N, K, ld, ptr(perm), ptr(diag), int(zero), ptr(out),
+                                                out.stride(0), ptr(kept), kept.stride(0) if keep else 0, stream_ptr()),
+          "b200q_gather_columns_keep")
+    return out, kept
+
+
 def permute_hessian(H: torch.Tensor, perm: torch.Tensor) -> torch.Tensor:
     _need_cuda(H, perm)
     K = H.shape[0]
@@ -470,17 +484,23 @@ def gptq_zero_dead_columns(diag: torch.Tensor, wf: torch.Tensor):
           "b200q_gptq_zero_dead_columns")
 
 
-def gptq_factor_async(H: torch.Tensor) -> torch.Tensor:
+def gptq_sweep_takes_blocks(N: int, K: int) -> bool:
+    """Whether ``gptq_sweep`` of an [N, K] weight can take the blocked form of its factor."""
+    return bool(_lib.load().b200q_gptq_sweep_takes_blocks(N, K))
+
+
+def gptq_factor_async(H: torch.Tensor, blocks: bool = False) -> torch.Tensor:
     """In place H -> U (upper, U^T U = H^-1) without waiting for the result.  Returns the device
-    status words for ``gptq_factor_status``; U is meaningless when the status is not 0."""
+    status words for ``gptq_factor_status``; U is meaningless when the status is not 0.
+    ``blocks``: the blocked form instead, for ``gptq_sweep(..., original=...)``."""
     _need_cuda(H)
     lib = _lib.load()
     K = H.shape[0]
     ws = torch.empty(max(lib.b200q_gptq_factor_workspace_bytes(K), 4), dtype=torch.uint8,
                      device=H.device)
     status = torch.zeros(4, dtype=torch.int32, device=H.device)
-    check(lib.b200q_gptq_factor(ptr(H), K, H.stride(0), ptr(ws), ptr(status), stream_ptr()),
-          "b200q_gptq_factor")
+    call = lib.b200q_gptq_factor_blocks if blocks else lib.b200q_gptq_factor
+    check(call(ptr(H), K, H.stride(0), ptr(ws), ptr(status), stream_ptr()), "b200q_gptq_factor")
     return status
 
 
@@ -498,8 +518,9 @@ def gptq_factor(H: torch.Tensor) -> int:
 
 
 def gptq_sweep(wf, U, scale, zp, args: QuantizationArgs, blocksize=128, col_group=None,
-               global_scale=None, return_status: bool = False):
-    """Runs the column sweep in place on wf; returns per-row losses, and with ``return_status``
+               global_scale=None, return_status: bool = False, original=None):
+    """Runs the column sweep in place on wf (with ``original``, the weights as they are, in rows of 16-byte pieces: U is the
+    blocked form); returns per-row losses, and with ``return_status``
     also the call's device status word (int32 [1]; non-zero: a bounded wait inside a
     trailing-update GEMM ran out and wf is incomplete)."""
     _need_cuda(wf, U, scale, zp, col_group, global_scale)
@@ -514,10 +535,16 @@ def gptq_sweep(wf, U, scale, zp, args: QuantizationArgs, blocksize=128, col_grou
     losses = torch.empty(N, dtype=torch.float32, device=wf.device)
     ws = torch.empty(max(lib.b200q_gptq_sweep_workspace_bytes(N, K, blocksize), 4) + 16,
                      dtype=torch.uint8, device=wf.device)
-    check(lib.b200q_gptq_sweep(ptr(wf), N, K, ld, ptr(U), 0 if U is None else U.stride(0),
-                               ptr(scale), _dt(scale), ptr(zp), ptr(col_group), ptr(global_scale),
-                               args.c_struct(), int(blocksize), ptr(losses), ptr(ws), stream_ptr()),
-          "b200q_gptq_sweep")
+    operands = (ptr(U), 0 if U is None else U.stride(0), ptr(scale), _dt(scale), ptr(zp), ptr(col_group),
+                ptr(global_scale), args.c_struct(), int(blocksize), ptr(losses), ptr(ws), stream_ptr())
+    if original is None:
+        check(lib.b200q_gptq_sweep(ptr(wf), N, K, ld, *operands), "b200q_gptq_sweep")
+    else:
+        _need_cuda(original)
+        if original.shape != wf.shape or original.stride(1) != 1:
+            raise ValueError("original must have the weight's shape and contiguous rows")
+        check(lib.b200q_gptq_sweep_blocks(ptr(wf), N, K, ld, ptr(original), _dt(original), original.stride(0), *operands),
+              "b200q_gptq_sweep_blocks")
     if return_status:
         return losses, ws[:4].view(torch.int32)
     return losses
