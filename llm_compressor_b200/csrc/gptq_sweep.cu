@@ -36,6 +36,7 @@ constexpr int kTileBytes = kBlockCols * kRowBytes;   // a block's columns of U f
 constexpr int kLag = 3;                      // errors of micro-block m reach columns from m + kLag on by MMAs
 constexpr int kBandCols = kLag * kMicro;     // columns of U that chain and feeder need of a micro-block's rows (8 rows at
                                              // most reach 5 half-blocks on)
+constexpr int kGoAhead = 8;                  // half-blocks before the end at which the next kernel may be set up
 constexpr int kErrSlots = 4;                 // micro-blocks whose errors are kept
 constexpr int kBandFloats = kMicro * kBandCols + kMicro;   // and the reciprocals of the pivots
 
@@ -464,6 +465,10 @@ sweep_block_kernel(const __grid_constant__ Params p) {
     for (int k = 0; k < kHalf / 2; ++k) x[k] = pair(sW[2 * k * S::kWld + r], sW[(2 * k + 1) * S::kWld + r]);
 #pragma unroll 1
     for (int n = 0; n < 2 * micros; ++n) {
+      // the next kernel's CTAs wait on the SMs that are free, where the helper stream makes the next slice of U meanwhile: not
+      // before the end is near (from the start on, where warps without a role said so, they kept that slice, which the product
+      // waits for, off the SMs until the sweep was over: 4096 x 4096 806 us, now 757; 4096 x 14336 4670, 4376)
+      if (n == 2 * micros - kGoAhead) chain_go();
       const int slot = (n >> 1) & (kSlots - 1), t0 = (n & 1) * kHalf;
       float* wcol = sW + n * kHalf * S::kWld + r;
       float* eo = sE + (((n >> 1) & (kErrSlots - 1)) * kMicro + t0) * ROWS + r;
@@ -859,7 +864,6 @@ sweep_block_kernel(const __grid_constant__ Params p) {
     else if (warp >= S::kOut && warp < S::kParams) out_role();
     else if (warp == S::kParams) param_role();
   }
-  chain_go();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (s_abort) {
