@@ -128,40 +128,96 @@ __device__ __forceinline__ void mma_block(const float* A, int lda, const float* 
 // 16-column step exactly eight 16-row blocks take part.  A step:
 //   warp 0 brings the 16 x 16 diagonal block up to date and factors it in registers, a lane per row: the next pivot
 //          is formed by its own lane and broadcast before the other columns are updated, no branches.  Meanwhile the
-//          other seven warps apply the step before to everything else.
+//          others apply the step before to everything else.
 //   four warps substitute the 128 active rows, a row a lane
+//
+// Sixteen warps.  The elimination and what follows it in the same step are the chain; the update of the step before has to
+// be through in that time, and warps on the eliminating warp's scheduler slow it down, so the twelve on the other three
+// take it.  Cycles, clocks read in the kernel: 2700 until the block is there, steps of 2600 to 3300 (the diagonal block's
+// update 360, its elimination 1300 to 2100, the more the longer the others are at their tiles: shuffles and shared-memory
+// loads share a pipe; substitution and operands 800), 1900 out; 29500 in all, 32200 with eight warps and tf32 pairs.
 constexpr int W16 = 16;
-constexpr int kCholSmemFloats = 2 * NB * LD + W16 * 20 + W16;
+constexpr int kCholThreads = 512;
+// A step's 128 active rows as operands: 16 hi and 16 lo halves and a power of two per row (tgemm::Operand), in rows of 80 bytes,
+// which ldmatrix reads without bank conflicts.  The rows are written once and read by up to ten products: split by every
+// reader into tf32 pairs, the update of a step took 3300 cycles, longer than the chain beside it.
+constexpr int kOpBytes = 80;
+constexpr int kCholSmemFloats = 2 * NB * LD + W16 * 20 + W16 + NB * kOpBytes / 4 + NB;
+
+__device__ __forceinline__ void ldmatrix4(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// o[16 x 8 NT] -= A B^T over 16 terms, A the operand rows from ra on, B those from rb on; column tiles from `tiles` on are left
+// out.  Lane (g, t) has rows g, g + 8 and columns 2 t, 2 t + 1 of every tile; o points at its first.
+template <int NT>
+__device__ __forceinline__ void subtract_product(float* o, uint32_t op, const float* scale, int ra, int rb, int tiles, int lane) {
+  float2 old[NT][2];   // (all of them before the products: loads cannot pass the stores below)
+#pragma unroll
+  for (int j = 0; j < NT; ++j)
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (j < tiles) old[j][h] = *reinterpret_cast<float2*>(o + h * 8 * LD + 8 * j);
+  uint32_t ah[4], al[4], bh[NT / 2][4], bl[NT / 2][4];
+  const uint32_t a = op + (ra + (lane & 15)) * kOpBytes + (lane >> 4) * 16;
+  const uint32_t b = op + (rb + (lane & 7) + (lane >> 4) * 8) * kOpBytes + ((lane >> 3) & 1) * 16;
+  ldmatrix4(a, ah);
+  ldmatrix4(a + 32, al);
+#pragma unroll
+  for (int j = 0; j < NT / 2; ++j) {
+    if (2 * j >= tiles) break;
+    ldmatrix4(b + j * 16 * kOpBytes, bh[j]);
+    ldmatrix4(b + j * 16 * kOpBytes + 32, bl[j]);
+  }
+  const float s0 = scale[ra + (lane >> 2)], s1 = scale[ra + (lane >> 2) + 8];
+#pragma unroll
+  for (int j = 0; j < NT; ++j) {
+    if (j >= tiles) break;
+    float x[4] = {0.f, 0.f, 0.f, 0.f}, y[4] = {0.f, 0.f, 0.f, 0.f};
+    const int e = 2 * (j & 1);
+    mma_f16(y, ah, bl[j / 2][e], bl[j / 2][e + 1]);
+    mma_f16(x, ah, bh[j / 2][e], bh[j / 2][e + 1]);
+    mma_f16(y, al, bh[j / 2][e], bh[j / 2][e + 1]);
+    const float2 sc = *reinterpret_cast<const float2*>(scale + rb + 8 * j + 2 * (lane & 3));
+    *reinterpret_cast<float2*>(o + 8 * j) = make_float2(fmaf(-(x[0] + y[0]) * s0, sc.x, old[j][0].x), fmaf(-(x[1] + y[1]) * s0, sc.y, old[j][0].y));
+    *reinterpret_cast<float2*>(o + 8 * LD + 8 * j) = make_float2(fmaf(-(x[2] + y[2]) * s1, sc.x, old[j][1].x), fmaf(-(x[3] + y[3]) * s1, sc.y, old[j][1].y));
+  }
+}
 
 // active row block s (0..7) of step kb: identity rows up to kb, whose inverse is being born, matrix rows after it
 __device__ __forceinline__ float* active_row(float* R, int ar, int kb) {
   return R + ((ar >> 4) <= kb ? NB + ar : ar) * LD;
 }
 
-__global__ void __launch_bounds__(kThreads, 1) chol_diag_kernel(Mat mt, int k0, int n) {
-  chain_wait();
+__global__ void __launch_bounds__(kCholThreads, 1) chol_diag_kernel(Mat mt, int k0, int n) {
   extern __shared__ __align__(16) float sm[];
   float* R = sm;                    // rows 0..127: the block, then L; rows 128..255: the identity, then L^-T
   float* Lt = R + 2 * NB * LD;      // [16][20] transposed diagonal block of the step
   float* rinv = Lt + W16 * 20;      // [16]
+  float* scale = rinv + W16;        // [128] inverse powers of the operand rows
+  unsigned char* rows_op = reinterpret_cast<unsigned char*>(scale + NB);
+  const uint32_t op = (uint32_t)__cvta_generic_to_shared(rows_op);
   float* A = mt.A + blockIdx.x * mt.batch + (int64_t)k0 * mt.lda + k0;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-#pragma unroll 16
-  for (int idx = tid; idx < NB * NB / 4; idx += kThreads) {
+  // (nothing reads what is above the diagonal of a matrix row or left of an identity row's block)
+  for (int idx = tid; idx < NB * NB / 4; idx += kCholThreads) {
     const int r = idx >> 5, c = (idx & 31) << 2;
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    float* e = &v.x;
-    if (r < n && c <= r) v = *reinterpret_cast<const float4*>(A + (int64_t)r * mt.lda + c);   // (rows are padded to 32)
-    float4 id = make_float4(0.f, 0.f, 0.f, 0.f);
-    float* d = &id.x;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (c + k > r) e[k] = 0.0f;
-      if (c + k == r) { d[k] = 1.0f; if (r >= n) e[k] = 1.0f; }   // identity padding beyond n
-    }
-    *reinterpret_cast<float4*>(R + r * LD + c) = v;
-    *reinterpret_cast<float4*>(R + (NB + r) * LD + c) = id;
+    const float4 id = make_float4(c == r ? 1.f : 0.f, c + 1 == r ? 1.f : 0.f, c + 2 == r ? 1.f : 0.f, c + 3 == r ? 1.f : 0.f);
+    if (c <= r && r >= n) *reinterpret_cast<float4*>(R + r * LD + c) = id;   // identity padding beyond n
+    if (c >= (r & ~(W16 - 1))) *reinterpret_cast<float4*>(R + (NB + r) * LD + c) = id;
   }
+  chain_wait();
+#pragma unroll
+  for (int i = 0; i < NB * NB / 4 / kCholThreads; ++i) {
+    const int idx = tid + i * kCholThreads, r = idx >> 5, c = (idx & 31) << 2;
+    if (c <= r && r < n) cp_async16(R + r * LD + c, A + (int64_t)r * mt.lda + c, 16);   // (rows are padded to 32)
+  }
+  cp_async_wait_all();
   __syncthreads();
   int bad = 0;   // first pivot that is not positive, + 1
 #pragma unroll 1
@@ -169,20 +225,7 @@ __global__ void __launch_bounds__(kThreads, 1) chol_diag_kernel(Mat mt, int k0, 
     const int c0 = kb * W16, p0 = c0 - W16;
     if (warp == 0) {
       if (kb > 0) {   // the diagonal block takes the step before
-        float acc[2][4];
-        float* o = R + (c0 + (lane >> 2)) * LD + c0 + 2 * (lane & 3);
-        float2 old[2][2];
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-          for (int h = 0; h < 2; ++h) old[j][h] = *reinterpret_cast<float2*>(o + h * 8 * LD + 8 * j);
-        mma_block<2, 2>(R + c0 * LD + p0, LD, R + c0 * LD + p0, LD, 1, W16, lane, acc);
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-          for (int h = 0; h < 2; ++h)
-            *reinterpret_cast<float2*>(o + h * 8 * LD + 8 * j) =
-                make_float2(old[j][h].x - acc[j][2 * h], old[j][h].y - acc[j][2 * h + 1]);
+        subtract_product<2>(R + (c0 + (lane >> 2)) * LD + c0 + 2 * (lane & 3), op, scale, c0, c0, 2, lane);
         __syncwarp();
       }
       float a[W16], ri;
@@ -231,7 +274,7 @@ __global__ void __launch_bounds__(kThreads, 1) chol_diag_kernel(Mat mt, int k0, 
         for (int j = 0; j < W16; ++j) Lt[j * 20 + lane] = (j <= lane) ? a[j] : 0.0f;
         rinv[lane] = ri;
       }
-    } else if (kb > 0) {
+    } else if (kb > 0 && (warp & 3)) {
       // everything else takes the step before: the eight row blocks that were active then x the columns from c0 on,
       // on and below the diagonal.  A warp takes 16 rows x 32 columns at a time.
       // Task list: kb identity row blocks with `wide` pairs of column blocks each, then matrix row blocks r = 0, 1, ...
@@ -239,7 +282,7 @@ __global__ void __launch_bounds__(kThreads, 1) chol_diag_kernel(Mat mt, int k0, 
       // warps' costs 180 cycles a skip, mostly instruction fetch.)
       const int wide = (9 - kb) / 2, left = kb * wide, half = (8 - kb) / 2;
       const int all = left + half * (half + 1) + (kb & 1) * (half + 1);
-      for (int t = warp - 1; t < all; t += 7) {
+      for (int t = (warp >> 2) * 3 + (warp & 3) - 1; t < all; t += 12) {
         int s, g;
         if (t < left) {
           s = t / wide; g = t - s * wide;
@@ -248,35 +291,19 @@ __global__ void __launch_bounds__(kThreads, 1) chol_diag_kernel(Mat mt, int k0, 
           g = u - q * (q + 1); s = kb + 2 * q;
           if (g > q) { g -= q + 1; ++s; }
         }
-        {
-          const bool matrix = s >= kb;
-          float* rows = R + ((matrix ? 0 : NB) + s * W16) * LD;
-          const int cc = c0 + g * 32;
-          float acc[4][4];
-          float* o = rows + (lane >> 2) * LD + cc + 2 * (lane & 3);
-          float2 old[4][2];   // (all of them before the products: loads cannot pass the stores below)
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-              if (cc + 8 * j < NB) old[j][h] = *reinterpret_cast<float2*>(o + h * 8 * LD + 8 * j);
-          mma_block<4, 2>(rows + p0, LD, R + cc * LD + p0, LD, 1, W16, lane, acc);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int cb = (cc >> 4) + (j >> 1);
-            if (cb >= 8 || (matrix && (cb > s || (s == kb && cb == kb)))) continue;   // outside, above, warp 0's
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-              *reinterpret_cast<float2*>(o + h * 8 * LD + 8 * j) =
-                  make_float2(old[j][h].x - acc[j][2 * h], old[j][h].y - acc[j][2 * h + 1]);
-          }
-        }
+        const bool matrix = s >= kb;
+        const int cc = c0 + g * 32, last = matrix ? s * W16 : NB - W16;   // first column of the last block of 16 to take
+        // (the diagonal block itself is the first warp's)
+        const int tiles = matrix && s == kb ? 0 : min(4, (last + W16 - cc) / 8);
+        subtract_product<4>(R + ((matrix ? 0 : NB) + s * W16 + (lane >> 2)) * LD + cc + 2 * (lane & 3), op, scale, s * W16, cc,
+                            tiles, lane);
       }
     }
     __syncthreads();
     if (warp < 4) {
       float a[W16];
-      float* row = active_row(R, warp * 32 + lane, kb) + c0;
+      const int ar = warp * 32 + lane;
+      float* row = active_row(R, ar, kb) + c0;
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const float4 v = *reinterpret_cast<const float4*>(row + 4 * q);
@@ -295,9 +322,22 @@ __global__ void __launch_bounds__(kThreads, 1) chol_diag_kernel(Mat mt, int k0, 
             if (4 * q + k > j) a[4 * q + k] = fmaf(-y, l[k], a[4 * q + k]);
         }
       }
+      float largest[4] = {0.f, 0.f, 0.f, 0.f}, to, back;
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
-        *reinterpret_cast<float4*>(row + 4 * q) = make_float4(a[4 * q], a[4 * q + 1], a[4 * q + 2], a[4 * q + 3]);
+      for (int j = 0; j < W16; ++j) largest[j & 3] = fmaxf(largest[j & 3], fabsf(a[j]));
+      tgemm::row_scale(fmaxf(fmaxf(largest[0], largest[1]), fmaxf(largest[2], largest[3])), to, back);
+      scale[ar] = back;
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        uint32_t hi[4], lo[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) tgemm::split_pair(a[8 * q + 2 * k] * to, a[8 * q + 2 * k + 1] * to, hi[k], lo[k]);
+        *reinterpret_cast<uint4*>(rows_op + ar * kOpBytes + q * 16) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        *reinterpret_cast<uint4*>(rows_op + ar * kOpBytes + 32 + q * 16) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q)   // (of the matrix rows nothing reads these any more)
+        if ((ar >> 4) <= kb) *reinterpret_cast<float4*>(row + 4 * q) = make_float4(a[4 * q], a[4 * q + 1], a[4 * q + 2], a[4 * q + 3]);
     }
     __syncthreads();
   }
@@ -306,10 +346,12 @@ __global__ void __launch_bounds__(kThreads, 1) chol_diag_kernel(Mat mt, int k0, 
     int* status = mt.status + 4 * blockIdx.x;
     if (atomicCAS(status, 0, B200Q_NOT_POSITIVE_DEFINITE) == 0) status[1] = k0 + bad - mt.pad;
   }
-  // D[j][i] = (L^-T)[i][j], zero above the diagonal; a thread turns 4 x 4 entries round
+  // D[j][i] = (L^-T)[i][j] in the 16 x 16 blocks on and below the diagonal, zero above it (whoever reads beyond these blocks
+  // takes zeros by himself); a thread turns 4 x 4 entries round
 #pragma unroll
-  for (int it = 0; it < NB * NB / 16 / kThreads; ++it) {
-    const int u = it * 8 + warp, i = (lane & 1) * 4 + (u & 15) * 8, j = (lane >> 1) * 4 + (u >> 4) * 64;
+  for (int it = 0; it < NB * NB / 16 / kCholThreads; ++it) {
+    const int u = it * 16 + warp, i = (lane & 1) * 4 + (u & 15) * 8, j = (lane >> 1) * 4 + (u >> 4) * 64;
+    if (i / W16 > j / W16) continue;
     float v[4][4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -437,7 +479,8 @@ __global__ void __launch_bounds__(kThreads) square_update_kernel(Mat mt, const f
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int idx = tid + q * kThreads, m = idx >> 3, c = (idx & 7) << 2;
-      cp_async16(Qs + m * 40 + c, src + (int64_t)m * ld + c, 16);
+      const bool zero = own && c0 - b0 + c > m;   // above D's diagonal
+      cp_async16(Qs + m * 40 + c, zero ? A : src + (int64_t)m * ld + c, zero ? 0 : 16);
     }
   }
   const int warp = tid >> 5, lane = tid & 31, tr = (warp & 1) * 16, tc = (warp >> 1) * 8;
@@ -597,7 +640,7 @@ static int factor(float* H, float* const* Hs, int batch, int64_t order, int64_t 
     const bool last = K1 >= K;
     for (int k = 0; k < inner; ++k) {
       const int bn = n - k * NB < NB ? n - k * NB : NB, below = n - k * NB - bn;
-      B200Q_TRY(launch_chained(chol_diag_kernel, dim3(batch), kThreads, chol_smem, st, mt, (int)K0 + k * NB, bn));
+      B200Q_TRY(launch_chained(chol_diag_kernel, dim3(batch), kCholThreads, chol_smem, st, mt, (int)K0 + k * NB, bn));
       B200Q_LAUNCH_CHECK();
       const int units = (below + kVec - 1) / kVec + k * NB / kVec;
       if (units == 0) continue;
