@@ -191,6 +191,10 @@ int b200q_quantize_pack(const void* W, int wdtype, int64_t N, int64_t K, int64_t
  * everything else returns B200Q_ERR_UNSUPPORTED.  col_scale: float [K]; out: bf16 [N, K]. */
 int b200q_scaled_fake_quantize(const void* W, int wdtype, int64_t N, int64_t K, int64_t ldw, const float* col_scale,
                                const b200q_qargs* qa, void* out, void* stream);
+/* The same for `count` weights of one width behind the same column scales (host arrays of pointers, rows and strides). */
+int b200q_scaled_fake_quantize_many(const void* const* W, int wdtype, int count, const int64_t* N, int64_t K,
+                                    const int64_t* ldw, const float* col_scale, const b200q_qargs* qa,
+                                    void* const* out, void* stream);
 
 /* Asymmetric zero points packed along dim 0 (pack_to_int32(zp, bits, packed_dim=0),
  * CT/compressors/pack_quantized/base.py:70-73): zp int8 [N,G] -> int32 [ceil(N*bits/32), G]. */

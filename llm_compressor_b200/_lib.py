@@ -66,6 +66,7 @@ SIGNATURES = {
     "b200q_observe_mse_noalloc": (_i, [_p, _i, _i64, _i64, _i64, _qa, _d, _i, _d, _f, _f, _p, _p, _p]),
     "b200q_fake_quantize": (_i, [_p, _i, _i64, _i64, _i64, _p, _i, _p, _p, _p, _qa, _p, _i64, _p]),
     "b200q_quantize_pack": (_i, [_p, _i, _i64, _i64, _i64, _p, _i, _p, _p, _p, _qa, _i, _p, _p]),
+    "b200q_scaled_fake_quantize_many": (_i, [_p, _i, _i, _p, _i64, _p, _p, _qa, _p, _p]),
     "b200q_scaled_fake_quantize": (_i, [_p, _i, _i64, _i64, _i64, _p, _qa, _p, _p]),
     "b200q_pack_zero_points": (_i, [_p, _i64, _i64, _i, _p, _p]),
     "b200q_compress_scale": (_i, [_p, _i, _i64, _i, _p, _p]),

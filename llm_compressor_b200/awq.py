@@ -167,9 +167,13 @@ def scaled_fake_quantize(weights, scales: torch.Tensor, layers, parent=None) -> 
     fake-quantised, divided by s in float32 and rounded again (base.py:647-709).  Under
     TENSOR_GROUP the q/k/v or gate/up siblings inside ``parent`` share their global scale, as
     ``fuse_weight_observers(parent)`` arranges in the reference."""
-    # schemes whose parameters come from the weight alone: one kernel per layer
+    # schemes whose parameters come from the weight alone: one kernel for all layers, or each
     schemes = [layer.quantization_scheme.weights for layer in layers]
     if all(a.strategy != "tensor_group" for a in schemes):
+        if len(weights) > 1 and all(a == schemes[0] for a in schemes) and len({w.device for w in weights}) == 1:
+            done = ops.scaled_fake_quantize_many(weights, scales, schemes[0])
+            if done is not None:
+                return done
         done = [ops.scaled_fake_quantize(w, scales, a) for w, a in zip(weights, schemes)]
         if all(d is not None for d in done):
             return done

@@ -247,6 +247,26 @@ def scaled_fake_quantize(w, col_scale: torch.Tensor, args: QuantizationArgs):
     return out
 
 
+def scaled_fake_quantize_many(ws, col_scale: torch.Tensor, args: QuantizationArgs):
+    """``scaled_fake_quantize`` of weights of one width in one launch (of at most eight of them), or None."""
+    _need_cuda(*ws, col_scale)
+    if any(w.dtype != torch.bfloat16 for w in ws) or col_scale.dtype != torch.float32 or not col_scale.is_contiguous():
+        return None
+    shapes = [_2d(w) for w in ws]
+    K, count = shapes[0][1], len(ws)
+    if any(s[1] != K for s in shapes):
+        return None
+    outs = [torch.empty((N, K), dtype=torch.bfloat16, device=w.device) for w, (N, _, _) in zip(ws, shapes)]
+    longs = ctypes.c_int64 * count
+    rc = _lib.load().b200q_scaled_fake_quantize_many(
+        longs(*[w.data_ptr() for w in ws]), _dt(ws[0]), count, longs(*[s[0] for s in shapes]), K,
+        longs(*[s[2] for s in shapes]), ptr(col_scale), args.c_struct(), longs(*[o.data_ptr() for o in outs]), stream_ptr())
+    if rc == -2:
+        return None
+    check(rc, "b200q_scaled_fake_quantize_many")
+    return outs
+
+
 def quantize_pack(w, scale, zp, args: QuantizationArgs, g_idx=None, global_scale=None,
                   pack_int8=False):
     """Storage codes: int32 words (int4, or int8 with pack_int8), int8 / float8 bytes, or

@@ -236,6 +236,19 @@ def test_scale_search_step_equals_the_element_wise_chain(kw, N, K):
     assert bits_equal(got, ref), mismatch(got, ref)
 
 
+# more weights than a launch takes, of different heights and strides, one and two chunks a lane, a part of a warp's columns
+@pytest.mark.parametrize("g,K", [(8, 264), (16, 48), (128, 1152), (256, 512)])
+def test_scale_search_step_of_many_weights(g, K):
+    args = QuantizationArgs(num_bits=4, type="int", symmetric=False, strategy="group", group_size=g)
+    ws = [synth_weight(200, K + 8 * (n % 2), seed=n).to(DEV)[-n:, :K] for n in (1, 33, 8, 200, 7, 64, 3, 9, 17)]
+    s = torch.exp(0.5 * torch.randn(K, generator=torch.Generator(device=DEV).manual_seed(1), device=DEV))
+    got = ops.scaled_fake_quantize_many(ws, s, args)
+    for w, out in zip(ws, got):
+        scaled = (w * s.view(1, -1)).to(w.dtype)
+        qp = ops.qparams(*ops.observe_minmax(scaled, args), args)
+        assert bits_equal(out, (ops.fake_quantize(scaled, qp[0], qp[1], args) / s.view(1, -1)).to(w.dtype))
+
+
 # table of powers: every code type, groups and whole rows, symmetric or not, rows that are no multiple of a CTA's
 @pytest.mark.parametrize("scheme", SCHEMES)
 @pytest.mark.parametrize("N,K", [(3, 128), (130, 640)])
