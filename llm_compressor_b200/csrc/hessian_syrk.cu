@@ -684,19 +684,24 @@ __global__ void __launch_bounds__(256) finalize_kernel(float* H0, float* const* 
   if (scales) scale = scales[blockIdx.y];
   // patches of 8 x 8 blocks: what the CTAs write at the same time makes whole 2 KB pieces of rows on both sides of the
   // diagonal (row by row of blocks, the mirrored side got 256-byte pieces 57 KB apart: 316 us at K = 14336)
+  // Bound by HBM: a CTA asks for its next block before it writes this one, without which 14336 columns took 265 us and not 220.
   const int nb = (int)((K + kFinTile - 1) / kFinTile), np = (nb + 7) / 8;
   const int64_t nblk = (int64_t)np * (np + 1) / 2 * 64;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;   // 16 quads of columns x 16 rows
-  for (int64_t blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
-    // blk -> (bi >= bj)
-    const int patch = (int)(blk >> 6), in = (int)blk & 63;
-    int bi = (int)((sqrtf(8.0f * (float)patch + 1.0f) - 1.0f) * 0.5f);
-    while (bi * (bi + 1) / 2 > patch) --bi;
-    while ((bi + 1) * (bi + 2) / 2 <= patch) ++bi;
-    const int bj = (patch - bi * (bi + 1) / 2) * 8 + (in & 7);
-    bi = bi * 8 + (in >> 3);
-    if (bi < bj || bi >= nb) continue;   // CTA-uniform
-    float4 v[4];
+  // the first block from blk on that exists, (bi >= bj); false: none
+  auto locate = [&](int64_t& blk, int& bi, int& bj) {
+    for (; blk < nblk; blk += gridDim.x) {
+      const int patch = (int)(blk >> 6), in = (int)blk & 63;
+      bi = (int)((sqrtf(8.0f * (float)patch + 1.0f) - 1.0f) * 0.5f);
+      while (bi * (bi + 1) / 2 > patch) --bi;
+      while ((bi + 1) * (bi + 2) / 2 <= patch) ++bi;
+      bj = (patch - bi * (bi + 1) / 2) * 8 + (in & 7);
+      bi = bi * 8 + (in >> 3);
+      if (bi >= bj && bi < nb) return true;
+    }
+    return false;
+  };
+  auto fetch = [&](int bi, int bj, float4 (&v)[4]) {
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const int64_t i = (int64_t)bi * kFinTile + ty + 16 * k, j = (int64_t)bj * kFinTile + tx * 4;
@@ -709,8 +714,22 @@ __global__ void __launch_bounds__(256) finalize_kernel(float* H0, float* const* 
             if (j + q < K) e[q] = H[i * ldh + j + q];
         }
       }
-      v[k].x *= scale; v[k].y *= scale; v[k].z *= scale; v[k].w *= scale;
     }
+  };
+  int64_t blk = blockIdx.x;
+  int bi = 0, bj = 0, ni = 0, nj = 0;
+  float4 next[4];
+  bool more = locate(blk, ni, nj);
+  if (more) fetch(ni, nj, next);
+  while (more) {
+    bi = ni; bj = nj;
+    float4 v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      v[k] = make_float4(next[k].x * scale, next[k].y * scale, next[k].z * scale, next[k].w * scale);
+    blk += gridDim.x;
+    more = locate(blk, ni, nj);
+    if (more) fetch(ni, nj, next);   // (asked for before this block is written)
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       float* t = &tile[ty + 16 * k][tx * 4];
