@@ -190,7 +190,7 @@ __device__ __forceinline__ Cand make_cand(float smn, float smx, const Cfg& c) {
   q.slow = !(q.s >= 0x1p-100f && q.s <= 0x1p100f);
   return q;
 }
-// |fake_quantize(x) - x| of a pair, sign bits cleared
+// fake_quantize(x) - x of a pair
 template <int KIND, bool SYM>
 __device__ __forceinline__ uint32_t pair_error(uint32_t w, const Cand& q, uint32_t qmin2, uint32_t qmax2) {
   const uint32_t zero = 0u, magic = 0x43404340u;   // {192, 192}: integers are 1 apart in [128, 256)
@@ -219,8 +219,18 @@ __device__ __forceinline__ uint32_t pair_error(uint32_t w, const Cand& q, uint32
   }
   if (!SYM) v = B200Q_BF2(__hsub2_rn, B200Q_B(v), B200Q_B(q.z2));
   v = B200Q_BF2(__hmul2_rn, B200Q_B(v), B200Q_B(q.s2));
-  v = B200Q_BF2(__hsub2_rn, B200Q_B(v), B200Q_B(w));
-  return v & 0x7FFF7FFFu;
+  return B200Q_BF2(__hsub2_rn, B200Q_B(v), B200Q_B(w));
+}
+// Twice the places of a pair's magnitudes, which are byte offsets: the signs leave at the top of either half.
+__device__ __forceinline__ uint32_t table_offsets(uint32_t d) {
+  const uint32_t i = (d << 1) & 0xFFFEFFFEu;
+  return i ^ ((i >> 4) & 0x0FFE0FFEu);
+}
+__device__ __forceinline__ float add_power(float sum, const unsigned char* tab, uint32_t offset) {
+  unsigned short p = *reinterpret_cast<const unsigned short*>(tab + offset);
+  float r;
+  asm("add.rn.f32.bf16 %0, %1, %2;" : "=f"(r) : "h"(p), "f"(sum));
+  return r;
 }
 // error sum of a chunk of 8 elements, in element order
 template <int KIND, bool SYM>
@@ -236,9 +246,9 @@ __device__ __forceinline__ float chunk_error(const uint32_t (&w)[4], const Cand&
   }
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    const uint32_t d = table_place(pair_error<KIND, SYM>(w[k], q, qmin2, qmax2));
-    err += __uint_as_float((uint32_t)tab[d & 0xFFFFu] << 16);
-    err += __uint_as_float((uint32_t)tab[d >> 16] << 16);
+    const uint32_t d = table_offsets(pair_error<KIND, SYM>(w[k], q, qmin2, qmax2));
+    err = add_power(err, reinterpret_cast<const unsigned char*>(tab), d & 0xFFFFu);
+    err = add_power(err, reinterpret_cast<const unsigned char*>(tab), d >> 16);
   }
   return err;
 }
