@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(256) mse_group_kernel(const void* __restrict__
 // so its rounded power is one of 32768: a table in shared memory, made once per call with powf.
 //
 // What bounds it: the table look-ups (about three cycles a warp, bank conflicts of 32 random entries) and about ten
-// instructions an element.  Evaluating exp2(norm * log2 d) instead costs two special-function results, checks against
+// instructions an element (4096 x 4096, groups of 128, 20 candidates: 186 us).  Evaluating exp2(norm * log2 d) instead costs two special-function results, checks against
 // rounding midpoints and a fallback: 685 us for 20 candidates on 4096 x 4096.
 constexpr int kTable = 32768;
 constexpr size_t kTableBytes = kTable * 2;

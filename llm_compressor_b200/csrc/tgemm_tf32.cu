@@ -669,7 +669,13 @@ int split_rows16(const float* src, int64_t ld_src, int64_t src_batch, int64_t ro
 }
 int split_update16(const UpdateOperand& u, int batch, cudaStream_t st) {
   const size_t smem = split_columns16_smem(kMaxDepth);
-  B200Q_TRY(cudaFuncSetAttribute(split_update16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  static thread_local int attr_device = -1;
+  int dev = 0;
+  B200Q_TRY(cudaGetDevice(&dev));
+  if (attr_device != dev) {
+    B200Q_TRY(cudaFuncSetAttribute(split_update16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    attr_device = dev;
+  }
   const int transposed = (int)((u.end + 31) / 32);
   const int64_t blocks = (u.first + u.rows + 7) / 8, cap = 3 * kNumSMs / batch + 1;
   B200Q_TRY(launch_chained(split_update16_kernel, dim3((unsigned)(transposed + (blocks < cap ? blocks : cap)), (unsigned)batch), 256,
@@ -838,14 +844,16 @@ int launch(const Job& j, cudaStream_t st) {
   const int most = pair ? pairs : ctas;
   const int units = (int)(p.num_tiles < most ? p.num_tiles : most);
   // where each CTA's (pair's) range starts: problem, row tile, column tile
-  int tm = 0;
-  int64_t before = 0, of = 0;   // tiles before row tile tm of problem `of`
+  // (without divisions: two of 64 bits for each of 148 took longer than the launch itself)
+  const int64_t share = p.num_tiles / units, rest = p.num_tiles % units;
+  int tm = 0, n = col_tiles(j, 0, p.tm_rows, p.tn_log2);
+  int64_t in = 0, before = 0, part = 0, b = 0;   // tile i * num_tiles / units of problem b, tiles before row tile tm
   for (int i = 0; i < units; ++i) {
-    const int64_t t = p.num_tiles * i / units, b = t / per_problem, in = t - b * per_problem;
-    if (b != of) { of = b; tm = 0; before = 0; }
-    int64_t n;
-    while (in >= before + (n = col_tiles(j, tm, p.tm_rows, p.tn_log2))) { before += n; ++tm; }
+    while (in >= per_problem) { in -= per_problem; ++b; tm = 0; before = 0; n = col_tiles(j, 0, p.tm_rows, p.tn_log2); }
+    while (in >= before + n) { before += n; n = col_tiles(j, ++tm, p.tm_rows, p.tn_log2); }
     p.start[i][0] = (uint16_t)b; p.start[i][1] = (uint16_t)tm; p.start[i][2] = (uint16_t)(in - before);
+    in += share;
+    if ((part += rest) >= units) { part -= units; ++in; }
   }
   const bool split_out = j.out_hi || j.X;
 #define B200Q_TILES(TN, PAIR)                                                                             \
