@@ -133,16 +133,17 @@ __device__ __forceinline__ void mma_block(const float* A, int lda, const float* 
 //
 // Sixteen warps.  The elimination and what follows it in the same step are the chain; the update of the step before has to
 // be through in that time, and warps on the eliminating warp's scheduler slow it down, so the twelve on the other three
-// take it.  Cycles, clocks read in the kernel: 2700 until the block is there, steps of 2600 to 3300 (the diagonal block's
-// update 360, its elimination 1300 to 2100, the more the longer the others are at their tiles: shuffles and shared-memory
-// loads share a pipe; substitution and operands 800), 1900 out; 29500 in all, 32200 with eight warps and tf32 pairs.
+// take it.  Cycles, clocks read in the kernel: 2700 until the block is there, steps of 2600 to 3200 (the diagonal block's
+// update 330, its elimination 1270 to 1500, substitution and operands 800; in the longer steps 400 until the others are
+// through), 1900 out; 28700 in all, 32200 with eight warps and tf32 pairs.
 constexpr int W16 = 16;
 constexpr int kCholThreads = 512;
 // A step's 128 active rows as operands: 16 hi and 16 lo halves and a power of two per row (tgemm::Operand), in rows of 80 bytes,
 // which ldmatrix reads without bank conflicts.  The rows are written once and read by up to ten products: split by every
 // reader into tf32 pairs, the update of a step took 3300 cycles, longer than the chain beside it.
 constexpr int kOpBytes = 80;
-constexpr int kCholSmemFloats = 2 * NB * LD + W16 * 20 + W16 + NB * kOpBytes / 4 + NB;
+constexpr int CLD = NB + 8;   // stride of the diagonal block's rows: a tile's pairs of columns conflict-free
+constexpr int kCholSmemFloats = 2 * NB * CLD + W16 * 20 + W16 + NB * kOpBytes / 4 + NB;
 
 __device__ __forceinline__ void ldmatrix4(uint32_t addr, uint32_t (&r)[4]) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
@@ -162,7 +163,7 @@ __device__ __forceinline__ void subtract_product(float* o, uint32_t op, const fl
   for (int j = 0; j < NT; ++j)
 #pragma unroll
     for (int h = 0; h < 2; ++h)
-      if (j < tiles) old[j][h] = *reinterpret_cast<float2*>(o + h * 8 * LD + 8 * j);
+      if (j < tiles) old[j][h] = *reinterpret_cast<float2*>(o + h * 8 * CLD + 8 * j);
   uint32_t ah[4], al[4], bh[NT / 2][4], bl[NT / 2][4];
   const uint32_t a = op + (ra + (lane & 15)) * kOpBytes + (lane >> 4) * 16;
   const uint32_t b = op + (rb + (lane & 7) + (lane >> 4) * 8) * kOpBytes + ((lane >> 3) & 1) * 16;
@@ -185,19 +186,19 @@ __device__ __forceinline__ void subtract_product(float* o, uint32_t op, const fl
     mma_f16(y, al, bh[j / 2][e], bh[j / 2][e + 1]);
     const float2 sc = *reinterpret_cast<const float2*>(scale + rb + 8 * j + 2 * (lane & 3));
     *reinterpret_cast<float2*>(o + 8 * j) = make_float2(fmaf(-(x[0] + y[0]) * s0, sc.x, old[j][0].x), fmaf(-(x[1] + y[1]) * s0, sc.y, old[j][0].y));
-    *reinterpret_cast<float2*>(o + 8 * LD + 8 * j) = make_float2(fmaf(-(x[2] + y[2]) * s1, sc.x, old[j][1].x), fmaf(-(x[3] + y[3]) * s1, sc.y, old[j][1].y));
+    *reinterpret_cast<float2*>(o + 8 * CLD + 8 * j) = make_float2(fmaf(-(x[2] + y[2]) * s1, sc.x, old[j][1].x), fmaf(-(x[3] + y[3]) * s1, sc.y, old[j][1].y));
   }
 }
 
 // active row block s (0..7) of step kb: identity rows up to kb, whose inverse is being born, matrix rows after it
 __device__ __forceinline__ float* active_row(float* R, int ar, int kb) {
-  return R + ((ar >> 4) <= kb ? NB + ar : ar) * LD;
+  return R + ((ar >> 4) <= kb ? NB + ar : ar) * CLD;
 }
 
 __global__ void __launch_bounds__(kCholThreads, 1) chol_diag_kernel(Mat mt, int k0, int n) {
   extern __shared__ __align__(16) float sm[];
   float* R = sm;                    // rows 0..127: the block, then L; rows 128..255: the identity, then L^-T
-  float* Lt = R + 2 * NB * LD;      // [16][20] transposed diagonal block of the step
+  float* Lt = R + 2 * NB * CLD;      // [16][20] transposed diagonal block of the step
   float* rinv = Lt + W16 * 20;      // [16]
   float* scale = rinv + W16;        // [128] inverse powers of the operand rows
   unsigned char* rows_op = reinterpret_cast<unsigned char*>(scale + NB);
@@ -208,14 +209,14 @@ __global__ void __launch_bounds__(kCholThreads, 1) chol_diag_kernel(Mat mt, int 
   for (int idx = tid; idx < NB * NB / 4; idx += kCholThreads) {
     const int r = idx >> 5, c = (idx & 31) << 2;
     const float4 id = make_float4(c == r ? 1.f : 0.f, c + 1 == r ? 1.f : 0.f, c + 2 == r ? 1.f : 0.f, c + 3 == r ? 1.f : 0.f);
-    if (c <= r && r >= n) *reinterpret_cast<float4*>(R + r * LD + c) = id;   // identity padding beyond n
-    if (c >= (r & ~(W16 - 1))) *reinterpret_cast<float4*>(R + (NB + r) * LD + c) = id;
+    if (c <= r && r >= n) *reinterpret_cast<float4*>(R + r * CLD + c) = id;   // identity padding beyond n
+    if (c >= (r & ~(W16 - 1))) *reinterpret_cast<float4*>(R + (NB + r) * CLD + c) = id;
   }
   chain_wait();
 #pragma unroll
   for (int i = 0; i < NB * NB / 4 / kCholThreads; ++i) {
     const int idx = tid + i * kCholThreads, r = idx >> 5, c = (idx & 31) << 2;
-    if (c <= r && r < n) cp_async16(R + r * LD + c, A + (int64_t)r * mt.lda + c, 16);   // (rows are padded to 32)
+    if (c <= r && r < n) cp_async16(R + r * CLD + c, A + (int64_t)r * mt.lda + c, 16);   // (rows are padded to 32)
   }
   cp_async_wait_all();
   __syncthreads();
@@ -225,11 +226,11 @@ __global__ void __launch_bounds__(kCholThreads, 1) chol_diag_kernel(Mat mt, int 
     const int c0 = kb * W16, p0 = c0 - W16;
     if (warp == 0) {
       if (kb > 0) {   // the diagonal block takes the step before
-        subtract_product<2>(R + (c0 + (lane >> 2)) * LD + c0 + 2 * (lane & 3), op, scale, c0, c0, 2, lane);
+        subtract_product<2>(R + (c0 + (lane >> 2)) * CLD + c0 + 2 * (lane & 3), op, scale, c0, c0, 2, lane);
         __syncwarp();
       }
       float a[W16], ri;
-      const float* src = R + (c0 + (lane & 15)) * LD + c0;
+      const float* src = R + (c0 + (lane & 15)) * CLD + c0;
       // the first pivot that `Exact` does not accept, + 1: the quick form takes positive normal numbers, the exact one
       // (rare, so out of the way) everything above zero.  Garbage from that pivot on.
       auto eliminate = [&](auto Exact) -> int {
@@ -240,10 +241,17 @@ __global__ void __launch_bounds__(kCholThreads, 1) chol_diag_kernel(Mat mt, int 
           const float4 v = *reinterpret_cast<const float4*>(src + 4 * q);
           a[4 * q] = v.x; a[4 * q + 1] = v.y; a[4 * q + 2] = v.z; a[4 * q + 3] = v.w;
         }
-        float piv = __shfl_sync(0xffffffffu, a[0], 0);
+        // Column j reaches column j + 1 by one shuffle, and the pivot there, t - x^2, is formed by every lane for itself; the
+        // columns behind take it from shared memory a column later, four a load.  (A shuffle for each of them: they and the
+        // other warps' loads share a pipe, 1300 to 2100 cycles
+        // for the 16 columns; now 1270 to 1500.)
+        float t = __shfl_sync(0xffffffffu, a[0], 0), l = 0.0f;
 #pragma unroll
         for (int j = 0; j < W16; ++j) {
-          float l, root;   // 1 / sqrt(piv)
+          const float x = j ? __shfl_sync(0xffffffffu, l, j) : 0.0f;
+          const float piv = fmaf(-x, x, t);
+          a[j] = fmaf(-l, x, a[j]);
+          float root;   // 1 / sqrt(piv)
           if constexpr (Exact) {
             first = (!(piv > 0.0f) && first == 0) ? j + 1 : first;
             root = __fdiv_rn(1.0f, __fsqrt_rn(piv));
@@ -257,11 +265,22 @@ __global__ void __launch_bounds__(kCholThreads, 1) chol_diag_kernel(Mat mt, int 
             l = (a[j] * r) * u;
             root = r * u;
           }
-          if (j + 1 < W16) piv = __shfl_sync(0xffffffffu, fmaf(-l, l, a[j + 1]), j + 1);
           a[j] = l;
           ri = (lane == j) ? root : ri;
+          if (j + 2 < W16) {
+            Lt[j * 20 + (lane & 15)] = l;
+            __syncwarp();
 #pragma unroll
-          for (int c = j + 1; c < W16; ++c) a[c] = fmaf(-l, __shfl_sync(0xffffffffu, l, c), a[c]);
+            for (int q = (j + 2) / 4; q < 4; ++q) {
+              const float4 v = *reinterpret_cast<const float4*>(Lt + j * 20 + 4 * q);
+              const float e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+              for (int k = 0; k < 4; ++k)
+                if (4 * q + k >= j + 2) a[4 * q + k] = fmaf(-l, e[k], a[4 * q + k]);
+            }
+          }
+          // (of the next column's own row, without this column yet)
+          if (j + 1 < W16) t = __shfl_sync(0xffffffffu, a[j + 1], j + 1);
         }
         return first;
       };
@@ -279,7 +298,8 @@ __global__ void __launch_bounds__(kCholThreads, 1) chol_diag_kernel(Mat mt, int 
       // on and below the diagonal.  A warp takes 16 rows x 32 columns at a time.
       // Task list: kb identity row blocks with `wide` pairs of column blocks each, then matrix row blocks r = 0, 1, ...
       // (s = kb + r) with r / 2 + 1 pairs.  (Counted out in closed form: a loop over all tasks that skips the other
-      // warps' costs 180 cycles a skip, mostly instruction fetch.)
+      // warps' costs 180 cycles a skip, mostly instruction fetch.  From a table the first task of a step begins 300 cycles
+      // sooner and takes 460 longer: what the tasks wait for is one another's loads, stores and products.)
       const int wide = (9 - kb) / 2, left = kb * wide, half = (8 - kb) / 2;
       const int all = left + half * (half + 1) + (kb & 1) * (half + 1);
       for (int t = (warp >> 2) * 3 + (warp & 3) - 1; t < all; t += 12) {
@@ -295,7 +315,7 @@ __global__ void __launch_bounds__(kCholThreads, 1) chol_diag_kernel(Mat mt, int 
         const int cc = c0 + g * 32, last = matrix ? s * W16 : NB - W16;   // first column of the last block of 16 to take
         // (the diagonal block itself is the first warp's)
         const int tiles = matrix && s == kb ? 0 : min(4, (last + W16 - cc) / 8);
-        subtract_product<4>(R + ((matrix ? 0 : NB) + s * W16 + (lane >> 2)) * LD + cc + 2 * (lane & 3), op, scale, s * W16, cc,
+        subtract_product<4>(R + ((matrix ? 0 : NB) + s * W16 + (lane >> 2)) * CLD + cc + 2 * (lane & 3), op, scale, s * W16, cc,
                             tiles, lane);
       }
     }
@@ -355,7 +375,7 @@ __global__ void __launch_bounds__(kCholThreads, 1) chol_diag_kernel(Mat mt, int 
     float v[4][4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const float4 q = *reinterpret_cast<const float4*>(R + (NB + i + k) * LD + j);
+      const float4 q = *reinterpret_cast<const float4*>(R + (NB + i + k) * CLD + j);
       v[k][0] = q.x; v[k][1] = q.y; v[k][2] = q.z; v[k][3] = q.w;
     }
 #pragma unroll
