@@ -525,36 +525,37 @@ __global__ void __launch_bounds__(kThreads) square_update_kernel(Mat mt, const f
 }
 
 // ---------------------------------------------------------------------------------------
-// Operand form of D (the square's inverse, zero above the diagonal) as rows.
-__global__ void __launch_bounds__(256) split_square_kernel(Mat mt, int K0, int n, float* d_hi, float* d_lo) {
-  chain_wait();
-  chain_go();
-  const float* A = mt.A + blockIdx.y * mt.batch + (int64_t)K0 * mt.lda + K0;
-  const int64_t db = (int64_t)blockIdx.y * OB * OB;
-  const int tr = blockIdx.x >> 4, tc = blockIdx.x & 15, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int r = tr * 32 + ty + 8 * i, c = tc * 32 + tx;
-    const float x = (r < n && c <= r) ? A[(int64_t)r * mt.lda + c] : 0.0f;
-    const float h = tgemm::tf32_rn(x);
-    d_hi[db + (int64_t)r * OB + c] = h;
-    d_lo[db + (int64_t)r * OB + c] = tgemm::tf32_rn(x - h);
-  }
-}
-
 // Rows [r0, r1) of the panel A[:, K0 : K0 + n] as they are, and columns [0, tcols) of the block row S[K0 : K0 + n, :]
-// transposed; operand row = matrix row or column, zero-padded to 32.
+// transposed; operand row = matrix row or column, zero-padded to 32.  The first `squares` CTAs, if any, make the operand form
+// of D (the square's inverse, zero above the diagonal) as rows instead: what the chain needs before the next block's rows of P,
+// in one launch.
+constexpr int kSquareCtas = OB / 32 * (OB / 32);
+struct SquareForm { float *hi, *lo; int ctas; };
 __global__ void __launch_bounds__(256) split_panel_kernel(Mat mt, int K0, int n, int r0, int r1, int tcols, float* hi,
-                                                          float* lo, int64_t dst_batch) {
+                                                          float* lo, int64_t dst_batch, const SquareForm square) {
   chain_wait();
   chain_go();
   __shared__ float tile[32][33];
   const float* A = mt.A + blockIdx.y * mt.batch;
+  if ((int)blockIdx.x < square.ctas) {
+    const float* S = A + (int64_t)K0 * mt.lda + K0;
+    const int64_t db = (int64_t)blockIdx.y * OB * OB;
+    const int tr = blockIdx.x >> 4, tc = blockIdx.x & 15, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = tr * 32 + ty + 8 * i, c = tc * 32 + tx;
+      const float x = (r < n && c <= r) ? S[(int64_t)r * mt.lda + c] : 0.0f;
+      const float h = tgemm::tf32_rn(x);
+      square.hi[db + (int64_t)r * OB + c] = h;
+      square.lo[db + (int64_t)r * OB + c] = tgemm::tf32_rn(x - h);
+    }
+    return;
+  }
   hi += blockIdx.y * dst_batch;
   lo += blockIdx.y * dst_batch;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int depth = (n + 31) / 32, direct = (r1 - r0 + 31) / 32 * depth, all = direct + tcols / 32 * depth;
-  for (int t = blockIdx.x; t < all; t += gridDim.x) {
+  for (int t = blockIdx.x - square.ctas; t < all; t += gridDim.x - square.ctas) {
     const bool rows = t < direct;
     const int u = rows ? t : t - direct, line = u / depth, m0 = (u - line * depth) * 32;
     float x[4];
@@ -726,13 +727,13 @@ static int factor(float* H, float* const* Hs, int batch, int64_t order, int64_t 
         F{f_hi, f_lo, OB, (int64_t)batch * OB, OB, 0}, Q{q_hi, q_lo, OB, (int64_t)batch * rows, rows, 0, q_scale};
     const int n2 = last ? 0 : (int)(K - K1 < OB ? K - K1 : OB);
     if (side_busy) B200Q_TRY(cudaStreamWaitEvent(st, side->done, 0));   // products of the step before
-    B200Q_TRY(launch_chained(split_square_kernel, dim3(OB / 32 * (OB / 32), batch), 256, 0, st, mt, (int)K0, n, d_hi, d_lo));
-    B200Q_LAUNCH_CHECK();
-    auto split_panel = [&](int64_t r0, int64_t r1, int64_t tcols, cudaStream_t on) -> int {
+    auto split_panel = [&](int64_t r0, int64_t r1, int64_t tcols, bool square, cudaStream_t on) -> int {
       const int64_t tiles = ((r1 - r0 + 31) / 32 + tcols / 32) * ((n + 31) / 32);
-      if (tiles == 0) return B200Q_OK;
-      B200Q_TRY(launch_chained(split_panel_kernel, grid(tiles, row_ctas), 256, 0, on, mt, (int)K0, n, (int)r0, (int)r1, (int)tcols, a_hi,
-                               a_lo, pb));
+      if (tiles == 0 && !square) return B200Q_OK;
+      const SquareForm form{d_hi, d_lo, square ? kSquareCtas : 0};
+      dim3 g = tiles ? grid(tiles, row_ctas) : dim3(0, (unsigned)batch, 1);
+      g.x += form.ctas;
+      B200Q_TRY(launch_chained(split_panel_kernel, g, 256, 0, on, mt, (int)K0, n, (int)r0, (int)r1, (int)tcols, a_hi, a_lo, pb, form));
       B200Q_LAUNCH_CHECK();
       return B200Q_OK;
     };
@@ -741,7 +742,7 @@ static int factor(float* H, float* const* Hs, int batch, int64_t order, int64_t 
     j.out_ld = OB; j.out_batch = pb; j.slice = slice;
     if (!last) {
       // the next block's rows of P and its square: all the chain needs
-      B200Q_RC(split_panel(K1, K1 + n2, 0, st));
+      B200Q_RC(split_panel(K1, K1 + n2, 0, true, st));
       if (side) {
         B200Q_TRY(cudaEventRecord(side->ready, st));
         B200Q_TRY(cudaStreamWaitEvent(bulk, side->ready, 0));
@@ -760,7 +761,7 @@ static int factor(float* H, float* const* Hs, int batch, int64_t order, int64_t 
     }
     // the other rows of P, and X[o,:o] with its transpose
     const int64_t left = blocks ? 0 : K0;   // columns before the square that take part
-    B200Q_RC(split_panel(K1 + n2, K, left, bulk));
+    B200Q_RC(split_panel(K1 + n2, K, left, last, bulk));
     Job r = j;
     r.set = tgemm::kPanel; r.skip0 = (int)left; r.skip1 = (int)(K1 + n2); r.M = (int)K;
     if (!last) r.out_hi = p_all;
