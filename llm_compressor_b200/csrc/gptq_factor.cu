@@ -24,8 +24,8 @@
 // beside them S as step o leaves it, -V[:o,o] U_oo, which no later step touches.  Then neither X[o,:o] nor S[i,:o] -= P_i X
 // is computed, 1/3 K^3 instead of 2/3 K^3 (gptq_sweep.cu: products across superblocks take w - q in place of the errors).
 // Its squares are the superblocks of the sweep, so the short one comes first, and the matrix begins with as many rows of the
-// identity as make its order a multiple of 32.  K = 14336: 6.6 ms (U: 9.7), 8192: 2.62 (2.92), 4096: 1.16 (1.22), 768: 0.215
-// (0.245).
+// identity as make its order a multiple of 32.  K = 14336: 6.2 ms (U: 9.7), 4096: 1.04 (1.10), 2048: 0.50 (0.53),
+// 1160: 0.31 (0.34).
 //
 // A pivot <= 0 (or NaN) sets the problem's status; the host then takes the reference's identity fallback.
 #include <type_traits>
